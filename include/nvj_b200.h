@@ -100,6 +100,18 @@ int nvj_kv_append(const void* new_k, const void* new_v, int src_dtype,
                   int32_t* status, nvj_stream_t stream);
 
 /*
+ * nvj_kv_append with the slots made on the way: token i goes where nvj_compute_slot_mapping(positions, block_tables,
+ * token_row_ids, ...) would send it, so that a step whose slot mapping nobody else reads needs no launch for it.
+ * num_slots = num_blocks * block_size; the valid rules are nvj_kv_append's without the explicit mask.
+ */
+int nvj_kv_append_mapped(const void* new_k, const void* new_v, int src_dtype, const int32_t* positions,
+                         const int32_t* block_tables, const int32_t* token_row_ids, int table_rows,
+                         int table_width, int block_size, const int32_t* query_start_loc, int qsl_rows,
+                         int packed, int n_rows, int n_cols, void* k_cache_layer, void* v_cache_layer,
+                         int cache_dtype, int64_t num_slots, int num_kv_heads, int head_dim,
+                         int32_t* status, nvj_stream_t stream);
+
+/*
  * Page-table (CSR) form of the append: page = kv_indices[kv_indptr[b] + pos / P],
  * cache[page, pos % P] = append[i].  Replaces the FP32 custom call
  * nanovllm_jax/kernels/cuda_fp32_ffi.py:323-382 (handler
@@ -289,6 +301,20 @@ int nvj_paged_decode_wide(const void* q, const void* k_cache_layer, const void* 
                           const int32_t* seq_lens, const int32_t* positions, int batch, int width,
                           float scale, float* out, void* workspace, size_t workspace_bytes,
                           nvj_stream_t stream);
+
+/*
+ * Decode attention over a window, for rows of `width` query tokens whose K/V are already appended: token t of row b
+ * attends keys p < min(seq_lens[b], max_kv_len) (0: no bound) and, with positions given, p <= positions[b * width + t].
+ * The masks of nanovllm_jax/kv_cache.py:852-998 (paged_attention_decode) in one call: no launch in front clips the
+ * lengths.  Width 1 takes every shape and dtype of nvj_paged_decode, wider rows what nvj_paged_decode_wide takes;
+ * workspace of nvj_paged_decode_wide_workspace_bytes.
+ */
+int nvj_paged_decode_window(const void* q, int q_dtype, const void* k_cache_layer, const void* v_cache_layer,
+                            int kv_dtype, int64_t num_blocks, int block_size, int num_kv_heads, int head_dim,
+                            int num_q_heads, const int32_t* block_tables, int table_width,
+                            const int32_t* seq_lens, const int32_t* positions, int batch, int width,
+                            int max_kv_len, float scale, float* out, void* workspace, size_t workspace_bytes,
+                            nvj_stream_t stream);
 
 /* ----------------------------------------------------------------- prefill */
 

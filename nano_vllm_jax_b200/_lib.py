@@ -42,6 +42,12 @@ SIGNATURES = {
                                       c_int, c_int, c_float, c_void_p, c_void_p, c_size_t, c_void_p]),
     "nvj_paged_decode_wide_form": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_void_p, c_void_p,
                                            c_int, c_int, c_float, c_void_p, c_void_p, c_size_t, c_int, c_void_p]),
+    "nvj_kv_append_mapped": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
+                                     c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int64, c_int, c_int,
+                                     c_void_p, c_void_p]),
+    "nvj_paged_decode_window": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_int, c_int,
+                                        c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p,
+                                        c_void_p, c_size_t, c_void_p]),
     "nvj_paged_decode": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int64, c_int, c_int,
                                  c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
                                  c_float, c_void_p, c_void_p, c_size_t, c_int, c_void_p]),
@@ -110,6 +116,8 @@ def load() -> ctypes.CDLL:
             return _lib
         if os.environ.get("NVJ_FORCE_REBUILD", "0") == "1" or not _build.LIB_PATH.exists():
             _build.build(force=True)
+        elif not _build.HOST_PATH.exists():
+            _build.build_host()
         lib = ctypes.CDLL(str(_build.LIB_PATH), mode=ctypes.RTLD_GLOBAL)
         for name, (restype, argtypes) in SIGNATURES.items():
             fn = getattr(lib, name)  # AttributeError here = header and library disagree

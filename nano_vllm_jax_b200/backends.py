@@ -105,17 +105,27 @@ class B200Backend:
                 raise ValueError("token_row_ids and positions must have matching shapes")
             if seq_lens.shape[0] != block_tables.shape[0]:
                 raise ValueError("seq_lens shape must align with packed prefill rows")
-            slot_mapping = kvc.compute_packed_slot_mapping(positions, block_tables, token_row_ids, block_size)
+            if block_size <= 0:
+                raise ValueError("block_size must be positive")
         else:
             if positions.shape[0] != block_tables.shape[0]:
                 raise ValueError("positions and block_tables batch dimensions must match")
             if positions.shape[0] != seq_lens.shape[0]:
                 raise ValueError("positions and seq_lens batch dimensions must match")
-            if is_prefill:
-                slot_mapping = kvc.compute_slot_mapping(positions, block_tables, block_size, is_prefill)
-            else:  # decode: made when first read (the fused append + decode kernel never reads it)
-                slot_mapping = lambda: kvc.compute_slot_mapping(positions, block_tables, block_size, is_prefill)  # noqa: E731
+        if is_prefill:
+            _k._cuda("positions", positions)
+            _k._cuda("block_table", block_tables)
+        # made when first read: the fused append + decode kernel and the plain append resolve the slots themselves
+        slot_mapping = kvc.SlotsFromTables(positions, block_tables, block_size, token_row_ids)
         batch, query_len = positions.shape
+        singles = pairs = None
+        if query_lens_host is not None and token_row_ids is not None:
+            singles = pairs = 0
+            for n in query_lens_host:
+                if n == 1:
+                    singles += 1
+                elif n > 1:
+                    pairs -= -int(n) // 64
         if query_start_loc is None:
             if is_prefill:
                 query_start_loc = torch.cat([torch.zeros(1, dtype=torch.int32, device=seq_lens.device),
@@ -136,13 +146,19 @@ class B200Backend:
             max_kv_len=block_tables.shape[1] * block_size if not is_prefill else None,
             token_row_ids=token_row_ids,
             max_query_len=max_query_len if max_query_len is not None else query_len,
-            single_token_rows=(sum(1 for n in query_lens_host if int(n) == 1)
-                               if (query_lens_host is not None and token_row_ids is not None) else None),
-            query_tile_pairs=(sum(-(-int(n) // 64) for n in query_lens_host if int(n) > 1)
-                              if (query_lens_host is not None and token_row_ids is not None) else None))
+            single_token_rows=singles, query_tile_pairs=pairs)
 
     # ---- append (backends.py:980-1067)
     def write_kv(self, layer_id, k, v, cache: KVCacheStorage, metadata: AttentionMetadata) -> KVCacheStorage:
+        unread = metadata.__dict__["slot_mapping"]
+        if type(unread) is kvc.SlotsFromTables:
+            done = _k.host().append(k, v, cache.k_cache, cache.v_cache, layer_id, None, unread.positions, unread.block_tables,
+                                    unread.token_row_ids, metadata.query_start_loc, unread.block_size)
+        else:
+            done = _k.host().append(k, v, cache.k_cache, cache.v_cache, layer_id, unread, None, None, metadata.token_row_ids,
+                                    metadata.query_start_loc, 0)
+        if done:
+            return KVCacheStorage(cache.k_cache, cache.v_cache)
         k_layer, _ = kvc._resolve_kv_layer(cache.k_cache, layer_id)
         v_layer, _ = kvc._resolve_kv_layer(cache.v_cache, layer_id)
         sm = metadata.slot_mapping.to(torch.int32)
@@ -186,6 +202,10 @@ class B200Backend:
         fused = (not is_prefill and query.shape[1] == 1 and k.shape[1] == 1 and v.shape[1] == 1
                  and cache.k_cache.ndim == 5 and metadata.positions is not None)
         if fused:
+            out = _k.host().fused_decode(query, k, v, cache.k_cache, cache.v_cache, metadata.block_tables, metadata.seq_lens,
+                                         metadata.positions, layer_id, block_size, scale, num_key_value_groups, 0)
+            if out is not None:
+                return KVCacheStorage(cache.k_cache, cache.v_cache), out
             out, k_cache, v_cache = _k.paged_decode_attention_with_kv_append(
                 query, k, v, cache.k_cache, cache.v_cache, metadata.block_tables.to(torch.int32),
                 metadata.seq_lens.to(torch.int32), metadata.positions, layer_id, block_size, scale,

@@ -3,22 +3,28 @@
 `build()` compiles every `.cu` file under `csrc/` (one object each, in parallel) and links them into
 `nano_vllm_jax_b200/libnvj_b200.so` (next to this file, so the built library
 travels with a snapshot of the source tree) and is a no-op when the library is
-newer than every source.  The pattern follows the reference's build-on-import of
+newer than every source.  Beside it, `build_host()` compiles `csrc/host/host_ops.cpp`
+(the host side of the hot calls, against torch's C++ headers) into the Python
+extension module `_nvj_host.so`; `build()` does both.  The pattern follows the reference's build-on-import of
 its own CUDA FFI library (nanovllm_jax/kernels/cuda_fp32_ffi.py:121-178) with the
 architecture fixed to sm_100a.
 """
 
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
+import sysconfig
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 INCLUDE = PKG_DIR.parent / "include"
 LIB_PATH = PKG_DIR / "libnvj_b200.so"
+HOST_SRC = CSRC / "host" / "host_ops.cpp"
+HOST_PATH = PKG_DIR / "_nvj_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -49,12 +55,36 @@ def nvcc_path() -> str | None:
     )
 
 
+def build_host(force: bool = False) -> Path:
+    """Compile the host extension module if needed and return its path."""
+    newest = max(p.stat().st_mtime for p in (HOST_SRC, INCLUDE / "nvj_b200.h"))
+    if not force and HOST_PATH.exists() and HOST_PATH.stat().st_mtime > newest:
+        return HOST_PATH
+    spec = importlib.util.find_spec("torch")
+    if spec is None or not spec.submodule_search_locations:
+        raise RuntimeError("torch not found: cannot build _nvj_host.so")
+    torch_dir = Path(spec.submodule_search_locations[0])
+    nvcc = nvcc_path()
+    cuda_include = Path(nvcc).resolve().parents[1] / "include" if nvcc else Path("/usr/local/cuda/include")
+    part = HOST_PATH.with_suffix(f".{os.getpid()}.part")  # moved into place whole: another process may be loading the old one
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-I", str(torch_dir / "include"), "-I", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"),
+           "-I", str(cuda_include), "-I", sysconfig.get_paths()["include"], "-o", str(part), str(HOST_SRC),
+           "-L", str(torch_dir / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError("g++ failed on host_ops.cpp:\n" + proc.stdout + proc.stderr)
+    part.replace(HOST_PATH)
+    return HOST_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile the library if needed and return its path.
+    """Compile the library and the host module if needed and return the library's path.
 
     Every `.cu` file becomes one object under `build/` (compiled in parallel, recompiled when the
     file or any header is newer than its object); the objects are then linked into the library.
     """
+    build_host(force)
     if not force and not _stale():
         return LIB_PATH
     nvcc = nvcc_path()

@@ -138,3 +138,38 @@ extern "C" int nvj_paged_decode_fused_append(const void* q, int q_dtype, const v
   p.scale = scale;
   return nvj::run_decode(p, workspace, workspace_bytes, variant, static_cast<cudaStream_t>(stream));
 }
+
+extern "C" int nvj_paged_decode_window(const void* q, int q_dtype, const void* k_cache_layer, const void* v_cache_layer,
+                                       int kv_dtype, int64_t num_blocks, int block_size, int num_kv_heads, int head_dim,
+                                       int num_q_heads, const int32_t* block_tables, int table_width,
+                                       const int32_t* seq_lens, const int32_t* positions, int batch, int width,
+                                       int max_kv_len, float scale, float* out, void* workspace, size_t workspace_bytes,
+                                       nvj_stream_t stream) {
+  using namespace nvj;
+  if (width < 1 || max_kv_len < 0) return NVJ_ERR_INVALID_ARGUMENT;
+  DecodeParams p{};
+  p.max_len = max_kv_len;
+  p.q = q;
+  p.k_cache = static_cast<const char*>(k_cache_layer);
+  p.v_cache = static_cast<const char*>(v_cache_layer);
+  p.block_tables = block_tables;
+  p.seq_lens = seq_lens;
+  p.out = out;
+  p.num_blocks = num_blocks;
+  p.batch = batch;
+  p.table_width = table_width;
+  p.block_size = block_size;
+  p.num_kv_heads = num_kv_heads;
+  p.num_q_heads = num_q_heads;
+  p.head_dim = head_dim;
+  p.q_dtype = q_dtype;
+  p.kv_dtype = kv_dtype;
+  p.scale = scale;
+  if (width == 1) {
+    p.cap_positions = positions;
+    return run_decode(p, workspace, workspace_bytes, 0, static_cast<cudaStream_t>(stream));
+  }
+  p.positions = positions;
+  p.width = width;
+  return run_decode_wide(p, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}

@@ -1,0 +1,494 @@
+// The host side of the path's hot calls: argument checks, output allocation and the C-ABI call in one crossing from
+// Python.  A decode step of a few rows keeps the GPU busy for ~10 us; the same steps in Python (tensor views and
+// conversions, environment look-ups, a foreign-function call of 25 arguments) took 45-55 us per call.
+//
+// Every function takes tensors as they come from the caller and serves the regular case only: CUDA tensors on one
+// device, int32 metadata, contiguous operands of the expected dtypes.  Anything else returns None and launches
+// nothing; the caller then takes the Python route, which converts what can be converted and raises what must be
+// raised, so that errors and results are the same whichever route a call takes.
+//
+// The entry points of libnvj_b200.so are resolved from the handle that Python has loaded.  Workspaces and status words
+// belong to Python (one per device and stream); this module keeps references to them.
+
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#include "../../../include/nvj_b200.h"
+
+namespace {
+
+// ---- what Python hands over once ------------------------------------------------------------------------------
+
+struct Library {
+  decltype(&nvj_paged_decode_fused_append) fused_append;
+  decltype(&nvj_paged_decode_window) window;
+  decltype(&nvj_kv_append) append;
+  decltype(&nvj_kv_append_mapped) append_mapped;
+  decltype(&nvj_paged_prefill_packed) prefill;
+  decltype(&nvj_paged_prefill_packed_part) prefill_part;
+  decltype(&nvj_qk_norm_rope_kv_append) norm_rope;
+  decltype(&nvj_compute_slot_mapping) slot_mapping;
+};
+Library lib;
+PyObject* cb_workspace;  // (device index, rows): makes Python create the workspace and hand it over
+PyObject* cb_status;     // (device index): the same for the status word
+PyObject* cb_failed;     // (status, name): raises
+PyObject* cb_strict;     // (device index, name, check workspace, check status word): reads the device status back
+
+struct Workspace {
+  int device;
+  void* stream;
+  at::Tensor buf;
+  long long max_batch;
+};
+struct StatusWord {
+  int device;
+  void* stream;
+  at::Tensor word;
+};
+// A handful of entries (one per stream in use), guarded by the interpreter lock.
+std::vector<Workspace>& workspaces() { static auto* v = new std::vector<Workspace>; return *v; }
+std::vector<StatusWord>& status_words() { static auto* v = new std::vector<StatusWord>; return *v; }
+
+bool env_is(const char* name, const char* value) {
+  const char* v = std::getenv(name);
+  return v && std::strcmp(v, value) == 0;
+}
+
+const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+int dtype_code(const at::Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kBFloat16: return NVJ_BF16;
+    case at::kHalf: return NVJ_F16;
+    case at::kFloat: return NVJ_F32;
+    default: return -1;
+  }
+}
+
+bool on(const at::Tensor& t, int device) { return t.is_cuda() && t.get_device() == device; }
+bool meta(const at::Tensor& t, int device) { return on(t, device) && t.scalar_type() == at::kInt && t.is_contiguous(); }
+const int32_t* i32(const at::Tensor& t) { return static_cast<const int32_t*>(t.data_ptr()); }
+
+void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
+
+// The workspace of (device, current stream) with room for `rows` rows; null with a Python error set.
+const Workspace* workspace_for(int device, void* stream, long long rows) {
+  for (int turn = 0; turn < 2; ++turn) {
+    for (const Workspace& w : workspaces())
+      if (w.device == device && w.stream == stream && w.max_batch >= rows) return &w;
+    PyObject* r = PyObject_CallFunction(cb_workspace, "iL", device, rows);
+    if (!r) return nullptr;
+    Py_DECREF(r);
+  }
+  PyErr_SetString(PyExc_RuntimeError, "no workspace for this stream");
+  return nullptr;
+}
+
+int32_t* status_for(int device, void* stream) {
+  for (int turn = 0; turn < 2; ++turn) {
+    for (const StatusWord& w : status_words())
+      if (w.device == device && w.stream == stream) return static_cast<int32_t*>(w.word.data_ptr());
+    PyObject* r = PyObject_CallFunction(cb_status, "i", device);
+    if (!r) return nullptr;
+    Py_DECREF(r);
+  }
+  PyErr_SetString(PyExc_RuntimeError, "no status word for this stream");
+  return nullptr;
+}
+
+at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, int device) {
+  return at::detail::empty_cuda(sizes, dtype, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), std::nullopt);
+}
+
+// A float32 output; NVJ_POISON_OUTPUT=1 (tests) starts it as NaN.
+at::Tensor output(at::IntArrayRef sizes, int device) {
+  at::Tensor t = empty(sizes, at::kFloat, device);
+  if (env_is("NVJ_POISON_OUTPUT", "1")) t.fill_(std::nan(""));
+  return t;
+}
+
+// After a call: a failure raises; NVJ_CHECK_STATUS=1 (tests) reads the device status back.  False: Python error set.
+bool finished(int rc, const char* what, int device, bool workspace, bool word) {
+  if (rc != NVJ_OK) {
+    PyObject* r = PyObject_CallFunction(cb_failed, "is", rc, what);
+    Py_XDECREF(r);
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, what);
+    return false;
+  }
+  if (env_is("NVJ_CHECK_STATUS", "1")) {
+    PyObject* r = PyObject_CallFunction(cb_strict, "isii", device, what, workspace ? 1 : 0, word ? 1 : 0);
+    if (!r) return false;
+    Py_DECREF(r);
+  }
+  return true;
+}
+
+#define NVJ_NONE() do { Py_RETURN_NONE; } while (0)
+#define NVJ_CALL(rc, call) do { Py_BEGIN_ALLOW_THREADS rc = (call); Py_END_ALLOW_THREADS } while (0)
+
+bool args_are(Py_ssize_t n, Py_ssize_t want) {
+  if (n == want) return true;
+  PyErr_Format(PyExc_TypeError, "%zd arguments expected, got %zd", want, n);
+  return false;
+}
+
+// A layer of a pair of 5-D caches [L, NB, bs, Hkv, D].
+struct Layer {
+  bool ok = false;
+  int device, dtype, block_size, hkv, d;
+  long long blocks;
+  char *k, *v;
+};
+Layer cache_layer(const at::Tensor* k, const at::Tensor* v, long long layer) {
+  Layer l;
+  if (!k || !v || !k->is_cuda() || k->dim() != 5 || v->dim() != 5 || k->sizes() != v->sizes() || k->dtype() != v->dtype()) return l;
+  l.device = k->get_device();
+  l.dtype = dtype_code(*k);
+  if (l.dtype < 0 || !on(*v, l.device) || !k->is_contiguous() || !v->is_contiguous() || layer < 0 || layer >= k->size(0)) return l;
+  l.blocks = k->size(1);
+  l.block_size = (int)k->size(2);
+  l.hkv = (int)k->size(3);
+  l.d = (int)k->size(4);
+  const size_t bytes = (size_t)l.blocks * l.block_size * l.hkv * l.d * k->element_size();
+  l.k = static_cast<char*>(k->data_ptr()) + layer * bytes;
+  l.v = static_cast<char*>(v->data_ptr()) + layer * bytes;
+  l.ok = true;
+  return l;
+}
+
+// ---- the calls ----------------------------------------------------------------------------------------------------
+
+// fused_decode(query, new_k, new_v, k_cache, v_cache, block_tables, seq_lens, positions | None, layer, block_size, scale,
+//              groups, variant) -> out [B, 1, Hq * D] float32
+PyObject* fused_decode(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 13)) return nullptr;
+  const at::Tensor *q = tensor(a[0]), *nk = tensor(a[1]), *nv = tensor(a[2]), *tab = tensor(a[5]), *len = tensor(a[6]);
+  const at::Tensor* pos = a[7] == Py_None ? nullptr : tensor(a[7]);
+  const long long layer = PyLong_AsLongLong(a[8]), bs = PyLong_AsLongLong(a[9]), groups = PyLong_AsLongLong(a[11]);
+  const double scale = PyFloat_AsDouble(a[10]);
+  const long long variant = PyLong_AsLongLong(a[12]);
+  if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
+  const Layer l = cache_layer(tensor(a[3]), tensor(a[4]), layer);
+  if (!l.ok || !q || !nk || !nv || !tab || !len || (!pos && a[7] != Py_None)) NVJ_NONE();
+  if (q->dim() != 4 || q->size(1) != 1 || nk->dim() != 4 || nk->size(1) != 1 || nk->sizes() != nv->sizes()) NVJ_NONE();
+  const long long batch = q->size(0), hq = q->size(2), d = q->size(3);
+  const int qdt = dtype_code(*q);
+  if (batch == 0 || l.block_size != bs || d != l.d || hq != l.hkv * groups || nk->size(0) != batch || nk->size(2) != l.hkv ||
+      nk->size(3) != l.d || (qdt != NVJ_F32 && qdt != l.dtype) || dtype_code(*nk) != l.dtype || dtype_code(*nv) != l.dtype)
+    NVJ_NONE();
+  if (!on(*q, l.device) || !on(*nk, l.device) || !on(*nv, l.device) || !q->is_contiguous() || !nk->is_contiguous() ||
+      !nv->is_contiguous() || !meta(*tab, l.device) || !meta(*len, l.device) || tab->dim() != 2 || tab->size(0) != batch ||
+      len->dim() != 1 || len->size(0) != batch || (pos && (!meta(*pos, l.device) || pos->numel() != batch)))
+    NVJ_NONE();
+  void* stream = stream_of(l.device);
+  const Workspace* ws = workspace_for(l.device, stream, batch);
+  if (!ws) return nullptr;
+  at::Tensor out = output({batch, 1, hq * d}, l.device);
+  void* wp = ws->buf.data_ptr();
+  const size_t wb = (size_t)ws->buf.numel();
+  int rc;
+  NVJ_CALL(rc, lib.fused_append(q->data_ptr(), qdt, nk->data_ptr(), nv->data_ptr(), pos ? i32(*pos) : nullptr, l.k, l.v, l.dtype,
+                                l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab), (int)tab->size(1), i32(*len), (int)batch,
+                                (float)scale, static_cast<float*>(out.data_ptr()), wp, wb, (int)variant, stream));
+  if (!finished(rc, "nvj_paged_decode_fused_append", l.device, true, false)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+}
+
+// window_decode(query [B, T, Hq, D], k_cache, v_cache, block_tables, seq_lens, positions [B, T] | None, layer, block_size,
+//               scale, groups, max_kv_len | None) -> out [B, T, Hq * D] float32
+PyObject* window_decode(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 11)) return nullptr;
+  const at::Tensor *q = tensor(a[0]), *tab = tensor(a[3]), *len = tensor(a[4]);
+  const at::Tensor* pos = a[5] == Py_None ? nullptr : tensor(a[5]);
+  const long long layer = PyLong_AsLongLong(a[6]), bs = PyLong_AsLongLong(a[7]), groups = PyLong_AsLongLong(a[9]);
+  const double scale = PyFloat_AsDouble(a[8]);
+  long long max_len = a[10] == Py_None ? -1 : PyLong_AsLongLong(a[10]);
+  if (a[10] != Py_None && max_len < 1) { PyErr_Clear(); NVJ_NONE(); }
+  if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
+  const Layer l = cache_layer(tensor(a[1]), tensor(a[2]), layer);
+  if (!l.ok || !q || !tab || !len || (!pos && a[5] != Py_None) || q->dim() != 4) NVJ_NONE();
+  const long long batch = q->size(0), width = q->size(1), hq = q->size(2), d = q->size(3);
+  const int qdt = dtype_code(*q);
+  if (batch == 0 || width < 1 || width > 16 || l.block_size != bs || d != l.d || hq != l.hkv * groups || qdt < 0) NVJ_NONE();
+  if (width > 1 && !(pos && qdt == NVJ_BF16 && l.dtype == NVJ_BF16 && hq == 8 && d == 256 && bs == 16 && l.hkv == 2)) NVJ_NONE();
+  if (!on(*q, l.device) || !q->is_contiguous() || !meta(*tab, l.device) || !meta(*len, l.device) || tab->dim() != 2 ||
+      tab->size(0) != batch || len->dim() != 1 || len->size(0) != batch ||
+      (pos && (!meta(*pos, l.device) || pos->dim() != 2 || pos->size(0) != batch || pos->size(1) != width)))
+    NVJ_NONE();
+  const long long span = tab->size(1) * bs;
+  if (max_len < 0) max_len = span;
+  if (max_len < 1 || max_len > span || max_len > l.blocks * bs || max_len > 0x7fffffffLL) NVJ_NONE();
+  void* stream = stream_of(l.device);
+  const Workspace* ws = workspace_for(l.device, stream, batch);
+  if (!ws) return nullptr;
+  at::Tensor out = output({batch, width, hq * d}, l.device);
+  void* wp = ws->buf.data_ptr();
+  const size_t wb = (size_t)ws->buf.numel();
+  int rc;
+  NVJ_CALL(rc, lib.window(q->data_ptr(), qdt, l.k, l.v, l.dtype, l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab),
+                          (int)tab->size(1), i32(*len), pos ? i32(*pos) : nullptr, (int)batch, (int)width, (int)max_len,
+                          (float)scale, static_cast<float*>(out.data_ptr()), wp, wb, stream));
+  if (rc == NVJ_ERR_UNSUPPORTED) NVJ_NONE();
+  if (!finished(rc, "nvj_paged_decode_window", l.device, true, false)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+}
+
+// append(new_k, new_v, k_cache, v_cache, layer, slot_mapping | None, positions, block_tables, token_row_ids | None,
+//        query_start_loc, block_size of the tables) -> True: token rows [rows, cols, Hkv, D] go to their slots; without a slot mapping the slots are
+// made from positions and tables in the same launch.
+PyObject* append(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 11)) return nullptr;
+  const at::Tensor *nk = tensor(a[0]), *nv = tensor(a[1]), *qsl = tensor(a[9]);
+  const long long layer = PyLong_AsLongLong(a[4]), bs = PyLong_AsLongLong(a[10]);
+  if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
+  const Layer l = cache_layer(tensor(a[2]), tensor(a[3]), layer);
+  if (!l.ok || !nk || !nv || !qsl || nk->dim() != 4 || nk->sizes() != nv->sizes() || nk->size(2) != l.hkv || nk->size(3) != l.d) NVJ_NONE();
+  const long long rows = nk->size(0), cols = nk->size(1);
+  const int dt = dtype_code(*nk);
+  if (rows * cols == 0 || dt < 0 || nv->dtype() != nk->dtype() || !on(*nk, l.device) || !on(*nv, l.device) || !nk->is_contiguous() ||
+      !nv->is_contiguous() || !meta(*qsl, l.device) || qsl->numel() < 1)
+    NVJ_NONE();
+  const bool packed = a[8] != Py_None;
+  const long long num_slots = l.blocks * l.block_size;
+  void* stream = stream_of(l.device);
+  int rc;
+  const char* what;
+  if (a[5] != Py_None) {
+    const at::Tensor* slots = tensor(a[5]);
+    if (!slots || !meta(*slots, l.device) || slots->dim() != 2 || slots->size(0) != rows || slots->size(1) != cols) NVJ_NONE();
+    int32_t* st = status_for(l.device, stream);
+    if (!st) return nullptr;
+    what = "nvj_kv_append";
+    NVJ_CALL(rc, lib.append(nk->data_ptr(), nv->data_ptr(), dt, i32(*slots), nullptr, i32(*qsl), (int)qsl->numel() - 1, packed ? 1 : 0,
+                            (int)rows, (int)cols, l.k, l.v, l.dtype, num_slots, l.hkv, l.d, st, stream));
+  } else {
+    const at::Tensor *pos = tensor(a[6]), *tab = tensor(a[7]), *rid = packed ? tensor(a[8]) : nullptr;
+    if (!pos || !tab || !meta(*pos, l.device) || !meta(*tab, l.device) || pos->dim() != 2 || pos->size(0) != rows || pos->size(1) != cols ||
+        tab->dim() != 2 || tab->size(0) == 0 || tab->size(1) == 0 || bs != l.block_size)
+      NVJ_NONE();
+    if (packed ? (!rid || !meta(*rid, l.device) || rid->sizes() != pos->sizes()) : tab->size(0) != rows) NVJ_NONE();
+    int32_t* st = status_for(l.device, stream);
+    if (!st) return nullptr;
+    what = "nvj_kv_append_mapped";
+    NVJ_CALL(rc, lib.append_mapped(nk->data_ptr(), nv->data_ptr(), dt, i32(*pos), i32(*tab), rid ? i32(*rid) : nullptr, (int)tab->size(0),
+                                   (int)tab->size(1), l.block_size, i32(*qsl), (int)qsl->numel() - 1, packed ? 1 : 0, (int)rows, (int)cols,
+                                   l.k, l.v, l.dtype, num_slots, l.hkv, l.d, st, stream));
+  }
+  if (!finished(rc, what, l.device, false, true)) return nullptr;
+  Py_RETURN_TRUE;
+}
+
+// packed_prefill(query [1, T, Hq, D], k_cache, v_cache, block_tables, kv_lens, positions, query_start_loc, layer, block_size,
+//                scale, groups, decode_rows | None) -> out [1, T, Hq * D] float32
+PyObject* packed_prefill(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 12)) return nullptr;
+  const at::Tensor *q = tensor(a[0]), *tab = tensor(a[3]), *len = tensor(a[4]), *pos = tensor(a[5]), *qsl = tensor(a[6]);
+  const long long layer = PyLong_AsLongLong(a[7]), bs = PyLong_AsLongLong(a[8]), groups = PyLong_AsLongLong(a[10]);
+  const double scale = PyFloat_AsDouble(a[9]);
+  const long long decode_rows = a[11] == Py_None ? -1 : PyLong_AsLongLong(a[11]);
+  if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
+  const Layer l = cache_layer(tensor(a[1]), tensor(a[2]), layer);
+  if (!l.ok || !q || !tab || !len || !pos || !qsl || q->dim() != 4 || q->size(0) != 1) NVJ_NONE();
+  const long long tokens = q->size(1), hq = q->size(2), d = q->size(3);
+  const int qdt = dtype_code(*q);
+  if (tokens == 0 || l.block_size != bs || d != l.d || hq != l.hkv * groups || qdt < 0 || !on(*q, l.device) || !q->is_contiguous()) NVJ_NONE();
+  if (!meta(*tab, l.device) || !meta(*len, l.device) || !meta(*pos, l.device) || !meta(*qsl, l.device) || tab->dim() != 2) NVJ_NONE();
+  const long long rows = tab->size(0);
+  if (len->dim() != 1 || len->size(0) != rows || pos->dim() != 2 || pos->size(0) != 1 || pos->size(1) != tokens || qsl->numel() != rows + 1) NVJ_NONE();
+  const char* env = std::getenv("NVJ_PREFILL_VARIANT");
+  const int variant = env ? std::atoi(env) : 0;
+  const bool model_shape = l.dtype == NVJ_BF16 && bs == 16 && l.hkv == 2 && d == 256 && hq == 8 && (qdt == NVJ_BF16 || qdt == NVJ_F32);
+  // decode rows and tiles side by side on two streams: the Python route forks and joins
+  if (model_shape && (variant == 0 || variant == 4 || variant == 5) && decode_rows > 0 && decode_rows < rows &&
+      !env_is("NVJ_MIXED_SIDE_BY_SIDE", "0") &&
+      (env_is("NVJ_MIXED_SIDE_BY_SIDE", "1") ||
+       c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None))
+    NVJ_NONE();
+  void* stream = stream_of(l.device);
+  int32_t* st = status_for(l.device, stream);
+  if (!st) return nullptr;
+  const bool tiles_only = model_shape && variant != 1 && decode_rows == 0 && !env_is("NVJ_PREFILL_KEY_SPLITS", "0");
+  const Workspace* ws = nullptr;
+  if (tiles_only || decode_rows != 0) {
+    ws = workspace_for(l.device, stream, rows);
+    if (!ws) return nullptr;
+  }
+  void* wp = ws ? ws->buf.data_ptr() : nullptr;
+  const size_t wb = ws ? (size_t)ws->buf.numel() : 0;
+  at::Tensor out = output({1, tokens, hq * d}, l.device);
+  int rc;
+  if (tiles_only) {
+    NVJ_CALL(rc, lib.prefill_part(q->data_ptr(), qdt, l.k, l.v, l.dtype, l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab),
+                                  (int)tab->size(1), i32(*len), i32(*pos), i32(*qsl), (int)rows, (int)tokens, (float)scale,
+                                  static_cast<float*>(out.data_ptr()), st, wp, wb, variant, 3, 0, stream));
+  } else {
+    NVJ_CALL(rc, lib.prefill(q->data_ptr(), qdt, l.k, l.v, l.dtype, l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab),
+                             (int)tab->size(1), i32(*len), i32(*pos), i32(*qsl), (int)rows, (int)tokens, (float)scale,
+                             static_cast<float*>(out.data_ptr()), st, wp, wb, variant, stream));
+  }
+  if (!finished(rc, "nvj_paged_prefill_packed", l.device, ws != nullptr, true)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+}
+
+// norm_rope(query, k, v, q_weight, k_weight, positions, slot_mapping, k_layer, v_layer, query_start_loc | None, packed, eps,
+//           inv_freq | None, rotary_dim) -> query for attention; text positions [rows, cols], cache layers [..., Hkv, D]
+PyObject* norm_rope(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 14)) return nullptr;
+  const at::Tensor *q = tensor(a[0]), *k = tensor(a[1]), *v = tensor(a[2]), *qw = tensor(a[3]), *kw = tensor(a[4]), *pos = tensor(a[5]),
+                   *slots = tensor(a[6]), *kl = tensor(a[7]), *vl = tensor(a[8]);
+  const at::Tensor *qsl = a[9] == Py_None ? nullptr : tensor(a[9]), *inv = a[12] == Py_None ? nullptr : tensor(a[12]);
+  const int packed = PyObject_IsTrue(a[10]);
+  const double eps = PyFloat_AsDouble(a[11]);
+  const long long rotary = PyLong_AsLongLong(a[13]);
+  if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
+  if (!q || !k || !v || !qw || !kw || !pos || !slots || !kl || !vl || (!qsl && a[9] != Py_None) || (!inv && rotary > 0)) NVJ_NONE();
+  if (!q->is_cuda() || q->dim() != 4 || k->dim() != 4 || k->sizes() != v->sizes() || q->size(0) != k->size(0) || q->size(1) != k->size(1)) NVJ_NONE();
+  const int dev = q->get_device();
+  const long long rows = q->size(0), cols = q->size(1), hq = q->size(2), d = q->size(3), hkv = k->size(2);
+  if (rows * cols == 0 || k->size(3) != d || kl->dim() < 3 || kl->sizes() != vl->sizes() || kl->size(-2) != hkv || kl->size(-1) != d) NVJ_NONE();
+  const int dt = dtype_code(*q), wdt = dtype_code(*qw);
+  if (dt < 0 || k->dtype() != q->dtype() || v->dtype() != q->dtype() || wdt < 0 || kw->dtype() != qw->dtype() || qw->numel() != d || kw->numel() != d ||
+      !qw->is_contiguous() || !kw->is_contiguous() || kl->dtype() != vl->dtype() || dtype_code(*kl) < 0 || !kl->is_contiguous() || !vl->is_contiguous())
+    NVJ_NONE();
+  for (const at::Tensor* t : {k, v, qw, kw, kl, vl}) if (!on(*t, dev)) NVJ_NONE();
+  if (inv && (!on(*inv, dev) || inv->scalar_type() != at::kFloat || inv->numel() * 2 < rotary)) NVJ_NONE();
+  if (!meta(*pos, dev) || !meta(*slots, dev) || pos->dim() != 2 || pos->numel() != rows * cols || slots->numel() != rows * cols || (qsl && !meta(*qsl, dev))) NVJ_NONE();
+  // tokens evenly spaced: one stride serves rows and columns (the query may be a view of a wider projection)
+  auto token_stride = [&](const at::Tensor& t, long long* stride) {
+    if (t.stride(3) != 1 || (rows > 1 && cols > 1 && t.stride(0) != t.stride(1) * cols)) return false;
+    *stride = cols > 1 ? t.stride(1) : (rows > 1 ? t.stride(0) : t.size(2) * d);
+    return true;
+  };
+  long long qs;
+  long long ks;
+  long long vs;
+  if (!token_stride(*q, &qs) || !token_stride(*k, &ks) || !token_stride(*v, &vs) || k->stride(2) != d || v->stride(2) != d) NVJ_NONE();
+  void* stream = stream_of(dev);
+  int32_t* st = status_for(dev, stream);
+  if (!st) return nullptr;
+  at::Tensor out = empty({rows, cols, hq, d}, q->scalar_type(), dev);
+  int rc;
+  NVJ_CALL(rc, lib.norm_rope(q->data_ptr(), qs, q->stride(2), k->data_ptr(), ks, v->data_ptr(), vs, dt, qw->data_ptr(), kw->data_ptr(), wdt,
+                             (float)eps, inv ? static_cast<const float*>(inv->data_ptr()) : nullptr, (int)rotary, i32(*pos), 1, nullptr, i32(*slots),
+                             nullptr, qsl ? i32(*qsl) : nullptr, qsl ? (int)qsl->numel() - 1 : 0, packed, (int)rows, (int)cols, kl->data_ptr(),
+                             vl->data_ptr(), dtype_code(*kl), kl->numel() / (hkv * d), (int)hq, (int)hkv, (int)d, out.data_ptr(), st, stream));
+  if (!finished(rc, "nvj_qk_norm_rope_kv_append", dev, false, true)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+}
+
+// slot_mapping(positions [rows, cols], block_tables, block_size, token_row_ids | None) -> int32 [rows, cols]
+PyObject* slot_mapping(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 4)) return nullptr;
+  const at::Tensor *pos = tensor(a[0]), *tab = tensor(a[1]), *rid = a[3] == Py_None ? nullptr : tensor(a[3]);
+  const long long bs = PyLong_AsLongLong(a[2]);
+  if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
+  if (!pos || !tab || (!rid && a[3] != Py_None) || !pos->is_cuda() || pos->dim() != 2 || tab->dim() != 2 || bs < 1) NVJ_NONE();
+  const int dev = pos->get_device();
+  if (!meta(*pos, dev) || !meta(*tab, dev) || tab->size(0) < 1 || tab->size(1) < 1) NVJ_NONE();
+  if (rid ? (!meta(*rid, dev) || rid->sizes() != pos->sizes()) : pos->size(0) > tab->size(0)) NVJ_NONE();
+  void* stream = stream_of(dev);
+  at::Tensor out = empty(pos->sizes(), at::kInt, dev);
+  int rc;
+  NVJ_CALL(rc, lib.slot_mapping(i32(*pos), i32(*tab), rid ? i32(*rid) : nullptr, (int)pos->size(0), (int)pos->size(1), (int)tab->size(0),
+                                (int)tab->size(1), (int)bs, static_cast<int32_t*>(out.data_ptr()), stream));
+  if (!finished(rc, "nvj_compute_slot_mapping", dev, false, false)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+}
+
+// ---- set-up ---------------------------------------------------------------------------------------------------------
+
+// init(library handle, workspace, status, failed, strict)
+PyObject* init(PyObject*, PyObject* args) {
+  unsigned long long handle;
+  PyObject *ws, *st, *failed, *strict;
+  if (!PyArg_ParseTuple(args, "KOOOO", &handle, &ws, &st, &failed, &strict)) return nullptr;
+  void* h = reinterpret_cast<void*>(handle);
+  const char* missing = nullptr;
+  auto get = [&](auto& fn, const char* name) {
+    fn = reinterpret_cast<std::decay_t<decltype(fn)>>(dlsym(h, name));
+    if (!fn) missing = name;
+  };
+  get(lib.fused_append, "nvj_paged_decode_fused_append");
+  get(lib.window, "nvj_paged_decode_window");
+  get(lib.append, "nvj_kv_append");
+  get(lib.append_mapped, "nvj_kv_append_mapped");
+  get(lib.prefill, "nvj_paged_prefill_packed");
+  get(lib.prefill_part, "nvj_paged_prefill_packed_part");
+  get(lib.norm_rope, "nvj_qk_norm_rope_kv_append");
+  get(lib.slot_mapping, "nvj_compute_slot_mapping");
+  if (missing) {
+    PyErr_Format(PyExc_ImportError, "libnvj_b200.so does not export %s", missing);
+    return nullptr;
+  }
+  for (PyObject* o : {ws, st, failed, strict}) Py_INCREF(o);
+  cb_workspace = ws; cb_status = st; cb_failed = failed; cb_strict = strict;
+  Py_RETURN_NONE;
+}
+
+// set_workspace(device index, stream, buffer, max_batch): replaces the one of that (device, stream)
+PyObject* set_workspace(PyObject*, PyObject* args) {
+  int device;
+  unsigned long long stream;
+  PyObject* buf;
+  long long max_batch;
+  if (!PyArg_ParseTuple(args, "iKOL", &device, &stream, &buf, &max_batch)) return nullptr;
+  const at::Tensor* t = tensor(buf);
+  if (!t) { PyErr_SetString(PyExc_TypeError, "buffer must be a tensor"); return nullptr; }
+  void* s = reinterpret_cast<void*>(stream);
+  for (Workspace& w : workspaces())
+    if (w.device == device && w.stream == s) { w.buf = *t; w.max_batch = max_batch; Py_RETURN_NONE; }
+  workspaces().push_back({device, s, *t, max_batch});
+  Py_RETURN_NONE;
+}
+
+PyObject* set_status_word(PyObject*, PyObject* args) {
+  int device;
+  unsigned long long stream;
+  PyObject* word;
+  if (!PyArg_ParseTuple(args, "iKO", &device, &stream, &word)) return nullptr;
+  const at::Tensor* t = tensor(word);
+  if (!t) { PyErr_SetString(PyExc_TypeError, "word must be a tensor"); return nullptr; }
+  void* s = reinterpret_cast<void*>(stream);
+  for (StatusWord& w : status_words())
+    if (w.device == device && w.stream == s) { w.word = *t; Py_RETURN_NONE; }
+  status_words().push_back({device, s, *t});
+  Py_RETURN_NONE;
+}
+
+// C++ exceptions become the Python ones that torch's own functions raise (out of memory among them).
+template <PyObject* (*Fn)(PyObject* const*, Py_ssize_t)>
+PyObject* entry(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return Fn(a, n);
+  END_HANDLE_TH_ERRORS
+}
+#define NVJ_FAST(fn, doc) {#fn, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<fn>)), METH_FASTCALL, doc}
+PyMethodDef methods[] = {
+    NVJ_FAST(fused_decode, "append + decode of one token per row, or None"),
+    NVJ_FAST(window_decode, "decode attention over a window, or None"),
+    NVJ_FAST(append, "append of new K/V rows, or None"),
+    NVJ_FAST(packed_prefill, "ragged packed attention, or None"),
+    NVJ_FAST(norm_rope, "norm + rope + append, or None"),
+    NVJ_FAST(slot_mapping, "flat cache slots of positions, or None"),
+    {"init", init, METH_VARARGS, "resolve the library's entry points and keep the callbacks"},
+    {"set_workspace", set_workspace, METH_VARARGS, "hand over a (device, stream)'s workspace"},
+    {"set_status_word", set_status_word, METH_VARARGS, "hand over a (device, stream)'s status word"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_nvj_host", "Host side of the hot calls.", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__nvj_host(void) { return PyModule_Create(&module); }

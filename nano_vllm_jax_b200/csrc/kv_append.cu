@@ -120,17 +120,8 @@ slot_mapping_kernel(const int32_t* positions, const int32_t* block_tables, const
                     int32_t* slots) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rows * n_cols) return;
-  int row = token_row_ids ? token_row_ids[i] : i / n_cols;
-  row = row < 0 ? 0 : (row >= table_rows ? table_rows - 1 : row);
-  const int pos = positions[i];
-  // floor division and a non-negative remainder, as jnp's // and % give for a negative position
-  // (nanovllm_jax/kv_cache.py:432-435); C's / and % would round toward zero
-  int col = pos / block_size, off = pos % block_size;
-  if (off < 0) { off += block_size; --col; }
-  // a negative block index wraps around once as NumPy / jnp indexing does, then the gather clamps
-  if (col < 0) col += table_width;
-  col = col < 0 ? 0 : (col >= table_width ? table_width - 1 : col);
-  slots[i] = block_tables[(long long)row * table_width + col] * block_size + off;
+  slots[i] = mapped_slot(block_tables, token_row_ids ? token_row_ids[i] : i / n_cols, positions[i], table_rows, table_width,
+                         block_size);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -215,6 +206,47 @@ extern "C" int nvj_kv_append(const void* new_k, const void* new_v, int src_dtype
   p.qsl_rows = qsl_rows;
   p.packed = packed;
   p.page_size = 1;
+  p.row_elems = num_kv_heads * head_dim;
+  p.src_dtype = src_dtype;
+  p.dst_dtype = cache_dtype;
+  return launch_append(p, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int nvj_kv_append_mapped(const void* new_k, const void* new_v, int src_dtype, const int32_t* positions,
+                                    const int32_t* block_tables, const int32_t* token_row_ids, int table_rows,
+                                    int table_width, int block_size, const int32_t* query_start_loc, int qsl_rows,
+                                    int packed, int n_rows, int n_cols, void* k_cache_layer, void* v_cache_layer,
+                                    int cache_dtype, int64_t num_slots, int num_kv_heads, int head_dim,
+                                    int32_t* status, nvj_stream_t stream) {
+  using namespace nvj;
+  if (n_rows < 0 || n_cols < 0 || num_slots < 0 || num_kv_heads <= 0 || head_dim <= 0 || table_rows <= 0 ||
+      table_width <= 0 || block_size <= 0)
+    return NVJ_ERR_INVALID_ARGUMENT;
+  if (!dtype_ok(src_dtype) || !dtype_ok(cache_dtype)) return NVJ_ERR_UNSUPPORTED;
+  if ((long long)n_rows * n_cols > 0x7fffffffLL / 32) return NVJ_ERR_UNSUPPORTED;
+  if (n_rows * n_cols == 0) return NVJ_OK;
+  if (!new_k || !new_v || !positions || !block_tables || !k_cache_layer || !v_cache_layer)
+    return NVJ_ERR_INVALID_ARGUMENT;
+  if (query_start_loc && qsl_rows < 0) return NVJ_ERR_INVALID_ARGUMENT;
+  if (!token_row_ids && n_rows > table_rows) return NVJ_ERR_INVALID_ARGUMENT;
+  AppendParams p{};
+  p.new_k = new_k;
+  p.new_v = new_v;
+  p.k_cache = k_cache_layer;
+  p.v_cache = v_cache_layer;
+  p.positions = positions;
+  p.block_tables = block_tables;
+  p.token_row_ids = token_row_ids;
+  p.table_rows = table_rows;
+  p.table_width = table_width;
+  p.query_start_loc = query_start_loc;
+  p.status = status;
+  p.num_slots = num_slots;
+  p.n_tokens = n_rows * n_cols;
+  p.n_cols = n_cols;
+  p.qsl_rows = qsl_rows;
+  p.packed = packed;
+  p.page_size = block_size;
   p.row_elems = num_kv_heads * head_dim;
   p.src_dtype = src_dtype;
   p.dst_dtype = cache_dtype;

@@ -23,6 +23,10 @@ struct AppendParams {
   const int32_t* kv_indices;
   const int32_t* kv_indptr;   // null: row b's table starts at b * table_width
   const int32_t* seq_lens;    // page-table mode, optional: rows with seq_lens[b] <= 0 are skipped
+  // mapped mode (block_tables set): the slot is made here from the token's position and its row's block table
+  const int32_t* block_tables;
+  const int32_t* token_row_ids;  // null: rectangular batch, row = i / n_cols
+  int table_rows;
   int32_t* status;
   long long num_slots;
   long long kv_indices_len;
@@ -38,12 +42,25 @@ struct AppendParams {
   int dst_dtype;
 };
 
+// Flat slot of position `pos` of row `row`: floor division and a non-negative remainder, as jnp's // and % give for a
+// negative position (nanovllm_jax/kv_cache.py:432-435; C's / and % would round toward zero); a negative block index
+// wraps around once as NumPy / jnp indexing does, then the gather clamps.
+__device__ __forceinline__ int mapped_slot(const int32_t* block_tables, int row, int pos, int table_rows, int table_width,
+                                           int block_size) {
+  row = row < 0 ? 0 : (row >= table_rows ? table_rows - 1 : row);
+  int col = pos / block_size, off = pos % block_size;
+  if (off < 0) { off += block_size; --col; }
+  if (col < 0) col += table_width;
+  col = col < 0 ? 0 : (col >= table_width ? table_width - 1 : col);
+  return block_tables[(long long)row * table_width + col] * block_size + off;
+}
+
 // Returns the flat destination slot of token i, or -1 when the token is masked
 // out or its slot lies outside the pool (the latter is flagged).
 __device__ __forceinline__ long long resolve_slot(const AppendParams& p, int i) {
   if (p.valid_mask && p.valid_mask[i] == 0) return -1;
   long long slot;
-  if (p.slot_mapping) {
+  if (p.slot_mapping || p.block_tables) {
     if (p.query_start_loc) {
       if (p.packed) {
         if (i >= p.query_start_loc[p.qsl_rows]) return -1;
@@ -53,7 +70,9 @@ __device__ __forceinline__ long long resolve_slot(const AppendParams& p, int i) 
         if (t >= p.query_start_loc[r + 1] - p.query_start_loc[r]) return -1;
       }
     }
-    slot = p.slot_mapping[i];
+    slot = p.slot_mapping ? p.slot_mapping[i]
+                          : mapped_slot(p.block_tables, p.token_row_ids ? p.token_row_ids[i] : i / p.n_cols, p.positions[i],
+                                        p.table_rows, p.table_width, p.page_size);
   } else {
     const int b = p.batch_indices ? p.batch_indices[i] : i;
     const int pos = p.positions[i];

@@ -32,6 +32,9 @@ struct DecodeParams {
   // fused append without positions: seq_lens holds every row's length BEFORE this step's token; the new row goes to
   // position seq_lens[b] and seq_lens[b] + 1 keys are attended (rows with seq_lens[b] <= 0 stay inactive)
   int pre_append;
+  // decode over an attention window (0 / null: none): at most max_len keys per row, and (width 1) keys p <= cap_positions[b]
+  int max_len;
+  const int32_t* cap_positions;
   // packed prefill through the generic kernel (nullable): query i belongs to the
   // table row r with query_start_loc[r] <= i < query_start_loc[r + 1] and attends
   // keys p <= query_positions[i]
@@ -77,6 +80,11 @@ struct DecodeParams {
 __device__ __forceinline__ int decode_row_len(const DecodeParams& p, int b) {
   int len = p.seq_lens[b];
   if (p.pre_append && len > 0) ++len;
+  if (p.max_len > 0) len = len < p.max_len ? len : p.max_len;
+  if (p.cap_positions) {
+    const int cap = p.cap_positions[b] + 1;
+    len = len < cap ? len : cap;
+  }
   if (p.packed_rows) {
     const int i = p.query_start_loc[b];
     if (p.query_start_loc[b + 1] - i != 1) return 0;
@@ -161,6 +169,7 @@ int launch_decode_generic(const DecodeParams& p, cudaStream_t stream);
 int launch_decode_pipelined(const DecodeParams& p, int num_ctas, cudaStream_t stream);
 int decode_wide_num_ctas();  // 1 per SM of the current device
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // tensor-core streaming kernels, width 1..8
+int run_decode_wide(DecodeParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);  // checks, carves, launches
 int launch_decode_umma(const DecodeParams& p, cudaStream_t stream);  // the tcgen05 form, rows already appended
 int append_decode_rows(const void* new_k, const void* new_v, const int32_t* positions,
                        const int32_t* seq_lens, void* k_cache, void* v_cache, int kv_dtype,

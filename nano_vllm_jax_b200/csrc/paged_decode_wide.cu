@@ -666,28 +666,41 @@ extern "C" int nvj_paged_decode_wide(const void* q, const void* k_cache_layer, c
                                     batch, width, scale, out, workspace, workspace_bytes, 0, stream);
 }
 
+namespace nvj {
+
+// Rows of several query tokens: everything but the workspace is in p (width, wide_form, pointers, shapes).
+int run_decode_wide(DecodeParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  if (p.batch < 0 || p.table_width < 0 || p.num_blocks < 0 || p.width < 1 || p.wide_form < 0 || p.wide_form > 2)
+    return NVJ_ERR_INVALID_ARGUMENT;
+  if (p.width > kWideMaxWidth || (p.wide_form == 1 && p.width > kWMaxWidth)) return NVJ_ERR_UNSUPPORTED;
+  if (p.q_dtype != NVJ_BF16 || p.kv_dtype != NVJ_BF16 || p.block_size != kBlk || p.num_kv_heads != kHkv ||
+      p.num_q_heads != kHq || p.head_dim != kD)
+    return NVJ_ERR_UNSUPPORTED;
+  if (p.batch == 0) return NVJ_OK;
+  if (!p.q || !p.k_cache || !p.v_cache || !p.block_tables || !p.seq_lens || !p.out) return NVJ_ERR_INVALID_ARGUMENT;
+  const uintptr_t al = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k_cache) |
+                       reinterpret_cast<uintptr_t>(p.v_cache) | reinterpret_cast<uintptr_t>(p.out) |
+                       reinterpret_cast<uintptr_t>(workspace);
+  if ((al & 15u) != 0) return NVJ_ERR_UNSUPPORTED;
+  const int n = decode_wide_num_ctas();
+  if (n <= 0) return NVJ_ERR_LAUNCH;
+  // rows of more than 8 tokens run on the tcgen05 form only, which parks two partials per pair of CTAs: n slots
+  const size_t ml_bytes = p.width > kWMaxWidth ? ws_round(sizeof(float) * n * p.width * kHq * 2) : wide_ml_bytes(n, p.width);
+  const size_t acc_bytes = p.width > kWMaxWidth ? ws_round(sizeof(float) * n * p.width * kHq * kD) : wide_acc_bytes(n, p.width);
+  const int carved = carve_decode_workspace(p, workspace, workspace_bytes, ml_bytes, acc_bytes);
+  if (carved != NVJ_OK) return carved;
+  return launch_decode_wide(p, stream);
+}
+
+}  // namespace nvj
+
 extern "C" int nvj_paged_decode_wide_form(const void* q, const void* k_cache_layer, const void* v_cache_layer, int64_t num_blocks,
                                           const int32_t* block_tables, int table_width, const int32_t* seq_lens,
                                           const int32_t* positions, int batch, int width, float scale, float* out,
                                           void* workspace, size_t workspace_bytes, int form, nvj_stream_t stream) {
   using namespace nvj;
-  if (batch < 0 || table_width < 0 || num_blocks < 0 || width < 1 || form < 0 || form > 2) return NVJ_ERR_INVALID_ARGUMENT;
-  if (width > kWideMaxWidth || (form == 1 && width > kWMaxWidth)) return NVJ_ERR_UNSUPPORTED;
-  if (batch == 0) return NVJ_OK;
-  if (!q || !k_cache_layer || !v_cache_layer || !block_tables || !seq_lens || !out) return NVJ_ERR_INVALID_ARGUMENT;
-  const uintptr_t al = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache_layer) |
-                       reinterpret_cast<uintptr_t>(v_cache_layer) | reinterpret_cast<uintptr_t>(out) |
-                       reinterpret_cast<uintptr_t>(workspace);
-  if ((al & 15u) != 0) return NVJ_ERR_UNSUPPORTED;
-  const int n = decode_wide_num_ctas();
-  if (n <= 0) return NVJ_ERR_LAUNCH;
   DecodeParams p{};
   p.batch = batch;
-  // rows of more than 8 tokens run on the tcgen05 form only, which parks two partials per pair of CTAs: n slots
-  const size_t ml_bytes = width > kWMaxWidth ? ws_round(sizeof(float) * n * width * kHq * 2) : wide_ml_bytes(n, width);
-  const size_t acc_bytes = width > kWMaxWidth ? ws_round(sizeof(float) * n * width * kHq * kD) : wide_acc_bytes(n, width);
-  const int carved = carve_decode_workspace(p, workspace, workspace_bytes, ml_bytes, acc_bytes);
-  if (carved != NVJ_OK) return carved;
   p.q = q;
   p.k_cache = static_cast<const char*>(k_cache_layer);
   p.v_cache = static_cast<const char*>(v_cache_layer);
@@ -706,5 +719,5 @@ extern "C" int nvj_paged_decode_wide_form(const void* q, const void* k_cache_lay
   p.q_dtype = NVJ_BF16;
   p.kv_dtype = NVJ_BF16;
   p.scale = scale;
-  return launch_decode_wide(p, static_cast<cudaStream_t>(stream));
+  return run_decode_wide(p, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }

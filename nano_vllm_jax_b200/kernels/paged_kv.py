@@ -23,6 +23,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -69,6 +70,46 @@ def _poison() -> bool:
     # Debug aid (tests set it): fill output buffers with NaN before a launch so that an
     # element the kernel fails to write cannot pass for a result left by an earlier call.
     return os.environ.get("NVJ_POISON_OUTPUT", "0") == "1"
+
+
+_host_module = None
+
+
+def host():
+    """The extension module that serves the regular case of the hot calls (csrc/host/host_ops.cpp): its functions
+    return None, and launch nothing, when an operand needs a conversion or an error message of the Python route."""
+    global _host_module
+    if _host_module is None:
+        lib = _lib.load()
+        from .. import _nvj_host
+        with _host_lock:
+            if _host_module is None:
+                _nvj_host.init(lib._handle, _lend_workspace, _lend_status_word, check, _strict_check)
+                _host_module = _nvj_host
+    return _host_module
+
+
+_host_lock = threading.Lock()
+
+
+def _lend_workspace(index, rows):
+    device = torch.device("cuda", index)
+    ws = _workspace(device, rows)
+    _host_module.set_workspace(index, _stream(device), ws.buf, ws.max_batch)
+
+
+def _lend_status_word(index):
+    device = torch.device("cuda", index)
+    _host_module.set_status_word(index, _stream(device), _status_word(device))
+
+
+def _strict_check(index, what, has_workspace, has_word):
+    device = torch.device("cuda", index)
+    if has_word:
+        _check_word(_status_word(device), what)
+    if has_workspace:
+        ws = _workspace(device, 0)
+        _check_word(ws.status_tensor(), what, ws)
 
 
 class DeviceStatusError(NvjError):
@@ -118,6 +159,8 @@ def _workspace(device: torch.device, batch: int) -> _Workspace:
             _retired_workspaces.append(ws)
         ws = _Workspace(device, max(batch, 256, 2 * (ws.max_batch if ws else 0)))
         _workspaces[key] = ws
+        if _host_module is not None:
+            _host_module.set_workspace(*key, ws.buf, ws.max_batch)
     return ws
 
 
@@ -185,6 +228,9 @@ def _check_nhd_cache(k_cache: torch.Tensor, v_cache: torch.Tensor) -> None:
 
 def compute_slot_mapping(positions, block_table, block_size, token_row_ids=None):
     """int32 slots for positions `[rows, cols]`; packed batches pass `token_row_ids` of the same shape."""
+    out = host().slot_mapping(positions, block_table, block_size, token_row_ids)
+    if out is not None:
+        return out
     lib = _lib.load()
     positions = _i32("positions", positions)
     block_table = _i32("block_table", block_table)
@@ -485,6 +531,10 @@ def paged_decode_attention_with_kv_append(query, new_k, new_v, k_cache, v_cache,
     `positions=None` is the pre-append form for device-resident metadata: `seq_lens` then holds the rows' lengths
     before this step's token (the token goes to position `seq_lens[b]`, `seq_lens[b] + 1` keys are attended) and is
     not written; `row_argmax(..., advance=...)` or the token gather's publish advances it at the end of the step."""
+    out = host().fused_decode(query, new_k, new_v, k_cache, v_cache, block_table, seq_lens, positions, layer_id, block_size,
+                              scale, num_key_value_groups, variant)
+    if out is not None:
+        return out, k_cache, v_cache
     if query.ndim != 4 or query.shape[1] != 1 or new_k.shape[1] != 1 or new_v.shape[1] != 1:
         raise ValueError("fused decode attention supports only width-1 decode")
     if k_cache.ndim != 5 or v_cache.ndim != 5:
@@ -652,6 +702,12 @@ def qk_norm_rope_kv_append(query, k, v, q_norm_weight, k_norm_weight, positions,
     position id, nanovllm_jax/model.py:3955) combined per frequency by `mrope_section` as
     nanovllm_jax/layers.py:79-139 does.  Fuses nanovllm_jax/model.py:3371-3396 with the append of 3539-3550.
     """
+    if valid_mask is None:
+        inv = (_inv_freq_tables.get((float(rope_theta), int(rotary_dim), query.device.index)) if rotary_dim > 0 else None)
+        q_out = host().norm_rope(query, k, v, q_norm_weight, k_norm_weight, positions, slot_mapping, k_cache_layer, v_cache_layer,
+                                 query_start_loc, packed, eps, inv, rotary_dim)
+        if q_out is not None:
+            return q_out, k_cache_layer, v_cache_layer
     lib = _lib.load()
     for name, t in (("query", query), ("k", k), ("v", v), ("k_cache_layer", k_cache_layer), ("v_cache_layer", v_cache_layer)):
         _cuda(name, t)

@@ -86,6 +86,22 @@ def _store_slot_mapping(self, value):
 AttentionMetadata.slot_mapping = property(_read_slot_mapping, _store_slot_mapping)
 
 
+class SlotsFromTables:
+    """The slot mapping of a batch, made from its positions and block tables when somebody reads it.  An append that
+    meets it unread makes the slots inside its own launch instead (nvj_kv_append_mapped)."""
+
+    __slots__ = ("positions", "block_tables", "block_size", "token_row_ids")
+
+    def __init__(self, positions, block_tables, block_size, token_row_ids=None):
+        self.positions, self.block_tables, self.block_size = positions, block_tables, block_size
+        self.token_row_ids = token_row_ids
+
+    def __call__(self):
+        if self.token_row_ids is not None:
+            return compute_packed_slot_mapping(self.positions, self.block_tables, self.token_row_ids, self.block_size)
+        return compute_slot_mapping(self.positions, self.block_tables, self.block_size)
+
+
 @dataclass
 class BlockTables:
     """Host-side allocation state snapshot (kv_cache.py:67-73)."""
@@ -256,6 +272,10 @@ def paged_attention_decode(query, k_cache, v_cache, block_table, kv_lens, block_
     Query width > 1 (speculative verification, rectangular prefill) applies the causal mask
     p <= positions[b, t]; such a batch travels the packed prefill route with rows of equal width.
     """
+    out = _k.host().window_decode(query, k_cache, v_cache, block_table, kv_lens, positions, layer_idx, block_size, scale,
+                                  num_key_value_groups, max_kv_len)
+    if out is not None:
+        return out if out_dtype is torch.float32 else out.to(_promoted(query, k_cache, out_dtype))
     batch, query_len, num_heads, head_dim = query.shape
     if query_len < 1:
         raise ValueError("decode attention requires query_len >= 1")
@@ -348,6 +368,12 @@ def paged_attention_prefill_packed(query, k_cache, v_cache, block_table, kv_lens
     route.  The pure reference path returns the cache dtype; so does this unless
     `out_dtype` is given.
     """
+    if positions.shape == token_row_ids.shape:
+        out = _k.host().packed_prefill(query, k_cache, v_cache, block_table, kv_lens, positions, query_start_loc, layer_idx,
+                                       block_size, scale, num_key_value_groups, num_decode_rows)
+        if out is not None:
+            dtype = out_dtype if out_dtype is not None else k_cache.dtype
+            return out if dtype is torch.float32 else out.to(dtype)
     if query.ndim != 4 or query.shape[0] != 1:
         raise ValueError("packed prefill query must have shape [1, token_bucket, heads, head_dim]")
     if positions.shape != token_row_ids.shape or positions.shape[0] != 1:

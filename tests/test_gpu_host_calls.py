@@ -1,0 +1,83 @@
+"""The host module's calls against the Python route: the same numbers from operands it declines (strided, int64) as from
+those it takes, slots made inside the append equal the slot mapping's, lengths capped inside the kernel equal lengths
+clipped in front of it."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import BS, SCALE, bits, decode_case, to_numpy, to_torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _strided(t):
+    """The same values behind a layout that the host module declines."""
+    return torch.stack([t, t], -1)[..., 0]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("rows", [1, 5])
+def test_fused_decode_takes_both_routes_alike(rows, dtype):
+    from nano_vllm_jax_b200.backends import B200Backend
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    from nano_vllm_jax_b200.kv_cache import KVCacheStorage
+    c = decode_case(3 + rows, 200, rows, 1, 300)
+    got = []
+    for odd in (False, True):
+        cache = KVCacheStorage(to_torch(c["k_cache"]).to(dtype), to_torch(c["v_cache"]).to(dtype))
+        args = [to_torch(c[n]).to(dtype) for n in ("q", "new_k", "new_v")]
+        tables, lens, pos = (to_torch(c[n]) for n in ("tables", "seq_lens", "positions"))
+        if odd:
+            args, lens, tables = [_strided(t) for t in args], lens.to(torch.int64), _strided(tables)
+            assert K.host().fused_decode(*args, cache.k_cache, cache.v_cache, tables, lens, pos, 0, BS, SCALE, 4, 0) is None
+        be = B200Backend()
+        md = be.build_attention_metadata(pos, tables, lens, BS, False)
+        cache, out = be.write_kv_and_attention(0, *args, cache, md, BS, SCALE, 4, False)
+        got.append((out, cache.k_cache, cache.v_cache))
+    for a, b in zip(*got):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        np.testing.assert_array_equal(bits(to_numpy(a)), bits(to_numpy(b)))
+
+
+@pytest.mark.parametrize("width,max_kv_len", [(1, None), (1, 37), (3, None), (3, 48), (6, 100)])
+def test_window_decode_equals_lengths_clipped_in_front(width, max_kv_len):
+    from nano_vllm_jax_b200 import kv_cache as kvc
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    c = decode_case(11, 300, 7, width, 400, empty_rows=(2,))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q = torch.randn((7, width, 8, 256), generator=g, device="cuda").to(torch.bfloat16)
+    k, v, tables, lens = (to_torch(c[n]) for n in ("k_cache", "v_cache", "tables", "seq_lens"))
+    pos = (lens[:, None] - width - 3 + torch.arange(width, device="cuda")[None]).to(torch.int32).contiguous()  # some negative
+    out = kvc.paged_attention_decode(q, k, v, tables, lens, BS, SCALE, 4, max_kv_len=max_kv_len, positions=pos, out_dtype=torch.float32)
+    capped = lens.clamp(max=max_kv_len or tables.shape[1] * BS)
+    if width == 1:
+        ref = K.paged_decode_attention(q[:, 0].contiguous(), k[0], v[0], tables, torch.minimum(capped, pos[:, 0] + 1), SCALE)
+    else:
+        ref = K.paged_decode_attention_wide(q, k[0], v[0], tables, capped, pos, SCALE)
+    assert torch.equal(out.reshape(-1), ref.reshape(-1))
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_append_makes_the_slots_that_the_slot_mapping_has(packed):
+    from nano_vllm_jax_b200.backends import B200Backend
+    from nano_vllm_jax_b200.kv_cache import KVCacheStorage
+    rng = np.random.default_rng(7)
+    (rows, cols), pool = ((1, 40) if packed else (4, 9)), 64
+    tables = to_torch(rng.permutation(pool)[:24].reshape(4, 6).astype(np.int32))
+    places = rng.permutation(96)[: rows * cols] if packed else np.stack([rng.permutation(96)[:cols] for _ in range(rows)])
+    pos = to_torch(places.reshape(rows, cols).astype(np.int32))
+    rid = to_torch(np.sort(rng.integers(-1, 6, size=(1, cols))).astype(np.int32)) if packed else None  # clipped to the table's rows
+    qsl = to_torch(np.array([0, 9, 18, 30, 35] if packed else [0, 9, 12, 21, 21], np.int32))
+    new = [to_torch(rng.standard_normal((rows, cols, 2, 256)).astype(np.float32)) for _ in range(2)]
+    got = []
+    for read_first in (False, True):
+        be = B200Backend()
+        cache = KVCacheStorage(*(torch.zeros((2, pool, BS, 2, 256), dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+        md = be.build_attention_metadata(pos, tables, to_torch(np.full(4, 96, np.int32)), BS, True, query_start_loc=qsl, token_row_ids=rid)
+        if read_first:
+            assert md.slot_mapping.shape == pos.shape
+        be.write_kv(1, *new, cache, md)
+        got.append(cache)
+    assert float(got[0].k_cache[1].float().abs().sum()) > 0 and not got[0].k_cache[0].any()
+    assert torch.equal(got[0].k_cache, got[1].k_cache) and torch.equal(got[0].v_cache, got[1].v_cache)
