@@ -193,8 +193,10 @@ int nvj_paged_decode_workspace_init(void* workspace, size_t workspace_bytes,
  *   variant      0 = auto, 1 = generic kernel; for the model's shape (bf16 cache, block_size 16,
  *                2 kv heads x 4 q heads, head_dim 256): 2 = bulk-copy pipelined kernel on the CUDA
  *                cores (bf16 or f32 queries), 3 = TMA-staged streaming kernel with the products on
- *                tensor-core tiles (bf16 queries; what auto picks first).  NVJ_ERR_UNSUPPORTED when
- *                2 or 3 is asked for another shape.
+ *                tensor-core tiles (bf16 queries; what auto picks for all but short bf16 batches); 4 = thread-block
+ *                clusters (the same head layout with a bf16, f16 or f32 cache; what auto picks for short
+ *                bf16 batches and for f16 and f32 caches).  NVJ_ERR_UNSUPPORTED when 2, 3 or 4 is asked
+ *                for another shape or dtype.
  */
 int nvj_paged_decode(const void* q, int q_dtype,
                      const void* k_cache_layer, const void* v_cache_layer, int kv_dtype,

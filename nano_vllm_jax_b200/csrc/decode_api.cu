@@ -14,6 +14,13 @@ static bool pipelined_shape(const DecodeParams& p) {
          (!p.new_k || (aligned16(p.new_k) && aligned16(p.new_v)));
 }
 
+// The cluster kernel takes the same head layout with any cache and query dtype.
+static bool cluster_shape(const DecodeParams& p) {
+  return p.block_size == kBlk && p.num_kv_heads == kHkv && p.num_q_heads == kHq && p.head_dim == kD && aligned16(p.q) &&
+         aligned16(p.k_cache) && aligned16(p.v_cache) && aligned16(p.out) &&
+         (!p.new_k || (aligned16(p.new_k) && aligned16(p.new_v) && !p.kv_indptr));
+}
+
 static int carve_workspace(DecodeParams& p, void* workspace, size_t bytes, int num_ctas) {
   return carve_decode_workspace(p, workspace, bytes, ws_ml_bytes(num_ctas), ws_acc_bytes(num_ctas));
 }
@@ -24,7 +31,7 @@ static int run_decode(DecodeParams& p, void* workspace, size_t workspace_bytes, 
       p.num_kv_heads <= 0 || p.num_q_heads <= 0 || p.head_dim <= 0)
     return NVJ_ERR_INVALID_ARGUMENT;
   if (p.num_q_heads % p.num_kv_heads != 0) return NVJ_ERR_INVALID_ARGUMENT;
-  if (variant < 0 || variant > 3) return NVJ_ERR_INVALID_ARGUMENT;
+  if (variant < 0 || variant > 4) return NVJ_ERR_INVALID_ARGUMENT;
   if (p.batch == 0) return NVJ_OK;
   if (!p.q || !p.k_cache || !p.v_cache || !p.block_tables || !p.seq_lens || !p.out)
     return NVJ_ERR_INVALID_ARGUMENT;
@@ -38,6 +45,14 @@ static int run_decode(DecodeParams& p, void* workspace, size_t workspace_bytes, 
   // The tensor-core streaming kernel (bf16 queries) first: one CTA per SM, whole blocks by TMA, products on
   // mma.sync tiles; it needs a tensor-map encoder from the driver.  Then the CUDA-core pipelined kernel.
   const bool mma_ok = fast_ok && p.q_dtype == NVJ_BF16;
+  const bool cluster_ok = cluster_shape(p);
+  if (variant == 4 && !cluster_ok) return NVJ_ERR_UNSUPPORTED;
+  const bool bf16 = p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16;
+  // Short bf16 batches and every f32 / f16 cache: the cluster kernel.
+  if (variant == 4 || (variant == 0 && cluster_ok && (bf16 ? !p.kv_indptr && decode_cluster_pays(p.batch, p.table_width) : !fast_ok))) {
+    const int rc4 = launch_decode_cluster(p, stream);
+    if (rc4 != NVJ_ERR_UNSUPPORTED || variant == 4) return rc4;
+  }
   if ((variant == 2 && !fast_ok) || (variant == 3 && !mma_ok)) return NVJ_ERR_UNSUPPORTED;
   if (variant == 3 || (variant == 0 && mma_ok)) {
     p.width = 1;

@@ -166,6 +166,8 @@ size_t prefill_split_bytes();
 
 int decode_num_ctas();  // 2 per SM of the current device
 int launch_decode_generic(const DecodeParams& p, cudaStream_t stream);
+int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream);  // short batches; f32 and f16 caches
+bool decode_cluster_pays(int batch, int table_width);  // a bf16 batch is short enough for it
 int launch_decode_pipelined(const DecodeParams& p, int num_ctas, cudaStream_t stream);
 int decode_wide_num_ctas();  // 1 per SM of the current device
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // tensor-core streaming kernels, width 1..8

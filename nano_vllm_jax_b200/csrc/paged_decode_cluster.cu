@@ -1,0 +1,736 @@
+// Paged GQA decode attention on thread-block clusters: the kernel for short batches, and for f32 / f16 caches, of the
+// model's head layout (16-token blocks, 2 KV heads x 4 query heads, head_dim 256).
+//
+// A short batch is bound by latency, not by bytes.  The streaming kernel (paged_decode_wide.cu) needs 12 - 13 us for any:
+// a scan that finds each CTA's range, block ids through shared memory, the first bulk copies, then a chain of fence,
+// counter and fold through the far L2 for every row that is cut over CTAs.  Here the split needs no scan and the merge
+// no counter:
+//   * one cluster of C CTAs per (row, KV head); the cluster's warps take the row's blocks in turn (f32: units of 4 keys).
+//     Block ids are requested together with the row's length (the table entry exists whatever the length is), so that K
+//     and V are the second trip to memory;
+//   * the warps merge through shared memory, the C CTAs through distributed shared memory: two cluster barriers instead
+//     of fences and counters; rank r writes its 1 / C of the output;
+//   * fused append: the cluster's first warp stores the new row, and whoever attends its key reads it from the operand.
+// Nothing waits on memory that somebody else must fill, so there is no wait to bound.
+// Measured (us per launch, K/V cold, lengths spread over [n / 4, n]; before: the streaming kernel): 4 rows of n = 512 tokens
+// 12.9 -> 5.9, 8 of 4096 20 -> 15, 48 of 1024 21.8 -> 16.2, 256 of 512 43.0 -> 34.4, 256 of 2048 114 -> 110.  f32: 8 rows of
+// 64 - 512 tokens 94 (the generic kernel) -> 9.
+// Semantics: nanovllm_jax/kv_cache.py:852-998 for width-1 queries, nanovllm_jax/kernels/full_attention_triton.py:373-485
+// for the fused append.
+
+#include <type_traits>
+
+#include "decode_parts.cuh"
+
+namespace nvj {
+
+constexpr int kClMaxCluster = 16;
+
+// ---- f32 caches (and f16 ones under f32 queries): fp32 products on the CUDA cores --------------------------------
+// Every warp keeps kClStages units of 4 keys in flight in a ring of its own in shared memory (16-byte cp.async); lane l
+// copies and later reads dims 8 l .. 8 l + 7 of every row, so the ring needs no barrier of any kind.  The 4 keys x 4 heads
+// partial dot products are reduced by a select-free butterfly: lanes hold keys and heads in permuted order.
+constexpr int kClWarps = 8;
+constexpr int kClThreads = kClWarps * 32;
+constexpr int kClUnit = 4;  // keys a warp takes at a time
+constexpr int kClStages = 3;
+
+// The ring [warp][stage][K | V][key][row], later the merge buffers.
+struct ClusterMerge {
+  alignas(16) float acc[kClWarps][kG][kD];  // per warp; the merged sums of the CTA end up in acc[0]
+  float2 ml[kClWarps][kG];                  // per warp (max, sum)
+  float2 ML[kG];                            // of the CTA
+};
+template <typename T>
+constexpr int cluster_smem_bytes() {
+  constexpr int ring = kClWarps * kClStages * 2 * kClUnit * kD * (int)sizeof(T);
+  return ring > (int)sizeof(ClusterMerge) ? ring : (int)sizeof(ClusterMerge);
+}
+
+// Eight elements of a row per lane, as loaded.
+template <typename T> struct ClRaw { uint4 v; };
+template <> struct ClRaw<float> { uint4 v, w; };
+
+// This lane's 16-byte pieces of a row: `at` is the lane's place in the ring's row, pieces 512 bytes apart.
+__device__ __forceinline__ void cl_copy16(uint32_t dst, const char* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cl_copy16_or_zero(uint32_t dst, const char* src, uint32_t size) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void cl_copy_row(uint32_t row, const char* src, int lane) {
+  if constexpr (sizeof(T) == 4) {  // dims 8 l .. 8 l + 3 in the row's first half, 8 l + 4 .. in its second: no bank conflicts
+    cl_copy16(row + lane * 16, src + lane * 32);
+    cl_copy16(row + 512 + lane * 16, src + lane * 32 + 16);
+  } else {
+    cl_copy16(row + lane * 16, src + lane * 16);
+  }
+}
+__device__ __forceinline__ uint4 cl_lds(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+template <typename T>
+__device__ __forceinline__ ClRaw<T> cl_read_row(uint32_t row, int lane) {
+  ClRaw<T> r;
+  r.v = cl_lds(row + lane * 16);
+  if constexpr (sizeof(T) == 4) r.w = cl_lds(row + 512 + lane * 16);
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ void cl_unpack(const ClRaw<T>& r, float2 (&o)[4]) {
+  if constexpr (sizeof(T) == 4) {
+    o[0] = make_float2(__uint_as_float(r.v.x), __uint_as_float(r.v.y));
+    o[1] = make_float2(__uint_as_float(r.v.z), __uint_as_float(r.v.w));
+    o[2] = make_float2(__uint_as_float(r.w.x), __uint_as_float(r.w.y));
+    o[3] = make_float2(__uint_as_float(r.w.z), __uint_as_float(r.w.w));
+  } else if constexpr (std::is_same<T, __half>::value) {
+    o[0] = __half22float2(*reinterpret_cast<const __half2*>(&r.v.x));
+    o[1] = __half22float2(*reinterpret_cast<const __half2*>(&r.v.y));
+    o[2] = __half22float2(*reinterpret_cast<const __half2*>(&r.v.z));
+    o[3] = __half22float2(*reinterpret_cast<const __half2*>(&r.v.w));
+  } else {
+    o[0] = bf16x2_to_float2(r.v.x);
+    o[1] = bf16x2_to_float2(r.v.y);
+    o[2] = bf16x2_to_float2(r.v.z);
+    o[3] = bf16x2_to_float2(r.v.w);
+  }
+}
+
+__device__ __forceinline__ uint32_t cl_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address of this CTA's shared-memory location in CTA `rank` of the cluster, and loads from there.
+__device__ __forceinline__ uint32_t cl_map(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float4 cl_ld4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 cl_ld2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+
+// The CTAs' sums [head][pitch] and (max, sum) pairs, at the same places in every CTA of the cluster, into the output: rank
+// r takes its 1 / ctas of the 256 float4 pieces of [4 heads][256 dims].
+__device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, const float2* ML, int ctas, uint32_t rank, int threads,
+                                                float* dst) {
+  const int per = kG * kD / 4 / ctas;
+  for (int i = threadIdx.x; i < per; i += threads) {
+    const int piece = (int)rank * per + i, h = piece >> 6, d = (piece & 63) * 4;
+    float2 e[kClMaxCluster];
+    float4 x[kClMaxCluster];
+#pragma unroll
+    for (int c = 0; c < kClMaxCluster; ++c) {
+      e[c] = make_float2(kNegBig, 0.f);
+      x[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < ctas) {
+        e[c] = cl_ld2(cl_map(ML + h, c));
+        x[c] = cl_ld4(cl_map(acc + h * pitch + d, c));
+      }
+    }
+    float M = kNegBig, L = 0.f;
+#pragma unroll
+    for (int c = 0; c < kClMaxCluster; ++c) M = fmaxf(M, e[c].x);
+    float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < kClMaxCluster; ++c) {
+      const float f = ex2_approx(e[c].x - M);
+      L = fmaf(e[c].y, f, L);
+      y.x = fmaf(x[c].x, f, y.x); y.y = fmaf(x[c].y, f, y.y); y.z = fmaf(x[c].z, f, y.z); y.w = fmaf(x[c].w, f, y.w);
+    }
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    reinterpret_cast<float4*>(dst)[piece] = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_cluster_kernel(DecodeParams p) {
+  extern __shared__ __align__(128) unsigned char cl_smem_raw[];
+  ClusterMerge& sm = *reinterpret_cast<ClusterMerge*>(cl_smem_raw);
+  constexpr int kRowB = kD * (int)sizeof(T), kTokB = kHkv * kRowB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b = blockIdx.z, kvh = blockIdx.y, ctas = gridDim.x;
+  const uint32_t rank = ctas > 1 ? cl_rank() : 0u;
+  const int first = (int)rank * kClWarps + warp, stride = ctas * kClWarps;  // this warp's units: first, first + stride, ...
+
+  // ---- first trip: the ids of this warp's first 32 units, the length, the query
+  const long long tbase = decode_table_base(p, b);
+  int pages = p.table_width;
+  if (p.kv_indptr) pages = p.kv_indptr[b + 1] - (int)tbase;
+  auto unit_id = [&](int i) {  // lane i of a batch: block id of unit i
+    const int jb = (first + i * stride) / (kBlk / kClUnit);
+    return jb < pages ? p.block_tables[tbase + jb] : -1;
+  };
+  int ids = unit_id(lane);
+  const int len = decode_row_len(p, b);  // the same in every thread of the cluster
+  const long long qi = decode_query_index(p, b);
+  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) return;  // not this pass's row (whole cluster)
+  // query heads in slot order (slot h of a lane holds head h ^ hperm), times scale * log2(e)
+  const int rperm = lane >> 3, h_own = (lane >> 1) & 3;
+  float2 q2[kG][4];
+#pragma unroll
+  for (int h = 0; h < kG; ++h) {
+    const long long off = (qi * kHq + kvh * kG + (h ^ h_own)) * kD + lane * 8;
+    if (p.q_dtype == NVJ_F32) {
+      const float4 x = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + off);
+      const float4 y = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + off + 4);
+      q2[h][0] = make_float2(x.x, x.y); q2[h][1] = make_float2(x.z, x.w);
+      q2[h][2] = make_float2(y.x, y.y); q2[h][3] = make_float2(y.z, y.w);
+    } else if (p.q_dtype == NVJ_BF16) {
+      ClRaw<__nv_bfloat16> r{*reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.q) + off)};
+      cl_unpack(r, q2[h]);
+    } else {
+      ClRaw<__half> r{*reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + off)};
+      cl_unpack(r, q2[h]);
+    }
+    const float c = p.scale * kLog2e;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { q2[h][i].x *= c; q2[h][i].y *= c; }
+  }
+
+  // ---- fused append: where the new row goes; its key (if attended) is read from the operand
+  int new_key = -1;
+  const char* new_k = nullptr;
+  const char* new_v = nullptr;
+  if (p.new_k && len > 0) {
+    const int pos = p.pre_append ? p.seq_lens[b] : p.positions[b];
+    new_k = static_cast<const char*>(p.new_k) + (long long)b * kTokB + kvh * kRowB;
+    new_v = static_cast<const char*>(p.new_v) + (long long)b * kTokB + kvh * kRowB;
+    if (pos >= 0) {
+      const int jt = pos / kBlk;
+      const long long tgt = jt < p.table_width ? (long long)p.block_tables[tbase + jt] : -1;
+      if (tgt >= 0 && tgt < p.num_blocks) {
+        if (pos < len) new_key = pos;
+        if (first == 0) {
+          const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB;
+#pragma unroll
+          for (int i = 0; i < (int)sizeof(T) / 2; ++i) {
+            const int o = (i * 32 + lane) * 16;
+            *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst + o) = *reinterpret_cast<const uint4*>(new_k + o);
+            *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst + o) = *reinterpret_cast<const uint4*>(new_v + o);
+          }
+        }
+      } else if (first == 0 && lane == 0) {
+        atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
+      }
+    } else if (!std::is_same<T, __nv_bfloat16>::value && first == 0 && lane == 0) {
+      atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
+    }
+  }
+
+  // ---- the warp's units: four keys at a time, key slot r of a lane holds key r ^ rperm of the unit
+  const int units = (len + kClUnit - 1) / kClUnit;
+  float2 acc[kG][4];
+  float m4[kG], m_own = kNegBig, l_part = 0.f;
+#pragma unroll
+  for (int h = 0; h < kG; ++h) {
+    m4[h] = kNegBig;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[h][i] = make_float2(0.f, 0.f);
+  }
+  // Row of key `key` of unit u, from the cache or (the step's own key) from the operand.  Keys behind the last attended one
+  // are read as that one again and masked below: no load depends on a branch, so all of a unit's loads go out together.
+  auto row_of = [&](const char* cache, const char* fresh, int u, long long blk, int key) -> const char* {
+    int t = u * kClUnit + key;
+    t = t < len ? t : len - 1;
+    const char* row = cache + (blk * kBlk + t % kBlk) * kTokB + kvh * kRowB;
+    return t == new_key ? fresh : row;
+  };
+  const uint32_t ring = smem_u32(cl_smem_raw) + warp * (kClStages * 2 * kClUnit * kRowB);
+  // all of a unit's rows into ring stage `stage`, as one group of copies
+  auto request = [&](int u, long long blk, int stage) {
+    const uint32_t at = ring + stage * (2 * kClUnit * kRowB);
+#pragma unroll
+    for (int r = 0; r < kClUnit; ++r) {
+      cl_copy_row<T>(at + r * kRowB, row_of(p.k_cache, new_k, u, blk, r), lane);
+      cl_copy_row<T>(at + (kClUnit + r) * kRowB, row_of(p.v_cache, new_v, u, blk, r), lane);
+    }
+  };
+  // The warp's i-th unit that lies in the pool, at or after unit u; a bad block id is flagged and its keys are left out.
+  int u = first, i = 0;
+  auto next_unit = [&](int& u, int& i) -> long long {
+    for (; u < units; u += stride, ++i) {
+      if ((i & 31) == 0 && i > 0) ids = unit_id(i + lane);
+      const long long blk = __shfl_sync(kFullMask, ids, i & 31);
+      if (blk >= 0 && blk < p.num_blocks) return blk;
+      if (lane == 0) atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
+    }
+    return 0;
+  };
+  int pending[kClStages];  // units in flight, in order (units: none)
+#pragma unroll
+  for (int st = 0; st < kClStages; ++st) {
+    const long long blk = next_unit(u, i);
+    pending[st] = u;
+    if (u < units) { request(u, blk, st); u += stride; ++i; }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int stage = 0; pending[0] < units; stage = stage + 1 == kClStages ? 0 : stage + 1) {
+    const int left = len - pending[0] * kClUnit;  // keys of the unit that are attended (at least one)
+    const uint32_t at = ring + stage * (2 * kClUnit * kRowB);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kClStages - 1) : "memory");
+    float s[16];
+#pragma unroll
+    for (int r = 0; r < kClUnit; ++r) {  // key slot r of a lane holds key r ^ rperm of the unit
+      float2 k2[4];
+      cl_unpack(cl_read_row<T>(at + (r ^ rperm) * kRowB, lane), k2);
+#pragma unroll
+      for (int h = 0; h < kG; ++h) {
+        float2 a = fma2(q2[h][0], k2[0], make_float2(0.f, 0.f));
+        a = fma2(q2[h][1], k2[1], a);
+        a = fma2(q2[h][2], k2[2], a);
+        a = fma2(q2[h][3], k2[3], a);
+        s[r * 4 + h] = a.x + a.y;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] += __shfl_xor_sync(kFullMask, s[e + 8], 16);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] += __shfl_xor_sync(kFullMask, s[e + 4], 8);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) s[e] += __shfl_xor_sync(kFullMask, s[e + 2], 4);
+    s[0] += __shfl_xor_sync(kFullMask, s[1], 2);
+    float sc = s[0] + __shfl_xor_sync(kFullMask, s[0], 1);  // score of (key rperm, head h_own)
+    if (rperm >= left) sc = -INFINITY;
+    float bm = fmaxf(sc, __shfl_xor_sync(kFullMask, sc, 8));
+    bm = fmaxf(bm, __shfl_xor_sync(kFullMask, bm, 16));
+    if (__any_sync(kFullMask, bm > m_own)) {
+#pragma unroll
+      for (int j = 0; j < kG; ++j) {
+        const float bj = __shfl_sync(kFullMask, bm, j * 2);
+        const float mn = fmaxf(m4[j], bj);
+        const float a = ex2_approx(m4[j] - mn);
+        m4[j] = mn;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { acc[j][c].x *= a; acc[j][c].y *= a; }
+        if (h_own == j) { l_part *= a; m_own = mn; }
+      }
+    }
+    const float pw = ex2_approx(sc - m_own);
+    l_part += pw;
+#pragma unroll
+    for (int r = 0; r < kClUnit; ++r) {
+      float2 v2[4];
+      cl_unpack(cl_read_row<T>(at + (kClUnit + r) * kRowB, lane), v2);
+#pragma unroll
+      for (int h = 0; h < kG; ++h) {
+        const float w = __shfl_sync(kFullMask, pw, r * 8 + h * 2);
+        const float2 ww = make_float2(w, w);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[h][c] = fma2(ww, v2[c], acc[h][c]);
+      }
+    }
+    // the stage is free (this lane alone reads what it copied): the next unit goes in
+#pragma unroll
+    for (int st = 0; st + 1 < kClStages; ++st) pending[st] = pending[st + 1];
+    const long long blk = next_unit(u, i);
+    pending[kClStages - 1] = u;
+    if (u < units) { request(u, blk, stage); u += stride; ++i; }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();  // the merge buffers lie over the rings
+
+  // ---- merge the eight warps, then the cluster
+  float lh = l_part;
+  lh += __shfl_xor_sync(kFullMask, lh, 8);
+  lh += __shfl_xor_sync(kFullMask, lh, 16);
+#pragma unroll
+  for (int h = 0; h < kG; ++h) {
+    const float l = __shfl_sync(kFullMask, lh, h * 2);
+    if (lane == 0) sm.ml[warp][h] = make_float2(m4[h], l);
+    *reinterpret_cast<float4*>(&sm.acc[warp][h][lane * 8]) = make_float4(acc[h][0].x, acc[h][0].y, acc[h][1].x, acc[h][1].y);
+    *reinterpret_cast<float4*>(&sm.acc[warp][h][lane * 8 + 4]) = make_float4(acc[h][2].x, acc[h][2].y, acc[h][3].x, acc[h][3].y);
+  }
+  __syncthreads();
+  float4 o;
+  float M, L;
+  const int h = threadIdx.x >> 6, d4 = (threadIdx.x & 63) * 4;  // thread = four dims of one head
+  {
+    M = kNegBig;
+#pragma unroll
+    for (int w = 0; w < kClWarps; ++w) M = fmaxf(M, sm.ml[w][h].x);
+    L = 0.f;
+    o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kClWarps; ++w) {
+      const float2 e = sm.ml[w][h];
+      const float f = ex2_approx(e.x - M);
+      const float4 x = *reinterpret_cast<const float4*>(&sm.acc[w][h][d4]);
+      L = fmaf(e.y, f, L);
+      o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
+    }
+  }
+  float* dst = p.out + (qi * kHq + kvh * kG) * kD;
+  if (ctas == 1) {
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    reinterpret_cast<float4*>(dst)[threadIdx.x] = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    return;
+  }
+  __syncthreads();  // acc[0] is overwritten
+  *reinterpret_cast<float4*>(&sm.acc[0][h][d4]) = o;
+  if ((threadIdx.x & 63) == 0) sm.ML[h] = make_float2(M, L);
+  cl_sync();
+  cl_fold_cluster(&sm.acc[0][0][0], kD, sm.ML, ctas, rank, kClThreads, dst);
+  cl_sync();  // nobody leaves while its shared memory is being read
+}
+
+// ---- 16-bit caches: the products on tensor-core tiles -------------------------------------------------------------
+// A warp's unit is a whole block (16 keys) of its KV head.  Both products are taken transposed, so that the four query
+// heads sit in the N = 8 columns of mma.m16n8k16 instead of wasting 12 of 16 rows:
+//   S^T = K Q^T   M = 16 keys, N = 8 columns (the four heads, twice), 16 steps over the dims;
+//   O^T = V^T P^T  M = 16 dims (16 tiles), N = 8: columns 0-3 take the weights rounded to 16 bits, columns 4-7 what the
+//                 rounding left over, so that one MMA carries both terms; they are added at the end.
+// 32 MMAs and 32 ldmatrix per block and head, an eighth of the instructions of the CUDA-core form above, which bound
+// that form at ~1500 cycles per unit of 4 keys and warp.  One block per warp is in flight: the next block's K rows are
+// requested as soon as the scores are computed, its V rows after the weighted sum, and three CTAs of 64 KiB overlap on an
+// SM.  (Three blocks per warp and one CTA per SM were measured: the same within 5% where CTAs are few, worse where they
+// are many.  What one SM takes in, ~57 GB/s, is the limit then, so a row's blocks must be spread over SMs instead.)
+constexpr int kCmWarps = 4;
+constexpr int kCmThreads = kCmWarps * 32;
+constexpr int kCmPitch = kD + 4;  // floats between the columns of a warp's output tile: conflict-free stores
+
+struct CmSmem {
+  union {
+    char ring[kCmWarps][2][kBlk][kD * 2];  // [warp][K | V][key][16-byte piece c of the row at c ^ (key & 7)]
+    struct {
+      float acc[kCmWarps][2 * kG][kCmPitch];  // [warp][column][dim]; the CTA's merged sums end up in acc[0][0 .. 3]
+      float2 ml[kCmWarps][kG];
+      float2 ML[kG];
+    } m;
+  };
+};
+
+__device__ __forceinline__ void cm_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void cm_ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ uint32_t cm_transpose(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+template <typename T>
+__device__ __forceinline__ void cm_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (std::is_same<T, __half>::value)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two weights as a 16-bit pair (x low): rounded, or with `rest` what the rounding left over.
+template <typename T>
+__device__ __forceinline__ uint32_t cm_pack(float x, float y, bool rest) {
+  if constexpr (std::is_same<T, __half>::value) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    return rest ? *reinterpret_cast<const uint32_t*>(&l) : *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
+    return rest ? *reinterpret_cast<const uint32_t*>(&l) : *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(DecodeParams p) {
+  extern __shared__ __align__(128) unsigned char cl_smem_raw[];
+  CmSmem& sm = *reinterpret_cast<CmSmem*>(cl_smem_raw);
+  constexpr int kRowB = kD * 2, kTokB = kHkv * kRowB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int b = blockIdx.z, kvh = blockIdx.y, ctas = gridDim.x;
+  const uint32_t rank = ctas > 1 ? cl_rank() : 0u;
+  const int first = (int)rank * kCmWarps + warp, stride = ctas * kCmWarps;  // this warp's blocks: first, first + stride, ...
+
+  // ---- first trip: the ids of this warp's first 32 blocks, the length, the query
+  const long long tbase = decode_table_base(p, b);
+  int pages = p.table_width;
+  if (p.kv_indptr) pages = p.kv_indptr[b + 1] - (int)tbase;
+  auto block_id = [&](int i) {
+    const int jb = first + i * stride;
+    return jb < pages ? p.block_tables[tbase + jb] : -1;
+  };
+  int ids = block_id(lane);
+  const int len = decode_row_len(p, b);
+  const long long qi = decode_query_index(p, b);
+  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) return;  // not this pass's row (whole cluster)
+  uint32_t qb[16][2];  // Q^T as the B operand: column g = head g & 3
+  {
+    const char* q = static_cast<const char*>(p.q) + ((qi * kHq + kvh * kG + (g & 3)) * kD) * 2;
+#pragma unroll
+    for (int ks = 0; ks < 16; ++ks) {
+      qb[ks][0] = *reinterpret_cast<const uint32_t*>(q + ks * 32 + t * 4);
+      qb[ks][1] = *reinterpret_cast<const uint32_t*>(q + ks * 32 + 16 + t * 4);
+    }
+  }
+
+  // ---- fused append: where the new row goes; its key (if attended) is read from the operand
+  int new_key = -1;
+  const char* new_k = nullptr;
+  const char* new_v = nullptr;
+  if (p.new_k && len > 0) {
+    const int pos = p.pre_append ? p.seq_lens[b] : p.positions[b];
+    new_k = static_cast<const char*>(p.new_k) + (long long)b * kTokB + kvh * kRowB + lane * 16;
+    new_v = static_cast<const char*>(p.new_v) + (long long)b * kTokB + kvh * kRowB + lane * 16;
+    if (pos >= 0) {
+      const int jt = pos / kBlk;
+      const long long tgt = jt < p.table_width ? (long long)p.block_tables[tbase + jt] : -1;
+      if (tgt >= 0 && tgt < p.num_blocks) {
+        if (pos < len) new_key = pos;
+        if (first == 0) {
+          const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB + lane * 16;
+          *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst) = *reinterpret_cast<const uint4*>(new_k);
+          *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst) = *reinterpret_cast<const uint4*>(new_v);
+        }
+      } else if (first == 0 && lane == 0) {
+        atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
+      }
+    } else if (!std::is_same<T, __nv_bfloat16>::value && first == 0 && lane == 0) {
+      atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
+    }
+  }
+
+  // ---- the warp's blocks
+  const int nb = (len + kBlk - 1) / kBlk;
+  int asked = 0;  // blocks requested so far
+  auto next_id = [&]() -> long long {  // id of block first + asked * stride; -1 (and the flag) outside the pool
+    if ((asked & 31) == 0 && asked > 0) ids = block_id(asked + lane);
+    const long long blk = __shfl_sync(kFullMask, ids, asked & 31);
+    if (blk >= 0 && blk < p.num_blocks) return blk;
+    if (lane == 0) atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
+    return -1;
+  };
+  const uint32_t k_at = smem_u32(sm.ring[warp][0]), v_at = smem_u32(sm.ring[warp][1]);
+  // The 16 rows of block jb of one operand into `at`, as one group of copies.  Keys behind the last attended one are read as
+  // that one again and masked below; a bad block is filled with zeros and masked.
+  auto request = [&](uint32_t at, const char* cache, const char* fresh, int jb, long long blk) {
+    if (jb < nb) {
+      const char* src = cache + (blk < 0 ? 0 : blk) * kBlk * kTokB + kvh * kRowB + lane * 16;
+      const int last = len - 1 - jb * kBlk, mine = new_key - jb * kBlk;
+      const uint32_t size = blk < 0 ? 0u : 16u;
+#pragma unroll
+      for (int r = 0; r < kBlk; ++r) {
+        const int rr = r < last ? r : (last < kBlk - 1 ? last : r);
+        cl_copy16_or_zero(at + r * kRowB + ((lane ^ (r & 7)) << 4), rr == mine ? fresh : src + rr * kTokB, size);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");  // (also an empty one: the waits count groups)
+  };
+  float o[16][4];
+#pragma unroll
+  for (int n = 0; n < 16; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+  float m[2] = {kNegBig, kNegBig}, l[2] = {0.f, 0.f};  // of heads (2 t) & 3, (2 t + 1) & 3
+  const float scale_log2 = p.scale * kLog2e;
+  const uint32_t k_row = k_at + ((lane & 7) + ((lane >> 3) & 1) * 8) * kRowB, k_piece = lane >> 4;
+  const uint32_t v_row = v_at + ((lane & 7) + (lane >> 4) * 8) * kRowB, v_piece = (lane >> 3) & 1;
+  long long blk = first < nb ? next_id() : -1;
+  request(k_at, p.k_cache, new_k, first, blk);
+  request(v_at, p.v_cache, new_v, first, blk);
+  for (int j = first; j < nb; j += stride) {
+    const int left = blk >= 0 ? len - j * kBlk : 0;  // keys of the block that are attended
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // K has landed
+    __syncwarp();
+    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};  // two chains of eight
+#pragma unroll
+    for (int ks = 0; ks < 16; ks += 2) {
+      uint32_t a[4];
+      cm_ldsm4(k_row + (((ks * 2 + k_piece) ^ (lane & 7)) << 4), a);
+      cm_mma<T>(s0, a, qb[ks][0], qb[ks][1]);
+      cm_ldsm4(k_row + (((ks * 2 + 2 + k_piece) ^ (lane & 7)) << 4), a);
+      cm_mma<T>(s1, a, qb[ks + 1][0], qb[ks + 1][1]);
+    }
+    __syncwarp();
+    const int jn = j + stride;
+    ++asked;
+    blk = jn < nb ? next_id() : -1;
+    request(k_at, p.k_cache, new_k, jn, blk);
+    float s[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] = g + (e >> 1) * 8 < left ? (s0[e] + s1[e]) * scale_log2 : kNegBig;
+    float alpha[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float mx = fmaxf(s[c], s[c + 2]);
+      mx = fmaxf(mx, __shfl_xor_sync(kFullMask, mx, 4));
+      mx = fmaxf(mx, __shfl_xor_sync(kFullMask, mx, 8));
+      mx = fmaxf(mx, __shfl_xor_sync(kFullMask, mx, 16));
+      const float mn = fmaxf(m[c], mx);
+      alpha[c] = ex2_approx(m[c] - mn);
+      m[c] = mn;
+      l[c] *= alpha[c];
+    }
+    if (__any_sync(kFullMask, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+      for (int n = 0; n < 16; ++n) {
+        o[n][0] *= alpha[0]; o[n][1] *= alpha[1];
+        o[n][2] *= alpha[0]; o[n][3] *= alpha[1];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] = ex2_approx(s[e] - m[e & 1]);
+    l[0] += s[0] + s[2];
+    l[1] += s[1] + s[3];
+    const uint32_t b0 = cm_transpose(cm_pack<T>(s[0], s[1], t >= 2)), b1 = cm_transpose(cm_pack<T>(s[2], s[3], t >= 2));
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // V has landed
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+      uint32_t a[4];
+      cm_ldsm4_t(v_row + (((n * 2 + v_piece) ^ (lane & 7)) << 4), a);
+      cm_mma<T>(o[n], a, b0, b1);
+    }
+    __syncwarp();
+    request(v_at, p.v_cache, new_v, jn, blk);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();  // the merge buffers lie over the rings
+
+  // ---- merge the warps, then the cluster
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    l[c] += __shfl_xor_sync(kFullMask, l[c], 4);
+    l[c] += __shfl_xor_sync(kFullMask, l[c], 8);
+    l[c] += __shfl_xor_sync(kFullMask, l[c], 16);
+    if (lane < 2) sm.m.ml[warp][2 * t + c] = make_float2(m[c], l[c]);
+  }
+#pragma unroll
+  for (int n = 0; n < 16; ++n) {
+    sm.m.acc[warp][2 * t][n * 16 + g] = o[n][0];
+    sm.m.acc[warp][2 * t + 1][n * 16 + g] = o[n][1];
+    sm.m.acc[warp][2 * t][n * 16 + g + 8] = o[n][2];
+    sm.m.acc[warp][2 * t + 1][n * 16 + g + 8] = o[n][3];
+  }
+  __syncthreads();
+  constexpr int kPieces = kG * kD / 4, kPer = kPieces / kCmThreads;  // float4 pieces of the output, and per thread
+  float* dst = p.out + (qi * kHq + kvh * kG) * kD;
+  float4 sum[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int piece = k * kCmThreads + threadIdx.x, h = piece >> 6, d4 = (piece & 63) * 4;
+    float M = kNegBig, L = 0.f;
+#pragma unroll
+    for (int w = 0; w < kCmWarps; ++w) M = fmaxf(M, sm.m.ml[w][h].x);
+    sum[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kCmWarps; ++w) {
+      const float2 e = sm.m.ml[w][h];
+      const float f = ex2_approx(e.x - M);
+      const float4 x = *reinterpret_cast<const float4*>(&sm.m.acc[w][h][d4]), y = *reinterpret_cast<const float4*>(&sm.m.acc[w][h + kG][d4]);
+      L = fmaf(e.y, f, L);
+      sum[k].x = fmaf(x.x + y.x, f, sum[k].x); sum[k].y = fmaf(x.y + y.y, f, sum[k].y);
+      sum[k].z = fmaf(x.z + y.z, f, sum[k].z); sum[k].w = fmaf(x.w + y.w, f, sum[k].w);
+    }
+    if (ctas == 1) {
+      const float inv = L > 0.f ? 1.f / L : 0.f;
+      reinterpret_cast<float4*>(dst)[piece] = make_float4(sum[k].x * inv, sum[k].y * inv, sum[k].z * inv, sum[k].w * inv);
+    } else if ((piece & 63) == 0) {
+      sm.m.ML[h] = make_float2(M, L);
+    }
+  }
+  if (ctas == 1) return;
+  __syncthreads();  // acc[0] is overwritten
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int piece = k * kCmThreads + threadIdx.x;
+    *reinterpret_cast<float4*>(&sm.m.acc[0][piece >> 6][(piece & 63) * 4]) = sum[k];
+  }
+  cl_sync();
+  cl_fold_cluster(&sm.m.acc[0][0][0], kCmPitch, sm.m.ML, ctas, rank, kCmThreads, dst);
+  cl_sync();  // nobody leaves while its shared memory is being read
+}
+
+template <class Kernel>
+static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const DecodeParams& p, int cluster, int threads, int smem,
+                           cudaStream_t stream) {
+  if (!once_per_device(opted_in, [&](int) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+               cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      }))
+    return NVJ_ERR_LAUNCH;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster, kHkv, p.batch);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
+}
+
+// CTAs per (row, KV head) for a batch whose longest row may have `blocks` blocks.  Doubled while the CTAs still fit the SMs
+// three at a time and every warp of the longest row finds a block; and, in batches of many CTAs, until no warp has more
+// than 12 blocks, so that the last CTAs to finish are short ones.  Clusters of 16 (no longer portable, and placed one by
+// one) only up to 2.2 CTAs per SM.  (Measured at 1 - 256 rows of 64 - 16384 tokens: within 3% of the best size of each.)
+static int cluster_size(int batch, int blocks, int sms) {
+  int c = 1;
+  while (c < kClMaxCluster && 2 * c * kCmWarps <= blocks) {
+    const long long next = 2LL * c * kHkv * batch;
+    const bool fits = 10 * next <= (c < 8 ? 30LL : 22LL) * sms;
+    if (!fits && (c >= 8 || blocks <= 12 * c * kCmWarps)) break;
+    c *= 2;
+  }
+  return c;
+}
+
+// Whether this kernel, at its best cluster size, beats the streaming kernel (paged_decode_wide.cu) on a bf16 batch.  The
+// streaming kernel costs ~12.5 us whatever the batch plus its bytes at the HBM rate; this one ~4.5 us plus ~1.25 us per
+// block of the longest warp while CTAs have an SM each, and the HBM rate beyond that, where the streaming kernel's equal
+// shares win once a CTA's own work gets long.  `table_width` bounds the blocks of a row; lengths are on the device.
+bool decode_cluster_pays(int batch, int table_width) {
+  const int sms = decode_wide_num_ctas();
+  if (sms <= 0) return false;
+  const int c = cluster_size(batch, table_width, sms);
+  const int per_warp = (table_width + c * kCmWarps - 1) / (c * kCmWarps);
+  if ((long long)c * kHkv * batch >= sms) return per_warp <= 12;
+  return 1.25 * per_warp <= 9.5 + 0.0026 * batch * table_width;  // 32 KiB per block, half of the widest on average, 6.3 TB/s
+}
+
+int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
+  if (p.batch > 65535) return NVJ_ERR_UNSUPPORTED;
+  const int sms = decode_wide_num_ctas();
+  if (sms <= 0) return NVJ_ERR_LAUNCH;
+  // (with a page list per row its width is not known here: as many CTAs as an ordinary row has use for)
+  const int cluster = cluster_size(p.batch, p.kv_indptr ? 64 : p.table_width, sms);
+  static PerDeviceFlags flags[4];
+  if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16)
+    return launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16>, flags[0], p, cluster, kCmThreads, (int)sizeof(CmSmem), stream);
+  if (p.kv_dtype == NVJ_F16 && p.q_dtype == NVJ_F16)
+    return launch_clusters(decode_cluster_mma_kernel<__half>, flags[1], p, cluster, kCmThreads, (int)sizeof(CmSmem), stream);
+  if (p.kv_dtype == NVJ_F32)
+    return launch_clusters(decode_cluster_kernel<float>, flags[2], p, cluster, kClThreads, cluster_smem_bytes<float>(), stream);
+  if (p.kv_dtype == NVJ_F16)
+    return launch_clusters(decode_cluster_kernel<__half>, flags[3], p, cluster, kClThreads, cluster_smem_bytes<__half>(), stream);
+  return NVJ_ERR_UNSUPPORTED;  // bf16 cache with another query dtype: the streaming kernel on the CUDA cores
+}
+
+}  // namespace nvj

@@ -1,0 +1,87 @@
+"""The cluster form of the decode kernel against the generic one: block, unit and warp boundaries of a row, every cluster
+size, every cache and query dtype, both forms of the fused append, and a block id outside the pool."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import BS, SCALE, bits, decode_case, to_numpy, to_torch
+
+pytestmark = pytest.mark.gpu
+
+TIGHT = {torch.bfloat16: 2e-3, torch.float16: 5e-4, torch.float32: 2e-5}
+
+
+def _case(seed, lens, width, dtype):
+    c = decode_case(seed, int(sum(-(-n // BS) for n in lens)) + 9, len(lens), 1, 1, width=width)
+    rng = np.random.default_rng(seed)
+    lens = np.asarray(lens, np.int32)
+    perm = rng.permutation(c["k_cache"].shape[1])
+    tables, o = np.zeros((len(lens), width), np.int32), 0
+    for b, n in enumerate(-(-lens // BS)):
+        tables[b, :n] = perm[o:o + n]
+        o += n
+    k, v = (to_torch(c[n]).to(dtype) for n in ("k_cache", "v_cache"))
+    for t in (k, v):  # what lies behind a row's last key must not reach the result
+        for b, n in enumerate(lens):
+            if n % BS:
+                t[0, int(tables[b, n // BS]), n % BS:] = float("nan")
+    return k, v, to_torch(tables), to_torch(lens), c
+
+
+# rows x table width (in blocks) pick the cluster size: 1, 2, 4, 8 and 16 CTAs per row and KV head
+@pytest.mark.parametrize("rows,width", [(3, 4), (3, 9), (3, 20), (3, 40), (2, 80), (40, 24), (150, 6)])
+@pytest.mark.parametrize("cache,query", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16), (torch.float32, torch.float32),
+                                         (torch.float16, torch.float32), (torch.float32, torch.bfloat16)])
+def test_cluster_decode_equals_the_generic_kernel(rows, width, cache, query):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    span = width * BS
+    edges = [n for n in (1, 3, 4, 15, 16, 17, 63, 64, 65, span - 16, span - 1, span, 0) if n <= span]
+    k, v, tables, lens, c = _case(rows + width, [edges[i % len(edges)] for i in range(rows)], width, cache)
+    q = to_torch(c["q"][:, 0]).to(query).contiguous()
+    got = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=4)
+    ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
+    assert float((got - ref).abs().max()) <= TIGHT[cache]
+    assert not got[lens == 0].any()
+
+
+@pytest.mark.parametrize("pre_append", [False, True])
+@pytest.mark.parametrize("cache", [torch.bfloat16, torch.float16, torch.float32])
+def test_cluster_decode_with_the_fused_append(cache, pre_append):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    lens = [1, 16, 17, 33, 0, 144, 129]
+    k, v, tables, t_lens, c = _case(5, lens, 9, cache)
+    q, nk, nv = (to_torch(c[n]).to(cache) for n in ("q", "new_k", "new_v"))
+    pos = (t_lens - 1).clamp(min=0).view(-1, 1).contiguous()
+    k2, v2 = k.clone(), v.clone()
+    for b, n in enumerate(lens):
+        if n:
+            block, off = int(tables[b, (n - 1) // BS]), (n - 1) % BS
+            k2[0, block, off], v2[0, block, off] = nk[b, 0], nv[b, 0]
+    ref = K.paged_decode_attention(q[:, 0].contiguous(), k2[0], v2[0], tables, t_lens, SCALE, variant=1)
+    before = torch.where(t_lens > 0, t_lens - 1, t_lens)
+    if pre_append:  # a row of length 1 would be inactive before its first token: leave it out of the comparison
+        ref = ref.clone()
+        ref[0] = 0
+        k2[0, int(tables[0, 0]), 0], v2[0, int(tables[0, 0]), 0] = k[0, int(tables[0, 0]), 0], v[0, int(tables[0, 0]), 0]
+    out, k, v = K.paged_decode_attention_with_kv_append(q, nk, nv, k, v, tables, before if pre_append else t_lens,
+                                                        None if pre_append else pos, 0, BS, SCALE, 4, variant=4)
+    assert float((out.view(7, 8, 256) - ref).abs().max()) <= TIGHT[cache]
+    for a, b in ((k, k2), (v, v2)):
+        np.testing.assert_array_equal(bits(to_numpy(a)), bits(to_numpy(b)))
+
+
+def test_cluster_decode_flags_a_bad_block_and_leaves_its_keys_out(monkeypatch):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    k, v, tables, lens, c = _case(8, [200, 90], 13, torch.bfloat16)
+    q = to_torch(c["q"][:, 0]).contiguous()
+    bad = tables.clone()
+    bad[0, 12] = k.shape[1]  # the row's last block: the result is the row without it
+    with pytest.raises(K.DeviceStatusError):
+        K.paged_decode_attention(q, k[0], v[0], bad, lens, SCALE, variant=4)
+    monkeypatch.setenv("NVJ_CHECK_STATUS", "0")
+    got = K.paged_decode_attention(q, k[0], v[0], bad, lens, SCALE, variant=4)
+    ref = K.paged_decode_attention(q, k[0], v[0], tables, torch.tensor([192, 90], dtype=torch.int32, device="cuda"), SCALE, variant=1)
+    with pytest.raises(K.DeviceStatusError):
+        K.check_device_status()
+    assert float((got - ref).abs().max()) <= 2e-3
