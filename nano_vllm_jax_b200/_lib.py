@@ -116,8 +116,6 @@ def load() -> ctypes.CDLL:
             return _lib
         if os.environ.get("NVJ_FORCE_REBUILD", "0") == "1" or not _build.LIB_PATH.exists():
             _build.build(force=True)
-        elif not _build.HOST_PATH.exists():
-            _build.build_host()
         lib = ctypes.CDLL(str(_build.LIB_PATH), mode=ctypes.RTLD_GLOBAL)
         for name, (restype, argtypes) in SIGNATURES.items():
             fn = getattr(lib, name)  # AttributeError here = header and library disagree
@@ -127,6 +125,15 @@ def load() -> ctypes.CDLL:
             raise NvjError("libnvj_b200.so has an unexpected ABI version")
         _lib = lib
         return lib
+
+
+def host_module():
+    """The host extension module (csrc/host/host_ops.cpp), built first if it is absent."""
+    import torch  # noqa: F401  (the module links against torch's libraries)
+    if not _build.HOST_PATH.exists():
+        _build.build_host()
+    from . import _nvj_host
+    return _nvj_host
 
 
 def check(status: int, what: str) -> None:

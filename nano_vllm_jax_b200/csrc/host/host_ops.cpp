@@ -40,6 +40,9 @@ struct Library {
   decltype(&nvj_paged_prefill_packed_part) prefill_part;
   decltype(&nvj_qk_norm_rope_kv_append) norm_rope;
   decltype(&nvj_compute_slot_mapping) slot_mapping;
+  decltype(&nvj_copy_blocks) copy_blocks;
+  decltype(&nvj_hybrid_snapshot_host_slots) snapshot;
+  decltype(&nvj_hybrid_restore_host_slots) restore;
 };
 Library lib;
 PyObject* cb_workspace;  // (device index, rows): makes Python create the workspace and hand it over
@@ -389,6 +392,63 @@ PyObject* norm_rope(PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(out));
 }
 
+// copy_blocks(k_cache, v_cache, src_ids, dst_ids) -> True
+PyObject* copy_blocks(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 4)) return nullptr;
+  const at::Tensor *k = tensor(a[0]), *v = tensor(a[1]), *src = tensor(a[2]), *dst = tensor(a[3]);
+  const Layer l = cache_layer(k, v, 0);
+  if (!l.ok || !src || !dst || !meta(*src, l.device) || !meta(*dst, l.device) || src->dim() != 1 || src->sizes() != dst->sizes()) NVJ_NONE();
+  const long long block = (long long)l.block_size * l.hkv * l.d * k->element_size();
+  void* stream = stream_of(l.device);
+  int32_t* st = status_for(l.device, stream);
+  if (!st) return nullptr;
+  int rc;
+  NVJ_CALL(rc, lib.copy_blocks(l.k, l.v, (int)k->size(0), l.blocks, block, l.blocks * block, i32(*src), i32(*dst), (int)src->numel(), st, stream));
+  if (!finished(rc, "nvj_copy_blocks", l.device, false, true)) return nullptr;
+  Py_RETURN_TRUE;
+}
+
+// hybrid_copy(conv_table | None, rec_table | None, conv_pool | None, rec_pool | None, table_slots, pool_slots, restore) -> True,
+// for slot lists of at most NVJ_HYBRID_HOST_SLOTS entries in host memory
+PyObject* hybrid_copy(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 7)) return nullptr;
+  const at::Tensor* t[4];
+  const at::Tensor* some = nullptr;
+  for (int i = 0; i < 4; ++i) {
+    t[i] = a[i] == Py_None ? nullptr : tensor(a[i]);
+    if (a[i] != Py_None && (!t[i] || !t[i]->is_cuda() || !t[i]->is_contiguous() || t[i]->dim() < 1 || t[i]->size(0) < 1)) NVJ_NONE();
+    if (t[i]) some = t[i];
+  }
+  if (!some || (t[0] == nullptr) != (t[2] == nullptr) || (t[1] == nullptr) != (t[3] == nullptr) || !PyList_Check(a[4]) || !PyList_Check(a[5])) NVJ_NONE();
+  const int device = some->get_device();
+  long long bytes[4] = {0, 0, 0, 0};
+  for (int i = 0; i < 4; ++i)
+    if (t[i]) {
+      if (t[i]->get_device() != device) NVJ_NONE();
+      bytes[i] = t[i]->numel() / t[i]->size(0) * t[i]->element_size();
+    }
+  const Py_ssize_t pairs = PyList_GET_SIZE(a[4]);
+  if (bytes[0] != bytes[2] || bytes[1] != bytes[3] || pairs != PyList_GET_SIZE(a[5]) || pairs > NVJ_HYBRID_HOST_SLOTS) NVJ_NONE();
+  int32_t slots[2][NVJ_HYBRID_HOST_SLOTS];
+  for (int side = 0; side < 2; ++side)
+    for (Py_ssize_t i = 0; i < pairs; ++i) {
+      const long long v = PyLong_AsLongLong(PyList_GET_ITEM(a[4 + side], i));
+      if (PyErr_Occurred() || v < INT32_MIN || v > INT32_MAX) { PyErr_Clear(); NVJ_NONE(); }
+      slots[side][i] = (int32_t)v;
+    }
+  const int restore = PyObject_IsTrue(a[6]);
+  void* stream = stream_of(device);
+  int32_t* st = status_for(device, stream);
+  if (!st) return nullptr;
+  auto ptr = [&](int i) { return t[i] ? t[i]->data_ptr() : nullptr; };
+  const long long table_rows = (t[1] ? t[1] : t[0])->size(0), pool_rows = (t[3] ? t[3] : t[2])->size(0);
+  int rc;
+  if (restore) NVJ_CALL(rc, lib.restore(ptr(0), ptr(2), bytes[0], ptr(1), ptr(3), bytes[1], table_rows, pool_rows, slots[0], slots[1], (int)pairs, st, stream));
+  else NVJ_CALL(rc, lib.snapshot(ptr(0), ptr(2), bytes[0], ptr(1), ptr(3), bytes[1], table_rows, pool_rows, slots[0], slots[1], (int)pairs, st, stream));
+  if (!finished(rc, restore ? "nvj_hybrid_restore" : "nvj_hybrid_snapshot", device, false, true)) return nullptr;
+  Py_RETURN_TRUE;
+}
+
 // slot_mapping(positions [rows, cols], block_tables, block_size, token_row_ids | None) -> int32 [rows, cols]
 PyObject* slot_mapping(PyObject* const* a, Py_ssize_t n) {
   if (!args_are(n, 4)) return nullptr;
@@ -406,6 +466,131 @@ PyObject* slot_mapping(PyObject* const* a, Py_ssize_t n) {
                                 (int)tab->size(1), (int)bs, static_cast<int32_t*>(out.data_ptr()), stream));
   if (!finished(rc, "nvj_compute_slot_mapping", dev, false, false)) return nullptr;
   return THPVariable_Wrap(std::move(out));
+}
+
+// ---- prefix hashes --------------------------------------------------------------------------------------------------
+
+// XXH64 (seed 0) over 64-bit words, after the published specification of the xxHash family: four lanes over stripes of four
+// words, the words left over, an avalanche.  Blocks are whole words, so the specification's byte tail never occurs.
+class WordHash {
+  static constexpr uint64_t kP1 = 0x9E3779B185EBCA87ull, kP2 = 0xC2B2AE3D27D4EB4Full, kP3 = 0x165667B19E3779F9ull,
+                            kP4 = 0x85EBCA77C2B2AE63ull, kP5 = 0x27D4EB2F165667C5ull;
+  static uint64_t rotate(uint64_t x, int r) { return (x << r) | (x >> (64 - r)); }
+  static uint64_t mix(uint64_t lane, uint64_t word) { return rotate(lane + word * kP2, 31) * kP1; }
+
+ public:
+  static uint64_t of(const uint64_t* w, size_t n) {
+    uint64_t h = kP5;
+    size_t i = 0;
+    if (n >= 4) {
+      uint64_t lane[4] = {kP1 + kP2, kP2, 0, 0 - kP1};
+      for (; i + 4 <= n; i += 4)
+        for (int k = 0; k < 4; ++k) lane[k] = mix(lane[k], w[i + k]);
+      h = rotate(lane[0], 1) + rotate(lane[1], 7) + rotate(lane[2], 12) + rotate(lane[3], 18);
+      for (uint64_t v : lane) h = (h ^ mix(0, v)) * kP1 + kP4;
+    }
+    h += 8 * n;
+    for (; i < n; ++i) h = rotate(h ^ mix(0, w[i]), 27) * kP1 + kP4;
+    h = (h ^ (h >> 33)) * kP2;
+    h = (h ^ (h >> 29)) * kP3;
+    return h ^ (h >> 32);
+  }
+};
+
+// hash_chain(token_ids, block_size, blocks, prefix | -1) -> digests of the first `blocks` full blocks of a token list, each
+// over its predecessor's digest (the first over `prefix` if there is one) and its own tokens as int64.  None when the
+// tokens are not a list of machine-size integers.
+PyObject* hash_chain(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 4)) return nullptr;
+  const long long bs = PyLong_AsLongLong(a[1]), blocks = PyLong_AsLongLong(a[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!PyList_CheckExact(a[0]) || !PyLong_CheckExact(a[3]) || bs < 1 || blocks < 0 || blocks > PyList_GET_SIZE(a[0]) / bs) NVJ_NONE();
+  int overflow = 0;
+  bool chained = !(PyLong_AsLongLongAndOverflow(a[3], &overflow) == -1 && !overflow);
+  std::vector<uint64_t> words((size_t)bs + 1);
+  words[0] = chained ? PyLong_AsUnsignedLongLongMask(a[3]) : 0;
+  PyObject* out = PyList_New((Py_ssize_t)blocks);
+  if (!out) return nullptr;
+  for (long long b = 0; b < blocks; ++b) {
+    for (long long i = 0; i < bs; ++i) {
+      PyObject* item = PyList_GET_ITEM(a[0], (Py_ssize_t)(b * bs + i));
+      const long long v = PyLong_CheckExact(item) ? PyLong_AsLongLongAndOverflow(item, &overflow) : (overflow = 1, 0);
+      if (overflow) { Py_DECREF(out); NVJ_NONE(); }
+      words[(size_t)i + 1] = (uint64_t)v;
+    }
+    const uint64_t h = chained ? WordHash::of(words.data(), words.size()) : WordHash::of(words.data() + 1, words.size() - 1);
+    words[0] = h;
+    chained = true;
+    PyObject* d = PyLong_FromUnsignedLongLong(h);
+    if (!d) { Py_DECREF(out); return nullptr; }
+    PyList_SET_ITEM(out, (Py_ssize_t)b, d);
+  }
+  return out;
+}
+
+// ---- a batch's host arrays ------------------------------------------------------------------------------------------
+
+// One int32 out of a Python integer (anything with __index__); false with OverflowError or TypeError set.
+bool as_i32(PyObject* o, int32_t* v) {
+  const long long x = PyLong_AsLongLong(o);
+  if (x == -1 && PyErr_Occurred()) return false;
+  if (x < INT32_MIN || x > INT32_MAX) {
+    PyErr_SetString(PyExc_OverflowError, "a batch entry does not fit 32 bits");
+    return false;
+  }
+  *v = (int32_t)x;
+  return true;
+}
+
+// pack_i32(address, words, parts, rows_at, rows, width) -> tuple of the rows, padded with zeros to `width`.
+// Fills `words` int32 at `address` (a pinned staging buffer): zeros, then every part (offset, list of ints), then the lists
+// in `rows` as a [len(rows), width] table at `rows_at`.
+PyObject* pack_i32(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 6)) return nullptr;
+  int32_t* base = reinterpret_cast<int32_t*>(PyLong_AsUnsignedLongLong(a[0]));
+  const long long words = PyLong_AsLongLong(a[1]), rows_at = PyLong_AsLongLong(a[3]), width = PyLong_AsLongLong(a[5]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!base || words < 0 || !PyList_Check(a[2]) || !PyList_Check(a[4]) || width < 0 || rows_at < 0 ||
+      rows_at + PyList_GET_SIZE(a[4]) * width > words) {
+    PyErr_SetString(PyExc_ValueError, "pack_i32: the parts do not fit the buffer");
+    return nullptr;
+  }
+  std::memset(base, 0, (size_t)words * sizeof(int32_t));
+  for (Py_ssize_t p = 0; p < PyList_GET_SIZE(a[2]); ++p) {
+    PyObject *part = PyList_GET_ITEM(a[2], p), *list;
+    long long at;
+    if (!PyArg_ParseTuple(part, "LO!", &at, &PyList_Type, &list)) return nullptr;
+    const Py_ssize_t len = PyList_GET_SIZE(list);
+    if (at < 0 || at + len > words) {
+      PyErr_SetString(PyExc_ValueError, "pack_i32: the parts do not fit the buffer");
+      return nullptr;
+    }
+    for (Py_ssize_t i = 0; i < len; ++i)
+      if (!as_i32(PyList_GET_ITEM(list, i), base + at + i)) return nullptr;
+  }
+  const Py_ssize_t rows = PyList_GET_SIZE(a[4]);
+  PyObject* zero = PyLong_FromLong(0);
+  PyObject* out = PyTuple_New(rows);
+  for (Py_ssize_t r = 0; out && r < rows; ++r) {
+    PyObject* list = PyList_GET_ITEM(a[4], r);
+    PyObject* row = PyList_Check(list) && PyList_GET_SIZE(list) <= width ? PyTuple_New((Py_ssize_t)width) : nullptr;
+    if (!row) {
+      if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "pack_i32: a row is no list or too long");
+      Py_CLEAR(out);
+      break;
+    }
+    PyTuple_SET_ITEM(out, r, row);
+    const Py_ssize_t len = PyList_GET_SIZE(list);
+    for (Py_ssize_t i = 0; i < (Py_ssize_t)width; ++i) {
+      PyObject* item = i < len ? PyList_GET_ITEM(list, i) : zero;
+      if (i < len && !as_i32(item, base + rows_at + r * width + i)) { Py_CLEAR(out); break; }
+      if (PyLong_CheckExact(item)) Py_INCREF(item);
+      else item = PyLong_FromLong(base[rows_at + r * width + i]);
+      PyTuple_SET_ITEM(row, i, item);
+    }
+  }
+  Py_DECREF(zero);
+  return out;
 }
 
 // ---- set-up ---------------------------------------------------------------------------------------------------------
@@ -429,6 +614,9 @@ PyObject* init(PyObject*, PyObject* args) {
   get(lib.prefill_part, "nvj_paged_prefill_packed_part");
   get(lib.norm_rope, "nvj_qk_norm_rope_kv_append");
   get(lib.slot_mapping, "nvj_compute_slot_mapping");
+  get(lib.copy_blocks, "nvj_copy_blocks");
+  get(lib.snapshot, "nvj_hybrid_snapshot_host_slots");
+  get(lib.restore, "nvj_hybrid_restore_host_slots");
   if (missing) {
     PyErr_Format(PyExc_ImportError, "libnvj_b200.so does not export %s", missing);
     return nullptr;
@@ -482,6 +670,10 @@ PyMethodDef methods[] = {
     NVJ_FAST(append, "append of new K/V rows, or None"),
     NVJ_FAST(packed_prefill, "ragged packed attention, or None"),
     NVJ_FAST(norm_rope, "norm + rope + append, or None"),
+    NVJ_FAST(hash_chain, "chained digests of a token list's blocks, or None"),
+    NVJ_FAST(copy_blocks, "cache[:, dst] = cache[:, src], or None"),
+    NVJ_FAST(hybrid_copy, "snapshot or restore of GDN state rows, or None"),
+    NVJ_FAST(pack_i32, "fill a staging buffer with a batch's lists"),
     NVJ_FAST(slot_mapping, "flat cache slots of positions, or None"),
     {"init", init, METH_VARARGS, "resolve the library's entry points and keep the callbacks"},
     {"set_workspace", set_workspace, METH_VARARGS, "hand over a (device, stream)'s workspace"},

@@ -80,12 +80,11 @@ def host():
     return None, and launch nothing, when an operand needs a conversion or an error message of the Python route."""
     global _host_module
     if _host_module is None:
-        lib = _lib.load()
-        from .. import _nvj_host
+        lib, module = _lib.load(), _lib.host_module()
         with _host_lock:
             if _host_module is None:
-                _nvj_host.init(lib._handle, _lend_workspace, _lend_status_word, check, _strict_check)
-                _host_module = _nvj_host
+                module.init(lib._handle, _lend_workspace, _lend_status_word, check, _strict_check)
+                _host_module = module
     return _host_module
 
 
@@ -776,6 +775,8 @@ def qk_norm_rope_kv_append(query, k, v, q_norm_weight, k_norm_weight, positions,
 
 def copy_blocks(k_cache, v_cache, src_ids, dst_ids):
     """cache[:, dst] = cache[:, src] on the 5-D caches, in place (src and dst sets disjoint)."""
+    if host().copy_blocks(k_cache, v_cache, src_ids, dst_ids):
+        return k_cache, v_cache
     lib = _lib.load()
     if k_cache.ndim != 5 or k_cache.shape != v_cache.shape:
         raise ValueError("copy_blocks requires 5-D caches of equal shape")
@@ -808,6 +809,8 @@ def hybrid_copy(conv_table, rec_table, conv_pool, rec_pool, table_slots, pool_sl
     `table_slots` / `pool_slots`: int32 CUDA tensors, or plain Python sequences of at most `HYBRID_HOST_SLOTS`
     ints, which ride in the kernel's parameters (no index upload in front of the launch).
     """
+    if host().hybrid_copy(conv_table, rec_table, conv_pool, rec_pool, table_slots, pool_slots, restore):
+        return
     lib = _lib.load()
     for name, t in (("conv_table", conv_table), ("rec_table", rec_table), ("conv_pool", conv_pool), ("rec_pool", rec_pool)):
         if t is not None and not (t.is_cuda and t.is_contiguous()):
