@@ -8,16 +8,21 @@ the layouts `Scheduler.build_scheduled_batch`, `_build_packed_prefill_batch` and
 `seq_lens=num_tokens`; packed batches hold every query token in one row of
 `token_bucket` entries with `token_row_ids`, padded with (token 0, position 0,
 row 0); padded rows have an all-zero table, `seq_len 0` and `seq_id -1`.
-Host lists are built with NumPy and moved to the device in one copy each.
+Host lists are written into one pinned staging buffer by the host extension and moved to the device in one copy (one
+pinned array and one copy per field took 0.4 ms for a 34-row mixed batch).
 """
 
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass, replace
 from typing import List, Optional, Sequence as Seq
 
-import numpy as np
 import torch
+
+from .. import _lib
+
+_pack_i32 = _lib.host_module().pack_i32
 
 
 @dataclass
@@ -49,20 +54,31 @@ class ScheduledBatch:
         return torch.diff(self.query_start_loc).to(torch.int32)
 
 
-def _dev(a, device) -> torch.Tensor:
-    t = torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32))
-    if torch.device(device).type == "cuda":
-        t = t.pin_memory().to(device, non_blocking=True)
-    return t
+def _to_device(parts, tables, width, device):
+    """The batch's int32 arrays on the device, from one staging buffer and one copy: `parts` is a list of (list of ints,
+    shape), `tables` the rows' block tables (padding rows empty lists).  Returns (tensors of the parts, the [rows, width]
+    table, the table as a tuple of tuples)."""
+    for t in tables:
+        if len(t) > width:
+            raise ValueError(f"scheduled block table needs {len(t)} blocks but bucket has {width}")
+    cuda = torch.device(device).type == "cuda"
+    offsets, sizes, total = [], [], 0
+    shapes = [shape for _, shape in parts] + [(len(tables), width)]
+    for shape in shapes:  # every array starts on a 16-byte boundary
+        n = math.prod(shape)
+        offsets.append(total)
+        sizes.append(n)
+        total += -(-n // 4) * 4
+    stage = torch.empty(max(total, 1), dtype=torch.int32, pin_memory=cuda)
+    host_tables = _pack_i32(stage.data_ptr(), total, [(at, values) for at, (values, _) in zip(offsets, parts)], offsets[-1],
+                            tables, width)
+    dev = stage.to(device, non_blocking=True) if cuda else stage
+    arrays = [dev[at:at + n].view(shape) for at, n, shape in zip(offsets, sizes, shapes)]
+    return arrays[:-1], arrays[-1], host_tables
 
 
-def _table_rows(seqs, width: int, pad_rows: int) -> np.ndarray:
-    tab = np.zeros((len(seqs) + pad_rows, width), np.int32)
-    for r, s in enumerate(seqs):
-        if len(s.block_table) > width:
-            raise ValueError(f"scheduled block table needs {len(s.block_table)} blocks but bucket has {width}")
-        tab[r, :len(s.block_table)] = s.block_table
-    return tab
+def _table_lists(seqs, pad_rows: int):
+    return [s.block_table if type(s.block_table) is list else list(s.block_table) for s in seqs] + [[]] * pad_rows
 
 
 def build_decode_batch(seqs, *, max_blocks_per_seq: Optional[int] = None,
@@ -74,18 +90,17 @@ def build_decode_batch(seqs, *, max_blocks_per_seq: Optional[int] = None,
         raise ValueError(f"scheduled batch has {n} seqs but bucket has {bucket}")
     width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
     pad = bucket - n
-    tokens = np.array([[s.last_token] for s in seqs] + [[0]] * pad, np.int32)
-    positions = np.array([[s.num_tokens - 1] for s in seqs] + [[0]] * pad, np.int32)
-    seq_lens = np.array([s.num_tokens for s in seqs] + [0] * pad, np.int32)
-    qsl = np.concatenate([[0], np.cumsum([1] * n + [0] * pad)]).astype(np.int32)
-    seq_ids = tuple([s.seq_id for s in seqs] + [-1] * pad)
-    tab = _table_rows(seqs, width, pad)
+    zeros = [0] * pad
+    lens = [s.num_tokens for s in seqs] + zeros
+    seq_ids = [s.seq_id for s in seqs] + [-1] * pad
+    (tokens, positions, seq_lens, qsl, ids), tab, host_tables = _to_device(
+        [([s.last_token for s in seqs] + zeros, (bucket, 1)), ([s.num_tokens - 1 for s in seqs] + zeros, (bucket, 1)),
+         (lens, (bucket,)), (list(range(n + 1)) + [n] * pad, (bucket + 1,)), (seq_ids, (bucket,))],
+        _table_lists(seqs, pad), width, device)
     return ScheduledBatch(
-        tokens=_dev(tokens, device), positions=_dev(positions, device), seq_ids=_dev(seq_ids, device),
-        query_start_loc=_dev(qsl, device), is_prefill=False, num_prefill_tokens=0, num_decode_tokens=n,
-        block_tables=_dev(tab, device), seq_lens=_dev(seq_lens, device), seq_ids_host=seq_ids,
-        query_lens_host=tuple([1] * n + [0] * pad), seq_lens_host=tuple(int(x) for x in seq_lens),
-        block_tables_host=tuple(tuple(int(x) for x in row) for row in tab))
+        tokens=tokens, positions=positions, seq_ids=ids, query_start_loc=qsl, is_prefill=False, num_prefill_tokens=0,
+        num_decode_tokens=n, block_tables=tab, seq_lens=seq_lens, seq_ids_host=tuple(seq_ids),
+        query_lens_host=tuple([1] * n + zeros), seq_lens_host=tuple(lens), block_tables_host=host_tables)
 
 
 def _pack(rows_tokens, rows_positions, seqs, seq_lens, finals, *, width, bucket_rows, token_bucket,
@@ -98,25 +113,26 @@ def _pack(rows_tokens, rows_positions, seqs, seq_lens, finals, *, width, bucket_
     if actual > token_bucket:
         raise ValueError(f"scheduled prefill needs {actual} tokens but bucket has {token_bucket}")
     pad_rows = bucket_rows - len(seqs)
-    pad = token_bucket - actual
-    toks = np.zeros((1, token_bucket), np.int32)
-    pos = np.zeros((1, token_bucket), np.int32)
-    rid = np.zeros((1, token_bucket), np.int32)
-    toks[0, :actual] = np.concatenate([np.asarray(t, np.int32) for t in rows_tokens])
-    pos[0, :actual] = np.concatenate([np.asarray(p, np.int32) for p in rows_positions])
-    rid[0, :actual] = np.repeat(np.arange(len(seqs), dtype=np.int32), qlens)
-    qsl = np.concatenate([[0], np.cumsum(qlens + [0] * pad_rows)]).astype(np.int32)
-    lens = np.array(list(seq_lens) + [0] * pad_rows, np.int32)
-    seq_ids = tuple([s.seq_id for s in seqs] + [-1] * pad_rows)
-    tab = _table_rows(seqs, width, pad_rows)
+    if pad_rows < 0:
+        raise ValueError(f"scheduled batch has {len(seqs)} seqs but bucket has {bucket_rows}")
+    toks, pos, rid, qsl = [], [], [], [0]
+    for r, (t, p, n) in enumerate(zip(rows_tokens, rows_positions, qlens)):
+        toks.extend(t)
+        pos.extend(p)
+        rid.extend([r] * n)
+        qsl.append(qsl[-1] + n)
+    qsl.extend([actual] * pad_rows)
+    lens = list(seq_lens) + [0] * pad_rows
+    seq_ids = [s.seq_id for s in seqs] + [-1] * pad_rows
+    row = (1, token_bucket)  # (the staging buffer starts as zeros: token 0, position 0, row 0 behind the last real token)
+    (tokens, positions, ids, qsl_dev, lens_dev, rids), tab, host_tables = _to_device(
+        [(toks, row), (pos, row), (seq_ids, (bucket_rows,)), (qsl, (bucket_rows + 1,)), (lens, (bucket_rows,)), (rid, row)],
+        _table_lists(seqs, pad_rows), width, device)
     return ScheduledBatch(
-        tokens=_dev(toks, device), positions=_dev(pos, device), seq_ids=_dev(seq_ids, device),
-        query_start_loc=_dev(qsl, device), is_prefill=True, num_prefill_tokens=actual, num_decode_tokens=0,
-        block_tables=_dev(tab, device), seq_lens=_dev(lens, device), prefill_is_final=list(finals),
-        seq_ids_host=seq_ids, query_lens_host=tuple(qlens + [0] * pad_rows),
-        seq_lens_host=tuple(int(x) for x in lens),
-        block_tables_host=tuple(tuple(int(x) for x in row) for row in tab),
-        packed_prefill=True, token_row_ids=_dev(rid, device))
+        tokens=tokens, positions=positions, seq_ids=ids, query_start_loc=qsl_dev, is_prefill=True, num_prefill_tokens=actual,
+        num_decode_tokens=0, block_tables=tab, seq_lens=lens_dev, prefill_is_final=list(finals), seq_ids_host=tuple(seq_ids),
+        query_lens_host=tuple(qlens + [0] * pad_rows), seq_lens_host=tuple(lens), block_tables_host=host_tables,
+        packed_prefill=True, token_row_ids=rids)
 
 
 def build_packed_prefill_batch(seqs, prefill_chunk_lens: Optional[Seq[int]] = None, *,
@@ -130,7 +146,7 @@ def build_packed_prefill_batch(seqs, prefill_chunk_lens: Optional[Seq[int]] = No
         if chunk <= 0:
             raise ValueError(f"Scheduled sequence {s.seq_id} has no executable tokens")
         end = start + chunk
-        toks.append(s.token_ids[start:end]); poss.append(list(range(start, end)))
+        toks.append(s.token_ids[start:end]); poss.append(range(start, end))
         lens.append(end); finals.append(end >= s.num_tokens)
     width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
     return _pack(toks, poss, seqs, lens, finals, width=width,
@@ -159,7 +175,7 @@ def build_mixed_prefill_decode_batch(*, decode_seqs, prefill_seqs, prefill_chunk
         if chunk <= 0:
             raise ValueError(f"Scheduled sequence {s.seq_id} has no executable prefill tokens")
         end = start + chunk
-        toks.append(s.token_ids[start:end]); poss.append(list(range(start, end)))
+        toks.append(s.token_ids[start:end]); poss.append(range(start, end))
         lens.append(end); finals.append(end >= s.num_tokens)
     seqs = list(decode_seqs) + list(prefill_seqs)
     width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
