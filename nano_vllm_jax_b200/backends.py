@@ -175,6 +175,11 @@ class B200Backend:
             if metadata.token_row_ids is not None:
                 if metadata.positions is None:
                     raise ValueError("metadata.positions is required for packed prefill attention")
+                out = _k.host().packed_prefill(query, cache.k_cache, cache.v_cache, metadata.block_tables, metadata.seq_lens,
+                                               metadata.positions, metadata.query_start_loc, layer_id, block_size, scale,
+                                               num_key_value_groups, metadata.single_token_rows)
+                if out is not None:
+                    return out
                 return kvc.paged_attention_prefill_packed(
                     query, cache.k_cache, cache.v_cache, metadata.block_tables, metadata.seq_lens,
                     metadata.positions, metadata.token_row_ids, metadata.query_start_loc, block_size, scale,
@@ -189,6 +194,10 @@ class B200Backend:
                                                num_key_value_groups, layer_idx=layer_id, out_dtype=f32)
         if metadata.positions is None:
             raise ValueError("metadata.positions is required for decode attention")
+        out = _k.host().window_decode(query, cache.k_cache, cache.v_cache, metadata.block_tables, metadata.seq_lens,
+                                      metadata.positions, layer_id, block_size, scale, num_key_value_groups, metadata.max_kv_len)
+        if out is not None:
+            return out
         if metadata.positions.shape[0] != metadata.block_tables.shape[0]:
             raise ValueError("positions and block_tables batch dimensions must match")
         return kvc.paged_attention_decode(query, cache.k_cache, cache.v_cache, metadata.block_tables,

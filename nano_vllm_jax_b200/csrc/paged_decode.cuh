@@ -52,6 +52,9 @@ struct DecodeParams {
   // upper bound on the CTAs of the streaming kernels (0: one, or two, per SM): a caller that runs another kernel
   // beside the decode pass leaves that kernel's SMs free
   int cta_limit;
+  // cluster kernel: launched while the kernel in front of it in the stream, which it does not depend on, still runs (that
+  // kernel has let its dependents go); it ends only after that kernel has, so that the stream's order holds behind both
+  int beside;
   // which wide kernel serves rows of several query tokens: 0 = automatic (mma.sync tiles up to width 4, tcgen05 beyond),
   // 1 = mma.sync tiles, 2 = tcgen05
   int wide_form;

@@ -108,6 +108,10 @@ __device__ __forceinline__ void cl_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// A launch that runs beside the kernel in front of it ends after that kernel: one CTA holds the grid open.
+__device__ __forceinline__ void cl_end_beside(const DecodeParams& p) {
+  if (p.beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 // Address of this CTA's shared-memory location in CTA `rank` of the cluster, and loads from there.
 __device__ __forceinline__ uint32_t cl_map(const void* p, uint32_t rank) {
   uint32_t a;
@@ -179,7 +183,10 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
   int ids = unit_id(lane);
   const int len = decode_row_len(p, b);  // the same in every thread of the cluster
   const long long qi = decode_query_index(p, b);
-  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) return;  // not this pass's row (whole cluster)
+  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) {  // not this pass's row (the whole cluster leaves)
+    cl_end_beside(p);
+    return;
+  }
   // query heads in slot order (slot h of a lane holds head h ^ hperm), times scale * log2(e)
   const int rperm = lane >> 3, h_own = (lane >> 1) & 3;
   float2 q2[kG][4];
@@ -380,6 +387,7 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
   if (ctas == 1) {
     const float inv = L > 0.f ? 1.f / L : 0.f;
     reinterpret_cast<float4*>(dst)[threadIdx.x] = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    cl_end_beside(p);
     return;
   }
   __syncthreads();  // acc[0] is overwritten
@@ -388,6 +396,7 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
   cl_sync();
   cl_fold_cluster(&sm.acc[0][0][0], kD, sm.ML, ctas, rank, kClThreads, dst);
   cl_sync();  // nobody leaves while its shared memory is being read
+  cl_end_beside(p);
 }
 
 // ---- 16-bit caches: the products on tensor-core tiles -------------------------------------------------------------
@@ -476,7 +485,10 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   int ids = block_id(lane);
   const int len = decode_row_len(p, b);
   const long long qi = decode_query_index(p, b);
-  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) return;  // not this pass's row (whole cluster)
+  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) {  // not this pass's row (the whole cluster leaves)
+    cl_end_beside(p);
+    return;
+  }
   uint32_t qb[16][2];  // Q^T as the B operand: column g = head g & 3
   {
     const char* q = static_cast<const char*>(p.q) + ((qi * kHq + kvh * kG + (g & 3)) * kD) * 2;
@@ -652,7 +664,10 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
       sm.m.ML[h] = make_float2(M, L);
     }
   }
-  if (ctas == 1) return;
+  if (ctas == 1) {
+    cl_end_beside(p);
+    return;
+  }
   __syncthreads();  // acc[0] is overwritten
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
@@ -662,6 +677,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   cl_sync();
   cl_fold_cluster(&sm.m.acc[0][0][0], kCmPitch, sm.m.ML, ctas, rank, kCmThreads, dst);
   cl_sync();  // nobody leaves while its shared memory is being read
+  cl_end_beside(p);
 }
 
 template <class Kernel>
@@ -677,13 +693,15 @@ static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cluster;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = p.beside ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 

@@ -19,7 +19,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, float* split_area, size_t split_bytes, cudaStream_t stream);
+                         int skip_single, int split_p, float* split_area, size_t split_bytes, int decode_follows, cudaStream_t stream);
 bool prefill_umma2_usable(float scale, long long num_blocks);
 int launch_prefill_umma(const void* q, int q_dtype, const char* k_cache, const char* v_cache,
                         long long num_blocks, const int32_t* block_tables, int table_width,
@@ -60,7 +60,7 @@ static int check_packed(const PackedArgs& a, bool* tile_ok) {
 // Rows that carry a single query token (the decode rows of a mixed batch), by the streaming decode kernel on at most
 // `cta_limit` CTAs (0: one per SM).  `out` is zero where this pass writes nothing.  NVJ_ERR_WORKSPACE when the
 // caller lent no usable workspace.
-static int run_single_token_rows(const PackedArgs& a, int cta_limit, cudaStream_t s) {
+static int run_single_token_rows(const PackedArgs& a, int cta_limit, int beside, cudaStream_t s) {
   const int num_ctas = decode_num_ctas();
   DecodeParams d{};
   d.batch = a.rows;
@@ -89,6 +89,11 @@ static int run_single_token_rows(const PackedArgs& a, int cta_limit, cudaStream_
   d.cta_limit = cta_limit;
   // bf16 queries: the tensor-core streaming kernel (it declines without a tensor-map encoder); else the CUDA-core one
   int rc = NVJ_ERR_UNSUPPORTED;
+  if (beside) {
+    d.beside = 1;
+    return launch_decode_cluster(d, s);
+  }
+  if (a.q_dtype == NVJ_BF16 && cta_limit == 0 && decode_cluster_pays(a.rows, a.table_width)) return launch_decode_cluster(d, s);
   if (a.q_dtype == NVJ_BF16) {
     d.width = 1;
     rc = launch_decode_wide(d, s);
@@ -105,10 +110,18 @@ static bool pair_kernel_serves(const PackedArgs& a) {
   return (a.variant == 0 || a.variant == 4 || a.variant == 5) && prefill_umma2_usable(a.scale, a.num_blocks);
 }
 
+// Whether the decode rows of a mixed batch run on the cluster kernel beside the tiles, in one stream: the two write different
+// rows and neither fills the machine.  The tiles are launched first and let the clusters start at once (programmatic
+// dependent launch); a cluster CTA is small (64 KiB, 128 threads) and fits wherever no tile CTA sits.  Six layers of 32
+// decode rows of up to 2048 tokens and two chunks of 256: 24.3 + 24.3 us per layer one behind the other.
+static bool rows_run_beside_tiles(const PackedArgs& a) {
+  return pair_kernel_serves(a) && a.q_dtype == NVJ_BF16 && decode_cluster_pays(a.rows, a.table_width);
+}
+
 // The query tiles: tcgen05 tiles first (CTA pairs, then single CTAs); they decline when the driver has no tensor-map
 // encoder or the scale is not positive, and the mma.sync tiles take over.  With skip_single the rows of one query
 // token are left to the pass above (and, unless the pair kernel serves the call, `out` has been zeroed by the caller).
-static int run_tiles(const PackedArgs& a, int skip_single, cudaStream_t s) {
+static int run_tiles(const PackedArgs& a, int skip_single, int decode_follows, cudaStream_t s) {
   const char* kc = static_cast<const char*>(a.k_cache_layer);
   const char* vc = static_cast<const char*>(a.v_cache_layer);
   const int variant = a.variant;
@@ -130,7 +143,7 @@ static int run_tiles(const PackedArgs& a, int skip_single, cudaStream_t s) {
     }
     const int rc = launch_prefill_umma2(a.q, a.q_dtype, kc, vc, a.num_blocks, a.block_tables, a.table_width, a.kv_lens, a.positions,
                                         a.query_start_loc, a.rows, a.token_bucket, a.scale, a.out, a.status, skip_single,
-                                        variant == 5 ? 0 : 1, split_area, split_bytes, s);
+                                        variant == 5 ? 0 : 1, split_area, split_bytes, decode_follows, s);
     if (rc != NVJ_ERR_UNSUPPORTED || variant != 0) return rc;
   }
   if (variant == 0 || variant == 3) {
@@ -199,15 +212,20 @@ extern "C" int nvj_paged_prefill_packed(const void* q, int q_dtype, const void* 
   // Rows that carry a single query token go to the streaming decode kernel when the caller lends it a decode
   // workspace; everything else goes to the tile kernel.
   int skip_single = 0;
+  if (workspace && rows > 0 && rows_run_beside_tiles(a)) {
+    // tiles first, on a few SMs; the decode rows' clusters start at once and take the rest
+    const int rc2 = run_tiles(a, 1, 1, s);
+    return rc2 != NVJ_OK ? rc2 : run_single_token_rows(a, 0, 1, s);
+  }
   if (workspace && rows > 0) {
     if (!pair_kernel_serves(a) &&
         cudaMemsetAsync(out, 0, sizeof(float) * (size_t)token_bucket * kHq * kD, s) != cudaSuccess)
       return NVJ_ERR_LAUNCH;
-    const int rc1 = run_single_token_rows(a, 0, s);
+    const int rc1 = run_single_token_rows(a, 0, 0, s);
     if (rc1 == NVJ_OK) skip_single = 1;
     else if (rc1 != NVJ_ERR_WORKSPACE) return rc1;
   }
-  return run_tiles(a, skip_single, s);
+  return run_tiles(a, skip_single, 0, s);
 }
 
 extern "C" int nvj_paged_prefill_packed_part(const void* q, int q_dtype, const void* k_cache_layer,
@@ -230,7 +248,7 @@ extern "C" int nvj_paged_prefill_packed_part(const void* q, int q_dtype, const v
   if (rc != NVJ_OK || token_bucket == 0) return rc;
   if (!tile_ok || variant == 1) return NVJ_ERR_UNSUPPORTED;  // the generic kernel serves a batch in one piece
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (part == 1) return run_single_token_rows(a, cta_limit, s);
+  if (part == 1) return run_single_token_rows(a, cta_limit, 0, s);
   if (part == 2 && !pair_kernel_serves(a)) return NVJ_ERR_UNSUPPORTED;  // the other tile kernels want a zeroed output
-  return run_tiles(a, part == 2 ? 1 : 0, s);
+  return run_tiles(a, part == 2 ? 1 : 0, 0, s);
 }

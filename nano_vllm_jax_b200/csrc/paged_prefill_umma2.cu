@@ -84,6 +84,7 @@ struct Umma2Params {
   float* part_ml;
   int4* tile_info;  // per (CTA of the x grid, KV head): {first token, tokens, splits, 0}, written by split 0 for the merge launch
   int pair_slots;
+  int decode_follows;  // the decode pass of the batch is launched behind this kernel to run beside it
 };
 
 struct Umma2Smem {
@@ -461,32 +462,49 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
 }
 
 // Which (table row, 32-token tile) the CTA with cluster index `cluster` of `clusters` and rank `rank` serves: the
-// heaviest pairs (the last tokens of a row see the most keys) get the lowest cluster indices.  One thread runs this.
-// row < 0: no tile (`idle` then numbers the clusters beyond the last pair 0, 1, ...).  `total` (the batch's number
-// of pairs) is complete only when `need_total`.
+// heaviest pairs (the last tokens of a row see the most keys) get the lowest cluster indices.  One warp runs this, 32 rows
+// at a time (one thread walking the rows paid a trip to the L2 for each: 7 of 24 us on a batch of 32 decode rows and two
+// chunks).  row < 0: no tile (`idle` then numbers the clusters beyond the last pair 0, 1, ...).  `total` (the batch's
+// number of pairs) is complete only when `need_total`.
 struct U2Tile {
   int row, tok0, ntok, pair_last_tok, idle, total;
 };
-__device__ __forceinline__ U2Tile u2_find_tile(const Umma2Params& p, int cluster, int clusters, int rank, bool need_total) {
+__device__ __forceinline__ U2Tile u2_find_tile(const Umma2Params& p, int cluster, int clusters, int rank, bool need_total, int lane) {
   U2Tile t{-1, 0, 0, 0, -1, 0};
   int idx = clusters - 1 - cluster;
-  for (int r = 0; r < p.rows; ++r) {
-    const int lo = p.query_start_loc[r];
-    int hi = p.query_start_loc[r + 1];
-    hi = hi < p.token_bucket ? hi : p.token_bucket;
-    int pairs = hi > lo ? (hi - lo + 2 * kU2Tokens - 1) / (2 * kU2Tokens) : 0;
-    if (p.skip_single && p.query_start_loc[r + 1] - lo == 1) pairs = 0;
-    t.total += pairs;
-    if (t.row < 0 && idx < pairs) {
-      t.row = r;
-      t.tok0 = lo + (2 * idx + rank) * kU2Tokens;
-      t.ntok = hi - t.tok0 < kU2Tokens ? hi - t.tok0 : kU2Tokens;
-      if (t.ntok < 0) t.ntok = 0;
-      const int pair_end = lo + (2 * idx + 2) * kU2Tokens;
-      t.pair_last_tok = (pair_end < hi ? pair_end : hi) - 1;
-      if (!need_total) break;
+  for (int base = 0; base < p.rows && (need_total || t.row < 0); base += 32) {
+    const int r = base + lane;
+    int lo = 0, hi = 0, pairs = 0;
+    if (r < p.rows) {
+      lo = p.query_start_loc[r];
+      const int end = p.query_start_loc[r + 1];
+      hi = end < p.token_bucket ? end : p.token_bucket;
+      pairs = hi > lo ? (hi - lo + 2 * kU2Tokens - 1) / (2 * kU2Tokens) : 0;
+      if (p.skip_single && end - lo == 1) pairs = 0;
     }
-    if (t.row < 0) idx -= pairs;
+    int incl = pairs;  // pairs of this lane's row and the ones before it in the group
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += n;
+    }
+    const int group = __shfl_sync(0xffffffffu, incl, 31);
+    t.total += group;
+    if (t.row >= 0) continue;
+    const unsigned hit = __ballot_sync(0xffffffffu, idx >= incl - pairs && idx < incl);
+    if (hit == 0) {
+      idx -= group;
+      continue;
+    }
+    const int at = __ffs(hit) - 1;
+    const int row_lo = __shfl_sync(0xffffffffu, lo, at), row_hi = __shfl_sync(0xffffffffu, hi, at);
+    const int pair = idx - __shfl_sync(0xffffffffu, incl - pairs, at);
+    t.row = base + at;
+    t.tok0 = row_lo + (2 * pair + rank) * kU2Tokens;
+    t.ntok = row_hi - t.tok0 < kU2Tokens ? row_hi - t.tok0 : kU2Tokens;
+    if (t.ntok < 0) t.ntok = 0;
+    const int pair_end = row_lo + (2 * pair + 2) * kU2Tokens;
+    t.pair_last_tok = (pair_end < row_hi ? pair_end : row_hi) - 1;
   }
   if (t.row < 0) t.idle = idx;
   return t;
@@ -527,8 +545,9 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   const int rank = (int)cluster_ctarank();  // == blockIdx.x & 1
   NVJ_U2_PHASE(0);
   NVJ_U2_NOTE(7, 0ull);
-  // a merge launch follows a launch with splits: let its CTAs take their places now (they wait for this grid to finish)
-  if (gridDim.z > 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // a merge launch follows a launch with splits: let its CTAs take their places now (they wait for this grid to finish);
+  // the decode pass of a mixed batch follows as well, and runs on the SMs this grid leaves
+  if (gridDim.z > 1 || p.decode_follows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.z > 0) {  // the extra splits leave at once when no row's key range is long enough to be split
     int any = 0;
     for (int rr = threadIdx.x; rr < p.rows; rr += kU2Threads) any |= p.kv_lens[rr] > (kU2SplitFrom - 1) * kU2Keys ? 1 : 0;
@@ -536,10 +555,12 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   }
 
   // ---- which (table row, pair of 32-token tiles) this cluster serves; both CTAs compute the same
-  if (threadIdx.x == 0) {
-    const U2Tile t = u2_find_tile(p, blockIdx.x >> 1, gridDim.x >> 1, rank, gridDim.z > 1);
-    sm.row = t.row; sm.tok0 = t.tok0; sm.ntok = t.ntok; sm.pair_last_tok = t.pair_last_tok; sm.abort_flag = 0;
-    sm.total_pairs = t.total; sm.idle_index = t.idle;
+  if (warp == 0) {
+    const U2Tile t = u2_find_tile(p, blockIdx.x >> 1, gridDim.x >> 1, rank, gridDim.z > 1, lane);
+    if (lane == 0) {
+      sm.row = t.row; sm.tok0 = t.tok0; sm.ntok = t.ntok; sm.pair_last_tok = t.pair_last_tok; sm.abort_flag = 0;
+      sm.total_pairs = t.total; sm.idle_index = t.idle;
+    }
   }
   __syncthreads();
   const int row = sm.row, tok0 = sm.tok0, ntok = sm.ntok;
@@ -750,7 +771,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, float* split_area, size_t split_bytes, cudaStream_t stream) {
+                         int skip_single, int split_p, float* split_area, size_t split_bytes, int decode_follows, cudaStream_t stream) {
   static PerDeviceFlags opted_in;
   constexpr int kSmemBytes = (int)sizeof(Umma2Smem) + 1024;
   static_assert(kSmemBytes <= 232448, "tiles exceed the shared memory of one CTA");
@@ -767,6 +788,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
   // decode-row pass of a mixed batch does the same for its rows: no memset launch in front of a batch.
   Umma2Params p{};
   p.zero_fill = 1;
+  p.decode_follows = decode_follows;
   p.q = q; p.q_dtype = q_dtype;
   p.block_tables = block_tables; p.kv_lens = kv_lens; p.positions = positions; p.query_start_loc = query_start_loc;
   p.out = out; p.status = status; p.num_blocks = num_blocks; p.rows = rows; p.token_bucket = token_bucket;

@@ -263,7 +263,9 @@ class BlockManager:
         self.may_append_slots(seq, 1)
 
     def may_append_slots(self, seq, num_slots: int) -> None:
-        table = seq.block_table
+        table, n, bs = seq.block_table, len(seq), self.block_size
+        if n % bs and (n + max(0, int(num_slots) - 1) + bs - 1) // bs <= len(table):
+            return  # no block is complete and the table has room: nearly every row of nearly every step
         if self._blocks_for(len(seq)) > len(table):
             last = len(table) - 1
             self._record_completed_block_hash(seq, last)

@@ -15,7 +15,8 @@ pinned array and one copy per field took 0.4 ms for a 34-row mixed batch).
 from __future__ import annotations
 
 import math
-from dataclasses import dataclass, replace
+from dataclasses import dataclass
+from itertools import accumulate
 from typing import List, Optional, Sequence as Seq
 
 import torch
@@ -62,19 +63,18 @@ def _to_device(parts, tables, width, device):
         if len(t) > width:
             raise ValueError(f"scheduled block table needs {len(t)} blocks but bucket has {width}")
     cuda = torch.device(device).type == "cuda"
-    offsets, sizes, total = [], [], 0
-    shapes = [shape for _, shape in parts] + [(len(tables), width)]
-    for shape in shapes:  # every array starts on a 16-byte boundary
-        n = math.prod(shape)
-        offsets.append(total)
-        sizes.append(n)
-        total += -(-n // 4) * 4
+    sizes = [math.prod(shape) for _, shape in parts]
+    sizes.append(len(tables) * width)
+    entries, at = [], 0
+    for (values, _), n in zip(parts, sizes):
+        entries.append((at, values))
+        at += n
+    total = at + sizes[-1]
     stage = torch.empty(max(total, 1), dtype=torch.int32, pin_memory=cuda)
-    host_tables = _pack_i32(stage.data_ptr(), total, [(at, values) for at, (values, _) in zip(offsets, parts)], offsets[-1],
-                            tables, width)
+    host_tables = _pack_i32(stage.data_ptr(), total, entries, at, tables, width)
     dev = stage.to(device, non_blocking=True) if cuda else stage
-    arrays = [dev[at:at + n].view(shape) for at, n, shape in zip(offsets, sizes, shapes)]
-    return arrays[:-1], arrays[-1], host_tables
+    arrays = [t if len(shape) == 1 else t.view(shape) for t, (_, shape) in zip(dev[:total].split(sizes), parts)]
+    return arrays, dev[at:total].view(len(tables), width), host_tables
 
 
 def _table_lists(seqs, pad_rows: int):
@@ -103,10 +103,9 @@ def build_decode_batch(seqs, *, max_blocks_per_seq: Optional[int] = None,
         query_lens_host=tuple([1] * n + zeros), seq_lens_host=tuple(lens), block_tables_host=host_tables)
 
 
-def _pack(rows_tokens, rows_positions, seqs, seq_lens, finals, *, width, bucket_rows, token_bucket,
-          device) -> ScheduledBatch:
-    qlens = [len(t) for t in rows_tokens]
-    actual = sum(qlens)
+def _pack(toks, pos, qlens, seqs, lens, finals, *, width, bucket_rows, token_bucket, device, mixed=False) -> ScheduledBatch:
+    """A packed batch from its rows' tokens and positions, laid end to end (row r has qlens[r] of them)."""
+    actual = len(toks)
     if actual <= 0:
         raise ValueError("packed prefill requires at least one executable token")
     token_bucket = actual if token_bucket is None else token_bucket
@@ -115,14 +114,15 @@ def _pack(rows_tokens, rows_positions, seqs, seq_lens, finals, *, width, bucket_
     pad_rows = bucket_rows - len(seqs)
     if pad_rows < 0:
         raise ValueError(f"scheduled batch has {len(seqs)} seqs but bucket has {bucket_rows}")
-    toks, pos, rid, qsl = [], [], [], [0]
-    for r, (t, p, n) in enumerate(zip(rows_tokens, rows_positions, qlens)):
-        toks.extend(t)
-        pos.extend(p)
-        rid.extend([r] * n)
-        qsl.append(qsl[-1] + n)
+    rid = []
+    for r, n in enumerate(qlens):
+        if n == 1:
+            rid.append(r)
+        else:
+            rid.extend([r] * n)
+    qsl = [0, *accumulate(qlens)]
     qsl.extend([actual] * pad_rows)
-    lens = list(seq_lens) + [0] * pad_rows
+    lens = lens + [0] * pad_rows
     seq_ids = [s.seq_id for s in seqs] + [-1] * pad_rows
     row = (1, token_bucket)  # (the staging buffer starts as zeros: token 0, position 0, row 0 behind the last real token)
     (tokens, positions, ids, qsl_dev, lens_dev, rids), tab, host_tables = _to_device(
@@ -132,24 +132,31 @@ def _pack(rows_tokens, rows_positions, seqs, seq_lens, finals, *, width, bucket_
         tokens=tokens, positions=positions, seq_ids=ids, query_start_loc=qsl_dev, is_prefill=True, num_prefill_tokens=actual,
         num_decode_tokens=0, block_tables=tab, seq_lens=lens_dev, prefill_is_final=list(finals), seq_ids_host=tuple(seq_ids),
         query_lens_host=tuple(qlens + [0] * pad_rows), seq_lens_host=tuple(lens), block_tables_host=host_tables,
-        packed_prefill=True, token_row_ids=rids)
+        packed_prefill=True, token_row_ids=rids, mixed_prefill_decode=mixed)
+
+
+def _add_row(toks, pos, qlens, lens, finals, s, start, end) -> None:
+    tokens = s.token_ids[start:end]
+    toks.extend(tokens)
+    pos.extend(range(start, start + len(tokens)))
+    qlens.append(len(tokens))
+    lens.append(end)
+    finals.append(end >= s.num_tokens)
 
 
 def build_packed_prefill_batch(seqs, prefill_chunk_lens: Optional[Seq[int]] = None, *,
                                max_blocks_per_seq: Optional[int] = None, batch_size_bucket: Optional[int] = None,
                                token_bucket: Optional[int] = None, device="cuda") -> ScheduledBatch:
     """Packed prefill: each row runs tokens [num_cached_tokens, +chunk) (scheduler.py:774-789, 1034-1098)."""
-    toks, poss, lens, finals = [], [], [], []
+    toks, pos, qlens, lens, finals = [], [], [], [], []
     for i, s in enumerate(seqs):
         start = s.num_cached_tokens
         chunk = s.num_tokens - start if prefill_chunk_lens is None else int(prefill_chunk_lens[i])
         if chunk <= 0:
             raise ValueError(f"Scheduled sequence {s.seq_id} has no executable tokens")
-        end = start + chunk
-        toks.append(s.token_ids[start:end]); poss.append(range(start, end))
-        lens.append(end); finals.append(end >= s.num_tokens)
+        _add_row(toks, pos, qlens, lens, finals, s, start, start + chunk)
     width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
-    return _pack(toks, poss, seqs, lens, finals, width=width,
+    return _pack(toks, pos, qlens, seqs, lens, finals, width=width,
                  bucket_rows=len(seqs) if batch_size_bucket is None else batch_size_bucket,
                  token_bucket=token_bucket, device=device)
 
@@ -165,21 +172,18 @@ def build_mixed_prefill_decode_batch(*, decode_seqs, prefill_seqs, prefill_chunk
         raise ValueError("mixed prefill/decode batch requires at least one prefill row")
     if len(prefill_seqs) != len(prefill_chunk_lens):
         raise ValueError("prefill_chunk_lens length must match prefill_seqs")
-    toks = [[s.last_token] for s in decode_seqs]
-    poss = [[s.num_tokens - 1] for s in decode_seqs]
+    toks = [s.last_token for s in decode_seqs]
     lens = [s.num_tokens for s in decode_seqs]
-    finals = [True] * len(decode_seqs)
+    pos = [n - 1 for n in lens]
+    qlens, finals = [1] * len(lens), [True] * len(lens)
     for s, c in zip(prefill_seqs, prefill_chunk_lens):
         start = s.num_cached_tokens
         chunk = min(int(c), s.num_prompt_tokens - start)
         if chunk <= 0:
             raise ValueError(f"Scheduled sequence {s.seq_id} has no executable prefill tokens")
-        end = start + chunk
-        toks.append(s.token_ids[start:end]); poss.append(range(start, end))
-        lens.append(end); finals.append(end >= s.num_tokens)
+        _add_row(toks, pos, qlens, lens, finals, s, start, start + chunk)
     seqs = list(decode_seqs) + list(prefill_seqs)
     width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
-    batch = _pack(toks, poss, seqs, lens, finals, width=width,
-                  bucket_rows=len(seqs) if batch_size_bucket is None else batch_size_bucket,
-                  token_bucket=token_bucket, device=device)
-    return replace(batch, mixed_prefill_decode=True)
+    return _pack(toks, pos, qlens, seqs, lens, finals, width=width,
+                 bucket_rows=len(seqs) if batch_size_bucket is None else batch_size_bucket,
+                 token_bucket=token_bucket, device=device, mixed=True)
