@@ -212,7 +212,7 @@ class B200Backend:
                  and cache.k_cache.ndim == 5 and metadata.positions is not None)
         if fused:
             out = _k.host().fused_decode(query, k, v, cache.k_cache, cache.v_cache, metadata.block_tables, metadata.seq_lens,
-                                         metadata.positions, layer_id, block_size, scale, num_key_value_groups, 0)
+                                         metadata.positions, layer_id, block_size, scale, num_key_value_groups, 0, None, None)
             if out is not None:
                 return KVCacheStorage(cache.k_cache, cache.v_cache), out
             out, k_cache, v_cache = _k.paged_decode_attention_with_kv_append(

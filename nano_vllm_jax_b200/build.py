@@ -70,7 +70,7 @@ def build_host(force: bool = False) -> Path:
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            "-I", str(torch_dir / "include"), "-I", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"),
            "-I", str(cuda_include), "-I", sysconfig.get_paths()["include"], "-o", str(part), str(HOST_SRC),
-           "-L", str(torch_dir / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+           "-L", str(torch_dir / "lib"), "-L", str(cuda_include.parent / "lib64"), "-lcudart", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError("g++ failed on host_ops.cpp:\n" + proc.stdout + proc.stderr)

@@ -16,6 +16,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -41,6 +42,7 @@ struct Library {
   decltype(&nvj_qk_norm_rope_kv_append) norm_rope;
   decltype(&nvj_compute_slot_mapping) slot_mapping;
   decltype(&nvj_copy_blocks) copy_blocks;
+  decltype(&nvj_copy_many_async) copy_many;
   decltype(&nvj_hybrid_snapshot_host_slots) snapshot;
   decltype(&nvj_hybrid_restore_host_slots) restore;
 };
@@ -48,7 +50,7 @@ Library lib;
 PyObject* cb_workspace;  // (device index, rows): makes Python create the workspace and hand it over
 PyObject* cb_status;     // (device index): the same for the status word
 PyObject* cb_failed;     // (status, name): raises
-PyObject* cb_strict;     // (device index, name, check workspace, check status word): reads the device status back
+PyObject* cb_strict;     // (device index, stream, name, check workspace, check status word): reads the device status back
 
 struct Workspace {
   int device;
@@ -124,7 +126,7 @@ at::Tensor output(at::IntArrayRef sizes, int device) {
 }
 
 // After a call: a failure raises; NVJ_CHECK_STATUS=1 (tests) reads the device status back.  False: Python error set.
-bool finished(int rc, const char* what, int device, bool workspace, bool word) {
+bool finished(int rc, const char* what, int device, void* stream, bool workspace, bool word) {
   if (rc != NVJ_OK) {
     PyObject* r = PyObject_CallFunction(cb_failed, "is", rc, what);
     Py_XDECREF(r);
@@ -132,7 +134,7 @@ bool finished(int rc, const char* what, int device, bool workspace, bool word) {
     return false;
   }
   if (env_is("NVJ_CHECK_STATUS", "1")) {
-    PyObject* r = PyObject_CallFunction(cb_strict, "isii", device, what, workspace ? 1 : 0, word ? 1 : 0);
+    PyObject* r = PyObject_CallFunction(cb_strict, "iKsii", device, reinterpret_cast<unsigned long long>(stream), what, workspace ? 1 : 0, word ? 1 : 0);
     if (!r) return false;
     Py_DECREF(r);
   }
@@ -175,14 +177,16 @@ Layer cache_layer(const at::Tensor* k, const at::Tensor* v, long long layer) {
 // ---- the calls ----------------------------------------------------------------------------------------------------
 
 // fused_decode(query, new_k, new_v, k_cache, v_cache, block_tables, seq_lens, positions | None, layer, block_size, scale,
-//              groups, variant) -> out [B, 1, Hq * D] float32
+//              groups, variant, out | None, stream | None) -> out [B, 1, Hq * D] float32.  A given `out` may lie in pinned host
+// memory (the kernels only write it), which spares the caller a copy; a given stream must have its workspace already.
 PyObject* fused_decode(PyObject* const* a, Py_ssize_t n) {
-  if (!args_are(n, 13)) return nullptr;
+  if (!args_are(n, 15)) return nullptr;
   const at::Tensor *q = tensor(a[0]), *nk = tensor(a[1]), *nv = tensor(a[2]), *tab = tensor(a[5]), *len = tensor(a[6]);
   const at::Tensor* pos = a[7] == Py_None ? nullptr : tensor(a[7]);
   const long long layer = PyLong_AsLongLong(a[8]), bs = PyLong_AsLongLong(a[9]), groups = PyLong_AsLongLong(a[11]);
   const double scale = PyFloat_AsDouble(a[10]);
   const long long variant = PyLong_AsLongLong(a[12]);
+  void* given = a[14] == Py_None ? nullptr : reinterpret_cast<void*>(PyLong_AsUnsignedLongLong(a[14]));
   if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
   const Layer l = cache_layer(tensor(a[3]), tensor(a[4]), layer);
   if (!l.ok || !q || !nk || !nv || !tab || !len || (!pos && a[7] != Py_None)) NVJ_NONE();
@@ -196,17 +200,25 @@ PyObject* fused_decode(PyObject* const* a, Py_ssize_t n) {
       !nv->is_contiguous() || !meta(*tab, l.device) || !meta(*len, l.device) || tab->dim() != 2 || tab->size(0) != batch ||
       len->dim() != 1 || len->size(0) != batch || (pos && (!meta(*pos, l.device) || pos->numel() != batch)))
     NVJ_NONE();
-  void* stream = stream_of(l.device);
+  void* stream = given ? given : stream_of(l.device);
   const Workspace* ws = workspace_for(l.device, stream, batch);
   if (!ws) return nullptr;
-  at::Tensor out = output({batch, 1, hq * d}, l.device);
+  at::Tensor out;
+  if (a[13] == Py_None) {
+    out = output({batch, 1, hq * d}, l.device);
+  } else {
+    const at::Tensor* o = tensor(a[13]);
+    if (!o || o->scalar_type() != at::kFloat || !o->is_contiguous() || o->numel() != batch * hq * d || !(on(*o, l.device) || (o->is_cpu() && o->is_pinned()))) NVJ_NONE();
+    out = *o;
+    if (env_is("NVJ_POISON_OUTPUT", "1")) out.fill_(std::nan(""));
+  }
   void* wp = ws->buf.data_ptr();
   const size_t wb = (size_t)ws->buf.numel();
   int rc;
   NVJ_CALL(rc, lib.fused_append(q->data_ptr(), qdt, nk->data_ptr(), nv->data_ptr(), pos ? i32(*pos) : nullptr, l.k, l.v, l.dtype,
                                 l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab), (int)tab->size(1), i32(*len), (int)batch,
                                 (float)scale, static_cast<float*>(out.data_ptr()), wp, wb, (int)variant, stream));
-  if (!finished(rc, "nvj_paged_decode_fused_append", l.device, true, false)) return nullptr;
+  if (!finished(rc, "nvj_paged_decode_fused_append", l.device, stream, true, false)) return nullptr;
   return THPVariable_Wrap(std::move(out));
 }
 
@@ -245,8 +257,48 @@ PyObject* window_decode(PyObject* const* a, Py_ssize_t n) {
                           (int)tab->size(1), i32(*len), pos ? i32(*pos) : nullptr, (int)batch, (int)width, (int)max_len,
                           (float)scale, static_cast<float*>(out.data_ptr()), wp, wb, stream));
   if (rc == NVJ_ERR_UNSUPPORTED) NVJ_NONE();
-  if (!finished(rc, "nvj_paged_decode_window", l.device, true, false)) return nullptr;
+  if (!finished(rc, "nvj_paged_decode_window", l.device, stream, true, false)) return nullptr;
   return THPVariable_Wrap(std::move(out));
+}
+
+// stage_in(targets, sources, on_first, streams (3), events (2)) -> True: copies sources[i] -> targets[i], the first `on_first`
+// pairs on the first stream and the rest on the second, and makes the third stream wait for both.  None, and nothing issued,
+// when a source differs from its target in dtype or size or is not contiguous.
+PyObject* stage_in(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 5)) return nullptr;
+  const long long split = PyLong_AsLongLong(a[2]);
+  unsigned long long st[3], ev[2];
+  if (PyErr_Occurred() || !PyTuple_Check(a[0]) || !PyTuple_Check(a[1]) || !PyArg_ParseTuple(a[3], "KKK", &st[0], &st[1], &st[2]) ||
+      !PyArg_ParseTuple(a[4], "KK", &ev[0], &ev[1]))
+    return nullptr;
+  constexpr Py_ssize_t kMost = 16;
+  void* dst[kMost];
+  const void* src[kMost];
+  size_t bytes[kMost];
+  const Py_ssize_t pairs = PyTuple_GET_SIZE(a[0]);
+  if (pairs != PyTuple_GET_SIZE(a[1]) || pairs > kMost || split < 0 || split > pairs) NVJ_NONE();
+  for (Py_ssize_t i = 0; i < pairs; ++i) {
+    const at::Tensor *d = tensor(PyTuple_GET_ITEM(a[0], i)), *s = tensor(PyTuple_GET_ITEM(a[1], i));
+    if (!d || !s || d->dtype() != s->dtype() || d->numel() != s->numel() || !d->is_contiguous() || !s->is_contiguous()) NVJ_NONE();
+    dst[i] = d->data_ptr();
+    src[i] = s->data_ptr();
+    bytes[i] = d->nbytes();
+  }
+  auto stream = [&](int i) { return reinterpret_cast<cudaStream_t>(st[i]); };
+  auto event = [&](int i) { return reinterpret_cast<cudaEvent_t>(ev[i]); };
+  int rc;
+  cudaError_t e = cudaSuccess;
+  Py_BEGIN_ALLOW_THREADS
+  rc = lib.copy_many(dst, src, bytes, (int)split, stream(0));
+  if (rc == NVJ_OK) rc = lib.copy_many(dst + split, src + split, bytes + split, (int)(pairs - split), stream(1));
+  for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+    e = cudaEventRecord(event(i), stream(i));
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream(2), event(i), 0);
+  }
+  Py_END_ALLOW_THREADS
+  if (rc == NVJ_OK && e != cudaSuccess) rc = NVJ_ERR_LAUNCH;
+  if (rc != NVJ_OK && !finished(rc, "nvj_copy_many_async", 0, nullptr, false, false)) return nullptr;
+  Py_RETURN_TRUE;
 }
 
 // append(new_k, new_v, k_cache, v_cache, layer, slot_mapping | None, positions, block_tables, token_row_ids | None,
@@ -290,7 +342,7 @@ PyObject* append(PyObject* const* a, Py_ssize_t n) {
                                    (int)tab->size(1), l.block_size, i32(*qsl), (int)qsl->numel() - 1, packed ? 1 : 0, (int)rows, (int)cols,
                                    l.k, l.v, l.dtype, num_slots, l.hkv, l.d, st, stream));
   }
-  if (!finished(rc, what, l.device, false, true)) return nullptr;
+  if (!finished(rc, what, l.device, stream, false, true)) return nullptr;
   Py_RETURN_TRUE;
 }
 
@@ -342,7 +394,7 @@ PyObject* packed_prefill(PyObject* const* a, Py_ssize_t n) {
                              (int)tab->size(1), i32(*len), i32(*pos), i32(*qsl), (int)rows, (int)tokens, (float)scale,
                              static_cast<float*>(out.data_ptr()), st, wp, wb, variant, stream));
   }
-  if (!finished(rc, "nvj_paged_prefill_packed", l.device, ws != nullptr, true)) return nullptr;
+  if (!finished(rc, "nvj_paged_prefill_packed", l.device, stream, ws != nullptr, true)) return nullptr;
   return THPVariable_Wrap(std::move(out));
 }
 
@@ -388,7 +440,7 @@ PyObject* norm_rope(PyObject* const* a, Py_ssize_t n) {
                              (float)eps, inv ? static_cast<const float*>(inv->data_ptr()) : nullptr, (int)rotary, i32(*pos), 1, nullptr, i32(*slots),
                              nullptr, qsl ? i32(*qsl) : nullptr, qsl ? (int)qsl->numel() - 1 : 0, packed, (int)rows, (int)cols, kl->data_ptr(),
                              vl->data_ptr(), dtype_code(*kl), kl->numel() / (hkv * d), (int)hq, (int)hkv, (int)d, out.data_ptr(), st, stream));
-  if (!finished(rc, "nvj_qk_norm_rope_kv_append", dev, false, true)) return nullptr;
+  if (!finished(rc, "nvj_qk_norm_rope_kv_append", dev, stream, false, true)) return nullptr;
   return THPVariable_Wrap(std::move(out));
 }
 
@@ -404,7 +456,7 @@ PyObject* copy_blocks(PyObject* const* a, Py_ssize_t n) {
   if (!st) return nullptr;
   int rc;
   NVJ_CALL(rc, lib.copy_blocks(l.k, l.v, (int)k->size(0), l.blocks, block, l.blocks * block, i32(*src), i32(*dst), (int)src->numel(), st, stream));
-  if (!finished(rc, "nvj_copy_blocks", l.device, false, true)) return nullptr;
+  if (!finished(rc, "nvj_copy_blocks", l.device, stream, false, true)) return nullptr;
   Py_RETURN_TRUE;
 }
 
@@ -445,7 +497,7 @@ PyObject* hybrid_copy(PyObject* const* a, Py_ssize_t n) {
   int rc;
   if (restore) NVJ_CALL(rc, lib.restore(ptr(0), ptr(2), bytes[0], ptr(1), ptr(3), bytes[1], table_rows, pool_rows, slots[0], slots[1], (int)pairs, st, stream));
   else NVJ_CALL(rc, lib.snapshot(ptr(0), ptr(2), bytes[0], ptr(1), ptr(3), bytes[1], table_rows, pool_rows, slots[0], slots[1], (int)pairs, st, stream));
-  if (!finished(rc, restore ? "nvj_hybrid_restore" : "nvj_hybrid_snapshot", device, false, true)) return nullptr;
+  if (!finished(rc, restore ? "nvj_hybrid_restore" : "nvj_hybrid_snapshot", device, stream, false, true)) return nullptr;
   Py_RETURN_TRUE;
 }
 
@@ -464,7 +516,7 @@ PyObject* slot_mapping(PyObject* const* a, Py_ssize_t n) {
   int rc;
   NVJ_CALL(rc, lib.slot_mapping(i32(*pos), i32(*tab), rid ? i32(*rid) : nullptr, (int)pos->size(0), (int)pos->size(1), (int)tab->size(0),
                                 (int)tab->size(1), (int)bs, static_cast<int32_t*>(out.data_ptr()), stream));
-  if (!finished(rc, "nvj_compute_slot_mapping", dev, false, false)) return nullptr;
+  if (!finished(rc, "nvj_compute_slot_mapping", dev, stream, false, false)) return nullptr;
   return THPVariable_Wrap(std::move(out));
 }
 
@@ -614,6 +666,7 @@ PyObject* init(PyObject*, PyObject* args) {
   get(lib.prefill_part, "nvj_paged_prefill_packed_part");
   get(lib.norm_rope, "nvj_qk_norm_rope_kv_append");
   get(lib.slot_mapping, "nvj_compute_slot_mapping");
+  get(lib.copy_many, "nvj_copy_many_async");
   get(lib.copy_blocks, "nvj_copy_blocks");
   get(lib.snapshot, "nvj_hybrid_snapshot_host_slots");
   get(lib.restore, "nvj_hybrid_restore_host_slots");
@@ -671,6 +724,7 @@ PyMethodDef methods[] = {
     NVJ_FAST(packed_prefill, "ragged packed attention, or None"),
     NVJ_FAST(norm_rope, "norm + rope + append, or None"),
     NVJ_FAST(hash_chain, "chained digests of a token list's blocks, or None"),
+    NVJ_FAST(stage_in, "a step's operands to the device on two streams, or None"),
     NVJ_FAST(copy_blocks, "cache[:, dst] = cache[:, src], or None"),
     NVJ_FAST(hybrid_copy, "snapshot or restore of GDN state rows, or None"),
     NVJ_FAST(pack_i32, "fill a staging buffer with a batch's lists"),

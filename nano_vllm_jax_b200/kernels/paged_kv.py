@@ -97,17 +97,22 @@ def _lend_workspace(index, rows):
     _host_module.set_workspace(index, _stream(device), ws.buf, ws.max_batch)
 
 
+def lend_workspace(device, rows) -> None:
+    """Give the host module the current stream's workspace for `rows` rows (for calls that name their stream)."""
+    host()
+    _lend_workspace(device.index if device.index is not None else torch.cuda.current_device(), rows)
+
+
 def _lend_status_word(index):
     device = torch.device("cuda", index)
     _host_module.set_status_word(index, _stream(device), _status_word(device))
 
 
-def _strict_check(index, what, has_workspace, has_word):
-    device = torch.device("cuda", index)
+def _strict_check(index, stream, what, has_workspace, has_word):
     if has_word:
-        _check_word(_status_word(device), what)
+        _check_word(_status_words[index, stream], what)
     if has_workspace:
-        ws = _workspace(device, 0)
+        ws = _workspaces[index, stream]
         _check_word(ws.status_tensor(), what, ws)
 
 
@@ -531,7 +536,7 @@ def paged_decode_attention_with_kv_append(query, new_k, new_v, k_cache, v_cache,
     before this step's token (the token goes to position `seq_lens[b]`, `seq_lens[b] + 1` keys are attended) and is
     not written; `row_argmax(..., advance=...)` or the token gather's publish advances it at the end of the step."""
     out = host().fused_decode(query, new_k, new_v, k_cache, v_cache, block_table, seq_lens, positions, layer_id, block_size,
-                              scale, num_key_value_groups, variant)
+                              scale, num_key_value_groups, variant, None, None)
     if out is not None:
         return out, k_cache, v_cache
     if query.ndim != 4 or query.shape[1] != 1 or new_k.shape[1] != 1 or new_v.shape[1] != 1:

@@ -30,7 +30,7 @@ def test_fused_decode_takes_both_routes_alike(rows, dtype):
         tables, lens, pos = (to_torch(c[n]) for n in ("tables", "seq_lens", "positions"))
         if odd:
             args, lens, tables = [_strided(t) for t in args], lens.to(torch.int64), _strided(tables)
-            assert K.host().fused_decode(*args, cache.k_cache, cache.v_cache, tables, lens, pos, 0, BS, SCALE, 4, 0) is None
+            assert K.host().fused_decode(*args, cache.k_cache, cache.v_cache, tables, lens, pos, 0, BS, SCALE, 4, 0, None, None) is None
         be = B200Backend()
         md = be.build_attention_metadata(pos, tables, lens, BS, False)
         cache, out = be.write_kv_and_attention(0, *args, cache, md, BS, SCALE, 4, False)
