@@ -130,10 +130,11 @@ __device__ __forceinline__ float2 cl_ld2(uint32_t a) {
 }
 
 // The CTAs' sums [head][pitch] and (max, sum) pairs, at the same places in every CTA of the cluster, into the output: rank
-// r takes its 1 / ctas of the 256 float4 pieces of [4 heads][256 dims].
+// r takes its 1 / ctas of the float4 pieces of [heads][256 dims].
+template <int kHeads>
 __device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, const float2* ML, int ctas, uint32_t rank, int threads,
                                                 float* dst) {
-  const int per = kG * kD / 4 / ctas;
+  const int per = kHeads * kD / 4 / ctas;
   for (int i = threadIdx.x; i < per; i += threads) {
     const int piece = (int)rank * per + i, h = piece >> 6, d = (piece & 63) * 4;
     float2 e[kClMaxCluster];
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
   *reinterpret_cast<float4*>(&sm.acc[0][h][d4]) = o;
   if ((threadIdx.x & 63) == 0) sm.ML[h] = make_float2(M, L);
   cl_sync();
-  cl_fold_cluster(&sm.acc[0][0][0], kD, sm.ML, ctas, rank, kClThreads, dst);
+  cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, rank, kClThreads, dst);
   cl_sync();  // nobody leaves while its shared memory is being read
   cl_end_beside(p);
 }
@@ -420,7 +421,7 @@ struct CmSmem {
     struct {
       float acc[kCmWarps][2 * kG][kCmPitch];  // [warp][column][dim]; the CTA's merged sums end up in acc[0][0 .. 3]
       float2 ml[kCmWarps][kG];
-      float2 ML[kG];
+      float2 ML[kHq];
     } m;
   };
 };
@@ -464,15 +465,16 @@ __device__ __forceinline__ uint32_t cm_pack(float x, float y, bool rest) {
   }
 }
 
-template <typename T>
+template <typename T, bool kBoth>
 __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(DecodeParams p) {
   extern __shared__ __align__(128) unsigned char cl_smem_raw[];
   CmSmem& sm = *reinterpret_cast<CmSmem*>(cl_smem_raw);
   constexpr int kRowB = kD * 2, kTokB = kHkv * kRowB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int b = blockIdx.z, kvh = blockIdx.y, ctas = gridDim.x;
+  const int b = blockIdx.z, kvh = kBoth ? warp & 1 : blockIdx.y, ctas = gridDim.x;
   const uint32_t rank = ctas > 1 ? cl_rank() : 0u;
-  const int first = (int)rank * kCmWarps + warp, stride = ctas * kCmWarps;  // this warp's blocks: first, first + stride, ...
+  constexpr int kWalkers = kBoth ? kCmWarps / 2 : kCmWarps;  // warps of the CTA that share a KV head's blocks
+  const int first = (int)rank * kWalkers + (kBoth ? warp >> 1 : warp), stride = ctas * kWalkers;  // this warp's blocks: first, first + stride, ...
 
   // ---- first trip: the ids of this warp's first 32 blocks, the length, the query
   const long long tbase = decode_table_base(p, b);
@@ -638,21 +640,25 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     sm.m.acc[warp][2 * t + 1][n * 16 + g + 8] = o[n][3];
   }
   __syncthreads();
-  constexpr int kPieces = kG * kD / 4, kPer = kPieces / kCmThreads;  // float4 pieces of the output, and per thread
-  float* dst = p.out + (qi * kHq + kvh * kG) * kD;
+  constexpr int kHeads = kBoth ? kHq : kG;
+  constexpr int kPieces = kHeads * kD / 4, kPer = kPieces / kCmThreads;  // float4 pieces of the output, and per thread
+  float* dst = p.out + (qi * kHq + (kBoth ? 0 : kvh * kG)) * kD;
   float4 sum[kPer];
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
-    const int piece = k * kCmThreads + threadIdx.x, h = piece >> 6, d4 = (piece & 63) * 4;
+    const int piece = k * kCmThreads + threadIdx.x, head = piece >> 6, h = head & (kG - 1), d4 = (piece & 63) * 4;
+    constexpr int kStep = kCmWarps / kWalkers;
+    const int w0 = kBoth ? head / kG : 0;  // the first warp of this head
     float M = kNegBig, L = 0.f;
 #pragma unroll
-    for (int w = 0; w < kCmWarps; ++w) M = fmaxf(M, sm.m.ml[w][h].x);
+    for (int w = 0; w < kWalkers; ++w) M = fmaxf(M, sm.m.ml[w0 + w * kStep][h].x);
     sum[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int w = 0; w < kCmWarps; ++w) {
-      const float2 e = sm.m.ml[w][h];
+    for (int w = 0; w < kWalkers; ++w) {
+      const float2 e = sm.m.ml[w0 + w * kStep][h];
       const float f = ex2_approx(e.x - M);
-      const float4 x = *reinterpret_cast<const float4*>(&sm.m.acc[w][h][d4]), y = *reinterpret_cast<const float4*>(&sm.m.acc[w][h + kG][d4]);
+      const float4 x = *reinterpret_cast<const float4*>(&sm.m.acc[w0 + w * kStep][h][d4]);
+      const float4 y = *reinterpret_cast<const float4*>(&sm.m.acc[w0 + w * kStep][h + kG][d4]);
       L = fmaf(e.y, f, L);
       sum[k].x = fmaf(x.x + y.x, f, sum[k].x); sum[k].y = fmaf(x.y + y.y, f, sum[k].y);
       sum[k].z = fmaf(x.z + y.z, f, sum[k].z); sum[k].w = fmaf(x.w + y.w, f, sum[k].w);
@@ -661,7 +667,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
       const float inv = L > 0.f ? 1.f / L : 0.f;
       reinterpret_cast<float4*>(dst)[piece] = make_float4(sum[k].x * inv, sum[k].y * inv, sum[k].z * inv, sum[k].w * inv);
     } else if ((piece & 63) == 0) {
-      sm.m.ML[h] = make_float2(M, L);
+      sm.m.ML[head] = make_float2(M, L);
     }
   }
   if (ctas == 1) {
@@ -675,13 +681,13 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     *reinterpret_cast<float4*>(&sm.m.acc[0][piece >> 6][(piece & 63) * 4]) = sum[k];
   }
   cl_sync();
-  cl_fold_cluster(&sm.m.acc[0][0][0], kCmPitch, sm.m.ML, ctas, rank, kCmThreads, dst);
+  cl_fold_cluster<kHeads>(&sm.m.acc[0][0][0], kCmPitch, sm.m.ML, ctas, rank, kCmThreads, dst);
   cl_sync();  // nobody leaves while its shared memory is being read
   cl_end_beside(p);
 }
 
 template <class Kernel>
-static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const DecodeParams& p, int cluster, int threads, int smem,
+static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const DecodeParams& p, int cluster, int heads, int threads, int smem,
                            cudaStream_t stream) {
   if (!once_per_device(opted_in, [&](int) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
@@ -689,7 +695,7 @@ static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
       }))
     return NVJ_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cluster, kHkv, p.batch);
+  cfg.gridDim = dim3(cluster, heads, p.batch);
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -705,16 +711,18 @@ static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
   return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
-// CTAs per (row, KV head) for a batch whose longest row may have `blocks` blocks.  Doubled while the CTAs still fit the SMs
-// three at a time and every warp of the longest row finds a block; and, in batches of many CTAs, until no warp has more
-// than 12 blocks, so that the last CTAs to finish are short ones.  Clusters of 16 (no longer portable, and placed one by
-// one) only up to 2.2 CTAs per SM.  (Measured at 1 - 256 rows of 64 - 16384 tokens: within 3% of the best size of each.)
-static int cluster_size(int batch, int blocks, int sms) {
+// CTAs per row (of one KV head, or with `both` of both) for a batch whose longest row may have `blocks` blocks.  Doubled
+// while the CTAs still fit the SMs three at a time (2.7: clusters do not pack every SM) and every warp of the longest row
+// finds a block; and, in batches of many CTAs, until no warp has more than 12 blocks, so that the last CTAs to finish are
+// short ones.  Clusters of 16 (no longer portable, and placed one by one) only up to 2.2 CTAs per SM.  (Measured at 1 - 256
+// rows of 64 - 16384 tokens: within 3% of the best size of each.)
+static int cluster_size(int batch, int blocks, int sms, bool both) {
+  const int walkers = both ? kCmWarps / 2 : kCmWarps, most = both ? 8 : kClMaxCluster;
   int c = 1;
-  while (c < kClMaxCluster && 2 * c * kCmWarps <= blocks) {
-    const long long next = 2LL * c * kHkv * batch;
-    const bool fits = 10 * next <= (c < 8 ? 30LL : 22LL) * sms;
-    if (!fits && (c >= 8 || blocks <= 12 * c * kCmWarps)) break;
+  while (c < most && 2 * c * walkers <= blocks) {
+    const long long next = 2LL * c * (both ? 1 : kHkv) * batch;
+    const bool fits = 100 * next <= (c < 8 ? 275LL : 220LL) * sms;
+    if (!fits && (c >= 8 || blocks <= 12 * c * walkers)) break;
     c *= 2;
   }
   return c;
@@ -727,7 +735,7 @@ static int cluster_size(int batch, int blocks, int sms) {
 bool decode_cluster_pays(int batch, int table_width) {
   const int sms = decode_wide_num_ctas();
   if (sms <= 0) return false;
-  const int c = cluster_size(batch, table_width, sms);
+  const int c = cluster_size(batch, table_width, sms, false);
   const int per_warp = (table_width + c * kCmWarps - 1) / (c * kCmWarps);
   if ((long long)c * kHkv * batch >= sms) return per_warp <= 12;
   return 1.25 * per_warp <= 9.5 + 0.0026 * batch * table_width;  // 32 KiB per block, half of the widest on average, 6.3 TB/s
@@ -738,16 +746,24 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   const int sms = decode_wide_num_ctas();
   if (sms <= 0) return NVJ_ERR_LAUNCH;
   // (with a page list per row its width is not known here: as many CTAs as an ordinary row has use for)
-  const int cluster = cluster_size(p.batch, p.kv_indptr ? 64 : p.table_width, sms);
-  static PerDeviceFlags flags[4];
+  const int blocks = p.kv_indptr ? 64 : p.table_width;
+  const int cluster = cluster_size(p.batch, blocks, sms, false);
+  // Both KV heads in one CTA where clusters stay below eight CTAs: the two halves of a block's rows are then read at about
+  // the same time (48 rows of up to 2048 tokens 26.0 -> 24.4 us); with eight and more CTAs per head the finer split wins.
+  const bool both = cluster < 8;
+  const int pair = both ? cluster_size(p.batch, blocks, sms, true) : 0;
+  static PerDeviceFlags flags[6];
+  const int smem = (int)sizeof(CmSmem);
   if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16)
-    return launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16>, flags[0], p, cluster, kCmThreads, (int)sizeof(CmSmem), stream);
+    return both ? launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, true>, flags[0], p, pair, 1, kCmThreads, smem, stream)
+                : launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, false>, flags[1], p, cluster, kHkv, kCmThreads, smem, stream);
   if (p.kv_dtype == NVJ_F16 && p.q_dtype == NVJ_F16)
-    return launch_clusters(decode_cluster_mma_kernel<__half>, flags[1], p, cluster, kCmThreads, (int)sizeof(CmSmem), stream);
+    return both ? launch_clusters(decode_cluster_mma_kernel<__half, true>, flags[2], p, pair, 1, kCmThreads, smem, stream)
+                : launch_clusters(decode_cluster_mma_kernel<__half, false>, flags[3], p, cluster, kHkv, kCmThreads, smem, stream);
   if (p.kv_dtype == NVJ_F32)
-    return launch_clusters(decode_cluster_kernel<float>, flags[2], p, cluster, kClThreads, cluster_smem_bytes<float>(), stream);
+    return launch_clusters(decode_cluster_kernel<float>, flags[4], p, cluster, kHkv, kClThreads, cluster_smem_bytes<float>(), stream);
   if (p.kv_dtype == NVJ_F16)
-    return launch_clusters(decode_cluster_kernel<__half>, flags[3], p, cluster, kClThreads, cluster_smem_bytes<__half>(), stream);
+    return launch_clusters(decode_cluster_kernel<__half>, flags[5], p, cluster, kHkv, kClThreads, cluster_smem_bytes<__half>(), stream);
   return NVJ_ERR_UNSUPPORTED;  // bf16 cache with another query dtype: the streaming kernel on the CUDA cores
 }
 
