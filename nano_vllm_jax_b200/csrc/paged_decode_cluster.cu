@@ -711,21 +711,24 @@ static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
   return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
-// CTAs per row (of one KV head, or with `both` of both) for a batch whose longest row may have `blocks` blocks.  Doubled
-// while the CTAs still fit the SMs three at a time (2.7: clusters do not pack every SM) and every warp of the longest row
-// finds a block; and, in batches of many CTAs, until no warp has more than 12 blocks, so that the last CTAs to finish are
-// short ones.  Clusters of 16 (no longer portable, and placed one by one) only up to 2.2 CTAs per SM.  (Measured at 1 - 256
-// rows of 64 - 16384 tokens: within 3% of the best size of each.)
-static int cluster_size(int batch, int blocks, int sms, bool both) {
-  const int walkers = both ? kCmWarps / 2 : kCmWarps, most = both ? 8 : kClMaxCluster;
+// CTAs per cluster for `groups` clusters of rows of up to `blocks` blocks, when a CTA walks `walkers` blocks at a time.
+// Doubled while the CTAs fit the SMs (`per_sm` hundredths of a CTA per SM) and a walker of the longest row has more than one
+// block; and, in batches of many CTAs, until none has more than 12, so that the last CTAs to finish are short ones.
+// Clusters of 16 (no longer portable, and placed one by one) only up to 2.2 CTAs per SM.  (Measured at 1 - 256 rows of
+// 64 - 16384 tokens: within 3% of the best size of each.)
+static int cluster_size(long long groups, int blocks, int sms, int walkers, int per_sm, int most) {
   int c = 1;
-  while (c < most && 2 * c * walkers <= blocks) {
-    const long long next = 2LL * c * (both ? 1 : kHkv) * batch;
-    const bool fits = 100 * next <= (c < 8 ? 275LL : 220LL) * sms;
+  while (c < most && c * walkers < blocks) {
+    const bool fits = 100 * 2 * c * groups <= (long long)(c < 8 || per_sm < 220 ? per_sm : 220) * sms;
     if (!fits && (c >= 8 || blocks <= 12 * c * walkers)) break;
     c *= 2;
   }
   return c;
+}
+// CTAs of 64 KiB go three to an SM; 2.75, because clusters do not pack every SM.
+constexpr int kCmPerSm = 275;
+static int cluster_per_head(int batch, int blocks, int sms) {
+  return cluster_size(2LL * batch, blocks, sms, kCmWarps, kCmPerSm, kClMaxCluster);
 }
 
 // Whether this kernel, at its best cluster size, beats the streaming kernel (paged_decode_wide.cu) on a bf16 batch.  The
@@ -735,7 +738,7 @@ static int cluster_size(int batch, int blocks, int sms, bool both) {
 bool decode_cluster_pays(int batch, int table_width) {
   const int sms = decode_wide_num_ctas();
   if (sms <= 0) return false;
-  const int c = cluster_size(batch, table_width, sms, false);
+  const int c = cluster_per_head(batch, table_width, sms);
   const int per_warp = (table_width + c * kCmWarps - 1) / (c * kCmWarps);
   if ((long long)c * kHkv * batch >= sms) return per_warp <= 12;
   return 1.25 * per_warp <= 9.5 + 0.0026 * batch * table_width;  // 32 KiB per block, half of the widest on average, 6.3 TB/s
@@ -747,11 +750,14 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   if (sms <= 0) return NVJ_ERR_LAUNCH;
   // (with a page list per row its width is not known here: as many CTAs as an ordinary row has use for)
   const int blocks = p.kv_indptr ? 64 : p.table_width;
-  const int cluster = cluster_size(p.batch, blocks, sms, false);
-  // Both KV heads in one CTA where clusters stay below eight CTAs: the two halves of a block's rows are then read at about
-  // the same time (48 rows of up to 2048 tokens 26.0 -> 24.4 us); with eight and more CTAs per head the finer split wins.
-  const bool both = cluster < 8;
-  const int pair = both ? cluster_size(p.batch, blocks, sms, true) : 0;
+  const int cluster = cluster_per_head(p.batch, blocks, sms);
+  // Both KV heads in one CTA where that still leaves every SM a CTA and clusters are small: the two halves of a block's
+  // rows are then read at about the same time (48 rows of up to 2048 tokens 26.0 -> 24.4 us).  In smaller batches, and with
+  // eight and more CTAs per head, the finer split wins (4 rows of up to 512 tokens 7.3 against 5.9 us).
+  const bool both = cluster < 8 && (long long)cluster * kHkv * p.batch >= sms;
+  const int pair = both ? cluster_size(p.batch, blocks, sms, kCmWarps / 2, kCmPerSm, 8) : 0;
+  // the CUDA-core form: eight warps, a quarter block each, one CTA of 192 KiB per SM (f16: two)
+  const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, p.kv_dtype == NVJ_F32 ? 100 : 200, kClMaxCluster);
   static PerDeviceFlags flags[6];
   const int smem = (int)sizeof(CmSmem);
   if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16)
@@ -761,9 +767,9 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
     return both ? launch_clusters(decode_cluster_mma_kernel<__half, true>, flags[2], p, pair, 1, kCmThreads, smem, stream)
                 : launch_clusters(decode_cluster_mma_kernel<__half, false>, flags[3], p, cluster, kHkv, kCmThreads, smem, stream);
   if (p.kv_dtype == NVJ_F32)
-    return launch_clusters(decode_cluster_kernel<float>, flags[4], p, cluster, kHkv, kClThreads, cluster_smem_bytes<float>(), stream);
+    return launch_clusters(decode_cluster_kernel<float>, flags[4], p, wide, kHkv, kClThreads, cluster_smem_bytes<float>(), stream);
   if (p.kv_dtype == NVJ_F16)
-    return launch_clusters(decode_cluster_kernel<__half>, flags[5], p, cluster, kHkv, kClThreads, cluster_smem_bytes<__half>(), stream);
+    return launch_clusters(decode_cluster_kernel<__half>, flags[5], p, wide, kHkv, kClThreads, cluster_smem_bytes<__half>(), stream);
   return NVJ_ERR_UNSUPPORTED;  // bf16 cache with another query dtype: the streaming kernel on the CUDA cores
 }
 
