@@ -27,15 +27,15 @@ namespace nvj {
 constexpr int kClMaxCluster = 16;
 
 // ---- f32 caches (and f16 ones under f32 queries): fp32 products on the CUDA cores --------------------------------
-// Every warp keeps kClStages units of 4 keys in flight in a ring of its own in shared memory (16-byte cp.async); lane l
-// copies and later reads dims 8 l .. 8 l + 7 of every row, so the ring needs no barrier of any kind.  The 4 keys x 4 heads
+// Every warp keeps a unit of 4 keys in flight in shared memory of its own (16-byte cp.async; the next unit's K rows are
+// requested as soon as the scores are computed, its V rows after the weighted sum); lane l
+// copies and later reads dims 8 l .. 8 l + 7 of every row, so this needs no barrier of any kind.  The 4 keys x 4 heads
 // partial dot products are reduced by a select-free butterfly: lanes hold keys and heads in permuted order.
-constexpr int kClWarps = 8;
+constexpr int kClWarps = 8;  // two CTAs per SM: a warp's chain of shuffles is long, four warps per scheduler overlap theirs
 constexpr int kClThreads = kClWarps * 32;
 constexpr int kClUnit = 4;  // keys a warp takes at a time
-constexpr int kClStages = 3;
 
-// The ring [warp][stage][K | V][key][row], later the merge buffers.
+// The rows in flight [warp][K | V][key][row], later the merge buffers.
 struct ClusterMerge {
   alignas(16) float acc[kClWarps][kG][kD];  // per warp; the merged sums of the CTA end up in acc[0]
   float2 ml[kClWarps][kG];                  // per warp (max, sum)
@@ -43,7 +43,7 @@ struct ClusterMerge {
 };
 template <typename T>
 constexpr int cluster_smem_bytes() {
-  constexpr int ring = kClWarps * kClStages * 2 * kClUnit * kD * (int)sizeof(T);
+  constexpr int ring = kClWarps * 2 * kClUnit * kD * (int)sizeof(T);
   return ring > (int)sizeof(ClusterMerge) ? ring : (int)sizeof(ClusterMerge);
 }
 
@@ -164,7 +164,7 @@ __device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, con
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_cluster_kernel(DecodeParams p) {
+__global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodeParams p) {
   extern __shared__ __align__(128) unsigned char cl_smem_raw[];
   ClusterMerge& sm = *reinterpret_cast<ClusterMerge*>(cl_smem_raw);
   constexpr int kRowB = kD * (int)sizeof(T), kTokB = kHkv * kRowB;
@@ -259,15 +259,14 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
     const char* row = cache + (blk * kBlk + t % kBlk) * kTokB + kvh * kRowB;
     return t == new_key ? fresh : row;
   };
-  const uint32_t ring = smem_u32(cl_smem_raw) + warp * (kClStages * 2 * kClUnit * kRowB);
-  // all of a unit's rows into ring stage `stage`, as one group of copies
-  auto request = [&](int u, long long blk, int stage) {
-    const uint32_t at = ring + stage * (2 * kClUnit * kRowB);
+  const uint32_t k_at = smem_u32(cl_smem_raw) + warp * (2 * kClUnit * kRowB), v_at = k_at + kClUnit * kRowB;
+  // the unit's rows of one operand, as one group of copies (also an empty one: the waits count groups)
+  auto request = [&](uint32_t at, const char* cache, const char* fresh, int u, long long blk) {
+    if (u < units) {
 #pragma unroll
-    for (int r = 0; r < kClUnit; ++r) {
-      cl_copy_row<T>(at + r * kRowB, row_of(p.k_cache, new_k, u, blk, r), lane);
-      cl_copy_row<T>(at + (kClUnit + r) * kRowB, row_of(p.v_cache, new_v, u, blk, r), lane);
+      for (int r = 0; r < kClUnit; ++r) cl_copy_row<T>(at + r * kRowB, row_of(cache, fresh, u, blk, r), lane);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // The warp's i-th unit that lies in the pool, at or after unit u; a bad block id is flagged and its keys are left out.
   int u = first, i = 0;
@@ -280,23 +279,17 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
     }
     return 0;
   };
-  int pending[kClStages];  // units in flight, in order (units: none)
-#pragma unroll
-  for (int st = 0; st < kClStages; ++st) {
-    const long long blk = next_unit(u, i);
-    pending[st] = u;
-    if (u < units) { request(u, blk, st); u += stride; ++i; }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  for (int stage = 0; pending[0] < units; stage = stage + 1 == kClStages ? 0 : stage + 1) {
-    const int left = len - pending[0] * kClUnit;  // keys of the unit that are attended (at least one)
-    const uint32_t at = ring + stage * (2 * kClUnit * kRowB);
-    asm volatile("cp.async.wait_group %0;" ::"n"(kClStages - 1) : "memory");
+  long long blk = next_unit(u, i);
+  request(k_at, p.k_cache, new_k, u, blk);
+  request(v_at, p.v_cache, new_v, u, blk);
+  while (u < units) {
+    const int left = len - u * kClUnit;  // keys of the unit that are attended (at least one)
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // K has landed
     float s[16];
 #pragma unroll
     for (int r = 0; r < kClUnit; ++r) {  // key slot r of a lane holds key r ^ rperm of the unit
       float2 k2[4];
-      cl_unpack(cl_read_row<T>(at + (r ^ rperm) * kRowB, lane), k2);
+      cl_unpack(cl_read_row<T>(k_at + (r ^ rperm) * kRowB, lane), k2);
 #pragma unroll
       for (int h = 0; h < kG; ++h) {
         float2 a = fma2(q2[h][0], k2[0], make_float2(0.f, 0.f));
@@ -306,6 +299,10 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
         s[r * 4 + h] = a.x + a.y;
       }
     }
+    u += stride;
+    ++i;
+    blk = next_unit(u, i);
+    request(k_at, p.k_cache, new_k, u, blk);
 #pragma unroll
     for (int e = 0; e < 8; ++e) s[e] += __shfl_xor_sync(kFullMask, s[e + 8], 16);
 #pragma unroll
@@ -331,10 +328,11 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
     }
     const float pw = ex2_approx(sc - m_own);
     l_part += pw;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // V has landed
 #pragma unroll
     for (int r = 0; r < kClUnit; ++r) {
       float2 v2[4];
-      cl_unpack(cl_read_row<T>(at + (kClUnit + r) * kRowB, lane), v2);
+      cl_unpack(cl_read_row<T>(v_at + r * kRowB, lane), v2);
 #pragma unroll
       for (int h = 0; h < kG; ++h) {
         const float w = __shfl_sync(kFullMask, pw, r * 8 + h * 2);
@@ -343,13 +341,7 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
         for (int c = 0; c < 4; ++c) acc[h][c] = fma2(ww, v2[c], acc[h][c]);
       }
     }
-    // the stage is free (this lane alone reads what it copied): the next unit goes in
-#pragma unroll
-    for (int st = 0; st + 1 < kClStages; ++st) pending[st] = pending[st + 1];
-    const long long blk = next_unit(u, i);
-    pending[kClStages - 1] = u;
-    if (u < units) { request(u, blk, stage); u += stride; ++i; }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    request(v_at, p.v_cache, new_v, u, blk);  // (this lane alone reads what it copied)
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();  // the merge buffers lie over the rings
@@ -366,23 +358,19 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
     *reinterpret_cast<float4*>(&sm.acc[warp][h][lane * 8 + 4]) = make_float4(acc[h][2].x, acc[h][2].y, acc[h][3].x, acc[h][3].y);
   }
   __syncthreads();
-  float4 o;
-  float M, L;
-  const int h = threadIdx.x >> 6, d4 = (threadIdx.x & 63) * 4;  // thread = four dims of one head
-  {
-    M = kNegBig;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  float M = kNegBig, L = 0.f;
+  static_assert(kClThreads == kG * kD / 4, "a thread merges four dims of one head");
+  const int h = threadIdx.x / (kD / 4), d4 = (threadIdx.x % (kD / 4)) * 4;
 #pragma unroll
-    for (int w = 0; w < kClWarps; ++w) M = fmaxf(M, sm.ml[w][h].x);
-    L = 0.f;
-    o = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int w = 0; w < kClWarps; ++w) M = fmaxf(M, sm.ml[w][h].x);
 #pragma unroll
-    for (int w = 0; w < kClWarps; ++w) {
-      const float2 e = sm.ml[w][h];
-      const float f = ex2_approx(e.x - M);
-      const float4 x = *reinterpret_cast<const float4*>(&sm.acc[w][h][d4]);
-      L = fmaf(e.y, f, L);
-      o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
-    }
+  for (int w = 0; w < kClWarps; ++w) {
+    const float2 e = sm.ml[w][h];
+    const float f = ex2_approx(e.x - M);
+    const float4 x = *reinterpret_cast<const float4*>(&sm.acc[w][h][d4]);
+    L = fmaf(e.y, f, L);
+    o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
   }
   float* dst = p.out + (qi * kHq + kvh * kG) * kD;
   if (ctas == 1) {
@@ -393,7 +381,7 @@ __global__ void __launch_bounds__(kClThreads, sizeof(T) == 4 ? 1 : 2) decode_clu
   }
   __syncthreads();  // acc[0] is overwritten
   *reinterpret_cast<float4*>(&sm.acc[0][h][d4]) = o;
-  if ((threadIdx.x & 63) == 0) sm.ML[h] = make_float2(M, L);
+  if (d4 == 0) sm.ML[h] = make_float2(M, L);
   cl_sync();
   cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, rank, kClThreads, dst);
   cl_sync();  // nobody leaves while its shared memory is being read
@@ -756,8 +744,8 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   // eight and more CTAs per head, the finer split wins (4 rows of up to 512 tokens 7.3 against 5.9 us).
   const bool both = cluster < 8 && (long long)cluster * kHkv * p.batch >= sms;
   const int pair = both ? cluster_size(p.batch, blocks, sms, kCmWarps / 2, kCmPerSm, 8) : 0;
-  // the CUDA-core form: eight warps, a quarter block each, one CTA of 192 KiB per SM (f16: two)
-  const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, p.kv_dtype == NVJ_F32 ? 100 : 200, kClMaxCluster);
+  // the CUDA-core form: eight warps, a quarter block each, two CTAs per SM (1.8: clusters do not find every SM)
+  const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 8);
   static PerDeviceFlags flags[6];
   const int smem = (int)sizeof(CmSmem);
   if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16)
