@@ -30,7 +30,7 @@ __device__ __forceinline__ void copy_span16(const char* src, char* dst, long lon
 #pragma unroll
     for (int u = 0; u < kCopyUnroll; ++u) {
       const long long c = base + u * kCopyThreads + threadIdx.x;
-      if (c < chunks) v[u] = ld_nc_u4(src + (c << 4));
+      if (c < chunks) v[u] = ld_stream_u4(src + (c << 4));
     }
 #pragma unroll
     for (int u = 0; u < kCopyUnroll; ++u) {
@@ -206,6 +206,8 @@ copy_blocks_kernel(char* k_cache, char* v_cache, long long num_blocks, long long
 __global__ void __launch_bounds__(kArgmaxThreads)
 row_argmax_kernel(const float* x, int row_len, int32_t* tokens, int32_t* seq_lens, int32_t* positions, long long capacity,
                   int32_t* status) {
+  pdl_wait();
+  pdl_release();
   const int token = row_argmax_cta(x + (long long)blockIdx.x * row_len, row_len);
   if (threadIdx.x == 0) {
     tokens[blockIdx.x] = token;
@@ -405,7 +407,7 @@ extern "C" int nvj_row_argmax(const float* x, int rows, int row_len, int32_t* to
   if (rows < 0 || row_len <= 0) return NVJ_ERR_INVALID_ARGUMENT;
   if (rows == 0) return NVJ_OK;
   if (!x || !tokens) return NVJ_ERR_INVALID_ARGUMENT;
-  row_argmax_kernel<<<rows, kArgmaxThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, row_len, tokens, nullptr, nullptr, 0, nullptr);
+  launch_after(row_argmax_kernel, rows, kArgmaxThreads, 0, static_cast<cudaStream_t>(stream), x, row_len, tokens, nullptr, nullptr, 0, nullptr);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
@@ -416,7 +418,7 @@ extern "C" int nvj_row_argmax_advance(const float* x, int rows, int row_len, int
   if (rows < 0 || row_len <= 0 || table_width < 0 || block_size <= 0) return NVJ_ERR_INVALID_ARGUMENT;
   if (rows == 0) return NVJ_OK;
   if (!x || !tokens || !seq_lens) return NVJ_ERR_INVALID_ARGUMENT;
-  row_argmax_kernel<<<rows, kArgmaxThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, row_len, tokens, seq_lens, positions,
+  launch_after(row_argmax_kernel, rows, kArgmaxThreads, 0, static_cast<cudaStream_t>(stream), x, row_len, tokens, seq_lens, positions,
                                                                                    (long long)table_width * block_size, status);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }

@@ -13,6 +13,8 @@ namespace nvj {
 
 // Same-dtype rows, row bytes a multiple of 16: pure 16-byte copies.
 __global__ void __launch_bounds__(256) append_copy16_kernel(AppendParams p, int row_bytes) {
+  pdl_wait();
+  pdl_release();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= p.n_tokens) return;
@@ -26,8 +28,8 @@ __global__ void __launch_bounds__(256) append_copy16_kernel(AppendParams p, int 
   uint4* dk = reinterpret_cast<uint4*>(static_cast<char*>(p.k_cache) + slot * row_bytes);
   uint4* dv = reinterpret_cast<uint4*>(static_cast<char*>(p.v_cache) + slot * row_bytes);
   for (int c = lane; c < chunks; c += 32) {
-    const uint4 a = ld_nc_u4(sk + c);
-    const uint4 b = ld_nc_u4(sv + c);
+    const uint4 a = ld_stream_u4(sk + c);
+    const uint4 b = ld_stream_u4(sv + c);
     dk[c] = a;
     dv[c] = b;
   }
@@ -45,6 +47,8 @@ __device__ __forceinline__ uint32_t pack_f16(float a, float b) {
 // f32 source rows narrowed to a 16-bit cache dtype, 8 elements per lane step.
 template <bool kToBf16>
 __global__ void __launch_bounds__(256) append_narrow_kernel(AppendParams p) {
+  pdl_wait();
+  pdl_release();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= p.n_tokens) return;
@@ -86,6 +90,8 @@ __device__ __forceinline__ void store_from_float(void* base, long long idx, int 
 
 // Any shape, any dtype pair: one warp per token, element-wise.
 __global__ void __launch_bounds__(256) append_scalar_kernel(AppendParams p) {
+  pdl_wait();
+  pdl_release();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= p.n_tokens) return;
@@ -118,6 +124,8 @@ __global__ void __launch_bounds__(256)
 slot_mapping_kernel(const int32_t* positions, const int32_t* block_tables, const int32_t* token_row_ids,
                     int n_rows, int n_cols, int table_rows, int table_width, int block_size,
                     int32_t* slots) {
+  pdl_wait();
+  pdl_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rows * n_cols) return;
   slots[i] = mapped_slot(block_tables, token_row_ids ? token_row_ids[i] : i / n_cols, positions[i], table_rows, table_width,
@@ -133,12 +141,12 @@ static int launch_append(const AppendParams& p, cudaStream_t stream) {
   const int src_es = dtype_size(p.src_dtype), dst_es = dtype_size(p.dst_dtype);
   const bool ptrs_ok = aligned16(p.new_k) && aligned16(p.new_v) && aligned16(p.k_cache) && aligned16(p.v_cache);
   if (p.src_dtype == p.dst_dtype && ptrs_ok && (p.row_elems * src_es) % 16 == 0) {
-    append_copy16_kernel<<<blocks, threads, 0, stream>>>(p, p.row_elems * src_es);
+    launch_after(append_copy16_kernel, blocks, threads, 0, stream, p, p.row_elems * src_es);
   } else if (p.src_dtype == NVJ_F32 && dst_es == 2 && ptrs_ok && p.row_elems % 8 == 0) {
-    if (p.dst_dtype == NVJ_BF16) append_narrow_kernel<true><<<blocks, threads, 0, stream>>>(p);
-    else append_narrow_kernel<false><<<blocks, threads, 0, stream>>>(p);
+    if (p.dst_dtype == NVJ_BF16) launch_after(append_narrow_kernel<true>, blocks, threads, 0, stream, p);
+    else launch_after(append_narrow_kernel<false>, blocks, threads, 0, stream, p);
   } else {
-    append_scalar_kernel<<<blocks, threads, 0, stream>>>(p);
+    launch_after(append_scalar_kernel, blocks, threads, 0, stream, p);
   }
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
@@ -303,7 +311,7 @@ extern "C" int nvj_compute_slot_mapping(const int32_t* positions, const int32_t*
   if (n == 0) return NVJ_OK;
   if (n > 0x7fffffffLL) return NVJ_ERR_UNSUPPORTED;
   if (!positions || !block_tables || !slot_mapping) return NVJ_ERR_INVALID_ARGUMENT;
-  nvj::slot_mapping_kernel<<<(unsigned)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  nvj::launch_after(nvj::slot_mapping_kernel, (unsigned)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream),
       positions, block_tables, token_row_ids, n_rows, n_cols, table_rows, table_width, block_size,
       slot_mapping);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;

@@ -149,13 +149,39 @@ __device__ __forceinline__ float2 ld_cg_f32x2(const float* p) {
   return v;
 }
 
-// Streaming 16-byte load that does not allocate in L1 (read-once data).
-__device__ __forceinline__ uint4 ld_nc_u4(const void* p) {
+// Streaming 16-byte load that does not allocate in L1 (read-once data).  Not the non-coherent form: a kernel's CTAs may be
+// resident while the kernel in front still writes what they will read (pdl_wait below).
+__device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
+}
+
+// ---- programmatic dependent launch --------------------------------------------------------------------------
+// The kernels of a step follow one another on one stream, and an ordinary launch leaves ~2 us between two of them: the
+// next grid's CTAs are only placed once the last one of this grid has gone and its writes have been flushed.  A kernel
+// launched by launch_after() may be placed while the kernel in front of it is still running (if that one has called
+// pdl_release(), which ours do as soon as they have started): its pdl_wait(), before its first access to global memory,
+// holds it until everything in front has completed and is visible.  Since every such kernel waits before it ends, the
+// stream's order holds for whatever follows.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... Params, class... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
 // Once-per-device set-up on the host (a kernel attribute, a cached device property), safe when several host

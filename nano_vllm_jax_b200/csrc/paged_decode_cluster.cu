@@ -110,7 +110,7 @@ __device__ __forceinline__ void cl_sync() {
 }
 // A launch that runs beside the kernel in front of it ends after that kernel: one CTA holds the grid open.
 __device__ __forceinline__ void cl_end_beside(const DecodeParams& p) {
-  if (p.beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (p.beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
 }
 // Address of this CTA's shared-memory location in CTA `rank` of the cluster, and loads from there.
 __device__ __forceinline__ uint32_t cl_map(const void* p, uint32_t rank) {
@@ -173,6 +173,8 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   const uint32_t rank = ctas > 1 ? cl_rank() : 0u;
   const int first = (int)rank * kClWarps + warp, stride = ctas * kClWarps;  // this warp's units: first, first + stride, ...
 
+  if (!p.beside) pdl_wait();
+  pdl_release();
   // ---- first trip: the ids of this warp's first 32 units, the length, the query
   const long long tbase = decode_table_base(p, b);
   int pages = p.table_width;
@@ -464,6 +466,8 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   constexpr int kWalkers = kBoth ? kCmWarps / 2 : kCmWarps;  // warps of the CTA that share a KV head's blocks
   const int first = (int)rank * kWalkers + (kBoth ? warp >> 1 : warp), stride = ctas * kWalkers;  // this warp's blocks: first, first + stride, ...
 
+  if (!p.beside) pdl_wait();
+  pdl_release();
   // ---- first trip: the ids of this warp's first 32 blocks, the length, the query
   const long long tbase = decode_table_base(p, b);
   int pages = p.table_width;
@@ -695,7 +699,7 @@ static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = p.beside ? 2 : 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 

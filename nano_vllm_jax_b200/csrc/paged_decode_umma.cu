@@ -184,7 +184,7 @@ __device__ __forceinline__ void ud_stage_q(UdSmem& sm, const DecodeParams& p, ui
   for (int half = 0; half < 2; ++half) {
     uint4 u[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) u[i] = real ? ld_nc_u4(src + half * 16 + i) : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < 16; ++i) u[i] = real ? ld_stream_u4(src + half * 16 + i) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int part = 0; part < 4; ++part) {  // 32 dims = 16 columns at a time
       uint32_t w[16];
@@ -335,6 +335,8 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&v_map)) : "memory");
     sm.start_b = p.batch; sm.start_j = 0; sm.abort_flag = 0;
   }
+  pdl_wait();
+  pdl_release();
   // ---- pass 1: total number of blocks; zero the output of inactive rows
   int mine = 0;
   for (int base = 0; base < p.batch; base += kDecodeThreads) {
@@ -413,6 +415,8 @@ decode_umma_merge_kernel(DecodeParams p, int ranges) {
   __shared__ float red[384];
   __shared__ long long sums[2][kDecodeThreads / 32];
   const int b = blockIdx.x, tok = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_wait();
+  pdl_release();
   // blocks (real and phantom: the sequence the tile kernel cut into ranges) in front of row b and in all rows
   long long before = 0, all = 0;
   for (int r = tid; r < p.batch; r += kDecodeThreads) {
@@ -533,9 +537,9 @@ int launch_decode_umma(const DecodeParams& p, cudaStream_t stream) {
     return NVJ_ERR_LAUNCH;
   DecodeParams q = p;
   q.row_end_cost = kUdRowEndCost;
-  decode_umma_kernel<<<2 * ranges, kDecodeThreads, kSmemBytes, stream>>>(k_map, v_map, q);
+  launch_after(decode_umma_kernel, 2 * ranges, kDecodeThreads, kSmemBytes, stream, k_map, v_map, q);
   if (cudaGetLastError() != cudaSuccess) return NVJ_ERR_LAUNCH;
-  decode_umma_merge_kernel<<<dim3(p.batch, p.width), kDecodeThreads, 0, stream>>>(q, ranges);
+  launch_after(decode_umma_merge_kernel, dim3(p.batch, p.width), kDecodeThreads, 0, stream, q, ranges);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 

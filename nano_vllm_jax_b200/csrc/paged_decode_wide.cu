@@ -338,6 +338,8 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&k_map)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&v_map)) : "memory");
   }
+  pdl_wait();
+  pdl_release();
   if (!p.kv_indptr) {
     const long long lines = ((long long)p.batch * p.table_width * (long long)sizeof(int32_t) + 127) / 128;
     const long long line = (long long)blockIdx.x * kDecodeThreads + threadIdx.x;
@@ -637,8 +639,8 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
                cudaFuncSetAttribute(decode_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
       }))
     return NVJ_ERR_LAUNCH;
-  if (p.width > 4) decode_wide_kernel<true><<<n, kDecodeThreads, smem, stream>>>(k_map, v_map, q);
-  else decode_wide_kernel<false><<<n, kDecodeThreads, smem, stream>>>(k_map, v_map, q);
+  if (p.width > 4) launch_after(decode_wide_kernel<true>, n, kDecodeThreads, smem, stream, k_map, v_map, q);
+  else launch_after(decode_wide_kernel<false>, n, kDecodeThreads, smem, stream, k_map, v_map, q);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 

@@ -19,7 +19,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, float* split_area, size_t split_bytes, int decode_follows, cudaStream_t stream);
+                         int skip_single, int split_p, float* split_area, size_t split_bytes, cudaStream_t stream);
 bool prefill_umma2_usable(float scale, long long num_blocks);
 int launch_prefill_umma(const void* q, int q_dtype, const char* k_cache, const char* v_cache,
                         long long num_blocks, const int32_t* block_tables, int table_width,
@@ -121,7 +121,7 @@ static bool rows_run_beside_tiles(const PackedArgs& a) {
 // The query tiles: tcgen05 tiles first (CTA pairs, then single CTAs); they decline when the driver has no tensor-map
 // encoder or the scale is not positive, and the mma.sync tiles take over.  With skip_single the rows of one query
 // token are left to the pass above (and, unless the pair kernel serves the call, `out` has been zeroed by the caller).
-static int run_tiles(const PackedArgs& a, int skip_single, int decode_follows, cudaStream_t s) {
+static int run_tiles(const PackedArgs& a, int skip_single, cudaStream_t s) {
   const char* kc = static_cast<const char*>(a.k_cache_layer);
   const char* vc = static_cast<const char*>(a.v_cache_layer);
   const int variant = a.variant;
@@ -143,7 +143,7 @@ static int run_tiles(const PackedArgs& a, int skip_single, int decode_follows, c
     }
     const int rc = launch_prefill_umma2(a.q, a.q_dtype, kc, vc, a.num_blocks, a.block_tables, a.table_width, a.kv_lens, a.positions,
                                         a.query_start_loc, a.rows, a.token_bucket, a.scale, a.out, a.status, skip_single,
-                                        variant == 5 ? 0 : 1, split_area, split_bytes, decode_follows, s);
+                                        variant == 5 ? 0 : 1, split_area, split_bytes, s);
     if (rc != NVJ_ERR_UNSUPPORTED || variant != 0) return rc;
   }
   if (variant == 0 || variant == 3) {
@@ -214,7 +214,7 @@ extern "C" int nvj_paged_prefill_packed(const void* q, int q_dtype, const void* 
   int skip_single = 0;
   if (workspace && rows > 0 && rows_run_beside_tiles(a)) {
     // tiles first, on a few SMs; the decode rows' clusters start at once and take the rest
-    const int rc2 = run_tiles(a, 1, 1, s);
+    const int rc2 = run_tiles(a, 1, s);
     return rc2 != NVJ_OK ? rc2 : run_single_token_rows(a, 0, 1, s);
   }
   if (workspace && rows > 0) {
@@ -225,7 +225,7 @@ extern "C" int nvj_paged_prefill_packed(const void* q, int q_dtype, const void* 
     if (rc1 == NVJ_OK) skip_single = 1;
     else if (rc1 != NVJ_ERR_WORKSPACE) return rc1;
   }
-  return run_tiles(a, skip_single, 0, s);
+  return run_tiles(a, skip_single, s);
 }
 
 extern "C" int nvj_paged_prefill_packed_part(const void* q, int q_dtype, const void* k_cache_layer,
@@ -250,5 +250,5 @@ extern "C" int nvj_paged_prefill_packed_part(const void* q, int q_dtype, const v
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (part == 1) return run_single_token_rows(a, cta_limit, 0, s);
   if (part == 2 && !pair_kernel_serves(a)) return NVJ_ERR_UNSUPPORTED;  // the other tile kernels want a zeroed output
-  return run_tiles(a, part == 2 ? 1 : 0, 0, s);
+  return run_tiles(a, part == 2 ? 1 : 0, s);
 }

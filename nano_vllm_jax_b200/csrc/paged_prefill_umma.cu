@@ -211,7 +211,7 @@ __device__ __forceinline__ void um_softmax_warps(UmmaSmem& sm, const UmmaPrefill
         const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.q) + qrow + part * 32);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const uint4 u = ld_nc_u4(src + i);
+          const uint4 u = ld_stream_u4(src + i);
           w[4 * i] = u.x; w[4 * i + 1] = u.y; w[4 * i + 2] = u.z; w[4 * i + 3] = u.w;
         }
       } else {

@@ -84,7 +84,6 @@ struct Umma2Params {
   float* part_ml;
   int4* tile_info;  // per (CTA of the x grid, KV head): {first token, tokens, splits, 0}, written by split 0 for the merge launch
   int pair_slots;
-  int decode_follows;  // the decode pass of the batch is launched behind this kernel to run beside it
 };
 
 struct Umma2Smem {
@@ -338,7 +337,7 @@ __device__ __forceinline__ void u2_request_q(const Umma2Params& p, int tok0, int
     const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.q) +
                                                       ((long long)(tok0 + tk) * kHq + kvh * kG) * kD) + lane;
 #pragma unroll
-    for (int h = 0; h < 4; ++h) u[a][h] = tk < ntok ? ld_nc_u4(src + h * 32) : make_uint4(0u, 0u, 0u, 0u);
+    for (int h = 0; h < 4; ++h) u[a][h] = tk < ntok ? ld_stream_u4(src + h * 32) : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -545,9 +544,10 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   const int rank = (int)cluster_ctarank();  // == blockIdx.x & 1
   NVJ_U2_PHASE(0);
   NVJ_U2_NOTE(7, 0ull);
-  // a merge launch follows a launch with splits: let its CTAs take their places now (they wait for this grid to finish);
-  // the decode pass of a mixed batch follows as well, and runs on the SMs this grid leaves
-  if (gridDim.z > 1 || p.decode_follows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait();
+  // whatever follows may take its places now: the merge launch of a batch with splits (its CTAs wait for this grid to
+  // finish), the decode pass of a mixed batch (it runs beside, on the SMs this grid leaves)
+  pdl_release();
   if (blockIdx.z > 0) {  // the extra splits leave at once when no row's key range is long enough to be split
     int any = 0;
     for (int rr = threadIdx.x; rr < p.rows; rr += kU2Threads) any |= p.kv_lens[rr] > (kU2SplitFrom - 1) * kU2Keys ? 1 : 0;
@@ -667,7 +667,8 @@ prefill_umma2_merge_kernel(const Umma2Params p) {
   const int kvh = blockIdx.y, part = blockIdx.z;
   // launched with programmatic stream serialization: the CTAs may be resident before the tile kernel has finished, and
   // wait here until all of it has completed and its writes are visible
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
+  pdl_release();
   const int4 info = __ldcg(p.tile_info + blockIdx.x * kHkv + kvh);
   const int tok0 = info.x, ntok = info.y, splits = info.z;
   if (splits <= 1) return;
@@ -771,7 +772,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, float* split_area, size_t split_bytes, int decode_follows, cudaStream_t stream) {
+                         int skip_single, int split_p, float* split_area, size_t split_bytes, cudaStream_t stream) {
   static PerDeviceFlags opted_in;
   constexpr int kSmemBytes = (int)sizeof(Umma2Smem) + 1024;
   static_assert(kSmemBytes <= 232448, "tiles exceed the shared memory of one CTA");
@@ -788,7 +789,6 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
   // decode-row pass of a mixed batch does the same for its rows: no memset launch in front of a batch.
   Umma2Params p{};
   p.zero_fill = 1;
-  p.decode_follows = decode_follows;
   p.q = q; p.q_dtype = q_dtype;
   p.block_tables = block_tables; p.kv_lens = kv_lens; p.positions = positions; p.query_start_loc = query_start_loc;
   p.out = out; p.status = status; p.num_blocks = num_blocks; p.rows = rows; p.token_bucket = token_bucket;
@@ -818,19 +818,11 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
     p.pair_slots = slots;
   }
   dim3 grid(2 * pairs, kHkv, splits);
-  prefill_umma2_kernel<<<grid, kU2Threads, kSmemBytes, stream>>>(k_map, v_map, p);
+  launch_after(prefill_umma2_kernel, grid, kU2Threads, kSmemBytes, stream, k_map, v_map, p);
   if (cudaGetLastError() != cudaSuccess) return NVJ_ERR_LAUNCH;
   if (splits > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs, kHkv, kU2MergeParts);
-    cfg.blockDim = dim3(kU2MergeThreads, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, prefill_umma2_merge_kernel, p) != cudaSuccess) return NVJ_ERR_LAUNCH;
+    if (launch_after(prefill_umma2_merge_kernel, dim3(2 * pairs, kHkv, kU2MergeParts), kU2MergeThreads, 0, stream, p) != cudaSuccess)
+      return NVJ_ERR_LAUNCH;
   }
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }

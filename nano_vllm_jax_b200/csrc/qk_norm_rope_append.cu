@@ -42,6 +42,8 @@ struct NormRopeParams {
 
 template <int E>  // elements per lane = D / 32
 __global__ void __launch_bounds__(256) qk_norm_rope_append_kernel(NormRopeParams p) {
+  pdl_wait();
+  pdl_release();
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int heads = p.hq + 2 * p.hkv;
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_append_kernel(NormRopeParams
                                   : (is_k ? p.k + token * p.k_token_stride : p.v + token * p.v_token_stride) + (long long)kvh * p.d;
   __nv_bfloat16 raw[E];
   if (E == 8) {
-    *reinterpret_cast<uint4*>(raw) = ld_nc_u4(reinterpret_cast<const uint4*>(src) + lane);
+    *reinterpret_cast<uint4*>(raw) = ld_stream_u4(reinterpret_cast<const uint4*>(src) + lane);
   } else {
 #pragma unroll
     for (int j = 0; j < E; ++j) raw[j] = src[lane * E + j];
@@ -185,8 +187,8 @@ extern "C" int nvj_qk_norm_rope_kv_append(const void* q, int64_t q_token_stride,
   const long long warps = tokens * (num_q_heads + 2 * num_kv_heads);
   const unsigned blocks = (unsigned)((warps + 7) / 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (e == 8) qk_norm_rope_append_kernel<8><<<blocks, 256, 0, s>>>(p);
-  else if (e == 4) qk_norm_rope_append_kernel<4><<<blocks, 256, 0, s>>>(p);
-  else qk_norm_rope_append_kernel<2><<<blocks, 256, 0, s>>>(p);
+  if (e == 8) launch_after(qk_norm_rope_append_kernel<8>, blocks, 256, 0, s, p);
+  else if (e == 4) launch_after(qk_norm_rope_append_kernel<4>, blocks, 256, 0, s, p);
+  else launch_after(qk_norm_rope_append_kernel<2>, blocks, 256, 0, s, p);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
