@@ -15,7 +15,7 @@ prefix exists) followed by the token ids as native int64 bytes.
 
 from __future__ import annotations
 
-from collections import OrderedDict
+from collections import deque
 from typing import Dict, Iterable, List, Optional, Set
 
 import numpy as np
@@ -25,7 +25,8 @@ from .. import _lib
 from ..kv_cache import BlockTables
 
 NO_HASH = -1
-_hash_chain = _lib.host_module().hash_chain
+_host = _lib.host_module()
+_hash_chain = _host.hash_chain
 
 
 class Block:
@@ -50,40 +51,75 @@ class Block:
 
 
 class _FreeList:
-    """FIFO of free block ids with O(1) removal of an arbitrary id (deque.remove is O(n))."""
+    """FIFO of free block ids with O(1) removal of an arbitrary id.
+
+    A queue in order and a set of what is free.  Removing an id from the middle (a cached block is taken again: rare)
+    leaves its entry in the queue as a stale one, which the head skips when it gets there; an id's stale entries always
+    lie in front of its live one.  (An ordered dictionary popped one item at a time took four times as long.)
+    """
 
     def __init__(self, ids: Iterable[int]):
-        self._d: "OrderedDict[int, None]" = OrderedDict((i, None) for i in ids)
+        self._queue = deque(ids)
+        self._free = set(self._queue)
+        self._stale: Dict[int, int] = {}
 
     def __len__(self) -> int:
-        return len(self._d)
+        return len(self._free)
 
     def __contains__(self, block_id: int) -> bool:
-        return block_id in self._d
+        return block_id in self._free
 
     def __iter__(self):
-        return iter(self._d)
+        stale = dict(self._stale)
+        for block_id in self._queue:
+            if stale.get(block_id, 0) > 0:
+                stale[block_id] -= 1
+            else:
+                yield block_id
+
+    def _skip_stale(self) -> None:
+        queue, stale = self._queue, self._stale
+        while stale and queue:
+            n = stale.get(queue[0], 0)
+            if n == 0:
+                return
+            if n == 1:
+                del stale[queue[0]]
+            else:
+                stale[queue[0]] = n - 1
+            queue.popleft()
 
     def __getitem__(self, index: int) -> int:
         if index != 0:
             raise IndexError("only the head of the free list is addressable")
-        return next(iter(self._d))
+        if not self._free:
+            raise StopIteration("no free block left")
+        self._skip_stale()
+        return self._queue[0]
 
     def remove(self, block_id: int) -> None:
-        del self._d[block_id]
+        self._free.remove(block_id)
+        self._stale[block_id] = self._stale.get(block_id, 0) + 1
 
     def append(self, block_id: int) -> None:
-        self._d[block_id] = None
+        self.extend((block_id,))
 
     def extend(self, block_ids: Iterable[int]) -> None:
-        self._d.update(dict.fromkeys(block_ids))
+        fresh = [i for i in block_ids if i not in self._free]
+        self._queue.extend(fresh)
+        self._free.update(fresh)
 
     def take(self, n: int) -> List[int]:
         """Remove and return the first n ids; StopIteration, and nothing removed, when there are fewer."""
-        if n > len(self._d):
+        if n > len(self._free):
             raise StopIteration("no free block left")
-        pop = self._d.popitem
-        return [pop(last=False)[0] for _ in range(n)]
+        pop, out = self._queue.popleft, []
+        while self._stale and len(out) < n:
+            self._skip_stale()
+            out.append(pop())
+        out.extend([pop() for _ in range(n - len(out))])
+        self._free.difference_update(out)
+        return out
 
 
 class BlockManager:
@@ -172,19 +208,8 @@ class BlockManager:
 
     def _cached_run(self, seq, digests, cacheable_hashes):
         """(ids of the published blocks of the longest reusable prefix, its digest)."""
-        hits, best, best_hash, bs, tokens = [], 0, None, self.block_size, seq.token_ids
-        published, blocks = self.hash_to_block_id, self.blocks
-        for idx, h in enumerate(digests):
-            bid = published.get(h, -1)
-            if bid == -1:
-                break
-            blk = blocks[bid]
-            if blk.hash != h or blk.token_ids != tokens[idx * bs:(idx + 1) * bs]:
-                break
-            hits.append(bid)
-            if cacheable_hashes is None or h in cacheable_hashes:
-                best, best_hash = idx + 1, h
-        return hits[:best], best_hash
+        tokens = seq.token_ids if type(seq.token_ids) is list else list(seq.token_ids)
+        return _host.cached_run(tokens, digests, self.block_size, self.hash_to_block_id, self.blocks, cacheable_hashes)
 
     def _num_required_blocks(self, seq, *, use_prefix_cache=True, cacheable_hashes=None) -> int:
         need = self._num_blocks(seq)
@@ -216,30 +241,16 @@ class BlockManager:
                 self._take_cached(bid)
         table.extend(hits)
         seq.num_cached_tokens = len(hits) * bs
-        first, full = len(hits), len(digests)
+        first = len(hits)
         fresh = free.take(self._num_blocks(seq) - first)
-        published = self.hash_to_block_id
-        for idx, bid in enumerate(fresh, first):
-            blk = blocks[bid]
-            assert blk.ref_count == 0
-            if blk.hash != NO_HASH and published.get(blk.hash) == bid:
-                del published[blk.hash]  # its old content is about to be overwritten
-            blk.ref_count = 1
-            if idx < full:  # recorded, but published only after compute
-                blk.hash, blk.token_ids = digests[idx], tokens[idx * bs:(idx + 1) * bs]
-            else:
-                blk.hash, blk.token_ids = NO_HASH, []
+        _host.take_fresh(blocks, fresh, first, digests, tokens if type(tokens) is list else list(tokens), bs, self.hash_to_block_id,
+                         NO_HASH)
         used.update(fresh)
         table.extend(fresh)
         seq.cached_prefix_hash = cached_hash if seq.num_cached_tokens > 0 else None
 
     def deallocate(self, seq) -> None:
-        blocks, gone = self.blocks, []
-        for bid in reversed(seq.block_table):
-            blk = blocks[bid]
-            blk.ref_count -= 1
-            if blk.ref_count == 0:
-                gone.append(bid)
+        gone = _host.drop_owner(self.blocks, seq.block_table)
         self.used_block_ids.difference_update(gone)
         self.free_block_ids.extend(gone)
         seq.num_cached_tokens = 0
