@@ -73,7 +73,7 @@ class B200Backend:
     def __init__(self, config=None, device: str | torch.device = "cuda"):
         self.config = config
         self.device = torch.device(device)
-        self._decode_qsl: dict = {}  # (rows, device) -> arange(rows + 1) of a decode batch
+        self._decode_qsl: dict = {}  # (rows, device index) -> arange(rows + 1) of a decode batch
         for field in ("full_attention_kv_append_impl", "full_attention_decode_impl", "full_attention_prefill_impl"):
             if config is not None and getattr(config, field, None) not in (None, "", "reference", B200_IMPL):
                 normalize_full_attention_impl(getattr(config, field))
@@ -94,6 +94,22 @@ class B200Backend:
                                  token_row_ids=None, max_query_len=None, query_lens_host=None) -> AttentionMetadata:
         # `query_lens_host` (the scheduler's host-side query lengths, engine/scheduler.py `query_lens_host`) is an
         # optional extension: it tells a packed batch how many rows hold a single token without a device read
+        if not is_prefill and token_row_ids is None:
+            shape = _k.host().decode_shape(positions, block_tables, seq_lens)
+            if shape is not None:  # a decode batch whose shapes agree: nothing below could complain
+                batch, query_len, width = shape
+                if query_start_loc is None:
+                    query_start_loc = self._decode_qsl.get((batch, seq_lens.get_device()))
+                    if query_start_loc is None:
+                        query_start_loc = self._one_token_per_row(batch, seq_lens)
+                return kvc.attention_metadata(
+                    slot_mapping=kvc.SlotsFromTables(positions, block_tables, block_size), block_tables=block_tables,
+                    seq_lens=seq_lens, query_start_loc=query_start_loc,
+                    num_prefill_tokens=0 if num_prefill_tokens is None else num_prefill_tokens,
+                    num_decode_tokens=batch if num_decode_tokens is None else num_decode_tokens, positions=positions,
+                    max_kv_len=width * block_size, token_row_ids=None,
+                    max_query_len=query_len if max_query_len is None else max_query_len, single_token_rows=None,
+                    query_tile_pairs=None)
         if positions.ndim != 2:
             raise ValueError("positions must be a 2D tensor [batch, query_len]")
         if block_tables.ndim != 2:
@@ -130,13 +146,8 @@ class B200Backend:
             if is_prefill:
                 query_start_loc = torch.cat([torch.zeros(1, dtype=torch.int32, device=seq_lens.device),
                                              torch.cumsum(seq_lens.to(torch.int32), 0).to(torch.int32)])
-            else:  # one query token per row: a constant per batch size, built once
-                key = (int(seq_lens.shape[0]), seq_lens.device)
-                query_start_loc = self._decode_qsl.get(key)
-                if query_start_loc is None:
-                    query_start_loc = torch.arange(key[0] + 1, dtype=torch.int32, device=seq_lens.device)
-                    if not (seq_lens.is_cuda and torch.cuda.is_current_stream_capturing()):
-                        self._decode_qsl[key] = query_start_loc
+            else:
+                query_start_loc = self._one_token_per_row(int(seq_lens.shape[0]), seq_lens)
         return AttentionMetadata(
             slot_mapping=slot_mapping, block_tables=block_tables, seq_lens=seq_lens,
             query_start_loc=query_start_loc,
@@ -147,6 +158,16 @@ class B200Backend:
             token_row_ids=token_row_ids,
             max_query_len=max_query_len if max_query_len is not None else query_len,
             single_token_rows=singles, query_tile_pairs=pairs)
+
+    def _one_token_per_row(self, rows, seq_lens):
+        """query_start_loc of a batch with one query token per row: a constant per batch size and device, built once."""
+        key = (rows, seq_lens.get_device() if seq_lens.is_cuda else -1)
+        qsl = self._decode_qsl.get(key)
+        if qsl is None:
+            qsl = torch.arange(rows + 1, dtype=torch.int32, device=seq_lens.device)
+            if not (seq_lens.is_cuda and torch.cuda.is_current_stream_capturing()):
+                self._decode_qsl[key] = qsl
+        return qsl
 
     # ---- append (backends.py:980-1067)
     def write_kv(self, layer_id, k, v, cache: KVCacheStorage, metadata: AttentionMetadata) -> KVCacheStorage:
@@ -208,13 +229,14 @@ class B200Backend:
     # ---- fused boundary (backends.py:1252-1461)
     def write_kv_and_attention(self, layer_id, query, k, v, cache: KVCacheStorage, metadata: AttentionMetadata,
                                block_size, scale, num_key_value_groups, is_prefill):
-        fused = (not is_prefill and query.shape[1] == 1 and k.shape[1] == 1 and v.shape[1] == 1
-                 and cache.k_cache.ndim == 5 and metadata.positions is not None)
-        if fused:
+        if not is_prefill and metadata.positions is not None:  # one token per row on the 5-D cache; anything else comes back as None
             out = _k.host().fused_decode(query, k, v, cache.k_cache, cache.v_cache, metadata.block_tables, metadata.seq_lens,
                                          metadata.positions, layer_id, block_size, scale, num_key_value_groups, 0, None, None)
             if out is not None:
                 return KVCacheStorage(cache.k_cache, cache.v_cache), out
+        fused = (not is_prefill and query.shape[1] == 1 and k.shape[1] == 1 and v.shape[1] == 1
+                 and cache.k_cache.ndim == 5 and metadata.positions is not None)
+        if fused:
             out, k_cache, v_cache = _k.paged_decode_attention_with_kv_append(
                 query, k, v, cache.k_cache, cache.v_cache, metadata.block_tables.to(torch.int32),
                 metadata.seq_lens.to(torch.int32), metadata.positions, layer_id, block_size, scale,

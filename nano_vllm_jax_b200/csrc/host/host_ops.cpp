@@ -501,6 +501,16 @@ PyObject* hybrid_copy(PyObject* const* a, Py_ssize_t n) {
   Py_RETURN_TRUE;
 }
 
+// decode_shape(positions [B, T], block_tables [B, W], seq_lens [B]) -> (B, T, W), or None unless they are CUDA tensors that agree
+PyObject* decode_shape(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 3)) return nullptr;
+  const at::Tensor *pos = tensor(a[0]), *tab = tensor(a[1]), *len = tensor(a[2]);
+  if (!pos || !tab || !len || pos->dim() != 2 || tab->dim() != 2 || len->dim() != 1 || !pos->is_cuda() || !tab->is_cuda() || !len->is_cuda() ||
+      pos->size(0) != tab->size(0) || pos->size(0) != len->size(0))
+    NVJ_NONE();
+  return Py_BuildValue("LLL", (long long)pos->size(0), (long long)pos->size(1), (long long)tab->size(1));
+}
+
 // slot_mapping(positions [rows, cols], block_tables, block_size, token_row_ids | None) -> int32 [rows, cols]
 PyObject* slot_mapping(PyObject* const* a, Py_ssize_t n) {
   if (!args_are(n, 4)) return nullptr;
@@ -578,6 +588,134 @@ PyObject* hash_chain(PyObject* const* a, Py_ssize_t n) {
     PyList_SET_ITEM(out, (Py_ssize_t)b, d);
   }
   return out;
+}
+
+// ---- the block manager's walks ----------------------------------------------------------------------------------------
+
+PyObject *str_ref_count, *str_hash, *str_token_ids;  // attribute names of a block
+
+// cached_run(token_ids, digests, block_size, published {digest: block id}, blocks, cacheable digests | None) -> (ids of the
+// published blocks of the longest reusable prefix, its digest | None): a block counts when it holds exactly these tokens.
+PyObject* cached_run(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 6)) return nullptr;
+  const long long bs = PyLong_AsLongLong(a[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!PyList_Check(a[0]) || !PyList_Check(a[1]) || !PyDict_Check(a[3]) || !PyList_Check(a[4]) || bs < 1 ||
+      PyList_GET_SIZE(a[1]) > PyList_GET_SIZE(a[0]) / bs) {
+    PyErr_SetString(PyExc_TypeError, "cached_run: lists and a dict expected");
+    return nullptr;
+  }
+  PyObject* hits = PyList_New(0);
+  if (!hits) return nullptr;
+  Py_ssize_t best = 0;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[1]); ++i) {
+    PyObject* digest = PyList_GET_ITEM(a[1], i);
+    PyObject* id = PyDict_GetItemWithError(a[3], digest);  // borrowed
+    if (!id) {
+      if (PyErr_Occurred()) { Py_DECREF(hits); return nullptr; }
+      break;
+    }
+    const long long at = PyLong_AsLongLong(id);
+    if (at < 0 || at >= PyList_GET_SIZE(a[4])) {
+      if (!PyErr_Occurred()) PyErr_SetString(PyExc_IndexError, "published block outside the pool");
+      Py_DECREF(hits);
+      return nullptr;
+    }
+    PyObject* block = PyList_GET_ITEM(a[4], (Py_ssize_t)at);
+    PyObject *hash = PyObject_GetAttr(block, str_hash), *held = PyObject_GetAttr(block, str_token_ids);
+    int same = hash && held ? PyObject_RichCompareBool(hash, digest, Py_EQ) : -1;
+    if (same == 1) same = PyList_Check(held) && PyList_GET_SIZE(held) == bs ? 1 : 0;
+    for (long long k = 0; same == 1 && k < bs; ++k)
+      same = PyObject_RichCompareBool(PyList_GET_ITEM(held, (Py_ssize_t)k), PyList_GET_ITEM(a[0], (Py_ssize_t)(i * bs + k)), Py_EQ);
+    Py_XDECREF(hash);
+    Py_XDECREF(held);
+    if (same < 0 || (same == 1 && PyList_Append(hits, id) < 0)) { Py_DECREF(hits); return nullptr; }
+    if (!same) break;
+    const int usable = a[5] == Py_None ? 1 : PySequence_Contains(a[5], digest);
+    if (usable < 0) { Py_DECREF(hits); return nullptr; }
+    if (usable) best = i + 1;
+  }
+  if (PyList_SetSlice(hits, best, PyList_GET_SIZE(hits), nullptr) < 0) { Py_DECREF(hits); return nullptr; }
+  PyObject* out = PyTuple_Pack(2, hits, best ? PyList_GET_ITEM(a[1], best - 1) : Py_None);
+  Py_DECREF(hits);
+  return out;
+}
+
+// take_fresh(blocks, ids, first, digests, token_ids, block_size, published, no_hash): block ids[k] becomes block first + k of
+// a sequence: owned once, with its digest and tokens when it is a full block; what it published before is withdrawn.
+PyObject* take_fresh(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 8)) return nullptr;
+  const long long first = PyLong_AsLongLong(a[2]), bs = PyLong_AsLongLong(a[5]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!PyList_Check(a[0]) || !PyList_Check(a[1]) || !PyList_Check(a[3]) || !PyList_Check(a[4]) || !PyDict_Check(a[6])) {
+    PyErr_SetString(PyExc_TypeError, "take_fresh: lists and a dict expected");
+    return nullptr;
+  }
+  PyObject* one = PyLong_FromLong(1);
+  bool ok = one != nullptr;
+  for (Py_ssize_t k = 0; ok && k < PyList_GET_SIZE(a[1]); ++k) {
+    PyObject* id = PyList_GET_ITEM(a[1], k);
+    const long long at = PyLong_AsLongLong(id);
+    if (at < 0 || at >= PyList_GET_SIZE(a[0])) {
+      if (!PyErr_Occurred()) PyErr_SetString(PyExc_IndexError, "free block outside the pool");
+      ok = false;
+      break;
+    }
+    PyObject* block = PyList_GET_ITEM(a[0], (Py_ssize_t)at);
+    PyObject *owners = PyObject_GetAttr(block, str_ref_count), *old = PyObject_GetAttr(block, str_hash);
+    ok = owners && old;
+    if (ok && PyObject_IsTrue(owners) != 0) {
+      PyErr_SetString(PyExc_AssertionError, "a free block has an owner");
+      ok = false;
+    }
+    const int had = ok ? PyObject_RichCompareBool(old, a[7], Py_NE) : 0;
+    if (had == 1) {  // its old content is about to be overwritten
+      PyObject* holder = PyDict_GetItemWithError(a[6], old);
+      const int mine = holder ? PyObject_RichCompareBool(holder, id, Py_EQ) : 0;
+      if (mine == 1) ok = PyDict_DelItem(a[6], old) == 0;
+      else ok = mine == 0 && !PyErr_Occurred();
+    } else if (had < 0) {
+      ok = false;
+    }
+    Py_XDECREF(owners);
+    Py_XDECREF(old);
+    const long long index = first + k;
+    const bool full = index < PyList_GET_SIZE(a[3]);
+    PyObject* tokens = ok ? (full ? PyList_GetSlice(a[4], (Py_ssize_t)(index * bs), (Py_ssize_t)((index + 1) * bs)) : PyList_New(0)) : nullptr;
+    ok = ok && tokens && PyObject_SetAttr(block, str_ref_count, one) == 0 &&
+         PyObject_SetAttr(block, str_hash, full ? PyList_GET_ITEM(a[3], (Py_ssize_t)index) : a[7]) == 0 &&
+         PyObject_SetAttr(block, str_token_ids, tokens) == 0;
+    Py_XDECREF(tokens);
+  }
+  Py_XDECREF(one);
+  if (!ok) return nullptr;
+  Py_RETURN_NONE;
+}
+
+// drop_owner(blocks, table) -> ids that have no owner left, last block of the table first
+PyObject* drop_owner(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 2)) return nullptr;
+  if (!PyList_Check(a[0]) || !PyList_Check(a[1])) { PyErr_SetString(PyExc_TypeError, "drop_owner: lists expected"); return nullptr; }
+  PyObject* gone = PyList_New(0);
+  for (Py_ssize_t k = PyList_GET_SIZE(a[1]); gone && k-- > 0;) {
+    PyObject* id = PyList_GET_ITEM(a[1], k);
+    const long long at = PyLong_AsLongLong(id);
+    bool ok = at >= 0 && at < PyList_GET_SIZE(a[0]);
+    if (ok) {
+      PyObject* block = PyList_GET_ITEM(a[0], (Py_ssize_t)at);
+      PyObject* owners = PyObject_GetAttr(block, str_ref_count);
+      const long long left = owners ? PyLong_AsLongLong(owners) - 1 : 0;
+      PyObject* fewer = owners && !PyErr_Occurred() ? PyLong_FromLongLong(left) : nullptr;
+      ok = fewer && PyObject_SetAttr(block, str_ref_count, fewer) == 0 && (left != 0 || PyList_Append(gone, id) == 0);
+      Py_XDECREF(owners);
+      Py_XDECREF(fewer);
+    }
+    if (!ok) {
+      if (!PyErr_Occurred()) PyErr_SetString(PyExc_IndexError, "block outside the pool");
+      Py_CLEAR(gone);
+    }
+  }
+  return gone;
 }
 
 // ---- a batch's host arrays ------------------------------------------------------------------------------------------
@@ -723,6 +861,10 @@ PyMethodDef methods[] = {
     NVJ_FAST(append, "append of new K/V rows, or None"),
     NVJ_FAST(packed_prefill, "ragged packed attention, or None"),
     NVJ_FAST(norm_rope, "norm + rope + append, or None"),
+    NVJ_FAST(decode_shape, "batch, query length and table width of a decode batch, or None"),
+    NVJ_FAST(cached_run, "published blocks of a sequence's longest reusable prefix"),
+    NVJ_FAST(take_fresh, "free blocks become a sequence's"),
+    NVJ_FAST(drop_owner, "a sequence gives its blocks up"),
     NVJ_FAST(hash_chain, "chained digests of a token list's blocks, or None"),
     NVJ_FAST(stage_in, "a step's operands to the device on two streams, or None"),
     NVJ_FAST(copy_blocks, "cache[:, dst] = cache[:, src], or None"),
@@ -737,4 +879,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_nvj_host", "Host side of the hot 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__nvj_host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__nvj_host(void) {
+  str_ref_count = PyUnicode_InternFromString("ref_count");
+  str_hash = PyUnicode_InternFromString("hash");
+  str_token_ids = PyUnicode_InternFromString("token_ids");
+  return str_ref_count && str_hash && str_token_ids ? PyModule_Create(&module) : nullptr;
+}
