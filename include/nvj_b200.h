@@ -389,6 +389,24 @@ int nvj_paged_prefill_packed_part(const void* q, int q_dtype,
                                   void* workspace, size_t workspace_bytes, int variant,
                                   int part, int cta_limit, nvj_stream_t stream);
 
+/*
+ * A whole batch (part 0) or its part 2 or 3, launched for exactly the number of 64-token query tiles that the caller has
+ * counted on the host: tile_pairs = sum of ceil(len / 64) over the rows that the tiles serve (part 0 with a workspace and
+ * part 2: rows of several query tokens; part 3: all rows); -1 = not counted.  A batch with more tiles than that is flagged
+ * NVJ_DEV_BAD_LENGTH and the tiles too many are left out.  No counterpart in the reference.
+ */
+int nvj_paged_prefill_packed_counted(const void* q, int q_dtype,
+                                     const void* k_cache_layer, const void* v_cache_layer, int kv_dtype,
+                                     int64_t num_blocks, int block_size, int num_kv_heads,
+                                     int head_dim, int num_q_heads,
+                                     const int32_t* block_tables, int table_width,
+                                     const int32_t* kv_lens, const int32_t* positions,
+                                     const int32_t* query_start_loc, int rows,
+                                     int token_bucket, float scale,
+                                     float* out, int32_t* status,
+                                     void* workspace, size_t workspace_bytes, int variant,
+                                     int part, int tile_pairs, nvj_stream_t stream);
+
 /* ------------------------------------------------------------------ copies */
 
 /*

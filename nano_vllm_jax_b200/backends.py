@@ -198,7 +198,7 @@ class B200Backend:
                     raise ValueError("metadata.positions is required for packed prefill attention")
                 out = _k.host().packed_prefill(query, cache.k_cache, cache.v_cache, metadata.block_tables, metadata.seq_lens,
                                                metadata.positions, metadata.query_start_loc, layer_id, block_size, scale,
-                                               num_key_value_groups, metadata.single_token_rows)
+                                               num_key_value_groups, metadata.single_token_rows, metadata.query_tile_pairs)
                 if out is not None:
                     return out
                 return kvc.paged_attention_prefill_packed(

@@ -37,8 +37,7 @@ struct Library {
   decltype(&nvj_paged_decode_window) window;
   decltype(&nvj_kv_append) append;
   decltype(&nvj_kv_append_mapped) append_mapped;
-  decltype(&nvj_paged_prefill_packed) prefill;
-  decltype(&nvj_paged_prefill_packed_part) prefill_part;
+  decltype(&nvj_paged_prefill_packed_counted) prefill;
   decltype(&nvj_qk_norm_rope_kv_append) norm_rope;
   decltype(&nvj_compute_slot_mapping) slot_mapping;
   decltype(&nvj_copy_blocks) copy_blocks;
@@ -347,13 +346,14 @@ PyObject* append(PyObject* const* a, Py_ssize_t n) {
 }
 
 // packed_prefill(query [1, T, Hq, D], k_cache, v_cache, block_tables, kv_lens, positions, query_start_loc, layer, block_size,
-//                scale, groups, decode_rows | None) -> out [1, T, Hq * D] float32
+//                scale, groups, decode_rows | None, tile_pairs | None) -> out [1, T, Hq * D] float32
 PyObject* packed_prefill(PyObject* const* a, Py_ssize_t n) {
-  if (!args_are(n, 12)) return nullptr;
+  if (!args_are(n, 13)) return nullptr;
   const at::Tensor *q = tensor(a[0]), *tab = tensor(a[3]), *len = tensor(a[4]), *pos = tensor(a[5]), *qsl = tensor(a[6]);
   const long long layer = PyLong_AsLongLong(a[7]), bs = PyLong_AsLongLong(a[8]), groups = PyLong_AsLongLong(a[10]);
   const double scale = PyFloat_AsDouble(a[9]);
   const long long decode_rows = a[11] == Py_None ? -1 : PyLong_AsLongLong(a[11]);
+  const long long pairs = a[12] == Py_None ? -1 : PyLong_AsLongLong(a[12]);
   if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
   const Layer l = cache_layer(tensor(a[1]), tensor(a[2]), layer);
   if (!l.ok || !q || !tab || !len || !pos || !qsl || q->dim() != 4 || q->size(0) != 1) NVJ_NONE();
@@ -385,15 +385,11 @@ PyObject* packed_prefill(PyObject* const* a, Py_ssize_t n) {
   const size_t wb = ws ? (size_t)ws->buf.numel() : 0;
   at::Tensor out = output({1, tokens, hq * d}, l.device);
   int rc;
-  if (tiles_only) {
-    NVJ_CALL(rc, lib.prefill_part(q->data_ptr(), qdt, l.k, l.v, l.dtype, l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab),
-                                  (int)tab->size(1), i32(*len), i32(*pos), i32(*qsl), (int)rows, (int)tokens, (float)scale,
-                                  static_cast<float*>(out.data_ptr()), st, wp, wb, variant, 3, 0, stream));
-  } else {
-    NVJ_CALL(rc, lib.prefill(q->data_ptr(), qdt, l.k, l.v, l.dtype, l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab),
-                             (int)tab->size(1), i32(*len), i32(*pos), i32(*qsl), (int)rows, (int)tokens, (float)scale,
-                             static_cast<float*>(out.data_ptr()), st, wp, wb, variant, stream));
-  }
+  // (the count is of rows of several tokens: it holds when a row of one is served by the decode kernel, or there is none)
+  const long long counted = decode_rows >= 0 && pairs >= 0 ? pairs : -1;
+  NVJ_CALL(rc, lib.prefill(q->data_ptr(), qdt, l.k, l.v, l.dtype, l.blocks, l.block_size, l.hkv, l.d, (int)hq, i32(*tab), (int)tab->size(1),
+                           i32(*len), i32(*pos), i32(*qsl), (int)rows, (int)tokens, (float)scale, static_cast<float*>(out.data_ptr()), st, wp,
+                           wb, variant, tiles_only ? 3 : 0, (int)counted, stream));
   if (!finished(rc, "nvj_paged_prefill_packed", l.device, stream, ws != nullptr, true)) return nullptr;
   return THPVariable_Wrap(std::move(out));
 }
@@ -800,8 +796,7 @@ PyObject* init(PyObject*, PyObject* args) {
   get(lib.window, "nvj_paged_decode_window");
   get(lib.append, "nvj_kv_append");
   get(lib.append_mapped, "nvj_kv_append_mapped");
-  get(lib.prefill, "nvj_paged_prefill_packed");
-  get(lib.prefill_part, "nvj_paged_prefill_packed_part");
+  get(lib.prefill, "nvj_paged_prefill_packed_counted");
   get(lib.norm_rope, "nvj_qk_norm_rope_kv_append");
   get(lib.slot_mapping, "nvj_compute_slot_mapping");
   get(lib.copy_many, "nvj_copy_many_async");

@@ -19,7 +19,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, float* split_area, size_t split_bytes, cudaStream_t stream);
+                         int skip_single, int split_p, int tile_pairs, float* split_area, size_t split_bytes, cudaStream_t stream);
 bool prefill_umma2_usable(float scale, long long num_blocks);
 int launch_prefill_umma(const void* q, int q_dtype, const char* k_cache, const char* v_cache,
                         long long num_blocks, const int32_t* block_tables, int table_width,
@@ -38,6 +38,7 @@ struct PackedArgs {
   const int32_t* kv_lens; const int32_t* positions; const int32_t* query_start_loc;
   int rows, token_bucket; float scale; float* out; int32_t* status;
   void* workspace; size_t workspace_bytes; int variant;
+  int tile_pairs = -1;  // what the caller counted on the host (-1: not told)
 };
 
 static int check_packed(const PackedArgs& a, bool* tile_ok) {
@@ -143,7 +144,7 @@ static int run_tiles(const PackedArgs& a, int skip_single, cudaStream_t s) {
     }
     const int rc = launch_prefill_umma2(a.q, a.q_dtype, kc, vc, a.num_blocks, a.block_tables, a.table_width, a.kv_lens, a.positions,
                                         a.query_start_loc, a.rows, a.token_bucket, a.scale, a.out, a.status, skip_single,
-                                        variant == 5 ? 0 : 1, split_area, split_bytes, s);
+                                        variant == 5 ? 0 : 1, a.tile_pairs, split_area, split_bytes, s);
     if (rc != NVJ_ERR_UNSUPPORTED || variant != 0) return rc;
   }
   if (variant == 0 || variant == 3) {
@@ -190,65 +191,68 @@ extern "C" size_t nvj_paged_prefill_workspace_bytes(int max_rows) {
   return ws_header_bytes(max_rows) + prefill_split_bytes() + ws_ml_bytes(n) + ws_acc_bytes(n);
 }
 
-extern "C" int nvj_paged_prefill_packed(const void* q, int q_dtype, const void* k_cache_layer,
-                                        const void* v_cache_layer, int kv_dtype,
-                                        int64_t num_blocks, int block_size, int num_kv_heads,
-                                        int head_dim, int num_q_heads,
-                                        const int32_t* block_tables, int table_width,
-                                        const int32_t* kv_lens, const int32_t* positions,
-                                        const int32_t* query_start_loc, int rows,
-                                        int token_bucket, float scale, float* out,
-                                        int32_t* status, void* workspace, size_t workspace_bytes,
-                                        int variant, nvj_stream_t stream) {
-  using namespace nvj;
-  const PackedArgs a{q, q_dtype, k_cache_layer, v_cache_layer, kv_dtype, num_blocks, block_size, num_kv_heads, head_dim,
-                     num_q_heads, block_tables, table_width, kv_lens, positions, query_start_loc, rows, token_bucket,
-                     scale, out, status, workspace, workspace_bytes, variant};
+namespace nvj {
+
+// A whole batch (part 0) or one part of it (nvj_paged_prefill_packed_part).
+static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t s) {
+  if (part < 0 || part > 3 || cta_limit < 0) return NVJ_ERR_INVALID_ARGUMENT;
   bool tile_ok = false;
   const int rc = check_packed(a, &tile_ok);
-  if (rc != NVJ_OK || token_bucket == 0) return rc;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (!tile_ok || variant == 1) return run_generic(a, s);
+  if (rc != NVJ_OK || a.token_bucket == 0) return rc;
+  if (part > 0) {
+    if (!tile_ok || a.variant == 1) return NVJ_ERR_UNSUPPORTED;  // the generic kernel serves a batch in one piece
+    if (part == 1) return run_single_token_rows(a, cta_limit, 0, s);
+    if (part == 2 && !pair_kernel_serves(a)) return NVJ_ERR_UNSUPPORTED;  // the other tile kernels want a zeroed output
+    return run_tiles(a, part == 2 ? 1 : 0, s);
+  }
+  if (!tile_ok || a.variant == 1) return run_generic(a, s);
   // Rows that carry a single query token go to the streaming decode kernel when the caller lends it a decode
   // workspace; everything else goes to the tile kernel.
   int skip_single = 0;
-  if (workspace && rows > 0 && rows_run_beside_tiles(a)) {
+  if (a.workspace && a.rows > 0 && rows_run_beside_tiles(a)) {
     // tiles first, on a few SMs; the decode rows' clusters start at once and take the rest
     const int rc2 = run_tiles(a, 1, s);
     return rc2 != NVJ_OK ? rc2 : run_single_token_rows(a, 0, 1, s);
   }
-  if (workspace && rows > 0) {
+  if (a.workspace && a.rows > 0) {
     if (!pair_kernel_serves(a) &&
-        cudaMemsetAsync(out, 0, sizeof(float) * (size_t)token_bucket * kHq * kD, s) != cudaSuccess)
+        cudaMemsetAsync(a.out, 0, sizeof(float) * (size_t)a.token_bucket * kHq * kD, s) != cudaSuccess)
       return NVJ_ERR_LAUNCH;
     const int rc1 = run_single_token_rows(a, 0, 0, s);
-    if (rc1 == NVJ_OK) skip_single = 1;
-    else if (rc1 != NVJ_ERR_WORKSPACE) return rc1;
+    if (rc1 == NVJ_OK) {
+      skip_single = 1;
+    } else if (rc1 != NVJ_ERR_WORKSPACE) {
+      return rc1;
+    } else {  // no room to serve the rows of one token: the tiles take them too, and the caller has not counted those
+      PackedArgs all = a;
+      all.tile_pairs = -1;
+      return run_tiles(all, 0, s);
+    }
   }
   return run_tiles(a, skip_single, s);
 }
 
-extern "C" int nvj_paged_prefill_packed_part(const void* q, int q_dtype, const void* k_cache_layer,
-                                             const void* v_cache_layer, int kv_dtype,
-                                             int64_t num_blocks, int block_size, int num_kv_heads,
-                                             int head_dim, int num_q_heads,
-                                             const int32_t* block_tables, int table_width,
-                                             const int32_t* kv_lens, const int32_t* positions,
-                                             const int32_t* query_start_loc, int rows,
-                                             int token_bucket, float scale, float* out,
-                                             int32_t* status, void* workspace, size_t workspace_bytes,
-                                             int variant, int part, int cta_limit, nvj_stream_t stream) {
-  using namespace nvj;
-  const PackedArgs a{q, q_dtype, k_cache_layer, v_cache_layer, kv_dtype, num_blocks, block_size, num_kv_heads, head_dim,
-                     num_q_heads, block_tables, table_width, kv_lens, positions, query_start_loc, rows, token_bucket,
-                     scale, out, status, workspace, workspace_bytes, variant};
-  if (part < 1 || part > 3 || cta_limit < 0) return NVJ_ERR_INVALID_ARGUMENT;
-  bool tile_ok = false;
-  const int rc = check_packed(a, &tile_ok);
-  if (rc != NVJ_OK || token_bucket == 0) return rc;
-  if (!tile_ok || variant == 1) return NVJ_ERR_UNSUPPORTED;  // the generic kernel serves a batch in one piece
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (part == 1) return run_single_token_rows(a, cta_limit, 0, s);
-  if (part == 2 && !pair_kernel_serves(a)) return NVJ_ERR_UNSUPPORTED;  // the other tile kernels want a zeroed output
-  return run_tiles(a, part == 2 ? 1 : 0, s);
+}  // namespace nvj
+
+#define NVJ_PACKED_PARAMS                                                                                                   \
+  const void *q, int q_dtype, const void *k_cache_layer, const void *v_cache_layer, int kv_dtype, int64_t num_blocks,      \
+      int block_size, int num_kv_heads, int head_dim, int num_q_heads, const int32_t *block_tables, int table_width,       \
+      const int32_t *kv_lens, const int32_t *positions, const int32_t *query_start_loc, int rows, int token_bucket,        \
+      float scale, float *out, int32_t *status, void *workspace, size_t workspace_bytes, int variant
+#define NVJ_PACKED_ARGS                                                                                                     \
+  q, q_dtype, k_cache_layer, v_cache_layer, kv_dtype, num_blocks, block_size, num_kv_heads, head_dim, num_q_heads,         \
+      block_tables, table_width, kv_lens, positions, query_start_loc, rows, token_bucket, scale, out, status, workspace,   \
+      workspace_bytes, variant
+
+extern "C" int nvj_paged_prefill_packed(NVJ_PACKED_PARAMS, nvj_stream_t stream) {
+  return nvj::run_packed(nvj::PackedArgs{NVJ_PACKED_ARGS}, 0, 0, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int nvj_paged_prefill_packed_part(NVJ_PACKED_PARAMS, int part, int cta_limit, nvj_stream_t stream) {
+  if (part < 1) return NVJ_ERR_INVALID_ARGUMENT;
+  return nvj::run_packed(nvj::PackedArgs{NVJ_PACKED_ARGS}, part, cta_limit, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int nvj_paged_prefill_packed_counted(NVJ_PACKED_PARAMS, int part, int tile_pairs, nvj_stream_t stream) {
+  return nvj::run_packed(nvj::PackedArgs{NVJ_PACKED_ARGS, tile_pairs}, part, 0, static_cast<cudaStream_t>(stream));
 }

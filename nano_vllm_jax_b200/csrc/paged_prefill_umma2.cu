@@ -75,6 +75,7 @@ struct Umma2Params {
   int32_t* status;
   long long num_blocks;
   int rows, token_bucket, table_width, skip_single, q_dtype;
+  int counted;    // 1: the launch has exactly the caller's number of pairs plus an idle one; more pairs are flagged
   int zero_fill;  // 1: the kernel itself zeroes what no tile writes (padding tokens, rows of several tokens without keys)
   int split_p;  // 1: P enters P V as two bf16 terms (hi + lo), 0: as one (the weights are then bf16-rounded)
   float scale;
@@ -544,76 +545,8 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   const int rank = (int)cluster_ctarank();  // == blockIdx.x & 1
   NVJ_U2_PHASE(0);
   NVJ_U2_NOTE(7, 0ull);
-  pdl_wait();
-  // whatever follows may take its places now: the merge launch of a batch with splits (its CTAs wait for this grid to
-  // finish), the decode pass of a mixed batch (it runs beside, on the SMs this grid leaves)
-  pdl_release();
-  if (blockIdx.z > 0) {  // the extra splits leave at once when no row's key range is long enough to be split
-    int any = 0;
-    for (int rr = threadIdx.x; rr < p.rows; rr += kU2Threads) any |= p.kv_lens[rr] > (kU2SplitFrom - 1) * kU2Keys ? 1 : 0;
-    if (!__syncthreads_or(any)) return;
-  }
-
-  // ---- which (table row, pair of 32-token tiles) this cluster serves; both CTAs compute the same
-  if (warp == 0) {
-    const U2Tile t = u2_find_tile(p, blockIdx.x >> 1, gridDim.x >> 1, rank, gridDim.z > 1, lane);
-    if (lane == 0) {
-      sm.row = t.row; sm.tok0 = t.tok0; sm.ntok = t.ntok; sm.pair_last_tok = t.pair_last_tok; sm.abort_flag = 0;
-      sm.total_pairs = t.total; sm.idle_index = t.idle;
-    }
-  }
-  __syncthreads();
-  const int row = sm.row, tok0 = sm.tok0, ntok = sm.ntok;
-  int4* info = gridDim.z > 1 && blockIdx.z == 0 && threadIdx.x == 0 ? p.tile_info + blockIdx.x * kHkv + kvh : nullptr;
-  if (row < 0) {  // the whole cluster leaves: nothing has been allocated or shared yet
-    if (info) *info = make_int4(0, 0, 0, 0);
-    if (p.zero_fill && sm.idle_index == 0 && blockIdx.z == 0) {
-      // the first idle cluster (there is always one) zeroes the padding tokens, a quarter per CTA of the cluster pair x KV head
-      int real = p.query_start_loc[p.rows];
-      real = real < p.token_bucket ? real : p.token_bucket;
-      const long long n4 = (long long)(p.token_bucket - real) * kHq * kD / 4;
-      float4* pad = reinterpret_cast<float4*>(p.out + (long long)real * kHq * kD);
-      const int part = rank * kHkv + kvh;
-      for (long long i = (long long)part * kU2Threads + threadIdx.x; i < n4; i += 2LL * kHkv * kU2Threads)
-        pad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    return;
-  }
-
-  int kv_len;
-  const int n_tiles = u2_key_tiles(p, row, tok0, rank, sm.pair_last_tok, lane, kv_len, threadIdx.x == 0 && rank == 0);
-  if (n_tiles == 0) {  // same decision in both CTAs; a row without keys produces zeros
-    if (info) *info = make_int4(tok0, ntok, 0, 0);
-    if (p.zero_fill && blockIdx.z == 0) {
-      for (int i = threadIdx.x; i < ntok * kG * (kD / 4); i += kU2Threads) {
-        const int t = i / (kG * (kD / 4)), rest = i - t * (kG * (kD / 4));
-        reinterpret_cast<float4*>(p.out + ((long long)(tok0 + t) * kHq + kvh * kG) * kD)[rest] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-    return;
-  }
-
-  // Key-range splits of this pair: as many as leave every split kU2MinSplitTiles tiles and as the batch's pairs
-  // leave pair slots for; the splits beyond that leave at once (both CTAs decide alike).
-  int splits = 1, tile0 = 0, my_tiles = n_tiles;
-  if (gridDim.z > 1) {
-    splits = u2_split_count(p, n_tiles, sm.total_pairs, (int)gridDim.z);
-    if (info) *info = make_int4(tok0, ntok, splits, 0);
-    if ((int)blockIdx.z >= splits) return;
-    tile0 = (int)blockIdx.z * n_tiles / splits;
-    my_tiles = ((int)blockIdx.z + 1) * n_tiles / splits - tile0;
-  }
-
-  // the query rows, and the block ids of the producer's first eight tiles, are asked for now and arrive while the
-  // pair is being set up
-  uint4 qv[4][4];
-  if (warp >= 2 && p.q_dtype == NVJ_BF16) u2_request_q(p, tok0, ntok, kvh, warp, lane, qv);
-  int first_ids = -1;
-  if (warp == 0) {
-    const int bi = tile0 * 4 + lane;
-    if (bi < (kv_len + kBlk - 1) / kBlk && bi < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + bi];
-  }
-
+  // The pair is set up before anything is read: this runs while the kernel in front (the append of the same tokens, usually)
+  // is still at work.
   if (warp == 1) tmem2_alloc(smem_u32(&sm.tmem_base), kU2TmemCols);
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&sm.q_full), 2 * kU2SoftmaxThreads);
@@ -634,6 +567,80 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   __syncthreads();
   cluster_sync_all();  // the peer's barriers exist before anything is sent to them
   tc_fence_after_sync();
+  pdl_wait();
+  // whatever follows may take its places now: the merge launch of a batch with splits (its CTAs wait for this grid to
+  // finish), the decode pass of a mixed batch (it runs beside, on the SMs this grid leaves)
+  pdl_release();
+  auto leave = [&] {  // the whole cluster leaves without having touched its tensor memory
+    cluster_sync_all();
+    if (warp == 1) tmem2_dealloc(sm.tmem_base, kU2TmemCols);
+  };
+  if (blockIdx.z > 0) {  // the extra splits leave at once when no row's key range is long enough to be split
+    int any = 0;
+    for (int rr = threadIdx.x; rr < p.rows; rr += kU2Threads) any |= p.kv_lens[rr] > (kU2SplitFrom - 1) * kU2Keys ? 1 : 0;
+    if (!__syncthreads_or(any)) return leave();
+  }
+
+  // ---- which (table row, pair of 32-token tiles) this cluster serves; both CTAs compute the same
+  if (warp == 0) {
+    const U2Tile t = u2_find_tile(p, blockIdx.x >> 1, gridDim.x >> 1, rank, gridDim.z > 1, lane);
+    if (lane == 0) {
+      sm.row = t.row; sm.tok0 = t.tok0; sm.ntok = t.ntok; sm.pair_last_tok = t.pair_last_tok; sm.abort_flag = 0;
+      sm.total_pairs = t.total; sm.idle_index = t.idle;
+    }
+  }
+  __syncthreads();
+  const int row = sm.row, tok0 = sm.tok0, ntok = sm.ntok;
+  if (p.counted && blockIdx.x == 0 && row >= 0 && threadIdx.x == 0) atomicOr(p.status, NVJ_DEV_BAD_LENGTH);
+  int4* info = gridDim.z > 1 && blockIdx.z == 0 && threadIdx.x == 0 ? p.tile_info + blockIdx.x * kHkv + kvh : nullptr;
+  if (row < 0) {
+    if (info) *info = make_int4(0, 0, 0, 0);
+    if (p.zero_fill && sm.idle_index == 0 && blockIdx.z == 0) {
+      // the first idle cluster (there is always one) zeroes the padding tokens, a quarter per CTA of the cluster pair x KV head
+      int real = p.query_start_loc[p.rows];
+      real = real < p.token_bucket ? real : p.token_bucket;
+      const long long n4 = (long long)(p.token_bucket - real) * kHq * kD / 4;
+      float4* pad = reinterpret_cast<float4*>(p.out + (long long)real * kHq * kD);
+      const int part = rank * kHkv + kvh;
+      for (long long i = (long long)part * kU2Threads + threadIdx.x; i < n4; i += 2LL * kHkv * kU2Threads)
+        pad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    return leave();
+  }
+
+  int kv_len;
+  const int n_tiles = u2_key_tiles(p, row, tok0, rank, sm.pair_last_tok, lane, kv_len, threadIdx.x == 0 && rank == 0);
+  if (n_tiles == 0) {  // same decision in both CTAs; a row without keys produces zeros
+    if (info) *info = make_int4(tok0, ntok, 0, 0);
+    if (p.zero_fill && blockIdx.z == 0) {
+      for (int i = threadIdx.x; i < ntok * kG * (kD / 4); i += kU2Threads) {
+        const int t = i / (kG * (kD / 4)), rest = i - t * (kG * (kD / 4));
+        reinterpret_cast<float4*>(p.out + ((long long)(tok0 + t) * kHq + kvh * kG) * kD)[rest] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    return leave();
+  }
+
+  // Key-range splits of this pair: as many as leave every split kU2MinSplitTiles tiles and as the batch's pairs
+  // leave pair slots for; the splits beyond that leave at once (both CTAs decide alike).
+  int splits = 1, tile0 = 0, my_tiles = n_tiles;
+  if (gridDim.z > 1) {
+    splits = u2_split_count(p, n_tiles, sm.total_pairs, (int)gridDim.z);
+    if (info) *info = make_int4(tok0, ntok, splits, 0);
+    if ((int)blockIdx.z >= splits) return leave();
+    tile0 = (int)blockIdx.z * n_tiles / splits;
+    my_tiles = ((int)blockIdx.z + 1) * n_tiles / splits - tile0;
+  }
+
+  // the query rows, and the block ids of the producer's first eight tiles
+  uint4 qv[4][4];
+  if (warp >= 2 && p.q_dtype == NVJ_BF16) u2_request_q(p, tok0, ntok, kvh, warp, lane, qv);
+  int first_ids = -1;
+  if (warp == 0) {
+    const int bi = tile0 * 4 + lane;
+    if (bi < (kv_len + kBlk - 1) / kBlk && bi < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + bi];
+  }
+
   const uint32_t tmem = sm.tmem_base;
   NVJ_U2_PHASE(1);
   NVJ_U2_NOTE(7, (unsigned long long)my_tiles);
@@ -772,7 +779,8 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, float* split_area, size_t split_bytes, cudaStream_t stream) {
+                         int skip_single, int split_p, int tile_pairs, float* split_area, size_t split_bytes,
+                         cudaStream_t stream) {
   static PerDeviceFlags opted_in;
   constexpr int kSmemBytes = (int)sizeof(Umma2Smem) + 1024;
   static_assert(kSmemBytes <= 232448, "tiles exceed the shared memory of one CTA");
@@ -793,7 +801,12 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
   p.block_tables = block_tables; p.kv_lens = kv_lens; p.positions = positions; p.query_start_loc = query_start_loc;
   p.out = out; p.status = status; p.num_blocks = num_blocks; p.rows = rows; p.token_bucket = token_bucket;
   p.table_width = table_width; p.skip_single = skip_single; p.scale = scale; p.split_p = split_p;
-  const int pairs = (token_bucket + 2 * kU2Tokens - 1) / (2 * kU2Tokens) + rows;
+  // Clusters: one per pair of tiles and one that stays idle (it zeroes the padding).  Without the caller's count, at most
+  // so many; the ones too many cost a batch of many rows and few tiles its start (34 rows, 8 pairs: 43 clusters per head,
+  // two waves of CTAs that only set themselves up and leave).
+  const int most_pairs = (token_bucket + 2 * kU2Tokens - 1) / (2 * kU2Tokens) + rows;
+  const int pairs = tile_pairs >= 0 && tile_pairs + 1 < most_pairs ? tile_pairs + 1 : most_pairs;
+  p.counted = pairs < most_pairs;
   // Key-range splits: only while the batch leaves pair slots free, as many as the lent area holds; the kernel settles
   // the number per pair from what the batch really holds.
   int splits = 1;

@@ -378,7 +378,7 @@ def paged_attention_prefill_packed(query, k_cache, v_cache, block_table, kv_lens
     """
     if positions.shape == token_row_ids.shape:
         out = _k.host().packed_prefill(query, k_cache, v_cache, block_table, kv_lens, positions, query_start_loc, layer_idx,
-                                       block_size, scale, num_key_value_groups, num_decode_rows)
+                                       block_size, scale, num_key_value_groups, num_decode_rows, query_tile_pairs)
         if out is not None:
             dtype = out_dtype if out_dtype is not None else k_cache.dtype
             return out if dtype is torch.float32 else out.to(dtype)

@@ -1,0 +1,54 @@
+"""Packed prefill launched for exactly the tiles that the host counted: the same rows as without the count, padding zeroed,
+and a count that is too small flagged instead of passing for a result."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import BS, SCALE, to_torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(qlens, cached, pad, seed):
+    rng = np.random.default_rng(seed)
+    lens = np.array([q + c for q, c in zip(qlens, cached)], np.int32)
+    need = -(-lens // BS)
+    tables, o = np.zeros((len(qlens), int(need.max())), np.int32), 0
+    perm = rng.permutation(int(need.sum()) + 8)
+    for r, n in enumerate(need):
+        tables[r, :n] = perm[o:o + n]
+        o += n
+    pos = np.concatenate([np.arange(c, c + q) for q, c in zip(qlens, cached)] + [np.zeros(pad, int)]).astype(np.int32)[None]
+    rid = np.concatenate([np.repeat(np.arange(len(qlens)), qlens), np.zeros(pad, int)]).astype(np.int32)[None]
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    cache = [torch.randn((1, int(need.sum()) + 8, BS, 2, 256), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    q = torch.randn((1, pos.shape[1], 8, 256), generator=g, device="cuda").to(torch.bfloat16)
+    return q, cache, to_torch(tables), to_torch(lens), to_torch(pos), to_torch(rid), to_torch(np.cumsum([0] + list(qlens)).astype(np.int32))
+
+
+@pytest.mark.parametrize("qlens,cached,pad", [
+    ((64,), (0,), 0), ((65, 2), (0, 70), 3), ((63, 64, 128), (5, 0, 300), 0),       # no decode rows: key ranges may be split
+    ((1, 1, 130, 1, 40), (40, 700, 0, 3, 90), 7), ((1,) * 40 + (2,), (33,) * 40 + (0,), 0),  # decode rows beside the tiles
+])
+def test_counted_launch_equals_the_uncounted_one(qlens, cached, pad):
+    from nano_vllm_jax_b200 import kv_cache as kvc
+    q, (k, v), tables, lens, pos, rid, qsl = _batch(qlens, cached, pad, len(qlens) + pad)
+    singles, pairs = sum(n == 1 for n in qlens), sum(-(-n // 64) for n in qlens if n > 1)
+
+    def run(count):
+        return kvc.paged_attention_prefill_packed(q, k, v, tables, lens, pos, rid, qsl, BS, SCALE, 4, out_dtype=torch.float32,
+                                                  num_decode_rows=singles, query_tile_pairs=count)
+
+    out, ref = run(pairs), run(None)
+    assert float((out - ref).abs().max()) <= 2e-3
+    assert not out[0, sum(qlens):].any() and not torch.isnan(out).any()
+
+
+def test_a_count_that_is_too_small_is_flagged(monkeypatch):
+    from nano_vllm_jax_b200 import kv_cache as kvc
+    from nano_vllm_jax_b200.kernels.paged_kv import DeviceStatusError
+    q, (k, v), tables, lens, pos, rid, qsl = _batch((200, 90), (0, 0), 0, 3)
+    with pytest.raises(DeviceStatusError):
+        kvc.paged_attention_prefill_packed(q, k, v, tables, lens, pos, rid, qsl, BS, SCALE, 4, out_dtype=torch.float32,
+                                           num_decode_rows=0, query_tile_pairs=3)
