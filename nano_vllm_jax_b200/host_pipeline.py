@@ -56,7 +56,7 @@ class _Slot:
     busy: bool = False
     graphs: Dict[int, torch.cuda.CUDAGraph] = field(default_factory=dict)  # per layer, with capture=True
     graph_out: Dict[int, torch.Tensor] = field(default_factory=dict)
-    inputs: tuple = ()           # (q, k, v, tables, positions, seq_lens): the targets of the step's operand copies
+    inputs: tuple = ()           # (q, positions, seq_lens, k, v, tables): the targets of the step's operand copies
     in_events: tuple = ()        # the raw handles of in_done
     d2h_lists: Dict[int, object] = field(default_factory=dict)  # per layer: host_out <- that layer's graph output
     sources: list = field(default_factory=list)
@@ -91,7 +91,7 @@ class HostDecodePipeline:
                 host_out=torch.empty((rows, 1, hq * d), dtype=torch.float32).pin_memory(),
                 in_done=(torch.cuda.Event(), torch.cuda.Event()), compute_done=torch.cuda.Event(), out_done=torch.cuda.Event()))
         for slot in self.slots:
-            slot.inputs = (slot.q, slot.k, slot.v, slot.tables, slot.positions, slot.seq_lens)
+            slot.inputs = (slot.q, slot.positions, slot.seq_lens, slot.k, slot.v, slot.tables)
             for event, stream in zip(slot.in_done, (self.h2d, self.h2d_rest)):
                 event.record(stream)  # (an event has a handle from its first record on)
             slot.in_events = tuple(event.cuda_event for event in slot.in_done)
@@ -117,15 +117,16 @@ class HostDecodePipeline:
         slot = self.slots[ticket % len(self.slots)]
         if slot.busy:
             slot.out_done.synchronize()  # its operands were consumed and its result has left the device
-        # the step's operands: the query on one stream, everything else on the other, the compute stream behind both
+        # the step's operands on two streams of about the same length (a small copy takes ~2 us whatever its size), the
+        # compute stream behind both
         host = _k.host()
-        srcs = (query, k, v, block_tables, positions, seq_lens)
-        if host.stage_in(slot.inputs, srcs, 1, self._in_streams, slot.in_events) is None:
+        srcs = (query, positions, seq_lens, k, v, block_tables)
+        if host.stage_in(slot.inputs, srcs, 3, self._in_streams, slot.in_events) is None:
             srcs = tuple(t.to(dst.dtype).contiguous() for t, dst in zip(srcs, slot.inputs))
-            for i, (t, dst) in enumerate(zip(srcs, slot.inputs)):
+            for i, t, dst in zip((0, 4, 5, 1, 2, 3), srcs, slot.inputs):
                 if t.numel() != dst.numel():
                     raise ValueError(f"operand {i} has {t.numel()} elements, the slot holds {dst.numel()}")
-            host.stage_in(slot.inputs, srcs, 1, self._in_streams, slot.in_events)
+            host.stage_in(slot.inputs, srcs, 3, self._in_streams, slot.in_events)
         slot.sources = srcs  # alive until the slot comes round again
         if after_compute is None and host.fused_decode(slot.q, slot.k, slot.v, self.cache.k_cache, self.cache.v_cache, slot.tables,
                                                        slot.seq_lens, slot.positions, layer_id, self.block_size, self.scale,
