@@ -56,7 +56,7 @@ struct DecodeParams {
   // kernel has let its dependents go); it ends only after that kernel has, so that the stream's order holds behind both
   int beside;
   // which wide kernel serves rows of several query tokens: 0 = automatic (mma.sync tiles up to width 4, tcgen05 beyond),
-  // 1 = mma.sync tiles, 2 = tcgen05
+  // 1 = mma.sync tiles, 2 = tcgen05, 3 = thread-block clusters
   int wide_form;
   // what a row end costs a CTA, in blocks (decode_parts.cuh); set by the launchers, the same for every kernel of a call
   int row_end_cost;
@@ -174,6 +174,8 @@ bool decode_cluster_pays(int batch, int table_width);  // a bf16 batch is short 
 int launch_decode_pipelined(const DecodeParams& p, int num_ctas, cudaStream_t stream);
 int decode_wide_num_ctas();  // 1 per SM of the current device
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // tensor-core streaming kernels, width 1..8
+int launch_decode_cluster_wide(const DecodeParams& p, cudaStream_t stream);  // rows of 2 - 4 tokens, few and short
+bool decode_cluster_wide_pays(const DecodeParams& p);
 int run_decode_wide(DecodeParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);  // checks, carves, launches
 int launch_decode_umma(const DecodeParams& p, cudaStream_t stream);  // the tcgen05 form, rows already appended
 int append_decode_rows(const void* new_k, const void* new_v, const int32_t* positions,

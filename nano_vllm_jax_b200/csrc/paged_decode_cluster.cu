@@ -20,11 +20,9 @@
 
 #include <type_traits>
 
-#include "decode_parts.cuh"
+#include "decode_cluster.cuh"
 
 namespace nvj {
-
-constexpr int kClMaxCluster = 16;
 
 // ---- f32 caches (and f16 ones under f32 queries): fp32 products on the CUDA cores --------------------------------
 // Every warp keeps a unit of 4 keys in flight in shared memory of its own (16-byte cp.async; the next unit's K rows are
@@ -54,9 +52,6 @@ template <> struct ClRaw<float> { uint4 v, w; };
 // This lane's 16-byte pieces of a row: `at` is the lane's place in the ring's row, pieces 512 bytes apart.
 __device__ __forceinline__ void cl_copy16(uint32_t dst, const char* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cl_copy16_or_zero(uint32_t dst, const char* src, uint32_t size) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
 }
 template <typename T>
 __device__ __forceinline__ void cl_copy_row(uint32_t row, const char* src, int lane) {
@@ -99,36 +94,10 @@ __device__ __forceinline__ void cl_unpack(const ClRaw<T>& r, float2 (&o)[4]) {
   }
 }
 
-__device__ __forceinline__ uint32_t cl_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cl_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // A launch that runs beside the kernel in front of it ends after that kernel: one CTA holds the grid open.
 __device__ __forceinline__ void cl_end_beside(const DecodeParams& p) {
   if (p.beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
 }
-// Address of this CTA's shared-memory location in CTA `rank` of the cluster, and loads from there.
-__device__ __forceinline__ uint32_t cl_map(const void* p, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ float4 cl_ld4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float2 cl_ld2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-  return v;
-}
-
 // The CTAs' sums [head][pitch] and (max, sum) pairs, at the same places in every CTA of the cluster, into the output: rank
 // r takes its 1 / ctas of the float4 pieces of [heads][256 dims].
 template <int kHeads>
@@ -416,45 +385,6 @@ struct CmSmem {
   };
 };
 
-__device__ __forceinline__ void cm_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void cm_ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ uint32_t cm_transpose(uint32_t x) {
-  uint32_t y;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
-  return y;
-}
-template <typename T>
-__device__ __forceinline__ void cm_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  if constexpr (std::is_same<T, __half>::value)
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  else
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// Two weights as a 16-bit pair (x low): rounded, or with `rest` what the rounding left over.
-template <typename T>
-__device__ __forceinline__ uint32_t cm_pack(float x, float y, bool rest) {
-  if constexpr (std::is_same<T, __half>::value) {
-    const __half2 h = __floats2half2_rn(x, y);
-    const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
-    return rest ? *reinterpret_cast<const uint32_t*>(&l) : *reinterpret_cast<const uint32_t*>(&h);
-  } else {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
-    return rest ? *reinterpret_cast<const uint32_t*>(&l) : *reinterpret_cast<const uint32_t*>(&h);
-  }
-}
-
 template <typename T, bool kBoth>
 __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(DecodeParams p) {
   extern __shared__ __align__(128) unsigned char cl_smem_raw[];
@@ -598,7 +528,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
       }
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) s[e] = ex2_approx(s[e] - m[e & 1]);
+    for (int e = 0; e < 4; ++e) s[e] = ex2_approx(s[e] - (m[e & 1] <= kNegBig ? 0.f : m[e & 1]));  // nothing attended yet: 0
     l[0] += s[0] + s[2];
     l[1] += s[1] + s[3];
     const uint32_t b0 = cm_transpose(cm_pack<T>(s[0], s[1], t >= 2)), b1 = cm_transpose(cm_pack<T>(s[2], s[3], t >= 2));
@@ -678,47 +608,6 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   cl_end_beside(p);
 }
 
-template <class Kernel>
-static int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const DecodeParams& p, int cluster, int heads, int threads, int smem,
-                           cudaStream_t stream) {
-  if (!once_per_device(opted_in, [&](int) {
-        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-               cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-      }))
-    return NVJ_ERR_LAUNCH;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cluster, heads, p.batch);
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
-}
-
-// CTAs per cluster for `groups` clusters of rows of up to `blocks` blocks, when a CTA walks `walkers` blocks at a time.
-// Doubled while the CTAs fit the SMs (`per_sm` hundredths of a CTA per SM) and a walker of the longest row has more than one
-// block; and, in batches of many CTAs, until none has more than 12, so that the last CTAs to finish are short ones.
-// Clusters of 16 (no longer portable, and placed one by one) only up to 2.2 CTAs per SM.  (Measured at 1 - 256 rows of
-// 64 - 16384 tokens: within 3% of the best size of each.)
-static int cluster_size(long long groups, int blocks, int sms, int walkers, int per_sm, int most) {
-  int c = 1;
-  while (c < most && c * walkers < blocks) {
-    const bool fits = 100 * 2 * c * groups <= (long long)(c < 8 || per_sm < 220 ? per_sm : 220) * sms;
-    if (!fits && (c >= 8 || blocks <= 12 * c * walkers)) break;
-    c *= 2;
-  }
-  return c;
-}
-// CTAs of 64 KiB go three to an SM; 2.75, because clusters do not pack every SM.
-constexpr int kCmPerSm = 275;
 static int cluster_per_head(int batch, int blocks, int sms) {
   return cluster_size(2LL * batch, blocks, sms, kCmWarps, kCmPerSm, kClMaxCluster);
 }

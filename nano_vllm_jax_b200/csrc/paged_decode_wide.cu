@@ -618,9 +618,15 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
     return NVJ_ERR_UNSUPPORTED;
   int n = decode_wide_num_ctas();
   if (n <= 0) return NVJ_ERR_LAUNCH;
-  // rows of 5 and more query tokens: the tcgen05 form (two 16-row tiles per warp pair make the mma.sync form
-  // compute-bound, and it ends at 8 tokens)
-  if (p.wide_form == 2 || (p.wide_form == 0 && p.width > 4)) {
+  if (p.wide_form == 3 || (p.wide_form == 0 && p.cta_limit <= 0 && decode_cluster_wide_pays(p)))
+    return launch_decode_cluster_wide(p, stream);
+  // Rows of 5 and more query tokens: the tcgen05 form (two 16-row tiles per warp pair make the mma.sync form
+  // compute-bound, and it ends at 8 tokens).  Below that the tcgen05 form answers sooner (4 tokens, 16 rows of 512 - 2048
+  // keys: 21.2 us against 29.7) and the mma.sync form streams better (128 rows of 1024 - 4096: 129 against 121); they meet at
+  // about 4096 blocks with 2 tokens (20.7 : 21.8 at 2048, 40.1 : 39.2 at 8192) and 12288 with 3 and 4 (39.6 : 44.5 at 8192,
+  // 70.2 : 70.8 and 69.4 : 68.3 at 16384).
+  const long long blocks = (long long)p.batch * p.table_width;
+  if (p.wide_form == 2 || (p.wide_form == 0 && p.width > 1 && (p.width > 4 || blocks <= (p.width == 2 ? 4096 : 12288)))) {
     const int rc = launch_decode_umma(p, stream);
     if (rc != NVJ_ERR_UNSUPPORTED || p.wide_form == 2) return rc;
   }
@@ -672,7 +678,7 @@ namespace nvj {
 
 // Rows of several query tokens: everything but the workspace is in p (width, wide_form, pointers, shapes).
 int run_decode_wide(DecodeParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  if (p.batch < 0 || p.table_width < 0 || p.num_blocks < 0 || p.width < 1 || p.wide_form < 0 || p.wide_form > 2)
+  if (p.batch < 0 || p.table_width < 0 || p.num_blocks < 0 || p.width < 1 || p.wide_form < 0 || p.wide_form > 3)
     return NVJ_ERR_INVALID_ARGUMENT;
   if (p.width > kWideMaxWidth || (p.wide_form == 1 && p.width > kWMaxWidth)) return NVJ_ERR_UNSUPPORTED;
   if (p.q_dtype != NVJ_BF16 || p.kv_dtype != NVJ_BF16 || p.block_size != kBlk || p.num_kv_heads != kHkv ||

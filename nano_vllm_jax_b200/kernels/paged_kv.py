@@ -424,8 +424,8 @@ def paged_decode_attention_wide(q, k_layer, v_layer, block_table, seq_lens, posi
 
     Token t of row b sees keys p < seq_lens[b] with p <= positions[b, t] (the reference's wide decode,
     nanovllm_jax/kv_cache.py:852-998); K and V of a row are read once for all of its tokens.
-    `form`: 0 automatic (mma.sync tiles up to 4 tokens per row, tcgen05 beyond), 1 mma.sync tiles (up to 8 tokens),
-    2 tcgen05.
+    `form`: 0 automatic (by tokens per row and size of the batch), 1 mma.sync tiles (up to 8 tokens), 2 tcgen05,
+    3 thread-block clusters (2..4 tokens).
     """
     if not wide_decode_supported(q, k_layer):
         raise ValueError("paged_decode_attention_wide: 2..16 bf16 query tokens per row over the bf16 cache [NB, 16, 2, 256]")

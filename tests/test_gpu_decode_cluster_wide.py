@@ -1,0 +1,61 @@
+"""The cluster form for rows of 2 - 4 query tokens against the streaming forms: both tile counts, block edges of a row, every
+cluster size, tokens that see nothing, and a block id outside the pool."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import BS, SCALE, decode_case, to_torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens", [2, 3, 4])
+@pytest.mark.parametrize("rows,width", [(3, 2), (3, 5), (2, 20), (1, 80), (40, 9), (150, 6)])
+def test_equals_the_streaming_form(tokens, rows, width):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    span = width * BS
+    edges = [n for n in (1, 15, 16, 17, 31, 33, span - 16, span - 1, span, 0) if n <= span]
+    lens = np.asarray([edges[(i + tokens) % len(edges)] for i in range(rows)], np.int32)
+    nblk = int((-(-lens // BS)).sum()) + 9
+    rng = np.random.default_rng(rows + tokens)
+    c = decode_case(tokens, nblk, rows, 1, 1, width=width)
+    perm, o = rng.permutation(nblk), 0
+    tables = np.zeros((rows, width), np.int32)
+    for b, n in enumerate(-(-lens // BS)):
+        tables[b, :n] = perm[o:o + n]
+        o += n
+    k, v = (to_torch(c[n])[0].to(torch.bfloat16) for n in ("k_cache", "v_cache"))
+    for t in (k, v):  # what lies behind a row's last key must not reach the result
+        for b, n in enumerate(lens):
+            if n % BS:
+                t[int(tables[b, n // BS]), n % BS:] = 1000.0
+    q = to_torch(rng.standard_normal((rows, tokens, 8, 256)).astype(np.float32)).to(torch.bfloat16)
+    pos = lens[:, None] - tokens + np.arange(tokens)[None]  # short rows: the first tokens see nothing
+    pos[::3, -1] = -1                                       # padding
+    args = q, k, v, to_torch(tables), to_torch(lens)
+    for p in (to_torch(pos.astype(np.int32)), None):
+        got = K.paged_decode_attention_wide(*args, p, SCALE, form=3)
+        ref = K.paged_decode_attention_wide(*args, p, SCALE, form=2)
+        assert float((got - ref).abs().max()) <= 2e-3
+        assert not got[args[4] == 0].any()
+        if p is not None:
+            assert not got[p < 0].any()
+
+
+def test_a_bad_block_is_flagged_and_left_out(monkeypatch):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    c = decode_case(3, 8, 2, 1, 1, width=4)
+    k, v = (to_torch(c[n])[0].to(torch.bfloat16) for n in ("k_cache", "v_cache"))
+    q = torch.randn((2, 3, 8, 256), device=k.device).to(torch.bfloat16)
+    lens = to_torch(np.asarray([40, 64], np.int32))
+    tables = to_torch(np.asarray([[0, 1, 8, 0], [3, 4, 5, 6]], np.int32))  # the pool ends at 7
+    with pytest.raises(K.DeviceStatusError):
+        K.paged_decode_attention_wide(q, k, v, tables, lens, None, SCALE, form=3)
+    monkeypatch.setenv("NVJ_CHECK_STATUS", "0")
+    got = K.paged_decode_attention_wide(q, k, v, tables, lens, None, SCALE, form=3)
+    with pytest.raises(K.DeviceStatusError):
+        K.check_device_status()
+    good = to_torch(np.asarray([[0, 1, 7, 0], [3, 4, 5, 6]], np.int32))
+    ref = K.paged_decode_attention_wide(q, k, v, good, torch.tensor([32, 64], dtype=torch.int32, device="cuda"), None, SCALE, form=2)
+    assert float((got - ref).abs().max()) <= 2e-3
