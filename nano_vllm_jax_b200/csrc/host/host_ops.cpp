@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
+#include <structmember.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -555,6 +556,41 @@ class WordHash {
   }
 };
 
+// The value of a plain int of machine size; false for anything else.  (Token ids are one digit: no call.)
+inline bool int_of(PyObject* o, long long* v) {
+  if (!PyLong_CheckExact(o)) return false;
+#if PY_VERSION_HEX >= 0x030C0000
+  const PyLongObject* i = reinterpret_cast<const PyLongObject*>(o);
+  if (PyUnstable_Long_IsCompact(i)) { *v = PyUnstable_Long_CompactValue(i); return true; }
+#endif
+  int overflow = 0;
+  *v = PyLong_AsLongLongAndOverflow(o, &overflow);
+  return !overflow;
+}
+
+// The chained digests of a token list's blocks, one at a time.
+class HashChain {
+  PyObject* tokens_;
+  long long bs_;
+  std::vector<uint64_t> words_;  // [predecessor's digest, the block's tokens]
+  bool chained_ = false;
+
+ public:
+  HashChain(PyObject* tokens, long long block_size) : tokens_(tokens), bs_(block_size), words_((size_t)block_size + 1) {}
+  void start_from(uint64_t digest) { words_[0] = digest; chained_ = true; }
+  // Digest of block b, the one behind the last asked for; false when its tokens are not machine-size integers.
+  bool next(long long b, uint64_t* h) {
+    for (long long i = 0; i < bs_; ++i) {
+      long long v;
+      if (!int_of(PyList_GET_ITEM(tokens_, (Py_ssize_t)(b * bs_ + i)), &v)) return false;
+      words_[(size_t)i + 1] = (uint64_t)v;
+    }
+    *h = chained_ ? WordHash::of(words_.data(), words_.size()) : WordHash::of(words_.data() + 1, words_.size() - 1);
+    start_from(*h);
+    return true;
+  }
+};
+
 // hash_chain(token_ids, block_size, blocks, prefix | -1) -> digests of the first `blocks` full blocks of a token list, each
 // over its predecessor's digest (the first over `prefix` if there is one) and its own tokens as int64.  None when the
 // tokens are not a list of machine-size integers.
@@ -564,21 +600,12 @@ PyObject* hash_chain(PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   if (!PyList_CheckExact(a[0]) || !PyLong_CheckExact(a[3]) || bs < 1 || blocks < 0 || blocks > PyList_GET_SIZE(a[0]) / bs) NVJ_NONE();
   int overflow = 0;
-  bool chained = !(PyLong_AsLongLongAndOverflow(a[3], &overflow) == -1 && !overflow);
-  std::vector<uint64_t> words((size_t)bs + 1);
-  words[0] = chained ? PyLong_AsUnsignedLongLongMask(a[3]) : 0;
+  HashChain chain(a[0], bs);
+  if (PyLong_AsLongLongAndOverflow(a[3], &overflow) != -1 || overflow) chain.start_from(PyLong_AsUnsignedLongLongMask(a[3]));
   PyObject* out = PyList_New((Py_ssize_t)blocks);
-  if (!out) return nullptr;
-  for (long long b = 0; b < blocks; ++b) {
-    for (long long i = 0; i < bs; ++i) {
-      PyObject* item = PyList_GET_ITEM(a[0], (Py_ssize_t)(b * bs + i));
-      const long long v = PyLong_CheckExact(item) ? PyLong_AsLongLongAndOverflow(item, &overflow) : (overflow = 1, 0);
-      if (overflow) { Py_DECREF(out); NVJ_NONE(); }
-      words[(size_t)i + 1] = (uint64_t)v;
-    }
-    const uint64_t h = chained ? WordHash::of(words.data(), words.size()) : WordHash::of(words.data() + 1, words.size() - 1);
-    words[0] = h;
-    chained = true;
+  for (long long b = 0; out && b < blocks; ++b) {
+    uint64_t h;
+    if (!chain.next(b, &h)) { Py_DECREF(out); NVJ_NONE(); }
     PyObject* d = PyLong_FromUnsignedLongLong(h);
     if (!d) { Py_DECREF(out); return nullptr; }
     PyList_SET_ITEM(out, (Py_ssize_t)b, d);
@@ -588,53 +615,156 @@ PyObject* hash_chain(PyObject* const* a, Py_ssize_t n) {
 
 // ---- the block manager's walks ----------------------------------------------------------------------------------------
 
-PyObject *str_ref_count, *str_hash, *str_token_ids;  // attribute names of a block
+// A block's attributes.  Blocks are objects with __slots__: where the type has a plain slot of that name it is read and
+// written in place (15 ns less per access; a 96-block sequence has some 500 of them), else through the attribute.
+enum BlockField { kRefCount, kHash, kTokenIds, kBlockFields };
+PyObject* block_field_names[kBlockFields];
 
-// cached_run(token_ids, digests, block_size, published {digest: block id}, blocks, cacheable digests | None) -> (ids of the
-// published blocks of the longest reusable prefix, its digest | None): a block counts when it holds exactly these tokens.
+class BlockSlots {
+  PyTypeObject* type_ = nullptr;
+  Py_ssize_t at_[kBlockFields];
+
+  PyObject** slot(PyObject* block, BlockField f) {
+    if (Py_TYPE(block) != type_) {
+      Py_INCREF(Py_TYPE(block));
+      Py_XDECREF(type_);
+      type_ = Py_TYPE(block);
+      for (int k = 0; k < kBlockFields; ++k) {
+        PyObject* d = PyObject_GetAttr(reinterpret_cast<PyObject*>(type_), block_field_names[k]);
+        at_[k] = -1;
+        if (d && Py_IS_TYPE(d, &PyMemberDescr_Type)) {
+          const PyMemberDef* m = reinterpret_cast<PyMemberDescrObject*>(d)->d_member;
+          if (m->type == T_OBJECT_EX && !(m->flags & READONLY)) at_[k] = m->offset;
+        }
+        if (!d) PyErr_Clear();
+        Py_XDECREF(d);
+      }
+    }
+    return at_[f] < 0 ? nullptr : reinterpret_cast<PyObject**>(reinterpret_cast<char*>(block) + at_[f]);
+  }
+
+ public:
+  PyObject* get(PyObject* block, BlockField f) {  // a new reference
+    PyObject** p = slot(block, f);
+    if (!p || !*p) return PyObject_GetAttr(block, block_field_names[f]);
+    Py_INCREF(*p);
+    return *p;
+  }
+  bool set(PyObject* block, BlockField f, PyObject* v) {
+    PyObject** p = slot(block, f);
+    if (!p) return PyObject_SetAttr(block, block_field_names[f], v) == 0;
+    PyObject* old = *p;
+    Py_INCREF(v);
+    *p = v;
+    Py_XDECREF(old);
+    return true;
+  }
+} block_slots;
+
+PyObject* block_at(PyObject* blocks, PyObject* id) {  // borrowed; IndexError outside the pool
+  const long long at = PyLong_AsLongLong(id);
+  if (at >= 0 && at < PyList_GET_SIZE(blocks)) return PyList_GET_ITEM(blocks, (Py_ssize_t)at);
+  if (!PyErr_Occurred()) PyErr_SetString(PyExc_IndexError, "block outside the pool");
+  return nullptr;
+}
+
+int same_token(PyObject* x, PyObject* y) {
+  long long u, v;
+  if (x == y) return 1;
+  return int_of(x, &u) && int_of(y, &v) ? u == v : PyObject_RichCompareBool(x, y, Py_EQ);
+}
+
+// cached_run(token_ids, digests | None, block_size, full blocks, published {digest: block id}, blocks, cacheable digests |
+// None, used ids) -> (ids of the published blocks of the longest reusable prefix, its digest | None, how many of them are in
+// use): a block counts when it holds exactly these tokens.  Digests are taken as the walk needs them when none are given;
+// None when that meets tokens which are not machine-size integers.
 PyObject* cached_run(PyObject* const* a, Py_ssize_t n) {
-  if (!args_are(n, 6)) return nullptr;
-  const long long bs = PyLong_AsLongLong(a[2]);
+  if (!args_are(n, 8)) return nullptr;
+  const long long bs = PyLong_AsLongLong(a[2]), full = PyLong_AsLongLong(a[3]);
   if (PyErr_Occurred()) return nullptr;
-  if (!PyList_Check(a[0]) || !PyList_Check(a[1]) || !PyDict_Check(a[3]) || !PyList_Check(a[4]) || bs < 1 ||
-      PyList_GET_SIZE(a[1]) > PyList_GET_SIZE(a[0]) / bs) {
-    PyErr_SetString(PyExc_TypeError, "cached_run: lists and a dict expected");
+  const bool lazy = a[1] == Py_None;
+  if (!PyList_Check(a[0]) || (!lazy && (!PyList_Check(a[1]) || PyList_GET_SIZE(a[1]) < full)) || !PyDict_Check(a[4]) ||
+      !PyList_Check(a[5]) || !PyAnySet_Check(a[7]) || bs < 1 || full > PyList_GET_SIZE(a[0]) / bs) {
+    PyErr_SetString(PyExc_TypeError, "cached_run: lists, a dict and a set expected");
     return nullptr;
   }
-  PyObject* hits = PyList_New(0);
-  if (!hits) return nullptr;
+  HashChain chain(a[0], bs);
+  PyObject *hits = PyList_New(0), *best_digest = nullptr;
   Py_ssize_t best = 0;
-  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[1]); ++i) {
-    PyObject* digest = PyList_GET_ITEM(a[1], i);
-    PyObject* id = PyDict_GetItemWithError(a[3], digest);  // borrowed
-    if (!id) {
-      if (PyErr_Occurred()) { Py_DECREF(hits); return nullptr; }
-      break;
+  long long live = 0, best_live = 0;
+  bool ok = hits != nullptr, whole = true;
+  for (long long i = 0; ok && i < full; ++i) {
+    PyObject* digest;
+    if (lazy) {
+      uint64_t h;
+      if (!(whole = chain.next(i, &h))) break;
+      digest = PyLong_FromUnsignedLongLong(h);
+      if (!(ok = digest != nullptr)) break;
+    } else {
+      digest = PyList_GET_ITEM(a[1], (Py_ssize_t)i);
+      Py_INCREF(digest);
     }
-    const long long at = PyLong_AsLongLong(id);
-    if (at < 0 || at >= PyList_GET_SIZE(a[4])) {
-      if (!PyErr_Occurred()) PyErr_SetString(PyExc_IndexError, "published block outside the pool");
-      Py_DECREF(hits);
-      return nullptr;
+    PyObject* id = PyDict_GetItemWithError(a[4], digest);  // borrowed
+    PyObject* block = id ? block_at(a[5], id) : nullptr;
+    ok = block || (!id && !PyErr_Occurred());
+    int same = 0;
+    if (block) {
+      PyObject *hash = block_slots.get(block, kHash), *held = block_slots.get(block, kTokenIds);
+      same = hash && held ? PyObject_RichCompareBool(hash, digest, Py_EQ) : -1;
+      if (same == 1) same = PyList_Check(held) && PyList_GET_SIZE(held) == bs ? 1 : 0;
+      for (long long k = 0; same == 1 && k < bs; ++k)
+        same = same_token(PyList_GET_ITEM(held, (Py_ssize_t)k), PyList_GET_ITEM(a[0], (Py_ssize_t)(i * bs + k)));
+      Py_XDECREF(hash);
+      Py_XDECREF(held);
     }
-    PyObject* block = PyList_GET_ITEM(a[4], (Py_ssize_t)at);
-    PyObject *hash = PyObject_GetAttr(block, str_hash), *held = PyObject_GetAttr(block, str_token_ids);
-    int same = hash && held ? PyObject_RichCompareBool(hash, digest, Py_EQ) : -1;
-    if (same == 1) same = PyList_Check(held) && PyList_GET_SIZE(held) == bs ? 1 : 0;
-    for (long long k = 0; same == 1 && k < bs; ++k)
-      same = PyObject_RichCompareBool(PyList_GET_ITEM(held, (Py_ssize_t)k), PyList_GET_ITEM(a[0], (Py_ssize_t)(i * bs + k)), Py_EQ);
-    Py_XDECREF(hash);
-    Py_XDECREF(held);
-    if (same < 0 || (same == 1 && PyList_Append(hits, id) < 0)) { Py_DECREF(hits); return nullptr; }
-    if (!same) break;
-    const int usable = a[5] == Py_None ? 1 : PySequence_Contains(a[5], digest);
-    if (usable < 0) { Py_DECREF(hits); return nullptr; }
-    if (usable) best = i + 1;
+    if (same == 1) {
+      const int used = PySet_Contains(a[7], id), usable = a[6] == Py_None ? 1 : PySequence_Contains(a[6], digest);
+      if (used < 0 || usable < 0 || PyList_Append(hits, id) < 0) same = -1;
+      live += used > 0;
+      if (same == 1 && usable) {
+        best = (Py_ssize_t)i + 1;
+        best_live = live;
+        Py_XDECREF(best_digest);
+        Py_INCREF(digest);
+        best_digest = digest;
+      }
+    }
+    Py_DECREF(digest);
+    ok = ok && same >= 0;
+    if (same != 1) break;
   }
-  if (PyList_SetSlice(hits, best, PyList_GET_SIZE(hits), nullptr) < 0) { Py_DECREF(hits); return nullptr; }
-  PyObject* out = PyTuple_Pack(2, hits, best ? PyList_GET_ITEM(a[1], best - 1) : Py_None);
-  Py_DECREF(hits);
+  ok = ok && PyList_SetSlice(hits, best, PyList_GET_SIZE(hits), nullptr) == 0;
+  PyObject* out = nullptr;
+  if (ok && !whole) { Py_INCREF(Py_None); out = Py_None; }
+  else if (ok) out = Py_BuildValue("OOL", hits, best_digest ? best_digest : Py_None, best_live);
+  Py_XDECREF(hits);
+  Py_XDECREF(best_digest);
   return out;
+}
+
+// add_owner(blocks, ids, used) -> those of the ids that are not in use, which stay as they are
+PyObject* add_owner(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 3)) return nullptr;
+  if (!PyList_Check(a[0]) || !PyList_Check(a[1]) || !PyAnySet_Check(a[2])) {
+    PyErr_SetString(PyExc_TypeError, "add_owner: lists and a set expected");
+    return nullptr;
+  }
+  PyObject* idle = PyList_New(0);
+  for (Py_ssize_t k = 0; idle && k < PyList_GET_SIZE(a[1]); ++k) {
+    PyObject* id = PyList_GET_ITEM(a[1], k);
+    const int used = PySet_Contains(a[2], id);
+    bool ok = used == 0 ? PyList_Append(idle, id) == 0 : used == 1;
+    if (used == 1) {
+      PyObject* block = block_at(a[0], id);
+      PyObject* owners = block ? block_slots.get(block, kRefCount) : nullptr;
+      PyObject* more = owners ? PyLong_FromLongLong(PyLong_AsLongLong(owners) + 1) : nullptr;
+      ok = more && !PyErr_Occurred() && block_slots.set(block, kRefCount, more);
+      Py_XDECREF(owners);
+      Py_XDECREF(more);
+    }
+    if (!ok) Py_CLEAR(idle);
+  }
+  return idle;
 }
 
 // take_fresh(blocks, ids, first, digests, token_ids, block_size, published, no_hash): block ids[k] becomes block first + k of
@@ -651,14 +781,9 @@ PyObject* take_fresh(PyObject* const* a, Py_ssize_t n) {
   bool ok = one != nullptr;
   for (Py_ssize_t k = 0; ok && k < PyList_GET_SIZE(a[1]); ++k) {
     PyObject* id = PyList_GET_ITEM(a[1], k);
-    const long long at = PyLong_AsLongLong(id);
-    if (at < 0 || at >= PyList_GET_SIZE(a[0])) {
-      if (!PyErr_Occurred()) PyErr_SetString(PyExc_IndexError, "free block outside the pool");
-      ok = false;
-      break;
-    }
-    PyObject* block = PyList_GET_ITEM(a[0], (Py_ssize_t)at);
-    PyObject *owners = PyObject_GetAttr(block, str_ref_count), *old = PyObject_GetAttr(block, str_hash);
+    PyObject* block = block_at(a[0], id);
+    if (!(ok = block != nullptr)) break;
+    PyObject *owners = block_slots.get(block, kRefCount), *old = block_slots.get(block, kHash);
     ok = owners && old;
     if (ok && PyObject_IsTrue(owners) != 0) {
       PyErr_SetString(PyExc_AssertionError, "a free block has an owner");
@@ -678,9 +803,8 @@ PyObject* take_fresh(PyObject* const* a, Py_ssize_t n) {
     const long long index = first + k;
     const bool full = index < PyList_GET_SIZE(a[3]);
     PyObject* tokens = ok ? (full ? PyList_GetSlice(a[4], (Py_ssize_t)(index * bs), (Py_ssize_t)((index + 1) * bs)) : PyList_New(0)) : nullptr;
-    ok = ok && tokens && PyObject_SetAttr(block, str_ref_count, one) == 0 &&
-         PyObject_SetAttr(block, str_hash, full ? PyList_GET_ITEM(a[3], (Py_ssize_t)index) : a[7]) == 0 &&
-         PyObject_SetAttr(block, str_token_ids, tokens) == 0;
+    ok = ok && tokens && block_slots.set(block, kRefCount, one) &&
+         block_slots.set(block, kHash, full ? PyList_GET_ITEM(a[3], (Py_ssize_t)index) : a[7]) && block_slots.set(block, kTokenIds, tokens);
     Py_XDECREF(tokens);
   }
   Py_XDECREF(one);
@@ -695,21 +819,14 @@ PyObject* drop_owner(PyObject* const* a, Py_ssize_t n) {
   PyObject* gone = PyList_New(0);
   for (Py_ssize_t k = PyList_GET_SIZE(a[1]); gone && k-- > 0;) {
     PyObject* id = PyList_GET_ITEM(a[1], k);
-    const long long at = PyLong_AsLongLong(id);
-    bool ok = at >= 0 && at < PyList_GET_SIZE(a[0]);
-    if (ok) {
-      PyObject* block = PyList_GET_ITEM(a[0], (Py_ssize_t)at);
-      PyObject* owners = PyObject_GetAttr(block, str_ref_count);
-      const long long left = owners ? PyLong_AsLongLong(owners) - 1 : 0;
-      PyObject* fewer = owners && !PyErr_Occurred() ? PyLong_FromLongLong(left) : nullptr;
-      ok = fewer && PyObject_SetAttr(block, str_ref_count, fewer) == 0 && (left != 0 || PyList_Append(gone, id) == 0);
-      Py_XDECREF(owners);
-      Py_XDECREF(fewer);
-    }
-    if (!ok) {
-      if (!PyErr_Occurred()) PyErr_SetString(PyExc_IndexError, "block outside the pool");
-      Py_CLEAR(gone);
-    }
+    PyObject* block = block_at(a[0], id);
+    PyObject* owners = block ? block_slots.get(block, kRefCount) : nullptr;
+    const long long left = owners ? PyLong_AsLongLong(owners) - 1 : 0;
+    PyObject* fewer = owners && !PyErr_Occurred() ? PyLong_FromLongLong(left) : nullptr;
+    const bool ok = fewer && block_slots.set(block, kRefCount, fewer) && (left != 0 || PyList_Append(gone, id) == 0);
+    Py_XDECREF(owners);
+    Py_XDECREF(fewer);
+    if (!ok) Py_CLEAR(gone);
   }
   return gone;
 }
@@ -858,6 +975,7 @@ PyMethodDef methods[] = {
     NVJ_FAST(norm_rope, "norm + rope + append, or None"),
     NVJ_FAST(decode_shape, "batch, query length and table width of a decode batch, or None"),
     NVJ_FAST(cached_run, "published blocks of a sequence's longest reusable prefix"),
+    NVJ_FAST(add_owner, "a sequence shares blocks that are in use"),
     NVJ_FAST(take_fresh, "free blocks become a sequence's"),
     NVJ_FAST(drop_owner, "a sequence gives its blocks up"),
     NVJ_FAST(hash_chain, "chained digests of a token list's blocks, or None"),
@@ -875,8 +993,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_nvj_host", "Host side of the hot 
 }  // namespace
 
 PyMODINIT_FUNC PyInit__nvj_host(void) {
-  str_ref_count = PyUnicode_InternFromString("ref_count");
-  str_hash = PyUnicode_InternFromString("hash");
-  str_token_ids = PyUnicode_InternFromString("token_ids");
-  return str_ref_count && str_hash && str_token_ids ? PyModule_Create(&module) : nullptr;
+  const char* names[kBlockFields] = {"ref_count", "hash", "token_ids"};
+  for (int k = 0; k < kBlockFields; ++k)
+    if (!(block_field_names[k] = PyUnicode_InternFromString(names[k]))) return nullptr;
+  return PyModule_Create(&module);
 }

@@ -15,7 +15,6 @@ prefix exists) followed by the token ids as native int64 bytes.
 
 from __future__ import annotations
 
-from collections import deque
 from typing import Dict, Iterable, List, Optional, Set
 
 import numpy as np
@@ -53,72 +52,84 @@ class Block:
 class _FreeList:
     """FIFO of free block ids with O(1) removal of an arbitrary id.
 
-    A queue in order and a set of what is free.  Removing an id from the middle (a cached block is taken again: rare)
-    leaves its entry in the queue as a stale one, which the head skips when it gets there; an id's stale entries always
-    lie in front of its live one.  (An ordered dictionary popped one item at a time took four times as long.)
+    A list and the index of its head, so that a sequence's blocks leave it as one slice and come back as one.  Removing an id
+    from the middle (a cached block is taken again: rare) leaves its entry in the queue as a stale one, which the head skips
+    when it gets there; an id's stale entries always lie in front of its live one.  Callers add only ids that are not free and
+    remove only free ones: an id is free exactly when its block has no owner.
     """
 
     def __init__(self, ids: Iterable[int]):
-        self._queue = deque(ids)
-        self._free = set(self._queue)
-        self._stale: Dict[int, int] = {}
+        self._queue: List[int] = list(ids)
+        self._head = 0
+        self._stale: Dict[int, int] = {}  # id -> entries to skip
+        self._len = len(self._queue)
 
     def __len__(self) -> int:
-        return len(self._free)
+        return self._len
 
     def __contains__(self, block_id: int) -> bool:
-        return block_id in self._free
+        return block_id in iter(self)
 
     def __iter__(self):
         stale = dict(self._stale)
-        for block_id in self._queue:
+        for block_id in self._queue[self._head:]:
             if stale.get(block_id, 0) > 0:
                 stale[block_id] -= 1
             else:
                 yield block_id
 
+    def _advance(self, n: int) -> None:
+        self._head += n
+        if self._head > 256 and 2 * self._head > len(self._queue):
+            del self._queue[:self._head]
+            self._head = 0
+
     def _skip_stale(self) -> None:
-        queue, stale = self._queue, self._stale
-        while stale and queue:
-            n = stale.get(queue[0], 0)
+        stale = self._stale
+        while stale and self._head < len(self._queue):
+            block_id = self._queue[self._head]
+            n = stale.get(block_id, 0)
             if n == 0:
                 return
             if n == 1:
-                del stale[queue[0]]
+                del stale[block_id]
             else:
-                stale[queue[0]] = n - 1
-            queue.popleft()
+                stale[block_id] = n - 1
+            self._advance(1)
 
     def __getitem__(self, index: int) -> int:
         if index != 0:
             raise IndexError("only the head of the free list is addressable")
-        if not self._free:
+        if not self._len:
             raise StopIteration("no free block left")
         self._skip_stale()
-        return self._queue[0]
+        return self._queue[self._head]
 
     def remove(self, block_id: int) -> None:
-        self._free.remove(block_id)
+        self._len -= 1
         self._stale[block_id] = self._stale.get(block_id, 0) + 1
 
     def append(self, block_id: int) -> None:
-        self.extend((block_id,))
+        self._queue.append(block_id)
+        self._len += 1
 
-    def extend(self, block_ids: Iterable[int]) -> None:
-        fresh = [i for i in block_ids if i not in self._free]
-        self._queue.extend(fresh)
-        self._free.update(fresh)
+    def extend(self, block_ids: List[int]) -> None:
+        self._queue.extend(block_ids)
+        self._len += len(block_ids)
 
     def take(self, n: int) -> List[int]:
         """Remove and return the first n ids; StopIteration, and nothing removed, when there are fewer."""
-        if n > len(self._free):
+        if n > self._len:
             raise StopIteration("no free block left")
-        pop, out = self._queue.popleft, []
+        out: List[int] = []
         while self._stale and len(out) < n:
             self._skip_stale()
-            out.append(pop())
-        out.extend([pop() for _ in range(n - len(out))])
-        self._free.difference_update(out)
+            out.append(self._queue[self._head])
+            self._advance(1)
+        rest = n - len(out)
+        out += self._queue[self._head:self._head + rest]
+        self._advance(rest)
+        self._len -= n
         return out
 
 
@@ -203,19 +214,22 @@ class BlockManager:
         chained digest is in the set (hybrid models need the GDN state of exactly
         that prefix).
         """
-        hits, best_hash = self._cached_run(seq, self._digests(seq), cacheable_hashes)
+        hits, best_hash, _ = self._cached_run(seq, cacheable_hashes)
         return len(hits) * self.block_size, best_hash
 
-    def _cached_run(self, seq, digests, cacheable_hashes):
-        """(ids of the published blocks of the longest reusable prefix, its digest)."""
+    def _cached_run(self, seq, cacheable_hashes, digests=None):
+        """(ids of the published blocks of the longest reusable prefix, its digest, how many of them a live sequence holds).
+        Without `digests` the walk takes them as far as it goes, which is one block beyond the published ones."""
         tokens = seq.token_ids if type(seq.token_ids) is list else list(seq.token_ids)
-        return _host.cached_run(tokens, digests, self.block_size, self.hash_to_block_id, self.blocks, cacheable_hashes)
+        full = min(seq.num_tokens, len(tokens)) // self.block_size
+        run = _host.cached_run(tokens, digests, self.block_size, full, self.hash_to_block_id, self.blocks, cacheable_hashes,
+                               self.used_block_ids)
+        return self._cached_run(seq, cacheable_hashes, self._digests(seq)) if run is None else run
 
     def _num_required_blocks(self, seq, *, use_prefix_cache=True, cacheable_hashes=None) -> int:
         need = self._num_blocks(seq)
         if use_prefix_cache:
-            hits, _ = self._cached_run(seq, self._digests(seq), cacheable_hashes)
-            need -= sum(1 for bid in hits if bid in self.used_block_ids)  # shared with a live sequence: costs no free block
+            need -= self._cached_run(seq, cacheable_hashes)[2]  # shared with a live sequence: costs no free block
         return need
 
     def can_allocate(self, seq, *, use_prefix_cache=True, cacheable_hashes=None) -> bool:
@@ -231,14 +245,11 @@ class BlockManager:
         seq.cached_prefix_hybrid_seeded = False
         seq.prefix_cache_enabled = bool(use_prefix_cache)
         digests = self._digests(seq)
-        hits, cached_hash = self._cached_run(seq, digests, cacheable_hashes) if use_prefix_cache else ([], None)
+        hits, cached_hash, _ = self._cached_run(seq, cacheable_hashes, digests) if use_prefix_cache else ([], None, 0)
         blocks, used, free, bs, tokens, table = (self.blocks, self.used_block_ids, self.free_block_ids, self.block_size,
                                                  seq.token_ids, seq.block_table)
-        for bid in hits:
-            if bid in used:
-                blocks[bid].ref_count += 1
-            else:
-                self._take_cached(bid)
+        for bid in _host.add_owner(blocks, hits, used):
+            self._take_cached(bid)
         table.extend(hits)
         seq.num_cached_tokens = len(hits) * bs
         first = len(hits)
