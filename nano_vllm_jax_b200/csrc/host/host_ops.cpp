@@ -835,8 +835,11 @@ PyObject* drop_owner(PyObject* const* a, Py_ssize_t n) {
 
 // One int32 out of a Python integer (anything with __index__); false with OverflowError or TypeError set.
 bool as_i32(PyObject* o, int32_t* v) {
-  const long long x = PyLong_AsLongLong(o);
-  if (x == -1 && PyErr_Occurred()) return false;
+  long long x;
+  if (!int_of(o, &x)) {
+    x = PyLong_AsLongLong(o);
+    if (x == -1 && PyErr_Occurred()) return false;
+  }
   if (x < INT32_MIN || x > INT32_MAX) {
     PyErr_SetString(PyExc_OverflowError, "a batch entry does not fit 32 bits");
     return false;
@@ -845,54 +848,101 @@ bool as_i32(PyObject* o, int32_t* v) {
   return true;
 }
 
-// pack_i32(address, words, parts, rows_at, rows, width) -> tuple of the rows, padded with zeros to `width`.
-// Fills `words` int32 at `address` (a pinned staging buffer): zeros, then every part (offset, list of ints), then the lists
-// in `rows` as a [len(rows), width] table at `rows_at`.
-PyObject* pack_i32(PyObject* const* a, Py_ssize_t n) {
-  if (!args_are(n, 6)) return nullptr;
-  int32_t* base = reinterpret_cast<int32_t*>(PyLong_AsUnsignedLongLong(a[0]));
-  const long long words = PyLong_AsLongLong(a[1]), rows_at = PyLong_AsLongLong(a[3]), width = PyLong_AsLongLong(a[5]);
-  if (PyErr_Occurred()) return nullptr;
-  if (!base || words < 0 || !PyList_Check(a[2]) || !PyList_Check(a[4]) || width < 0 || rows_at < 0 ||
-      rows_at + PyList_GET_SIZE(a[4]) * width > words) {
-    PyErr_SetString(PyExc_ValueError, "pack_i32: the parts do not fit the buffer");
-    return nullptr;
-  }
-  std::memset(base, 0, (size_t)words * sizeof(int32_t));
-  for (Py_ssize_t p = 0; p < PyList_GET_SIZE(a[2]); ++p) {
-    PyObject *part = PyList_GET_ITEM(a[2], p), *list;
-    long long at;
-    if (!PyArg_ParseTuple(part, "LO!", &at, &PyList_Type, &list)) return nullptr;
-    const Py_ssize_t len = PyList_GET_SIZE(list);
-    if (at < 0 || at + len > words) {
-      PyErr_SetString(PyExc_ValueError, "pack_i32: the parts do not fit the buffer");
-      return nullptr;
-    }
-    for (Py_ssize_t i = 0; i < len; ++i)
-      if (!as_i32(PyList_GET_ITEM(list, i), base + at + i)) return nullptr;
-  }
-  const Py_ssize_t rows = PyList_GET_SIZE(a[4]);
-  PyObject* zero = PyLong_FromLong(0);
-  PyObject* out = PyTuple_New(rows);
-  for (Py_ssize_t r = 0; out && r < rows; ++r) {
-    PyObject* list = PyList_GET_ITEM(a[4], r);
-    PyObject* row = PyList_Check(list) && PyList_GET_SIZE(list) <= width ? PyTuple_New((Py_ssize_t)width) : nullptr;
+bool fill_i32(PyObject* list, int32_t* to) {
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i)
+    if (!as_i32(PyList_GET_ITEM(list, i), to + i)) return false;
+  return true;
+}
+
+// The block tables `rows`, padded with zeros to `width`: as int32 to `to` (zeros already), as a tuple of tuples in return.
+PyObject* fill_tables(PyObject* rows, Py_ssize_t width, int32_t* to) {
+  PyObject *zero = PyLong_FromLong(0), *out = PyTuple_New(PyList_GET_SIZE(rows));
+  for (Py_ssize_t r = 0; out && r < PyList_GET_SIZE(rows); ++r, to += width) {
+    PyObject* list = PySequence_Fast(PyList_GET_ITEM(rows, r), "a block table is a sequence");
+    PyObject* row = list && PySequence_Fast_GET_SIZE(list) <= width ? PyTuple_New(width) : nullptr;
     if (!row) {
-      if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "pack_i32: a row is no list or too long");
+      if (!PyErr_Occurred())
+        PyErr_Format(PyExc_ValueError, "scheduled block table needs %zd blocks but bucket has %zd", PySequence_Fast_GET_SIZE(list), width);
+      Py_XDECREF(list);
       Py_CLEAR(out);
       break;
     }
     PyTuple_SET_ITEM(out, r, row);
-    const Py_ssize_t len = PyList_GET_SIZE(list);
-    for (Py_ssize_t i = 0; i < (Py_ssize_t)width; ++i) {
-      PyObject* item = i < len ? PyList_GET_ITEM(list, i) : zero;
-      if (i < len && !as_i32(item, base + rows_at + r * width + i)) { Py_CLEAR(out); break; }
+    const Py_ssize_t len = PySequence_Fast_GET_SIZE(list);
+    bool ok = true;
+    for (Py_ssize_t i = 0; ok && i < len; ++i) {
+      PyObject* item = PySequence_Fast_GET_ITEM(list, i);
+      if (!(ok = as_i32(item, to + i))) break;
       if (PyLong_CheckExact(item)) Py_INCREF(item);
-      else item = PyLong_FromLong(base[rows_at + r * width + i]);
+      else ok = (item = PyLong_FromLong(to[i])) != nullptr;
       PyTuple_SET_ITEM(row, i, item);
     }
+    for (Py_ssize_t i = len; ok && i < width; ++i) {
+      Py_INCREF(zero);
+      PyTuple_SET_ITEM(row, i, zero);
+    }
+    Py_DECREF(list);
+    if (!ok) Py_CLEAR(out);
   }
-  Py_DECREF(zero);
+  Py_XDECREF(zero);
+  return out;
+}
+
+// pack_batch(parts, rows, width, device index | -1) -> ([a tensor per part], the [len(rows), width] table, the same table as a
+// tuple of tuples).  A part is (list of ints, shape); what the list does not fill of its shape is zero.  All of it is written
+// into one staging buffer (pinned for a GPU) and crosses in one copy; the tensors are views of the one device buffer.
+PyObject* pack_batch(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 4)) return nullptr;
+  const long long width = PyLong_AsLongLong(a[2]), device = PyLong_AsLongLong(a[3]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!PyList_Check(a[0]) || !PyList_Check(a[1]) || width < 0) {
+    PyErr_SetString(PyExc_TypeError, "pack_batch: lists expected");
+    return nullptr;
+  }
+  struct Part { PyObject* list; int64_t shape[2], at; int dims; };
+  std::vector<Part> parts((size_t)PyList_GET_SIZE(a[0]));
+  int64_t total = 0;
+  for (size_t k = 0; k < parts.size(); ++k) {
+    Part& p = parts[k];
+    PyObject *entry = PyList_GET_ITEM(a[0], (Py_ssize_t)k), *shape;
+    if (!PyArg_ParseTuple(entry, "O!O!", &PyList_Type, &p.list, &PyTuple_Type, &shape)) return nullptr;
+    p.dims = (int)PyTuple_GET_SIZE(shape);
+    p.at = total;
+    int64_t count = 1;
+    for (int d = 0; d < p.dims && d < 2; ++d) {
+      p.shape[d] = PyLong_AsLongLong(PyTuple_GET_ITEM(shape, d));
+      if (PyErr_Occurred()) return nullptr;
+      count *= p.shape[d];
+    }
+    if (p.dims < 1 || p.dims > 2 || count < PyList_GET_SIZE(p.list)) {
+      PyErr_SetString(PyExc_ValueError, "pack_batch: a part is longer than its shape");
+      return nullptr;
+    }
+    total += count;
+  }
+  const int64_t rows = PyList_GET_SIZE(a[1]), rows_at = total;
+  total += rows * width;
+  at::AutoDispatchBelowADInplaceOrView plain;  // integers: nothing here is differentiable
+  at::Tensor stage = at::empty({total > 0 ? total : 1}, at::TensorOptions(at::kInt).pinned_memory(device >= 0));
+  int32_t* words = static_cast<int32_t*>(stage.data_ptr());
+  std::memset(words, 0, (size_t)total * sizeof(int32_t));
+  for (const Part& p : parts)
+    if (!fill_i32(p.list, words + p.at)) return nullptr;
+  PyObject* host = fill_tables(a[1], (Py_ssize_t)width, words + rows_at);
+  if (!host) return nullptr;
+  at::Tensor dev = stage;
+  if (device >= 0) {
+    dev = empty(stage.sizes(), at::kInt, (int)device);
+    dev.copy_(stage, /*non_blocking=*/true);
+  }
+  PyObject* views = PyList_New((Py_ssize_t)parts.size());
+  for (size_t k = 0; views && k < parts.size(); ++k) {
+    const Part& p = parts[k];
+    const int64_t strides[2] = {p.dims == 2 ? p.shape[1] : 1, 1};
+    PyList_SET_ITEM(views, (Py_ssize_t)k, THPVariable_Wrap(dev.as_strided({p.shape, (size_t)p.dims}, {strides, (size_t)p.dims}, p.at)));
+  }
+  PyObject* out = views ? Py_BuildValue("NNN", views, THPVariable_Wrap(dev.as_strided({rows, width}, {width, 1}, rows_at)), host) : nullptr;
+  if (!views) Py_DECREF(host);
   return out;
 }
 
@@ -982,7 +1032,7 @@ PyMethodDef methods[] = {
     NVJ_FAST(stage_in, "a step's operands to the device on two streams, or None"),
     NVJ_FAST(copy_blocks, "cache[:, dst] = cache[:, src], or None"),
     NVJ_FAST(hybrid_copy, "snapshot or restore of GDN state rows, or None"),
-    NVJ_FAST(pack_i32, "fill a staging buffer with a batch's lists"),
+    NVJ_FAST(pack_batch, "a batch's lists on the device"),
     NVJ_FAST(slot_mapping, "flat cache slots of positions, or None"),
     {"init", init, METH_VARARGS, "resolve the library's entry points and keep the callbacks"},
     {"set_workspace", set_workspace, METH_VARARGS, "hand over a (device, stream)'s workspace"},

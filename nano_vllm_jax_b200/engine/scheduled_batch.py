@@ -14,7 +14,6 @@ pinned array and one copy per field took 0.4 ms for a 34-row mixed batch).
 
 from __future__ import annotations
 
-import math
 from dataclasses import dataclass
 from itertools import accumulate
 from typing import List, Optional, Sequence as Seq
@@ -23,7 +22,7 @@ import torch
 
 from .. import _lib
 
-_pack_i32 = _lib.host_module().pack_i32
+_pack_batch = _lib.host_module().pack_batch
 
 
 @dataclass
@@ -59,26 +58,18 @@ def _to_device(parts, tables, width, device):
     """The batch's int32 arrays on the device, from one staging buffer and one copy: `parts` is a list of (list of ints,
     shape), `tables` the rows' block tables (padding rows empty lists).  Returns (tensors of the parts, the [rows, width]
     table, the table as a tuple of tuples)."""
-    for t in tables:
-        if len(t) > width:
-            raise ValueError(f"scheduled block table needs {len(t)} blocks but bucket has {width}")
-    cuda = torch.device(device).type == "cuda"
-    sizes = [math.prod(shape) for _, shape in parts]
-    sizes.append(len(tables) * width)
-    entries, at = [], 0
-    for (values, _), n in zip(parts, sizes):
-        entries.append((at, values))
-        at += n
-    total = at + sizes[-1]
-    stage = torch.empty(max(total, 1), dtype=torch.int32, pin_memory=cuda)
-    host_tables = _pack_i32(stage.data_ptr(), total, entries, at, tables, width)
-    dev = stage.to(device, non_blocking=True) if cuda else stage
-    arrays = [t if len(shape) == 1 else t.view(shape) for t, (_, shape) in zip(dev[:total].split(sizes), parts)]
-    return arrays, dev[at:total].view(len(tables), width), host_tables
+    device = torch.device(device)
+    index = -1
+    if device.type == "cuda":
+        torch.cuda.init()
+        index = torch.cuda.current_device() if device.index is None else device.index
+    return _pack_batch(parts, tables, width, index)
 
 
-def _table_lists(seqs, pad_rows: int):
-    return [s.block_table if type(s.block_table) is list else list(s.block_table) for s in seqs] + [[]] * pad_rows
+def _tables(seqs, width: Optional[int]):
+    """The rows' block tables, and the width of the batch's table: the given one or that of the longest."""
+    tables = [s.block_table for s in seqs]
+    return tables, width or max(1, max(map(len, tables)))
 
 
 def build_decode_batch(seqs, *, max_blocks_per_seq: Optional[int] = None,
@@ -88,7 +79,7 @@ def build_decode_batch(seqs, *, max_blocks_per_seq: Optional[int] = None,
     bucket = n if batch_size_bucket is None else batch_size_bucket
     if n > bucket:
         raise ValueError(f"scheduled batch has {n} seqs but bucket has {bucket}")
-    width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
+    tables, width = _tables(seqs, max_blocks_per_seq)
     pad = bucket - n
     zeros = [0] * pad
     lens = [s.num_tokens for s in seqs] + zeros
@@ -96,14 +87,14 @@ def build_decode_batch(seqs, *, max_blocks_per_seq: Optional[int] = None,
     (tokens, positions, seq_lens, qsl, ids), tab, host_tables = _to_device(
         [([s.last_token for s in seqs] + zeros, (bucket, 1)), ([s.num_tokens - 1 for s in seqs] + zeros, (bucket, 1)),
          (lens, (bucket,)), (list(range(n + 1)) + [n] * pad, (bucket + 1,)), (seq_ids, (bucket,))],
-        _table_lists(seqs, pad), width, device)
+        tables + [[]] * pad, width, device)
     return ScheduledBatch(
         tokens=tokens, positions=positions, seq_ids=ids, query_start_loc=qsl, is_prefill=False, num_prefill_tokens=0,
         num_decode_tokens=n, block_tables=tab, seq_lens=seq_lens, seq_ids_host=tuple(seq_ids),
         query_lens_host=tuple([1] * n + zeros), seq_lens_host=tuple(lens), block_tables_host=host_tables)
 
 
-def _pack(toks, pos, qlens, seqs, lens, finals, *, width, bucket_rows, token_bucket, device, mixed=False) -> ScheduledBatch:
+def _pack(toks, pos, qlens, seqs, lens, finals, *, max_blocks, bucket_rows, token_bucket, device, mixed=False) -> ScheduledBatch:
     """A packed batch from its rows' tokens and positions, laid end to end (row r has qlens[r] of them)."""
     actual = len(toks)
     if actual <= 0:
@@ -114,6 +105,7 @@ def _pack(toks, pos, qlens, seqs, lens, finals, *, width, bucket_rows, token_buc
     pad_rows = bucket_rows - len(seqs)
     if pad_rows < 0:
         raise ValueError(f"scheduled batch has {len(seqs)} seqs but bucket has {bucket_rows}")
+    tables, width = _tables(seqs, max_blocks)
     rid = []
     for r, n in enumerate(qlens):
         if n == 1:
@@ -127,7 +119,7 @@ def _pack(toks, pos, qlens, seqs, lens, finals, *, width, bucket_rows, token_buc
     row = (1, token_bucket)  # (the staging buffer starts as zeros: token 0, position 0, row 0 behind the last real token)
     (tokens, positions, ids, qsl_dev, lens_dev, rids), tab, host_tables = _to_device(
         [(toks, row), (pos, row), (seq_ids, (bucket_rows,)), (qsl, (bucket_rows + 1,)), (lens, (bucket_rows,)), (rid, row)],
-        _table_lists(seqs, pad_rows), width, device)
+        tables + [[]] * pad_rows, width, device)
     return ScheduledBatch(
         tokens=tokens, positions=positions, seq_ids=ids, query_start_loc=qsl_dev, is_prefill=True, num_prefill_tokens=actual,
         num_decode_tokens=0, block_tables=tab, seq_lens=lens_dev, prefill_is_final=list(finals), seq_ids_host=tuple(seq_ids),
@@ -155,8 +147,7 @@ def build_packed_prefill_batch(seqs, prefill_chunk_lens: Optional[Seq[int]] = No
         if chunk <= 0:
             raise ValueError(f"Scheduled sequence {s.seq_id} has no executable tokens")
         _add_row(toks, pos, qlens, lens, finals, s, start, start + chunk)
-    width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
-    return _pack(toks, pos, qlens, seqs, lens, finals, width=width,
+    return _pack(toks, pos, qlens, seqs, lens, finals, max_blocks=max_blocks_per_seq,
                  bucket_rows=len(seqs) if batch_size_bucket is None else batch_size_bucket,
                  token_bucket=token_bucket, device=device)
 
@@ -183,7 +174,6 @@ def build_mixed_prefill_decode_batch(*, decode_seqs, prefill_seqs, prefill_chunk
             raise ValueError(f"Scheduled sequence {s.seq_id} has no executable prefill tokens")
         _add_row(toks, pos, qlens, lens, finals, s, start, start + chunk)
     seqs = list(decode_seqs) + list(prefill_seqs)
-    width = max_blocks_per_seq or max(1, max(len(s.block_table) for s in seqs))
-    return _pack(toks, pos, qlens, seqs, lens, finals, width=width,
+    return _pack(toks, pos, qlens, seqs, lens, finals, max_blocks=max_blocks_per_seq,
                  bucket_rows=len(seqs) if batch_size_bucket is None else batch_size_bucket,
                  token_bucket=token_bucket, device=device, mixed=True)
