@@ -79,14 +79,18 @@ struct DecodeParams {
   float scale;
 };
 
-// Keys row b attends: seq_lens[b], clipped to what its page list can hold.
+// Keys row b attends: seq_lens[b], clipped to what its page list can hold.  kWindow: the call may limit them further (a kernel
+// without a spare register pays 1% for code that a decode step never reaches).
+template <bool kWindow = true>
 __device__ __forceinline__ int decode_row_len(const DecodeParams& p, int b) {
   int len = p.seq_lens[b];
   if (p.pre_append && len > 0) ++len;
-  if (p.max_len > 0) len = len < p.max_len ? len : p.max_len;
-  if (p.cap_positions) {
-    const int cap = p.cap_positions[b] + 1;
-    len = len < cap ? len : cap;
+  if constexpr (kWindow) {
+    if (p.max_len > 0) len = len < p.max_len ? len : p.max_len;
+    if (p.cap_positions) {
+      const int cap = p.cap_positions[b] + 1;
+      len = len < cap ? len : cap;
+    }
   }
   if (p.packed_rows) {
     const int i = p.query_start_loc[b];

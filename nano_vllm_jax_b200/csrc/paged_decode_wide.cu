@@ -322,7 +322,9 @@ __device__ __forceinline__ void w_finish_segment(const DecodeParams& p, WideSmem
   if (tid == 0) p.counters[s.b] = 0;
 }
 
-template <bool kDual>
+// kWindow: decode_row_len.  A decode step has no window: 128 rows of 8192 - 32768 keys take 784 us (886 once the power cap is
+// reached) without the limits compiled in and 793 (898) with them.
+template <bool kDual, bool kWindow>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
 decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, DecodeParams p) {
   extern __shared__ unsigned char w_smem_raw[];
@@ -351,7 +353,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   for (int base = 0; base < p.batch; base += kDecodeThreads) {
     const int b = base + threadIdx.x;
     int len = 0;
-    if (b < p.batch) len = decode_row_len(p, b);
+    if (b < p.batch) len = decode_row_len<kWindow>(p, b);
     if (base == 0) first_n = blocks_in_sequence(p, (len + kBlk - 1) / kBlk);
     mine += blocks_in_sequence(p, (len + kBlk - 1) / kBlk);
     // rows without keys get zeros; in a packed batch only the rows this pass owns (one query token) are touched
@@ -384,7 +386,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   for (int base = 0; base < p.batch && carry <= g0; base += kDecodeThreads) {
     const int b = base + threadIdx.x;
     int n = 0;
-    if (b < p.batch) n = blocks_in_sequence(p, (decode_row_len(p, b) + kBlk - 1) / kBlk);
+    if (b < p.batch) n = blocks_in_sequence(p, (decode_row_len<kWindow>(p, b) + kBlk - 1) / kBlk);
     int chunk_total = 0;
     const long long excl = carry + cta_inclusive_scan(n, sm.scan, chunk_total) - n;
     if (n > 0 && excl <= g0 && g0 < excl + n) { sm.start_b = b; sm.start_j = (int)(g0 - excl); }
@@ -399,7 +401,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   }
   __syncthreads();
   NVJ_PHASE(2);
-  const int n_iters = blocks_in_range(p, sm.start_b, sm.start_j, g0, g1);  // the range's real blocks
+  const int n_iters = blocks_in_range<kWindow>(p, sm.start_b, sm.start_j, g0, g1);  // the range's real blocks
   if (n_iters == 0) return;
 #ifdef NVJ_PHASE_TIMING
   {
@@ -414,7 +416,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
 
   FillState fs;
   fs.b = sm.start_b; fs.jn = sm.start_j; fs.g = g0; fs.j = 0; fs.nsegs = 0; fs.has = false;
-  fill_ring(p, sm, fs, g1, 0, n_iters < kRing ? n_iters : kRing);
+  fill_ring<kWindow>(p, sm, fs, g1, 0, n_iters < kRing ? n_iters : kRing);
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int n = 0; n < kWStages && n < n_iters; ++n) w_issue_block(p, sm, &k_map, &v_map, n, false);
@@ -429,7 +431,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   const int fg = lane >> 2, ft = lane & 3;
   const float c = p.scale * kLog2e;
   WideState st;
-  while (next_seg(p, b, j, g, g1, s)) {
+  while (next_seg<kWindow>(p, b, j, g, g1, s)) {
     // query rows of this KV head as A fragments: row = token * 4 + head of the group; rows past the width are zero
     // (packed_rows: the row's single query token sits at query_start_loc[b]; its length is already capped by its position)
     const long long qbase = p.packed_rows ? (long long)p.query_start_loc[s.b] : (long long)s.b * p.width;
@@ -483,7 +485,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
       if ((it & (kRing / 2 - 1)) == 0 && it > 0) {
         named_bar_sync(1, kDecodeThreads);
         const int n0 = it + kRing / 2;
-        if (n0 < n_iters) fill_ring(p, sm, fs, g1, n0, n_iters - n0 < kRing / 2 ? n_iters - n0 : kRing / 2);
+        if (n0 < n_iters) fill_ring<kWindow>(p, sm, fs, g1, n0, n_iters - n0 < kRing / 2 ? n_iters - n0 : kRing / 2);
         named_bar_sync(1, kDecodeThreads);
       }
       if (!kDual && (it & 1) != par) continue;
@@ -641,12 +643,14 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
   static PerDeviceFlags smem_opted_in;
   const int smem = (int)sizeof(WideSmem) + 1024;
   if (!once_per_device(smem_opted_in, [smem](int) {
-        return cudaFuncSetAttribute(decode_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-               cudaFuncSetAttribute(decode_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+        return cudaFuncSetAttribute(decode_wide_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+               cudaFuncSetAttribute(decode_wide_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+               cudaFuncSetAttribute(decode_wide_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
       }))
     return NVJ_ERR_LAUNCH;
-  if (p.width > 4) launch_after(decode_wide_kernel<true>, n, kDecodeThreads, smem, stream, k_map, v_map, q);
-  else launch_after(decode_wide_kernel<false>, n, kDecodeThreads, smem, stream, k_map, v_map, q);
+  const bool window = p.max_len > 0 || p.cap_positions;
+  auto* kernel = p.width > 4 ? decode_wide_kernel<true, true> : window ? decode_wide_kernel<false, true> : decode_wide_kernel<false, false>;
+  launch_after(kernel, n, kDecodeThreads, smem, stream, k_map, v_map, q);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
