@@ -553,6 +553,17 @@ int nvj_selftest_bounded_wait(int32_t* status, int32_t* returned, nvj_stream_t s
 int nvj_copy_many_async(void* const* dst, const void* const* src, const size_t* bytes, int n,
                         nvj_stream_t stream);
 
+/*
+ * The same n copies out of pinned host memory in one kernel launch, for a step whose copies would take longer one by one than
+ * the kernel they feed.  NVJ_ERR_UNSUPPORTED, and nothing issued, when n > 8, a source is not pinned host memory, an
+ * address is not a multiple of 16 bytes or a size not one of 4.  The kernel needs room on the SMs: beside one that fills them (the streaming
+ * decode kernels) it waits for that to end.  No counterpart in the reference.
+ */
+int nvj_stage_in(void* const* dst, const void* const* src, const size_t* bytes, int n, nvj_stream_t stream);
+
+/* 1 when nvj_paged_decode* serves a bf16 batch of this size with the cluster kernel, else 0. */
+int nvj_paged_decode_on_clusters(int batch, int table_width);
+
 /* ------------------------------------------------------------------ tokens */
 
 /*

@@ -96,6 +96,8 @@ SIGNATURES = {
     "nvj_selftest_bounded_wait": (c_int, [c_void_p, c_void_p, c_void_p]),
     "nvj_paged_prefill_workspace_bytes": (c_size_t, [c_int]),
     "nvj_copy_many_async": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
+    "nvj_stage_in": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
+    "nvj_paged_decode_on_clusters": (c_int, [c_int, c_int]),
     "nvj_row_argmax": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "nvj_row_argmax_advance": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),
 }

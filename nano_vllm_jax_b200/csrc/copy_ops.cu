@@ -401,6 +401,100 @@ extern "C" int nvj_copy_many_async(void* const* dst, const void* const* src, con
   return NVJ_OK;
 }
 
+namespace nvj {
+
+// A step's operands out of pinned host memory, all of them in one launch.  Bound by the PCIe round trip (~2 us) and rate: every
+// thread has four 16-byte loads in flight, a CTA 16 KiB, and 28 CTAs ask for the 460 KB of a 64-row step at once.  Six copies by
+// the copy engines took 42 us on two streams, most of it the engines' latency per copy; this takes ~14.  The loads are volatile:
+// the host writes these buffers between the launches.
+constexpr int kStageMost = 8, kStageThreads = 256, kStagePer = 4, kStageCtas = 64;
+struct StageList {
+  const uint4* src[kStageMost];
+  uint4* dst[kStageMost];
+  long long end[kStageMost];  // 16-byte pieces of the pairs up to this one
+  int last_words[kStageMost];  // 4-byte words of the pair's last piece
+  int n;
+};
+__global__ void __launch_bounds__(kStageThreads) stage_in_kernel(const __grid_constant__ StageList list) {
+  const long long pieces = list.end[list.n - 1];
+  constexpr long long kSpan = kStageThreads * kStagePer;
+  for (long long base = blockIdx.x * kSpan + threadIdx.x; base < pieces; base += gridDim.x * kSpan) {
+    uint4 x[kStagePer];
+    uint4* to[kStagePer];
+    int words[kStagePer];
+#pragma unroll
+    for (int k = 0; k < kStagePer; ++k) {
+      long long i = base + (long long)k * kStageThreads;
+      to[k] = nullptr;
+      if (i >= pieces) continue;
+      int e = 0;
+      while (i >= list.end[e]) ++e;
+      words[k] = i == list.end[e] - 1 ? list.last_words[e] : 4;
+      if (e > 0) i -= list.end[e - 1];
+      to[k] = list.dst[e] + i;
+      if (words[k] == 4) {
+        x[k] = __ldcv(list.src[e] + i);
+      } else {
+        const unsigned* s = reinterpret_cast<const unsigned*>(list.src[e] + i);
+        x[k].x = __ldcv(s);
+        if (words[k] > 1) x[k].y = __ldcv(s + 1);
+        if (words[k] > 2) x[k].z = __ldcv(s + 2);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kStagePer; ++k) {
+      if (!to[k]) continue;
+      if (words[k] == 4) {
+        *to[k] = x[k];
+      } else {
+        unsigned* d = reinterpret_cast<unsigned*>(to[k]);
+        d[0] = x[k].x;
+        if (words[k] > 1) d[1] = x[k].y;
+        if (words[k] > 2) d[2] = x[k].z;
+      }
+    }
+  }
+}
+
+// The device's address of a pinned host buffer, null for anything else.  (Both ends: a buffer may be registered in part.)
+static const void* pinned_device_address(const void* p, size_t bytes) {
+  cudaPointerAttributes first, last;
+  if (cudaPointerGetAttributes(&first, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&last, static_cast<const char*>(p) + bytes - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
+      static_cast<const char*>(last.devicePointer) - static_cast<const char*>(first.devicePointer) != (ptrdiff_t)(bytes - 1))
+    return nullptr;
+  return first.devicePointer;
+}
+
+}  // namespace nvj
+
+extern "C" int nvj_stage_in(void* const* dst, const void* const* src, const size_t* bytes, int n, nvj_stream_t stream) {
+  using namespace nvj;
+  if (n < 0 || (n > 0 && (!dst || !src || !bytes))) return NVJ_ERR_INVALID_ARGUMENT;
+  if (n > kStageMost) return NVJ_ERR_UNSUPPORTED;
+  StageList list{};
+  long long pieces = 0;
+  for (int i = 0; i < n; ++i) {
+    if (bytes[i] == 0) continue;
+    if (!dst[i] || !src[i]) return NVJ_ERR_INVALID_ARGUMENT;
+    const void* from = (bytes[i] & 3) || !aligned16(dst[i]) ? nullptr : pinned_device_address(src[i], bytes[i]);
+    if (!from || !aligned16(from)) return NVJ_ERR_UNSUPPORTED;
+    list.src[list.n] = static_cast<const uint4*>(from);
+    list.dst[list.n] = static_cast<uint4*>(dst[i]);
+    pieces += (long long)((bytes[i] + 15) >> 4);
+    list.last_words[list.n] = (bytes[i] & 15) ? (int)((bytes[i] & 15) >> 2) : 4;
+    list.end[list.n++] = pieces;
+  }
+  if (list.n == 0) return NVJ_OK;
+  const long long ctas = (pieces + kStageThreads * kStagePer - 1) / (kStageThreads * kStagePer);
+  stage_in_kernel<<<(int)(ctas < kStageCtas ? ctas : kStageCtas), kStageThreads, 0, static_cast<cudaStream_t>(stream)>>>(list);
+  return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
+}
+
 extern "C" int nvj_row_argmax(const float* x, int rows, int row_len, int32_t* tokens,
                               nvj_stream_t stream) {
   using namespace nvj;

@@ -154,6 +154,10 @@ extern "C" int nvj_paged_decode_fused_append(const void* q, int q_dtype, const v
   return nvj::run_decode(p, workspace, workspace_bytes, variant, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int nvj_paged_decode_on_clusters(int batch, int table_width) {
+  return batch > 0 && table_width > 0 && nvj::decode_cluster_pays(batch, table_width) ? 1 : 0;
+}
+
 extern "C" int nvj_paged_decode_window(const void* q, int q_dtype, const void* k_cache_layer, const void* v_cache_layer,
                                        int kv_dtype, int64_t num_blocks, int block_size, int num_kv_heads, int head_dim,
                                        int num_q_heads, const int32_t* block_tables, int table_width,

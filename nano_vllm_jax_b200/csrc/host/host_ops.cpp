@@ -43,6 +43,7 @@ struct Library {
   decltype(&nvj_compute_slot_mapping) slot_mapping;
   decltype(&nvj_copy_blocks) copy_blocks;
   decltype(&nvj_copy_many_async) copy_many;
+  decltype(&nvj_stage_in) stage_in;
   decltype(&nvj_hybrid_snapshot_host_slots) snapshot;
   decltype(&nvj_hybrid_restore_host_slots) restore;
 };
@@ -261,11 +262,12 @@ PyObject* window_decode(PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(out));
 }
 
-// stage_in(targets, sources, on_first, streams (3), events (2)) -> True: copies sources[i] -> targets[i], the first `on_first`
-// pairs on the first stream and the rest on the second, and makes the third stream wait for both.  None, and nothing issued,
-// when a source differs from its target in dtype or size or is not contiguous.
+// stage_in(targets, sources, on_first, streams (3), events (2), by kernel) -> True: copies sources[i] -> targets[i] and makes the
+// third stream wait for them: in one kernel on the first stream if so asked and the sources are pinned, else the first
+// `on_first` pairs by the copy engines on the first stream and the rest on the second.  None, and nothing issued, when a source
+// differs from its target in dtype or size or is not contiguous.
 PyObject* stage_in(PyObject* const* a, Py_ssize_t n) {
-  if (!args_are(n, 5)) return nullptr;
+  if (!args_are(n, 6)) return nullptr;
   const long long split = PyLong_AsLongLong(a[2]);
   unsigned long long st[3], ev[2];
   if (PyErr_Occurred() || !PyTuple_Check(a[0]) || !PyTuple_Check(a[1]) || !PyArg_ParseTuple(a[3], "KKK", &st[0], &st[1], &st[2]) ||
@@ -286,18 +288,23 @@ PyObject* stage_in(PyObject* const* a, Py_ssize_t n) {
   }
   auto stream = [&](int i) { return reinterpret_cast<cudaStream_t>(st[i]); };
   auto event = [&](int i) { return reinterpret_cast<cudaEvent_t>(ev[i]); };
-  int rc;
+  const bool by_kernel = PyObject_IsTrue(a[5]) == 1;
+  int rc = NVJ_ERR_UNSUPPORTED, streams = 1;
   cudaError_t e = cudaSuccess;
   Py_BEGIN_ALLOW_THREADS
-  rc = lib.copy_many(dst, src, bytes, (int)split, stream(0));
-  if (rc == NVJ_OK) rc = lib.copy_many(dst + split, src + split, bytes + split, (int)(pairs - split), stream(1));
-  for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+  if (by_kernel) rc = lib.stage_in(dst, src, bytes, (int)pairs, stream(0));
+  if (rc == NVJ_ERR_UNSUPPORTED) {
+    streams = 2;
+    rc = lib.copy_many(dst, src, bytes, (int)split, stream(0));
+    if (rc == NVJ_OK) rc = lib.copy_many(dst + split, src + split, bytes + split, (int)(pairs - split), stream(1));
+  }
+  for (int i = 0; i < streams && e == cudaSuccess; ++i) {
     e = cudaEventRecord(event(i), stream(i));
     if (e == cudaSuccess) e = cudaStreamWaitEvent(stream(2), event(i), 0);
   }
   Py_END_ALLOW_THREADS
   if (rc == NVJ_OK && e != cudaSuccess) rc = NVJ_ERR_LAUNCH;
-  if (rc != NVJ_OK && !finished(rc, "nvj_copy_many_async", 0, nullptr, false, false)) return nullptr;
+  if (rc != NVJ_OK && !finished(rc, "nvj_stage_in or nvj_copy_many_async", 0, nullptr, false, false)) return nullptr;
   Py_RETURN_TRUE;
 }
 
@@ -967,6 +974,7 @@ PyObject* init(PyObject*, PyObject* args) {
   get(lib.norm_rope, "nvj_qk_norm_rope_kv_append");
   get(lib.slot_mapping, "nvj_compute_slot_mapping");
   get(lib.copy_many, "nvj_copy_many_async");
+  get(lib.stage_in, "nvj_stage_in");
   get(lib.copy_blocks, "nvj_copy_blocks");
   get(lib.snapshot, "nvj_hybrid_snapshot_host_slots");
   get(lib.restore, "nvj_hybrid_restore_host_slots");
@@ -1029,7 +1037,7 @@ PyMethodDef methods[] = {
     NVJ_FAST(take_fresh, "free blocks become a sequence's"),
     NVJ_FAST(drop_owner, "a sequence gives its blocks up"),
     NVJ_FAST(hash_chain, "chained digests of a token list's blocks, or None"),
-    NVJ_FAST(stage_in, "a step's operands to the device on two streams, or None"),
+    NVJ_FAST(stage_in, "a step's operands to the device, or None"),
     NVJ_FAST(copy_blocks, "cache[:, dst] = cache[:, src], or None"),
     NVJ_FAST(hybrid_copy, "snapshot or restore of GDN state rows, or None"),
     NVJ_FAST(pack_batch, "a batch's lists on the device"),

@@ -11,7 +11,8 @@ step i + 1's operands and step i - 1's result while step i computes:
     compute stream  append+decode(i)     append+decode(i+1)
     d2h stream      result(i-1)          result(i)
 
-The operands go in on two streams (most of their time is the copies' latency, not their bytes).  A step without an
+The operands of a short step go in by one kernel that reads the pinned buffers, those of a longer one by the copy engines on
+two streams (most of their time is the copies' latency, not their bytes).  A step without an
 `after_compute` has no result copy at all: the decode kernels only write their output, so they write it straight into the
 slot's pinned buffer, and the host waits 20 us less for 64 rows.
 
@@ -36,6 +37,7 @@ from typing import Dict, Optional
 
 import torch
 
+from . import _lib
 from .backends import B200Backend
 from .kernels import paged_kv as _k
 from .kv_cache import KVCacheStorage
@@ -78,7 +80,15 @@ class HostDecodePipeline:
         hq = hkv * num_key_value_groups
         self.backend, self.cache, self.capture = backend, cache, bool(capture)
         self.rows, self.block_size, self.scale, self.groups = rows, block_size, scale, num_key_value_groups
-        self.h2d, self.h2d_rest, self.compute, self.d2h = (torch.cuda.Stream(dev) for _ in range(4))
+        # (priority: the staging kernel's few CTAs take the places that the decode kernel's leave)
+        self.h2d, self.h2d_rest, self.compute, self.d2h = (torch.cuda.Stream(dev, priority=p) for p in (-1, 0, 0, 0))
+        # One kernel instead of six copies while a step is about as short as its copies: eight steps of 4 rows of 128 - 512
+        # keys 223 -> 162 us, 32 of 256 - 2048 341 -> 280, 48 of 128 - 4096 461 -> 429, 64 of 512 - 4096 (16384 blocks) 561 ->
+        # 558.  Longer steps hide the copy engines (160 rows of 1024 - 4096 keys: 1251 against 1280 us), and the streaming
+        # kernel holds every SM to its end: the staging kernel is for the batches that run on clusters.
+        dtype = cache.k_cache.dtype
+        self._stage_by_kernel = (query_dtype == dtype and rows * table_width <= 16384 and
+                                 (dtype != torch.bfloat16 or bool(_lib.load().nvj_paged_decode_on_clusters(rows, table_width))))
         self.slots = []
         for _ in range(depth):
             self.slots.append(_Slot(
@@ -117,16 +127,16 @@ class HostDecodePipeline:
         slot = self.slots[ticket % len(self.slots)]
         if slot.busy:
             slot.out_done.synchronize()  # its operands were consumed and its result has left the device
-        # the step's operands on two streams of about the same length (a small copy takes ~2 us whatever its size), the
-        # compute stream behind both
+        # the step's operands in one launch, or on two streams of about the same length (a small copy takes ~2 us whatever
+        # its size); the compute stream behind them
         host = _k.host()
         srcs = (query, positions, seq_lens, k, v, block_tables)
-        if host.stage_in(slot.inputs, srcs, 3, self._in_streams, slot.in_events) is None:
+        if host.stage_in(slot.inputs, srcs, 3, self._in_streams, slot.in_events, self._stage_by_kernel) is None:
             srcs = tuple(t.to(dst.dtype).contiguous() for t, dst in zip(srcs, slot.inputs))
             for i, t, dst in zip((0, 4, 5, 1, 2, 3), srcs, slot.inputs):
                 if t.numel() != dst.numel():
                     raise ValueError(f"operand {i} has {t.numel()} elements, the slot holds {dst.numel()}")
-            host.stage_in(slot.inputs, srcs, 3, self._in_streams, slot.in_events)
+            host.stage_in(slot.inputs, srcs, 3, self._in_streams, slot.in_events, False)
         slot.sources = srcs  # alive until the slot comes round again
         if after_compute is None and host.fused_decode(slot.q, slot.k, slot.v, self.cache.k_cache, self.cache.v_cache, slot.tables,
                                                        slot.seq_lens, slot.positions, layer_id, self.block_size, self.scale,
