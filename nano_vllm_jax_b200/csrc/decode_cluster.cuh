@@ -103,18 +103,24 @@ inline int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
   return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
-// CTAs per cluster for `groups` clusters of rows of up to `blocks` blocks, when a CTA walks `walkers` blocks at a time.
-// Doubled while the CTAs fit the SMs (`per_sm` hundredths of a CTA per SM) and a walker of the longest row has more than one
-// block; and, in batches of many CTAs, until none has more than 12, so that the last CTAs to finish are short ones.
-// Clusters of 16 (no longer portable, and placed one by one) only up to 2.2 CTAs per SM.  (Measured at 1 - 256 rows of
-// 64 - 16384 tokens: within 3% of the best size of each.)
+// CTAs per cluster for `groups` clusters of rows of up to `blocks` blocks, when a CTA walks `walkers` blocks at a time: as many
+// as fit the SMs (`per_sm` hundredths of a CTA per SM), at most one per `walkers` blocks of the longest row; and, in batches
+// of many CTAs, doubled (up to 8) until no walker has more than 12 blocks, so that the last CTAs to finish are short ones.
+// Clusters of more than 8 (no longer portable, and placed one by one) only up to 2.2 CTAs per SM.  Any size will do, not only
+// powers of two: with those, 28 rows of 128 - 2048 keys took 21.1 us (18.3 with 7 CTAs), 32 rows 21.1 (19.7 with 6), 64 rows of
+// 64 - 512 14.9 (13.9 with 3), 64 of 512 - 4096 57.7 (56.2 with 6).  (Measured at 4 - 160 rows: within 3% of each one's best.)
 inline int cluster_size(long long groups, int blocks, int sms, int walkers, int per_sm, int most) {
-  int c = 1;
-  while (c < most && c * walkers < blocks) {
-    const bool fits = 100 * 2 * c * groups <= (long long)(c < 8 || per_sm < 220 ? per_sm : 220) * sms;
-    if (!fits && (c >= 8 || blocks <= 12 * c * walkers)) break;
-    c *= 2;
+  auto fitting = [&](int hundredths) { return (int)((long long)hundredths * sms / (100 * groups)); };
+  int c = fitting(per_sm);
+  if (c > 8) {
+    c = fitting(per_sm < 220 ? per_sm : 220);
+    c = c > 8 ? c : 8;
   }
+  c = c > 1 ? c : 1;
+  while (c < 8 && blocks > 12 * c * walkers) c = c < 4 ? 2 * c : 8;
+  const int useful = (blocks + walkers - 1) / walkers;
+  c = c < useful ? c : useful > 1 ? useful : 1;
+  c = c < most ? c : most;
   return c;
 }
 // CTAs of 64 KiB go three to an SM; 2.75, because clusters do not pack every SM.

@@ -103,9 +103,11 @@ __device__ __forceinline__ void cl_end_beside(const DecodeParams& p) {
 template <int kHeads>
 __device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, const float2* ML, int ctas, uint32_t rank, int threads,
                                                 float* dst) {
-  const int per = kHeads * kD / 4 / ctas;
+  constexpr int kPieces = kHeads * kD / 4;
+  const int per = (kPieces + ctas - 1) / ctas;
   for (int i = threadIdx.x; i < per; i += threads) {
     const int piece = (int)rank * per + i, h = piece >> 6, d = (piece & 63) * 4;
+    if (piece >= kPieces) break;
     float2 e[kClMaxCluster];
     float4 x[kClMaxCluster];
 #pragma unroll
@@ -632,10 +634,10 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   // (with a page list per row its width is not known here: as many CTAs as an ordinary row has use for)
   const int blocks = p.kv_indptr ? 64 : p.table_width;
   const int cluster = cluster_per_head(p.batch, blocks, sms);
-  // Both KV heads in one CTA where that still leaves every SM a CTA and clusters are small: the two halves of a block's
-  // rows are then read at about the same time (48 rows of up to 2048 tokens 26.0 -> 24.4 us).  In smaller batches, and with
-  // eight and more CTAs per head, the finer split wins (4 rows of up to 512 tokens 7.3 against 5.9 us).
-  const bool both = cluster < 8 && (long long)cluster * kHkv * p.batch >= sms;
+  // Both KV heads in one CTA once three CTAs per row and head do not fit (68 rows): the two halves of a block's rows are then
+  // read at about the same time (128 rows of 64 - 512 keys: 21.1 us with 3 CTAs per row, 22.5 with 2 per head).  Below that the
+  // finer split per head is as fast or faster.
+  const bool both = 100LL * 3 * kHkv * p.batch > (long long)kCmPerSm * sms;
   const int pair = both ? cluster_size(p.batch, blocks, sms, kCmWarps / 2, kCmPerSm, 8) : 0;
   // the CUDA-core form: eight warps, a quarter block each, two CTAs per SM (1.8: clusters do not find every SM)
   const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 8);

@@ -29,8 +29,9 @@ def _case(seed, lens, width, dtype):
     return k, v, to_torch(tables), to_torch(lens), c
 
 
-# rows x table width (in blocks) pick the cluster size: 1, 2, 4, 8 and 16 CTAs per row and KV head
-@pytest.mark.parametrize("rows,width", [(3, 4), (3, 9), (3, 20), (3, 40), (2, 80), (40, 24), (150, 6)])
+# rows x table width (in blocks) pick the cluster size: 1, 3, 5, 10 and 16 CTAs per row and KV head in small batches, then 7, 5
+# and 3, then 3 and 2 CTAs per row for both heads
+@pytest.mark.parametrize("rows,width", [(3, 4), (3, 9), (3, 20), (3, 40), (2, 80), (28, 30), (40, 24), (60, 14), (130, 9), (150, 6)])
 @pytest.mark.parametrize("cache,query", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16), (torch.float32, torch.float32),
                                          (torch.float16, torch.float32), (torch.float32, torch.bfloat16)])
 def test_cluster_decode_equals_the_generic_kernel(rows, width, cache, query):
