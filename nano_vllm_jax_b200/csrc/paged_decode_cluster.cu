@@ -633,12 +633,20 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   if (sms <= 0) return NVJ_ERR_LAUNCH;
   // (with a page list per row its width is not known here: as many CTAs as an ordinary row has use for)
   const int blocks = p.kv_indptr ? 64 : p.table_width;
-  const int cluster = cluster_per_head(p.batch, blocks, sms);
+  // Beside another kernel: the SMs that it leaves (cta_limit), three CTAs to each; the ones too many start when it ends (six
+  // layers of 64 decode rows and two 256-token chunks, which take 32 SMs, 268 -> 259 us; 48 rows and three of 384 273 -> 255).
+  // Not the few rows that get eight CTAs and more: they leave SMs free.
+  int cluster = cluster_per_head(p.batch, blocks, sms), room = sms, per_sm = kCmPerSm;
+  if (p.beside && p.cta_limit > 0 && cluster < 8) {
+    room = p.cta_limit;
+    per_sm = 300;
+    cluster = cluster_size(2LL * p.batch, blocks, room, kCmWarps, per_sm, kClMaxCluster);
+  }
   // Both KV heads in one CTA once three CTAs per row and head do not fit (68 rows): the two halves of a block's rows are then
   // read at about the same time (128 rows of 64 - 512 keys: 21.1 us with 3 CTAs per row, 22.5 with 2 per head).  Below that the
   // finer split per head is as fast or faster.
   const bool both = 100LL * 3 * kHkv * p.batch > (long long)kCmPerSm * sms;
-  const int pair = both ? cluster_size(p.batch, blocks, sms, kCmWarps / 2, kCmPerSm, 8) : 0;
+  const int pair = both ? cluster_size(p.batch, blocks, room, kCmWarps / 2, per_sm, 8) : 0;
   // the CUDA-core form: eight warps, a quarter block each, two CTAs per SM (1.8: clusters do not find every SM)
   const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 8);
   static PerDeviceFlags flags[6];

@@ -210,9 +210,10 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
   // workspace; everything else goes to the tile kernel.
   int skip_single = 0;
   if (a.workspace && a.rows > 0 && rows_run_beside_tiles(a)) {
-    // tiles first, on a few SMs; the decode rows' clusters start at once and take the rest
-    const int rc2 = run_tiles(a, 1, s);
-    return rc2 != NVJ_OK ? rc2 : run_single_token_rows(a, 0, 1, s);
+    // tiles first, on a few SMs (a CTA pair per KV head and 64 tokens); the decode rows' clusters start at once and take the rest
+    const int rc2 = run_tiles(a, 1, s), sms = decode_wide_num_ctas();
+    const int rest = a.tile_pairs > 0 ? sms - 2 * kHkv * a.tile_pairs : sms;
+    return rc2 != NVJ_OK ? rc2 : run_single_token_rows(a, rest > sms / 2 ? rest : sms / 2, 1, s);
   }
   if (a.workspace && a.rows > 0) {
     if (!pair_kernel_serves(a) &&
