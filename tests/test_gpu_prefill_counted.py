@@ -30,6 +30,7 @@ def _batch(qlens, cached, pad, seed):
 @pytest.mark.parametrize("qlens,cached,pad", [
     ((64,), (0,), 0), ((65, 2), (0, 70), 3), ((63, 64, 128), (5, 0, 300), 0),       # no decode rows: key ranges may be split
     ((1, 1, 130, 1, 40), (40, 700, 0, 3, 90), 7), ((1,) * 40 + (2,), (33,) * 40 + (0,), 0),  # decode rows beside the tiles
+    ((1,) * 30 + (300,) * 8, (500,) * 30 + (0,) * 8, 0),                            # ... and tiles on every SM
 ])
 def test_counted_launch_equals_the_uncounted_one(qlens, cached, pad):
     from nano_vllm_jax_b200 import kv_cache as kvc
