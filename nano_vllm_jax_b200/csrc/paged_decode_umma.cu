@@ -336,7 +336,6 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     sm.start_b = p.batch; sm.start_j = 0; sm.abort_flag = 0;
   }
   pdl_wait();
-  pdl_release();
   // ---- pass 1: total number of blocks; zero the output of inactive rows
   int mine = 0;
   for (int base = 0; base < p.batch; base += kDecodeThreads) {
@@ -371,7 +370,10 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     if (n > 0 && excl <= g0 && g0 < excl + n) { sm.start_b = b; sm.start_j = (int)(g0 - excl); }
     carry += chunk_total;
   }
-  if (warp == 2) tmem_alloc(smem_u32(&sm.tmem_base), kUdTmemCols);
+  if (warp == 2) {  // tensor memory between the wait and the release (umma.cuh)
+    tmem_alloc(smem_u32(&sm.tmem_base), kUdTmemCols);
+    if (lane == 0) pdl_release();
+  }
   if (threadIdx.x == 0) {
     for (int i = 0; i < kUdStages; ++i) {
       mbar_init(smem_u32(&sm.full_bar[i]), 1);

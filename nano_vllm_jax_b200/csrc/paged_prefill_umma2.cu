@@ -545,9 +545,8 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   const int rank = (int)cluster_ctarank();  // == blockIdx.x & 1
   NVJ_U2_PHASE(0);
   NVJ_U2_NOTE(7, 0ull);
-  // The pair is set up before anything is read: this runs while the kernel in front (the append of the same tokens, usually)
-  // is still at work.
-  if (warp == 1) tmem2_alloc(smem_u32(&sm.tmem_base), kU2TmemCols);
+  // The pair's barriers are set up before anything is read: this runs while the kernel in front (the append of the same
+  // tokens, usually) is still at work.
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&sm.q_full), 2 * kU2SoftmaxThreads);
     for (int i = 0; i < kU2Stages; ++i) {
@@ -563,14 +562,15 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     mbar_init(smem_u32(&sm.x_full), kU2SoftmaxThreads);
     mbar_fence_init();
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  cluster_sync_all();  // the peer's barriers exist before anything is sent to them
-  tc_fence_after_sync();
+  cluster_sync_all();  // the peer's barriers exist before anything is sent to them (this barrier covers the CTA's own threads)
   pdl_wait();
-  // whatever follows may take its places now: the merge launch of a batch with splits (its CTAs wait for this grid to
-  // finish), the decode pass of a mixed batch (it runs beside, on the SMs this grid leaves)
-  pdl_release();
+  // Tensor memory between the wait and the release (umma.cuh).  Whatever follows may take its places behind it: the merge
+  // launch of a batch with splits (its CTAs wait for this grid to finish), the decode pass of a mixed batch (it runs beside, on
+  // the SMs this grid leaves).
+  if (warp == 1) {
+    tmem2_alloc(smem_u32(&sm.tmem_base), kU2TmemCols);
+    if (lane == 0) pdl_release();
+  }
   auto leave = [&] {  // the whole cluster leaves without having touched its tensor memory
     cluster_sync_all();
     if (warp == 1) tmem2_dealloc(sm.tmem_base, kU2TmemCols);
@@ -589,7 +589,9 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
       sm.total_pairs = t.total; sm.idle_index = t.idle;
     }
   }
+  tc_fence_before_sync();
   __syncthreads();
+  tc_fence_after_sync();
   const int row = sm.row, tok0 = sm.tok0, ntok = sm.ntok;
   if (p.counted && blockIdx.x == 0 && row >= 0 && threadIdx.x == 0) atomicOr(p.status, NVJ_DEV_BAD_LENGTH);
   int4* info = gridDim.z > 1 && blockIdx.z == 0 && threadIdx.x == 0 ? p.tile_info + blockIdx.x * kHkv + kvh : nullptr;

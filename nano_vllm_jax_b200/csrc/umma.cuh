@@ -11,6 +11,10 @@
 
 namespace nvj {
 
+// An allocation waits until the SM has the columns free.  Where grids overlap (programmatic dependent launch) a CTA that held
+// columns while it waits for the grid in front would keep that grid's CTAs from theirs, and neither would ever end.  So a
+// kernel takes its tensor memory behind pdl_wait(), when nothing in front of it is left to want any, and calls pdl_release()
+// only behind the allocation, so that the grid behind it, whatever that one does first, finds every CTA's columns taken.
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
