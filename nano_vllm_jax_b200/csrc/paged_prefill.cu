@@ -58,16 +58,21 @@ static int check_packed(const PackedArgs& a, bool* tile_ok) {
   return NVJ_OK;
 }
 
+// The caller's workspace, carved for the decode rows of the batch; NVJ_ERR_WORKSPACE when it lent none that is usable.
+static int carve_for_decode_rows(const PackedArgs& a, DecodeParams& d) {
+  const int num_ctas = decode_num_ctas();
+  d.batch = a.rows;
+  if (!a.workspace || num_ctas <= 0 || a.rows <= 0) return NVJ_ERR_WORKSPACE;
+  return carve_decode_workspace(d, a.workspace, a.workspace_bytes, ws_ml_bytes(num_ctas), ws_acc_bytes(num_ctas));
+}
+
 // Rows that carry a single query token (the decode rows of a mixed batch), by the streaming decode kernel on at most
 // `cta_limit` CTAs (0: one per SM).  `out` is zero where this pass writes nothing.  NVJ_ERR_WORKSPACE when the
 // caller lent no usable workspace.
 static int run_single_token_rows(const PackedArgs& a, int cta_limit, int beside, cudaStream_t s) {
   const int num_ctas = decode_num_ctas();
   DecodeParams d{};
-  d.batch = a.rows;
-  if (!a.workspace || num_ctas <= 0 || a.rows <= 0 ||
-      carve_decode_workspace(d, a.workspace, a.workspace_bytes, ws_ml_bytes(num_ctas), ws_acc_bytes(num_ctas)) != NVJ_OK)
-    return NVJ_ERR_WORKSPACE;
+  if (carve_for_decode_rows(a, d) != NVJ_OK) return NVJ_ERR_WORKSPACE;
   d.q = a.q;
   d.k_cache = static_cast<const char*>(a.k_cache_layer);
   d.v_cache = static_cast<const char*>(a.v_cache_layer);
@@ -209,7 +214,8 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
   // Rows that carry a single query token go to the streaming decode kernel when the caller lends it a decode
   // workspace; everything else goes to the tile kernel.
   int skip_single = 0;
-  if (a.workspace && a.rows > 0 && rows_run_beside_tiles(a)) {
+  DecodeParams carved{};  // (looked at before the tiles go out: without room for the decode rows the tiles take those too)
+  if (carve_for_decode_rows(a, carved) == NVJ_OK && rows_run_beside_tiles(a)) {
     // tiles first, on a few SMs (a CTA pair per KV head and 64 tokens); the decode rows' clusters start at once and take the rest
     const int rc2 = run_tiles(a, 1, s), sms = decode_wide_num_ctas();
     const int rest = a.tile_pairs > 0 ? sms - 2 * kHkv * a.tile_pairs : sms;

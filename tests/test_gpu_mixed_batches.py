@@ -1,0 +1,51 @@
+"""Mixed batches (decode rows beside query tiles) through the C ABI and the backend: what the caller lends, how many rows there
+are, and calls that follow one another without the host waiting in between."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import BS, SCALE, to_torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(qlens, cached, seed, layers=1, spare=8):
+    """A packed batch whose row r has qlens[r] tokens behind cached[r] cached ones, and N(0, 1) operands for it."""
+    rng = np.random.default_rng(seed)
+    lens = np.array([q + c for q, c in zip(qlens, cached)], np.int32)
+    need = -(-lens // BS)
+    pool = int(need.sum()) + spare
+    tables, o, perm = np.zeros((len(qlens), int(need.max())), np.int32), 0, rng.permutation(pool)
+    for r, n in enumerate(need):
+        tables[r, :n] = perm[o:o + n]
+        o += n
+    pos = np.concatenate([np.arange(c, c + q) for q, c in zip(qlens, cached)]).astype(np.int32)[None]
+    rid = np.repeat(np.arange(len(qlens)), qlens).astype(np.int32)[None]
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    normal = lambda *shape: torch.randn(shape, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    t = pos.shape[1]
+    return {"q": normal(1, t, 8, 256), "k": normal(1, t, 2, 256), "v": normal(1, t, 2, 256),
+            "cache": [normal(layers, pool, BS, 2, 256) for _ in range(2)], "tables": to_torch(tables), "lens": to_torch(lens),
+            "pos": to_torch(pos), "rid": to_torch(rid), "qsl": to_torch(np.cumsum([0] + list(qlens)).astype(np.int32)),
+            "qlens": tuple(qlens)}
+
+
+def _packed(b, out, status, workspace, nbytes):
+    from nano_vllm_jax_b200 import _lib
+    k, v = b["cache"]
+    return _lib.load().nvj_paged_prefill_packed(
+        b["q"].data_ptr(), _lib.NVJ_BF16, k.data_ptr(), v.data_ptr(), _lib.NVJ_BF16, k.shape[1], BS, 2, 256, 8, b["tables"].data_ptr(),
+        b["tables"].shape[1], b["lens"].data_ptr(), b["pos"].data_ptr(), b["qsl"].data_ptr(), b["tables"].shape[0], b["q"].shape[1], SCALE,
+        out.data_ptr(), status.data_ptr(), workspace, nbytes, 0, torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("nbytes,shift", [(512, 0), (1 << 24, 8)])  # too small; not on a 16-byte boundary
+def test_a_workspace_that_cannot_be_used_leaves_the_decode_rows_to_the_tiles(nbytes, shift):
+    b = _batch((1, 40, 1, 1, 70), (60, 0, 17, 300, 5), 1)
+    out, ref = (torch.full((112 + 1, 2048), float("nan"), device="cuda")[: sum(b["qlens"])] for _ in range(2))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    room = torch.zeros(nbytes + 16, dtype=torch.uint8, device="cuda")
+    assert _packed(b, ref, status, None, 0) == 0
+    assert _packed(b, out, status, room.data_ptr() + shift, nbytes) == 0
+    assert int(status) == 0 and torch.equal(out, ref) and not torch.isnan(out).any() and not room.any()
