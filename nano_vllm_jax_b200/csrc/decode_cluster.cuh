@@ -9,6 +9,7 @@
 namespace nvj {
 
 constexpr int kClMaxCluster = 16;
+constexpr int kClMaxRows = 65535;  // a row per grid z
 
 __device__ __forceinline__ void cl_copy16_or_zero(uint32_t dst, const char* src, uint32_t size) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");

@@ -620,7 +620,7 @@ static int cluster_per_head(int batch, int blocks, int sms) {
 // shares win once a CTA's own work gets long.  `table_width` bounds the blocks of a row; lengths are on the device.
 bool decode_cluster_pays(int batch, int table_width) {
   const int sms = decode_wide_num_ctas();
-  if (sms <= 0) return false;
+  if (sms <= 0 || batch > kClMaxRows) return false;
   const int c = cluster_per_head(batch, table_width, sms);
   const int per_warp = (table_width + c * kCmWarps - 1) / (c * kCmWarps);
   if ((long long)c * kHkv * batch >= sms) return per_warp <= 12;
@@ -628,7 +628,7 @@ bool decode_cluster_pays(int batch, int table_width) {
 }
 
 int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
-  if (p.batch > 65535) return NVJ_ERR_UNSUPPORTED;
+  if (p.batch > kClMaxRows) return NVJ_ERR_UNSUPPORTED;
   const int sms = decode_wide_num_ctas();
   if (sms <= 0) return NVJ_ERR_LAUNCH;
   // (with a page list per row its width is not known here: as many CTAs as an ordinary row has use for)

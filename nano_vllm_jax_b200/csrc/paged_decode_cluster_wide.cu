@@ -270,7 +270,7 @@ static int launch_tiles(const DecodeParams& p, int cluster, cudaStream_t stream)
 }
 
 static bool cw_takes(const DecodeParams& p) {
-  return p.width >= 2 && p.width <= kCwMaxWidth && p.batch <= 65535 && !p.new_k && !p.packed_rows && !p.kv_indptr;
+  return p.width >= 2 && p.width <= kCwMaxWidth && p.batch <= kClMaxRows && !p.new_k && !p.packed_rows && !p.kv_indptr;
 }
 static int cw_cluster(const DecodeParams& p, int sms) { return cluster_size(p.batch, p.table_width, sms, 1, kCmPerSm, kClMaxCluster); }
 

@@ -49,3 +49,31 @@ def test_a_workspace_that_cannot_be_used_leaves_the_decode_rows_to_the_tiles(nby
     assert _packed(b, ref, status, None, 0) == 0
     assert _packed(b, out, status, room.data_ptr() + shift, nbytes) == 0
     assert int(status) == 0 and torch.equal(out, ref) and not torch.isnan(out).any() and not room.any()
+
+
+@pytest.mark.parametrize("chunk", [0, 70])  # decode rows alone, and beside tiles
+def test_more_rows_than_a_grid_holds_are_served(chunk):
+    rows = 65536 + 3
+    qlens = [1] * rows + [chunk] * (chunk > 0)
+    n, t = len(qlens), sum(qlens)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    pool = 64
+    cache = [torch.randn((1, pool, BS, 2, 256), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    width = -(-max(chunk, 1) // BS)
+    tables = torch.randint(0, pool, (n, width), generator=g, device="cuda", dtype=torch.int32)
+    lens = torch.randint(1, BS + 1, (n,), generator=g, device="cuda", dtype=torch.int32)
+    q = torch.randn((1, t, 8, 256), generator=g, device="cuda").to(torch.bfloat16)
+    pos = torch.full((1, t), width * BS - 1, dtype=torch.int32, device="cuda")
+    if chunk:
+        lens[-1] = chunk
+        pos[0, rows:] = torch.arange(chunk, device="cuda", dtype=torch.int32)
+    qsl = to_torch(np.cumsum([0] + qlens).astype(np.int32))
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    out = K.packed_paged_prefill_attention(q, cache[0][0], cache[1][0], tables, lens, pos, qsl, BS, SCALE, 4)[0]
+    # one block per decode row, in plain torch, the rows behind the grid's limit and some in front of it
+    for r in list(range(rows - 5, rows)) + [0, 40000]:
+        keys, vals = (c[0, int(tables[r, 0]), : int(lens[r])].float() for c in cache)
+        s = torch.einsum("hgd,thd->hgt", q[0, r].float().view(2, 4, 256), keys) * SCALE
+        ref = torch.einsum("hgt,thd->hgd", torch.softmax(s, -1), vals).reshape(-1)
+        assert float((out[r] - ref).abs().max()) <= 2e-3
+    assert not torch.isnan(out).any()
