@@ -149,6 +149,16 @@ __device__ __forceinline__ float2 ld_cg_f32x2(const float* p) {
   return v;
 }
 
+// One word handed from one grid to another that runs at the same time.
+__device__ __forceinline__ void st_release_gpu(int32_t* p, int32_t v) {
+  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int32_t ld_acquire_gpu(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Streaming 16-byte load that does not allocate in L1 (read-once data).  Not the non-coherent form: a kernel's CTAs may be
 // resident while the kernel in front still writes what they will read (pdl_wait below).
 __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {

@@ -52,9 +52,12 @@ struct DecodeParams {
   // upper bound on the CTAs of the streaming kernels (0: one, or two, per SM): a caller that runs another kernel
   // beside the decode pass leaves that kernel's SMs free
   int cta_limit;
-  // cluster kernel: launched while the kernel in front of it in the stream, which it does not depend on, still runs (that
-  // kernel has let its dependents go); it ends only after that kernel has, so that the stream's order holds behind both
-  int beside;
+  // cluster kernel (nullable): launched while the kernel in front of it in the stream, whose results it does not need, still
+  // runs.  That kernel, once everything in front of IT is visible, sets this word of the workspace (release) and lets its
+  // dependents go; a CTA that reads it as set (acquire) therefore sees all of that too, one that does not waits for the kernel
+  // in front like any other.  The launch ends only after the kernel in front has, so that the stream's order holds behind
+  // both, and leaves the word zero.
+  int32_t* beside;
   // which wide kernel serves rows of several query tokens: 0 = automatic (mma.sync tiles up to width 4, tcgen05 beyond),
   // 1 = mma.sync tiles, 2 = tcgen05, 3 = thread-block clusters
   int wide_form;
@@ -124,6 +127,7 @@ __device__ __forceinline__ long long decode_table_base(const DecodeParams& p, in
 }
 
 constexpr size_t kWsAlign = 256;
+constexpr int kWsBesideWord = 8;  // index of an int32 in the status word's line
 __host__ __device__ inline size_t ws_round(size_t x) { return (x + kWsAlign - 1) / kWsAlign * kWsAlign; }
 // A row that is cut into more than kTreeMergeMin partials is merged in two levels: the CTAs of
 // one group of kMergeGroup consecutive CTA ids fold their partials into one group partial, and
@@ -145,12 +149,12 @@ inline size_t ws_acc_bytes(int num_ctas) { return ws_round(sizeof(float) * ws_sl
 // Carves a decode workspace of `bytes` bytes for a call with p.batch rows whose partial results need `ml_bytes` and
 // `acc_bytes`.  One buffer serves calls of any batch size, width and kernel one after another, so nothing a call
 // writes may land where a later call keeps state that must start at zero:
-//   [0, 64)              status word
+//   [0, 64)              status word; at kWsBesideWord the word of a launch beside another one (DecodeParams::beside)
 //   [64, 320)            group arrival counters
 //   [320, 320 + 4 rows)  row arrival counters
 //   ... unused, or the partial outputs of the prefill kernel's key-range splits, which end where the next part begins ...
 //   the last ml_bytes + acc_bytes of the buffer: partial (max, sum) pairs and accumulators
-// The counters are zero before the first use and every launch leaves them zero again; the partials are always
+// The counters and that word are zero before the first use and every launch leaves them zero again; the partials are always
 // written before they are read.  Because the partials are anchored at the END of the buffer, a call with few rows
 // cannot leave them inside the counter area of a later call with more rows (anchored behind the call's own
 // counters they would: a 256-row call after a 4-row call then found garbage in its counters and never merged

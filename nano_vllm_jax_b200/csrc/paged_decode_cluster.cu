@@ -94,9 +94,13 @@ __device__ __forceinline__ void cl_unpack(const ClRaw<T>& r, float2 (&o)[4]) {
   }
 }
 
-// A launch that runs beside the kernel in front of it ends after that kernel: one CTA holds the grid open.
+// A launch that runs beside the kernel in front of it ends after that kernel: one CTA holds the grid open, and then clears the
+// word that told the CTAs to go ahead (whoever has not read it yet waits for the kernel in front, which has ended by now).
 __device__ __forceinline__ void cl_end_beside(const DecodeParams& p) {
-  if (p.beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
+  if (p.beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+    pdl_wait();
+    if (threadIdx.x == 0) st_release_gpu(p.beside, 0);
+  }
 }
 // The CTAs' sums [head][pitch] and (max, sum) pairs, at the same places in every CTA of the cluster, into the output: rank
 // r takes its 1 / ctas of the float4 pieces of [heads][256 dims].
@@ -144,7 +148,7 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   const uint32_t rank = ctas > 1 ? cl_rank() : 0u;
   const int first = (int)rank * kClWarps + warp, stride = ctas * kClWarps;  // this warp's units: first, first + stride, ...
 
-  if (!p.beside) pdl_wait();
+  pdl_wait();
   pdl_release();
   // ---- first trip: the ids of this warp's first 32 units, the length, the query
   const long long tbase = decode_table_base(p, b);
@@ -157,10 +161,7 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   int ids = unit_id(lane);
   const int len = decode_row_len(p, b);  // the same in every thread of the cluster
   const long long qi = decode_query_index(p, b);
-  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) {  // not this pass's row (the whole cluster leaves)
-    cl_end_beside(p);
-    return;
-  }
+  if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) return;  // not this pass's row (the whole cluster leaves)
   // query heads in slot order (slot h of a lane holds head h ^ hperm), times scale * log2(e)
   const int rperm = lane >> 3, h_own = (lane >> 1) & 3;
   float2 q2[kG][4];
@@ -349,7 +350,6 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   if (ctas == 1) {
     const float inv = L > 0.f ? 1.f / L : 0.f;
     reinterpret_cast<float4*>(dst)[threadIdx.x] = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
-    cl_end_beside(p);
     return;
   }
   __syncthreads();  // acc[0] is overwritten
@@ -358,7 +358,6 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   cl_sync();
   cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, rank, kClThreads, dst);
   cl_sync();  // nobody leaves while its shared memory is being read
-  cl_end_beside(p);
 }
 
 // ---- 16-bit caches: the products on tensor-core tiles -------------------------------------------------------------
@@ -398,7 +397,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   constexpr int kWalkers = kBoth ? kCmWarps / 2 : kCmWarps;  // warps of the CTA that share a KV head's blocks
   const int first = (int)rank * kWalkers + (kBoth ? warp >> 1 : warp), stride = ctas * kWalkers;  // this warp's blocks: first, first + stride, ...
 
-  if (!p.beside) pdl_wait();
+  if (!p.beside || ld_acquire_gpu(p.beside) == 0) pdl_wait();
   pdl_release();
   // ---- first trip: the ids of this warp's first 32 blocks, the length, the query
   const long long tbase = decode_table_base(p, b);

@@ -19,7 +19,8 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, int tile_pairs, float* split_area, size_t split_bytes, cudaStream_t stream);
+                         int skip_single, int split_p, int tile_pairs, float* split_area, size_t split_bytes, int32_t* beside,
+                         cudaStream_t stream);
 bool prefill_umma2_usable(float scale, long long num_blocks);
 int launch_prefill_umma(const void* q, int q_dtype, const char* k_cache, const char* v_cache,
                         long long num_blocks, const int32_t* block_tables, int table_width,
@@ -69,7 +70,7 @@ static int carve_for_decode_rows(const PackedArgs& a, DecodeParams& d) {
 // Rows that carry a single query token (the decode rows of a mixed batch), by the streaming decode kernel on at most
 // `cta_limit` CTAs (0: one per SM).  `out` is zero where this pass writes nothing.  NVJ_ERR_WORKSPACE when the
 // caller lent no usable workspace.
-static int run_single_token_rows(const PackedArgs& a, int cta_limit, int beside, cudaStream_t s) {
+static int run_single_token_rows(const PackedArgs& a, int cta_limit, int32_t* beside, cudaStream_t s) {
   const int num_ctas = decode_num_ctas();
   DecodeParams d{};
   if (carve_for_decode_rows(a, d) != NVJ_OK) return NVJ_ERR_WORKSPACE;
@@ -96,7 +97,7 @@ static int run_single_token_rows(const PackedArgs& a, int cta_limit, int beside,
   // bf16 queries: the tensor-core streaming kernel (it declines without a tensor-map encoder); else the CUDA-core one
   int rc = NVJ_ERR_UNSUPPORTED;
   if (beside) {
-    d.beside = 1;
+    d.beside = beside;
     return launch_decode_cluster(d, s);
   }
   if (a.q_dtype == NVJ_BF16 && cta_limit == 0 && decode_cluster_pays(a.rows, a.table_width)) return launch_decode_cluster(d, s);
@@ -118,7 +119,8 @@ static bool pair_kernel_serves(const PackedArgs& a) {
 
 // Whether the decode rows of a mixed batch run on the cluster kernel beside the tiles, in one stream: the two write different
 // rows and neither fills the machine.  The tiles are launched first and let the clusters start at once (programmatic
-// dependent launch); a cluster CTA is small (64 KiB, 128 threads) and fits wherever no tile CTA sits.  Six layers of 32
+// dependent launch); a cluster CTA is small (64 KiB, 128 threads) and fits wherever no tile CTA sits.  What the append in
+// front of the tiles wrote reaches the clusters through a word that the tiles set (DecodeParams::beside).  Six layers of 32
 // decode rows of up to 2048 tokens and two chunks of 256: 24.3 + 24.3 us per layer one behind the other.
 static bool rows_run_beside_tiles(const PackedArgs& a) {
   return pair_kernel_serves(a) && a.q_dtype == NVJ_BF16 && decode_cluster_pays(a.rows, a.table_width);
@@ -127,7 +129,7 @@ static bool rows_run_beside_tiles(const PackedArgs& a) {
 // The query tiles: tcgen05 tiles first (CTA pairs, then single CTAs); they decline when the driver has no tensor-map
 // encoder or the scale is not positive, and the mma.sync tiles take over.  With skip_single the rows of one query
 // token are left to the pass above (and, unless the pair kernel serves the call, `out` has been zeroed by the caller).
-static int run_tiles(const PackedArgs& a, int skip_single, cudaStream_t s) {
+static int run_tiles(const PackedArgs& a, int skip_single, int32_t* beside, cudaStream_t s) {
   const char* kc = static_cast<const char*>(a.k_cache_layer);
   const char* vc = static_cast<const char*>(a.v_cache_layer);
   const int variant = a.variant;
@@ -149,7 +151,7 @@ static int run_tiles(const PackedArgs& a, int skip_single, cudaStream_t s) {
     }
     const int rc = launch_prefill_umma2(a.q, a.q_dtype, kc, vc, a.num_blocks, a.block_tables, a.table_width, a.kv_lens, a.positions,
                                         a.query_start_loc, a.rows, a.token_bucket, a.scale, a.out, a.status, skip_single,
-                                        variant == 5 ? 0 : 1, a.tile_pairs, split_area, split_bytes, s);
+                                        variant == 5 ? 0 : 1, a.tile_pairs, split_area, split_bytes, beside, s);
     if (rc != NVJ_ERR_UNSUPPORTED || variant != 0) return rc;
   }
   if (variant == 0 || variant == 3) {
@@ -206,9 +208,9 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
   if (rc != NVJ_OK || a.token_bucket == 0) return rc;
   if (part > 0) {
     if (!tile_ok || a.variant == 1) return NVJ_ERR_UNSUPPORTED;  // the generic kernel serves a batch in one piece
-    if (part == 1) return run_single_token_rows(a, cta_limit, 0, s);
+    if (part == 1) return run_single_token_rows(a, cta_limit, nullptr, s);
     if (part == 2 && !pair_kernel_serves(a)) return NVJ_ERR_UNSUPPORTED;  // the other tile kernels want a zeroed output
-    return run_tiles(a, part == 2 ? 1 : 0, s);
+    return run_tiles(a, part == 2 ? 1 : 0, nullptr, s);
   }
   if (!tile_ok || a.variant == 1) return run_generic(a, s);
   // Rows that carry a single query token go to the streaming decode kernel when the caller lends it a decode
@@ -217,15 +219,19 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
   DecodeParams carved{};  // (looked at before the tiles go out: without room for the decode rows the tiles take those too)
   if (carve_for_decode_rows(a, carved) == NVJ_OK && rows_run_beside_tiles(a)) {
     // tiles first, on a few SMs (a CTA pair per KV head and 64 tokens); the decode rows' clusters start at once and take the rest
-    const int rc2 = run_tiles(a, 1, s), sms = decode_wide_num_ctas();
+    int32_t* word = static_cast<int32_t*>(a.workspace) + kWsBesideWord;
+    const int rc2 = run_tiles(a, 1, word, s), sms = decode_wide_num_ctas();
+    if (rc2 != NVJ_OK) return rc2;
     const int rest = a.tile_pairs > 0 ? sms - 2 * kHkv * a.tile_pairs : sms;
-    return rc2 != NVJ_OK ? rc2 : run_single_token_rows(a, rest > sms / 2 ? rest : sms / 2, 1, s);
+    const int rc1 = run_single_token_rows(a, rest > sms / 2 ? rest : sms / 2, word, s);
+    if (rc1 != NVJ_OK) cudaMemsetAsync(word, 0, sizeof(int32_t), s);  // nobody is left who would clear it
+    return rc1;
   }
   if (a.workspace && a.rows > 0) {
     if (!pair_kernel_serves(a) &&
         cudaMemsetAsync(a.out, 0, sizeof(float) * (size_t)a.token_bucket * kHq * kD, s) != cudaSuccess)
       return NVJ_ERR_LAUNCH;
-    const int rc1 = run_single_token_rows(a, 0, 0, s);
+    const int rc1 = run_single_token_rows(a, 0, nullptr, s);
     if (rc1 == NVJ_OK) {
       skip_single = 1;
     } else if (rc1 != NVJ_ERR_WORKSPACE) {
@@ -233,10 +239,10 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
     } else {  // no room to serve the rows of one token: the tiles take them too, and the caller has not counted those
       PackedArgs all = a;
       all.tile_pairs = -1;
-      return run_tiles(all, 0, s);
+      return run_tiles(all, 0, nullptr, s);
     }
   }
-  return run_tiles(a, skip_single, s);
+  return run_tiles(a, skip_single, nullptr, s);
 }
 
 }  // namespace nvj

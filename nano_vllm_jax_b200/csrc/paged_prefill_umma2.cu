@@ -76,6 +76,7 @@ struct Umma2Params {
   long long num_blocks;
   int rows, token_bucket, table_width, skip_single, q_dtype;
   int counted;    // 1: the launch has exactly the caller's number of pairs plus an idle one; more pairs are flagged
+  int32_t* beside;  // nullable: set once what lies in front of this grid is visible (DecodeParams::beside)
   int zero_fill;  // 1: the kernel itself zeroes what no tile writes (padding tokens, rows of several tokens without keys)
   int split_p;  // 1: P enters P V as two bf16 terms (hi + lo), 0: as one (the weights are then bf16-rounded)
   float scale;
@@ -569,7 +570,10 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   // the SMs this grid leaves).
   if (warp == 1) {
     tmem2_alloc(smem_u32(&sm.tmem_base), kU2TmemCols);
-    if (lane == 0) pdl_release();
+    if (lane == 0) {
+      if (p.beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) st_release_gpu(p.beside, 1);
+      pdl_release();
+    }
   }
   auto leave = [&] {  // the whole cluster leaves without having touched its tensor memory
     cluster_sync_all();
@@ -782,7 +786,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
                          int skip_single, int split_p, int tile_pairs, float* split_area, size_t split_bytes,
-                         cudaStream_t stream) {
+                         int32_t* beside, cudaStream_t stream) {
   static PerDeviceFlags opted_in;
   constexpr int kSmemBytes = (int)sizeof(Umma2Smem) + 1024;
   static_assert(kSmemBytes <= 232448, "tiles exceed the shared memory of one CTA");
@@ -803,6 +807,7 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
   p.block_tables = block_tables; p.kv_lens = kv_lens; p.positions = positions; p.query_start_loc = query_start_loc;
   p.out = out; p.status = status; p.num_blocks = num_blocks; p.rows = rows; p.token_bucket = token_bucket;
   p.table_width = table_width; p.skip_single = skip_single; p.scale = scale; p.split_p = split_p;
+  p.beside = beside;
   // Clusters: one per pair of tiles and one that stays idle (it zeroes the padding).  Without the caller's count, at most
   // so many; the ones too many cost a batch of many rows and few tiles its start (34 rows, 8 pairs: 43 clusters per head,
   // two waves of CTAs that only set themselves up and leave).

@@ -77,3 +77,65 @@ def test_more_rows_than_a_grid_holds_are_served(chunk):
         ref = torch.einsum("hgt,thd->hgd", torch.softmax(s, -1), vals).reshape(-1)
         assert float((out[r] - ref).abs().max()) <= 2e-3
     assert not torch.isnan(out).any()
+
+
+# ---- calls in flight: kernels of one stream overlap (programmatic dependent launch), so nothing may depend on the host waiting
+
+def _calls(kind, n):
+    """n calls of one kind, each a function () -> outputs; all of them rewrite the same new rows of the same cache layer, so that
+    a call that runs ahead of the one in front, or lags behind it, reads other keys."""
+    from nano_vllm_jax_b200.backends import B200Backend
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    from nano_vllm_jax_b200.kv_cache import KVCacheStorage
+    be = B200Backend()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    if kind in ("mixed", "mixed, tiles everywhere", "chunk"):
+        qlens = {"mixed": (1,) * 32 + (250, 260), "mixed, tiles everywhere": (1,) * 30 + (300,) * 8, "chunk": (40, 130, 342)}[kind]
+        b = _batch(qlens, [(37 * i) % 900 + 16 for i in range(len(qlens))], 3)
+        md = be.build_attention_metadata(b["pos"], b["tables"], b["lens"], BS, True, query_start_loc=b["qsl"], token_row_ids=b["rid"],
+                                         query_lens_host=b["qlens"])
+        shape, prefill = (1, sum(qlens)), True
+    else:
+        rows, width = {"verify 5": (24, 5), "verify 3": (5, 3), "norm": (48, 1), "decode": (16, 1)}[kind]
+        b = _batch((width,) * rows, [(53 * i) % 1200 + 3 for i in range(rows)], 4)
+        pos = b["pos"].view(rows, width)
+        md = be.build_attention_metadata(pos, b["tables"], b["lens"], BS, False,
+                                         query_start_loc=None if width == 1 else torch.arange(rows + 1, device="cuda", dtype=torch.int32) * width)
+        shape, prefill = (rows, width), False
+    cache = KVCacheStorage(*b["cache"])
+    normal = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    weight = [normal(256) * 0.1 for _ in range(2)]
+
+    def call(q, k, v):
+        if kind == "norm":
+            q, _, _ = K.qk_norm_rope_kv_append(q, k, v, *weight, pos, md.slot_mapping, cache.k_cache[0], cache.v_cache[0], eps=1e-6,
+                                               rope_theta=1e7, rotary_dim=64)
+            return be.attention(0, q, cache, md, BS, SCALE, 4, False)
+        return be.write_kv_and_attention(0, q, k, v, cache, md, BS, SCALE, 4, prefill)[1]
+
+    operands = [(normal(*shape, 8, 256), normal(*shape, 2, 256), normal(*shape, 2, 256)) for _ in range(n)]
+    return [lambda o=o: call(*o) for o in operands], cache
+
+
+@pytest.mark.parametrize("kind", ["mixed", "mixed, tiles everywhere", "chunk", "verify 5", "verify 3", "norm", "decode"])
+def test_calls_in_flight_give_what_they_give_one_by_one(kind, monkeypatch):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    monkeypatch.setenv("NVJ_CHECK_STATUS", "0")   # no status word read back,
+    monkeypatch.setenv("NVJ_POISON_OUTPUT", "0")  # and no fill between two calls
+    calls, cache = _calls(kind, 8)
+    start = cache.k_cache.clone(), cache.v_cache.clone()
+    one_by_one = []
+    for c in calls:
+        one_by_one.append(c())
+        torch.cuda.synchronize()
+    after = cache.k_cache.clone(), cache.v_cache.clone()
+    for _ in range(20):
+        cache.k_cache.copy_(start[0])
+        cache.v_cache.copy_(start[1])
+        outs = [c() for c in calls]
+        for a, b in zip(outs, one_by_one):
+            assert torch.equal(a, b)
+        assert torch.equal(cache.k_cache, after[0]) and torch.equal(cache.v_cache, after[1])
+    K.check_device_status()
+    ws = K._workspaces[torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream]
+    assert not ws.buf[:64].any()  # the word that lets the decode rows run beside the tiles is left zero
