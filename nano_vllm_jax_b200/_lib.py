@@ -135,7 +135,9 @@ def load() -> ctypes.CDLL:
 
 def host_module():
     """The host extension module (csrc/host/host_ops.cpp), built first if it is absent."""
-    import torch  # noqa: F401  (the module links against torch's libraries)
+    import torch  # (the module links against torch's libraries)
+    if torch.version.cuda is None:
+        raise ImportError("the host extension needs a CUDA build of torch")
     if not _build.HOST_PATH.exists():
         _build.build_host()
     from . import _nvj_host

