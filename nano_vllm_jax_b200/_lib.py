@@ -8,6 +8,7 @@ raises on a non-zero status.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_uint32, c_uint64, c_void_p
@@ -133,15 +134,30 @@ def load() -> ctypes.CDLL:
         return lib
 
 
+_host = None
+_host_lock = threading.Lock()
+
+
 def host_module():
-    """The host extension module (csrc/host/host_ops.cpp), built first if it is absent."""
+    """The host extension module (csrc/host/host_ops.cpp) of this Python and torch, built first if it is absent."""
+    global _host
+    with _host_lock:
+        if _host is None:
+            _host = _load_host()
+        return _host
+
+
+def _load_host():
     import torch  # (the module links against torch's libraries)
     if torch.version.cuda is None:
         raise ImportError("the host extension needs a CUDA build of torch")
-    if not _build.HOST_PATH.exists():
+    path = _build.host_path()
+    if not path.exists():
         _build.build_host()
-    from . import _nvj_host
-    return _nvj_host
+    spec = importlib.util.spec_from_file_location(f"{__package__}._nvj_host", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
 
 
 def check(status: int, what: str) -> None:

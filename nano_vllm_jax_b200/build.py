@@ -5,17 +5,18 @@
 travels with a snapshot of the source tree) and is a no-op when the library is
 newer than every source.  Beside it, `build_host()` compiles `csrc/host/host_ops.cpp`
 (the host side of the hot calls, against torch's C++ headers) into the Python
-extension module `_nvj_host.so`; `build()` does both.  The pattern follows the reference's build-on-import of
+extension module `_nvj_host.<tag>.so`; `build()` does both.  The pattern follows the reference's build-on-import of
 its own CUDA FFI library (nanovllm_jax/kernels/cuda_fp32_ffi.py:121-178) with the
 architecture fixed to sm_100a.
 """
 
 from __future__ import annotations
 
-import importlib.util
 import os
+import re
 import shutil
 import subprocess
+import sys
 import sysconfig
 from pathlib import Path
 
@@ -24,7 +25,6 @@ CSRC = PKG_DIR / "csrc"
 INCLUDE = PKG_DIR.parent / "include"
 LIB_PATH = PKG_DIR / "libnvj_b200.so"
 HOST_SRC = CSRC / "host" / "host_ops.cpp"
-HOST_PATH = PKG_DIR / "_nvj_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -55,18 +55,25 @@ def nvcc_path() -> str | None:
     )
 
 
+def host_path() -> Path:
+    """Where the host extension of this Python and this torch lies.  Its C++ interface to both is theirs to change with any
+    version, so the file carries the two in its name: after a change of either the old one is not found and a new one is built."""
+    import torch
+    tag = re.sub(r"[^A-Za-z0-9]+", "_", f"{sys.implementation.cache_tag} torch {torch.__version__}")
+    return PKG_DIR / f"_nvj_host.{tag}.so"
+
+
 def build_host(force: bool = False) -> Path:
     """Compile the host extension module if needed and return its path."""
+    target = host_path()
     newest = max(p.stat().st_mtime for p in (HOST_SRC, INCLUDE / "nvj_b200.h"))
-    if not force and HOST_PATH.exists() and HOST_PATH.stat().st_mtime > newest:
-        return HOST_PATH
-    spec = importlib.util.find_spec("torch")
-    if spec is None or not spec.submodule_search_locations:
-        raise RuntimeError("torch not found: cannot build _nvj_host.so")
-    torch_dir = Path(spec.submodule_search_locations[0])
+    if not force and target.exists() and target.stat().st_mtime > newest:
+        return target
+    import torch
+    torch_dir = Path(torch.__file__).parent
     nvcc = nvcc_path()
     cuda_include = Path(nvcc).resolve().parents[1] / "include" if nvcc else Path("/usr/local/cuda/include")
-    part = HOST_PATH.with_suffix(f".{os.getpid()}.part")  # moved into place whole: another process may be loading the old one
+    part = target.with_suffix(f".{os.getpid()}.part")  # moved into place whole: another process may be loading the old one
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            "-I", str(torch_dir / "include"), "-I", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"),
            "-I", str(cuda_include), "-I", sysconfig.get_paths()["include"], "-o", str(part), str(HOST_SRC),
@@ -74,8 +81,8 @@ def build_host(force: bool = False) -> Path:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError("g++ failed on host_ops.cpp:\n" + proc.stdout + proc.stderr)
-    part.replace(HOST_PATH)
-    return HOST_PATH
+    part.replace(target)
+    return target
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -121,6 +128,4 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 if __name__ == "__main__":
-    import sys
-
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
