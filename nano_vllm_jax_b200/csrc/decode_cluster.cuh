@@ -106,11 +106,11 @@ inline int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
 
 // CTAs per cluster for `groups` clusters of rows of up to `blocks` blocks, when a CTA walks `walkers` blocks at a time: as many
 // as fit the SMs (`per_sm` hundredths of a CTA per SM), at most one per `walkers` blocks of the longest row; and, in batches
-// of many CTAs, doubled (up to 8) until no walker has more than 12 blocks, so that the last CTAs to finish are short ones.
+// of many CTAs, doubled (up to `grown`) until no walker has more than 12 blocks, so that the last CTAs to finish are short ones.
 // Clusters of more than 8 (no longer portable, and placed one by one) only up to 2.2 CTAs per SM.  Any size will do, not only
 // powers of two: with those, 28 rows of 128 - 2048 keys took 21.1 us (18.3 with 7 CTAs), 32 rows 21.1 (19.7 with 6), 64 rows of
 // 64 - 512 14.9 (13.9 with 3), 64 of 512 - 4096 57.7 (56.2 with 6).  (Measured at 4 - 160 rows: within 3% of each one's best.)
-inline int cluster_size(long long groups, int blocks, int sms, int walkers, int per_sm, int most) {
+inline int cluster_size(long long groups, int blocks, int sms, int walkers, int per_sm, int grown, int most) {
   auto fitting = [&](int hundredths) { return (int)((long long)hundredths * sms / (100 * groups)); };
   int c = fitting(per_sm);
   if (c > 8) {
@@ -118,7 +118,7 @@ inline int cluster_size(long long groups, int blocks, int sms, int walkers, int 
     c = c > 8 ? c : 8;
   }
   c = c > 1 ? c : 1;
-  while (c < 8 && blocks > 12 * c * walkers) c = c < 4 ? 2 * c : 8;
+  while (c < grown && blocks > 12 * c * walkers) c = c < 4 ? 2 * c : grown;
   const int useful = (blocks + walkers - 1) / walkers;
   c = c < useful ? c : useful > 1 ? useful : 1;
   c = c < most ? c : most;

@@ -609,21 +609,51 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   cl_end_beside(p);
 }
 
-static int cluster_per_head(int batch, int blocks, int sms) {
-  return cluster_size(2LL * batch, blocks, sms, kCmWarps, kCmPerSm, kClMaxCluster);
+// The tensor-core form's launch for a batch: CTAs per cluster, and whether a CTA takes both KV heads of a row or one.
+struct ClusterForm {
+  bool both;
+  int ctas, walkers;  // walkers: warps of a CTA that share a KV head's blocks
+
+  long long total(int batch) const { return (long long)ctas * batch * (both ? 1 : kHkv); }
+  int per_walker(int blocks) const { return (blocks + ctas * walkers - 1) / (ctas * walkers); }
+};
+// `room` SMs with `per_sm` hundredths of a CTA each; `blocks` bounds a row's blocks, lengths are on the device.
+static ClusterForm cluster_form(int batch, int blocks, int sms, int room, int per_sm) {
+  // Both KV heads in one CTA once three CTAs per row and head do not fit (68 rows): the two halves of a block's rows are then
+  // read at about the same time (128 rows of 64 - 512 keys: 21.1 us with 3 CTAs per row, 22.5 with 2 per head).  Below that the
+  // finer split per head is as fast or faster.
+  const bool both = 100LL * 3 * kHkv * batch > (long long)kCmPerSm * sms;
+  if (!both) return {false, cluster_size(2LL * batch, blocks, room, kCmWarps, per_sm, 8, kClMaxCluster), kCmWarps};
+  ClusterForm f{true, cluster_size(batch, blocks, room, kCmWarps / 2, per_sm, 4, 8), kCmWarps / 2};
+  // More than four CTAs per row only beyond 24 blocks per walker, and then six where they fill the places (three to an SM) more
+  // than 2.5 times, eight where they do not: a CTA that finds no block costs its start all the same.  256 rows under a table of
+  // 128 blocks, filled to 1/4 - 1 and to 1/32 - 1/8 of it: 112 and 42 us with eight, 114 and 28 with four (streaming kernel 113
+  // and 30); 263 blocks: 209 and 52 with eight, 212 and 44 with six (217 and 42).
+  if (f.per_walker(blocks) > 24 && f.ctas < 6) f.ctas = 2LL * 6 * batch > 15LL * sms ? 6 : 8;
+  return f;
 }
 
-// Whether this kernel, at its best cluster size, beats the streaming kernel (paged_decode_wide.cu) on a bf16 batch.  The
-// streaming kernel costs ~12.5 us whatever the batch plus its bytes at the HBM rate; this one ~4.5 us plus ~1.25 us per
-// block of the longest warp while CTAs have an SM each, and the HBM rate beyond that, where the streaming kernel's equal
-// shares win once a CTA's own work gets long.  `table_width` bounds the blocks of a row; lengths are on the device.
+// Whether this kernel, launched as cluster_form() says, beats the streaming kernel (paged_decode_wide.cu) on a bf16 batch.
+// While CTAs have an SM each: the streaming kernel costs ~12.5 us whatever the batch plus its bytes at the HBM rate, this one
+// ~4.5 us plus ~1.25 us per block of the longest warp.  Beyond that, where the streaming kernel's equal shares win once a CTA's
+// own work gets long, by the blocks of a walker, and with an eye on rows much shorter than the table (a server that pads its
+// tables), for which a CTA without a block is pure cost.  Measured at 48 - 512 rows and 32 - 512 blocks, rows of 1/4 - 1
+// and of 1/32 - 1/8 of the table, in the tables of cluster_form and here (us, clusters : streaming):
+//   eight CTAs per row and head that fill the places more than twice: 67 rows under 384 blocks 88 : 90 and 25 : 22;
+//   160 rows under 192, eight per row: 105 : 106 and 32 : 27;
+//   places filled between once and 5/3 times, 24 blocks per walker: 160 rows under 192, four per row: 110 : 106 and 23 : 27;
+//   at 16 per walker: 160 under 128 75 : 76 and 19 : 23, 128 under 192 (six) 87 : 87 and 21 : 24.
 bool decode_cluster_pays(int batch, int table_width) {
   const int sms = decode_wide_num_ctas();
   if (sms <= 0 || batch > kClMaxRows) return false;
-  const int c = cluster_per_head(batch, table_width, sms);
-  const int per_warp = (table_width + c * kCmWarps - 1) / (c * kCmWarps);
-  if ((long long)c * kHkv * batch >= sms) return per_warp <= 12;
-  return 1.25 * per_warp <= 9.5 + 0.0026 * batch * table_width;  // 32 KiB per block, half of the widest on average, 6.3 TB/s
+  const ClusterForm f = cluster_form(batch, table_width, sms, sms, kCmPerSm);
+  const long long total = f.total(batch);
+  const int per_walker = f.per_walker(table_width);
+  if (total < sms) return 1.25 * per_walker <= 9.5 + 0.0026 * batch * table_width;  // 32 KiB per block, half of the widest on average, 6.3 TB/s
+  if (f.ctas == 8 && total > 6LL * sms) return false;
+  if (!f.both) return per_walker <= 12;
+  if (total > 3LL * sms && total < 5LL * sms) return per_walker <= 16;
+  return per_walker <= (f.ctas == 6 ? 32 : 24);
 }
 
 int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
@@ -635,27 +665,18 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   // Beside another kernel: the SMs that it leaves (cta_limit), three CTAs to each; the ones too many start when it ends (six
   // layers of 64 decode rows and two 256-token chunks, which take 32 SMs, 268 -> 259 us; 48 rows and three of 384 273 -> 255).
   // Not the few rows that get eight CTAs and more: they leave SMs free.
-  int cluster = cluster_per_head(p.batch, blocks, sms), room = sms, per_sm = kCmPerSm;
-  if (p.beside && p.cta_limit > 0 && cluster < 8) {
-    room = p.cta_limit;
-    per_sm = 300;
-    cluster = cluster_size(2LL * p.batch, blocks, room, kCmWarps, per_sm, kClMaxCluster);
-  }
-  // Both KV heads in one CTA once three CTAs per row and head do not fit (68 rows): the two halves of a block's rows are then
-  // read at about the same time (128 rows of 64 - 512 keys: 21.1 us with 3 CTAs per row, 22.5 with 2 per head).  Below that the
-  // finer split per head is as fast or faster.
-  const bool both = 100LL * 3 * kHkv * p.batch > (long long)kCmPerSm * sms;
-  const int pair = both ? cluster_size(p.batch, blocks, room, kCmWarps / 2, per_sm, 8) : 0;
+  ClusterForm form = cluster_form(p.batch, blocks, sms, sms, kCmPerSm);
+  if (p.beside && p.cta_limit > 0 && (form.both || form.ctas < 8)) form = cluster_form(p.batch, blocks, sms, p.cta_limit, 300);
   // the CUDA-core form: eight warps, a quarter block each, two CTAs per SM (1.8: clusters do not find every SM)
-  const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 8);
+  const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 8, 8);
   static PerDeviceFlags flags[6];
   const int smem = (int)sizeof(CmSmem);
   if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16)
-    return both ? launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, true>, flags[0], p, pair, 1, kCmThreads, smem, stream)
-                : launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, false>, flags[1], p, cluster, kHkv, kCmThreads, smem, stream);
+    return form.both ? launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, true>, flags[0], p, form.ctas, 1, kCmThreads, smem, stream)
+                : launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, false>, flags[1], p, form.ctas, kHkv, kCmThreads, smem, stream);
   if (p.kv_dtype == NVJ_F16 && p.q_dtype == NVJ_F16)
-    return both ? launch_clusters(decode_cluster_mma_kernel<__half, true>, flags[2], p, pair, 1, kCmThreads, smem, stream)
-                : launch_clusters(decode_cluster_mma_kernel<__half, false>, flags[3], p, cluster, kHkv, kCmThreads, smem, stream);
+    return form.both ? launch_clusters(decode_cluster_mma_kernel<__half, true>, flags[2], p, form.ctas, 1, kCmThreads, smem, stream)
+                : launch_clusters(decode_cluster_mma_kernel<__half, false>, flags[3], p, form.ctas, kHkv, kCmThreads, smem, stream);
   if (p.kv_dtype == NVJ_F32)
     return launch_clusters(decode_cluster_kernel<float>, flags[4], p, wide, kHkv, kClThreads, cluster_smem_bytes<float>(), stream);
   if (p.kv_dtype == NVJ_F16)

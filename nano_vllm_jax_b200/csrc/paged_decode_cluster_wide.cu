@@ -272,7 +272,7 @@ static int launch_tiles(const DecodeParams& p, int cluster, cudaStream_t stream)
 static bool cw_takes(const DecodeParams& p) {
   return p.width >= 2 && p.width <= kCwMaxWidth && p.batch <= kClMaxRows && !p.new_k && !p.packed_rows && !p.kv_indptr;
 }
-static int cw_cluster(const DecodeParams& p, int sms) { return cluster_size(p.batch, p.table_width, sms, 1, kCmPerSm, kClMaxCluster); }
+static int cw_cluster(const DecodeParams& p, int sms) { return cluster_size(p.batch, p.table_width, sms, 1, kCmPerSm, 8, kClMaxCluster); }
 
 // Where the clusters beat the streaming forms: few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs
 // that are resident at once.  Beyond 4 tokens a block takes 1.5 us and the tcgen05 form is the faster one from 4 blocks on.

@@ -86,3 +86,23 @@ def test_cluster_decode_flags_a_bad_block_and_leaves_its_keys_out(monkeypatch):
     with pytest.raises(K.DeviceStatusError):
         K.check_device_status()
     assert float((got - ref).abs().max()) <= 2e-3
+
+
+# the launched form's own numbers decide (CTAs per row, blocks per walking warp, how often the CTAs fill their places); rows far
+# shorter than the table, the case a padded table makes, in every form: 5, 8, 6 and 6 CTAs per row for both heads, 8 per head
+@pytest.mark.parametrize("rows,width,pays", [(68, 200, True), (96, 263, True), (130, 100, True), (256, 263, True), (67, 384, False),
+                                             (160, 144, False), (123, 263, False), (256, 400, False), (70000, 4, False)])
+def test_short_rows_under_a_wide_table(rows, width, pays):
+    from nano_vllm_jax_b200 import _lib
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert bool(_lib.load().nvj_paged_decode_on_clusters(rows, width)) == pays
+    if rows > 1000:
+        return
+    lens = [1 + (37 * i) % 150 for i in range(rows - 2)] + [0, width * BS - 5]
+    k, v, tables, lens, c = _case(rows, lens, width, torch.bfloat16)
+    k, v = k.nan_to_num(), v.nan_to_num()  # (what the streaming kernel reads behind a row's last key must be finite)
+    q = to_torch(c["q"][:, 0]).contiguous()
+    ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
+    for variant in (0, 4):
+        assert float((K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=variant) - ref).abs().max()) <= 2e-3
