@@ -82,12 +82,13 @@ class HostDecodePipeline:
         self.rows, self.block_size, self.scale, self.groups = rows, block_size, scale, num_key_value_groups
         # (priority: the staging kernel's few CTAs take the places that the decode kernel's leave)
         self.h2d, self.h2d_rest, self.compute, self.d2h = (torch.cuda.Stream(dev, priority=p) for p in (-1, 0, 0, 0))
-        # One kernel instead of six copies while a step is about as short as its copies: eight steps of 4 rows of 128 - 512
-        # keys 223 -> 162 us, 32 of 256 - 2048 341 -> 280, 48 of 128 - 4096 461 -> 429, 64 of 512 - 4096 (16384 blocks) 561 ->
-        # 558.  Longer steps hide the copy engines (160 rows of 1024 - 4096 keys: 1251 against 1280 us), and the streaming
-        # kernel holds every SM to its end: the staging kernel is for the batches that run on clusters.
+        # One kernel instead of six copies while a step is about as short as its copies.  Eight steps, kernel : engines (us, rows
+        # of 1/8 - 1 of the table): 4 x 457 blocks 226 : 360, 32 x 253 356 : 401, 64 x 191 447 : 470, 96 x 128 471 : 504, 256 x 64
+        # 664 : 703, 64 x 255 548 : 556, 96 x 192 630 : 641, 128 x 160 655 : 661 (20480 blocks); then they part: 96 x 255
+        # 736 : 744, 256 x 96 810 : 780, 128 x 256 933 : 949, 256 x 128 967 : 952, 256 x 256 1652 : 1647.  And only for batches that
+        # run on clusters: the streaming kernel holds every SM to its end (64 x 318 880 : 870, 32 x 505 671 : 662).
         dtype = cache.k_cache.dtype
-        self._stage_by_kernel = (query_dtype == dtype and rows * table_width <= 16384 and
+        self._stage_by_kernel = (query_dtype == dtype and rows * table_width <= 20480 and
                                  (dtype != torch.bfloat16 or bool(_lib.load().nvj_paged_decode_on_clusters(rows, table_width))))
         self.slots = []
         for _ in range(depth):
