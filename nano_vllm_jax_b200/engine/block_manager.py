@@ -15,7 +15,7 @@ prefix exists) followed by the token ids as native int64 bytes.
 
 from __future__ import annotations
 
-from typing import Dict, Iterable, List, Optional, Set
+from typing import Dict, List, Optional, Set
 
 import numpy as np
 import xxhash
@@ -55,11 +55,14 @@ class _FreeList:
     A list and the index of its head, so that a sequence's blocks leave it as one slice and come back as one.  Removing an id
     from the middle (a cached block is taken again: rare) leaves its entry in the queue as a stale one, which the head skips
     when it gets there; an id's stale entries always lie in front of its live one.  Callers add only ids that are not free and
-    remove only free ones: an id is free exactly when its block has no owner.
+    remove only free ones.  An id is free exactly when it is not in `used` (the manager's set of owned blocks, which it keeps in
+    step), so that asking for one costs a look-up.
     """
 
-    def __init__(self, ids: Iterable[int]):
+    def __init__(self, ids: range, used: Set[int]):
         self._queue: List[int] = list(ids)
+        self._ids = ids
+        self._used = used
         self._head = 0
         self._stale: Dict[int, int] = {}  # id -> entries to skip
         self._len = len(self._queue)
@@ -68,7 +71,7 @@ class _FreeList:
         return self._len
 
     def __contains__(self, block_id: int) -> bool:
-        return block_id in iter(self)
+        return block_id in self._ids and block_id not in self._used
 
     def __iter__(self):
         stale = dict(self._stale)
@@ -138,8 +141,8 @@ class BlockManager:
         self.block_size = block_size
         self.blocks: List[Block] = [Block(i) for i in range(num_blocks)]
         self.hash_to_block_id: Dict[int, int] = {}
-        self.free_block_ids = _FreeList(range(num_blocks))
         self.used_block_ids: Set[int] = set()
+        self.free_block_ids = _FreeList(range(num_blocks), self.used_block_ids)
 
     # ------------------------------------------------------------------ hashing
     @classmethod

@@ -140,3 +140,30 @@ def test_lookahead_reserve_and_trim():
     bm.trim_append_slots(s, 1)
     assert len(s.block_table) == 2
     assert bm.stats() == {"total_blocks": 4, "free_blocks": 2, "used_blocks": 2}
+
+
+def test_asking_whether_a_block_is_free_is_a_look_up():
+    import random
+
+    r, bm, live = random.Random(3), BlockManager(num_blocks=60, block_size=2), []
+    for i in range(300):
+        if live and r.random() < 0.5:
+            bm.deallocate(live.pop(r.randrange(len(live))))
+        else:
+            s = _seq([r.randrange(4) for _ in range(r.randrange(1, 14))], i)
+            if bm.can_allocate(s):
+                bm.allocate(s)
+                bm.record_computed_prefix(s, s.num_tokens, publish=True)
+                live.append(s)
+        free = list(bm.free_block_ids)
+        assert [b in bm.free_block_ids for b in range(60)] == [b in free for b in range(60)]
+        assert -1 not in bm.free_block_ids and 60 not in bm.free_block_ids and None not in bm.free_block_ids
+
+    class Walked(Exception):
+        pass
+
+    def walk(self):
+        raise Walked
+
+    bm.free_block_ids.__class__ = type("Counted", (type(bm.free_block_ids),), {"__iter__": walk})
+    assert (5 in bm.free_block_ids) == (5 not in bm.used_block_ids)  # without a walk over the queue
