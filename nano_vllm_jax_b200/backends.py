@@ -128,11 +128,14 @@ class B200Backend:
                 raise ValueError("positions and block_tables batch dimensions must match")
             if positions.shape[0] != seq_lens.shape[0]:
                 raise ValueError("positions and seq_lens batch dimensions must match")
-        if is_prefill:
-            _k._cuda("positions", positions)
-            _k._cuda("block_table", block_tables)
-        # made when first read: the fused append + decode kernel and the plain append resolve the slots themselves
-        slot_mapping = kvc.SlotsFromTables(positions, block_tables, block_size, token_row_ids)
+        # A prefill's slots are made here and stay what they are; a decode batch's when an append or a reader wants them (the
+        # fused append + decode kernel and the append resolve them in their own launch).
+        if token_row_ids is not None:
+            slot_mapping = kvc.compute_packed_slot_mapping(positions, block_tables, token_row_ids, block_size)
+        elif is_prefill:
+            slot_mapping = kvc.compute_slot_mapping(positions, block_tables, block_size, is_prefill)
+        else:
+            slot_mapping = kvc.SlotsFromTables(positions, block_tables, block_size)
         batch, query_len = positions.shape
         singles = pairs = None
         if query_lens_host is not None and token_row_ids is not None:
@@ -174,7 +177,7 @@ class B200Backend:
         unread = metadata.__dict__["slot_mapping"]
         if type(unread) is kvc.SlotsFromTables:
             done = _k.host().append(k, v, cache.k_cache, cache.v_cache, layer_id, None, unread.positions, unread.block_tables,
-                                    unread.token_row_ids, metadata.query_start_loc, unread.block_size)
+                                    None, metadata.query_start_loc, unread.block_size)
         else:
             done = _k.host().append(k, v, cache.k_cache, cache.v_cache, layer_id, unread, None, None, metadata.token_row_ids,
                                     metadata.query_start_loc, 0)

@@ -309,8 +309,8 @@ PyObject* stage_in(PyObject* const* a, Py_ssize_t n) {
 }
 
 // append(new_k, new_v, k_cache, v_cache, layer, slot_mapping | None, positions, block_tables, token_row_ids | None,
-//        query_start_loc, block_size of the tables) -> True: token rows [rows, cols, Hkv, D] go to their slots; without a slot mapping the slots are
-// made from positions and tables in the same launch.
+//        query_start_loc, block_size of the tables) -> True: token rows [rows, cols, Hkv, D] go to their slots; without a slot mapping the slots of
+// a rectangular batch are made from positions and tables in the same launch.
 PyObject* append(PyObject* const* a, Py_ssize_t n) {
   if (!args_are(n, 11)) return nullptr;
   const at::Tensor *nk = tensor(a[0]), *nv = tensor(a[1]), *qsl = tensor(a[9]);
@@ -337,16 +337,15 @@ PyObject* append(PyObject* const* a, Py_ssize_t n) {
     NVJ_CALL(rc, lib.append(nk->data_ptr(), nv->data_ptr(), dt, i32(*slots), nullptr, i32(*qsl), (int)qsl->numel() - 1, packed ? 1 : 0,
                             (int)rows, (int)cols, l.k, l.v, l.dtype, num_slots, l.hkv, l.d, st, stream));
   } else {
-    const at::Tensor *pos = tensor(a[6]), *tab = tensor(a[7]), *rid = packed ? tensor(a[8]) : nullptr;
-    if (!pos || !tab || !meta(*pos, l.device) || !meta(*tab, l.device) || pos->dim() != 2 || pos->size(0) != rows || pos->size(1) != cols ||
-        tab->dim() != 2 || tab->size(0) == 0 || tab->size(1) == 0 || bs != l.block_size)
+    const at::Tensor *pos = tensor(a[6]), *tab = tensor(a[7]);
+    if (packed || !pos || !tab || !meta(*pos, l.device) || !meta(*tab, l.device) || pos->dim() != 2 || pos->size(0) != rows || pos->size(1) != cols ||
+        tab->dim() != 2 || tab->size(0) != rows || tab->size(1) == 0 || bs != l.block_size)
       NVJ_NONE();
-    if (packed ? (!rid || !meta(*rid, l.device) || rid->sizes() != pos->sizes()) : tab->size(0) != rows) NVJ_NONE();
     int32_t* st = status_for(l.device, stream);
     if (!st) return nullptr;
     what = "nvj_kv_append_mapped";
-    NVJ_CALL(rc, lib.append_mapped(nk->data_ptr(), nv->data_ptr(), dt, i32(*pos), i32(*tab), rid ? i32(*rid) : nullptr, (int)tab->size(0),
-                                   (int)tab->size(1), l.block_size, i32(*qsl), (int)qsl->numel() - 1, packed ? 1 : 0, (int)rows, (int)cols,
+    NVJ_CALL(rc, lib.append_mapped(nk->data_ptr(), nv->data_ptr(), dt, i32(*pos), i32(*tab), nullptr, (int)tab->size(0),
+                                   (int)tab->size(1), l.block_size, i32(*qsl), (int)qsl->numel() - 1, 0, (int)rows, (int)cols,
                                    l.k, l.v, l.dtype, num_slots, l.hkv, l.d, st, stream));
   }
   if (!finished(rc, what, l.device, stream, false, true)) return nullptr;

@@ -52,7 +52,8 @@ class AttentionMetadata:
 
     `slot_mapping` may be given as a zero-argument callable; it is then computed when first read.  A width-1 decode
     step that goes through the fused append + attention kernel never reads it (the kernel resolves the slots from the
-    block table itself), so the step is spared a launch.
+    block table itself), so the step is spared a launch, and an append that meets it unread makes the slots in its own launch.
+    Everything else refers to the given tensors: the caller leaves them as they are until the batch's last layer has run.
     """
 
     slot_mapping: torch.Tensor
@@ -95,18 +96,16 @@ def attention_metadata(**fields) -> AttentionMetadata:
 
 
 class SlotsFromTables:
-    """The slot mapping of a batch, made from its positions and block tables when somebody reads it.  An append that
-    meets it unread makes the slots inside its own launch instead (nvj_kv_append_mapped)."""
+    """The slot mapping of a decode batch, made from its positions and block tables when somebody reads it.  An append that
+    meets it unread makes the slots inside its own launch instead (nvj_kv_append_mapped), from what the tensors hold by then,
+    as the fused append of one token per row does."""
 
-    __slots__ = ("positions", "block_tables", "block_size", "token_row_ids")
+    __slots__ = ("positions", "block_tables", "block_size")
 
-    def __init__(self, positions, block_tables, block_size, token_row_ids=None):
+    def __init__(self, positions, block_tables, block_size):
         self.positions, self.block_tables, self.block_size = positions, block_tables, block_size
-        self.token_row_ids = token_row_ids
 
     def __call__(self):
-        if self.token_row_ids is not None:
-            return compute_packed_slot_mapping(self.positions, self.block_tables, self.token_row_ids, self.block_size)
         return compute_slot_mapping(self.positions, self.block_tables, self.block_size)
 
 

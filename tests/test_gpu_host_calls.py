@@ -81,3 +81,26 @@ def test_append_makes_the_slots_that_the_slot_mapping_has(packed):
         got.append(cache)
     assert float(got[0].k_cache[1].float().abs().sum()) > 0 and not got[0].k_cache[0].any()
     assert torch.equal(got[0].k_cache, got[1].k_cache) and torch.equal(got[0].v_cache, got[1].v_cache)
+
+
+@pytest.mark.parametrize("kind", ["decode", "prefill", "packed"])
+@pytest.mark.parametrize("read_first", [False, True])
+def test_when_the_slots_of_a_batch_are_made(kind, read_first):
+    """A prefill's with its metadata, a decode batch's when they are read or appended to."""
+    from nano_vllm_jax_b200.backends import B200Backend
+    from nano_vllm_jax_b200.kv_cache import KVCacheStorage
+    shape = (1, 6) if kind == "packed" else (2, 3)
+    pos = torch.tensor([[0, 1, 2], [16, 17, 18]], dtype=torch.int32, device="cuda").view(shape)
+    rid = torch.tensor([[0, 0, 0, 1, 1, 1]], dtype=torch.int32, device="cuda") if kind == "packed" else None
+    tables = torch.tensor([[3, 1], [0, 2]], dtype=torch.int32, device="cuda")
+    cache = KVCacheStorage(*(torch.zeros((1, 4, BS, 2, 256), dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+    be = B200Backend()
+    md = be.build_attention_metadata(pos, tables, torch.tensor([3, 19], dtype=torch.int32, device="cuda"), BS, kind != "decode",
+                                     query_start_loc=torch.tensor([0, 3, 6], dtype=torch.int32, device="cuda"), token_row_ids=rid)
+    if read_first:
+        md.slot_mapping
+    pos += 4  # between the metadata and the append
+    new = torch.ones((*shape, 2, 256), device="cuda", dtype=torch.bfloat16)
+    be.write_kv(0, new, new, cache, md)
+    moved = 4 if kind == "decode" and not read_first else 0
+    assert cache.k_cache[0, :, :, 0, 0].nonzero().tolist() == [[b, t + moved] for b in (2, 3) for t in range(3)]
