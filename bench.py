@@ -50,11 +50,15 @@ TOKEN_BYTES = 2 * HKV * D * 2  # K + V row of one token, bf16
 BLOCK_BYTES = BS * TOKEN_BYTES  # one block of K plus one block of V
 FALLBACK_HBM_GBS = 6650.0
 MIN_TIMED_STEPS = 100
-# dram__bytes_read.sum + dram__bytes_write.sum of decode_wide_kernel in an ncu capture of `--workload c2small`
-# (one launch) and the algorithmic bytes of that launch.  K/V traffic grows in proportion to the tokens
-# read, so a launch of another workload is scaled by its own algorithmic bytes.
-NCU_C2SMALL_DRAM_BYTES = 354.93e6
-NCU_C2SMALL_ALGORITHMIC_BYTES = 356.35e6
+# The kernel a workload's decode launch runs (the library's own rule, by rows and table width), and dram__bytes_read.sum +
+# dram__bytes_write.sum of one launch of it under ncu with that launch's algorithmic bytes.  K/V traffic grows in proportion to
+# the tokens read, so a launch of another size is scaled by its own algorithmic bytes.
+DECODE_KERNELS = {
+    True: dict(name="decode_cluster_mma_kernel (fused append + paged GQA decode on thread-block clusters, tensor-core tiles)",
+               dram=1351.09e6, algorithmic=1346.54e6, capture="256 rows of 1024 - 4096 tokens"),
+    False: dict(name="decode_wide_kernel at width 1 (fused append + paged GQA decode, TMA-staged, tensor-core tiles)",
+                dram=354.93e6, algorithmic=356.35e6, capture="--workload c2small on that kernel"),
+}
 
 WORKLOADS = {
     # rows: per rank (weak) or overall (strong); pool: blocks per rank, or None = sized from the free memory
@@ -325,6 +329,7 @@ def run_b200(args, w):
         dist.init_process_group("nccl", device_id=dev)
 
     from nano_vllm_jax_b200.backends import B200Backend
+    from nano_vllm_jax_b200 import _lib
     from nano_vllm_jax_b200.kernels import paged_kv as K
     from nano_vllm_jax_b200.kv_cache import KVCacheStorage
 
@@ -599,6 +604,7 @@ def run_b200(args, w):
         per_rank = sorted(float(t.item()) for t in every)
         rank_kernel_us = {"min": per_rank[0], "median": statistics.median(per_rank), "max": per_rank[-1]}
 
+    decode_kernel = DECODE_KERNELS[bool(_lib.load().nvj_paged_decode_on_clusters(rows, tables.shape[1]))]
     # roofline of the fused append+decode kernel: bytes of the timed launches over their duration
     kernel_ms = [e0.elapsed_time(e1) for _, e0, e1 in timed_events]
     ms_kernel = sum(kernel_ms)
@@ -658,13 +664,14 @@ def run_b200(args, w):
             "gpu_launches": 2 * K_steps,
             "step_mode": step_mode,
             "eager_value": total_rows / (ms_eager / K_steps * 1e-3), "eager_ms_per_step": ms_eager / K_steps,
-            "roofline": {"bound": "hbm", "kernel": "decode_wide_kernel at width 1 (fused append + paged GQA decode, TMA-staged, tensor-core tiles)",
+            "roofline": {"bound": "hbm", "kernel": decode_kernel["name"],
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_kind + " HBM copy bandwidth", "frac_of_8TBs_nominal": achieved / 8000.0,
                          "bytes_per_launch": bytes_per_launch, "us_per_launch": us_per_launch, "kernel_timing": kernel_timing,
                          "launch_us": percentiles([m * 1e3 for m in kernel_ms]),
-                         "traffic": NCU_C2SMALL_DRAM_BYTES / NCU_C2SMALL_ALGORITHMIC_BYTES * bytes_per_launch,
-                         "traffic_source": "dram bytes of one ncu-captured launch of --workload c2small (354.93 MB for 356.35 MB "
+                         "traffic": decode_kernel["dram"] / decode_kernel["algorithmic"] * bytes_per_launch,
+                         "traffic_source": f"dram bytes of one ncu-captured launch ({decode_kernel['capture']}: "
+                                           f"{decode_kernel['dram'] / 1e6:.2f} MB for {decode_kernel['algorithmic'] / 1e6:.2f} MB "
                                            "algorithmic) scaled to this launch by algorithmic bytes"},
             "rank_ms": rank_ms, "rank_kernel_us": rank_kernel_us, "gather_us": gather_us,
             "parity_check": parity,
