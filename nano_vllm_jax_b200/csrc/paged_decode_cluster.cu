@@ -667,8 +667,11 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   // Not the few rows that get eight CTAs and more: they leave SMs free.
   ClusterForm form = cluster_form(p.batch, blocks, sms, sms, kCmPerSm);
   if (p.beside && p.cta_limit > 0 && (form.both || form.ctas < 8)) form = cluster_form(p.batch, blocks, sms, p.cta_limit, 300);
-  // the CUDA-core form: eight warps, a quarter block each, two CTAs per SM (1.8: clusters do not find every SM)
-  const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 8, 8);
+  // The CUDA-core form: eight warps, a quarter block each, two CTAs per SM (1.8: clusters do not find every SM).  More than four
+  // CTAs per row and head by the table's width alone only where eight fill the places at most twice (37 rows): f32, 32 rows under
+  // 512 blocks 243 us with eight and 265 with four (rows of 1/4 - 1 of the table), 44 and 40 (1/32 - 1/8); 256 rows 1482 and 1447,
+  // 272 and 216; 512 rows of 16 - 128 keys 252 and 127 (the generic kernel 115).
+  const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 16LL * p.batch <= 4LL * sms ? 8 : 4, 8);
   static PerDeviceFlags flags[6];
   const int smem = (int)sizeof(CmSmem);
   if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16)

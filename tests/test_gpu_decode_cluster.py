@@ -106,3 +106,15 @@ def test_short_rows_under_a_wide_table(rows, width, pays):
     ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
     for variant in (0, 4):
         assert float((K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=variant) - ref).abs().max()) <= 2e-3
+
+
+@pytest.mark.parametrize("rows,width", [(37, 100), (38, 100), (150, 60)])  # 8, 4 and 4 CTAs per row and head
+@pytest.mark.parametrize("cache,query", [(torch.float32, torch.float32), (torch.float16, torch.float32)])
+def test_short_rows_under_a_wide_table_on_the_cuda_cores(rows, width, cache, query):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    lens = [1 + (37 * i) % 150 for i in range(rows - 2)] + [0, width * BS - 5]
+    k, v, tables, lens, c = _case(rows, lens, width, cache)
+    q = to_torch(c["q"][:, 0]).to(query).contiguous()
+    ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
+    got = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE)
+    assert float((got - ref).abs().max()) <= TIGHT[cache]
