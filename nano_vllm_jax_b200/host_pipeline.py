@@ -110,7 +110,10 @@ class HostDecodePipeline:
         self._compute_handle = self.compute.cuda_stream
         with torch.cuda.stream(self.compute):
             _k.lend_workspace(dev, rows)
-        self.compute.wait_stream(torch.cuda.current_stream(dev))  # whatever prepared the cache comes first
+        # Whatever prepared the cache comes first, and whatever last used the memory that the slots now hold (it is this stream's
+        # to the allocator).
+        for stream in (self.h2d, self.h2d_rest, self.compute):
+            stream.wait_stream(torch.cuda.current_stream(dev))
         self.submitted = 0
         self.h2d_bytes_per_step = sum(t.numel() * t.element_size() for t in
                                       (self.slots[0].q, self.slots[0].k, self.slots[0].v, self.slots[0].tables,

@@ -63,3 +63,51 @@ def test_pipelined_host_steps_equal_serial_steps_and_the_oracle(capture):
     want = R.paged_attention_decode(to_numpy(q), to_numpy(serial.k_cache), to_numpy(serial.v_cache), c["tables"],
                                     lens.numpy(), BS, SCALE, 4, positions=pos.numpy().reshape(rows, 1))
     assert np.abs(outs[-1].numpy().reshape(want.shape) - want).max() <= 2e-3
+
+
+def _pipe(rows=64, blocks=250):
+    from nano_vllm_jax_b200.backends import B200Backend
+    from nano_vllm_jax_b200.host_pipeline import HostDecodePipeline
+    from nano_vllm_jax_b200.kv_cache import KVCacheStorage
+
+    cache = KVCacheStorage(*(torch.zeros((1, 256, BS, 2, 256), dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+    pipe = HostDecodePipeline(B200Backend(), cache, rows, blocks, BS, SCALE, 4, depth=2)
+    tables = torch.arange(blocks, dtype=torch.int32).repeat(rows, 1)
+    tables[:, -1] = torch.arange(rows) % 6 + 250  # (every row's last block is where its new key goes)
+    step = [torch.zeros((rows, 1, h, 256), dtype=torch.bfloat16).pin_memory() for h in (8, 2, 2)]
+    step += [tables.pin_memory(), torch.full((rows, 1), blocks * BS - 1, dtype=torch.int32).pin_memory(),
+             torch.full((rows,), blocks * BS, dtype=torch.int32).pin_memory()]
+    return pipe, step
+
+
+def test_the_copies_wait_for_whoever_had_the_slots_memory(monkeypatch):
+    import gc
+    import time
+
+    monkeypatch.setenv("NVJ_CHECK_STATUS", "0")  # (reading the status word back waits)
+    real, made = torch.cuda.Stream, []
+
+    def stream(*args, **kwargs):  # the second pipeline gets the first one's streams, and with them their workspaces
+        if "stream_id" in kwargs:
+            return real(*args, **kwargs)
+        made.append(made[len(made) % 4] if len(made) >= 4 else real(*args, **kwargs))
+        return made[-1]
+
+    monkeypatch.setattr(torch.cuda, "Stream", stream)
+    pipe, step = _pipe()
+    pipe.submit(0, *step)
+    pipe.drain()
+    torch.cuda.synchronize()
+    cache, backend = pipe.cache, pipe.backend
+    del pipe
+    gc.collect()  # its device and pinned buffers are the allocators' again: nothing below waits for an allocation
+    torch.cuda._sleep(200_000_000)  # ~0.1 s on the stream whose memory the new slots take
+    asleep = torch.cuda.Event()
+    asleep.record()
+    from nano_vllm_jax_b200.host_pipeline import HostDecodePipeline
+    pipe = HostDecodePipeline(backend, cache, 64, 250, BS, SCALE, 4, depth=2)
+    pipe.submit(0, *step)
+    time.sleep(0.01)
+    landed = pipe.slots[0].in_done[0].query()
+    assert not asleep.query(), "the sleep was too short for this host"
+    assert not landed
