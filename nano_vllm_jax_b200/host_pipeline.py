@@ -32,6 +32,7 @@ then be capturable (no host synchronisation) and the same callable on every step
 from __future__ import annotations
 
 import os
+import weakref
 from dataclasses import dataclass, field
 from typing import Dict, Optional
 
@@ -63,6 +64,12 @@ class _Slot:
     d2h_lists: Dict[int, object] = field(default_factory=dict)  # per layer: host_out <- that layer's graph output
     sources: list = field(default_factory=list)
     last_out: Optional[torch.Tensor] = None
+
+
+def _wait_for_slots(slots) -> None:
+    for slot in slots:
+        if slot.busy:
+            slot.out_done.synchronize()
 
 
 class HostDecodePipeline:
@@ -114,6 +121,9 @@ class HostDecodePipeline:
         # to the allocator).
         for stream in (self.h2d, self.h2d_rest, self.compute):
             stream.wait_stream(torch.cuda.current_stream(dev))
+        # Steps in flight use the slots' buffers, pinned ones among them, on streams that the allocators do not know of: a pipeline
+        # that is dropped hands them back only when its last step has left the GPU.
+        weakref.finalize(self, _wait_for_slots, self.slots)
         self.submitted = 0
         self.h2d_bytes_per_step = sum(t.numel() * t.element_size() for t in
                                       (self.slots[0].q, self.slots[0].k, self.slots[0].v, self.slots[0].tables,

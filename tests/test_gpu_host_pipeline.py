@@ -111,3 +111,13 @@ def test_the_copies_wait_for_whoever_had_the_slots_memory(monkeypatch):
     landed = pipe.slots[0].in_done[0].query()
     assert not asleep.query(), "the sleep was too short for this host"
     assert not landed
+
+
+def test_a_dropped_pipeline_waits_for_its_steps(monkeypatch):
+    monkeypatch.setenv("NVJ_CHECK_STATUS", "0")
+    pipe, step = _pipe()
+    for _ in range(2):
+        pipe.submit(0, *step)
+    events = [s.out_done for s in pipe.slots]
+    del pipe
+    assert all(e.query() for e in events)
