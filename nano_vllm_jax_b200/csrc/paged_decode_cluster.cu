@@ -13,8 +13,8 @@
 //   * fused append: the cluster's first warp stores the new row, and whoever attends its key reads it from the operand.
 // Nothing waits on memory that somebody else must fill, so there is no wait to bound.
 // Measured (us per launch, K/V cold, lengths spread over [n / 4, n]; before: the streaming kernel): 4 rows of n = 512 tokens
-// 12.9 -> 5.9, 8 of 4096 20 -> 15, 48 of 1024 21.8 -> 16.2, 256 of 512 43.0 -> 34.4, 256 of 2048 114 -> 110.  f32: 8 rows of
-// 64 - 512 tokens 94 (the generic kernel) -> 9.
+// 12.2 -> 5.3, 8 of 4096 19.9 -> 13.7, 48 of 1024 21.8 -> 16.6, 256 of 512 41.4 -> 39.1, 256 of 2048 113 -> 112.  f32: 8 rows of
+// 64 - 512 tokens 221 (the generic kernel) -> 10.5.
 // Semantics: nanovllm_jax/kv_cache.py:852-998 for width-1 queries, nanovllm_jax/kernels/full_attention_triton.py:373-485
 // for the fused append.
 
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
       } else if (first == 0 && lane == 0) {
         atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
       }
-    } else if (!std::is_same<T, __nv_bfloat16>::value && first == 0 && lane == 0) {
+    } else if (first == 0 && lane == 0) {
       atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
     }
   }
