@@ -130,12 +130,13 @@ class B200Backend:
                 raise ValueError("positions and seq_lens batch dimensions must match")
         # A prefill's slots are made here and stay what they are; a decode batch's when an append or a reader wants them (the
         # fused append + decode kernel and the append resolve them in their own launch).
-        if token_row_ids is not None:
-            slot_mapping = kvc.compute_packed_slot_mapping(positions, block_tables, token_row_ids, block_size)
-        elif is_prefill:
-            slot_mapping = kvc.compute_slot_mapping(positions, block_tables, block_size, is_prefill)
-        else:
+        if not is_prefill:
             slot_mapping = kvc.SlotsFromTables(positions, block_tables, block_size)
+        else:
+            slot_mapping = _k.host().slot_mapping(positions, block_tables, block_size, token_row_ids)
+            if slot_mapping is None:  # operands to convert, or to complain about
+                slot_mapping = (kvc.compute_slot_mapping(positions, block_tables, block_size, is_prefill) if token_row_ids is None else
+                                kvc.compute_packed_slot_mapping(positions, block_tables, token_row_ids, block_size))
         batch, query_len = positions.shape
         singles = pairs = None
         if query_lens_host is not None and token_row_ids is not None:
