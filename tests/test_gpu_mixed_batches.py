@@ -139,3 +139,29 @@ def test_calls_in_flight_give_what_they_give_one_by_one(kind, monkeypatch):
     K.check_device_status()
     ws = K._workspaces[torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream]
     assert not ws.buf[:64].any()  # the word that lets the decode rows run beside the tiles is left zero
+
+
+def test_decode_rows_beside_tiles_replay_from_a_graph(monkeypatch):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    monkeypatch.setenv("NVJ_CHECK_STATUS", "0")
+    monkeypatch.setenv("NVJ_POISON_OUTPUT", "0")
+    monkeypatch.setenv("NVJ_MIXED_SIDE_BY_SIDE", "0")  # one stream, as launched eagerly
+    calls, cache = _calls("mixed", 3)
+    start = cache.k_cache.clone(), cache.v_cache.clone()
+    ref = [c() for c in calls]
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        calls[0]()
+    stream.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        outs = [c() for c in calls]
+    for _ in range(5):
+        cache.k_cache.copy_(start[0])
+        cache.v_cache.copy_(start[1])
+        graph.replay()
+        for a, b in zip(outs, ref):
+            assert torch.equal(a, b)
+    ws = K._workspaces[torch.cuda.current_device(), stream.cuda_stream]
+    torch.cuda.synchronize()
+    assert not ws.buf[:64].any()
