@@ -110,6 +110,18 @@ class B200Backend:
                     max_kv_len=width * block_size, token_row_ids=None,
                     max_query_len=query_len if max_query_len is None else max_query_len, single_token_rows=None,
                     query_tile_pairs=None)
+        # A prefill's slots are made here and stay what they are; a decode batch's when an append or a reader wants them (the
+        # fused append + decode kernel and the append resolve them in their own launch).
+        made = _k.host().prefill_slots(positions, block_tables, seq_lens, block_size, token_row_ids) if is_prefill else None
+        if made is not None and query_start_loc is not None:  # a prefill batch whose shapes agree: as above
+            slots, batch, query_len = made
+            singles, pairs = self._count_rows(query_lens_host) if token_row_ids is not None else (None, None)
+            return kvc.attention_metadata(
+                slot_mapping=slots, block_tables=block_tables, seq_lens=seq_lens, query_start_loc=query_start_loc,
+                num_prefill_tokens=batch * query_len if num_prefill_tokens is None else num_prefill_tokens,
+                num_decode_tokens=0 if num_decode_tokens is None else num_decode_tokens, positions=positions, max_kv_len=None,
+                token_row_ids=token_row_ids, max_query_len=query_len if max_query_len is None else max_query_len,
+                single_token_rows=singles, query_tile_pairs=pairs)
         if positions.ndim != 2:
             raise ValueError("positions must be a 2D tensor [batch, query_len]")
         if block_tables.ndim != 2:
@@ -128,24 +140,16 @@ class B200Backend:
                 raise ValueError("positions and block_tables batch dimensions must match")
             if positions.shape[0] != seq_lens.shape[0]:
                 raise ValueError("positions and seq_lens batch dimensions must match")
-        # A prefill's slots are made here and stay what they are; a decode batch's when an append or a reader wants them (the
-        # fused append + decode kernel and the append resolve them in their own launch).
-        if not is_prefill:
-            slot_mapping = kvc.SlotsFromTables(positions, block_tables, block_size)
+        if made is not None:
+            slot_mapping = made[0]
+        elif token_row_ids is not None:
+            slot_mapping = kvc.compute_packed_slot_mapping(positions, block_tables, token_row_ids, block_size)
+        elif is_prefill:
+            slot_mapping = kvc.compute_slot_mapping(positions, block_tables, block_size, is_prefill)
         else:
-            slot_mapping = _k.host().slot_mapping(positions, block_tables, block_size, token_row_ids)
-            if slot_mapping is None:  # operands to convert, or to complain about
-                slot_mapping = (kvc.compute_slot_mapping(positions, block_tables, block_size, is_prefill) if token_row_ids is None else
-                                kvc.compute_packed_slot_mapping(positions, block_tables, token_row_ids, block_size))
+            slot_mapping = kvc.SlotsFromTables(positions, block_tables, block_size)
         batch, query_len = positions.shape
-        singles = pairs = None
-        if query_lens_host is not None and token_row_ids is not None:
-            singles = pairs = 0
-            for n in query_lens_host:
-                if n == 1:
-                    singles += 1
-                elif n > 1:
-                    pairs -= -int(n) // 64
+        singles, pairs = self._count_rows(query_lens_host) if token_row_ids is not None else (None, None)
         if query_start_loc is None:
             if is_prefill:
                 query_start_loc = torch.cat([torch.zeros(1, dtype=torch.int32, device=seq_lens.device),
@@ -162,6 +166,19 @@ class B200Backend:
             token_row_ids=token_row_ids,
             max_query_len=max_query_len if max_query_len is not None else query_len,
             single_token_rows=singles, query_tile_pairs=pairs)
+
+    @staticmethod
+    def _count_rows(query_lens):
+        """(rows of one query token, 64-token tiles of the others); nothing of a batch whose lengths the host does not know."""
+        if query_lens is None:
+            return None, None
+        singles = pairs = 0
+        for n in query_lens:
+            if n == 1:
+                singles += 1
+            elif n > 1:
+                pairs -= -int(n) // 64
+        return singles, pairs
 
     def _one_token_per_row(self, rows, seq_lens):
         """query_start_loc of a batch with one query token per row: a constant per batch size and device, built once."""

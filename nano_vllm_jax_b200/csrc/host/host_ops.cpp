@@ -514,23 +514,50 @@ PyObject* decode_shape(PyObject* const* a, Py_ssize_t n) {
   return Py_BuildValue("LLL", (long long)pos->size(0), (long long)pos->size(1), (long long)tab->size(1));
 }
 
+// The int32 slots [rows, cols] of positions, from the rows' block tables: 1, or 0 when an operand has to be converted or complained
+// about, or -1 with a Python error set.
+int make_slots(const at::Tensor* pos, const at::Tensor* tab, const at::Tensor* rid, long long bs, at::Tensor* out) {
+  if (!pos || !tab || !pos->is_cuda() || pos->dim() != 2 || tab->dim() != 2 || bs < 1) return 0;
+  const int dev = pos->get_device();
+  if (!meta(*pos, dev) || !meta(*tab, dev) || tab->size(0) < 1 || tab->size(1) < 1) return 0;
+  if (rid ? (!meta(*rid, dev) || rid->sizes() != pos->sizes()) : pos->size(0) > tab->size(0)) return 0;
+  void* stream = stream_of(dev);
+  *out = empty(pos->sizes(), at::kInt, dev);
+  int rc;
+  NVJ_CALL(rc, lib.slot_mapping(i32(*pos), i32(*tab), rid ? i32(*rid) : nullptr, (int)pos->size(0), (int)pos->size(1), (int)tab->size(0),
+                                (int)tab->size(1), (int)bs, static_cast<int32_t*>(out->data_ptr()), stream));
+  return finished(rc, "nvj_compute_slot_mapping", dev, stream, false, false) ? 1 : -1;
+}
+
 // slot_mapping(positions [rows, cols], block_tables, block_size, token_row_ids | None) -> int32 [rows, cols]
 PyObject* slot_mapping(PyObject* const* a, Py_ssize_t n) {
   if (!args_are(n, 4)) return nullptr;
-  const at::Tensor *pos = tensor(a[0]), *tab = tensor(a[1]), *rid = a[3] == Py_None ? nullptr : tensor(a[3]);
+  const at::Tensor* rid = a[3] == Py_None ? nullptr : tensor(a[3]);
   const long long bs = PyLong_AsLongLong(a[2]);
   if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
-  if (!pos || !tab || (!rid && a[3] != Py_None) || !pos->is_cuda() || pos->dim() != 2 || tab->dim() != 2 || bs < 1) NVJ_NONE();
-  const int dev = pos->get_device();
-  if (!meta(*pos, dev) || !meta(*tab, dev) || tab->size(0) < 1 || tab->size(1) < 1) NVJ_NONE();
-  if (rid ? (!meta(*rid, dev) || rid->sizes() != pos->sizes()) : pos->size(0) > tab->size(0)) NVJ_NONE();
-  void* stream = stream_of(dev);
-  at::Tensor out = empty(pos->sizes(), at::kInt, dev);
-  int rc;
-  NVJ_CALL(rc, lib.slot_mapping(i32(*pos), i32(*tab), rid ? i32(*rid) : nullptr, (int)pos->size(0), (int)pos->size(1), (int)tab->size(0),
-                                (int)tab->size(1), (int)bs, static_cast<int32_t*>(out.data_ptr()), stream));
-  if (!finished(rc, "nvj_compute_slot_mapping", dev, stream, false, false)) return nullptr;
+  if (!rid && a[3] != Py_None) NVJ_NONE();
+  at::Tensor out;
+  const int made = make_slots(tensor(a[0]), tensor(a[1]), rid, bs, &out);
+  if (made < 0) return nullptr;
+  if (made == 0) NVJ_NONE();
   return THPVariable_Wrap(std::move(out));
+}
+
+// prefill_slots(positions [rows, cols], block_tables, seq_lens, block_size, token_row_ids | None) -> (slots, rows, cols) of a prefill
+// batch whose shapes agree
+PyObject* prefill_slots(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 5)) return nullptr;
+  const at::Tensor *pos = tensor(a[0]), *tab = tensor(a[1]), *len = tensor(a[2]), *rid = a[4] == Py_None ? nullptr : tensor(a[4]);
+  const long long bs = PyLong_AsLongLong(a[3]);
+  if (PyErr_Occurred()) { PyErr_Clear(); NVJ_NONE(); }
+  if (!pos || !tab || !len || (!rid && a[4] != Py_None) || pos->dim() != 2 || tab->dim() != 2 || len->dim() != 1 ||
+      len->size(0) != tab->size(0) || (!rid && pos->size(0) != tab->size(0)))
+    NVJ_NONE();
+  at::Tensor out;
+  const int made = make_slots(pos, tab, rid, bs, &out);
+  if (made < 0) return nullptr;
+  if (made == 0) NVJ_NONE();
+  return Py_BuildValue("NLL", THPVariable_Wrap(std::move(out)), (long long)pos->size(0), (long long)pos->size(1));
 }
 
 // ---- prefix hashes --------------------------------------------------------------------------------------------------
@@ -1041,6 +1068,7 @@ PyMethodDef methods[] = {
     NVJ_FAST(hybrid_copy, "snapshot or restore of GDN state rows, or None"),
     NVJ_FAST(pack_batch, "a batch's lists on the device"),
     NVJ_FAST(slot_mapping, "flat cache slots of positions, or None"),
+    NVJ_FAST(prefill_slots, "flat cache slots of a prefill batch and its shape, or None"),
     {"init", init, METH_VARARGS, "resolve the library's entry points and keep the callbacks"},
     {"set_workspace", set_workspace, METH_VARARGS, "hand over a (device, stream)'s workspace"},
     {"set_status_word", set_status_word, METH_VARARGS, "hand over a (device, stream)'s status word"},
