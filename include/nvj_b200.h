@@ -166,8 +166,8 @@ int nvj_qk_norm_rope_kv_append(const void* q, int64_t q_token_stride, int64_t q_
 /*
  * Bytes of caller-owned scratch the decode entry points need for `max_batch`
  * rows on the current device.  The front of the buffer (64 bytes of status, 256 bytes of group
- * counters, 4 bytes per row) holds the status word and the arrival counters and must be zero before the
- * first use (nvj_paged_decode_workspace_init does that); the kernels leave them zero again on success.
+ * counters, 4 bytes per row) holds the status word, the word that lets a mixed batch's decode rows run beside its
+ * tiles and the arrival counters, and must be zero before the first use (nvj_paged_decode_workspace_init does that); the kernels leave them zero again on success.
  * The partial results live at the END of the buffer, so one buffer serves calls of any batch size up to
  * `max_batch`, of either decode entry point and of any width, one after another: pass the same
  * `workspace_bytes` (the buffer's size) on every call.  One workspace serves one stream at a time.
@@ -332,8 +332,8 @@ int nvj_paged_decode_window(const void* q, int q_dtype, const void* k_cache_laye
  *   out        [token_bucket, num_q_heads, head_dim] float32
  *   workspace  nullable decode workspace (nvj_paged_decode_workspace_bytes(rows)); when given,
  *              rows that hold exactly one query token (the decode rows of a mixed batch,
- *              nanovllm_jax/engine/scheduler.py:956-1032) are served by the streaming decode
- *              kernel instead of a query tile.  A workspace of nvj_paged_prefill_workspace_bytes(rows)
+ *              nanovllm_jax/engine/scheduler.py:956-1032) are served by a decode
+ *              kernel instead of a query tile (one too small or not 16-byte aligned leaves them to the tiles).  A workspace of nvj_paged_prefill_workspace_bytes(rows)
  *              bytes also lets the CTA-pair tile kernel (variants 0, 4, 5) split every tile's key
  *              range over several CTA pairs when the batch is too short to fill the GPU (a
  *              512-token chunk is 16 pairs on 74 pair slots): the splits park their un-normalised
@@ -561,7 +561,7 @@ int nvj_copy_many_async(void* const* dst, const void* const* src, const size_t* 
  */
 int nvj_stage_in(void* const* dst, const void* const* src, const size_t* bytes, int n, nvj_stream_t stream);
 
-/* 1 when nvj_paged_decode* serves a bf16 batch of this size with the cluster kernel, else 0. */
+/* 1 when nvj_paged_decode* serves a bf16 batch of this size with the cluster kernel, else 0 (more than 65535 rows among others). */
 int nvj_paged_decode_on_clusters(int batch, int table_width);
 
 /* ------------------------------------------------------------------ tokens */
