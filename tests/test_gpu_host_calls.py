@@ -104,3 +104,26 @@ def test_when_the_slots_of_a_batch_are_made(kind, read_first):
     be.write_kv(0, new, new, cache, md)
     moved = 4 if kind == "decode" and not read_first else 0
     assert cache.k_cache[0, :, :, 0, 0].nonzero().tolist() == [[b, t + moved] for b in (2, 3) for t in range(3)]
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_the_mapped_append_writes_what_the_slot_mapping_says(packed):
+    """nvj_kv_append_mapped against nvj_compute_slot_mapping + nvj_kv_append: row ids outside the table, rows shorter than the batch."""
+    from nano_vllm_jax_b200 import _lib
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    lib, rng = _lib.load(), np.random.default_rng(8)
+    (rows, cols), pool = ((1, 40) if packed else (4, 9)), 64
+    tables = to_torch(rng.permutation(pool)[:24].reshape(4, 6).astype(np.int32))
+    pos = to_torch(np.stack([rng.permutation(96)[:cols] for _ in range(rows)]).astype(np.int32))
+    rid = to_torch(np.sort(rng.integers(-1, 6, size=(1, cols))).astype(np.int32)) if packed else None
+    qsl = to_torch(np.array([0, 9, 18, 30, 35] if packed else [0, 9, 12, 21, 21], np.int32))
+    new = [to_torch(rng.standard_normal((rows, cols, 2, 256)).astype(np.float32)).to(torch.bfloat16) for _ in range(2)]
+    want, got = ([torch.zeros((pool, BS, 2, 256), dtype=torch.bfloat16, device="cuda") for _ in range(2)] for _ in range(2))
+    K.kv_append_slots(*new, K.compute_slot_mapping(pos, tables, BS, rid), *want, query_start_loc=qsl, packed=packed)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rc = lib.nvj_kv_append_mapped(new[0].data_ptr(), new[1].data_ptr(), _lib.NVJ_BF16, pos.data_ptr(), tables.data_ptr(),
+                                  rid.data_ptr() if packed else None, 4, 6, BS, qsl.data_ptr(), 4, int(packed), rows, cols,
+                                  got[0].data_ptr(), got[1].data_ptr(), _lib.NVJ_BF16, pool * BS, 2, 256, status.data_ptr(),
+                                  torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and int(status) == 0 and float(want[0].float().abs().sum()) > 0
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
