@@ -624,6 +624,9 @@ static ClusterForm cluster_form(int batch, int blocks, int sms, int room, int pe
   // finer split per head is as fast or faster.
   const bool both = 100LL * 3 * kHkv * batch > (long long)kCmPerSm * sms;
   if (!both) return {false, cluster_size(2LL * batch, blocks, room, kCmWarps, per_sm, 8, kClMaxCluster), kCmWarps};
+  // On the SMs that another kernel leaves, the places are few and eight CTAs per row fill them evenly (96 rows of up to 2048 keys
+  // beside three chunks of 300, 88 SMs, six layers: 380 us, with four, which fill them 1.5 times, 396).
+  if (room < sms) return {true, cluster_size(batch, blocks, room, kCmWarps / 2, per_sm, 8, 8), kCmWarps / 2};
   ClusterForm f{true, cluster_size(batch, blocks, room, kCmWarps / 2, per_sm, 4, 8), kCmWarps / 2};
   // More than four CTAs per row only beyond 24 blocks per walker, and then six where they fill the places (three to an SM) more
   // than 2.5 times, eight where they do not: a CTA that finds no block costs its start all the same.  256 rows under a table of
