@@ -56,7 +56,7 @@ MIN_TIMED_STEPS = 100
 DECODE_KERNELS = {
     True: dict(name="decode_cluster_mma_kernel (fused append + paged GQA decode on thread-block clusters, tensor-core tiles)",
                dram=1351.09e6, algorithmic=1346.54e6, capture="256 rows of 1024 - 4096 tokens"),
-    False: dict(name="decode_wide_kernel at width 1 (fused append + paged GQA decode, TMA-staged, tensor-core tiles)",
+    False: dict(name="decode_stream_kernel (fused append + paged GQA decode, TMA-staged, tensor-core tiles)",
                 dram=354.93e6, algorithmic=356.35e6, capture="--workload c2small on that kernel"),
 }
 

@@ -250,4 +250,53 @@ __device__ __forceinline__ void fold_parts(const DecodeParams& p, float* red, in
   }
 }
 
+// A row that several CTAs share, once this CTA (its kDecodeThreads threads, all of which call it) has stored its partial: counts
+// the partial in; the CTA that delivers the row's last one folds them all, token by token, in two levels when there are many.
+// `qbase`: the row's first query token in the output.  `red` is the fold's scratch, `last_flag` a word of shared memory.
+template <int kBatch = 13>
+__device__ __forceinline__ void finish_shared_row(const DecodeParams& p, float* red, int& last_flag, const Seg& s, const Partition& pt,
+                                                  long long qbase, int tid) {
+  const int slot_rows = p.width * kHq;  // rows of one partial slot: [token][head]
+  const long long row_g0 = s.g0 - s.j0;
+  const int c_lo = pt.cta_of(row_g0);
+  const int c_hi = pt.cta_of(row_g0 + s.nb - 1);
+  const int grid = gridDim.x;
+  const bool tree = c_hi - c_lo + 1 > kTreeMergeMin;
+  const int cg = blockIdx.x / kMergeGroup, g_lo = c_lo / kMergeGroup, g_hi = c_hi / kMergeGroup;
+  const int first = tree ? max(c_lo, cg * kMergeGroup) : c_lo;
+  const int last = tree ? min(c_hi, cg * kMergeGroup + kMergeGroup - 1) : c_hi;
+  int32_t* counter = tree ? p.group_counters + 2 * cg + (cg == g_lo ? 1 : 0) : p.counters + s.b;
+  __threadfence();
+  named_bar_sync(1, kDecodeThreads);
+  if (tid == 0) last_flag = (atomicAdd(counter, 1) == last - first) ? 1 : 0;
+  named_bar_sync(1, kDecodeThreads);
+  if (!last_flag) return;
+  __threadfence();
+  if (!tree) {
+    for (int tok = 0; tok < p.width; ++tok) {
+      fold_parts<true, kBatch>(p, red, tid, 0, c_lo, c_lo, c_hi - c_lo + 1, (qbase + tok) * kHq, slot_rows, tok * kHq);
+      named_bar_sync(1, kDecodeThreads);
+    }
+    if (tid == 0) *counter = 0;
+    return;
+  }
+  for (int tok = 0; tok < p.width; ++tok) {
+    fold_parts<false, kBatch>(p, red, tid, 0, first, c_lo, last - first + 1, 2LL * grid + 2 * cg + (cg == g_lo ? 1 : 0), slot_rows,
+                          tok * kHq);
+    named_bar_sync(1, kDecodeThreads);
+  }
+  if (tid == 0) *counter = 0;
+  __threadfence();
+  named_bar_sync(1, kDecodeThreads);
+  if (tid == 0) last_flag = (atomicAdd(p.counters + s.b, 1) == g_hi - g_lo) ? 1 : 0;
+  named_bar_sync(1, kDecodeThreads);
+  if (!last_flag) return;
+  __threadfence();
+  for (int tok = 0; tok < p.width; ++tok) {
+    fold_parts<true, kBatch>(p, red, tid, 2LL * grid, g_lo, g_lo, g_hi - g_lo + 1, (qbase + tok) * kHq, slot_rows, tok * kHq);
+    named_bar_sync(1, kDecodeThreads);
+  }
+  if (tid == 0) p.counters[s.b] = 0;
+}
+
 }  // namespace nvj

@@ -182,6 +182,7 @@ bool decode_cluster_pays(int batch, int table_width);  // a bf16 batch is short 
 int launch_decode_pipelined(const DecodeParams& p, int num_ctas, cudaStream_t stream);
 int decode_wide_num_ctas();  // 1 per SM of the current device
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // tensor-core streaming kernels, width 1..8
+int launch_decode_stream(const DecodeParams& p, cudaStream_t stream);  // one query token per row, bf16
 int launch_decode_cluster_wide(const DecodeParams& p, cudaStream_t stream);  // rows of 2 - 4 tokens, few and short
 bool decode_cluster_wide_pays(const DecodeParams& p);
 int run_decode_wide(DecodeParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);  // checks, carves, launches

@@ -43,17 +43,6 @@
 
 namespace nvj {
 
-// Development aid, compiled in only with -DNVJ_PHASE_TIMING: thread 0 of every CTA stamps the global timer at the
-// kernel's phase boundaries, and nvj_debug_phase_ns copies the stamps out.
-#ifdef NVJ_PHASE_TIMING
-__device__ unsigned long long g_phase_ns[256][12];  // slots 0-7: stamps; 8: the SM the CTA ran on; 9: its number of blocks; 10: ns spent finishing segments; 11: folds it did
-#define NVJ_PHASE(i) do { if (threadIdx.x == 0) g_phase_ns[blockIdx.x][i] = global_timer_ns(); } while (0)
-#define NVJ_PHASE_NOTE(i, v) do { if (threadIdx.x == 0) g_phase_ns[blockIdx.x][i] = (v); } while (0)
-#else
-#define NVJ_PHASE(i) do { } while (0)
-#define NVJ_PHASE_NOTE(i, v) do { } while (0)
-#endif
-
 // An even number, so that a stage always holds blocks of the same parity and is read by the same four warps: a
 // parity wait can only tell two consecutive phases of an mbarrier apart, and a warp that waited for every other
 // phase of a stage's barrier could take an unfinished phase for the one after it, release the stage early and
@@ -78,16 +67,6 @@ struct WideSmem {
   int is_last;
   int abort_flag;
 };
-
-// One whole block (16 KiB) of the 4-D view {64 dims, token, 64-dim chunk, kv head} of a cache layer.
-__device__ __forceinline__ void w_tma_block(uint32_t dst, const CUtensorMap* map, int token, uint32_t bar) {
-  uint64_t policy;  // every block is read once: do not let it displace what the L2 is good for
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(token), "r"(0), "r"(0), "r"(bar), "l"(policy)
-      : "memory");
-}
 
 __device__ __forceinline__ void w_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -121,9 +100,11 @@ __device__ __forceinline__ void w_issue_block(const DecodeParams& p, WideSmem& s
   const uint32_t full = smem_u32(&sm.full_bar[stage]);
   const int blk = sm.ring_blk[n & (kRing - 1)];
   if (sm.ring_rows[n & (kRing - 1)] > 0) {
+    uint64_t policy;  // every block is read once: do not let it displace what the L2 is good for
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     mbar_arrive_expect_tx(full, 2u * kTileBytes);
-    w_tma_block(smem_u32(sm.tiles[stage][0]), k_map, blk * kBlk, full);
-    w_tma_block(smem_u32(sm.tiles[stage][1]), v_map, blk * kBlk, full);
+    tma_load_block(smem_u32(sm.tiles[stage][0]), k_map, blk * kBlk, full, policy);
+    tma_load_block(smem_u32(sm.tiles[stage][1]), v_map, blk * kBlk, full, policy);
   } else {
     mbar_arrive(full);
   }
@@ -143,7 +124,7 @@ struct WideState {
 // `rows` keys of the block exist, the block starts at key `key0` of the row.
 __device__ __forceinline__ void w_process_block(uint32_t kt, uint32_t vt, int lane, int dh, int rows, int key0, float c,
                                                 WideState& st) {
-  const int g = lane >> 2, t = lane & 3;
+  const int t = lane & 3;
   // ---- scores
   float s[2][4];
 #pragma unroll
@@ -245,7 +226,7 @@ __device__ __forceinline__ void w_finish_segment(const DecodeParams& p, WideSmem
   }
   named_bar_sync(1, kDecodeThreads);
   const bool whole_row = (s.j0 == 0 && s.j1 == s.nb);
-  const long long qbase = p.packed_rows ? (long long)p.query_start_loc[s.b] : (long long)s.b * p.width;  // first query token
+  const long long qbase = (long long)s.b * p.width;  // first query token
   const int slot = partial_slot(blockIdx.x, s.j0 == 0);
   const int slot_rows = p.width * kHq;  // rows of one partial slot: [token][head]
   if (kDual || par == 0) {
@@ -277,54 +258,10 @@ __device__ __forceinline__ void w_finish_segment(const DecodeParams& p, WideSmem
     named_bar_sync(1, kDecodeThreads);  // the exchange buffer is free again
     return;
   }
-  // ---- cross-CTA: count this partial in; the last arrival folds
-  const long long row_g0 = s.g0 - s.j0;
-  const int c_lo = pt.cta_of(row_g0);
-  const int c_hi = pt.cta_of(row_g0 + s.nb - 1);
-  const int grid = gridDim.x;
-  const bool tree = c_hi - c_lo + 1 > kTreeMergeMin;
-  const int cg = blockIdx.x / kMergeGroup, g_lo = c_lo / kMergeGroup, g_hi = c_hi / kMergeGroup;
-  const int first = tree ? max(c_lo, cg * kMergeGroup) : c_lo;
-  const int last = tree ? min(c_hi, cg * kMergeGroup + kMergeGroup - 1) : c_hi;
-  int32_t* counter = tree ? p.group_counters + 2 * cg + (cg == g_lo ? 1 : 0) : p.counters + s.b;
-  __threadfence();
-  named_bar_sync(1, kDecodeThreads);
-  if (tid == 0) sm.is_last = (atomicAdd(counter, 1) == last - first) ? 1 : 0;
-  named_bar_sync(1, kDecodeThreads);
-  NVJ_PHASE(7);
-  if (!sm.is_last) return;
-  __threadfence();
-  if (!tree) {
-    for (int tok = 0; tok < p.width; ++tok) {
-      fold_parts<true, 13>(p, sm.red, tid, 0, c_lo, c_lo, c_hi - c_lo + 1, (qbase + tok) * kHq, slot_rows, tok * kHq);
-      named_bar_sync(1, kDecodeThreads);
-    }
-    if (tid == 0) *counter = 0;
-    return;
-  }
-  for (int tok = 0; tok < p.width; ++tok) {
-    fold_parts<false, 13>(p, sm.red, tid, 0, first, c_lo, last - first + 1, 2LL * grid + 2 * cg + (cg == g_lo ? 1 : 0), slot_rows,
-                      tok * kHq);
-    named_bar_sync(1, kDecodeThreads);
-  }
-  if (tid == 0) *counter = 0;
-  __threadfence();
-  named_bar_sync(1, kDecodeThreads);
-  if (tid == 0) sm.is_last = (atomicAdd(p.counters + s.b, 1) == g_hi - g_lo) ? 1 : 0;
-  named_bar_sync(1, kDecodeThreads);
-  if (!sm.is_last) return;
-  __threadfence();
-  for (int tok = 0; tok < p.width; ++tok) {
-    fold_parts<true, 13>(p, sm.red, tid, 2LL * grid, g_lo, g_lo, g_hi - g_lo + 1, (qbase + tok) * kHq, slot_rows,
-                     tok * kHq);
-    named_bar_sync(1, kDecodeThreads);
-  }
-  if (tid == 0) p.counters[s.b] = 0;
+  finish_shared_row(p, sm.red, sm.is_last, s, pt, qbase, tid);
 }
 
-// kWindow: decode_row_len.  A decode step has no window: 128 rows of 8192 - 32768 keys take 784 us (886 once the power cap is
-// reached) without the limits compiled in and 793 (898) with them.
-template <bool kDual, bool kWindow>
+template <bool kDual>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
 decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, DecodeParams p) {
   extern __shared__ unsigned char w_smem_raw[];
@@ -332,7 +269,6 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grid = gridDim.x;
 
-  NVJ_PHASE(0);
   // The kernel opens with three dependent trips to memory (lengths -> block ids -> K/V blocks).  While the first is
   // under way, pull what the others will need towards the SM: the tensor maps, and this CTA's share of the block
   // tables into the L2 (all CTAs together cover the tables, so the second trip ends in the L2 for everyone).
@@ -353,16 +289,13 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   for (int base = 0; base < p.batch; base += kDecodeThreads) {
     const int b = base + threadIdx.x;
     int len = 0;
-    if (b < p.batch) len = decode_row_len<kWindow>(p, b);
+    if (b < p.batch) len = decode_row_len(p, b);
     if (base == 0) first_n = blocks_in_sequence(p, (len + kBlk - 1) / kBlk);
     mine += blocks_in_sequence(p, (len + kBlk - 1) / kBlk);
-    // rows without keys get zeros; in a packed batch only the rows this pass owns (one query token) are touched
-    const bool mine_to_zero = b < p.batch && len <= 0 && (b % grid) == (int)blockIdx.x &&
-                              (!p.packed_rows || p.query_start_loc[b + 1] - p.query_start_loc[b] == 1);
-    const unsigned idle = __ballot_sync(kFullMask, mine_to_zero);
+    const unsigned idle = __ballot_sync(kFullMask, b < p.batch && len <= 0 && (b % grid) == (int)blockIdx.x);  // rows without keys
     for (unsigned m = idle; m; m &= m - 1) {
       const int bb = base + (warp << 5) + (__ffs(m) - 1);
-      float4* o = reinterpret_cast<float4*>(p.out + (p.packed_rows ? (long long)p.query_start_loc[bb] : (long long)bb * p.width) * kHq * kD);
+      float4* o = reinterpret_cast<float4*>(p.out + (long long)bb * p.width * kHq * kD);
       for (int i = lane; i < p.width * kHq * kD / 4; i += 32) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
@@ -374,7 +307,6 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   const long long g0 = pt.start(blockIdx.x);
   const long long g1 = pt.start(blockIdx.x + 1);
   if (g0 == g1) return;
-  NVJ_PHASE(1);
 
   // ---- pass 2: locate (row, block) of g0
   long long carry = 0;
@@ -386,7 +318,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   for (int base = 0; base < p.batch && carry <= g0; base += kDecodeThreads) {
     const int b = base + threadIdx.x;
     int n = 0;
-    if (b < p.batch) n = blocks_in_sequence(p, (decode_row_len<kWindow>(p, b) + kBlk - 1) / kBlk);
+    if (b < p.batch) n = blocks_in_sequence(p, (decode_row_len(p, b) + kBlk - 1) / kBlk);
     int chunk_total = 0;
     const long long excl = carry + cta_inclusive_scan(n, sm.scan, chunk_total) - n;
     if (n > 0 && excl <= g0 && g0 < excl + n) { sm.start_b = b; sm.start_j = (int)(g0 - excl); }
@@ -400,28 +332,16 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     mbar_fence_init();
   }
   __syncthreads();
-  NVJ_PHASE(2);
-  const int n_iters = blocks_in_range<kWindow>(p, sm.start_b, sm.start_j, g0, g1);  // the range's real blocks
+  const int n_iters = blocks_in_range(p, sm.start_b, sm.start_j, g0, g1);  // the range's real blocks
   if (n_iters == 0) return;
-#ifdef NVJ_PHASE_TIMING
-  {
-    unsigned smid;
-    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-    NVJ_PHASE_NOTE(8, (unsigned long long)smid);
-    NVJ_PHASE_NOTE(9, (unsigned long long)n_iters);
-    NVJ_PHASE_NOTE(10, 0ull);
-    NVJ_PHASE_NOTE(11, 0ull);
-  }
-#endif
 
   FillState fs;
   fs.b = sm.start_b; fs.jn = sm.start_j; fs.g = g0; fs.j = 0; fs.nsegs = 0; fs.has = false;
-  fill_ring<kWindow>(p, sm, fs, g1, 0, n_iters < kRing ? n_iters : kRing);
+  fill_ring(p, sm, fs, g1, 0, n_iters < kRing ? n_iters : kRing);
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int n = 0; n < kWStages && n < n_iters; ++n) w_issue_block(p, sm, &k_map, &v_map, n, false);
   }
-  NVJ_PHASE(3);
 
   int b = sm.start_b, j = sm.start_j;
   long long g = g0;
@@ -431,10 +351,9 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   const int fg = lane >> 2, ft = lane & 3;
   const float c = p.scale * kLog2e;
   WideState st;
-  while (next_seg<kWindow>(p, b, j, g, g1, s)) {
+  while (next_seg(p, b, j, g, g1, s)) {
     // query rows of this KV head as A fragments: row = token * 4 + head of the group; rows past the width are zero
-    // (packed_rows: the row's single query token sits at query_start_loc[b]; its length is already capped by its position)
-    const long long qbase = p.packed_rows ? (long long)p.query_start_loc[s.b] : (long long)s.b * p.width;
+    const long long qbase = (long long)s.b * p.width;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int row = fg + 8 * r, tok = (kDual ? 4 * par : 0) + (row >> 2);
@@ -446,7 +365,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
         st.qa[ks][r] = real ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 2 * ft) : 0u;
         st.qa[ks][r + 2] = real ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8 + 2 * ft) : 0u;
       }
-      st.pos[r] = real ? (p.positions && !p.new_k ? p.positions[qbase + tok] : 0x7fffffff) : -1;
+      st.pos[r] = real ? (p.positions ? p.positions[qbase + tok] : 0x7fffffff) : -1;
       st.m[r] = kNegBig;
       st.l[r] = 0.f;
     }
@@ -455,51 +374,17 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
 #pragma unroll
       for (int e = 0; e < 4; ++e) st.o[n][e] = 0.f;
 
-    // Fused append (width 1).  The CTA that owns block min(pos / 16, nb - 1) of the row writes the new K/V row
-    // (one warp per KV head); its copy of that block may race with the store, so every warp that reads the block
-    // overwrites the row in the staged tile, from the same source, once the copy has landed: no fence is needed
-    // and nothing waits for the store.
-    int patch_j = -1, patch_t = 0;
-    if (p.new_k) {
-      const int pos = p.pre_append ? p.seq_lens[s.b] : p.positions[s.b];
-      const int jt = pos >> 4;
-      const int jw = jt < s.nb - 1 ? jt : s.nb - 1;
-      if (pos >= 0 && jw >= s.j0 && jw < s.j1) {
-        const long long tgt = jt < p.table_width ? (long long)p.block_tables[decode_table_base(p, s.b) + jt] : -1;
-        if (tgt >= 0 && tgt < p.num_blocks) {
-          if (par == 0 && dh == 0) {
-            const long long src = (long long)s.b * kTokenBytes + kvh * kRowBytes + lane * 16;
-            const long long dst = (tgt * kBlk + (pos & 15)) * kTokenBytes + kvh * kRowBytes + lane * 16;
-            *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst) =
-                *reinterpret_cast<const uint4*>(static_cast<const char*>(p.new_k) + src);
-            *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst) =
-                *reinterpret_cast<const uint4*>(static_cast<const char*>(p.new_v) + src);
-          }
-          if (jt == jw && pos < s.len) { patch_j = jw; patch_t = pos & 15; }
-        } else if (warp == 0 && lane == 0) {
-          atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
-        }
-      }
-    }
     for (int jb = s.j0; jb < s.j1; ++jb, ++it) {
       if ((it & (kRing / 2 - 1)) == 0 && it > 0) {
         named_bar_sync(1, kDecodeThreads);
         const int n0 = it + kRing / 2;
-        if (n0 < n_iters) fill_ring<kWindow>(p, sm, fs, g1, n0, n_iters - n0 < kRing / 2 ? n_iters - n0 : kRing / 2);
+        if (n0 < n_iters) fill_ring(p, sm, fs, g1, n0, n_iters - n0 < kRing / 2 ? n_iters - n0 : kRing / 2);
         named_bar_sync(1, kDecodeThreads);
       }
       if (!kDual && (it & 1) != par) continue;
       const int stage = it % kWStages;
       mbar_wait(smem_u32(&sm.full_bar[stage]), (uint32_t)(it / kWStages) & 1u, &sm.abort_flag, p.status);
       const int rows = sm.ring_rows[it & (kRing - 1)];
-      if (it == 0) NVJ_PHASE(4);
-      if (jb == patch_j) {  // lane l carries 16-byte piece l of the KV head's 512-byte row; the source is cache-hot
-        const long long src = (long long)s.b * kTokenBytes + kvh * kRowBytes + lane * 16;
-        const uint32_t off = kvh * 8192 + (lane >> 3) * 2048 + patch_t * 128 + (((lane & 7) ^ (patch_t & 7)) << 4);
-        *reinterpret_cast<uint4*>(sm.tiles[stage][0] + off) = *reinterpret_cast<const uint4*>(static_cast<const char*>(p.new_k) + src);
-        *reinterpret_cast<uint4*>(sm.tiles[stage][1] + off) = *reinterpret_cast<const uint4*>(static_cast<const char*>(p.new_v) + src);
-        __syncwarp();
-      }
       if (rows > 0)
         w_process_block(smem_u32(sm.tiles[stage][0]) + kvh * 8192, smem_u32(sm.tiles[stage][1]) + kvh * 8192, lane, dh, rows,
                         jb * kBlk, c, st);
@@ -512,18 +397,7 @@ decode_wide_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
       }
       __syncwarp();
     }
-    NVJ_PHASE(5);
-#ifdef NVJ_PHASE_TIMING
-    const unsigned long long fin0 = global_timer_ns();
-#endif
     w_finish_segment<kDual>(p, sm, s, st, warp, lane, pt);
-#ifdef NVJ_PHASE_TIMING
-    if (threadIdx.x == 0) {
-      g_phase_ns[blockIdx.x][10] += global_timer_ns() - fin0;
-      g_phase_ns[blockIdx.x][11] += (unsigned long long)sm.is_last;
-    }
-#endif
-    NVJ_PHASE(6);
   }
   // Only after a timeout can copies still be in flight with nobody waiting for them: hold the
   // CTA's shared memory until they have landed.
@@ -595,6 +469,10 @@ bool tensor_map_cached(CUtensorMap* map, int kind, const void* base, uint64_t ex
   return true;
 }
 
+bool block_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t tokens) {
+  return w_encode_fn() && tensor_map_cached(map, 0, cache_layer, tokens, w_make_map);
+}
+
 static PerDeviceFlags g_wide_ctas;  // 0 = not queried yet
 
 int decode_wide_num_ctas() {  // one per SM of the current device
@@ -618,7 +496,7 @@ static size_t wide_acc_bytes(int n, int width) { return ws_round(sizeof(float) *
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
   if (p.width < 1 || p.width > kWideMaxWidth || p.num_blocks < 1 || p.num_blocks * kBlk > 0x7fffffffLL || !w_encode_fn())
     return NVJ_ERR_UNSUPPORTED;
-  int n = decode_wide_num_ctas();
+  const int n = decode_wide_num_ctas();
   if (n <= 0) return NVJ_ERR_LAUNCH;
   if (p.wide_form == 3 || (p.wide_form == 0 && p.cta_limit <= 0 && decode_cluster_wide_pays(p)))
     return launch_decode_cluster_wide(p, stream);
@@ -633,34 +511,25 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
     if (rc != NVJ_ERR_UNSUPPORTED || p.wide_form == 2) return rc;
   }
   if (p.width > kWMaxWidth) return NVJ_ERR_UNSUPPORTED;
-  if (p.cta_limit > 0 && p.cta_limit < n) n = p.cta_limit;
+  if (p.width == 1) return launch_decode_stream(p, stream);
   DecodeParams q = p;
   q.row_end_cost = kRowEndCost;
   CUtensorMap k_map, v_map;
-  if (!tensor_map_cached(&k_map, 0, p.k_cache, (uint64_t)p.num_blocks * kBlk, w_make_map) ||
-      !tensor_map_cached(&v_map, 0, p.v_cache, (uint64_t)p.num_blocks * kBlk, w_make_map))
+  if (!block_map_cached(&k_map, p.k_cache, (uint64_t)p.num_blocks * kBlk) || !block_map_cached(&v_map, p.v_cache, (uint64_t)p.num_blocks * kBlk))
     return NVJ_ERR_UNSUPPORTED;
   static PerDeviceFlags smem_opted_in;
   const int smem = (int)sizeof(WideSmem) + 1024;
   if (!once_per_device(smem_opted_in, [smem](int) {
-        return cudaFuncSetAttribute(decode_wide_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-               cudaFuncSetAttribute(decode_wide_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-               cudaFuncSetAttribute(decode_wide_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+        return cudaFuncSetAttribute(decode_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+               cudaFuncSetAttribute(decode_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
       }))
     return NVJ_ERR_LAUNCH;
-  const bool window = p.max_len > 0 || p.cap_positions;
-  auto* kernel = p.width > 4 ? decode_wide_kernel<true, true> : window ? decode_wide_kernel<false, true> : decode_wide_kernel<false, false>;
-  launch_after(kernel, n, kDecodeThreads, smem, stream, k_map, v_map, q);
+  launch_after(p.width > 4 ? decode_wide_kernel<true> : decode_wide_kernel<false>, n, kDecodeThreads, smem, stream, k_map, v_map, q);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
 }  // namespace nvj
 
-#ifdef NVJ_PHASE_TIMING
-extern "C" int nvj_debug_phase_ns(unsigned long long* host_out) {  // [256][8]
-  return cudaMemcpyFromSymbol(host_out, nvj::g_phase_ns, sizeof(nvj::g_phase_ns)) == cudaSuccess ? 0 : 1;
-}
-#endif
 
 extern "C" size_t nvj_paged_decode_wide_workspace_bytes(int max_batch) {
   using namespace nvj;

@@ -84,6 +84,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
 }
+// One whole block (16 KiB, both KV heads) of a cache layer through its block_map_cached() view, for data that is read once.
+__device__ __forceinline__ void tma_load_block(uint32_t dst, const CUtensorMap* map, int token, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(token), "r"(0), "r"(0), "r"(bar), "l"(policy)
+      : "memory");
+}
 
 // Shared-memory matrix descriptor, 128-byte swizzle (layout type 2), descriptor version 1.
 // Offsets are in bytes; the 4 low bits are dropped by the encoding.
@@ -148,5 +155,8 @@ __device__ __forceinline__ bool um_elect_one() {
 // keyed by base address and extent (a map holds nothing else), and calls `make` only on a miss.
 typedef bool (*TensorMapMaker)(CUtensorMap* map, const void* base, uint64_t extent);
 bool tensor_map_cached(CUtensorMap* map, int kind, const void* base, uint64_t extent, TensorMapMaker make);
+// A bf16 cache layer of `tokens` tokens as {64 dims, token, 64-dim chunk, kv head}: a box is one 16-token block of both KV heads and
+// lands as [kv head][chunk][16 tokens][128 B] with the 128-byte swizzle.
+bool block_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t tokens);
 
 }  // namespace nvj
