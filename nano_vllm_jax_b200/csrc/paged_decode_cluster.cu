@@ -467,11 +467,16 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     if (jb < nb) {
       const char* src = cache + (blk < 0 ? 0 : blk) * kBlk * kTokB + kvh * kRowB + lane * 16;
       const int last = len - 1 - jb * kBlk, mine = new_key - jb * kBlk;
-      const uint32_t size = blk < 0 ? 0u : 16u;
+      if (blk >= 0 && last >= kBlk - 1 && (unsigned)mine >= (unsigned)kBlk) {  // a whole block as it lies in the cache: constant offsets
 #pragma unroll
-      for (int r = 0; r < kBlk; ++r) {
-        const int rr = r < last ? r : (last < kBlk - 1 ? last : r);
-        cl_copy16_or_zero(at + r * kRowB + ((lane ^ (r & 7)) << 4), rr == mine ? fresh : src + rr * kTokB, size);
+        for (int r = 0; r < kBlk; ++r) cl_copy16(at + r * kRowB + ((lane ^ (r & 7)) << 4), src + r * kTokB);
+      } else {
+        const uint32_t size = blk < 0 ? 0u : 16u;
+#pragma unroll 8
+        for (int r = 0; r < kBlk; ++r) {
+          const int rr = r < last ? r : (last < kBlk - 1 ? last : r);
+          cl_copy16_or_zero(at + r * kRowB + ((lane ^ (r & 7)) << 4), rr == mine ? fresh : src + rr * kTokB, size);
+        }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");  // (also an empty one: the waits count groups)
