@@ -58,22 +58,28 @@ __device__ __forceinline__ int mapped_slot(const int32_t* block_tables, int row,
 // Returns the flat destination slot of token i, or -1 when the token is masked
 // out or its slot lies outside the pool (the latter is flagged).
 __device__ __forceinline__ long long resolve_slot(const AppendParams& p, int i) {
-  if (p.valid_mask && p.valid_mask[i] == 0) return -1;
   long long slot;
   if (p.slot_mapping || p.block_tables) {
+    // What decides about the token and what makes its slot are asked for together: one trip to memory for a mapping, two for a table
+    // (three and four one after the other, most of what a small batch's append takes).
+    const int mask = p.valid_mask ? p.valid_mask[i] : 1;
+    const int r = p.packed ? 0 : i / p.n_cols;
+    int count = 0x7fffffff, at = i;  // the token counts if at < count
     if (p.query_start_loc) {
       if (p.packed) {
-        if (i >= p.query_start_loc[p.qsl_rows]) return -1;
+        count = p.query_start_loc[p.qsl_rows];
       } else {
-        const int r = i / p.n_cols, t = i - r * p.n_cols;
         if (r >= p.qsl_rows) return -1;
-        if (t >= p.query_start_loc[r + 1] - p.query_start_loc[r]) return -1;
+        count = p.query_start_loc[r + 1] - p.query_start_loc[r];
+        at = i - r * p.n_cols;
       }
     }
     slot = p.slot_mapping ? p.slot_mapping[i]
                           : mapped_slot(p.block_tables, p.token_row_ids ? p.token_row_ids[i] : i / p.n_cols, p.positions[i],
                                         p.table_rows, p.table_width, p.page_size);
+    if (mask == 0 || at >= count) return -1;
   } else {
+    if (p.valid_mask && p.valid_mask[i] == 0) return -1;
     const int b = p.batch_indices ? p.batch_indices[i] : i;
     const int pos = p.positions[i];
     if (b < 0 || b >= p.batch || pos < 0) {

@@ -131,3 +131,25 @@ def test_multimodal_three_row_positions(rows, cols):
     q3, _, _ = K.qk_norm_rope_kv_append(*args, to_torch(np.stack([c["pos"]] * 3)), to_torch(c["slots"]), kc3[0], vc3[0])
     torch.cuda.synchronize()
     assert torch.equal(q1, q3) and torch.equal(kc1, kc3) and torch.equal(vc1, vc3)
+
+
+@pytest.mark.parametrize("rot", [64, 128, 256])  # one, two and four sets of 32 frequencies per warp
+def test_large_angles_and_wide_rotations_against_64_bits(rot):
+    """Positions up to 2^24: the fp32 angle's cosine and sine in 64 bits.  The kernel's are within 2e-7 of those (an fp32 rounding of
+    the reduced angle and one of the result), so a bf16 rounding flips in about 2e-7 / 2^-9 = 1e-4 of the cases."""
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    c = _case(rot, 40, 1, 64)
+    rng = np.random.default_rng(rot)
+    pos = np.exp2(rng.uniform(0, 24, size=c["pos"].shape)).astype(np.int32)
+    kc, vc = to_torch(c["kc"]), to_torch(c["vc"])
+    q_out, _, _ = K.qk_norm_rope_kv_append(to_torch(c["qg"])[..., :256], to_torch(c["k"]), to_torch(c["v"]), to_torch(c["qw"]), to_torch(c["kw"]),
+                                           to_torch(pos), to_torch(c["slots"]), kc[0], vc[0], rope_theta=1e7, rotary_dim=rot)
+    y = N.rms_norm(c["qg"][..., :256], c["qw"]).astype(np.float32)
+    ang = (pos.astype(np.float32)[..., None] * K.rope_inv_freq(1e7, rot, "cuda").cpu().numpy()).astype(np.float64)[:, :, None, :]
+    cos, sin = (f(ang).astype(np.float32).astype(bfloat16).astype(np.float32) for f in (np.cos, np.sin))
+    a, b = y[..., : rot // 2], y[..., rot // 2: rot]
+    want = np.concatenate([a * cos - b * sin, b * cos + a * sin, y[..., rot:]], axis=-1).astype(bfloat16)
+    got = to_numpy(q_out).reshape(want.shape)
+    w = want.astype(np.float32)
+    assert (np.abs(got.astype(np.float32) - w) <= 2.0 ** -7 * np.abs(w).max(axis=-1, keepdims=True)).all()
+    assert (_ulp_diff(got, want) > 0).mean() < 2e-3
