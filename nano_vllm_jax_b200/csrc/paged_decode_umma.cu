@@ -54,7 +54,7 @@ constexpr int kUdMaxWidth = 16;  // 64 query rows per KV head: two softmax warps
 constexpr int kUdRowEndCost = 6;  // what a row end costs a CTA here, in blocks (6 and 12 measured alike, 18 and 24 worse)
 
 struct UdSmem {
-  alignas(1024) char k[kUdStages][4][kUdTileBlocks * kBlk * 128];  // [stage][64-d chunk][64 keys][128 B], swizzled
+  alignas(1024) char k[kUdStages][kUdTileBlocks][kUdHalfBlock];    // [stage][block][8-key group][64-d chunk][8 keys][128 B], swizzled
   alignas(1024) char v[kUdStages][kUdTileBlocks][kUdHalfBlock];    // [stage][block][64-d chunk][16 keys][128 B], swizzled
   alignas(8) unsigned long long full_bar[kUdStages], empty_bar[kUdStages], q_full, s_full[2], p_full, pv_done, o_free;
   float red[384];
@@ -63,13 +63,18 @@ struct UdSmem {
   uint32_t tmem_base;
 };
 
-// One box of the 4-D view {64 dims, token, 64-dim chunk, kv head} of a cache layer: with the V map all four chunks of
-// one KV head's half of a block (8 KiB), with the K map one chunk of it (2 KiB).
-__device__ __forceinline__ void ud_tma_box(uint32_t dst, const CUtensorMap* map, int token, int chunk, int kvh, uint32_t bar,
-                                           uint64_t policy) {
+// One KV head's half of a block (8 KiB): V through the view of ud_make_v_map ...
+__device__ __forceinline__ void ud_tma_v(uint32_t dst, const CUtensorMap* map, int token, int kvh, uint32_t bar, uint64_t policy) {
   asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(token), "r"(chunk), "r"(kvh), "r"(bar), "l"(policy)
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %2, %4}], [%5], %6;"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(token), "r"(kvh), "r"(bar), "l"(policy)
+      : "memory");
+}
+// ... and K through that of ud_make_k_map.  `group` counts groups of eight tokens.
+__device__ __forceinline__ void ud_tma_k(uint32_t dst, const CUtensorMap* map, int group, int kvh, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %2, %2, %3, %4}], [%5], %6;"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(group), "r"(kvh), "r"(bar), "l"(policy)
       : "memory");
 }
 
@@ -103,8 +108,8 @@ __device__ __forceinline__ void ud_producer(const CUtensorMap* k_map, const CUte
         for (int i = 0; i < cnt; ++i) {
           const int blk = __shfl_sync(kFullMask, id, i0 + i);
           const int token = blk >= 0 ? blk * kBlk : oob;
-          if (lane < 4) ud_tma_box(smem_u32(&sm.k[stage][lane][0]) + i * (kBlk * 128), k_map, token, lane, kvh, fb, policy);
-          else if (lane == 4) ud_tma_box(smem_u32(&sm.v[stage][i][0]), v_map, token, 0, kvh, fb, policy);
+          if (lane == 0) ud_tma_k(smem_u32(&sm.k[stage][i][0]), k_map, token / 8, kvh, fb, policy);
+          else if (lane == 1) ud_tma_v(smem_u32(&sm.v[stage][i][0]), v_map, token, kvh, fb, policy);
         }
         __syncwarp();
       }
@@ -121,11 +126,11 @@ __device__ __forceinline__ bool ud_issue_s(UdSmem& sm, const DecodeParams& p, ui
   tc_fence_after_sync();
   if (um_elect_one()) {
     constexpr uint32_t idesc = umma_idesc(kUdTileBlocks * kBlk, false);
-    const uint64_t k_desc = k_desc0 + (uint64_t)((stage * 4 * kUdTileBlocks * kBlk * 128) >> 4);
+    const uint64_t k_desc = k_desc0 + (uint64_t)((stage * kUdTileBlocks * kUdHalfBlock) >> 4);
     const uint32_t d = tmem + kUdColS + (gt & 1u) * 64;
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks)  // 16 dims per MMA: 8 columns of Q; K chunk ks / 4, 32 bytes into its swizzled rows
-      umma_bf16_ts(d, tmem + kUdColQ + ks * 8, k_desc + (uint64_t)(((ks >> 2) * (kUdTileBlocks * kBlk * 128) + (ks & 3) * 32) >> 4),
+      umma_bf16_ts(d, tmem + kUdColQ + ks * 8, k_desc + (uint64_t)(((ks >> 2) * (8 * 128) + (ks & 3) * 32) >> 4),
                    idesc, ks > 0 ? 1u : 0u);
     umma_commit(smem_u32(&sm.s_full[gt & 1u]));
   }
@@ -135,7 +140,7 @@ __device__ __forceinline__ bool ud_issue_s(UdSmem& sm, const DecodeParams& p, ui
 
 __device__ __forceinline__ void ud_mma_warp(UdSmem& sm, const DecodeParams& p, uint32_t tmem, int b, int j, long long g,
                                             long long g1) {
-  const uint64_t k_desc0 = umma_desc(smem_u32(&sm.k[0][0][0]), 16, 1024);          // K: keys are rows, dims contracted
+  const uint64_t k_desc0 = umma_desc(smem_u32(&sm.k[0][0][0]), 16, 4 * 8 * 128);   // K: keys are rows (groups of 8: 4 KiB apart), dims contracted
   const uint64_t v_desc0 = umma_desc(smem_u32(&sm.v[0][0][0]), kBlk * 128, 1024);  // V: 64-d chunks 2 KiB apart, keys contracted
   Seg s;
   uint32_t gt = 0;  // tiles so far, over all segments: picks the stage, the score buffer and the barrier phases
@@ -503,15 +508,25 @@ static UdEncodeTiledFn ud_encode_fn() {
 }
 
 // A cache layer [token, kv head, 256] bf16 seen as {64 dims, token, 64-dim chunk, kv head}: one box of {64, 16, 4, 1}
-// is one KV head's half of a block and lands as [chunk][16 tokens][128 B] with the 128-byte swizzle in every panel;
-// a box of {64, 16, 1, 1} is one such panel.
-template <int kChunks>
-static bool ud_make_map(CUtensorMap* map, const void* base, uint64_t tokens) {
+// is one KV head's half of a block and lands as [chunk][16 tokens][128 B] with the 128-byte swizzle in every panel.
+static bool ud_make_v_map(CUtensorMap* map, const void* base, uint64_t tokens) {
   const cuuint64_t dims[4] = {64, tokens, 4, (cuuint64_t)kHkv};
   const cuuint64_t strides[3] = {(cuuint64_t)kTokenBytes, 128, (cuuint64_t)kRowBytes};
-  const cuuint32_t box[4] = {64, (cuuint32_t)kBlk, kChunks, 1};
+  const cuuint32_t box[4] = {64, (cuuint32_t)kBlk, 4, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   return ud_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// The same with the tokens in groups of eight, {64 dims, token of the group, 64-dim chunk, group, kv head}: a box of {64, 8, 4, 2, 1}
+// lands as [group][chunk][8 tokens][128 B], so that the groups of a tile of several blocks are evenly spaced (4 KiB), as the
+// rows of one operand have to be.
+static bool ud_make_k_map(CUtensorMap* map, const void* base, uint64_t tokens) {
+  const cuuint64_t dims[5] = {64, 8, 4, tokens / 8, (cuuint64_t)kHkv};
+  const cuuint64_t strides[4] = {(cuuint64_t)kTokenBytes, 128, 8 * (cuuint64_t)kTokenBytes, (cuuint64_t)kRowBytes};
+  const cuuint32_t box[5] = {64, 8, 4, kBlk / 8, 1};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return ud_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -527,8 +542,8 @@ int launch_decode_umma(const DecodeParams& p, cudaStream_t stream) {
   if (ctas < 2) return NVJ_ERR_LAUNCH;
   const int ranges = ctas / 2;
   CUtensorMap k_map, v_map;
-  if (!tensor_map_cached(&k_map, 4, p.k_cache, (uint64_t)p.num_blocks * kBlk, ud_make_map<1>) ||
-      !tensor_map_cached(&v_map, 3, p.v_cache, (uint64_t)p.num_blocks * kBlk, ud_make_map<4>))
+  if (!tensor_map_cached(&k_map, 4, p.k_cache, (uint64_t)p.num_blocks * kBlk, ud_make_k_map) ||
+      !tensor_map_cached(&v_map, 3, p.v_cache, (uint64_t)p.num_blocks * kBlk, ud_make_v_map))
     return NVJ_ERR_UNSUPPORTED;
   static PerDeviceFlags smem_opted_in;
   constexpr int kSmemBytes = (int)sizeof(UdSmem) + 1024;
