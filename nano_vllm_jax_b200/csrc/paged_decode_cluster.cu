@@ -26,8 +26,10 @@ namespace nvj {
 
 // ---- f32 caches (and f16 ones under f32 queries): fp32 products on the CUDA cores --------------------------------
 // Every warp keeps a unit of 4 keys in flight in shared memory of its own (16-byte cp.async; the next unit's K rows are
-// requested as soon as the scores are computed, its V rows after the weighted sum); lane l
-// copies and later reads dims 8 l .. 8 l + 7 of every row, so this needs no barrier of any kind.  The 4 keys x 4 heads
+// requested as soon as the scores are computed, its V rows after the weighted sum); lane l copies and later reads the same
+// eight dims of every row, so this needs no barrier of any kind: 8 l .. 8 l + 7 of a 16-bit row, 4 l .. 4 l + 3 and
+// 128 + 4 l .. of an f32 row.  (Every copy of a warp is then 512 bytes in a row.  With 8 l .. of an f32 row each copy took half of
+// 32 sectors, and every sector crossed from the L2 twice.)  The 4 keys x 4 heads
 // partial dot products are reduced by a select-free butterfly: lanes hold keys and heads in permuted order.
 constexpr int kClWarps = 8;  // two CTAs per SM: a warp's chain of shuffles is long, four warps per scheduler overlap theirs
 constexpr int kClThreads = kClWarps * 32;
@@ -55,12 +57,8 @@ __device__ __forceinline__ void cl_copy16(uint32_t dst, const char* src) {
 }
 template <typename T>
 __device__ __forceinline__ void cl_copy_row(uint32_t row, const char* src, int lane) {
-  if constexpr (sizeof(T) == 4) {  // dims 8 l .. 8 l + 3 in the row's first half, 8 l + 4 .. in its second: no bank conflicts
-    cl_copy16(row + lane * 16, src + lane * 32);
-    cl_copy16(row + 512 + lane * 16, src + lane * 32 + 16);
-  } else {
-    cl_copy16(row + lane * 16, src + lane * 16);
-  }
+  cl_copy16(row + lane * 16, src + lane * 16);
+  if constexpr (sizeof(T) == 4) cl_copy16(row + 512 + lane * 16, src + 512 + lane * 16);
 }
 __device__ __forceinline__ uint4 cl_lds(uint32_t a) {
   uint4 v;
@@ -162,23 +160,29 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   const int len = decode_row_len(p, b);  // the same in every thread of the cluster
   const long long qi = decode_query_index(p, b);
   if (p.packed_rows && p.query_start_loc[b + 1] - p.query_start_loc[b] != 1) return;  // not this pass's row (the whole cluster leaves)
+  constexpr bool kFull = sizeof(T) == 4;
+  const int d0 = lane * (kFull ? 4 : 8), d1 = kFull ? kD / 2 + lane * 4 : lane * 8 + 4;  // this lane's dims: four from each
   // query heads in slot order (slot h of a lane holds head h ^ hperm), times scale * log2(e)
   const int rperm = lane >> 3, h_own = (lane >> 1) & 3;
   float2 q2[kG][4];
 #pragma unroll
   for (int h = 0; h < kG; ++h) {
-    const long long off = (qi * kHq + kvh * kG + (h ^ h_own)) * kD + lane * 8;
-    if (p.q_dtype == NVJ_F32) {
-      const float4 x = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + off);
-      const float4 y = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + off + 4);
-      q2[h][0] = make_float2(x.x, x.y); q2[h][1] = make_float2(x.z, x.w);
-      q2[h][2] = make_float2(y.x, y.y); q2[h][3] = make_float2(y.z, y.w);
-    } else if (p.q_dtype == NVJ_BF16) {
-      ClRaw<__nv_bfloat16> r{*reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.q) + off)};
-      cl_unpack(r, q2[h]);
-    } else {
-      ClRaw<__half> r{*reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + off)};
-      cl_unpack(r, q2[h]);
+    const long long off = (qi * kHq + kvh * kG + (h ^ h_own)) * kD;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const long long at = off + (i ? d1 : d0);
+      if (p.q_dtype == NVJ_F32) {
+        const float4 x = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + at);
+        q2[h][2 * i] = make_float2(x.x, x.y); q2[h][2 * i + 1] = make_float2(x.z, x.w);
+      } else {
+        const uint2 x = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(p.q) + at);
+        if (p.q_dtype == NVJ_BF16) {
+          q2[h][2 * i] = bf16x2_to_float2(x.x); q2[h][2 * i + 1] = bf16x2_to_float2(x.y);
+        } else {
+          q2[h][2 * i] = __half22float2(*reinterpret_cast<const __half2*>(&x.x));
+          q2[h][2 * i + 1] = __half22float2(*reinterpret_cast<const __half2*>(&x.y));
+        }
+      }
     }
     const float c = p.scale * kLog2e;
 #pragma unroll
@@ -328,8 +332,8 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   for (int h = 0; h < kG; ++h) {
     const float l = __shfl_sync(kFullMask, lh, h * 2);
     if (lane == 0) sm.ml[warp][h] = make_float2(m4[h], l);
-    *reinterpret_cast<float4*>(&sm.acc[warp][h][lane * 8]) = make_float4(acc[h][0].x, acc[h][0].y, acc[h][1].x, acc[h][1].y);
-    *reinterpret_cast<float4*>(&sm.acc[warp][h][lane * 8 + 4]) = make_float4(acc[h][2].x, acc[h][2].y, acc[h][3].x, acc[h][3].y);
+    *reinterpret_cast<float4*>(&sm.acc[warp][h][d0]) = make_float4(acc[h][0].x, acc[h][0].y, acc[h][1].x, acc[h][1].y);
+    *reinterpret_cast<float4*>(&sm.acc[warp][h][d1]) = make_float4(acc[h][2].x, acc[h][2].y, acc[h][3].x, acc[h][3].y);
   }
   __syncthreads();
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
