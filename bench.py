@@ -474,7 +474,7 @@ def run_b200(args, w):
 
     # The same step replayed from a CUDA graph over device-resident metadata: fused append + decode (pre-append form:
     # the row's token goes to position seq_lens[b]) -> token argmax that also advances the lengths, one graph launch
-    # of two kernels per step.  With N > 1 the argmax launch also publishes the tokens to every rank over NVLink and
+    # of one or two kernels per step.  With N > 1 the argmax launch also publishes the tokens to every rank over NVLink and
     # collects the step before.
     from nano_vllm_jax_b200.engine.resident_decode import DecodeStepGraph, ResidentDecodeMetadata
     meta = ResidentDecodeMetadata(rows, tables.shape[1], BS, device=dev)
@@ -604,7 +604,8 @@ def run_b200(args, w):
         per_rank = sorted(float(t.item()) for t in every)
         rank_kernel_us = {"min": per_rank[0], "median": statistics.median(per_rank), "max": per_rank[-1]}
 
-    decode_kernel = DECODE_KERNELS[bool(_lib.load().nvj_paged_decode_on_clusters(rows, tables.shape[1]))]
+    on_clusters = bool(_lib.load().nvj_paged_decode_on_clusters(rows, tables.shape[1]))
+    decode_kernel = DECODE_KERNELS[on_clusters]
     # roofline of the fused append+decode kernel: bytes of the timed launches over their duration
     kernel_ms = [e0.elapsed_time(e1) for _, e0, e1 in timed_events]
     ms_kernel = sum(kernel_ms)
@@ -659,9 +660,9 @@ def run_b200(args, w):
                             "from pinned host memory and its whole result back; compute stage "
                             + ("replayed from a CUDA graph per slot" if pipe_capture else "launched eagerly"),
                     "serial_value": total_rows / (ms_e2e_serial / K_steps * 1e-3), "serial_ms_per_step": ms_e2e_serial / K_steps},
-            # per step of the timed pass: fused append+decode, token argmax with the metadata advance (N > 1: the same
-            # launch also collects and publishes)
-            "gpu_launches": 2 * K_steps,
+            # per step of the timed pass: fused append+decode and the token argmax with the metadata advance, in one launch where
+            # the batch runs on clusters (N > 1: a second launch, which also collects and publishes)
+            "gpu_launches": (1 if world == 1 and on_clusters else 2) * K_steps,
             "step_mode": step_mode,
             "eager_value": total_rows / (ms_eager / K_steps * 1e-3), "eager_ms_per_step": ms_eager / K_steps,
             "roofline": {"bound": "hbm", "kernel": decode_kernel["name"],

@@ -236,6 +236,20 @@ int nvj_paged_decode_fused_append(const void* q, int q_dtype,
                                   int variant, nvj_stream_t stream);
 
 /*
+ * A whole decode step over device-resident metadata: the pre-append form of nvj_paged_decode_fused_append, then what
+ * nvj_row_argmax_advance does with its output (tokens[b] = index of row b's first largest output value; seq_lens and, unless
+ * NULL, positions advanced).  One launch where the batch runs on thread-block clusters (the token pick then is part of the
+ * attention kernel), two otherwise; the results are those of the two calls.
+ */
+int nvj_paged_decode_append_pick(const void* q, int q_dtype, const void* new_k, const void* new_v,
+                                 void* k_cache_layer, void* v_cache_layer, int kv_dtype,
+                                 int64_t num_blocks, int block_size, int num_kv_heads, int head_dim,
+                                 int num_q_heads, const int32_t* block_tables, int table_width,
+                                 int32_t* seq_lens, int32_t* positions, int batch, float scale, float* out,
+                                 int32_t* tokens, void* workspace, size_t workspace_bytes, nvj_stream_t stream);
+
+
+/*
  * nvj_paged_decode for callers that cannot allocate device memory (no counterpart
  * in the reference).  A custom-call handler that only receives its operands, or a
  * plugin that runs inside another runtime's memory pool, has nowhere to keep the

@@ -57,6 +57,9 @@ SIGNATURES = {
                                               c_int, c_int, c_void_p, c_int, c_void_p, c_int,
                                               c_float, c_void_p, c_void_p, c_size_t, c_int,
                                               c_void_p]),
+    "nvj_paged_decode_append_pick": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int, c_int,
+                                             c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p,
+                                             c_void_p, c_void_p, c_size_t, c_void_p]),
     "nvj_paged_decode_static_scratch": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int64, c_int,
                                                 c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int,
                                                 c_float, c_void_p, c_void_p, c_void_p]),

@@ -25,6 +25,13 @@ static int carve_workspace(DecodeParams& p, void* workspace, size_t bytes, int n
   return carve_decode_workspace(p, workspace, bytes, ws_ml_bytes(num_ctas), ws_acc_bytes(num_ctas));
 }
 
+// The token pick of a step whose attention kernel does not make it.
+static int pick_behind(const DecodeParams& p, int32_t* tokens, cudaStream_t stream) {
+  return tokens ? nvj_row_argmax_advance(p.out, p.batch, p.num_q_heads * p.head_dim, tokens, p.pick_lens, p.pick_positions, p.table_width,
+                                         p.block_size, p.status, stream)
+                : NVJ_OK;
+}
+
 static int run_decode(DecodeParams& p, void* workspace, size_t workspace_bytes, int variant,
                       cudaStream_t stream) {
   if (p.batch < 0 || p.table_width < 0 || p.num_blocks < 0 || p.block_size <= 0 ||
@@ -50,17 +57,25 @@ static int run_decode(DecodeParams& p, void* workspace, size_t workspace_bytes, 
   const bool bf16 = p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16;
   // Short bf16 batches and every f32 / f16 cache: the cluster kernel.
   if (variant == 4 || (variant == 0 && cluster_ok && (bf16 ? !p.kv_indptr && decode_cluster_pays(p.batch, p.table_width) : !fast_ok))) {
+    int32_t* const wanted = p.pick_tokens;
+    if (wanted && !decode_cluster_picks(p)) p.pick_tokens = nullptr;
     const int rc4 = launch_decode_cluster(p, stream);
+    if (rc4 == NVJ_OK && wanted && !p.pick_tokens) return pick_behind(p, wanted, stream);
+    p.pick_tokens = wanted;
     if (rc4 != NVJ_ERR_UNSUPPORTED || variant == 4) return rc4;
   }
   if ((variant == 2 && !fast_ok) || (variant == 3 && !mma_ok)) return NVJ_ERR_UNSUPPORTED;
   if (variant == 3 || (variant == 0 && mma_ok)) {
     p.width = 1;
     const int rc3 = launch_decode_wide(p, stream);
+    if (rc3 == NVJ_OK) return pick_behind(p, p.pick_tokens, stream);
     if (rc3 != NVJ_ERR_UNSUPPORTED || variant == 3) return rc3;
     p.width = 0;
   }
-  if (variant == 2 || (variant == 0 && fast_ok)) return launch_decode_pipelined(p, num_ctas, stream);
+  if (variant == 2 || (variant == 0 && fast_ok)) {
+    const int rc2 = launch_decode_pipelined(p, num_ctas, stream);
+    return rc2 == NVJ_OK ? pick_behind(p, p.pick_tokens, stream) : rc2;
+  }
   if (p.new_k) {
     if (p.kv_indptr) return NVJ_ERR_UNSUPPORTED;
     const int a = append_decode_rows(p.new_k, p.new_v, p.pre_append ? p.seq_lens : p.positions, p.seq_lens,
@@ -70,7 +85,8 @@ static int run_decode(DecodeParams& p, void* workspace, size_t workspace_bytes, 
                                      p.batch, p.status, stream);
     if (a != NVJ_OK) return a;
   }
-  return launch_decode_generic(p, stream);
+  const int rc1 = launch_decode_generic(p, stream);
+  return rc1 == NVJ_OK ? pick_behind(p, p.pick_tokens, stream) : rc1;
 }
 
 }  // namespace nvj
@@ -152,6 +168,37 @@ extern "C" int nvj_paged_decode_fused_append(const void* q, int q_dtype, const v
   p.kv_dtype = kv_dtype;
   p.scale = scale;
   return nvj::run_decode(p, workspace, workspace_bytes, variant, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int nvj_paged_decode_append_pick(const void* q, int q_dtype, const void* new_k, const void* new_v, void* k_cache_layer,
+                                            void* v_cache_layer, int kv_dtype, int64_t num_blocks, int block_size, int num_kv_heads,
+                                            int head_dim, int num_q_heads, const int32_t* block_tables, int table_width,
+                                            int32_t* seq_lens, int32_t* positions, int batch, float scale, float* out,
+                                            int32_t* tokens, void* workspace, size_t workspace_bytes, nvj_stream_t stream) {
+  if (batch > 0 && (!new_k || !new_v || !tokens)) return NVJ_ERR_INVALID_ARGUMENT;
+  nvj::DecodeParams p{};
+  p.q = q;
+  p.k_cache = static_cast<const char*>(k_cache_layer);
+  p.v_cache = static_cast<const char*>(v_cache_layer);
+  p.block_tables = block_tables;
+  p.seq_lens = seq_lens;
+  p.new_k = new_k;
+  p.new_v = new_v;
+  p.pick_tokens = tokens;
+  p.pick_lens = seq_lens;
+  p.pick_positions = positions;
+  p.out = out;
+  p.num_blocks = num_blocks;
+  p.batch = batch;
+  p.table_width = table_width;
+  p.block_size = block_size;
+  p.num_kv_heads = num_kv_heads;
+  p.num_q_heads = num_q_heads;
+  p.head_dim = head_dim;
+  p.q_dtype = q_dtype;
+  p.kv_dtype = kv_dtype;
+  p.scale = scale;
+  return nvj::run_decode(p, workspace, workspace_bytes, 0, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nvj_paged_decode_on_clusters(int batch, int table_width) {

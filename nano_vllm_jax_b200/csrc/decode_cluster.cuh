@@ -40,6 +40,10 @@ __device__ __forceinline__ float2 cl_ld2(uint32_t a) {
   return v;
 }
 
+__device__ __forceinline__ void cl_st2(uint32_t a, float x, int y) {
+  asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(__float_as_uint(x)), "r"(y) : "memory");
+}
+
 __device__ __forceinline__ void cm_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -79,16 +83,17 @@ __device__ __forceinline__ uint32_t cm_pack(float x, float y, bool rest) {
   }
 }
 
-template <class Kernel>
-inline int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const DecodeParams& p, int cluster, int heads, int threads, int smem,
-                           cudaStream_t stream) {
+// Clusters of `cluster` CTAs: one per row and KV head (`heads` of them), or per row where they span the heads (cluster.y).
+template <class... Params, class... Args>
+inline int launch_clusters(void (*kernel)(Params...), PerDeviceFlags& opted_in, const DecodeParams& p, dim3 cluster, int heads, int threads,
+                           int smem, cudaStream_t stream, const Args&... args) {
   if (!once_per_device(opted_in, [&](int) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
                cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
       }))
     return NVJ_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cluster, heads, p.batch);
+  cfg.gridDim = dim3(cluster.x, heads, p.batch);
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -96,12 +101,12 @@ inline int launch_clusters(Kernel kernel, PerDeviceFlags& opted_in, const Decode
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster;
-  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.x = cluster.x;
+  attr[0].val.clusterDim.y = cluster.y;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
 // CTAs per cluster for `groups` clusters of rows of up to `blocks` blocks, when a CTA walks `walkers` blocks at a time: as many

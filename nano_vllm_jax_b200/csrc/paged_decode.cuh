@@ -58,6 +58,11 @@ struct DecodeParams {
   // in front like any other.  The launch ends only after the kernel in front has, so that the stream's order holds behind
   // both, and leaves the word zero.
   int32_t* beside;
+  // token pick in the same launch (nullable; pre-append form on the cluster kernel only, decode_cluster_picks): the index of the
+  // row's first largest output value goes to pick_tokens[b], and the row's resident metadata is advanced as advance_row does
+  int32_t* pick_tokens;
+  int32_t* pick_lens;       // the rows' lengths: seq_lens, writable
+  int32_t* pick_positions;  // nullable
   // which wide kernel serves rows of several query tokens: 0 = automatic (mma.sync tiles up to width 4, tcgen05 beyond),
   // 1 = mma.sync tiles, 2 = tcgen05, 3 = thread-block clusters
   int wide_form;
@@ -179,6 +184,7 @@ int decode_num_ctas();  // 2 per SM of the current device
 int launch_decode_generic(const DecodeParams& p, cudaStream_t stream);
 int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream);  // short batches; f32 and f16 caches
 bool decode_cluster_pays(int batch, int table_width);  // a bf16 batch is short enough for it
+bool decode_cluster_picks(const DecodeParams& p);      // its launch for this call would serve pick_tokens too
 int launch_decode_pipelined(const DecodeParams& p, int num_ctas, cudaStream_t stream);
 int decode_wide_num_ctas();  // 1 per SM of the current device
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // tensor-core streaming kernels, width 1..8

@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "decode_cluster.cuh"
+#include "row_argmax.cuh"
 
 namespace nvj {
 
@@ -102,13 +103,14 @@ __device__ __forceinline__ void cl_end_beside(const DecodeParams& p) {
 }
 // The CTAs' sums [head][pitch] and (max, sum) pairs, at the same places in every CTA of the cluster, into the output: rank
 // r takes its 1 / ctas of the float4 pieces of [heads][256 dims].
-template <int kHeads>
-__device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, const float2* ML, int ctas, uint32_t rank, int threads,
-                                                float* dst) {
+// `store` gets a piece's index and its four values; `base`: the cluster's rank of the first of these CTAs.
+template <int kHeads, class Store>
+__device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, const float2* ML, int ctas, int rank, int base, int threads,
+                                                Store store) {
   constexpr int kPieces = kHeads * kD / 4;
   const int per = (kPieces + ctas - 1) / ctas;
   for (int i = threadIdx.x; i < per; i += threads) {
-    const int piece = (int)rank * per + i, h = piece >> 6, d = (piece & 63) * 4;
+    const int piece = rank * per + i, h = piece >> 6, d = (piece & 63) * 4;
     if (piece >= kPieces) break;
     float2 e[kClMaxCluster];
     float4 x[kClMaxCluster];
@@ -117,8 +119,8 @@ __device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, con
       e[c] = make_float2(kNegBig, 0.f);
       x[c] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < ctas) {
-        e[c] = cl_ld2(cl_map(ML + h, c));
-        x[c] = cl_ld4(cl_map(acc + h * pitch + d, c));
+        e[c] = cl_ld2(cl_map(ML + h, base + c));
+        x[c] = cl_ld4(cl_map(acc + h * pitch + d, base + c));
       }
     }
     float M = kNegBig, L = 0.f;
@@ -132,7 +134,7 @@ __device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, con
       y.x = fmaf(x[c].x, f, y.x); y.y = fmaf(x[c].y, f, y.y); y.z = fmaf(x[c].z, f, y.z); y.w = fmaf(x[c].w, f, y.w);
     }
     const float inv = L > 0.f ? 1.f / L : 0.f;
-    reinterpret_cast<float4*>(dst)[piece] = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+    store(piece, make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv));
   }
 }
 
@@ -360,7 +362,8 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   *reinterpret_cast<float4*>(&sm.acc[0][h][d4]) = o;
   if (d4 == 0) sm.ML[h] = make_float2(M, L);
   cl_sync();
-  cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, rank, kClThreads, dst);
+  cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, (int)rank, 0, kClThreads,
+                      [&](int piece, float4 y) { reinterpret_cast<float4*>(dst)[piece] = y; });
   cl_sync();  // nobody leaves while its shared memory is being read
 }
 
@@ -388,18 +391,22 @@ struct CmSmem {
       float2 ML[kHq];
     } m;
   };
+  float2 pick[kClMaxCluster];  // in the cluster's first CTA: every CTA's best output value and (as bits) its index
+  float2 pick_warp[kCmWarps];
 };
 
-template <typename T, bool kBoth>
+// kPick: the token pick of a decode step (DecodeParams::pick_tokens).  All CTAs of a row then form one cluster, also where
+// they take a KV head each.
+template <typename T, bool kBoth, bool kPick>
 __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(DecodeParams p) {
   extern __shared__ __align__(128) unsigned char cl_smem_raw[];
   CmSmem& sm = *reinterpret_cast<CmSmem*>(cl_smem_raw);
   constexpr int kRowB = kD * 2, kTokB = kHkv * kRowB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int b = blockIdx.z, kvh = kBoth ? warp & 1 : blockIdx.y, ctas = gridDim.x;
-  const uint32_t rank = ctas > 1 ? cl_rank() : 0u;
+  const int rank = blockIdx.x;  // among the CTAs that share the head's (or both heads') blocks
   constexpr int kWalkers = kBoth ? kCmWarps / 2 : kCmWarps;  // warps of the CTA that share a KV head's blocks
-  const int first = (int)rank * kWalkers + (kBoth ? warp >> 1 : warp), stride = ctas * kWalkers;  // this warp's blocks: first, first + stride, ...
+  const int first = rank * kWalkers + (kBoth ? warp >> 1 : warp), stride = ctas * kWalkers;  // this warp's blocks: first, first + stride, ...
 
   if (!p.beside || ld_acquire_gpu(p.beside) == 0) pdl_wait();
   pdl_release();
@@ -575,6 +582,14 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   constexpr int kHeads = kBoth ? kHq : kG;
   constexpr int kPieces = kHeads * kD / 4, kPer = kPieces / kCmThreads;  // float4 pieces of the output, and per thread
   float* dst = p.out + (qi * kHq + (kBoth ? 0 : kvh * kG)) * kD;
+  ArgBest best;
+  auto store = [&](int piece, float4 y) {
+    reinterpret_cast<float4*>(dst)[piece] = y;
+    if constexpr (kPick) {
+      const int i = (kBoth ? 0 : kvh * kG * kD) + piece * 4;
+      best.take(y.x, i); best.take(y.y, i + 1); best.take(y.z, i + 2); best.take(y.w, i + 3);
+    }
+  };
   float4 sum[kPer];
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
@@ -597,24 +612,41 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     }
     if (ctas == 1) {
       const float inv = L > 0.f ? 1.f / L : 0.f;
-      reinterpret_cast<float4*>(dst)[piece] = make_float4(sum[k].x * inv, sum[k].y * inv, sum[k].z * inv, sum[k].w * inv);
+      store(piece, make_float4(sum[k].x * inv, sum[k].y * inv, sum[k].z * inv, sum[k].w * inv));
     } else if ((piece & 63) == 0) {
       sm.m.ML[head] = make_float2(M, L);
     }
   }
-  if (ctas == 1) {
-    cl_end_beside(p);
-    return;
-  }
-  __syncthreads();  // acc[0] is overwritten
+  if (ctas > 1) {
+    __syncthreads();  // acc[0] is overwritten
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int piece = k * kCmThreads + threadIdx.x;
-    *reinterpret_cast<float4*>(&sm.m.acc[0][piece >> 6][(piece & 63) * 4]) = sum[k];
+    for (int k = 0; k < kPer; ++k) {
+      const int piece = k * kCmThreads + threadIdx.x;
+      *reinterpret_cast<float4*>(&sm.m.acc[0][piece >> 6][(piece & 63) * 4]) = sum[k];
+    }
+    cl_sync();
+    cl_fold_cluster<kHeads>(&sm.m.acc[0][0][0], kCmPitch, sm.m.ML, ctas, rank, kPick && !kBoth ? kvh * ctas : 0, kCmThreads, store);
   }
-  cl_sync();
-  cl_fold_cluster<kHeads>(&sm.m.acc[0][0][0], kCmPitch, sm.m.ML, ctas, rank, kCmThreads, dst);
-  cl_sync();  // nobody leaves while its shared memory is being read
+  const int members = kPick && !kBoth ? kHkv * ctas : ctas;  // CTAs of the cluster
+  if constexpr (kPick) {
+    if (members > 1 && ctas == 1) cl_sync();  // (no barrier so far: the cluster's first CTA has to have started)
+    best.reduce_warp();
+    if (lane == 0) sm.pick_warp[warp] = make_float2(best.v, __int_as_float(best.i));
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int w = 1; w < kCmWarps; ++w) best.take(sm.pick_warp[w].x, __float_as_int(sm.pick_warp[w].y));
+      if (members > 1) cl_st2(cl_map(&sm.pick[kBoth ? rank : kvh * ctas + rank], 0), best.v, best.i);
+    }
+  }
+  if (members > 1) cl_sync();  // nobody leaves while its shared memory is being read; every candidate has arrived
+  if constexpr (kPick) {
+    if (threadIdx.x == 0 && rank == 0 && (kBoth || kvh == 0)) {
+      for (int c = 1; c < members; ++c) best.take(sm.pick[c].x, __float_as_int(sm.pick[c].y));
+      p.pick_tokens[b] = best.index();
+      advance_row(p.pick_lens, p.pick_positions, b, (long long)p.table_width * p.block_size, p.status);  // (all of the row's CTAs have read it)
+    }
+  }
   cl_end_beside(p);
 }
 
@@ -668,6 +700,18 @@ bool decode_cluster_pays(int batch, int table_width) {
   return per_walker <= (f.ctas == 6 ? 32 : 24);
 }
 
+// For the token pick a row's CTAs are one cluster, over both heads: 9 - 16 CTAs per head do not fit one, and more than ten in all
+// (placed by the GPC, three or four to one) only pay while they leave places free.  Eight steps of a graph, picked here : behind: 20
+// rows of 375 - 1500 keys (16 CTAs) 122 : 134 us, 25 rows 170 : 164, 28 (14) 180 : 150, 32 (12) 168 : 153, 37 of 1450 - 2900 (10)
+// 303 : 313, 54 of 117 - 468 (6) 117 : 137, 8 of 50 - 200 79 : 95, 256 of 1024 - 4096 (4, both heads each) 1640 : 1662.
+bool decode_cluster_picks(const DecodeParams& p) {
+  const int sms = decode_wide_num_ctas();
+  if (sms <= 0 || !p.pre_append || p.kv_dtype != NVJ_BF16 || p.q_dtype != NVJ_BF16 || p.kv_indptr || p.packed_rows) return false;
+  const ClusterForm f = cluster_form(p.batch, p.table_width, sms, sms, kCmPerSm);
+  const int members = kHkv * f.ctas;
+  return f.both || members <= 10 || (members <= kClMaxCluster && 100LL * members * p.batch <= 225LL * sms);
+}
+
 int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   if (p.batch > kClMaxRows) return NVJ_ERR_UNSUPPORTED;
   const int sms = decode_wide_num_ctas();
@@ -684,18 +728,25 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   // 512 blocks 243 us with eight and 265 with four (rows of 1/4 - 1 of the table), 44 and 40 (1/32 - 1/8); 256 rows 1482 and 1447,
   // 272 and 216; 512 rows of 16 - 128 keys 252 and 127 (the generic kernel 115).
   const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 16LL * p.batch <= 4LL * sms ? 8 : 4, 8);
-  static PerDeviceFlags flags[6];
+  static PerDeviceFlags flags[8];
   const int smem = (int)sizeof(CmSmem);
-  if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16)
-    return form.both ? launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, true>, flags[0], p, form.ctas, 1, kCmThreads, smem, stream)
-                : launch_clusters(decode_cluster_mma_kernel<__nv_bfloat16, false>, flags[1], p, form.ctas, kHkv, kCmThreads, smem, stream);
+  auto both = [&](auto* kernel, PerDeviceFlags& f) { return launch_clusters(kernel, f, p, dim3(form.ctas), 1, kCmThreads, smem, stream, p); };
+  auto each = [&](auto* kernel, PerDeviceFlags& f, int heads_per_cluster) {
+    return launch_clusters(kernel, f, p, dim3(form.ctas, heads_per_cluster), kHkv, kCmThreads, smem, stream, p);
+  };
+  if (p.kv_dtype == NVJ_BF16 && p.q_dtype == NVJ_BF16) {
+    if (p.pick_tokens)
+      return form.both ? both(decode_cluster_mma_kernel<__nv_bfloat16, true, true>, flags[6])
+                       : each(decode_cluster_mma_kernel<__nv_bfloat16, false, true>, flags[7], kHkv);
+    return form.both ? both(decode_cluster_mma_kernel<__nv_bfloat16, true, false>, flags[0])
+                     : each(decode_cluster_mma_kernel<__nv_bfloat16, false, false>, flags[1], 1);
+  }
   if (p.kv_dtype == NVJ_F16 && p.q_dtype == NVJ_F16)
-    return form.both ? launch_clusters(decode_cluster_mma_kernel<__half, true>, flags[2], p, form.ctas, 1, kCmThreads, smem, stream)
-                : launch_clusters(decode_cluster_mma_kernel<__half, false>, flags[3], p, form.ctas, kHkv, kCmThreads, smem, stream);
+    return form.both ? both(decode_cluster_mma_kernel<__half, true, false>, flags[2]) : each(decode_cluster_mma_kernel<__half, false, false>, flags[3], 1);
   if (p.kv_dtype == NVJ_F32)
-    return launch_clusters(decode_cluster_kernel<float>, flags[4], p, wide, kHkv, kClThreads, cluster_smem_bytes<float>(), stream);
+    return launch_clusters(decode_cluster_kernel<float>, flags[4], p, dim3(wide), kHkv, kClThreads, cluster_smem_bytes<float>(), stream, p);
   if (p.kv_dtype == NVJ_F16)
-    return launch_clusters(decode_cluster_kernel<__half>, flags[5], p, wide, kHkv, kClThreads, cluster_smem_bytes<__half>(), stream);
+    return launch_clusters(decode_cluster_kernel<__half>, flags[5], p, dim3(wide), kHkv, kClThreads, cluster_smem_bytes<__half>(), stream, p);
   return NVJ_ERR_UNSUPPORTED;  // bf16 cache with another query dtype: the streaming kernel on the CUDA cores
 }
 

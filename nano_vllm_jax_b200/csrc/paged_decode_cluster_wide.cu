@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kCwThreads, 3) decode_cluster_wide_kernel(Deco
 template <int kTiles>
 static int launch_tiles(const DecodeParams& p, int cluster, cudaStream_t stream) {
   static PerDeviceFlags opted_in;
-  return launch_clusters(decode_cluster_wide_kernel<kTiles>, opted_in, p, cluster, 1, kCwThreads, (int)sizeof(CwSmem<kTiles>), stream);
+  return launch_clusters(decode_cluster_wide_kernel<kTiles>, opted_in, p, dim3(cluster), 1, kCwThreads, (int)sizeof(CwSmem<kTiles>), stream, p);
 }
 
 static bool cw_takes(const DecodeParams& p) {

@@ -21,11 +21,24 @@ __device__ __forceinline__ void advance_row(int32_t* seq_lens, int32_t* position
   seq_lens[b] = len + 1;
 }
 
+// A candidate of an argmax: the first maximum wins; NaNs are never taken up.
+struct ArgBest {
+  float v = -INFINITY;
+  int i = 0x7fffffff;
+  __device__ __forceinline__ void take(float ov, int oi) {
+    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
+  }
+  __device__ __forceinline__ void reduce_warp() {  // the best of the warp, in every lane
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) take(__shfl_xor_sync(kFullMask, v, o), __shfl_xor_sync(kFullMask, i, o));
+  }
+  __device__ __forceinline__ int index() const { return i == 0x7fffffff ? 0 : i; }  // a row of NaNs: 0
+};
+
 // Argmax of `row_len` floats by one CTA of kArgmaxThreads threads: the first maximum wins, NaNs are never
 // selected unless the whole row is NaN (then index 0).  The result is valid in thread 0.
 __device__ __forceinline__ int row_argmax_cta(const float* row, int row_len) {
-  float best = -INFINITY;
-  int best_i = 0x7fffffff;
+  ArgBest best;
   if ((row_len & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
     // 16-byte loads, four in flight per thread: the row is read in one or two round trips instead of row_len / 128
     const float4* row4 = reinterpret_cast<const float4*>(row);
@@ -42,31 +55,21 @@ __device__ __forceinline__ int row_argmax_cta(const float* row, int row_len) {
         const int i0 = (base + u * blockDim.x) * 4;
         const float e[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (e[c] > best || (e[c] == best && i0 + c < best_i)) { best = e[c]; best_i = i0 + c; }
+        for (int c = 0; c < 4; ++c) best.take(e[c], i0 + c);
       }
     }
   } else {
-    for (int i = threadIdx.x; i < row_len; i += blockDim.x) {
-      const float v = row[i];
-      if (v > best || (v == best && i < best_i)) { best = v; best_i = i; }
-    }
+    for (int i = threadIdx.x; i < row_len; i += blockDim.x) best.take(row[i], i);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(kFullMask, best, o);
-    const int oi = __shfl_xor_sync(kFullMask, best_i, o);
-    if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
-  }
+  best.reduce_warp();
   __shared__ float sv[kArgmaxThreads / 32];
   __shared__ int si[kArgmaxThreads / 32];
-  if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = best_i; }
+  if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best.v; si[threadIdx.x >> 5] = best.i; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < kArgmaxThreads / 32; ++w)
-      if (sv[w] > best || (sv[w] == best && si[w] < best_i)) { best = sv[w]; best_i = si[w]; }
+    for (int w = 1; w < kArgmaxThreads / 32; ++w) best.take(sv[w], si[w]);
   }
-  return best_i == 0x7fffffff ? 0 : best_i;
+  return best.index();
 }
 
 }  // namespace nvj

@@ -12,8 +12,8 @@ costs no host-to-device traffic for metadata.  Here the same arrays are torch CU
                            (the only per-step host work, and only when a row crosses a block
                            boundary), `load()` (re)installs a batch.
   DecodeStepGraph          captures  fused append + paged decode -> token pick + advance
-                           once and replays it: one graph launch per step, two kernels back to
-                           back, and nothing is allocated or copied per step.  The decode pass
+                           once and replays it: one graph launch per step of one kernel (two for
+                           long rows and with a token gather), and nothing is allocated or copied per step.  The decode pass
                            runs in its pre-append form (a row's token goes to position
                            seq_lens[b], seq_lens[b] + 1 keys are attended) and the token pick
                            advances the lengths for the next step in the same launch.  On
@@ -157,15 +157,16 @@ class DecodeStepGraph:
 
     def _step(self):
         m = self.meta
+        if self.token_gather is None:  # one launch where the batch runs on clusters, else two
+            out = _k.paged_decode_step(self.query, self.new_k, self.new_v, self.k_cache, self.v_cache, m.block_tables, m.seq_lens,
+                                       m.positions, self.layer_id, m.block_size, self.scale, self.groups, self._tokens)
+            return out, self._tokens
         out, _, _ = _k.paged_decode_attention_with_kv_append(self.query, self.new_k, self.new_v, self.k_cache, self.v_cache,
                                                              m.block_tables, m.seq_lens, None, self.layer_id, m.block_size,
                                                              self.scale, self.groups)
-        advance = (m.seq_lens, m.positions, m.table_width, m.block_size)
-        if self.token_gather is None:
-            return out, _k.row_argmax(out.view(m.rows, -1), self._tokens, advance=advance)
         # one launch: collect the step before, pick this step's tokens, publish them, advance the lengths
         return out, self.token_gather.publish_argmax(out.view(m.rows, -1), self._tokens, collect_out=self.gathered,
-                                                     advance=advance)
+                                                     advance=(m.seq_lens, m.positions, m.table_width, m.block_size))
 
     def flush(self) -> Optional[torch.Tensor]:
         """Collect the tokens of the last replayed step into `gathered` (several GPUs only)."""

@@ -563,6 +563,50 @@ def paged_decode_attention_with_kv_append(query, new_k, new_v, k_cache, v_cache,
     return out.reshape(batch, 1, hq * d), k_cache, v_cache
 
 
+def paged_decode_step(query, new_k, new_v, k_cache, v_cache, block_table, seq_lens, positions, layer_id, block_size, scale,
+                      num_key_value_groups, tokens):
+    """A decode step of one layer over device-resident metadata: `paged_decode_attention_with_kv_append(positions=None)`, then
+    `row_argmax` of its output into `tokens` (int32 `[B]`) that advances `seq_lens` and `positions` (None: not kept); one launch
+    where the batch runs on clusters.  Returns out `[B, 1, Hq*D]` fp32."""
+    if query.ndim != 4 or query.shape[1] != 1 or new_k.shape[1] != 1 or new_v.shape[1] != 1:
+        raise ValueError("a decode step takes one token per row")
+    if k_cache.ndim != 5 or v_cache.ndim != 5:
+        raise ValueError("a decode step requires cache shape [num_layers, num_pages, page_size, num_kv_heads, head_dim]")
+    if not 0 <= layer_id < k_cache.shape[0]:
+        raise ValueError(f"layer_idx {layer_id} is out of bounds for {k_cache.shape[0]} layers")
+    if k_cache.shape[2] != block_size:
+        raise ValueError("block_size must match the cache page size")
+    k_layer, v_layer, dt = k_cache[layer_id], v_cache[layer_id], k_cache.dtype
+    _check_nhd_cache(k_layer, v_layer)
+    batch, _, hq, d = query.shape
+    pages, _, hkv, dk = k_layer.shape
+    if d != dk or hq != hkv * num_key_value_groups:
+        raise ValueError("num_key_value_groups does not match the head counts")
+    if new_k.shape != (batch, 1, hkv, d) or new_v.shape != (batch, 1, hkv, d):
+        raise ValueError("new_k and new_v must have shape [batch, 1, num_kv_heads, head_dim]")
+    q, nk, nv = _cuda("query", query), _cuda("new_k", new_k).to(dt).contiguous(), _cuda("new_v", new_v).to(dt).contiguous()
+    q = (q if q.dtype in (torch.float32, dt) else q.to(dt)).contiguous()
+    block_table = _i32("block_table", block_table)
+    if block_table.ndim != 2 or block_table.shape[0] != batch:
+        raise ValueError("block_table must have shape [batch, max_blocks_per_seq]")
+    if _cuda("tokens", tokens).dtype != torch.int32 or tokens.shape != (batch,) or not tokens.is_contiguous():
+        raise ValueError("tokens must be a contiguous int32 [batch] tensor")
+    seq_lens, positions, width, _ = _advance_args((seq_lens, positions, block_table.shape[1], block_size), batch)
+    out = torch.empty((batch, 1, hq * d), dtype=torch.float32, device=q.device)
+    if batch == 0:
+        return out
+    if _poison():
+        out.fill_(float("nan"))
+    ws = _workspace(q.device, batch)
+    check(_lib.load().nvj_paged_decode_append_pick(
+        _ptr(q), _dt(q), _ptr(nk), _ptr(nv), _ptr(k_layer), _ptr(v_layer), _dt(k_layer), pages, int(block_size), hkv, d, hq,
+        _ptr(block_table), width, _ptr(seq_lens), _ptr(positions), batch, float(scale), _ptr(out), _ptr(tokens), _ptr(ws.buf),
+        ws.nbytes, _stream(q.device)), "nvj_paged_decode_append_pick")
+    if _strict():
+        _check_word(ws.status_tensor(), "nvj_paged_decode_append_pick", ws)
+    return out
+
+
 # --------------------------------------------------------------------------- prefill
 
 def packed_paged_prefill_attention(query, k_cache_layer, v_cache_layer, block_table, kv_lens, positions,

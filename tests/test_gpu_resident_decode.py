@@ -141,3 +141,43 @@ def test_token_pick_with_advance_is_pick_plus_advance():
     with pytest.raises(K.DeviceStatusError):  # row 4 is full now
         K.row_argmax(x, advance=(meta.seq_lens, None, 2, 16))
     assert meta.seq_lens.tolist() == [0, 3, 17, 18, 32, 0]
+
+
+# rows x table width in blocks pick the launch: 1 CTA per row and head (a cluster of both heads), 8, 16 (too many for one cluster: a
+# second launch picks), 5, then 1, 2 and 4 CTAs per row for both heads, and the streaming kernel
+@pytest.mark.parametrize("rows,width", [(3, 4), (3, 32), (3, 80), (40, 24), (150, 6), (200, 30), (70, 100), (20, 420)])
+def test_a_step_in_one_call_equals_attention_then_token_pick(rows, width):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    c = decode_case(rows + width, 4000, rows, 1, 1, width=width)
+    rng = np.random.default_rng(rows * width)
+    span = width * BS
+    lens = np.array([[0, 1, BS, span - 1, min(span - 1, 37)][b % 5] if b != 1 else 1 + b for b in range(rows)], np.int32)
+    tables = to_torch(rng.integers(0, 3000, size=(rows, width)).astype(np.int32))
+    last = 3000 + np.arange(rows)  # the block that takes a row's token is the row's own
+    for b, n in enumerate(lens):
+        tables[b, n // BS] = int(last[b])
+    q, nk, nv = (to_torch(c[n]) for n in ("q", "new_k", "new_v"))
+    k_a, v_a = to_torch(c["k_cache"]), to_torch(c["v_cache"])
+    k_b, v_b = k_a.clone(), v_a.clone()
+    lens_a, pos_a = to_torch(lens), torch.zeros((rows, 1), dtype=torch.int32, device="cuda")
+    lens_b, pos_b = lens_a.clone(), pos_a.clone()
+    ref, _, _ = K.paged_decode_attention_with_kv_append(q, nk, nv, k_a, v_a, tables, lens_a, None, 0, BS, SCALE, 4)
+    want = K.row_argmax(ref.view(rows, -1), advance=(lens_a, pos_a, width, BS))
+    tokens = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    got = K.paged_decode_step(q, nk, nv, k_b, v_b, tables, lens_b, pos_b, 0, BS, SCALE, 4, tokens)
+    # the same kernel where a row's clusters have the same size: 16 CTAs per head become 8 only without the token pick's limit
+    assert torch.equal(got, ref)
+    assert torch.equal(tokens, want) and torch.equal(lens_a, lens_b) and torch.equal(pos_a, pos_b)
+    assert torch.equal(k_a.view(torch.uint8), k_b.view(torch.uint8)) and torch.equal(v_a.view(torch.uint8), v_b.view(torch.uint8))
+
+
+def test_a_step_leaves_a_row_without_room_alone_and_flags_it():
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    c = decode_case(3, 64, 2, 1, 1, width=2)
+    q, nk, nv = (to_torch(c[n]) for n in ("q", "new_k", "new_v"))
+    k, v = to_torch(c["k_cache"]), to_torch(c["v_cache"])
+    tables = torch.tensor([[1, 2], [3, 4]], dtype=torch.int32, device="cuda")
+    lens, tokens = torch.tensor([2 * BS, 5], dtype=torch.int32, device="cuda"), torch.zeros(2, dtype=torch.int32, device="cuda")
+    with pytest.raises(K.DeviceStatusError):
+        K.paged_decode_step(q, nk, nv, k, v, tables, lens, None, 0, BS, SCALE, 4, tokens)
+    assert lens.tolist() == [2 * BS, 6]
