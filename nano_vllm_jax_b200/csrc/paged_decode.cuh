@@ -157,7 +157,7 @@ inline size_t ws_acc_bytes(int num_ctas) { return ws_round(sizeof(float) * ws_sl
 //   [0, 64)              status word; at kWsBesideWord the word of a launch beside another one (DecodeParams::beside)
 //   [64, 320)            group arrival counters
 //   [320, 320 + 4 rows)  row arrival counters
-//   ... unused, or the partial outputs of the prefill kernel's key-range splits, which end where the next part begins ...
+//   ... unused ...
 //   the last ml_bytes + acc_bytes of the buffer: partial (max, sum) pairs and accumulators
 // The counters and that word are zero before the first use and every launch leaves them zero again; the partials are always
 // written before they are read.  Because the partials are anchored at the END of the buffer, a call with few rows
@@ -176,9 +176,6 @@ inline int carve_decode_workspace(DecodeParams& p, void* workspace, size_t bytes
   p.part_ml = reinterpret_cast<float*>(w + end - acc_bytes - ml_bytes);
   return NVJ_OK;
 }
-
-// Bytes that the prefill kernel's key-range splits may need for their partial outputs on the current device.
-size_t prefill_split_bytes();
 
 int decode_num_ctas();  // 2 per SM of the current device
 int launch_decode_generic(const DecodeParams& p, cudaStream_t stream);

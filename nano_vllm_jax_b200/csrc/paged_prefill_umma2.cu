@@ -19,15 +19,16 @@
 // A cluster barrier after set-up and one before the tensor memory is freed fence the pair.
 // Every mbarrier wait is bounded; a timeout flags NVJ_DEV_TIMEOUT and both CTAs still reach
 // the final cluster barrier and free their tensor memory.
-// Short batches (a 512-token chunk is 16 CTA pairs on 74 pair slots) split every tile's key range over up to
-// kU2MaxSplits pairs (blockIdx.z): each split writes its un-normalised rows and their (max, sum) to a workspace and
-// is done; prefill_umma2_merge_kernel, launched behind this kernel, folds the splits of every tile into the output
-// with the whole GPU (a first build let the pair that arrived last fold its tile alone: ~10 us of round trips to
-// the L2 on two SMs, so that only key ranges of 16 tiles or more were worth splitting).
+// Short batches (a 512-token chunk is 18 CTA pairs on 74 pair slots) split every tile's key range over up to kU2MaxSplits pairs
+// (blockIdx.z), which form one cluster: each leaves its un-normalised rows and their (max, sum) in its shared memory, and
+// behind a cluster barrier every CTA folds its share of the rows out of all of them and writes it.  (The splits used to go through
+// a workspace and a second launch that folded them: 128 KiB written and read again per CTA, and 4 us; the chunk behind 1024
+// cached tokens 23.8 -> 21.9 us, 64 tokens behind 400 18.5 -> 16.3.)
 // Semantics: nanovllm_jax/kv_cache.py:831-849, nanovllm_jax/kernels/full_attention_triton.py:51-145.
 
 #include <cstddef>
 
+#include "cluster.cuh"
 #include "paged_decode.cuh"
 #include "umma.cuh"
 
@@ -46,13 +47,12 @@ constexpr uint32_t kU2LeaderMask = 0xFEFFFFFFu;         // clears the CTA-rank b
 constexpr float kU2Log2e = 1.4426950408889634f;
 constexpr float kU2RescaleGap = 8.f;
 constexpr int kU2MaxSplits = 4;
-// What a split costs: its rows go out to the workspace (~1 us) and the merge launch behind the kernel (~5 us for the
-// batch, whatever the number of splits).  A key tile costs a pair ~1 us.  Key ranges of kU2SplitFrom tiles or more
-// are split into pieces of at least kU2MinSplitTiles tiles.
-constexpr int kU2SplitFrom = 8;
-constexpr int kU2MinSplitTiles = 3;
-constexpr int kU2MergeThreads = 256;
-constexpr int kU2MergeParts = 8;  // CTAs of the merge launch per CTA tile: 4 of its 32 tokens each
+// A key tile costs a pair ~1 us, a split the barrier and the fold, ~2 us.  Key ranges of kU2SplitFrom tiles or more are split into
+// pieces of at least kU2MinSplitTiles tiles: from 4 on 100 tokens behind 220 take 18.7 us instead of 16.9, from 8 on 64 behind 400
+// 19.0 instead of 16.3 and 400 behind none 18.4 instead of 17.4.  Four pieces only while the pairs' clusters of eight CTAs all fit
+// (15 here): a tile of 16 - 18 pairs and heads gets three (512 tokens behind 3584: 39.5 us, 36.6 with four and a second launch).
+constexpr int kU2SplitFrom = 6;
+constexpr int kU2MinSplitTiles = 2;
 
 // Development aid, compiled in only with -DNVJ_PHASE_TIMING: the first softmax thread of every CTA stamps the global
 // timer at the kernel's phase boundaries (slot 7: the number of key tiles), nvj_debug_prefill_phase_ns copies them out.
@@ -80,12 +80,8 @@ struct Umma2Params {
   int zero_fill;  // 1: the kernel itself zeroes what no tile writes (padding tokens, rows of several tokens without keys)
   int split_p;  // 1: P enters P V as two bf16 terms (hi + lo), 0: as one (the weights are then bf16-rounded)
   float scale;
-  // key-range splits (gridDim.z > 1): un-normalised rows [split][token][head][kD], their (max, sum)
-  // [split][token][head][2]; pair slots of the device
-  float* part_o;
-  float* part_ml;
-  int4* tile_info;  // per (CTA of the x grid, KV head): {first token, tokens, splits, 0}, written by split 0 for the merge launch
-  int pair_slots;
+  // key-range splits (gridDim.z > 1)
+  int pair_slots;  // CTA pairs that run at once
 };
 
 struct Umma2Smem {
@@ -98,21 +94,12 @@ struct Umma2Smem {
   // this CTA's query rows on their way into tensor memory: [token][head of the group][32 pieces of 16 B], the pieces
   // of token t stored at (piece ^ (t & 7)) so that both the row-wise fill and the token-wise read are conflict-free
   alignas(16) char qstage[kU2Tokens * kG * kD * 2];
-  float own_ml[2][kU2Rows];  // this split's (max, sum) per row, for the fold
+  float2 own_ml[kU2Rows];  // this split's (max, sum) per row, for the fold
   uint32_t tmem_base;
   int row, tok0, ntok, pair_last_tok, idle_index, abort_flag, total_pairs;
 };
 
 // ---- cta_group::2 wrappers ---------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tmem2_alloc(uint32_t smem_dst, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -129,10 +116,11 @@ __device__ __forceinline__ void umma2_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, 
       ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
-// arrives, once the MMAs issued so far have retired, on the barrier at this offset in both CTAs of the pair
+// arrives, once the MMAs issued so far have retired, on the barrier at this offset in both CTAs of the pair (ranks 2 z and 2 z + 1
+// of the cluster)
 __device__ __forceinline__ void umma2_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"((uint16_t)3) : "memory");
+               ::"r"(bar), "h"((uint16_t)(3u << (2 * blockIdx.z))) : "memory");
 }
 // One box into this CTA's shared memory; the bytes are counted on CTA 0's barrier at `bar`'s offset.
 __device__ __forceinline__ void tma2_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
@@ -343,6 +331,9 @@ __device__ __forceinline__ void u2_request_q(const Umma2Params& p, int tok0, int
   }
 }
 
+// Where the 16-byte piece `c` of row `r` of the output tile lies in the freed stages, in floats.
+__device__ __forceinline__ int u2_piece(int r, int c) { return r * kD + (((c & ~7) | ((c ^ r) & 7)) << 2); }
+
 // ---- warps 2-9 of both CTAs: Q staging, softmax, epilogue for this CTA's 128 rows -------------
 __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Params& p, uint32_t tmem, int tok0, int ntok,
                                                  int kvh, int kv_len, int tile0, int n_tiles, int splits, int warp, int lane,
@@ -420,7 +411,7 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
   }
   tc_fence_after_sync();
   const float inv = splits > 1 ? 1.f : (l_row > 0.f ? 1.f / l_row : 0.f);  // a split leaves its rows un-normalised
-  if (splits > 1 && half == 0) { sm.own_ml[0][r] = m_row; sm.own_ml[1][r] = l_row; }
+  if (splits > 1 && half == 0) sm.own_ml[r] = make_float2(m_row, l_row);
   // The K and V stages (128 KiB, contiguous) are free now: every copy has landed and every product has retired.  The
   // normalised rows are laid down there, [row][256 floats] with the 16-byte pieces of row r stored at (piece ^ (r & 7))
   // inside their group of eight, and leave as whole 512-byte runs per warp instruction.  (Stored straight from the
@@ -442,24 +433,73 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
   named_bar_sync(1, kU2SoftmaxThreads);
   if (*reinterpret_cast<volatile int*>(&sm.abort_flag)) return;  // somebody gave up: the same answer in every thread
   const int sw = (warp - 2) & 7;
-  const long long split_rows = (long long)p.token_bucket * kHq;  // rows of one split's partial area
-  {
-    float* base = splits > 1 ? p.part_o + (long long)blockIdx.z * split_rows * kD : p.out;
+  if (splits > 1) return;  // u2_fold_splits takes the rows from here
 #pragma unroll 4
-    for (int a = 0; a < kU2Rows / 8; ++a) {
-      const int rr = sw * (kU2Rows / 8) + a, tk = rr & 31, hd = rr >> 5;
-      if (tk >= ntok) continue;
-      const long long g = (long long)(tok0 + tk) * kHq + kvh * kG + hd;
+  for (int a = 0; a < kU2Rows / 8; ++a) {
+    const int rr = sw * (kU2Rows / 8) + a, tk = rr & 31, hd = rr >> 5;
+    if (tk >= ntok) continue;
+    const long long g = (long long)(tok0 + tk) * kHq + kvh * kG + hd;
 #pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {
-        const int c = h2 * 32 + lane;
-        reinterpret_cast<float4*>(base + g * kD)[c] = *reinterpret_cast<const float4*>(stage + rr * kD + (((c & ~7) | ((c ^ rr) & 7)) << 2));
-      }
-      if (splits > 1 && lane == 0)
-        *reinterpret_cast<float2*>(p.part_ml + ((long long)blockIdx.z * split_rows + g) * 2) = make_float2(sm.own_ml[0][rr], sm.own_ml[1][rr]);
+    for (int h2 = 0; h2 < 2; ++h2) {
+      const int c = h2 * 32 + lane;
+      reinterpret_cast<float4*>(p.out + g * kD)[c] = *reinterpret_cast<const float4*>(stage + u2_piece(rr, c));
     }
   }
-  NVJ_U2_PHASE(5);  // a split is done here: the merge launch folds the splits
+  NVJ_U2_PHASE(5);
+}
+
+// The splits' rows, staged by all of them (the same 128 rows in the CTAs of this rank of every pair), into the output: split z of n
+// takes rows [128 z / n, 128 (z + 1) / n), a warp two rows at a time, every split's pieces requested before anything is used.
+__device__ __forceinline__ void u2_fold_splits(const Umma2Smem& sm, const Umma2Params& p, int tok0, int ntok, int kvh, int rank, int splits,
+                                               int warp, int lane) {
+  const float* stage = reinterpret_cast<const float*>(&sm.k[0][0][0]);
+  constexpr int kWarps = kU2Threads / 32;
+  const int row0 = (int)blockIdx.z * kU2Rows / splits, row1 = ((int)blockIdx.z + 1) * kU2Rows / splits;
+  for (int r0 = row0 + warp; r0 < row1; r0 += 2 * kWarps) {
+    float2 e[2];
+    float4 x[2][kU2MaxSplits][2];
+    bool real[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int rr = r0 + k * kWarps;
+      real[k] = rr < row1 && (rr & 31) < ntok;
+      e[k] = make_float2(-INFINITY, 0.f);  // lane s < splits: that split's (max, sum) of the row
+      if (real[k] && lane < splits) e[k] = cl_ld2(cl_map(&sm.own_ml[rr], 2 * lane + rank));
+#pragma unroll
+      for (int s = 0; s < kU2MaxSplits; ++s)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          x[k][s][h] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (real[k] && s < splits) x[k][s][h] = cl_ld4(cl_map(stage + u2_piece(rr, h * 32 + lane), 2 * s + rank));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (!real[k]) continue;
+      const int rr = r0 + k * kWarps;
+      float big = e[k].x;
+#pragma unroll
+      for (int o = 1; o < kU2MaxSplits; o <<= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+      float w = e[k].x == -INFINITY ? 0.f : ex2_approx(e[k].x - big);
+      float total = w * e[k].y;
+#pragma unroll
+      for (int o = 1; o < kU2MaxSplits; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+      w = total > 0.f ? w / total : 0.f;  // lanes 0 .. kU2MaxSplits - 1 hold their split's normalised weight
+      float4* dst = reinterpret_cast<float4*>(p.out + ((long long)(tok0 + (rr & 31)) * kHq + kvh * kG + (rr >> 5)) * kD);
+      float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll
+      for (int s = 0; s < kU2MaxSplits; ++s) {
+        const float ws = __shfl_sync(0xffffffffu, w, s);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          acc[h].x = fmaf(x[k][s][h].x, ws, acc[h].x); acc[h].y = fmaf(x[k][s][h].y, ws, acc[h].y);
+          acc[h].z = fmaf(x[k][s][h].z, ws, acc[h].z); acc[h].w = fmaf(x[k][s][h].w, ws, acc[h].w);
+        }
+      }
+      dst[lane] = acc[0];
+      dst[32 + lane] = acc[1];
+    }
+  }
 }
 
 // Which (table row, 32-token tile) the CTA with cluster index `cluster` of `clusters` and rank `rank` serves: the
@@ -536,14 +576,14 @@ __device__ __forceinline__ int u2_split_count(const Umma2Params& p, int n_tiles,
   return splits > 1 ? splits : 1;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kU2Threads, 1)
+__global__ void __launch_bounds__(kU2Threads, 1)
 prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                      const Umma2Params p) {
   extern __shared__ unsigned char u2_smem_raw[];
   Umma2Smem& sm = *reinterpret_cast<Umma2Smem*>((reinterpret_cast<uintptr_t>(u2_smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.y;
-  const int rank = (int)cluster_ctarank();  // == blockIdx.x & 1
+  const int rank = blockIdx.x & 1;  // in the pair; 2 blockIdx.z + rank in the cluster
   NVJ_U2_PHASE(0);
   NVJ_U2_NOTE(7, 0ull);
   // The pair's barriers are set up before anything is read: this runs while the kernel in front (the append of the same
@@ -563,11 +603,10 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     mbar_init(smem_u32(&sm.x_full), kU2SoftmaxThreads);
     mbar_fence_init();
   }
-  cluster_sync_all();  // the peer's barriers exist before anything is sent to them (this barrier covers the CTA's own threads)
+  cl_sync();  // the peer's barriers exist before anything is sent to them (this barrier covers the CTA's own threads)
   pdl_wait();
-  // Tensor memory between the wait and the release (umma.cuh).  Whatever follows may take its places behind it: the merge
-  // launch of a batch with splits (its CTAs wait for this grid to finish), the decode pass of a mixed batch (it runs beside, on
-  // the SMs this grid leaves).
+  // Tensor memory between the wait and the release (umma.cuh).  Whatever follows may take its places behind it, the decode pass of
+  // a mixed batch among it (it runs beside, on the SMs this grid leaves).
   if (warp == 1) {
     tmem2_alloc(smem_u32(&sm.tmem_base), kU2TmemCols);
     if (lane == 0) {
@@ -576,7 +615,7 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     }
   }
   auto leave = [&] {  // the whole cluster leaves without having touched its tensor memory
-    cluster_sync_all();
+    cl_sync();
     if (warp == 1) tmem2_dealloc(sm.tmem_base, kU2TmemCols);
   };
   if (blockIdx.z > 0) {  // the extra splits leave at once when no row's key range is long enough to be split
@@ -598,9 +637,7 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   tc_fence_after_sync();
   const int row = sm.row, tok0 = sm.tok0, ntok = sm.ntok;
   if (p.counted && blockIdx.x == 0 && row >= 0 && threadIdx.x == 0) atomicOr(p.status, NVJ_DEV_BAD_LENGTH);
-  int4* info = gridDim.z > 1 && blockIdx.z == 0 && threadIdx.x == 0 ? p.tile_info + blockIdx.x * kHkv + kvh : nullptr;
   if (row < 0) {
-    if (info) *info = make_int4(0, 0, 0, 0);
     if (p.zero_fill && sm.idle_index == 0 && blockIdx.z == 0) {
       // the first idle cluster (there is always one) zeroes the padding tokens, a quarter per CTA of the cluster pair x KV head
       int real = p.query_start_loc[p.rows];
@@ -614,10 +651,16 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     return leave();
   }
 
+  // the query rows, and the block ids of the producer's first eight tiles where those do not depend on the number of splits, are
+  // asked for together with what bounds the key range
+  uint4 qv[4][4];
+  if (warp >= 2 && p.q_dtype == NVJ_BF16) u2_request_q(p, tok0, ntok, kvh, warp, lane, qv);
+  int first_ids = -1;
+  if (warp == 0 && gridDim.z == 1 && lane < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + lane];
+
   int kv_len;
   const int n_tiles = u2_key_tiles(p, row, tok0, rank, sm.pair_last_tok, lane, kv_len, threadIdx.x == 0 && rank == 0);
   if (n_tiles == 0) {  // same decision in both CTAs; a row without keys produces zeros
-    if (info) *info = make_int4(tok0, ntok, 0, 0);
     if (p.zero_fill && blockIdx.z == 0) {
       for (int i = threadIdx.x; i < ntok * kG * (kD / 4); i += kU2Threads) {
         const int t = i / (kG * (kD / 4)), rest = i - t * (kG * (kD / 4));
@@ -628,23 +671,21 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   }
 
   // Key-range splits of this pair: as many as leave every split kU2MinSplitTiles tiles and as the batch's pairs
-  // leave pair slots for; the splits beyond that leave at once (both CTAs decide alike).
+  // leave pair slots for; the splits beyond that have nothing to do (all CTAs of the cluster decide alike).
   int splits = 1, tile0 = 0, my_tiles = n_tiles;
   if (gridDim.z > 1) {
     splits = u2_split_count(p, n_tiles, sm.total_pairs, (int)gridDim.z);
-    if (info) *info = make_int4(tok0, ntok, splits, 0);
-    if ((int)blockIdx.z >= splits) return leave();
+    if ((int)blockIdx.z >= splits) {
+      if (splits > 1) cl_sync();  // the others' barrier in front of their fold
+      return leave();
+    }
     tile0 = (int)blockIdx.z * n_tiles / splits;
     my_tiles = ((int)blockIdx.z + 1) * n_tiles / splits - tile0;
   }
 
-  // the query rows, and the block ids of the producer's first eight tiles
-  uint4 qv[4][4];
-  if (warp >= 2 && p.q_dtype == NVJ_BF16) u2_request_q(p, tok0, ntok, kvh, warp, lane, qv);
-  int first_ids = -1;
-  if (warp == 0) {
+  if (warp == 0 && gridDim.z > 1) {
     const int bi = tile0 * 4 + lane;
-    if (bi < (kv_len + kBlk - 1) / kBlk && bi < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + bi];
+    if (bi < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + bi];
   }
 
   const uint32_t tmem = sm.tmem_base;
@@ -657,76 +698,18 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
 
   tc_fence_before_sync();
   __syncthreads();
+  if (splits > 1) {
+    cl_sync();  // every split's rows are staged
+    u2_fold_splits(sm, p, tok0, ntok, kvh, rank, splits, warp, lane);
+    NVJ_U2_PHASE(5);
+  }
   if (sm.abort_flag) {  // give copies and MMAs in flight time to land before memory is released
     const unsigned long long t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
-  cluster_sync_all();  // CTA 0's MMAs read this CTA's shared and tensor memory until its last commit
+  cl_sync();  // CTA 0's MMAs read this CTA's shared and tensor memory until its last commit; the other splits its rows
   NVJ_U2_PHASE(6);
   if (warp == 1) tmem2_dealloc(tmem, kU2TmemCols);
-}
-
-// Behind prefill_umma2_kernel in stream order (no counters, no fences): folds the key-range splits of every tile into the
-// output.  Grid = the tile kernel's (x, y) with kU2MergeParts CTAs per CTA tile (4 of its 32 tokens each).  Split 0 of
-// every tile left {first token, tokens, splits} in the workspace, so a CTA is two trips to memory: that record, then
-// every split's (max, sum) and both 16-byte pieces per lane of its rows, all requested before anything is used.  (A
-// build that found its tile and its splits again from the batch's metadata took 8.8 us: five trips.)
-// Warp w folds token 4 part + w / 2, heads 2 (w & 1) and 2 (w & 1) + 1 of the group.
-static_assert(kU2MaxSplits == 4 && kU2Tokens % kU2MergeParts == 0 && kU2MergeThreads == 64 * (kU2Tokens / kU2MergeParts),
-              "the merge launch maps a warp to (token, two heads) and reduces over four lanes");
-__global__ void __launch_bounds__(kU2MergeThreads)
-prefill_umma2_merge_kernel(const Umma2Params p) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.y, part = blockIdx.z;
-  // launched with programmatic stream serialization: the CTAs may be resident before the tile kernel has finished, and
-  // wait here until all of it has completed and its writes are visible
-  pdl_wait();
-  pdl_release();
-  const int4 info = __ldcg(p.tile_info + blockIdx.x * kHkv + kvh);
-  const int tok0 = info.x, ntok = info.y, splits = info.z;
-  if (splits <= 1) return;
-  const int tk = part * (kU2Tokens / kU2MergeParts) + (warp >> 1);
-  if (tk >= ntok) return;
-  const long long split_rows = (long long)p.token_bucket * kHq;
-  float2 e[2];
-  float4 x[2][kU2MaxSplits][2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const long long g = (long long)(tok0 + tk) * kHq + kvh * kG + (warp & 1) * 2 + h;
-    e[h] = make_float2(-INFINITY, 0.f);  // lane s2 < splits: that split's (max, sum) of the row
-    if (lane < splits) e[h] = __ldcg(reinterpret_cast<const float2*>(p.part_ml + ((long long)lane * split_rows + g) * 2));
-#pragma unroll
-    for (int s2 = 0; s2 < kU2MaxSplits; ++s2) {
-      const float4* src = reinterpret_cast<const float4*>(p.part_o + ((long long)s2 * split_rows + g) * kD);
-      x[h][s2][0] = s2 < splits ? __ldcg(src + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-      x[h][s2][1] = s2 < splits ? __ldcg(src + 32 + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const long long g = (long long)(tok0 + tk) * kHq + kvh * kG + (warp & 1) * 2 + h;
-    float big = e[h].x;
-#pragma unroll
-    for (int o = 1; o < kU2MaxSplits; o <<= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
-    float w = e[h].x == -INFINITY ? 0.f : ex2_approx(e[h].x - big);
-    float total = w * e[h].y;
-#pragma unroll
-    for (int o = 1; o < kU2MaxSplits; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    w = total > 0.f ? w / total : 0.f;  // lanes 0 .. kU2MaxSplits - 1 hold their split's normalised weight
-    float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-#pragma unroll
-    for (int s2 = 0; s2 < kU2MaxSplits; ++s2) {
-      const float ws = __shfl_sync(0xffffffffu, w, s2);
-#pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {
-        acc[h2].x = fmaf(x[h][s2][h2].x, ws, acc[h2].x); acc[h2].y = fmaf(x[h][s2][h2].y, ws, acc[h2].y);
-        acc[h2].z = fmaf(x[h][s2][h2].z, ws, acc[h2].z); acc[h2].w = fmaf(x[h][s2][h2].w, ws, acc[h2].w);
-      }
-    }
-    float4* dst = reinterpret_cast<float4*>(p.out + g * kD);
-    dst[lane] = acc[0];
-    dst[32 + lane] = acc[1];
-  }
 }
 
 typedef CUresult (*U2EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -759,14 +742,6 @@ static int u2_pair_slots() {  // CTA pairs that run at once: half the SMs of the
   return n;
 }
 
-// Room for the un-normalised rows and (max, sum) pairs of the splits of the largest batch that is split at all:
-// splits x tokens never exceeds the pair slots x 64 tokens (plus one pair per split of rounding).
-size_t prefill_split_bytes() {
-  const int slots = u2_pair_slots();
-  const size_t tokens = (size_t)(slots > 0 ? slots : 74) * 2 * kU2Tokens / kHkv + (size_t)kU2MaxSplits * 2 * kU2Tokens;
-  return ws_round(sizeof(float) * tokens * kHq * (kD + 2)) + ws_round(sizeof(int4) * 2 * (tokens / (2 * kU2Tokens) + 4096) * kHkv);
-}
-
 static bool u2_make_map(CUtensorMap* map, const void* base, uint64_t outer) {
   const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)kHkv, outer};
   const cuuint64_t strides[2] = {(cuuint64_t)kRowBytes, (cuuint64_t)kRowBytes * kHkv};
@@ -777,6 +752,52 @@ static bool u2_make_map(CUtensorMap* map, const void* base, uint64_t outer) {
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+constexpr int kU2SmemBytes = (int)sizeof(Umma2Smem) + 1024;
+static_assert(kU2SmemBytes <= 232448, "tiles exceed the shared memory of one CTA");
+
+// The launch of a grid of (2 x pairs, KV heads, splits) CTAs in clusters of a pair's splits, with the attributes in `attr`.
+static cudaLaunchConfig_t u2_config(dim3 grid, cudaStream_t stream, cudaLaunchAttribute (&attr)[2]) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kU2Threads, 1, 1);
+  cfg.dynamicSmemBytes = kU2SmemBytes;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = grid.z;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cfg;
+}
+static cudaError_t u2_launch(dim3 grid, cudaStream_t stream, const CUtensorMap& k_map, const CUtensorMap& v_map, const Umma2Params& p) {
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = u2_config(grid, stream, attr);
+  return cudaLaunchKernelEx(&cfg, prefill_umma2_kernel, k_map, v_map, p);
+}
+// Clusters of `splits` pairs that the current device holds at once (asked for once per device; 0 when it does not say).
+static int u2_clusters_at_once(int splits) {
+  static PerDeviceFlags known[kU2MaxSplits + 1];  // the number + 1
+  const int dev = current_device();
+  if (dev < 0) return 0;
+  int n = known[splits].v[dev].load(std::memory_order_acquire);
+  if (n == 0) {
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = u2_config(dim3(2 * 74, kHkv, splits), nullptr, attr);
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, prefill_umma2_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    n = clusters + 1;
+    known[splits].v[dev].store(n, std::memory_order_release);
+  }
+  return n - 1;
+}
+
 // Whether launch_prefill_umma2 will take a batch with these parameters (a caller that knows so need not zero the output).
 bool prefill_umma2_usable(float scale, long long num_blocks) { return scale > 0.f && num_blocks >= 1 && u2_encode_fn() != nullptr; }
 
@@ -785,14 +806,11 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          long long num_blocks, const int32_t* block_tables, int table_width,
                          const int32_t* kv_lens, const int32_t* positions, const int32_t* query_start_loc,
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
-                         int skip_single, int split_p, int tile_pairs, float* split_area, size_t split_bytes,
-                         int32_t* beside, cudaStream_t stream) {
+                         int skip_single, int split_p, int tile_pairs, bool may_split, int32_t* beside, cudaStream_t stream) {
   static PerDeviceFlags opted_in;
-  constexpr int kSmemBytes = (int)sizeof(Umma2Smem) + 1024;
-  static_assert(kSmemBytes <= 232448, "tiles exceed the shared memory of one CTA");
   if (!(scale > 0.f) || num_blocks < 1 || !u2_encode_fn()) return NVJ_ERR_UNSUPPORTED;
   if (!once_per_device(opted_in, [](int) {
-        return cudaFuncSetAttribute(prefill_umma2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess;
+        return cudaFuncSetAttribute(prefill_umma2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kU2SmemBytes) == cudaSuccess;
       }))
     return NVJ_ERR_LAUNCH;
   CUtensorMap k_map, v_map;
@@ -814,37 +832,16 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
   const int most_pairs = (token_bucket + 2 * kU2Tokens - 1) / (2 * kU2Tokens) + rows;
   const int pairs = tile_pairs >= 0 && tile_pairs + 1 < most_pairs ? tile_pairs + 1 : most_pairs;
   p.counted = pairs < most_pairs;
-  // Key-range splits: only while the batch leaves pair slots free, as many as the lent area holds; the kernel settles
-  // the number per pair from what the batch really holds.
+  // Key-range splits: only while the batch leaves pair slots free, by the most pairs that it can hold (a batch of many short rows
+  // is launched whole: its extra splits would only scan the rows and leave, 200 us on 256 rows of 4 tokens); the kernel settles
+  // the number per pair from what the batch really holds.  The pairs of a tile are one cluster, and a GPC has room for whole ones only.
   int splits = 1;
-  const int slots = u2_pair_slots();
-  if (split_area && slots > 0) {
-    // by the most clusters the batch can hold (a batch of many short rows is launched whole: its extra splits would
-    // only scan the rows and leave, 200 us on 256 rows of 4 tokens)
-    const int most = pairs * kHkv;
-    splits = slots / most < kU2MaxSplits ? slots / most : kU2MaxSplits;
-    const size_t per_split = sizeof(float) * (size_t)token_bucket * kHq * (kD + 2);
-    const size_t info_bytes = ws_round(sizeof(int4) * 2 * (size_t)pairs * kHkv);
-    const size_t room = split_bytes < prefill_split_bytes() ? split_bytes : prefill_split_bytes();
-    while (splits > 1 && ws_round(per_split * splits) + info_bytes > room) --splits;
-    if (splits < 1) splits = 1;
-    // The partials end where the lent area ends: its low end borders arrival counters of calls with more rows.
-    split_area = reinterpret_cast<float*>(reinterpret_cast<char*>(split_area) + split_bytes - ws_round(per_split * splits) - info_bytes);
+  if (may_split) {
+    p.pair_slots = u2_pair_slots();
+    for (int s = 2; s <= kU2MaxSplits && s * pairs * kHkv <= p.pair_slots; ++s)
+      if ((pairs - 1) * kHkv <= u2_clusters_at_once(s)) splits = s;  // (one pair per head, if not more, is idle and leaves at once)
   }
-  if (splits > 1) {
-    p.part_o = split_area;
-    p.part_ml = split_area + (size_t)splits * token_bucket * kHq * kD;
-    p.tile_info = reinterpret_cast<int4*>(reinterpret_cast<char*>(split_area) + ws_round(sizeof(float) * (size_t)splits * token_bucket * kHq * (kD + 2)));
-    p.pair_slots = slots;
-  }
-  dim3 grid(2 * pairs, kHkv, splits);
-  launch_after(prefill_umma2_kernel, grid, kU2Threads, kSmemBytes, stream, k_map, v_map, p);
-  if (cudaGetLastError() != cudaSuccess) return NVJ_ERR_LAUNCH;
-  if (splits > 1) {
-    if (launch_after(prefill_umma2_merge_kernel, dim3(2 * pairs, kHkv, kU2MergeParts), kU2MergeThreads, 0, stream, p) != cudaSuccess)
-      return NVJ_ERR_LAUNCH;
-  }
-  return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
+  return u2_launch(dim3(2 * pairs, kHkv, splits), stream, k_map, v_map, p) == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;
 }
 
 }  // namespace nvj

@@ -53,3 +53,20 @@ def test_a_count_that_is_too_small_is_flagged(monkeypatch):
     with pytest.raises(DeviceStatusError):
         kvc.paged_attention_prefill_packed(q, k, v, tables, lens, pos, rid, qsl, BS, SCALE, 4, out_dtype=torch.float32,
                                            num_decode_rows=0, query_tile_pairs=3)
+
+
+# key ranges around where a pair is split (5, 6, 7 tiles of 64 keys), long ones in 4, 3 and 2 pieces as the batch leaves room, a row
+# of each kind in one launch, rows without keys, and a batch whose pairs do not all fit beside each other in clusters of four
+@pytest.mark.parametrize("qlens,cached,pad", [
+    ((2,), (5 * 64 - 3,), 1), ((64,), (5 * 64,), 0), ((33, 64), (6 * 64, 6 * 64 + 1), 5), ((2, 130, 70, 5), (0, 1500, 300, 900), 9),
+    ((64,) * 6, (1000, 0, 350, 330, 2000, 64), 0), ((64,) * 8, (700,) * 8, 3), ((300, 200, 90), (512, 1024, 0), 0), ((64,) * 20, (800,) * 20, 0),
+])
+def test_split_key_ranges_equal_the_kernel_that_never_splits(qlens, cached, pad):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    q, (k, v), tables, lens, pos, rid, qsl = _batch(qlens, cached, pad, sum(qlens))
+    pairs = sum(-(-n // 64) for n in qlens)
+    args = (q, k[0], v[0], tables, lens, pos, qsl, BS, SCALE, 4)
+    ref = K.packed_paged_prefill_attention(*args, variant=3, num_decode_rows=0)
+    for count in (pairs, None):
+        out = K.packed_paged_prefill_attention(*args, variant=4, num_decode_rows=0, query_tile_pairs=count)
+        assert float((out - ref).abs().max()) <= 2e-3 and not out[0, sum(qlens):].any()
