@@ -274,13 +274,20 @@ static bool cw_takes(const DecodeParams& p) {
 }
 static int cw_cluster(const DecodeParams& p, int sms) { return cluster_size(p.batch, p.table_width, sms, 1, kCmPerSm, 8, kClMaxCluster); }
 
-// Where the clusters beat the streaming forms: few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs
-// that are resident at once.  Beyond 4 tokens a block takes 1.5 us and the tcgen05 form is the faster one from 4 blocks on.
+// Where the clusters beat the tcgen05 form: few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs that are
+// resident at once.  Clusters : tcgen05, us, by table width, rows and CTAs per row: 3 tokens, 7 blocks per CTA, 32 x 64 (10 CTAs)
+// 20.7 : 21.1, 64 x 40 (6) 21.0 : 24.0, 128 x 16 (3, 6 blocks) 18.4 : 25.9; 8 blocks per CTA, 16 x 128 (16) 22.1 : 20.7, 4 x 128 15.9 : 15.9;
+// more CTAs than places, 140 x 40 40.7 : 36.2.  4 tokens: 64 x 40 22.9 : 24.9, 16 x 32 15.1 : 14.8, 16 x 128 23.7 : 21.4.  2 tokens: 16 x 128
+// 18.3 : 21.2, 64 x 40 18.5 : 24.0, 2 x 157 (10 blocks) 14.6 : 15.3, 8 x 256 (16 blocks) 23.4 : 22.7.  And many short rows, of which
+// every one costs the tcgen05 form a change of rows: 256 x 16 29.2 : 36.9, 36.3 : 38.6 and 39.1 : 40.9 (2, 3 and 4 tokens), 400 x 4
+// 14.3 : 34.4, 18.6 : 37.4 and 20.0 : 40.8, 200 x 25 31.0 : 35.8, 37.7 : 37.5 and 40.2 : 39.4.  Beyond 4 tokens a block takes 1.5 us
+// and the tcgen05 form is the faster one from 4 blocks on.
 bool decode_cluster_wide_pays(const DecodeParams& p) {
   const int sms = decode_wide_num_ctas();
   if (!cw_takes(p) || sms <= 0) return false;
   const int c = cw_cluster(p, sms), per_cta = (p.table_width + c - 1) / c;
-  return p.width == 2 ? per_cta <= 12 && 4LL * c * p.batch <= 7 * sms : per_cta <= 8 && (long long)c * p.batch <= sms;
+  if (p.batch >= 100 && p.table_width <= (p.width == 2 ? 25 : 16)) return true;
+  return per_cta <= (p.width == 2 ? 12 : 7) && 100LL * c * p.batch <= (long long)kCmPerSm * sms;
 }
 
 // Rows of 2 - 4 bf16 query tokens over a dense table, already appended.

@@ -13,20 +13,24 @@
 // Work split.  The blocks of all rows form one sequence cut into equal ranges as in the other decode kernels
 // (decode_parts.cuh), but a range belongs to a PAIR of CTAs, one per KV head: CTA 2c + h streams head h's half of
 // every block of range c, so every K/V byte still crosses HBM once.  Keys are walked in tiles of up to four blocks
-// that never straddle a row; a tile's K lands as [64-d chunk][64 keys][128 B] (one 2 KiB TMA box per block and
-// chunk, so that the whole tile is one N = 64 operand), its V block by block as [chunk][16 keys][128 B] (one 8 KiB
-// box per block: P V contracts 16 keys per MMA anyway).  One CTA per SM (192 KiB of shared memory: three tiles in
-// flight; 512 TMEM columns).
+// that never straddle a row; a block's K lands as [8-key group][64-d chunk][8 keys][128 B] (the groups of a tile are then evenly
+// spaced and the whole tile is one N = 64 operand), its V as [chunk][16 keys][128 B] (P V contracts 16 keys per MMA), one 8 KiB
+// TMA box each.  One CTA per SM (192 KiB of shared memory: three tiles of K and of V in flight; 512 TMEM columns: query rows,
+// scores, weights, output).
 //   warp 0   (and warp 1 for rows of more than 8 tokens: a warp may only touch the 32 TMEM lanes of its quarter)
-//            softmax and epilogue: lane r = query row r = token * 4 + head of the group.  Per row segment it stages
-//            the query rows into tensor memory, per tile of up to four blocks (64 keys) reads the scores
-//            (tcgen05.ld), masks (key < length, key <= the token's position), keeps the running maximum lazily (O in
-//            tensor memory is rescaled only when a tile exceeds it by 2^8) and writes the weights back over the
-//            scores as two bf16 terms (hi + lo); at the end of the segment it reads O and stores the row (whole row
-//            in this range) or the un-normalised partial with its (max, sum).
-//   warp 3   producer: block ids straight from the block table (32 at a time), TMA boxes into the ring.
-//   warp 2   MMA issue: S(t) = Q K(t)^T into one of two score buffers, O += P(t) V(t) once the weights are
-//            written; S(t + 2) follows P V (t).  tcgen05.commit releases ring stages and signals the softmax warp.
+//            softmax: lane r = query row r = token * 4 + head of the group.  Per tile it reads the scores (tcgen05.ld), which frees
+//            them for the next tile's, masks (key < length, key <= the token's position), keeps the running maximum lazily (O
+//            in tensor memory is rescaled only when a tile exceeds it by 2^8) and writes the weights as two bf16 terms (hi + lo).
+//            At the end of a row segment it reads half of O's columns: the row (whole row in this range) or the un-normalised
+//            partial with its (max, sum).
+//   warp 4   (and 5) on the same lanes: the other half of O, and the next segment's query rows into tensor memory as soon as the
+//            segment's last scores have been computed.
+//   warp 2   MMA issue: S(t + 1) = Q K(t + 1)^T while the softmax is at work on S(t), then O += P(t) V(t) once the weights are
+//            written.  tcgen05.commit releases ring stages and signals the other warps.  (With the weights written over their
+//            scores, S(t + 2) had to follow P V(t): 1.77 us per tile whose bytes take 1.45.  Three score buffers, the query rows
+//            in shared memory instead: 77 us where this form takes 65 and that one took 70; an MMA that reads 128 rows of A from
+//            there is slow.)
+//   warp 3   K producer, warp 7 V producer: block ids straight from the block table (32 at a time), TMA boxes into the rings.
 // A row cut over several ranges is folded afterwards by decode_umma_merge_kernel (one CTA per row, stream order
 // instead of counters and fences): the merge costs a second small launch, which rows of this width can afford.
 // Every wait is bounded; on a timeout the kernel flags NVJ_DEV_TIMEOUT, stops issuing, lets copies in flight land
@@ -46,23 +50,33 @@ constexpr int kUdStages = 3;      // tiles (K and V of one KV head for up to 64 
 constexpr int kUdTileBlocks = 4;  // blocks per tile: 64 keys
 constexpr int kUdTmemCols = 512;
 constexpr int kUdColQ = 0;        // query rows as the A operand: 256 bf16 per row = 128 columns
-constexpr int kUdColS = 128;      // two score buffers of 64 columns; the weights (hi: 32 columns, lo: 32) overwrite theirs
+constexpr int kUdColS = 128;      // scores of a tile
+constexpr int kUdColP = 192;      // its weights: hi 32 columns, lo 32
 constexpr int kUdColO = 256;      // output accumulator: columns [256, 512)
 constexpr int kUdHalfBlock = kBlk * kD * 2;  // K (or V) of one KV head of one block: 8 KiB
 constexpr float kUdRescaleGap = 8.f;
 constexpr int kUdMaxWidth = 16;  // 64 query rows per KV head: two softmax warps
-constexpr int kUdRowEndCost = 6;  // what a row end costs a CTA here, in blocks (6 and 12 measured alike, 18 and 24 worse)
+constexpr int kUdRowEndCost = 9;  // what a row end costs a CTA here, in blocks (128 rows of 5 tokens: 125.7 us with 3, 125.0 with 6, 124.5 with 9)
 
 struct UdSmem {
   alignas(1024) char k[kUdStages][kUdTileBlocks][kUdHalfBlock];    // [stage][block][8-key group][64-d chunk][8 keys][128 B], swizzled
   alignas(1024) char v[kUdStages][kUdTileBlocks][kUdHalfBlock];    // [stage][block][64-d chunk][16 keys][128 B], swizzled
-  alignas(8) unsigned long long full_bar[kUdStages], empty_bar[kUdStages], q_full, s_full[2], p_full, pv_done, o_free;
-  float red[384];
+  alignas(8) unsigned long long k_full[kUdStages], k_empty[kUdStages], v_full[kUdStages], v_empty[kUdStages],
+      q_full, q_free, s_full, s_read, p_full, pv_done, o_ready[2], o_free;
+  float inv[64];  // per query row: what the segment's output is scaled by
   int scan[16];
   int start_b, start_j, abort_flag;
   uint32_t tmem_base;
 };
 
+// Position in a ring of kUdStages.
+struct UdRing {
+  int at = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void step() {
+    if (++at == kUdStages) { at = 0; phase ^= 1u; }
+  }
+};
 // One KV head's half of a block (8 KiB): V through the view of ud_make_v_map ...
 __device__ __forceinline__ void ud_tma_v(uint32_t dst, const CUtensorMap* map, int token, int kvh, uint32_t bar, uint64_t policy) {
   asm volatile(
@@ -78,14 +92,18 @@ __device__ __forceinline__ void ud_tma_k(uint32_t dst, const CUtensorMap* map, i
       : "memory");
 }
 
-// ---- warp 3: TMA loads --------------------------------------------------------------------------
-__device__ __forceinline__ void ud_producer(const CUtensorMap* k_map, const CUtensorMap* v_map, const DecodeParams& p,
-                                            UdSmem& sm, int kvh, int b, int j, long long g, long long g1, int lane) {
+// ---- warps 3 and 7: TMA loads of K and of V --------------------------------------------------------------
+// The first round of stages is all the K warp's, in the order in which the tiles want it (with both warps at it, the first tile's K
+// would share the SM's intake with its V).
+template <bool kK>
+__device__ __forceinline__ void ud_producer(const CUtensorMap* k_map, const CUtensorMap* v_map, const DecodeParams& p, UdSmem& sm, int kvh,
+                                            int b, int j, long long g, long long g1, int lane) {
   const int oob = (int)(p.num_blocks * kBlk);  // a box that starts here is filled with zeros
   uint64_t policy;  // every block is read once: do not let it displace what the L2 is good for
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   Seg s;
-  uint32_t gt = 0;  // tiles so far, over all segments
+  UdRing at;
+  bool reuse = false;  // the stage has been used before
   while (next_seg(p, b, j, g, g1, s)) {
     const long long tbase = decode_table_base(p, s.b);
     for (int jb = s.j0; jb < s.j1; jb += 32) {  // 32 block ids = 8 tiles at a time
@@ -98,145 +116,163 @@ __device__ __forceinline__ void ud_producer(const CUtensorMap* k_map, const CUte
           id = -1;
         }
       }
-      for (int i0 = 0; i0 < n; i0 += kUdTileBlocks, ++gt) {
+      for (int i0 = 0; i0 < n; i0 += kUdTileBlocks) {
         const int cnt = n - i0 < kUdTileBlocks ? n - i0 : kUdTileBlocks;
-        const int stage = (int)(gt % kUdStages);
-        if (gt >= kUdStages && !um_wait(&sm.empty_bar[stage], ((gt / kUdStages) - 1) & 1u, &sm.abort_flag, p.status)) return;
-        const uint32_t fb = smem_u32(&sm.full_bar[stage]);
-        if (lane == 0) mbar_arrive_expect_tx(fb, (uint32_t)cnt * 2u * kUdHalfBlock);
-        __syncwarp();
-        for (int i = 0; i < cnt; ++i) {
-          const int blk = __shfl_sync(kFullMask, id, i0 + i);
-          const int token = blk >= 0 ? blk * kBlk : oob;
-          if (lane == 0) ud_tma_k(smem_u32(&sm.k[stage][i][0]), k_map, token / 8, kvh, fb, policy);
-          else if (lane == 1) ud_tma_v(smem_u32(&sm.v[stage][i][0]), v_map, token, kvh, fb, policy);
+        if (reuse && !um_wait(kK ? &sm.k_empty[at.at] : &sm.v_empty[at.at], at.phase ^ 1u, &sm.abort_flag, p.status)) return;
+        const int blk = __shfl_sync(kFullMask, id, i0 + (lane & (kUdTileBlocks - 1)));
+        const int token = blk >= 0 ? blk * kBlk : oob;
+        if (kK) {
+          const uint32_t full = smem_u32(&sm.k_full[at.at]);
+          if (lane == 0) mbar_arrive_expect_tx(full, (uint32_t)cnt * kUdHalfBlock);
+          __syncwarp();
+          if (lane < cnt) ud_tma_k(smem_u32(&sm.k[at.at][lane][0]), k_map, token / 8, kvh, full, policy);  // a lane per block
+        }
+        if (kK != reuse) {
+          const uint32_t full = smem_u32(&sm.v_full[at.at]);
+          if (lane == 0) mbar_arrive_expect_tx(full, (uint32_t)cnt * kUdHalfBlock);
+          __syncwarp();
+          if (lane < cnt) ud_tma_v(smem_u32(&sm.v[at.at][lane][0]), v_map, token, kvh, full, policy);
         }
         __syncwarp();
+        at.step();
+        if (at.at == 0) reuse = true;
       }
     }
   }
 }
 
 // ---- warp 2: MMA issue --------------------------------------------------------------------------
-// Scores of tile `gt` (stage gt % kUdStages) into score buffer gt & 1: columns of blocks the tile does not have are
-// computed from whatever the stage holds there and masked by the softmax warp.
-__device__ __forceinline__ bool ud_issue_s(UdSmem& sm, const DecodeParams& p, uint32_t tmem, uint64_t k_desc0, uint32_t gt) {
-  const int stage = (int)(gt % kUdStages);
-  if (!um_wait(&sm.full_bar[stage], (gt / kUdStages) & 1u, &sm.abort_flag, p.status)) return false;
-  tc_fence_after_sync();
-  if (um_elect_one()) {
-    constexpr uint32_t idesc = umma_idesc(kUdTileBlocks * kBlk, false);
-    const uint64_t k_desc = k_desc0 + (uint64_t)((stage * kUdTileBlocks * kUdHalfBlock) >> 4);
-    const uint32_t d = tmem + kUdColS + (gt & 1u) * 64;
-#pragma unroll
-    for (int ks = 0; ks < 16; ++ks)  // 16 dims per MMA: 8 columns of Q; K chunk ks / 4, 32 bytes into its swizzled rows
-      umma_bf16_ts(d, tmem + kUdColQ + ks * 8, k_desc + (uint64_t)(((ks >> 2) * (8 * 128) + (ks & 3) * 32) >> 4),
-                   idesc, ks > 0 ? 1u : 0u);
-    umma_commit(smem_u32(&sm.s_full[gt & 1u]));
+// Walks the range's tiles: once for the scores, once for the weighted sums.
+struct UdTiles {
+  Seg s;
+  int b, j, t, nt, seg;  // tile t of the segment's nt; segments so far
+  long long g;
+  UdRing at;
+  bool have;
+  __device__ __forceinline__ void enter(const DecodeParams& p, long long g1) {
+    have = next_seg(p, b, j, g, g1, s);
+    t = 0;
+    nt = have ? (s.j1 - s.j0 + kUdTileBlocks - 1) / kUdTileBlocks : 0;
   }
-  __syncwarp();
-  return true;
-}
+  __device__ __forceinline__ void step(const DecodeParams& p, long long g1) {
+    at.step();
+    if (++t == nt) { ++seg; enter(p, g1); }
+  }
+};
 
 __device__ __forceinline__ void ud_mma_warp(UdSmem& sm, const DecodeParams& p, uint32_t tmem, int b, int j, long long g,
                                             long long g1) {
   const uint64_t k_desc0 = umma_desc(smem_u32(&sm.k[0][0][0]), 16, 4 * 8 * 128);   // K: keys are rows (groups of 8: 4 KiB apart), dims contracted
   const uint64_t v_desc0 = umma_desc(smem_u32(&sm.v[0][0][0]), kBlk * 128, 1024);  // V: 64-d chunks 2 KiB apart, keys contracted
-  Seg s;
-  uint32_t gt = 0;  // tiles so far, over all segments: picks the stage, the score buffer and the barrier phases
-  uint32_t seg = 0;
-  while (next_seg(p, b, j, g, g1, s)) {
-    const int nblk = s.j1 - s.j0, nt = (nblk + kUdTileBlocks - 1) / kUdTileBlocks;
-    if (!um_wait(&sm.q_full, seg & 1u, &sm.abort_flag, p.status)) return;
-    for (int t = 0; t < 2 && t < nt; ++t)
-      if (!ud_issue_s(sm, p, tmem, k_desc0, gt + t)) return;
-    for (int t = 0; t < nt; ++t, ++gt) {
-      const int cnt = nblk - t * kUdTileBlocks < kUdTileBlocks ? nblk - t * kUdTileBlocks : kUdTileBlocks;
-      const int stage = (int)(gt % kUdStages);
-      if (!um_wait(&sm.p_full, gt & 1u, &sm.abort_flag, p.status)) return;
-      // the first P V of a segment overwrites O: the segment before must have been read out
-      if (t == 0 && seg > 0 && !um_wait(&sm.o_free, (seg - 1) & 1u, &sm.abort_flag, p.status)) return;
-      tc_fence_after_sync();
-      if (um_elect_one()) {
-        constexpr uint32_t idesc = umma_idesc(kD, true);
-        const uint32_t pa = tmem + kUdColS + (gt & 1u) * 64;
-        for (int i = 0; i < cnt; ++i) {  // 16 keys per MMA: 8 columns of P, the block's two 8-key groups of V
-          const uint64_t dv = v_desc0 + (uint64_t)(((stage * kUdTileBlocks + i) * kUdHalfBlock) >> 4);
-          umma_bf16_ts(tmem + kUdColO, pa + i * 8, dv, idesc, (t > 0 || i > 0) ? 1u : 0u);
-          umma_bf16_ts(tmem + kUdColO, pa + 32 + i * 8, dv, idesc, 1u);
-        }
-        umma_commit(smem_u32(&sm.empty_bar[stage]));
-        umma_commit(smem_u32(&sm.pv_done));
-      }
-      __syncwarp();
-      // S(t + 2) overwrites the columns P V (t) reads P(t) from, and every phase of pv_done is observed in turn
-      if (!um_wait(&sm.pv_done, gt & 1u, &sm.abort_flag, p.status)) return;
-      if (t + 2 < nt && !ud_issue_s(sm, p, tmem, k_desc0, gt + 2)) return;
+  UdTiles sc{};  // the next scores to be issued
+  sc.b = b; sc.j = j; sc.g = g;
+  sc.enter(p, g1);
+  UdTiles pv = sc;  // the next weighted sum
+  uint32_t scored = 0, done = 0;  // tiles so far
+  // Scores of the next tile (columns of blocks that the tile does not have are computed from whatever the stage holds there and
+  // masked by the softmax warp), once the softmax has read the scores before.
+  auto issue_scores = [&] {
+    if (sc.t == 0 && !um_wait(&sm.q_full, (uint32_t)sc.seg & 1u, &sm.abort_flag, p.status)) return false;
+    if (!um_wait(&sm.k_full[sc.at.at], sc.at.phase, &sm.abort_flag, p.status)) return false;
+    if (scored > 0 && !um_wait(&sm.s_read, (scored - 1) & 1u, &sm.abort_flag, p.status)) return false;
+    tc_fence_after_sync();
+    if (um_elect_one()) {
+      constexpr uint32_t idesc = umma_idesc(kUdTileBlocks * kBlk, false);
+      const uint64_t k_desc = k_desc0 + (uint64_t)((sc.at.at * kUdTileBlocks * kUdHalfBlock) >> 4);
+#pragma unroll
+      for (int ks = 0; ks < 16; ++ks)  // 16 dims per MMA: 8 columns of Q; K chunk ks / 4, 32 bytes into its swizzled rows
+        umma_bf16_ts(tmem + kUdColS, tmem + kUdColQ + ks * 8, k_desc + (uint64_t)(((ks >> 2) * (8 * 128) + (ks & 3) * 32) >> 4), idesc,
+                     ks > 0 ? 1u : 0u);
+      umma_commit(smem_u32(&sm.s_full));
+      umma_commit(smem_u32(&sm.k_empty[sc.at.at]));
+      if (sc.t == sc.nt - 1) umma_commit(smem_u32(&sm.q_free));
     }
-    ++seg;
+    __syncwarp();
+    sc.step(p, g1);
+    ++scored;
+    return true;
+  };
+  while (pv.have) {
+    if (scored == done && !issue_scores()) return;
+    // The next tile's scores go first, unless they would have to wait for keys or queries; those of the first tiles, whose keys have
+    // been on their way from the start, in any case.  (Looking at both barriers in turn until one is ready takes more from the other
+    // warps than it gives: 66.0 -> 68.5 us.)
+    if (sc.have && scored == done + 1 &&
+        (scored < kUdStages || (um_test(&sm.k_full[sc.at.at], sc.at.phase) && (sc.t > 0 || um_test(&sm.q_full, (uint32_t)sc.seg & 1u)))) &&
+        !issue_scores())
+      return;
+    if (!um_wait(&sm.v_full[pv.at.at], pv.at.phase, &sm.abort_flag, p.status)) return;
+    if (!um_wait(&sm.p_full, done & 1u, &sm.abort_flag, p.status)) return;
+    // the first P V of a segment overwrites O: the segment before must have been read out
+    if (pv.t == 0 && pv.seg > 0 && !um_wait(&sm.o_free, (uint32_t)(pv.seg - 1) & 1u, &sm.abort_flag, p.status)) return;
+    tc_fence_after_sync();
+    if (um_elect_one()) {
+      constexpr uint32_t idesc = umma_idesc(kD, true);
+      const int nblk = pv.s.j1 - pv.s.j0, cnt = nblk - pv.t * kUdTileBlocks < kUdTileBlocks ? nblk - pv.t * kUdTileBlocks : kUdTileBlocks;
+      for (int i = 0; i < cnt; ++i) {  // 16 keys per MMA: 8 columns of P, the block's two 8-key groups of V
+        const uint64_t dv = v_desc0 + (uint64_t)(((pv.at.at * kUdTileBlocks + i) * kUdHalfBlock) >> 4);
+        umma_bf16_ts(tmem + kUdColO, tmem + kUdColP + i * 8, dv, idesc, (pv.t > 0 || i > 0) ? 1u : 0u);
+        umma_bf16_ts(tmem + kUdColO, tmem + kUdColP + 32 + i * 8, dv, idesc, 1u);
+      }
+      umma_commit(smem_u32(&sm.v_empty[pv.at.at]));
+      umma_commit(smem_u32(&sm.pv_done));
+    }
+    __syncwarp();
+    ++done;
+    pv.step(p, g1);
   }
 }
 
-// Query rows of one table row into tensor memory: lane = row (token * 4 + head), 256 dims -> 128 columns, two bf16 per
-// column; sixteen 16-byte loads in flight at a time (one at a time, the eight round trips to memory cost a segment
-// more than its epilogue).  `tmem` addresses this warp's lanes; `row` = 32 * warp + lane.  Arrives on q_full.
-__device__ __forceinline__ void ud_stage_q(UdSmem& sm, const DecodeParams& p, uint32_t tmem, int kvh, int row_b, int row) {
+// A segment's output out of tensor memory, columns [128 half, 128 half + 128): the row, or the range's partial.
+__device__ __forceinline__ void ud_store_output(const UdSmem& sm, const DecodeParams& p, uint32_t tmem, const Seg& s, int kvh, int range, int row,
+                                                int half) {
   const int tok = row >> 2, head = row & 3;
-  const bool real = tok < p.width;
-  const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.q) +
-                                                    (((long long)row_b * p.width + (real ? tok : 0)) * kHq + kvh * kG + head) * kD);
+  const bool whole_row = (s.j0 == 0 && s.j1 == s.nb);
+  const int slot = partial_slot(range, s.j0 == 0);
+  const float inv = sm.inv[row];
+  const long long at = whole_row ? ((long long)s.b * p.width + tok) * kHq + kvh * kG + head
+                                 : (long long)slot * (p.width * kHq) + tok * kHq + kvh * kG + head;
+  float* dst = (whole_row ? p.out : p.part_acc) + at * kD + half * (kD / 2);
 #pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    uint4 u[16];
+  for (int cc = 0; cc < kD / 64; ++cc) {
+    float o[32];
+    tmem_ld32(tmem + kUdColO + half * (kD / 2) + cc * 32, o);
+    if (tok < p.width) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) u[i] = real ? ld_stream_u4(src + half * 16 + i) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-    for (int part = 0; part < 4; ++part) {  // 32 dims = 16 columns at a time
-      uint32_t w[16];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        w[4 * i] = u[part * 4 + i].x; w[4 * i + 1] = u[part * 4 + i].y; w[4 * i + 2] = u[part * 4 + i].z; w[4 * i + 3] = u[part * 4 + i].w;
-      }
-      tmem_st16(tmem + kUdColQ + half * 64 + part * 16, w);
+      for (int i = 0; i < 32; i += 4)
+        *reinterpret_cast<float4*>(dst + cc * 32 + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
     }
   }
-  tmem_st_wait();
-  tc_fence_before_sync();
-  mbar_arrive(smem_u32(&sm.q_full));
 }
 
-// ---- warps 0 and 1: query staging, softmax, epilogue ----------------------------------------------------
+// ---- warps 0 and 1: softmax, half of the output ------------------------------------------------------------
 __device__ __forceinline__ void ud_softmax_warp(UdSmem& sm, const DecodeParams& p, uint32_t tmem, int kvh, int b, int j,
                                                 long long g, long long g1, int range, int row) {
   const int tok = row >> 2, head = row & 3;
   const bool real = tok < p.width;
   const float scale_log2 = p.scale * kLog2e;
-  const int slot_rows = p.width * kHq;
-  Seg s, nxt;
-  uint32_t gt = 0;
-  bool have = next_seg(p, b, j, g, g1, s);
-  if (have) ud_stage_q(sm, p, tmem, kvh, s.b, row);
-  while (have) {
-    const long long qbase = (long long)s.b * p.width;
-    bool have_next = false;
-    const int my_pos = real ? (p.positions ? p.positions[qbase + tok] : 0x7fffffff) : -1;
+  Seg s;
+  uint32_t done = 0;  // tiles so far
+  while (next_seg(p, b, j, g, g1, s)) {
+    const int my_pos = real ? (p.positions ? p.positions[(long long)s.b * p.width + tok] : 0x7fffffff) : -1;
     const int last_key = my_pos < s.len - 1 ? my_pos : s.len - 1;  // last key this row may see
     float m_row = -INFINITY, l_row = 0.f;                           // m_row in units of log2(e) * scale
     const int nblk = s.j1 - s.j0, nt = (nblk + kUdTileBlocks - 1) / kUdTileBlocks;
-    for (int t = 0; t < nt; ++t, ++gt) {
-      const uint32_t s_tmem = tmem + kUdColS + (gt & 1u) * 64;
-      if (!um_wait(&sm.s_full[gt & 1u], (gt >> 1) & 1u, &sm.abort_flag, p.status)) return;
+    for (int t = 0; t < nt; ++t, ++done) {
+      if (!um_wait(&sm.s_full, done & 1u, &sm.abort_flag, p.status)) return;
       tc_fence_after_sync();
       float sc[64];
       {
         float a[32];
-        tmem_ld32(s_tmem, a);
+        tmem_ld32(tmem + kUdColS, a);
 #pragma unroll
         for (int i = 0; i < 32; ++i) sc[i] = a[i];
-        tmem_ld32(s_tmem + 32, a);
+        tmem_ld32(tmem + kUdColS + 32, a);
 #pragma unroll
         for (int i = 0; i < 32; ++i) sc[32 + i] = a[i];
       }
+      tc_fence_before_sync();
+      mbar_arrive(smem_u32(&sm.s_read));
       const int cnt = nblk - t * kUdTileBlocks < kUdTileBlocks ? nblk - t * kUdTileBlocks : kUdTileBlocks;
       int lim = last_key - (s.j0 + t * kUdTileBlocks) * kBlk;  // columns [0, lim] are visible
       lim = lim < cnt * kBlk - 1 ? lim : cnt * kBlk - 1;       // columns of blocks the tile does not have hold old scores
@@ -251,7 +287,7 @@ __device__ __forceinline__ void ud_softmax_warp(UdSmem& sm, const DecodeParams& 
         m_row = tmax;
       } else if (__any_sync(kFullMask, tmax > m_row + kUdRescaleGap)) {
         // rare: raise the maxima and rescale O, once the last P V has landed
-        if (!um_wait(&sm.pv_done, (gt - 1) & 1u, &sm.abort_flag, p.status)) return;
+        if (!um_wait(&sm.pv_done, (done - 1) & 1u, &sm.abort_flag, p.status)) return;
         tc_fence_after_sync();
         const float m_new = fmaxf(m_row, tmax);
         const float f = m_new == -INFINITY ? 1.f : ex2_approx(m_row - m_new);
@@ -277,58 +313,93 @@ __device__ __forceinline__ void ud_softmax_warp(UdSmem& sm, const DecodeParams& 
         hi[e] = *reinterpret_cast<const uint32_t*>(&h);
         lo[e] = *reinterpret_cast<const uint32_t*>(&r2);
       }
-      // every phase of pv_done is observed in turn (a parity wait tells only two consecutive phases apart)
-      if (gt >= 1 && !um_wait(&sm.pv_done, (gt - 1) & 1u, &sm.abort_flag, p.status)) return;
+      // P V of the tile before has read its weights (every phase of pv_done is observed in turn: a parity wait tells only two
+      // consecutive phases apart)
+      if (done >= 1 && !um_wait(&sm.pv_done, (done - 1) & 1u, &sm.abort_flag, p.status)) return;
       {  // P(t) as the A operand of P V: keys 2j, 2j + 1 in column j; hi in columns [0, 32), lo in [32, 64)
         uint32_t w[16];
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) w[i] = q4 < 2 ? hi[(q4 & 1) * 16 + i] : lo[(q4 & 1) * 16 + i];
-          tmem_st16(s_tmem + q4 * 16, w);
+          tmem_st16(tmem + kUdColP + q4 * 16, w);
         }
       }
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(smem_u32(&sm.p_full));
-      if (t == nt - 1) {
-        // The segment's last scores have been read, so all of its S products have retired and the query columns are
-        // free: the next row's queries go in now, and its first scores are computed while this segment's output is
-        // still being read out below (the MMA warp holds the next P V back until o_free).
-        have_next = next_seg(p, b, j, g, g1, nxt);
-        if (have_next) ud_stage_q(sm, p, tmem, kvh, nxt.b, row);
-      }
     }
-    // ---- end of the segment: O -> the output row (the whole row lies in this range) or this range's partial
-    if (!um_wait(&sm.pv_done, (gt - 1) & 1u, &sm.abort_flag, p.status)) return;
+    // ---- end of the segment: half of O for the warp that helps, half here
+    if (!um_wait(&sm.pv_done, (done - 1) & 1u, &sm.abort_flag, p.status)) return;
     tc_fence_after_sync();
     const bool whole_row = (s.j0 == 0 && s.j1 == s.nb);
-    const float inv = whole_row ? (l_row > 0.f ? 1.f / l_row : 0.f) : 1.f;
-    const int slot = partial_slot(range, s.j0 == 0);
-    const int row_in_slot = tok * kHq + kvh * kG + head;
-    float* dst = whole_row ? p.out + ((qbase + tok) * kHq + kvh * kG + head) * kD
-                           : p.part_acc + ((long long)slot * slot_rows + row_in_slot) * kD;
-#pragma unroll 1
-    for (int cc = 0; cc < kD / 32; ++cc) {
-      float o[32];
-      tmem_ld32(tmem + kUdColO + cc * 32, o);
-      if (real) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          *reinterpret_cast<float4*>(dst + cc * 32 + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
-      }
-    }
+    sm.inv[row] = whole_row ? (l_row > 0.f ? 1.f / l_row : 0.f) : 1.f;
+    tc_fence_before_sync();
+    mbar_arrive(smem_u32(&sm.o_ready[row >> 5]));
+    ud_store_output(sm, p, tmem, s, kvh, range, row, 0);
     if (real && !whole_row)
-      *reinterpret_cast<float2*>(p.part_ml + ((long long)slot * slot_rows + row_in_slot) * 2) =
+      *reinterpret_cast<float2*>(p.part_ml + ((long long)partial_slot(range, s.j0 == 0) * (p.width * kHq) + tok * kHq + kvh * kG + head) * 2) =
           make_float2(m_row == -INFINITY ? kNegBig : m_row, l_row);
     tc_fence_before_sync();  // the next segment's first P V overwrites what was just read
-    if (have_next) mbar_arrive(smem_u32(&sm.o_free));
-    s = nxt;
-    have = have_next;
+    mbar_arrive(smem_u32(&sm.o_free));
   }
 }
 
-__global__ void __launch_bounds__(kDecodeThreads, 1)
+// ---- warps 4 and 5: query rows, the other half of the output -----------------------------------------------
+// Query row `row` of table row `row_b` into tensor memory: 256 dims -> 128 columns, two bf16 per column; sixteen 16-byte loads in
+// flight at a time (one at a time, the eight round trips to memory cost a segment more than its epilogue), the first sixteen
+// before the wait for the columns.  `n`: segments staged before.
+__device__ __forceinline__ bool ud_stage_q(UdSmem& sm, const DecodeParams& p, uint32_t tmem, int kvh, int row_b, int row, uint32_t n) {
+  const int tok = row >> 2, head = row & 3;
+  const bool real = tok < p.width;
+  const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.q) +
+                                                    (((long long)row_b * p.width + (real ? tok : 0)) * kHq + kvh * kG + head) * kD);
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint4 u[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) u[i] = real ? ld_stream_u4(src + half * 16 + i) : make_uint4(0u, 0u, 0u, 0u);
+    if (half == 0 && n > 0) {  // the last scores of the segment before have been computed
+      if (!um_wait(&sm.q_free, (n - 1) & 1u, &sm.abort_flag, p.status)) return false;
+      tc_fence_after_sync();
+    }
+#pragma unroll
+    for (int part = 0; part < 4; ++part) {  // 32 dims = 16 columns at a time
+      uint32_t w[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        w[4 * i] = u[part * 4 + i].x; w[4 * i + 1] = u[part * 4 + i].y; w[4 * i + 2] = u[part * 4 + i].z; w[4 * i + 3] = u[part * 4 + i].w;
+      }
+      tmem_st16(tmem + kUdColQ + half * 64 + part * 16, w);
+    }
+  }
+  tmem_st_wait();
+  tc_fence_before_sync();
+  mbar_arrive(smem_u32(&sm.q_full));
+  return true;
+}
+
+__device__ __forceinline__ void ud_helper_warp(UdSmem& sm, const DecodeParams& p, uint32_t tmem, int kvh, int b, int j, long long g,
+                                               long long g1, int range, int row) {
+  Seg s, nxt;
+  bool have = next_seg(p, b, j, g, g1, s);
+  if (have && !ud_stage_q(sm, p, tmem, kvh, s.b, row, 0)) return;
+  for (uint32_t n = 0; have; ++n) {
+    const bool more = next_seg(p, b, j, g, g1, nxt);
+    if (more && !ud_stage_q(sm, p, tmem, kvh, nxt.b, row, n + 1)) return;
+    if (!um_wait(&sm.o_ready[row >> 5], n & 1u, &sm.abort_flag, p.status)) return;
+    tc_fence_after_sync();
+    ud_store_output(sm, p, tmem, s, kvh, range, row, 1);
+    tc_fence_before_sync();
+    mbar_arrive(smem_u32(&sm.o_free));
+    s = nxt;
+    have = more;
+  }
+}
+
+// 168 registers: a CTA of the merge launch (256 x 88) then fits beside this one and waits in place (16 rows of 4 tokens over 512 - 2048
+// keys 23.2 -> 22.4 us).
+__global__ void __maxnreg__(168)
 decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, DecodeParams p) {
   extern __shared__ unsigned char ud_smem_raw[];
   UdSmem& sm = *reinterpret_cast<UdSmem*>((reinterpret_cast<uintptr_t>(ud_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -339,14 +410,38 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&k_map)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&v_map)) : "memory");
     sm.start_b = p.batch; sm.start_j = 0; sm.abort_flag = 0;
+    for (int i = 0; i < kUdStages; ++i) {
+      mbar_init(smem_u32(&sm.k_full[i]), 1);
+      mbar_init(smem_u32(&sm.k_empty[i]), 1);
+      mbar_init(smem_u32(&sm.v_full[i]), 1);
+      mbar_init(smem_u32(&sm.v_empty[i]), 1);
+    }
+    const uint32_t quarters = p.width > 8 ? 2u : 1u;  // of the TMEM lanes: 32 query rows each
+    mbar_init(smem_u32(&sm.q_full), 32 * quarters);
+    mbar_init(smem_u32(&sm.q_free), 1);
+    mbar_init(smem_u32(&sm.s_full), 1);
+    mbar_init(smem_u32(&sm.s_read), 32 * quarters);
+    mbar_init(smem_u32(&sm.o_ready[0]), 32);
+    mbar_init(smem_u32(&sm.o_ready[1]), 32);
+    mbar_init(smem_u32(&sm.p_full), 32 * quarters);
+    mbar_init(smem_u32(&sm.pv_done), 1);
+    mbar_init(smem_u32(&sm.o_free), 64 * quarters);
+    mbar_fence_init();
   }
   pdl_wait();
+  // this CTA's share of the block tables into the L2, while the lengths are on their way
+  {
+    const long long lines = ((long long)p.batch * p.table_width * (long long)sizeof(int32_t) + 127) / 128;
+    const long long line = (long long)blockIdx.x * kDecodeThreads + threadIdx.x;
+    if (line < lines) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.block_tables) + line * 128));
+  }
   // ---- pass 1: total number of blocks; zero the output of inactive rows
-  int mine = 0;
+  int mine = 0, first_n = 0;
   for (int base = 0; base < p.batch; base += kDecodeThreads) {
     const int b = base + threadIdx.x;
     int len = 0;
     if (b < p.batch) len = decode_row_len(p, b);
+    if (base == 0) first_n = blocks_in_sequence(p, (len + kBlk - 1) / kBlk);
     mine += blocks_in_sequence(p, (len + kBlk - 1) / kBlk);
     const unsigned idle = __ballot_sync(kFullMask, b < p.batch && len <= 0 && (b % (int)gridDim.x) == (int)blockIdx.x);
     for (unsigned m = idle; m; m &= m - 1) {
@@ -356,7 +451,7 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     }
   }
   int total = 0;
-  cta_inclusive_scan(mine, sm.scan, total);
+  const int incl = cta_inclusive_scan(mine, sm.scan, total);
   if (total == 0) return;
   const Partition pt = make_partition(total, ranges);
   if (range >= pt.n) return;
@@ -366,6 +461,11 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
 
   // ---- pass 2: locate (row, block) of g0
   long long carry = 0;
+  if (p.batch <= kDecodeThreads) {  // one row per thread: the scan of pass 1 has the answer already
+    const long long excl = incl - first_n;
+    if (first_n > 0 && excl <= g0 && g0 < excl + first_n) { sm.start_b = threadIdx.x; sm.start_j = (int)(g0 - excl); }
+    carry = g0 + 1;  // skips the loop below
+  }
   for (int base = 0; base < p.batch && carry <= g0; base += kDecodeThreads) {
     const int b = base + threadIdx.x;
     int n = 0;
@@ -379,30 +479,21 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     tmem_alloc(smem_u32(&sm.tmem_base), kUdTmemCols);
     if (lane == 0) pdl_release();
   }
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kUdStages; ++i) {
-      mbar_init(smem_u32(&sm.full_bar[i]), 1);
-      mbar_init(smem_u32(&sm.empty_bar[i]), 1);
-    }
-    const uint32_t softmax_threads = p.width > 8 ? 64u : 32u;
-    mbar_init(smem_u32(&sm.q_full), softmax_threads);
-    mbar_init(smem_u32(&sm.s_full[0]), 1);
-    mbar_init(smem_u32(&sm.s_full[1]), 1);
-    mbar_init(smem_u32(&sm.p_full), softmax_threads);
-    mbar_init(smem_u32(&sm.pv_done), 1);
-    mbar_init(smem_u32(&sm.o_free), softmax_threads);
-    mbar_fence_init();
-  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = sm.tmem_base;
   const int b0 = sm.start_b, j0 = sm.start_j;
 
-  if (warp == 0 || (warp == 1 && p.width > 8))  // this warp's quarter of the TMEM lanes: rows 32 * warp ..
-    ud_softmax_warp(sm, p, tmem + ((uint32_t)(warp * 32) << 16), kvh, b0, j0, g0, g1, range, warp * 32 + lane);
-  else if (warp == 2) ud_mma_warp(sm, p, tmem, b0, j0, g0, g1);
-  else if (warp == 3) ud_producer(&k_map, &v_map, p, sm, kvh, b0, j0, g0, g1, lane);
+  const int quarter = warp & 3;  // of the TMEM lanes that this warp may touch: rows 32 * quarter ..
+  const uint32_t mine_tmem = tmem + ((uint32_t)(quarter * 32) << 16);
+  if (warp == 2) ud_mma_warp(sm, p, tmem, b0, j0, g0, g1);
+  else if (warp == 3) ud_producer<true>(&k_map, &v_map, p, sm, kvh, b0, j0, g0, g1, lane);
+  else if (warp == 7) ud_producer<false>(&k_map, &v_map, p, sm, kvh, b0, j0, g0, g1, lane);
+  else if (quarter == 0 || (quarter == 1 && p.width > 8)) {
+    if (warp < 4) ud_softmax_warp(sm, p, mine_tmem, kvh, b0, j0, g0, g1, range, quarter * 32 + lane);
+    else ud_helper_warp(sm, p, mine_tmem, kvh, b0, j0, g0, g1, range, quarter * 32 + lane);
+  }
 
   tc_fence_before_sync();
   __syncthreads();

@@ -500,13 +500,10 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
   if (n <= 0) return NVJ_ERR_LAUNCH;
   if (p.wide_form == 3 || (p.wide_form == 0 && p.cta_limit <= 0 && decode_cluster_wide_pays(p)))
     return launch_decode_cluster_wide(p, stream);
-  // Rows of 5 and more query tokens: the tcgen05 form (two 16-row tiles per warp pair make the mma.sync form
-  // compute-bound, and it ends at 8 tokens).  Below that the tcgen05 form answers sooner (4 tokens, 16 rows of 512 - 2048
-  // keys: 21.2 us against 29.7) and the mma.sync form streams better (128 rows of 1024 - 4096: 129 against 121); they meet at
-  // about 4096 blocks with 2 tokens (20.7 : 21.8 at 2048, 40.1 : 39.2 at 8192) and 12288 with 3 and 4 (39.6 : 44.5 at 8192,
-  // 70.2 : 70.8 and 69.4 : 68.3 at 16384).
-  const long long blocks = (long long)p.batch * p.table_width;
-  if (p.wide_form == 2 || (p.wide_form == 0 && p.width > 1 && (p.width > 4 || blocks <= (p.width == 2 ? 4096 : 12288)))) {
+  // The tcgen05 form for rows of 3 and more query tokens (mma.sync : tcgen05, us, 3 tokens over 1024 - 4096 keys: 64 rows 68.6 : 63.8, 192
+  // rows 184 : 172; 4 tokens: 64 rows 70.5 : 65.3, 192 rows 220 : 176, at the board's power limit; it ends at 8 tokens).  With 2
+  // they meet at about 32768 blocks: 64 rows 64.6 : 63.5, 128 rows 114.1 : 113.6, 192 rows 163 : 170.
+  if (p.wide_form == 2 || (p.wide_form == 0 && (p.width > 2 || (p.width == 2 && (long long)p.batch * p.table_width <= 32768)))) {
     const int rc = launch_decode_umma(p, stream);
     if (rc != NVJ_ERR_UNSUPPORTED || p.wide_form == 2) return rc;
   }

@@ -141,6 +141,19 @@ __device__ __forceinline__ bool um_wait(unsigned long long* bar, uint32_t parity
   return __all_sync(0xffffffffu, ok);
 }
 
+// Whether the phase has completed, without waiting; the same in every lane of the (converged) warp.
+__device__ __forceinline__ bool um_test(unsigned long long* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, ok != 0);
+}
+
 // One lane of a converged warp (the lowest); unlike a comparison with the lane index this keeps
 // the code that follows eligible for the uniform datapath the MMA instructions are issued from.
 __device__ __forceinline__ bool um_elect_one() {

@@ -142,3 +142,27 @@ def test_rows_of_nine_to_sixteen_tokens_take_the_tcgen05_form(width):
     from nano_vllm_jax_b200._lib import NvjError
     with pytest.raises(NvjError):  # the mma.sync form ends at 8
         _run(c, q, tables, lens, pos, 1)
+
+
+@pytest.mark.parametrize("width", [3, 5, 8, 9, 16])
+@pytest.mark.parametrize("lens", [[1 + (29 * i) % 90 for i in range(300)], [0, 64, 65, 0, 128, 129, 4000, 17, 1, 191, 192, 193] * 3], ids=["short", "ragged"])
+def test_rows_that_follow_one_another_in_a_range(lens, width):
+    """Ranges that hold several rows of a tile or two, and ones that end in the middle of a row: the next row's queries, scores and
+    output follow while the row before is still being read out; more rows than one scan takes."""
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    rows, need = len(lens), [-(-max(n, 1) // BS) for n in lens]
+    g = torch.Generator(device="cuda").manual_seed(rows + width)
+    pool = sum(need) + 3
+    k, v = (torch.randn((pool, BS, 2, 256), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    perm = torch.randperm(pool, generator=g, device="cuda").to(torch.int32)
+    tables, o = torch.zeros((rows, max(need)), dtype=torch.int32, device="cuda"), 0
+    for b, n in enumerate(need):
+        tables[b, :n] = perm[o:o + n]
+        o += n
+    t_lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    pos = (t_lens[:, None] - width + torch.arange(width, dtype=torch.int32, device="cuda")).contiguous()  # (some before the row's start)
+    q = torch.randn((rows, width, 8, 256), generator=g, device="cuda").to(torch.bfloat16)
+    got = K.paged_decode_attention_wide(q, k, v, tables, t_lens, pos, SCALE, form=2)
+    qsl = torch.arange(rows + 1, dtype=torch.int32, device="cuda") * width
+    ref = K.packed_paged_prefill_attention(q.view(1, rows * width, 8, 256), k, v, tables, t_lens, pos.view(1, -1), qsl, BS, SCALE, 4, variant=1)
+    assert float((got.view(-1) - ref.view(-1)).abs().max()) <= 2e-3
