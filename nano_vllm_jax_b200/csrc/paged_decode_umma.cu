@@ -84,7 +84,7 @@ __device__ __forceinline__ void ud_tma_v(uint32_t dst, const CUtensorMap* map, i
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(token), "r"(kvh), "r"(bar), "l"(policy)
       : "memory");
 }
-// ... and K through that of ud_make_k_map.  `group` counts groups of eight tokens.
+// ... and K through the grouped one of four chunks.  `group` counts groups of eight tokens.
 __device__ __forceinline__ void ud_tma_k(uint32_t dst, const CUtensorMap* map, int group, int kvh, uint32_t bar, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %2, %2, %3, %4}], [%5], %6;"
@@ -609,18 +609,21 @@ static bool ud_make_v_map(CUtensorMap* map, const void* base, uint64_t tokens) {
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// The same with the tokens in groups of eight, {64 dims, token of the group, 64-dim chunk, group, kv head}: a box of {64, 8, 4, 2, 1}
-// lands as [group][chunk][8 tokens][128 B], so that the groups of a tile of several blocks are evenly spaced (4 KiB), as the
-// rows of one operand have to be.
-static bool ud_make_k_map(CUtensorMap* map, const void* base, uint64_t tokens) {
+template <int kChunks>
+static bool ud_make_grouped_map(CUtensorMap* map, const void* base, uint64_t tokens) {
   const cuuint64_t dims[5] = {64, 8, 4, tokens / 8, (cuuint64_t)kHkv};
   const cuuint64_t strides[4] = {(cuuint64_t)kTokenBytes, 128, 8 * (cuuint64_t)kTokenBytes, (cuuint64_t)kRowBytes};
-  const cuuint32_t box[5] = {64, 8, 4, kBlk / 8, 1};
+  const cuuint32_t box[5] = {64, 8, kChunks, kBlk / 8, 1};
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   return ud_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+bool grouped_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t tokens, int chunks) {
+  return ud_encode_fn() && (chunks == 4 ? tensor_map_cached(map, 4, cache_layer, tokens, ud_make_grouped_map<4>)
+                                        : tensor_map_cached(map, 2, cache_layer, tokens, ud_make_grouped_map<2>));
+}
+bool tensor_maps_available() { return ud_encode_fn() != nullptr; }
 
 // p as launch_decode_wide takes it (width 1..8, carved workspace whose partial area holds ws_slots(decode_wide_num_ctas())
 // slots of width * kHq rows).  NVJ_ERR_UNSUPPORTED: no tensor-map encoder, a scale that is not positive (row maxima are
@@ -633,7 +636,7 @@ int launch_decode_umma(const DecodeParams& p, cudaStream_t stream) {
   if (ctas < 2) return NVJ_ERR_LAUNCH;
   const int ranges = ctas / 2;
   CUtensorMap k_map, v_map;
-  if (!tensor_map_cached(&k_map, 4, p.k_cache, (uint64_t)p.num_blocks * kBlk, ud_make_k_map) ||
+  if (!grouped_map_cached(&k_map, p.k_cache, (uint64_t)p.num_blocks * kBlk, 4) ||
       !tensor_map_cached(&v_map, 3, p.v_cache, (uint64_t)p.num_blocks * kBlk, ud_make_v_map))
     return NVJ_ERR_UNSUPPORTED;
   static PerDeviceFlags smem_opted_in;

@@ -14,8 +14,8 @@
 // warps 2-9 softmax); what crosses the pair:
 //   * both producers' TMA loads complete on CTA 0's full barriers (cp.async.bulk.tensor with
 //     .cta_group::2 and the barrier address of rank 0); no load is a multicast;
-//   * `tcgen05.commit` with a two-CTA mask releases K/V stages and S buffers in both CTAs;
-//   * the softmax threads of both CTAs arrive on CTA 0's "Q staged" and "P written" barriers.
+//   * `tcgen05.commit` with a two-CTA mask releases K/V stages and hands scores over in both CTAs;
+//   * the softmax warps of both CTAs arrive on CTA 0's "Q staged", "S read" and "P written" barriers.
 // A cluster barrier after set-up and one before the tensor memory is freed fence the pair.
 // Every mbarrier wait is bounded; a timeout flags NVJ_DEV_TIMEOUT and both CTAs still reach
 // the final cluster barrier and free their tensor memory.
@@ -41,7 +41,7 @@ constexpr int kU2Stages = 4;
 constexpr int kU2Threads = 320;
 constexpr int kU2SoftmaxThreads = 256;
 constexpr int kU2TmemCols = 512;
-constexpr int kU2ColQ = 0, kU2ColS = 128, kU2ColO = 256;
+constexpr int kU2ColQ = 0, kU2ColS = 128, kU2ColP = 192, kU2ColO = 256;  // queries, scores, weights (hi, lo), output
 constexpr uint32_t kU2TileBytes = kU2Keys * kRowBytes;  // a whole K (or V) tile: both CTAs' halves, 32 KiB
 constexpr uint32_t kU2LeaderMask = 0xFEFFFFFFu;         // clears the CTA-rank bit of a shared::cluster address
 constexpr float kU2Log2e = 1.4426950408889634f;
@@ -85,11 +85,11 @@ struct Umma2Params {
 };
 
 struct Umma2Smem {
-  alignas(1024) char k[kU2Stages][4][32 * 128];  // [stage][64-d chunk][this CTA's 32 keys][128 B]
-  alignas(1024) char v[kU2Stages][2][64 * 128];  // [stage][this CTA's two 64-d chunks][64 keys][128 B]
-  // used in CTA 0 only: q_full, k_full, v_full, p_full; used in both: the rest
+  alignas(1024) char k[kU2Stages][2][8192];  // [stage][this CTA's two blocks][8-key group][64-d chunk][8 keys][128 B]
+  alignas(1024) char v[kU2Stages][4][4096];  // [stage][block][8-key group][this CTA's two 64-d chunks][8 keys][128 B]
+  // used in CTA 0 only: q_full, k_full, v_full, s_read, p_full; used in both: the rest
   alignas(8) unsigned long long q_full, k_full[kU2Stages], v_full[kU2Stages], k_empty[kU2Stages], v_empty[kU2Stages],
-      s_full[2], p_full, pv_done, x_full;
+      s_full, s_read, p_full, pv_done, x_full;
   float xchg[2][2][kU2Rows];
   // this CTA's query rows on their way into tensor memory: [token][head of the group][32 pieces of 16 B], the pieces
   // of token t stored at (piece ^ (t & 7)) so that both the row-wise fill and the token-wise read are conflict-free
@@ -122,17 +122,22 @@ __device__ __forceinline__ void umma2_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"((uint16_t)(3u << (2 * blockIdx.z))) : "memory");
 }
-// One box into this CTA's shared memory; the bytes are counted on CTA 0's barrier at `bar`'s offset.
-__device__ __forceinline__ void tma2_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+// One box of a grouped view into this CTA's shared memory; the bytes are counted on CTA 0's barrier at `bar`'s offset.
+__device__ __forceinline__ void tma2_load_5d(uint32_t dst, const CUtensorMap* map, int chunk, int group, int kvh, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar & kU2LeaderMask)
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3, %4, %5}], [%6];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(chunk), "r"(group), "r"(kvh), "r"(bar & kU2LeaderMask)
       : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
   // default semantics (release at CTA scope): what the arrival publishes lives in tensor memory and is ordered by
   // tcgen05.wait::st + tcgen05.fence; a cluster-scope release here cost ~1700 cycles per arrival
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & kU2LeaderMask) : "memory");
+}
+// One arrival for a warp, once all of its lanes have come here.
+__device__ __forceinline__ void u2_arrive_warp(uint32_t bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive_leader(bar);
 }
 // Instruction descriptor, kind::f16, fp32 accumulate, bf16 A and B, M = 256 over the pair.
 __device__ __forceinline__ constexpr uint32_t umma2_idesc(int n, bool b_mn_major) {
@@ -144,7 +149,7 @@ __device__ __forceinline__ void u2_producer(const CUtensorMap* k_map, const CUte
                                             Umma2Smem& sm, int row, int kvh, int kv_len, int tile0, int n_tiles, int rank,
                                             int lane, int first_ids) {
   const int need_blocks = (kv_len + kBlk - 1) / kBlk;
-  const int oob = (int)(p.num_blocks * kBlk);  // a box that starts here is filled with zeros
+  const int oob = (int)(p.num_blocks * (kBlk / 8));  // a box that starts here is filled with zeros
   int ids = -1;
   for (int t = 0; t < n_tiles; ++t) {
     const int s = t % kU2Stages;
@@ -164,7 +169,7 @@ __device__ __forceinline__ void u2_producer(const CUtensorMap* k_map, const CUte
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int id = __shfl_sync(0xffffffffu, ids, (t & 7) * 4 + b);
-      z[b] = id >= 0 ? id * kBlk : oob;
+      z[b] = id >= 0 ? id * (kBlk / 8) : oob;
     }
     if (t >= kU2Stages && !um_wait(&sm.k_empty[s], reuse_parity, &sm.abort_flag, p.status)) break;
     if (lane == 0) {
@@ -172,9 +177,7 @@ __device__ __forceinline__ void u2_producer(const CUtensorMap* k_map, const CUte
       if (rank == 0) mbar_arrive_expect_tx(kb, kU2TileBytes);  // both CTAs' halves are counted here
 #pragma unroll
       for (int b2 = 0; b2 < 2; ++b2)  // this CTA's keys: cache blocks 2 rank, 2 rank + 1 of the tile
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          tma2_load_3d(smem_u32(&sm.k[s][c][0]) + b2 * (kBlk * 128), k_map, c * 64, kvh, rank ? z[2 + b2] : z[b2], kb);
+        tma2_load_5d(smem_u32(&sm.k[s][b2][0]), k_map, 0, rank ? z[2 + b2] : z[b2], kvh, kb);
     }
     if (t >= kU2Stages && !um_wait(&sm.v_empty[s], reuse_parity, &sm.abort_flag, p.status)) break;
     if (lane == 0) {
@@ -182,28 +185,29 @@ __device__ __forceinline__ void u2_producer(const CUtensorMap* k_map, const CUte
       if (rank == 0) mbar_arrive_expect_tx(vb, kU2TileBytes);
 #pragma unroll
       for (int b = 0; b < 4; ++b)  // all keys, this CTA's head dims: 64-d chunks 2 rank, 2 rank + 1
-#pragma unroll
-        for (int c2 = 0; c2 < 2; ++c2)
-          tma2_load_3d(smem_u32(&sm.v[s][c2][0]) + b * (kBlk * 128), v_map, (2 * rank + c2) * 64, kvh, z[b], vb);
+        tma2_load_5d(smem_u32(&sm.v[s][b][0]), v_map, 2 * rank, z[b], kvh, vb);
     }
     __syncwarp();
   }
 }
 
 // ---- warp 1 of CTA 0: MMA issue for the pair -------------------------------------------------
+// S(t + 1) is issued as soon as the softmax has read S(t), P V(t) behind it once the weights are written: while the weights of
+// one tile are on their way the tensor pipe has the scores of the next.  (With the weights written over their scores, in two
+// buffers, S(t + 2) had to wait for P V(t) to retire: 2030 cycles per pair and tile, 1640 of them MMAs.)
 __device__ __forceinline__ bool u2_issue_s(Umma2Smem& sm, const Umma2Params& p, uint32_t tmem, uint64_t k_desc0, int t,
                                            int stage, uint32_t full_parity) {
   if (!um_wait(&sm.k_full[stage], full_parity, &sm.abort_flag, p.status)) return false;
+  if (t > 0 && !um_wait(&sm.s_read, (t - 1) & 1, &sm.abort_flag, p.status)) return false;
   tc_fence_after_sync();
   if (um_elect_one()) {
     constexpr uint32_t idesc = umma2_idesc(kU2Keys, false);
-    const uint64_t k_desc = k_desc0 + (uint64_t)((stage * 4 * 32 * 128) >> 4);
-    const uint32_t d = tmem + kU2ColS + (t & 1) * kU2Keys;
+    const uint64_t k_desc = k_desc0 + (uint64_t)((stage * (int)sizeof(sm.k[0])) >> 4);
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks)  // 16 dims per MMA: 8 columns of Q; K chunk ks / 4, 32 bytes into its swizzled rows
-      umma2_bf16_ts(d, tmem + kU2ColQ + ks * 8, k_desc + (uint64_t)(((ks >> 2) * (32 * 128) + (ks & 3) * 32) >> 4), idesc,
+      umma2_bf16_ts(tmem + kU2ColS, tmem + kU2ColQ + ks * 8, k_desc + (uint64_t)(((ks >> 2) * (8 * 128) + (ks & 3) * 32) >> 4), idesc,
                     ks > 0 ? 1u : 0u);
-    umma2_commit_pair(smem_u32(&sm.s_full[t & 1]));
+    umma2_commit_pair(smem_u32(&sm.s_full));
     umma2_commit_pair(smem_u32(&sm.k_empty[stage]));
   }
   __syncwarp();
@@ -211,37 +215,30 @@ __device__ __forceinline__ bool u2_issue_s(Umma2Smem& sm, const Umma2Params& p, 
 }
 
 __device__ __forceinline__ void u2_mma_warp(Umma2Smem& sm, const Umma2Params& p, uint32_t tmem, int n_tiles) {
-  const uint64_t k_desc0 = umma_desc(smem_u32(&sm.k[0][0][0]), 16, 1024);
-  const uint64_t v_desc0 = umma_desc(smem_u32(&sm.v[0][0][0]), kU2Keys * 128, 1024);
+  const uint64_t k_desc0 = umma_desc(smem_u32(&sm.k[0][0][0]), 16, 4 * 8 * 128);       // keys are rows, groups of 8 4 KiB apart
+  const uint64_t v_desc0 = umma_desc(smem_u32(&sm.v[0][0][0]), 8 * 128, 2 * 8 * 128);  // 64-d chunks 1 KiB apart, groups of 8 keys 2
   if (!um_wait(&sm.q_full, 0, &sm.abort_flag, p.status)) return;
   if (!u2_issue_s(sm, p, tmem, k_desc0, 0, 0, 0)) return;
-  if (n_tiles > 1 && !u2_issue_s(sm, p, tmem, k_desc0, 1, 1, 0)) return;
-  int sv = 0, sk = 2 % kU2Stages;
-  uint32_t pv = 0, pk = 2 / kU2Stages;
+  int sv = 0, sk = 1 % kU2Stages;
+  uint32_t pv = 0, pk = 1 / kU2Stages;
   for (int t = 0; t < n_tiles; ++t) {
+    if (t + 1 < n_tiles && !u2_issue_s(sm, p, tmem, k_desc0, t + 1, sk, pk)) return;
     if (!um_wait(&sm.v_full[sv], pv, &sm.abort_flag, p.status)) return;
     if (!um_wait(&sm.p_full, t & 1, &sm.abort_flag, p.status)) return;
     tc_fence_after_sync();
     if (um_elect_one()) {
       constexpr uint32_t idesc = umma2_idesc(kD, true);
-      const uint64_t v_desc = v_desc0 + (uint64_t)((sv * 2 * kU2Keys * 128) >> 4);
-      const uint32_t pa = tmem + kU2ColS + (t & 1) * kU2Keys;
+      const uint64_t v_desc = v_desc0 + (uint64_t)((sv * (int)sizeof(sm.v[0])) >> 4);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {  // 16 keys per MMA: 8 columns of P, two 8-key groups of V
-        const uint64_t dv = v_desc + (uint64_t)((kk * 2048) >> 4);
-        umma2_bf16_ts(tmem + kU2ColO, pa + kk * 8, dv, idesc, (t > 0 || kk > 0) ? 1u : 0u);
-        if (p.split_p) umma2_bf16_ts(tmem + kU2ColO, pa + 32 + kk * 8, dv, idesc, 1u);
+        const uint64_t dv = v_desc + (uint64_t)((kk * 4096) >> 4);
+        umma2_bf16_ts(tmem + kU2ColO, tmem + kU2ColP + kk * 8, dv, idesc, (t > 0 || kk > 0) ? 1u : 0u);
+        if (p.split_p) umma2_bf16_ts(tmem + kU2ColO, tmem + kU2ColP + 32 + kk * 8, dv, idesc, 1u);
       }
       umma2_commit_pair(smem_u32(&sm.v_empty[sv]));
       umma2_commit_pair(smem_u32(&sm.pv_done));
     }
     __syncwarp();
-    // S(t + 2) overwrites the columns P V (t) reads P(t) from; MMAs of different shapes are not
-    // ordered against each other, so wait for P V (t) to retire first
-    if (t + 2 < n_tiles) {
-      if (!um_wait(&sm.pv_done, t & 1, &sm.abort_flag, p.status)) return;
-      if (!u2_issue_s(sm, p, tmem, k_desc0, t + 2, sk, pk)) return;
-    }
     if (++sv == kU2Stages) { sv = 0; pv ^= 1u; }
     if (++sk == kU2Stages) { sk = 0; pk ^= 1u; }
   }
@@ -258,12 +255,13 @@ __device__ __forceinline__ bool u2_softmax_tiles(Umma2Smem& sm, const Umma2Param
   const float scale_log2 = p.scale * kU2Log2e;
   for (int t = 0; t < n_tiles; ++t) {
     const int b = t & 1;
-    const uint32_t s_tmem = my_tmem + kU2ColS + b * kU2Keys;
-    if (!um_wait(&sm.s_full[b], (t >> 1) & 1, &sm.abort_flag, p.status)) return false;
+    if (!um_wait(&sm.s_full, t & 1, &sm.abort_flag, p.status)) return false;
     if (t == 0) NVJ_U2_PHASE(3);
     tc_fence_after_sync();
     float s[32];
-    tmem_ld32(s_tmem + half * 32, s);
+    tmem_ld32(my_tmem + kU2ColS + half * 32, s);
+    tc_fence_before_sync();
+    u2_arrive_warp(smem_u32(&sm.s_read));
     const int lim = last_key - (tile0 + t) * kU2Keys - half * 32;
     float hmax = -INFINITY;
     if (lim >= 31) {
@@ -306,13 +304,14 @@ __device__ __forceinline__ bool u2_softmax_tiles(Umma2Smem& sm, const Umma2Param
       hi[e] = *reinterpret_cast<const uint32_t*>(&h);
       lo[e] = *reinterpret_cast<const uint32_t*>(&g);
     }
-    // every phase of pv_done is observed in turn (parity waits tell only two phases apart)
+    // P V of the tile before has read its weights; every phase of pv_done is observed in turn (parity waits tell only two phases
+    // apart)
     if (t >= 1 && !um_wait(&sm.pv_done, (t - 1) & 1, &sm.abort_flag, p.status)) return false;
-    tmem_st16(s_tmem + half * 16, hi);
-    if (p.split_p) tmem_st16(s_tmem + 32 + half * 16, lo);
+    tmem_st16(my_tmem + kU2ColP + half * 16, hi);
+    if (p.split_p) tmem_st16(my_tmem + kU2ColP + 32 + half * 16, lo);
     tmem_st_wait();
     tc_fence_before_sync();
-    mbar_arrive_leader(smem_u32(&sm.p_full));
+    u2_arrive_warp(smem_u32(&sm.p_full));
   }
   return true;
 }
@@ -368,7 +367,7 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
     }
     tmem_st_wait();
     tc_fence_before_sync();
-    mbar_arrive_leader(smem_u32(&sm.q_full));
+    u2_arrive_warp(smem_u32(&sm.q_full));
     NVJ_U2_PHASE(2);
   } else {  // fp32 queries: every thread converts its own row
     const long long qrow = ((long long)(tok0 + token) * kHq + kvh * kG + hl) * kD + half * (kD / 2);
@@ -392,7 +391,7 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
     }
     tmem_st_wait();
     tc_fence_before_sync();
-    mbar_arrive_leader(smem_u32(&sm.q_full));
+    u2_arrive_warp(smem_u32(&sm.q_full));
     NVJ_U2_PHASE(2);
   }
   float m_row = -INFINITY, l_row = 0.f;
@@ -589,16 +588,16 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   // The pair's barriers are set up before anything is read: this runs while the kernel in front (the append of the same
   // tokens, usually) is still at work.
   if (threadIdx.x == 0) {
-    mbar_init(smem_u32(&sm.q_full), 2 * kU2SoftmaxThreads);
+    mbar_init(smem_u32(&sm.q_full), 2 * kU2SoftmaxThreads / 32);
     for (int i = 0; i < kU2Stages; ++i) {
       mbar_init(smem_u32(&sm.k_full[i]), 1);
       mbar_init(smem_u32(&sm.v_full[i]), 1);
       mbar_init(smem_u32(&sm.k_empty[i]), 1);
       mbar_init(smem_u32(&sm.v_empty[i]), 1);
     }
-    mbar_init(smem_u32(&sm.s_full[0]), 1);
-    mbar_init(smem_u32(&sm.s_full[1]), 1);
-    mbar_init(smem_u32(&sm.p_full), 2 * kU2SoftmaxThreads);
+    mbar_init(smem_u32(&sm.s_full), 1);
+    mbar_init(smem_u32(&sm.s_read), 2 * kU2SoftmaxThreads / 32);
+    mbar_init(smem_u32(&sm.p_full), 2 * kU2SoftmaxThreads / 32);
     mbar_init(smem_u32(&sm.pv_done), 1);
     mbar_init(smem_u32(&sm.x_full), kU2SoftmaxThreads);
     mbar_fence_init();
@@ -712,22 +711,6 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   if (warp == 1) tmem2_dealloc(tmem, kU2TmemCols);
 }
 
-typedef CUresult (*U2EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static U2EncodeTiledFn u2_encode_fn() {
-  static U2EncodeTiledFn fn = [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult res;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &res) != cudaSuccess ||
-        res != cudaDriverEntryPointSuccess)
-      ptr = nullptr;
-    return reinterpret_cast<U2EncodeTiledFn>(ptr);
-  }();
-  return fn;
-}
-
 static int u2_pair_slots() {  // CTA pairs that run at once: half the SMs of the current device
   static PerDeviceFlags slots;
   const int dev = current_device();
@@ -740,16 +723,6 @@ static int u2_pair_slots() {  // CTA pairs that run at once: half the SMs of the
     slots.v[dev].store(n, std::memory_order_release);
   }
   return n;
-}
-
-static bool u2_make_map(CUtensorMap* map, const void* base, uint64_t outer) {
-  const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)kHkv, outer};
-  const cuuint64_t strides[2] = {(cuuint64_t)kRowBytes, (cuuint64_t)kRowBytes * kHkv};
-  const cuuint32_t box[3] = {64, 1, (cuuint32_t)kBlk};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return u2_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 constexpr int kU2SmemBytes = (int)sizeof(Umma2Smem) + 1024;
@@ -799,7 +772,7 @@ static int u2_clusters_at_once(int splits) {
 }
 
 // Whether launch_prefill_umma2 will take a batch with these parameters (a caller that knows so need not zero the output).
-bool prefill_umma2_usable(float scale, long long num_blocks) { return scale > 0.f && num_blocks >= 1 && u2_encode_fn() != nullptr; }
+bool prefill_umma2_usable(float scale, long long num_blocks) { return scale > 0.f && num_blocks >= 1 && tensor_maps_available(); }
 
 // Returns NVJ_ERR_UNSUPPORTED when the driver offers no tensor-map encoder or the scale is not positive.
 int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const char* v_cache,
@@ -808,14 +781,14 @@ int launch_prefill_umma2(const void* q, int q_dtype, const char* k_cache, const 
                          int rows, int token_bucket, float scale, float* out, int32_t* status,
                          int skip_single, int split_p, int tile_pairs, bool may_split, int32_t* beside, cudaStream_t stream) {
   static PerDeviceFlags opted_in;
-  if (!(scale > 0.f) || num_blocks < 1 || !u2_encode_fn()) return NVJ_ERR_UNSUPPORTED;
+  if (!(scale > 0.f) || num_blocks < 1 || !tensor_maps_available()) return NVJ_ERR_UNSUPPORTED;
   if (!once_per_device(opted_in, [](int) {
         return cudaFuncSetAttribute(prefill_umma2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kU2SmemBytes) == cudaSuccess;
       }))
     return NVJ_ERR_LAUNCH;
   CUtensorMap k_map, v_map;
-  if (!tensor_map_cached(&k_map, 2, k_cache, (uint64_t)num_blocks * kBlk, u2_make_map) ||
-      !tensor_map_cached(&v_map, 2, v_cache, (uint64_t)num_blocks * kBlk, u2_make_map))
+  if (!grouped_map_cached(&k_map, k_cache, (uint64_t)num_blocks * kBlk, 4) ||
+      !grouped_map_cached(&v_map, v_cache, (uint64_t)num_blocks * kBlk, 2))
     return NVJ_ERR_UNSUPPORTED;
   // The kernel zeroes what no tile writes itself (padding tokens, rows of several tokens without keys), and the
   // decode-row pass of a mixed batch does the same for its rows: no memset launch in front of a batch.

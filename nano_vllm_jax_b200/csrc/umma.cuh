@@ -171,5 +171,10 @@ bool tensor_map_cached(CUtensorMap* map, int kind, const void* base, uint64_t ex
 // A bf16 cache layer of `tokens` tokens as {64 dims, token, 64-dim chunk, kv head}: a box is one 16-token block of both KV heads and
 // lands as [kv head][chunk][16 tokens][128 B] with the 128-byte swizzle.
 bool block_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t tokens);
+// The layer with its tokens in groups of eight, {64 dims, token of the group, 64-dim chunk, group, kv head}: a box is `chunks` (2 or 4)
+// chunks of one KV head's half of a block and lands as [group][chunk][8 tokens][128 B], so that the groups of a tile of several
+// blocks are evenly spaced, as the rows of one operand have to be, whatever its number of blocks.
+bool grouped_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t tokens, int chunks);
+bool tensor_maps_available();  // the driver has an encoder
 
 }  // namespace nvj
