@@ -89,7 +89,7 @@ struct Umma2Smem {
   alignas(1024) char v[kU2Stages][4][4096];  // [stage][block][8-key group][this CTA's two 64-d chunks][8 keys][128 B]
   // used in CTA 0 only: q_full, k_full, v_full, s_read, p_full; used in both: the rest
   alignas(8) unsigned long long q_full, k_full[kU2Stages], v_full[kU2Stages], k_empty[kU2Stages], v_empty[kU2Stages],
-      s_full, s_read, p_full, pv_done, x_full;
+      s_full, s_read, p_full, pv_done, x_full[4];  // x_full: per quarter of the rows, whose two warps share them
   float xchg[2][2][kU2Rows];
   // this CTA's query rows on their way into tensor memory: [token][head of the group][32 pieces of 16 B], the pieces
   // of token t stored at (piece ^ (t & 7)) so that both the row-wise fill and the token-wise read are conflict-free
@@ -272,8 +272,9 @@ __device__ __forceinline__ bool u2_softmax_tiles(Umma2Smem& sm, const Umma2Param
       for (int i = 0; i < 32; ++i) { s[i] = i <= lim ? s[i] : -INFINITY; hmax = fmaxf(hmax, s[i]); }
     }
     sm.xchg[b][half][r] = hmax;
-    mbar_arrive(smem_u32(&sm.x_full));
-    if (!um_wait(&sm.x_full, t & 1, &sm.abort_flag, p.status)) return false;
+    __syncwarp();
+    if ((r & 31) == 0) mbar_arrive(smem_u32(&sm.x_full[r >> 5]));
+    if (!um_wait(&sm.x_full[r >> 5], t & 1, &sm.abort_flag, p.status)) return false;
     const float tmax = fmaxf(hmax, sm.xchg[b][half ^ 1][r]) * scale_log2;  // scale > 0
     if (t == 0) {
       m_row = tmax;
@@ -295,15 +296,21 @@ __device__ __forceinline__ bool u2_softmax_tiles(Umma2Smem& sm, const Umma2Param
     }
     const float neg_m = m_row == -INFINITY ? 0.f : -m_row;
     uint32_t hi[16], lo[16];
+    const float2 c2 = make_float2(scale_log2, scale_log2), m2 = make_float2(neg_m, neg_m);
+    float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const float p0 = ex2_approx(fmaf(s[2 * e], scale_log2, neg_m)), p1 = ex2_approx(fmaf(s[2 * e + 1], scale_log2, neg_m));
-      l_row += p0 + p1;
-      const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-      const __nv_bfloat162 g = __floats2bfloat162_rn(p0 - __low2float(h), p1 - __high2float(h));
+    for (int e = 0; e < 16; ++e) {  // two keys at a time, packed fp32 arithmetic
+      float2 w = fma2(make_float2(s[2 * e], s[2 * e + 1]), c2, m2);
+      w.x = ex2_approx(w.x);
+      w.y = ex2_approx(w.y);
+      sum = __fadd2_rn(sum, w);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(w.x, w.y);
+      const float2 rest = fma2(make_float2(__low2float(h), __high2float(h)), make_float2(-1.f, -1.f), w);  // exact
+      const __nv_bfloat162 g = __floats2bfloat162_rn(rest.x, rest.y);
       hi[e] = *reinterpret_cast<const uint32_t*>(&h);
       lo[e] = *reinterpret_cast<const uint32_t*>(&g);
     }
+    l_row += sum.x + sum.y;
     // P V of the tile before has read its weights; every phase of pv_done is observed in turn (parity waits tell only two phases
     // apart)
     if (t >= 1 && !um_wait(&sm.pv_done, (t - 1) & 1, &sm.abort_flag, p.status)) return false;
@@ -401,8 +408,9 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
   NVJ_U2_PHASE(4);
   if (alive) {
     sm.xchg[n_tiles & 1][half][r] = l_row;
-    mbar_arrive(smem_u32(&sm.x_full));
-    alive = um_wait(&sm.x_full, n_tiles & 1, &sm.abort_flag, p.status);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sm.x_full[quarter]));
+    alive = um_wait(&sm.x_full[quarter], n_tiles & 1, &sm.abort_flag, p.status);
   }
   if (alive) {
     l_row += sm.xchg[n_tiles & 1][half ^ 1][r];
@@ -599,7 +607,7 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     mbar_init(smem_u32(&sm.s_read), 2 * kU2SoftmaxThreads / 32);
     mbar_init(smem_u32(&sm.p_full), 2 * kU2SoftmaxThreads / 32);
     mbar_init(smem_u32(&sm.pv_done), 1);
-    mbar_init(smem_u32(&sm.x_full), kU2SoftmaxThreads);
+    for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&sm.x_full[i]), 2);
     mbar_fence_init();
   }
   cl_sync();  // the peer's barriers exist before anything is sent to them (this barrier covers the CTA's own threads)
