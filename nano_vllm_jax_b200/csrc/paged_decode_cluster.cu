@@ -12,9 +12,9 @@
 //     of fences and counters; rank r writes its 1 / C of the output;
 //   * fused append: the cluster's first warp stores the new row, and whoever attends its key reads it from the operand.
 // Nothing waits on memory that somebody else must fill, so there is no wait to bound.
-// Measured (us per launch, K/V cold, lengths spread over [n / 4, n]; before: the streaming kernel): 4 rows of n = 512 tokens
-// 12.2 -> 5.3, 8 of 4096 19.9 -> 13.7, 48 of 1024 21.8 -> 16.6, 256 of 512 41.4 -> 39.1, 256 of 2048 113 -> 112.  f32: 8 rows of
-// 64 - 512 tokens 221 (the generic kernel) -> 10.5.
+// Measured (us per launch, K/V cold, lengths spread over [n / 4, n]; the streaming kernel : this one): 4 rows of n = 512 tokens
+// 10.6 : 5.5, 8 of 4096 19.1 : 13.2, 48 of 1024 19.1 : 16.5, 256 of 2048 108 : 106, 256 of 4096 204 : 200 (a first build, whose every
+// copy selected its row, took 8% more).  f32: 8 rows of 64 - 512 tokens 221 (the generic kernel) : 7.4.
 // Semantics: nanovllm_jax/kv_cache.py:852-998 for width-1 queries, nanovllm_jax/kernels/full_attention_triton.py:373-485
 // for the fused append.
 
@@ -677,16 +677,18 @@ static ClusterForm cluster_form(int batch, int blocks, int sms, int room, int pe
   return f;
 }
 
-// Whether this kernel, launched as cluster_form() says, beats the streaming kernel (paged_decode_wide.cu) on a bf16 batch.
-// While CTAs have an SM each: the streaming kernel costs ~12.5 us whatever the batch plus its bytes at the HBM rate, this one
-// ~4.5 us plus ~1.25 us per block of the longest warp.  Beyond that, where the streaming kernel's equal shares win once a CTA's
+// Whether this kernel, launched as cluster_form() says, beats the streaming kernel (paged_decode_stream.cu) on a bf16 batch.
+// While CTAs have an SM each: the streaming kernel costs ~11 us whatever the batch plus its bytes at the HBM rate, this one
+// ~4.5 us plus ~1.1 us per block of the longest warp.  Beyond that, where the streaming kernel's equal shares win once a CTA's
 // own work gets long, by the blocks of a walker, and with an eye on rows much shorter than the table (a server that pads its
-// tables), for which a CTA without a block is pure cost.  Measured at 48 - 512 rows and 32 - 512 blocks, rows of 1/4 - 1
-// and of 1/32 - 1/8 of the table, in the tables of cluster_form and here (us, clusters : streaming):
-//   eight CTAs per row and head that fill the places more than twice: 67 rows under 384 blocks 88 : 90 and 25 : 22;
-//   160 rows under 192, eight per row: 105 : 106 and 32 : 27;
-//   places filled between once and 5/3 times, 24 blocks per walker: 160 rows under 192, four per row: 110 : 106 and 23 : 27;
-//   at 16 per walker: 160 under 128 75 : 76 and 19 : 23, 128 under 192 (six) 87 : 87 and 21 : 24.
+// tables), for which a CTA without a block is pure cost.  Measured at 2 - 512 rows and 24 - 512 blocks, rows of 1/4 - 1
+// and of 1/32 - 1/8 of the table (us, clusters : streaming):
+//   eight CTAs and more per row and head that all find a place, 16 blocks per walker: 16 rows under 512 blocks 33.3 : 35.2 and
+//   10.0 : 13.4, 24 under 512 45.8 : 47.7 and 11.2 : 14.4; that do not, 32 under 400 47.8 : 48.1 and 15.7 : 14.6;
+//   eight CTAs per row and head that fill the places more than twice: 67 rows under 320 71.0 : 73.4 and 22.2 : 19.0;
+//   160 rows under 200, eight per row: 103.9 : 105.4 and 31.5 : 23.1; under 160, four per row, which fill the places between once
+//   and 5/3 times with 20 blocks per walker: 87.6 : 89.3 and 21.5 : 21.3; with 16, under 128, 71.4 : 72.2 and 19.2 : 20.0;
+//   256 rows under 256 200.0 : 204.5 and 41.0 : 35.2, under 128 106.4 : 108.2 and 27.4 : 24.5.
 bool decode_cluster_pays(int batch, int table_width) {
   const int sms = decode_wide_num_ctas();
   if (sms <= 0 || batch > kClMaxRows) return false;
@@ -695,7 +697,7 @@ bool decode_cluster_pays(int batch, int table_width) {
   const int per_walker = f.per_walker(table_width);
   if (total < sms) return 1.25 * per_walker <= 9.5 + 0.0026 * batch * table_width;  // 32 KiB per block, half of the widest on average, 6.3 TB/s
   if (f.ctas == 8 && total > 6LL * sms) return false;
-  if (!f.both) return per_walker <= 12;
+  if (!f.both) return per_walker <= (f.ctas >= 8 && 100 * total <= (long long)kCmPerSm * sms ? 16 : 12);
   if (total > 3LL * sms && total < 5LL * sms) return per_walker <= 16;
   return per_walker <= (f.ctas == 6 ? 32 : 24);
 }
@@ -724,9 +726,9 @@ int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
   ClusterForm form = cluster_form(p.batch, blocks, sms, sms, kCmPerSm);
   if (p.beside && p.cta_limit > 0 && (form.both || form.ctas < 8)) form = cluster_form(p.batch, blocks, sms, p.cta_limit, 300);
   // The CUDA-core form: eight warps, a quarter block each, two CTAs per SM (1.8: clusters do not find every SM).  More than four
-  // CTAs per row and head by the table's width alone only where eight fill the places at most twice (37 rows): f32, 32 rows under
-  // 512 blocks 243 us with eight and 265 with four (rows of 1/4 - 1 of the table), 44 and 40 (1/32 - 1/8); 256 rows 1482 and 1447,
-  // 272 and 216; 512 rows of 16 - 128 keys 252 and 127 (the generic kernel 115).
+  // CTAs per row and head by the table's width alone only where eight fill the places at most twice (37 rows): f32, 32 rows of
+  // 2000 - 8000 keys 111 us with eight and 116 with four, of 256 - 1024 under a table of 8192 23.9 and 21.2; 128 rows of 512 - 2048
+  // 115 and 109, of 256 - 1024 under 8192 77 and 63; 256 rows of 512 - 2048 223 and 203.
   const int wide = cluster_size(2LL * p.batch, blocks, sms, kClWarps * kClUnit / kBlk, 180, 16LL * p.batch <= 4LL * sms ? 8 : 4, 8);
   static PerDeviceFlags flags[8];
   const int smem = (int)sizeof(CmSmem);

@@ -11,8 +11,8 @@
 //     group are half of the N = 8 columns and the weights as hi + lo fill them: 32 mma.sync and 32 ldmatrix per block and head.
 //     (The untransposed form that rows of several tokens use spends 128 and 48 on it: four of its sixteen tile rows are real, and
 //     two warps repeat each block's scores.)
-//   * A ninth warp feeds the ring: it walks the rows, holds the block ids of the next 32 blocks (and asks for the 32 behind them,
-//     and for the next row's, in advance) and waits for a slot to be given back.  Nobody else waits for anything but its own
+//   * A ninth warp feeds the ring: it walks the rows, holds the block ids of the next 32 blocks (and asks for the 32 behind them
+//     and for the next row's in advance) and waits for a slot to be given back.  Nobody else waits for anything but its own
 //     copies, except at the end of a row, where the walkers' sums meet in shared memory.
 // The split over CTAs, the partials and their fold are the CUDA-core kernel's (decode_parts.cuh).
 // Measured (us per launch, back to back; before: the untransposed form): 128 rows of 8192 - 32768 keys 906 -> 775 once the board
@@ -46,7 +46,7 @@ constexpr int kStThreads = kDecodeThreads + 128;
 constexpr int kStConsumerRegs = 240, kStProducerRegs = 24;
 static_assert(kDecodeThreads * kStConsumerRegs + 128 * kStProducerRegs <= kStThreads * 168, "more registers than the launch has");
 constexpr int kStPitch = kD + 4;  // floats between the heads of a warp's sums: conflict-free stores
-constexpr int kStRowEndCost = 6;  // blocks that a row end costs a CTA (decode_parts.cuh)
+constexpr int kStRowEndCost = 9;  // blocks that a row end costs a CTA (decode_parts.cuh): 32 rows of 512 - 4096 keys 34.1 us with 1, 33.3 with 6, 32.5 with 9
 
 struct StreamSmem {
   alignas(1024) char tiles[kStWalkers][kStSlots][kTileBytes];
@@ -83,8 +83,8 @@ __device__ __forceinline__ void st_producer(const CUtensorMap* k_map, const CUte
   bool have = next_seg<kWindow>(p, b, j, g, g1, s);
   int ids = have ? ids_at(s, s.j0) : -1;
   while (have) {
-    const bool more = next_seg<kWindow>(p, b, j, g, g1, nxt);
-    const int next_first = more ? ids_at(nxt, nxt.j0) : -1;
+    bool more = false;
+    int next_first = -1;
     for (int jb = s.j0; jb < s.j1; jb += 32) {
       const int ahead = ids_at(s, jb + 32);
       const int n = s.j1 - jb < 32 ? s.j1 - jb : 32;
@@ -117,6 +117,10 @@ __device__ __forceinline__ void st_producer(const CUtensorMap* k_map, const CUte
         if (++wk == kStWalkers) { wk = 0; at = c; reuse = again; }
       }
       ids = ahead;
+      if (jb == s.j0) {  // the row behind this one, once the first copies are on their way
+        more = next_seg<kWindow>(p, b, j, g, g1, nxt);
+        if (more) next_first = ids_at(nxt, nxt.j0);
+      }
     }
     s = nxt;
     ids = next_first;

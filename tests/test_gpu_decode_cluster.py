@@ -118,3 +118,19 @@ def test_short_rows_under_a_wide_table_on_the_cuda_cores(rows, width, cache, que
     ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
     got = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE)
     assert float((got - ref).abs().max()) <= TIGHT[cache]
+
+
+# eight CTAs and more per row and head, all resident: up to 16 blocks per walker; 32 rows' eight are not
+@pytest.mark.parametrize("rows,width,pays", [(16, 512, True), (24, 512, True), (24, 520, False), (32, 400, False), (8, 2048, False)])
+def test_few_rows_of_many_blocks(rows, width, pays):
+    from nano_vllm_jax_b200 import _lib
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert bool(_lib.load().nvj_paged_decode_on_clusters(rows, width)) == pays
+    if rows * width > 8192:
+        return
+    lens = [1 + (1037 * i) % (width * BS) for i in range(rows - 1)] + [width * BS]
+    k, v, tables, lens, c = _case(rows, lens, width, torch.bfloat16)
+    q = to_torch(c["q"][:, 0]).contiguous()
+    ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
+    assert float((K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE) - ref).abs().max()) <= 2e-3
