@@ -286,8 +286,10 @@ bool decode_cluster_wide_pays(const DecodeParams& p) {
   const int sms = decode_wide_num_ctas();
   if (!cw_takes(p) || sms <= 0) return false;
   const int c = cw_cluster(p, sms), per_cta = (p.table_width + c - 1) / c;
+  const long long ctas = (long long)c * p.batch;
   if (p.batch >= 100 && p.table_width <= (p.width == 2 ? 25 : 16)) return true;
-  return per_cta <= (p.width == 2 ? 12 : 7) && 100LL * c * p.batch <= (long long)kCmPerSm * sms;
+  if (p.width > 2 && per_cta == 8) return ctas <= sms;  // 0 - 2 us slower than tcgen05 there, at half its error against 64 bits
+  return per_cta <= (p.width == 2 ? 12 : 7) && 100 * ctas <= (long long)kCmPerSm * sms;
 }
 
 // Rows of 2 - 4 bf16 query tokens over a dense table, already appended.

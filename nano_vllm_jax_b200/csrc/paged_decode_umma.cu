@@ -56,7 +56,7 @@ constexpr int kUdColO = 256;      // output accumulator: columns [256, 512)
 constexpr int kUdHalfBlock = kBlk * kD * 2;  // K (or V) of one KV head of one block: 8 KiB
 constexpr float kUdRescaleGap = 8.f;
 constexpr int kUdMaxWidth = 16;  // 64 query rows per KV head: two softmax warps
-constexpr int kUdRowEndCost = 9;  // what a row end costs a CTA here, in blocks (128 rows of 5 tokens: 125.7 us with 3, 125.0 with 6, 124.5 with 9)
+constexpr int kUdRowEndCost = 6;  // what a row end costs a CTA here, in blocks (128 rows of 5 tokens: 125.7 us with 3, 125.0 with 6, 124.5 with 9)
 
 struct UdSmem {
   alignas(1024) char k[kUdStages][kUdTileBlocks][kUdHalfBlock];    // [stage][block][8-key group][64-d chunk][8 keys][128 B], swizzled

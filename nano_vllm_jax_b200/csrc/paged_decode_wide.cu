@@ -500,10 +500,13 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
   if (n <= 0) return NVJ_ERR_LAUNCH;
   if (p.wide_form == 3 || (p.wide_form == 0 && p.cta_limit <= 0 && decode_cluster_wide_pays(p)))
     return launch_decode_cluster_wide(p, stream);
-  // The tcgen05 form for rows of 3 and more query tokens (mma.sync : tcgen05, us, 3 tokens over 1024 - 4096 keys: 64 rows 68.6 : 63.8, 192
-  // rows 184 : 172; 4 tokens: 64 rows 70.5 : 65.3, 192 rows 220 : 176, at the board's power limit; it ends at 8 tokens).  With 2
-  // they meet at about 32768 blocks: 64 rows 64.6 : 63.5, 128 rows 114.1 : 113.6, 192 rows 163 : 170.
-  if (p.wide_form == 2 || (p.wide_form == 0 && (p.width > 2 || (p.width == 2 && (long long)p.batch * p.table_width <= 32768)))) {
+  // Rows of 5 and more query tokens: the tcgen05 form (the mma.sync form is compute-bound there and ends at 8 tokens).  Below
+  // that the tcgen05 form is the faster one up to 32768 blocks with 2 tokens and always with 3 and 4 (mma.sync : tcgen05, us, 4 tokens over
+  // 1024 - 4096 keys: 64 rows 70.5 : 65.3, 192 rows 220 : 176), but it carries one sum in tensor memory over all keys of a row's
+  // part, where the mma.sync form has eight short ones: against 64 bits 64 rows of 2 tokens are off by 4.4e-6 of their size with
+  // it, 2.4e-6 without.  So it serves the smaller batches alone, where it wins most (16 rows of 512 - 2048 keys 20.9 : 29.7).
+  const long long blocks = (long long)p.batch * p.table_width;
+  if (p.wide_form == 2 || (p.wide_form == 0 && p.width > 1 && (p.width > 4 || blocks <= (p.width == 2 ? 4096 : 12288)))) {
     const int rc = launch_decode_umma(p, stream);
     if (rc != NVJ_ERR_UNSUPPORTED || p.wide_form == 2) return rc;
   }
