@@ -301,10 +301,11 @@ int nvj_paged_decode_static_scratch(const void* q, int q_dtype,
 size_t nvj_paged_decode_wide_workspace_bytes(int max_batch);
 /*
  * nvj_paged_decode_wide_form: the same call with the kernel chosen by the caller.  form 0 = automatic (what
- * nvj_paged_decode_wide does: widths 1-4 on mma.sync tiles, 16 query rows per warp; widths 5-8 on tcgen05, the 4 x width
+ * nvj_paged_decode_wide does: width 1 on the streaming decode kernel; few or short rows of 2-4 tokens in thread-block
+ * clusters, else on tcgen05 while the batch is small and on mma.sync tiles beyond; widths 5-16 on tcgen05, the 4 x width
  * query rows of a KV head in a 128-row tile with scores and output in tensor memory, a row cut over several CTA pairs
- * folded by a second small launch), 1 = mma.sync tiles (widths 5-8: two row tiles per warp pair, ~1.9x the width-1
- * time; NVJ_ERR_UNSUPPORTED beyond 8), 2 = tcgen05 at any width 1-16 (NVJ_ERR_UNSUPPORTED without a tensor-map
+ * folded by a second small launch), 1 = mma.sync tiles (widths 5-8: two row tiles per warp pair, ~1.9x the time of one
+ * token per row; NVJ_ERR_UNSUPPORTED beyond 8), 2 = tcgen05 at any width 1-16 (NVJ_ERR_UNSUPPORTED without a tensor-map
  * encoder or for scale <= 0).
  */
 int nvj_paged_decode_wide_form(const void* q, const void* k_cache_layer, const void* v_cache_layer,
@@ -383,8 +384,8 @@ int nvj_paged_prefill_packed(const void* q, int q_dtype,
  *   part 1   rows that hold exactly one query token, on the streaming decode kernel with at most `cta_limit` CTAs
  *            (0 = one per SM; give the SM count minus the CTAs of part 2); `workspace` is required
  *   part 2   every other row, on the CTA-pair tile kernel (variant 0, 4 or 5; NVJ_ERR_UNSUPPORTED for another variant,
- *            or when that kernel cannot run: call nvj_paged_prefill_packed instead); `workspace` (nullable, NOT the
- *            buffer part 1 is using at the same time) only gives the key-range splits of a short batch their room
+ *            or when that kernel cannot run: call nvj_paged_prefill_packed instead); `workspace` (nullable) is
+ *            not used
  *   part 3   all rows on the tile kernel, which then zeroes what it does not write itself (no zeroed `out` needed):
  *            a batch without decode rows that still wants the key-range splits
  * The reference runs a mixed batch through one packed attention call; the split has no counterpart there.

@@ -46,7 +46,7 @@ struct DecodeParams {
   // writes out[i] and attends min(seq_lens[b], query_positions[i] + 1) keys.  Other rows are left
   // alone (no zero fill): the prefill kernel owns them.
   int packed_rows;
-  // query tokens per row of the wide kernel (2..4; 0 elsewhere): q is [batch, width, heads, dim], out
+  // query tokens per row of the wide kernels (2..16; 0 elsewhere): q is [batch, width, heads, dim], out
   // [batch, width, heads * dim], positions (nullable) [batch, width]
   int width;
   // upper bound on the CTAs of the streaming kernels (0: one, or two, per SM): a caller that runs another kernel
@@ -63,7 +63,7 @@ struct DecodeParams {
   int32_t* pick_tokens;
   int32_t* pick_lens;       // the rows' lengths: seq_lens, writable
   int32_t* pick_positions;  // nullable
-  // which wide kernel serves rows of several query tokens: 0 = automatic (mma.sync tiles up to width 4, tcgen05 beyond),
+  // which wide kernel serves rows of several query tokens: 0 = automatic (launch_decode_wide),
   // 1 = mma.sync tiles, 2 = tcgen05, 3 = thread-block clusters
   int wide_form;
   // what a row end costs a CTA, in blocks (decode_parts.cuh); set by the launchers, the same for every kernel of a call
@@ -184,7 +184,7 @@ bool decode_cluster_pays(int batch, int table_width);  // a bf16 batch is short 
 bool decode_cluster_picks(const DecodeParams& p);      // its launch for this call would serve pick_tokens too
 int launch_decode_pipelined(const DecodeParams& p, int num_ctas, cudaStream_t stream);
 int decode_wide_num_ctas();  // 1 per SM of the current device
-int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // tensor-core streaming kernels, width 1..8
+int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // rows of 1 - 16 tokens: picks the form
 int launch_decode_stream(const DecodeParams& p, cudaStream_t stream);  // one query token per row, bf16
 int launch_decode_cluster_wide(const DecodeParams& p, cudaStream_t stream);  // rows of 2 - 4 tokens, few and short
 bool decode_cluster_wide_pays(const DecodeParams& p);

@@ -625,7 +625,7 @@ bool grouped_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t toke
 }
 bool tensor_maps_available() { return ud_encode_fn() != nullptr; }
 
-// p as launch_decode_wide takes it (width 1..8, carved workspace whose partial area holds ws_slots(decode_wide_num_ctas())
+// p as launch_decode_wide takes it (width 2..16, carved workspace whose partial area holds ws_slots(decode_wide_num_ctas())
 // slots of width * kHq rows).  NVJ_ERR_UNSUPPORTED: no tensor-map encoder, a scale that is not positive (row maxima are
 // taken before scaling), the packed or the appending form.
 int launch_decode_umma(const DecodeParams& p, cudaStream_t stream) {

@@ -1,11 +1,9 @@
-// Paged GQA decode attention with the products on tensor-core tiles, for rows of 1..8 query tokens:
-// the decode step proper (width 1, with the optional fused append of the step's new K/V row) and
-// the verification of speculated tokens / multi-token prediction (width 2..8).  Cache shape of the
-// model's full-attention layer: bf16, 16-token blocks, 2 KV heads x 4 query heads, head_dim 256.
+// Paged GQA decode attention with the products on tensor-core tiles, for rows of 2..8 query tokens: the
+// verification of speculated tokens / multi-token prediction.  (One token per row: paged_decode_stream.cu.)  Cache
+// shape of the model's full-attention layer: bf16, 16-token blocks, 2 KV heads x 4 query heads, head_dim 256.
 //
 // The kernel is HBM-bound: every K/V byte is read from HBM exactly once.  On the CUDA cores the dot
-// products take half of the issue slots at width 1 and would make the kernel compute-bound beyond
-// it, so the scores and the weighted sums run on the tensor cores (mma.sync m16n8k16, bf16 in, fp32
+// products would make it compute-bound, so the scores and the weighted sums run on the tensor cores (mma.sync m16n8k16, bf16 in, fp32
 // accumulate): the width * 4 query rows of one KV head fill one 16-row tile.  Around the arithmetic
 // the scheme is the CUDA-core kernel's (paged_decode.cu, decode_parts.cuh): all blocks of all
 // rows form one sequence cut into equal ranges, one per CTA (one CTA per SM here, the accumulators
@@ -27,12 +25,10 @@
 //     ROWS: both read every staged block, one for tokens 0..3, the other for tokens 4..7, and
 //     nothing is merged between them.  K/V still cross HBM once; the tensor work per block doubles
 //     and every warp now walks every block, which makes this form bound by a warp's chain of dependent
-//     tile products (width 8 takes ~1.9x the width-1 time; entering the softmax weights as one bf16
+//     tile products (width 8 takes ~1.9x the time of one token per row; entering the softmax weights as one bf16
 //     term instead of two was measured: 11% faster at 4e-3 instead of 2e-3 error, not taken).
 // Semantics: nanovllm_jax/kv_cache.py:852-998 (key p of row b is visible to token t when
-// p < seq_lens[b] and, at width > 1 with positions given, p <= positions[b, t]); the fused append
-// follows nanovllm_jax/kernels/full_attention_triton.py:373-485 (positions are then the slots the
-// new rows go to).
+// p < seq_lens[b] and, with positions given, p <= positions[b, t]).
 
 #include <cuda.h>
 
@@ -491,7 +487,7 @@ int decode_wide_num_ctas() {  // one per SM of the current device
 static size_t wide_ml_bytes(int n, int width) { return ws_round(sizeof(float) * ws_slots(n) * width * kHq * 2); }
 static size_t wide_acc_bytes(int n, int width) { return ws_round(sizeof(float) * ws_slots(n) * width * kHq * kD); }
 
-// p carries everything but the tensor maps: pointers, shapes, width (1..4) and the carved workspace, whose
+// p carries everything but the tensor maps: pointers, shapes, width and the carved workspace, whose
 // partial area holds ws_slots(decode_wide_num_ctas()) slots of width * kHq rows.
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
   if (p.width < 1 || p.width > kWideMaxWidth || p.num_blocks < 1 || p.num_blocks * kBlk > 0x7fffffffLL || !w_encode_fn())
