@@ -57,7 +57,7 @@ DECODE_KERNELS = {
     True: dict(name="decode_cluster_mma_kernel (fused append + paged GQA decode on thread-block clusters, tensor-core tiles)",
                dram=1351.09e6, algorithmic=1346.54e6, capture="256 rows of 1024 - 4096 tokens"),
     False: dict(name="decode_stream_kernel (fused append + paged GQA decode, TMA-staged, tensor-core tiles)",
-                dram=354.93e6, algorithmic=356.35e6, capture="--workload c2small on that kernel"),
+                dram=354.09e6, algorithmic=349.20e6, capture="64 rows of 1024 - 4096 tokens, no append"),
 }
 
 WORKLOADS = {

@@ -53,3 +53,19 @@ def test_a_bad_index_leaves_the_other_rows_right():
     want = torch.zeros_like(p)
     want[5], want[4] = t[0], t[3]
     assert torch.equal(p, want)
+
+
+def test_copies_that_follow_one_another_see_each_other():
+    """Every copy reads what the one in front of it in the stream has written, with nothing in between to wait for."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    table, pool = torch.randn(4, 40_000, device="cuda", generator=g), torch.zeros(4, 40_000, device="cuda")
+    k = torch.randn(2, 12, 16, 2, 256, device="cuda", generator=g).bfloat16()
+    v = torch.randn(2, 12, 16, 2, 256, device="cuda", generator=g).bfloat16()
+    first, k0, v0 = table[0].clone(), k[:, 0].clone(), v[:, 0].clone()
+    pairs = [torch.tensor([[i], [i + 1]], dtype=torch.int32, device="cuda") for i in range(11)]
+    for i in range(11):  # row 0 -> pool row 0 -> table row 1 -> ..., block 0 -> block 1 -> ...
+        paged_kv.hybrid_copy(None, table, None, pool, [i % 4], [i % 4], restore=False)
+        paged_kv.hybrid_copy(None, table, None, pool, [(i + 1) % 4], [i % 4], restore=True)
+        paged_kv.copy_blocks(k, v, *pairs[i])
+    assert all(torch.equal(x, first) for x in (*table, *pool))
+    assert all(torch.equal(k[:, i], k0) and torch.equal(v[:, i], v0) for i in range(12))
