@@ -144,14 +144,14 @@ def test_token_pick_with_advance_is_pick_plus_advance():
 
 
 # rows x table width in blocks pick the launch: 1 CTA per row and head (a cluster of both heads), 8, 16 (too many for one cluster: a
-# second launch picks), 5, then 1, 2 and 4 CTAs per row for both heads, and the streaming kernel
-@pytest.mark.parametrize("rows,width", [(3, 4), (3, 32), (3, 80), (40, 24), (150, 6), (200, 30), (70, 100), (20, 420)])
+# second launch picks), 5, then 1, 2 and 4 CTAs per row for both heads, 10 per head (a second launch), and the streaming kernel
+@pytest.mark.parametrize("rows,width", [(3, 4), (3, 32), (3, 80), (40, 24), (150, 6), (200, 30), (70, 100), (20, 420), (20, 700)])
 def test_a_step_in_one_call_equals_attention_then_token_pick(rows, width):
     from nano_vllm_jax_b200.kernels import paged_kv as K
     c = decode_case(rows + width, 4000, rows, 1, 1, width=width)
     rng = np.random.default_rng(rows * width)
     span = width * BS
-    lens = np.array([[0, 1, BS, span - 1, min(span - 1, 37)][b % 5] if b != 1 else 1 + b for b in range(rows)], np.int32)
+    lens = np.array([[0, 2, BS, span - 1, min(span - 1, 37)][b % 5] for b in range(rows)], np.int32)
     tables = to_torch(rng.integers(0, 3000, size=(rows, width)).astype(np.int32))
     last = 3000 + np.arange(rows)  # the block that takes a row's token is the row's own
     for b, n in enumerate(lens):
@@ -165,8 +165,8 @@ def test_a_step_in_one_call_equals_attention_then_token_pick(rows, width):
     want = K.row_argmax(ref.view(rows, -1), advance=(lens_a, pos_a, width, BS))
     tokens = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
     got = K.paged_decode_step(q, nk, nv, k_b, v_b, tables, lens_b, pos_b, 0, BS, SCALE, 4, tokens)
-    # the same kernel where a row's clusters have the same size: 16 CTAs per head become 8 only without the token pick's limit
-    assert torch.equal(got, ref)
+    assert bool(K._lib.load().nvj_paged_decode_on_clusters(rows, width)) == (width < 700)
+    assert torch.equal(got, ref)  # (the token pick changes neither the kernel nor the size of a row's cluster)
     assert torch.equal(tokens, want) and torch.equal(lens_a, lens_b) and torch.equal(pos_a, pos_b)
     assert torch.equal(k_a.view(torch.uint8), k_b.view(torch.uint8)) and torch.equal(v_a.view(torch.uint8), v_b.view(torch.uint8))
 
