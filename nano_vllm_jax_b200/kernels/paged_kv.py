@@ -892,15 +892,16 @@ def hybrid_copy(conv_table, rec_table, conv_pool, rec_pool, table_slots, pool_sl
 
 
 def _advance_args(advance, rows):
-    """(seq_lens, positions or None, table_width, block_size) of a step's resident metadata, checked."""
+    """(seq_lens, positions or None, table_width, block_size) of a step's resident metadata, checked.  The tensors are written in
+    place, so they are looked at as the caller holds them: a contiguous copy of a strided view would be advanced instead of it."""
     seq_lens, positions, table_width, block_size = advance
-    seq_lens = _i32("seq_lens", seq_lens)
-    if seq_lens.shape != (rows,) or not seq_lens.is_contiguous():
+    if _cuda("seq_lens", seq_lens).shape != (rows,) or not seq_lens.is_contiguous():
         raise ValueError("advance: seq_lens must be a contiguous int32 [rows] tensor")
+    seq_lens = _i32("seq_lens", seq_lens)
     if positions is not None:
-        positions = _i32("positions", positions)
-        if positions.numel() != rows or not positions.is_contiguous():
+        if _cuda("positions", positions).numel() != rows or not positions.is_contiguous():
             raise ValueError("advance: positions must be a contiguous int32 tensor of one entry per row")
+        positions = _i32("positions", positions)
     return seq_lens, positions, int(table_width), int(block_size)
 
 
