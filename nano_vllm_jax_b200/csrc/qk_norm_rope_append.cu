@@ -43,6 +43,23 @@ struct NormRopeParams {
   float eps;
 };
 
+// Cosine and sine of an fp32 angle with the relative accuracy of fp32, also next to their zeros.  CUDA's cosf and sinf reduce a large
+// angle by a slow path with a stack frame, and a kernel with a stack frame starts 1 us later; so the angle is reduced here.  In units of
+// pi it is hi + lo, the exact product with 1/pi to two doubles (Dekker's product, by one fused multiply-add); taking off the nearest
+// half leaves |r| <= 1/4 that is good to 2^-53 of itself but for ~1e-32 of the angle, so that rounding it to fp32 loses 2^-24 of
+// it and not 2^-24 of 1 (as half turns, |r| <= 1, did: up to 27% of a cosine at the integers next to an odd multiple of pi/2).
+__device__ __forceinline__ void cos_sin(float angle, float& c, float& s) {
+  constexpr double kInvPi = 0x1.45f306dc9c883p-2, kInvPiRest = -0x1.6b01ec5417056p-56;  // 1/pi as the sum of two doubles
+  const double a = (double)angle, hi = a * kInvPi, lo = fma(a, kInvPiRest, fma(a, kInvPi, -hi));
+  const double halves = rint(2.0 * hi);
+  const int quarter = (int)(halves - 4.0 * floor(0.25 * halves));  // 0 .. 3
+  float sr, cr;
+  sincospif((float)(fma(-0.5, halves, hi) + lo), &sr, &cr);
+  const float cq = (quarter & 1) ? sr : cr, sq = (quarter & 1) ? cr : sr;
+  c = (quarter == 1 || quarter == 2) ? -cq : cq;
+  s = (quarter & 2) ? -sq : sq;
+}
+
 template <int E>  // elements per lane = D / 32
 __global__ void __launch_bounds__(256) qk_norm_rope_append_kernel(NormRopeParams p) {
   pdl_wait();
@@ -109,8 +126,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_append_kernel(NormRopeParams
   for (int j = 0; j < E; ++j) y[j] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(__fmul_rn(x[j], r), __fadd_rn(1.f, w[j]))));
 
   // ---- partial rotary embedding on the first `rot` elements.  Lane i makes the cosine and sine of frequency i (and 32 + i, ...) for
-  // the whole warp; the lanes that rotate fetch theirs.  The angle, which CUDA's cosf would reduce by a slow path with a stack frame
-  // when it is large (a kernel with a stack frame starts 1 us later), is reduced to half turns in double precision.
+  // the whole warp; the lanes that rotate fetch theirs.
   const int half = p.rot / 2, half_lanes = half / E;  // a power of two
   if (half > 0) {
     float other[E];
@@ -124,9 +140,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_append_kernel(NormRopeParams
       if (i < half) {
         const int m = i % 3;
         const float pos = (m == 1 && i < p.h_limit) ? pos3[1] : ((m == 2 && i < p.w_limit) ? pos3[2] : pos3[0]);
-        double t = (double)__fmul_rn(pos, p.inv_freq[i]) * 0.31830988618379067154;  // in units of pi
-        t -= 2.0 * rint(0.5 * t);
-        sincospif((float)t, &s, &c);
+        cos_sin(__fmul_rn(pos, p.inv_freq[i]), c, s);
         c = __bfloat162float(__float2bfloat16_rn(c));
         s = __bfloat162float(__float2bfloat16_rn(s));
       }

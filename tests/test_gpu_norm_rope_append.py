@@ -48,7 +48,6 @@ def test_fused_norm_rope_append_matches_the_oracle(rows, cols, d, rot):
     torch.cuda.synchronize()
     # V rows are copies: bit-exact, and nothing but the addressed slots changed
     np.testing.assert_array_equal(bits(to_numpy(vc)), bits(ref_v))
-    # K and q: the same roundings as the oracle up to the last bf16 step where a sum of squares or a cosine differs in its last fp32 bit
     # K and q: the same roundings as the oracle except where a sum of squares, a cosine or a sine differs in its last
     # fp32 bit and flips a bf16 rounding: rare, and then one bf16 step of the operands (a rotated element that nearly
     # cancels is many steps of ITSELF away, so the bound is taken against the head row's magnitude)
@@ -135,8 +134,8 @@ def test_multimodal_three_row_positions(rows, cols):
 
 @pytest.mark.parametrize("rot", [64, 128, 256])  # one, two and four sets of 32 frequencies per warp
 def test_large_angles_and_wide_rotations_against_64_bits(rot):
-    """Positions up to 2^24: the fp32 angle's cosine and sine in 64 bits.  The kernel's are within 2e-7 of those (an fp32 rounding of
-    the reduced angle and one of the result), so a bf16 rounding flips in about 2e-7 / 2^-9 = 1e-4 of the cases."""
+    """Positions up to 2^24: the fp32 angle's cosine and sine in 64 bits.  The kernel's are within 2^-22 of their
+    size of those, so a bf16 rounding flips in about 2^-22 / 2^-8 = 6e-5 of the cases."""
     from nano_vllm_jax_b200.kernels import paged_kv as K
     c = _case(rot, 40, 1, 64)
     rng = np.random.default_rng(rot)
@@ -153,3 +152,43 @@ def test_large_angles_and_wide_rotations_against_64_bits(rot):
     w = want.astype(np.float32)
     assert (np.abs(got.astype(np.float32) - w) <= 2.0 ** -7 * np.abs(w).max(axis=-1, keepdims=True)).all()
     assert (_ulp_diff(got, want) > 0).mean() < 2e-3
+
+
+def _cosines_and_sines(pos, inv):
+    """The kernel's bf16 cosines and sines of positions x frequencies: the norm gives exactly 1 in the first half of the rotated
+    elements and 0 in the second, so the rotation returns them as they are."""
+    from nano_vllm_jax_b200 import _lib
+    n, rot = len(pos), 2 * len(inv)
+    q = torch.zeros((n, 8, 256), dtype=torch.bfloat16, device="cuda")
+    q[..., : rot // 2] = 1
+    w = torch.full((256,), (rot / 512) ** 0.5 - 1, device="cuda")  # undoes 1 / rms; within an fp32 rounding or two of 1, so 1 in bf16
+    k = torch.zeros((n, 2, 256), dtype=torch.bfloat16, device="cuda")
+    caches, out = torch.zeros((2, n, 2, 256), dtype=torch.bfloat16, device="cuda"), torch.empty_like(q)
+    p, slots = (torch.as_tensor(np.asarray(x, np.int32)).cuda() for x in (pos, np.arange(n)))
+    f = torch.as_tensor(inv).cuda()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.load().nvj_qk_norm_rope_kv_append(
+        q.data_ptr(), 8 * 256, 256, k.data_ptr(), 512, k.data_ptr(), 512, _lib.NVJ_BF16, w.data_ptr(), w.data_ptr(), _lib.NVJ_F32, 0.0,
+        f.data_ptr(), rot, p.data_ptr(), 1, None, slots.data_ptr(), None, None, 0, 0, n, 1, caches[0].data_ptr(),
+        caches[1].data_ptr(), _lib.NVJ_BF16, n, 8, 2, 256, out.data_ptr(), status.data_ptr(), torch.cuda.current_stream().cuda_stream),
+        "nvj_qk_norm_rope_kv_append")
+    assert not int(status)
+    got = to_numpy(out)[:, 0].astype(np.float64)
+    return got[:, : rot // 2], got[:, rot // 2: rot]
+
+
+@pytest.mark.parametrize("theta", [1.0, 1e7])
+def test_cosine_and_sine_near_their_zeros_keep_fp32_accuracy(theta):
+    """Off by half a bf16 step (2^-8: 8 bits of significand) and a few fp32 roundings (of the reduced angle 2^-24, of sincospif's result
+    2^-23; 2^-21 is allowed) of the value itself, also where that is nearly 0: the integers next to multiples of pi / 2 (theta 1:
+    frequency 1), and positions over the whole range on the model's frequencies."""
+    inv = (1.0 / np.float32(theta) ** (np.arange(0, 64, 2, dtype=np.float32) / np.float32(64))).astype(np.float32)
+    if theta == 1.0:
+        turns = np.arange(1, 1 << 22) * (2 / np.pi)
+        pos = 1 + np.argsort(np.abs(turns - np.rint(turns)))[:512]
+    else:
+        pos = np.exp2(np.random.default_rng(7).uniform(0, 24, 20000)).astype(np.int64)
+    ang = (pos.astype(np.float32)[:, None] * inv).astype(np.float64)
+    for name, got, want in zip(("cos", "sin"), _cosines_and_sines(pos, inv), (np.cos(ang), np.sin(ang))):
+        off = np.abs(got - want) / np.abs(want)
+        assert off.max() <= 2.0 ** -8 + 2.0 ** -21, f"{name}: {off.max():.2e} at position {pos[off.max(axis=1).argmax()]}"
