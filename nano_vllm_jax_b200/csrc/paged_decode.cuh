@@ -87,6 +87,12 @@ struct DecodeParams {
   float scale;
 };
 
+// Rows of 2 - 4 tokens that the automatic choice gives to the mma.sync tiles instead of tcgen05 (launch_decode_wide has the reason),
+// unless clusters serve them.
+inline bool wide_takes_mma_sync(const DecodeParams& p) {
+  return p.width <= 4 && (long long)p.batch * p.table_width > (p.width == 2 ? 4096 : 12288);
+}
+
 // Keys row b attends: seq_lens[b], clipped to what its page list can hold.  kWindow: the call may limit them further (a kernel
 // without a spare register pays 1% for code that a decode step never reaches).
 template <bool kWindow = true>

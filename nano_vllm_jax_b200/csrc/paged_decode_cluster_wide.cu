@@ -272,7 +272,14 @@ static int launch_tiles(const DecodeParams& p, int cluster, cudaStream_t stream)
 static bool cw_takes(const DecodeParams& p) {
   return p.width >= 2 && p.width <= kCwMaxWidth && p.batch <= kClMaxRows && !p.new_k && !p.packed_rows && !p.kv_indptr;
 }
-static int cw_cluster(const DecodeParams& p, int sms) { return cluster_size(p.batch, p.table_width, sms, 1, kCmPerSm, 8, kClMaxCluster); }
+// Two CTAs at least where the mma.sync form is the alternative: it sums every other block of a row apart, one CTA all of them in a
+// row, which is further from 64-bit attention (600 rows under 8 blocks, 2 tokens, plain / peaked / offset values: 1.84e-6 / 7.5e-7 / 4.1e-7 of
+// the result's size with one CTA, 1.71e-6 / 6.5e-7 / 3.5e-7 with two, 1.70e-6 / 6.4e-7 / 3.5e-7 mma.sync; tcgen05, the alternative below
+// that line, 2.03e-6 / 1.1e-6 / 4.5e-7).  They cost 33 -> 38 us there (mma.sync 48).
+static int cw_cluster(const DecodeParams& p, int sms) {
+  const int c = cluster_size(p.batch, p.table_width, sms, 1, kCmPerSm, 8, kClMaxCluster);
+  return c == 1 && p.table_width > 1 && wide_takes_mma_sync(p) ? 2 : c;
+}
 
 // Where the clusters beat the tcgen05 form: few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs that are
 // resident at once.  Clusters : tcgen05, us, by table width, rows and CTAs per row: 3 tokens, 7 blocks per CTA, 32 x 64 (10 CTAs)

@@ -502,8 +502,7 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
   // part, where the mma.sync form has eight short ones: against 64 bits 64 rows of 2 tokens are off by 4.4e-6 of their size with
   // it, 2.4e-6 without.  So it serves the smaller batches alone, where it wins most (4 tokens: 16 rows
   // of 512 - 2048 keys 31.1 : 23.2, 32 rows of 1024 - 4096 46.0 : 39.3).
-  const long long blocks = (long long)p.batch * p.table_width;
-  if (p.wide_form == 2 || (p.wide_form == 0 && p.width > 1 && (p.width > 4 || blocks <= (p.width == 2 ? 4096 : 12288)))) {
+  if (p.wide_form == 2 || (p.wide_form == 0 && p.width > 1 && !wide_takes_mma_sync(p))) {
     const int rc = launch_decode_umma(p, stream);
     if (rc != NVJ_ERR_UNSUPPORTED || p.wide_form == 2) return rc;
   }
