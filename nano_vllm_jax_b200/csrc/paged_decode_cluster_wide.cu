@@ -281,20 +281,27 @@ static int cw_cluster(const DecodeParams& p, int sms) {
   return c == 1 && p.table_width > 1 && wide_takes_mma_sync(p) ? 2 : c;
 }
 
-// Where the clusters beat the tcgen05 form: few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs that are
-// resident at once.  Clusters : tcgen05, us, by table width, rows and CTAs per row: 3 tokens, 7 blocks per CTA, 32 x 64 (10 CTAs)
+// Where the clusters beat the form that serves the rows otherwise: tcgen05 up to 4096 blocks of table (2 tokens) and 12288 (3 and 4),
+// mma.sync beyond (wide_takes_mma_sync).  First, few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs that
+// are resident at once.  Clusters : tcgen05, us, by table width, rows and CTAs per row: 3 tokens, 7 blocks per CTA, 32 x 64 (10 CTAs)
 // 20.7 : 21.1, 64 x 40 (6) 21.0 : 24.0, 128 x 16 (3, 6 blocks) 18.4 : 25.9; 8 blocks per CTA, 16 x 128 (16) 22.1 : 20.7, 4 x 128 15.9 : 15.9;
 // more CTAs than places, 140 x 40 40.7 : 36.2.  4 tokens: 64 x 40 22.9 : 24.9, 16 x 32 15.1 : 14.8, 16 x 128 23.7 : 21.4.  2 tokens: 16 x 128
-// 18.3 : 21.2, 64 x 40 18.5 : 24.0, 2 x 157 (10 blocks) 14.6 : 15.3, 8 x 256 (16 blocks) 23.4 : 22.7.  And many short rows, of which
-// every one costs the tcgen05 form a change of rows: 256 x 16 29.2 : 36.9, 36.3 : 38.6 and 39.1 : 40.9 (2, 3 and 4 tokens), 400 x 4
-// 14.3 : 34.4, 18.6 : 37.4 and 20.0 : 40.8, 200 x 25 31.0 : 35.8, 37.7 : 37.5 and 40.2 : 39.4.  Beyond 4 tokens a block takes 1.5 us
-// and the tcgen05 form is the faster one from 4 blocks on.
+// 18.3 : 21.2, 64 x 40 18.5 : 24.0, 2 x 157 (10 blocks) 14.6 : 15.3, 8 x 256 (16 blocks) 23.4 : 22.7; mma.sync: 50 x 96 30.6 : 30.1.
+// Second, many short rows, of which every one costs the other forms a change of rows.  Rows of 1/4 - 1 and of 1/32 - 1/8 of the
+// table; against tcgen05: 100 x 16 14.7 : 23.1 and 8.7 : 15.9 (2 tokens), 256 x 16 36.3 : 39.1 and 18.1 : 24.5 (3), 39.4 : 41.6 and
+// 20.6 : 26.8 (4), 1000 x 12 70.3 : 110.7 and 33.3 : 78.4 (3).  Against mma.sync, 2 tokens: up to 24 blocks, which two CTAs share, 400 x
+// 12 32.5 : 41.3 and 16.0 : 24.1, 2000 x 24 186.8 : 222.7 and 82.3 : 94.0, 4000 x 2 148 : 165 and 144 : 156, 16000 x 12 917 : 1151 and 572 : 674;
+// from 25 on four CTAs, which only pay while they are few: 200 x 25 32.5 : 35.7 and 15.8 : 19.5, 400 x 25 56.9 : 56.8 and 29.5 : 29.3, 600 x
+// 25 80.8 : 77.5 and 44.2 : 37.6, 2000 x 25 243 : 228 and 143 : 93.  3 and 4 tokens against mma.sync: ahead by 3 - 8% where the rows fill
+// the table, behind by as much where they do not, 1000 x 16 95.2 : 101.5 and 52.3 : 53.0, 2000 x 8 132.6 : 140.9 and 96.8 : 92.5 (3 tokens),
+// 150.7 : 155.9 and 115.8 : 105.4 (4), so they end at its line.
+// Beyond 4 tokens a block takes 1.5 us and the tcgen05 form is the faster one from 4 blocks on.
 bool decode_cluster_wide_pays(const DecodeParams& p) {
   const int sms = decode_wide_num_ctas();
   if (!cw_takes(p) || sms <= 0) return false;
   const int c = cw_cluster(p, sms), per_cta = (p.table_width + c - 1) / c;
   const long long ctas = (long long)c * p.batch;
-  if (p.batch >= 100 && p.table_width <= (p.width == 2 ? 25 : 16)) return true;
+  if (p.batch >= 100 && (p.width == 2 ? p.table_width <= (p.batch <= 400 ? 25 : 24) : p.table_width <= 16 && !wide_takes_mma_sync(p))) return true;
   if (p.width > 2 && per_cta == 8) return ctas <= sms;  // 0 - 2 us slower than tcgen05 there, at half its error against 64 bits
   return per_cta <= (p.width == 2 ? 12 : 7) && 100 * ctas <= (long long)kCmPerSm * sms;
 }

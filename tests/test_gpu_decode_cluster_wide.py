@@ -95,3 +95,17 @@ def test_many_short_rows_are_as_near_64_bits_as_on_mma_sync(rows, width, tokens,
     want = _in_64_bits(*args)
     off = [float((K.paged_decode_attention_wide(*args, SCALE, form=f).view_as(want) - want).norm()) for f in (0, 1)]
     assert off[0] <= 1.03 * off[1]
+
+
+# both sides of every end of the rule for many short rows: 2 tokens at 24 and 25 blocks, 3 and 4 tokens at 16 blocks and at 12288 blocks
+# of table in all; and of the rule for few blocks per CTA (the forms: 1 mma.sync, 2 tcgen05, 3 clusters)
+@pytest.mark.parametrize("tokens,rows,width,form", [(2, 100, 25, 3), (2, 400, 25, 3), (2, 401, 25, 1), (2, 401, 24, 3), (2, 2000, 24, 3), (2, 2000, 25, 1),
+                                                    (2, 130, 30, 3), (2, 160, 25, 3), (2, 160, 26, 1), (3, 768, 16, 3), (3, 769, 16, 1),
+                                                    (4, 3072, 4, 3), (4, 3073, 4, 1), (4, 200, 17, 2), (3, 64, 40, 3), (3, 64, 43, 2)])
+def test_the_form_that_the_rule_takes(tokens, rows, width, form):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines are drawn for 148 SMs")
+    args = _batch(rows + width, rows, width, tokens)
+    auto, *by_form = (K.paged_decode_attention_wide(*args, SCALE, form=f) for f in (0, 1, 2, 3))
+    assert [f for f, out in enumerate(by_form, 1) if torch.equal(out, auto)] == [form]  # (no two forms sum in one order)
