@@ -49,11 +49,10 @@ __device__ __forceinline__ bool next_seg(const DecodeParams& p, int& b, int& j, 
 }
 
 // Real blocks in the range [g, g1) that starts at position j of row b.
-template <bool kWindow = true>
 __device__ __forceinline__ int blocks_in_range(const DecodeParams& p, int b, int j, long long g, long long g1) {
   Seg s;
   int n = 0;
-  while (next_seg<kWindow>(p, b, j, g, g1, s)) n += s.j1 - s.j0;
+  while (next_seg(p, b, j, g, g1, s)) n += s.j1 - s.j0;
   return n;
 }
 
@@ -97,12 +96,12 @@ struct FillState {
 // their first K/V copies later than the others.  Asynchronous 4-byte copies of the ids with a second walk that checks
 // them were measured: the late CTAs gained 1.8 us, the others lost 0.8, the kernel's time did not change; an L1
 // prefetch of the next segment's ids ahead of every segment cost 3 us at kernel level.)
-template <bool kWindow = true, class Smem>
+template <class Smem>
 __device__ __forceinline__ void fill_ring(const DecodeParams& p, Smem& sm, FillState& f,
                                           long long g1, int n0, int count) {
   while (count > 0) {
     if (!f.has || f.j >= f.s.j1) {
-      if (!next_seg<kWindow>(p, f.b, f.jn, f.g, g1, f.s)) break;
+      if (!next_seg(p, f.b, f.jn, f.g, g1, f.s)) break;
       f.j = f.s.j0;
       f.has = true;
       ++f.nsegs;

@@ -26,7 +26,9 @@
 //     nothing is merged between them.  K/V still cross HBM once; the tensor work per block doubles
 //     and every warp now walks every block, which makes this form bound by a warp's chain of dependent
 //     tile products (width 8 takes ~1.9x the time of one token per row; entering the softmax weights as one bf16
-//     term instead of two was measured: 11% faster at 4e-3 instead of 2e-3 error, not taken).
+//     term instead of two was measured: 11% faster at 4e-3 instead of 2e-3 error, not taken).  The tcgen05 form
+//     (paged_decode_umma.cu) is the faster one there; this one serves a scale <= 0, which that does not
+//     take, and callers that ask for it (form 1).
 // Semantics: nanovllm_jax/kv_cache.py:852-998 (key p of row b is visible to token t when
 // p < seq_lens[b] and, with positions given, p <= positions[b, t]).
 

@@ -166,3 +166,18 @@ def test_rows_that_follow_one_another_in_a_range(lens, width):
     qsl = torch.arange(rows + 1, dtype=torch.int32, device="cuda") * width
     ref = K.packed_paged_prefill_attention(q.view(1, rows * width, 8, 256), k, v, tables, t_lens, pos.view(1, -1), qsl, BS, SCALE, 4, variant=1)
     assert float((got.view(-1) - ref.view(-1)).abs().max()) <= 2e-3
+
+
+@pytest.mark.parametrize("width", [2, 5, 8])
+@pytest.mark.parametrize("scale", [-SCALE, 0.0])
+def test_a_scale_that_is_not_positive(width, scale):
+    """The tcgen05 form takes row maxima before scaling and refuses it; the automatic choice then is the mma.sync form (clusters at 2)."""
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    lens = [40, 0, 700, 17, 1500]
+    c, q, tables, lens, pos = _case(61 + width, 256, lens, width)
+    got = to_numpy(K.paged_decode_attention_wide(to_torch(q), to_torch(c["k_cache"][0]), to_torch(c["v_cache"][0]), to_torch(tables),
+                                                 to_torch(lens), to_torch(pos), scale))
+    ref = R.paged_attention_decode(q, c["k_cache"], c["v_cache"], tables, lens, BS, scale, 4, positions=pos)
+    live = lens > 0
+    assert np.abs(got[live] - ref[live]).max() <= TIGHT
+    assert not got[~live].any()
