@@ -388,7 +388,8 @@ int nvj_paged_prefill_packed(const void* q, int q_dtype,
  *            or when that kernel cannot run: call nvj_paged_prefill_packed instead); `workspace` (nullable) is
  *            not used
  *   part 3   all rows on the tile kernel, which then zeroes what it does not write itself (no zeroed `out` needed):
- *            a batch without decode rows that still wants the key-range splits
+ *            a batch without decode rows.  With a `workspace` its key ranges may be split (nothing is written there); without, they
+ *            stay whole
  * The reference runs a mixed batch through one packed attention call; the split has no counterpart there.
  */
 int nvj_paged_prefill_packed_part(const void* q, int q_dtype,

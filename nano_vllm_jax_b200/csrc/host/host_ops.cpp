@@ -382,9 +382,9 @@ PyObject* packed_prefill(PyObject* const* a, Py_ssize_t n) {
   void* stream = stream_of(l.device);
   int32_t* st = status_for(l.device, stream);
   if (!st) return nullptr;
-  const bool tiles_only = model_shape && variant != 1 && decode_rows == 0 && !env_is("NVJ_PREFILL_KEY_SPLITS", "0");
+  const bool tiles_only = model_shape && variant != 1 && decode_rows == 0;  // a workspace lent to the tiles lets them split key ranges
   const Workspace* ws = nullptr;
-  if (tiles_only || decode_rows != 0) {
+  if (tiles_only ? !env_is("NVJ_PREFILL_KEY_SPLITS", "0") : decode_rows != 0) {
     ws = workspace_for(l.device, stream, rows);
     if (!ws) return nullptr;
   }

@@ -128,15 +128,16 @@ static bool rows_run_beside_tiles(const PackedArgs& a) {
 
 // The query tiles: tcgen05 tiles first (CTA pairs, then single CTAs); they decline when the driver has no tensor-map
 // encoder or the scale is not positive, and the mma.sync tiles take over.  With skip_single the rows of one query
-// token are left to the pass above (and, unless the pair kernel serves the call, `out` has been zeroed by the caller).
-static int run_tiles(const PackedArgs& a, int skip_single, int32_t* beside, cudaStream_t s) {
+// token are left to the pass above (and, unless the pair kernel serves the call, `out` has been zeroed by the caller).  may_split: the
+// pair kernel may cut key ranges (not beside decode rows, which want the SMs).
+static int run_tiles(const PackedArgs& a, int skip_single, bool may_split, int32_t* beside, cudaStream_t s) {
   const char* kc = static_cast<const char*>(a.k_cache_layer);
   const char* vc = static_cast<const char*>(a.v_cache_layer);
   const int variant = a.variant;
   if (variant == 0 || variant == 4 || variant == 5) {
     const int rc = launch_prefill_umma2(a.q, a.q_dtype, kc, vc, a.num_blocks, a.block_tables, a.table_width, a.kv_lens, a.positions,
                                         a.query_start_loc, a.rows, a.token_bucket, a.scale, a.out, a.status, skip_single,
-                                        variant == 5 ? 0 : 1, a.tile_pairs, !skip_single, beside, s);
+                                        variant == 5 ? 0 : 1, a.tile_pairs, may_split, beside, s);
     if (rc != NVJ_ERR_UNSUPPORTED || variant != 0) return rc;
   }
   if (variant == 0 || variant == 3) {
@@ -195,7 +196,7 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
     if (!tile_ok || a.variant == 1) return NVJ_ERR_UNSUPPORTED;  // the generic kernel serves a batch in one piece
     if (part == 1) return run_single_token_rows(a, cta_limit, nullptr, s);
     if (part == 2 && !pair_kernel_serves(a)) return NVJ_ERR_UNSUPPORTED;  // the other tile kernels want a zeroed output
-    return run_tiles(a, part == 2 ? 1 : 0, nullptr, s);
+    return run_tiles(a, part == 2 ? 1 : 0, part == 3 && a.workspace, nullptr, s);
   }
   if (!tile_ok || a.variant == 1) return run_generic(a, s);
   // Rows that carry a single query token go to the streaming decode kernel when the caller lends it a decode
@@ -205,7 +206,7 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
   if (carve_for_decode_rows(a, carved) == NVJ_OK && rows_run_beside_tiles(a)) {
     // tiles first, on a few SMs (a CTA pair per KV head and 64 tokens); the decode rows' clusters start at once and take the rest
     int32_t* word = static_cast<int32_t*>(a.workspace) + kWsBesideWord;
-    const int rc2 = run_tiles(a, 1, word, s), sms = decode_wide_num_ctas();
+    const int rc2 = run_tiles(a, 1, false, word, s), sms = decode_wide_num_ctas();
     if (rc2 != NVJ_OK) return rc2;
     const int rest = a.tile_pairs > 0 ? sms - 2 * kHkv * a.tile_pairs : sms;
     const int rc1 = run_single_token_rows(a, rest > sms / 2 ? rest : sms / 2, word, s);
@@ -224,10 +225,10 @@ static int run_packed(const PackedArgs& a, int part, int cta_limit, cudaStream_t
     } else {  // no room to serve the rows of one token: the tiles take them too, and the caller has not counted those
       PackedArgs all = a;
       all.tile_pairs = -1;
-      return run_tiles(all, 0, nullptr, s);
+      return run_tiles(all, 0, true, nullptr, s);
     }
   }
-  return run_tiles(a, skip_single, nullptr, s);
+  return run_tiles(a, skip_single, !skip_single, nullptr, s);
 }
 
 }  // namespace nvj

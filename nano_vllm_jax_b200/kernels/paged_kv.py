@@ -693,10 +693,10 @@ def packed_paged_prefill_attention(query, k_cache_layer, v_cache_layer, block_ta
             cur.wait_stream(side)
             check(rc1, "nvj_paged_prefill_packed_part (decode rows)")
             check(rc2, "nvj_paged_prefill_packed_part (tiles)")
-    elif model_shape and variant != 1 and num_decode_rows == 0 and os.environ.get("NVJ_PREFILL_KEY_SPLITS", "1") != "0":
-        # no decode rows: the tile kernel alone (it zero-fills what it does not write), with the workspace lent for
-        # the key-range splits of a short batch
-        ws = _workspace(q.device, rows)
+    elif model_shape and variant != 1 and num_decode_rows == 0:
+        # no decode rows: the tile kernel alone (it zero-fills what it does not write), with the workspace that says it may
+        # split the key ranges of a short batch (NVJ_PREFILL_KEY_SPLITS=0: they stay whole)
+        ws = _workspace(q.device, rows) if os.environ.get("NVJ_PREFILL_KEY_SPLITS", "1") != "0" else None
         check(call(lib.nvj_paged_prefill_packed_part, ws, 3, 0), "nvj_paged_prefill_packed_part (tiles, all rows)")
     else:
         ws = _workspace(q.device, rows) if (num_decode_rows is None or num_decode_rows > 0) else None

@@ -70,3 +70,24 @@ def test_split_key_ranges_equal_the_kernel_that_never_splits(qlens, cached, pad)
     for count in (pairs, None):
         out = K.packed_paged_prefill_attention(*args, variant=4, num_decode_rows=0, query_tile_pairs=count)
         assert float((out - ref).abs().max()) <= 2e-3 and not out[0, sum(qlens):].any()
+
+
+@pytest.mark.parametrize("route", ["python", "extension"])
+def test_key_ranges_stay_whole_where_the_caller_says_so(monkeypatch, route):
+    """NVJ_PREFILL_KEY_SPLITS=0: bit for bit what the same rows give beside a decode row, whose batch is never split."""
+    from nano_vllm_jax_b200 import kv_cache as kvc
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    q, (k, v), tables, lens, pos, rid, qsl = _batch((130, 64, 1), (1500, 700, 20), 0, 9)
+
+    def run(rows):
+        n = int(qsl[rows])
+        if route == "python":
+            return K.packed_paged_prefill_attention(q[:, :n], k[0], v[0], tables[:rows], lens[:rows], pos[:, :n], qsl[: rows + 1], BS, SCALE, 4,
+                                                    variant=4, num_decode_rows=rows - 2)[0, :194]
+        return kvc.paged_attention_prefill_packed(q[:, :n], k, v, tables[:rows], lens[:rows], pos[:, :n], rid[:, :n], qsl[: rows + 1], BS, SCALE,
+                                                  4, out_dtype=torch.float32, num_decode_rows=rows - 2)[0, :194]
+
+    whole, split = run(3), run(2)
+    assert not torch.equal(whole, split) and float((whole - split).abs().max()) <= 2e-3
+    monkeypatch.setenv("NVJ_PREFILL_KEY_SPLITS", "0")
+    assert torch.equal(run(2).view(torch.int32), whole.view(torch.int32))
