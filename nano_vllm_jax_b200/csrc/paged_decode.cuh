@@ -192,7 +192,7 @@ int launch_decode_pipelined(const DecodeParams& p, int num_ctas, cudaStream_t st
 int decode_wide_num_ctas();  // 1 per SM of the current device
 int launch_decode_wide(const DecodeParams& p, cudaStream_t stream);  // rows of 1 - 16 tokens: picks the form
 int launch_decode_stream(const DecodeParams& p, cudaStream_t stream);  // one query token per row, bf16
-int launch_decode_cluster_wide(const DecodeParams& p, cudaStream_t stream);  // rows of 2 - 4 tokens, few and short
+int launch_decode_cluster_wide(const DecodeParams& p, cudaStream_t stream);  // rows of 2 - 4 tokens, few or short
 bool decode_cluster_wide_pays(const DecodeParams& p);
 int run_decode_wide(DecodeParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);  // checks, carves, launches
 int launch_decode_umma(const DecodeParams& p, cudaStream_t stream);  // the tcgen05 form, rows already appended

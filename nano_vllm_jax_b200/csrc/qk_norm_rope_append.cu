@@ -48,6 +48,7 @@ struct NormRopeParams {
 // pi it is hi + lo, the exact product with 1/pi to two doubles (Dekker's product, by one fused multiply-add); taking off the nearest
 // half leaves |r| <= 1/4 that is good to 2^-53 of itself but for ~1e-32 of the angle, so that rounding it to fp32 loses 2^-24 of
 // it and not 2^-24 of 1 (as half turns, |r| <= 1, did: up to 27% of a cosine at the integers next to an odd multiple of pi/2).
+// Against half turns: nothing up to 512 tokens (6.4 us), 4096 29.2 -> 29.8, 16384 114.7 -> 116.4.
 __device__ __forceinline__ void cos_sin(float angle, float& c, float& s) {
   constexpr double kInvPi = 0x1.45f306dc9c883p-2, kInvPiRest = -0x1.6b01ec5417056p-56;  // 1/pi as the sum of two doubles
   const double a = (double)angle, hi = a * kInvPi, lo = fma(a, kInvPiRest, fma(a, kInvPi, -hi));

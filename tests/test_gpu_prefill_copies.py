@@ -308,8 +308,8 @@ def test_row_argmax_first_maximum_wins():
 
 def test_short_chunk_with_key_range_splits_matches_the_unsplit_kernels_and_the_oracle():
     """A 512-token chunk behind a 512-token prefix, plus a ragged second row: too few CTA pairs to fill the GPU, so the
-    pair kernel splits every tile's key range (the wrapper lends it the workspace); the single-CTA tile kernel never
-    splits.  Both must agree with the oracle, and a second split call must give what the first gave."""
+    pair kernel splits every tile's key range (the wrapper lends a workspace, which allows it to); the single-CTA tile kernel
+    never splits.  Both must agree with the oracle, and a second split call must give what the first gave."""
     import numpy as np
     import torch
     from helpers import BS, SCALE, to_numpy, to_torch
@@ -336,7 +336,7 @@ def test_short_chunk_with_key_range_splits_matches_the_unsplit_kernels_and_the_o
     args = (tk[0], tv[0], to_torch(tables), to_torch(lens), to_torch(pos), to_torch(qsl), BS, SCALE, 4)
     outs = {}
     first = None
-    for variant in (4, 3, 4):  # the split path twice: the workspace is reused as the first call left it
+    for variant in (4, 3, 4):  # the split path twice
         outs[variant] = to_numpy(K.packed_paged_prefill_attention(tq, *args, variant=variant, num_decode_rows=0)).reshape(bucket, 8, 256)
         if variant == 4 and first is None:
             first = outs[4].copy()
@@ -395,9 +395,9 @@ def test_hybrid_state_batch_gather_and_store_match_indexing():
     full.store_batch([0, 1, 2], whole)
 
 
-def test_split_prefill_with_its_merge_launch_replays_from_a_cuda_graph():
-    """The tile kernel and the merge launch behind it (a programmatic dependent launch) captured into one CUDA graph:
-    the replay gives what the eager call gave, also after the inputs changed."""
+def test_split_prefill_replays_from_a_cuda_graph():
+    """The tile kernel whose key-range splits are clusters, captured into a CUDA graph: the replay gives what the eager call
+    gave, also after the inputs changed."""
     import numpy as np
     import torch
     from helpers import BS, SCALE, to_torch
