@@ -349,10 +349,11 @@ int nvj_paged_decode_window(const void* q, int q_dtype, const void* k_cache_laye
  *   workspace  nullable decode workspace (nvj_paged_decode_workspace_bytes(rows)); when given,
  *              rows that hold exactly one query token (the decode rows of a mixed batch,
  *              nanovllm_jax/engine/scheduler.py:956-1032) are served by a decode
- *              kernel instead of a query tile (one too small or not 16-byte aligned leaves them to the tiles).  Batches without such rows
- *              that are too short to fill the GPU have every tile's key range split over several CTA pairs
- *              (variants 0, 4, 5; a 512-token chunk is 16 pairs on 74 pair slots), which fold their rows
- *              inside a cluster.  nvj_paged_prefill_workspace_bytes(rows) bytes are enough for the decode rows.
+ *              kernel instead of a query tile (one too small or not 16-byte aligned leaves them to the tiles).
+ *              nvj_paged_prefill_workspace_bytes(rows) bytes are enough for them.  Without one all rows go to the
+ *              tiles, and a batch too short to fill the GPU has every tile's key range split over several CTA pairs
+ *              (variants 0, 4, 5; a 512-token chunk is 16 pairs on 74 pair slots), which fold their rows inside a
+ *              cluster; part 3 of nvj_paged_prefill_packed_part is the same with the choice.
  *   variant    0 = automatic; 1 = generic CUDA-core kernel (any shape or dtype); for the model's
  *              shape (bf16 cache, block 16, 2 KV x 4 query heads, head_dim 256): 2 = mma.sync
  *              tiles of 16 tokens, 3 = tcgen05 tiles of 32 tokens with accumulators in tensor
