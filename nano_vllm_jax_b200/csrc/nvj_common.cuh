@@ -159,6 +159,16 @@ __device__ __forceinline__ int32_t ld_acquire_gpu(const int32_t* p) {
   return v;
 }
 
+__device__ __forceinline__ int32_t ld_relaxed_gpu(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// `bytes` (a multiple of 16) from a 16-byte boundary on, into the L2.
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // Streaming 16-byte load that does not allocate in L1 (read-once data).  Not the non-coherent form: a kernel's CTAs may be
 // resident while the kernel in front still writes what they will read (pdl_wait below).
 __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
@@ -173,7 +183,7 @@ __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
 // The kernels of a step follow one another on one stream, and an ordinary launch leaves ~2 us between two of them: the
 // next grid's CTAs are only placed once the last one of this grid has gone and its writes have been flushed.  A kernel
 // launched by launch_after() may be placed while the kernel in front of it is still running (if that one has called
-// pdl_release(), which ours do as soon as they have started): its pdl_wait(), before its first access to global memory,
+// pdl_release(), which ours do as soon as they have started): its pdl_wait(), before its first access to global memory (hints apart),
 // holds it until everything in front has completed and is visible.  Since every such kernel waits before it ends, the
 // stream's order holds for whatever follows.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -395,6 +395,22 @@ struct CmSmem {
   float2 pick_warp[kCmWarps];
 };
 
+// Ahead of pdl_wait(), while the append in front is at work and memory is idle: K and V rows of block jb, the first that this warp
+// will walk, on their way into the L2.  What is read here may be about to change, so it is a hint and nothing else: relaxed loads
+// (they leave no line in the L1 that a load behind the wait could find), an id that is checked against the pool, a prefetch.
+// Measured, six layers of norm + RoPE + append and this: 48 rows of 128 - 2048 keys 164.2 -> 154.3 us, 200 of 64 - 512 186 -> 174, 256 of
+// 1024 - 4096 1254 -> 1247; with the two first blocks 164.9, and with the append letting its dependents go before its own wait 163.5
+// (both take bandwidth from the kernel that still runs).  Only where the rows have been appended by a launch of their own: in front
+// of a fused append may be anything, and where that has long ended the extra trip to memory is lost (64 rows from host memory 512.8 ->
+// 517.2); and only in CTAs that start together (256 rows, fused, 1674 -> 1683).
+__device__ __forceinline__ void cm_prefetch_block(const DecodeParams& p, int b, int kvh, int jb, int lane) {
+  if ((int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) >= p.early_ctas || jb >= p.table_width) return;
+  const int len = ld_relaxed_gpu(p.seq_lens + b), blk = ld_relaxed_gpu(p.block_tables + (long long)b * p.table_width + jb);
+  if (len <= jb * kBlk || blk < 0 || blk >= p.num_blocks) return;
+  const char* cache = lane < kBlk ? p.k_cache : p.v_cache;
+  l2_prefetch(cache + ((long long)blk * kBlk + (lane & (kBlk - 1))) * kTokenBytes + kvh * kRowBytes, kRowBytes);
+}
+
 // kPick: the token pick of a decode step (DecodeParams::pick_tokens).  All CTAs of a row then form one cluster, also where
 // they take a KV head each.
 template <typename T, bool kBoth, bool kPick>
@@ -408,6 +424,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   constexpr int kWalkers = kBoth ? kCmWarps / 2 : kCmWarps;  // warps of the CTA that share a KV head's blocks
   const int first = rank * kWalkers + (kBoth ? warp >> 1 : warp), stride = ctas * kWalkers;  // this warp's blocks: first, first + stride, ...
 
+  cm_prefetch_block(p, b, kvh, first, lane);
   if (!p.beside || ld_acquire_gpu(p.beside) == 0) pdl_wait();
   pdl_release();
   // ---- first trip: the ids of this warp's first 32 blocks, the length, the query
@@ -714,10 +731,12 @@ bool decode_cluster_picks(const DecodeParams& p) {
   return f.both || members <= 10 || (members <= kClMaxCluster && 100LL * members * p.batch <= 225LL * sms);
 }
 
-int launch_decode_cluster(const DecodeParams& p, cudaStream_t stream) {
-  if (p.batch > kClMaxRows) return NVJ_ERR_UNSUPPORTED;
+int launch_decode_cluster(const DecodeParams& call, cudaStream_t stream) {
+  if (call.batch > kClMaxRows) return NVJ_ERR_UNSUPPORTED;
   const int sms = decode_wide_num_ctas();
   if (sms <= 0) return NVJ_ERR_LAUNCH;
+  DecodeParams p = call;
+  p.early_ctas = p.new_k || p.kv_indptr || p.packed_rows || p.beside ? 0 : 3 * sms;  // three CTAs to an SM
   // (with a page list per row its width is not known here: as many CTAs as an ordinary row has use for)
   const int blocks = p.kv_indptr ? 64 : p.table_width;
   // Beside another kernel: the SMs that it leaves (cta_limit), three CTAs to each; the ones too many start when it ends (six

@@ -134,3 +134,25 @@ def test_few_rows_of_many_blocks(rows, width, pays):
     q = to_torch(c["q"][:, 0]).contiguous()
     ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
     assert float((K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE) - ref).abs().max()) <= 2e-3
+
+
+# What the kernel looks at ahead of its wait is a hint: here the kernel in front changes the lengths (rows gain a key, some a block)
+# and the tables hold ids outside the pool behind the last block.  CTAs with the hint and, beyond three to an SM, without it.
+@pytest.mark.parametrize("rows,width", [(3, 5), (48, 20), (300, 6)])
+def test_lengths_that_the_kernel_in_front_changes(rows, width, monkeypatch):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    monkeypatch.setenv("NVJ_CHECK_STATUS", "1")  # nothing may be flagged
+    before = [(0, 15, 16, 47, width * BS - 1, 33)[i % 6] for i in range(rows)]
+    k, v, tables, lens, c = _case(rows, [n + 1 if n else 0 for n in before], width, torch.bfloat16)
+    used = torch.arange(width, device="cuda")[None] * BS < lens[:, None]
+    tables = torch.where(used, tables, torch.full_like(tables, k.shape[1] + 7))
+    q = to_torch(c["q"][:, 0]).contiguous()
+    ref = K.paged_decode_attention(q, k[0], v[0], tables, lens, SCALE, variant=1)
+    x = torch.randn(rows, 2048, device="cuda")
+    for _ in range(3):
+        now = torch.tensor(before, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        K.row_argmax(x, advance=(now, None, width, BS))
+        got = K.paged_decode_attention(q, k[0], v[0], tables, now, SCALE, variant=4)
+        assert torch.equal(now, lens)
+        assert float((got - ref).abs().max()) <= 2e-3
