@@ -149,6 +149,24 @@ __device__ __forceinline__ Partition make_partition(long long total, int grid) {
   return pt;
 }
 
+// What the tcgen05 wide kernels tell the launch that folds their partials: per range, the row that its beginning cuts first (its blocks
+// lie in ranges first .. last, this one is first + 1), or b = -1.  In the workspace behind the (max, sum) pairs of 2 * ranges slots.
+struct alignas(16) UmmaCut {
+  int b, first, last, unused;
+};
+constexpr UmmaCut kNoCut = {-1, 0, 0, 0};
+__device__ __forceinline__ UmmaCut* umma_cuts(const DecodeParams& p, int ranges) {
+  return reinterpret_cast<UmmaCut*>(p.part_ml + (size_t)2 * ranges * p.width * kHq * 2);
+}
+__host__ __device__ inline size_t umma_cuts_bytes(int ranges) { return ws_round(sizeof(UmmaCut) * ranges); }
+// That of range `range`, which begins at position j of row b (phantom blocks counted) and at g0 of the sequence.
+__device__ __forceinline__ UmmaCut umma_cut(const DecodeParams& p, const Partition& pt, int range, int b, int j, long long g0) {
+  const int nb = (decode_row_len(p, b) + kBlk - 1) / kBlk;
+  const long long row_g0 = g0 - j;
+  const int first = pt.cta_of(row_g0);
+  if (j == 0 || j >= nb || first != range - 1) return kNoCut;
+  return UmmaCut{b, first, pt.cta_of(row_g0 + nb - 1), 0};
+}
 // Where a CTA parks its partial result for a row it shares with other CTAs: a
 // CTA holds at most one segment that continues a row begun elsewhere (slot 2c)
 // and at most one that begins a row finished elsewhere (slot 2c + 1).

@@ -499,11 +499,11 @@ int launch_decode_wide(const DecodeParams& p, cudaStream_t stream) {
   if (p.wide_form == 3 || (p.wide_form == 0 && p.cta_limit <= 0 && decode_cluster_wide_pays(p)))
     return launch_decode_cluster_wide(p, stream);
   // Rows of 5 and more query tokens: the tcgen05 form (the mma.sync form is compute-bound there and ends at 8 tokens).  Below
-  // that the tcgen05 form is the faster one up to 32768 blocks with 2 tokens and always with 3 and 4 (mma.sync : tcgen05, us, 4 tokens over
-  // 1024 - 4096 keys: 64 rows 70.5 : 65.3, 192 rows 220 : 176), but it carries one sum in tensor memory over all keys of a row's
-  // part, where the mma.sync form has eight short ones: against 64 bits 64 rows of 2 tokens are off by 4.4e-6 of their size with
-  // it, 2.4e-6 without.  So it serves the smaller batches alone, where it wins most (4 tokens: 16 rows
-  // of 512 - 2048 keys 31.1 : 23.2, 32 rows of 1024 - 4096 46.0 : 39.3).
+  // that the tcgen05 form is the faster one too (mma.sync : tcgen05, us, 4 tokens over 1024 - 4096 keys: 64 rows 70 : 62, 192 rows 220 :
+  // 176), but its three sums in tensor memory over all keys of a row's part are longer than the eight of the mma.sync form: against 64
+  // bits 64 rows of 2 tokens over 1024 - 4096 keys, plain / peaked / offset values, are off by 2.5e-6 / 2.0e-6 / 0.7e-6 of their size with it,
+  // by 2.4e-6 / 1.2e-6 / 1.1e-6 without.  So it serves the smaller batches alone, where it wins most (4 tokens: 16 rows of 512 - 2048 keys
+  // 29.1 : 16.3, 50 rows under 60 blocks 29.8 : 22.9).
   if (p.wide_form == 2 || (p.wide_form == 0 && p.width > 1 && !wide_takes_mma_sync(p))) {
     const int rc = launch_decode_umma(p, stream);
     if (rc != NVJ_ERR_UNSUPPORTED || p.wide_form == 2) return rc;
@@ -564,7 +564,8 @@ int run_decode_wide(DecodeParams& p, void* workspace, size_t workspace_bytes, cu
   const int n = decode_wide_num_ctas();
   if (n <= 0) return NVJ_ERR_LAUNCH;
   // rows of more than 8 tokens run on the tcgen05 form only, which parks two partials per pair of CTAs: n slots
-  const size_t ml_bytes = p.width > kWMaxWidth ? ws_round(sizeof(float) * n * p.width * kHq * 2) : wide_ml_bytes(n, p.width);
+  // (and what they cut where: umma_cuts; the wider forms have slots to spare)
+  const size_t ml_bytes = p.width > kWMaxWidth ? ws_round(sizeof(float) * n * p.width * kHq * 2) + umma_cuts_bytes(n) : wide_ml_bytes(n, p.width);
   const size_t acc_bytes = p.width > kWMaxWidth ? ws_round(sizeof(float) * n * p.width * kHq * kD) : wide_acc_bytes(n, p.width);
   const int carved = carve_decode_workspace(p, workspace, workspace_bytes, ml_bytes, acc_bytes);
   if (carved != NVJ_OK) return carved;

@@ -33,6 +33,14 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
+// The same with A through a shared-memory descriptor.
+__device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -51,6 +59,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+// 8 columns; the values are there behind tmem_ld_wait() and, for the compiler, tmem_loaded()
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_loaded(float (&v)[8]) {
+  asm volatile("" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]));
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
   asm volatile(
@@ -92,6 +111,21 @@ __device__ __forceinline__ void tma_load_block(uint32_t dst, const CUtensorMap* 
       : "memory");
 }
 
+// One KV head's half of a block (8 KiB): V through the view of half_block_maps ...
+__device__ __forceinline__ void tma_load_v_half(uint32_t dst, const CUtensorMap* map, int token, int kvh, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %2, %4}], [%5], %6;"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(token), "r"(kvh), "r"(bar), "l"(policy)
+      : "memory");
+}
+// ... and K through the grouped one of four chunks.  `group` counts groups of eight tokens.
+__device__ __forceinline__ void tma_load_k_half(uint32_t dst, const CUtensorMap* map, int group, int kvh, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %2, %2, %3, %4}], [%5], %6;"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(group), "r"(kvh), "r"(bar), "l"(policy)
+      : "memory");
+}
+
 // Shared-memory matrix descriptor, 128-byte swizzle (layout type 2), descriptor version 1.
 // Offsets are in bytes; the 4 low bits are dropped by the encoding.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr, uint32_t leading_bytes, uint32_t stride_bytes) {
@@ -107,6 +141,8 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr, uint32_t leadi
 __device__ __forceinline__ constexpr uint32_t umma_idesc(int n, bool b_mn_major) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
 }
+
+constexpr uint32_t kUmmaTransposedA = 1u << 15;  // A from shared memory with its rows contiguous
 
 // try_wait that lets the hardware park the warp for up to `hint_ns` until the phase completes:
 // a warp that polls in a tight loop would take issue slots from the MMA warp on its scheduler.
@@ -175,6 +211,8 @@ bool block_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t tokens
 // chunks of one KV head's half of a block and lands as [group][chunk][8 tokens][128 B], so that the groups of a tile of several
 // blocks are evenly spaced, as the rows of one operand have to be, whatever its number of blocks.
 bool grouped_map_cached(CUtensorMap* map, const void* cache_layer, uint64_t tokens, int chunks);
+// A layer's K and V for tma_load_k_half and tma_load_v_half.
+bool half_block_maps(CUtensorMap* k_map, CUtensorMap* v_map, const void* k_layer, const void* v_layer, uint64_t tokens);
 bool tensor_maps_available();  // the driver has an encoder
 
 }  // namespace nvj
