@@ -14,6 +14,11 @@ __device__ __forceinline__ void cl_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same where nothing that was stored is read behind it: it does not wait for this thread's stores to be visible.
+__device__ __forceinline__ void cl_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // Address of this CTA's shared-memory location in CTA `rank` of the cluster, and loads from there.
 __device__ __forceinline__ uint32_t cl_map(const void* p, uint32_t rank) {
   uint32_t a;

@@ -169,6 +169,12 @@ __device__ __forceinline__ int32_t ld_relaxed_gpu(const int32_t* p) {
   asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+// A load that the compiler leaves where it stands among others of its kind.
+__device__ __forceinline__ int32_t ld_in_turn(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 // `bytes` (a multiple of 16) from a 16-byte boundary on, into the L2.
 __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");

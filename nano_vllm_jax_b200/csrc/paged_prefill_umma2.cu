@@ -89,14 +89,17 @@ struct Umma2Smem {
   alignas(1024) char v[kU2Stages][4][4096];  // [stage][block][8-key group][this CTA's two 64-d chunks][8 keys][128 B]
   // used in CTA 0 only: q_full, k_full, v_full, s_read, p_full; used in both: the rest
   alignas(8) unsigned long long q_full, k_full[kU2Stages], v_full[kU2Stages], k_empty[kU2Stages], v_empty[kU2Stages],
-      s_full, s_read, p_full, pv_done, x_full[4];  // x_full: per quarter of the rows, whose two warps share them
-  float xchg[2][2][kU2Rows];
+      s_full[2], s_read, o_full;  // s_full: [tile & 1]; o_full: every product has retired
+  unsigned long long p_full[2], pv_done[2][2];  // per half of a tile's keys: weights written; the product that reads them retired [tile & 1]
+  unsigned long long m_full[4][2];  // per quarter of the rows: the reference of an even / odd tile has been settled
+  float m_row[2][kU2Rows];          // the reference itself [tile & 1]
+  float2 sums[2][kU2Rows];          // at the end: each group's (reference, sum of weights)
   // this CTA's query rows on their way into tensor memory: [token][head of the group][32 pieces of 16 B], the pieces
   // of token t stored at (piece ^ (t & 7)) so that both the row-wise fill and the token-wise read are conflict-free
   alignas(16) char qstage[kU2Tokens * kG * kD * 2];
   float2 own_ml[kU2Rows];  // this split's (max, sum) per row, for the fold
   uint32_t tmem_base;
-  int row, tok0, ntok, pair_last_tok, idle_index, abort_flag, total_pairs;
+  int abort_flag;
 };
 
 // ---- cta_group::2 wrappers ---------------------------------------------------------------------
@@ -192,9 +195,11 @@ __device__ __forceinline__ void u2_producer(const CUtensorMap* k_map, const CUte
 }
 
 // ---- warp 1 of CTA 0: MMA issue for the pair -------------------------------------------------
-// S(t + 1) is issued as soon as the softmax has read S(t), P V(t) behind it once the weights are written: while the weights of
-// one tile are on their way the tensor pipe has the scores of the next.  (With the weights written over their scores, in two
-// buffers, S(t + 2) had to wait for P V(t) to retire: 2030 cycles per pair and tile, 1640 of them MMAs.)
+// S(t + 2) is issued as soon as the softmax has read S(t + 1), in front of P V(t), which waits for its weights half a tile at a time.  From
+// its scores to its weights a tile takes ~2000 cycles, its products 1640: with one tile of scores ahead (and all softmax
+// warps on the same tile) a lone pair took 1.02 us per tile, now 0.93; one tile ahead with two softmax groups, or with the weights in
+// halves as well, still 1.02.  1000 tokens behind 4000 56.8 -> 51.6 us, 2000 of four prompts 25.5 -> 23.8, 512 behind 1024 21.1 -> 20.0; under the
+// power cap, 16384 of one prompt, 1145 -> 1138.
 __device__ __forceinline__ bool u2_issue_s(Umma2Smem& sm, const Umma2Params& p, uint32_t tmem, uint64_t k_desc0, int t,
                                            int stage, uint32_t full_parity) {
   if (!um_wait(&sm.k_full[stage], full_parity, &sm.abort_flag, p.status)) return false;
@@ -207,7 +212,7 @@ __device__ __forceinline__ bool u2_issue_s(Umma2Smem& sm, const Umma2Params& p, 
     for (int ks = 0; ks < 16; ++ks)  // 16 dims per MMA: 8 columns of Q; K chunk ks / 4, 32 bytes into its swizzled rows
       umma2_bf16_ts(tmem + kU2ColS, tmem + kU2ColQ + ks * 8, k_desc + (uint64_t)(((ks >> 2) * (8 * 128) + (ks & 3) * 32) >> 4), idesc,
                     ks > 0 ? 1u : 0u);
-    umma2_commit_pair(smem_u32(&sm.s_full));
+    umma2_commit_pair(smem_u32(&sm.s_full[t & 1]));
     umma2_commit_pair(smem_u32(&sm.k_empty[stage]));
   }
   __syncwarp();
@@ -218,87 +223,103 @@ __device__ __forceinline__ void u2_mma_warp(Umma2Smem& sm, const Umma2Params& p,
   const uint64_t k_desc0 = umma_desc(smem_u32(&sm.k[0][0][0]), 16, 4 * 8 * 128);       // keys are rows, groups of 8 4 KiB apart
   const uint64_t v_desc0 = umma_desc(smem_u32(&sm.v[0][0][0]), 8 * 128, 2 * 8 * 128);  // 64-d chunks 1 KiB apart, groups of 8 keys 2
   if (!um_wait(&sm.q_full, 0, &sm.abort_flag, p.status)) return;
-  if (!u2_issue_s(sm, p, tmem, k_desc0, 0, 0, 0)) return;
-  int sv = 0, sk = 1 % kU2Stages;
-  uint32_t pv = 0, pk = 1 / kU2Stages;
+  auto scores = [&](int t) { return t >= n_tiles || u2_issue_s(sm, p, tmem, k_desc0, t, t % kU2Stages, (t / kU2Stages) & 1); };
+  if (!scores(0) || !scores(1)) return;
   for (int t = 0; t < n_tiles; ++t) {
-    if (t + 1 < n_tiles && !u2_issue_s(sm, p, tmem, k_desc0, t + 1, sk, pk)) return;
-    if (!um_wait(&sm.v_full[sv], pv, &sm.abort_flag, p.status)) return;
-    if (!um_wait(&sm.p_full, t & 1, &sm.abort_flag, p.status)) return;
-    tc_fence_after_sync();
-    if (um_elect_one()) {
-      constexpr uint32_t idesc = umma2_idesc(kD, true);
-      const uint64_t v_desc = v_desc0 + (uint64_t)((sv * (int)sizeof(sm.v[0])) >> 4);
+    if (!scores(t + 2)) return;
+    const int sv = t % kU2Stages;
+    if (!um_wait(&sm.v_full[sv], (t / kU2Stages) & 1, &sm.abort_flag, p.status)) return;
+    constexpr uint32_t idesc = umma2_idesc(kD, true);
+    const uint64_t v_desc = v_desc0 + (uint64_t)((sv * (int)sizeof(sm.v[0])) >> 4);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {  // 16 keys per MMA: 8 columns of P, two 8-key groups of V
-        const uint64_t dv = v_desc + (uint64_t)((kk * 4096) >> 4);
-        umma2_bf16_ts(tmem + kU2ColO, tmem + kU2ColP + kk * 8, dv, idesc, (t > 0 || kk > 0) ? 1u : 0u);
-        if (p.split_p) umma2_bf16_ts(tmem + kU2ColO, tmem + kU2ColP + 32 + kk * 8, dv, idesc, 1u);
+    for (int h = 0; h < 2; ++h) {  // 32 keys: their columns are free again while the other half is multiplied
+      if (!um_wait(&sm.p_full[h], t & 1, &sm.abort_flag, p.status)) return;
+      tc_fence_after_sync();
+      if (um_elect_one()) {
+#pragma unroll
+        for (int kk = 2 * h; kk < 2 * h + 2; ++kk) {  // 16 keys per MMA: 8 columns of P, two 8-key groups of V
+          const uint64_t dv = v_desc + (uint64_t)((kk * 4096) >> 4);
+          umma2_bf16_ts(tmem + kU2ColO, tmem + kU2ColP + kk * 8, dv, idesc, (t > 0 || kk > 0) ? 1u : 0u);
+          if (p.split_p) umma2_bf16_ts(tmem + kU2ColO, tmem + kU2ColP + 32 + kk * 8, dv, idesc, 1u);
+        }
+        umma2_commit_pair(smem_u32(&sm.pv_done[t & 1][h]));
+        if (h == 1) {
+          umma2_commit_pair(smem_u32(&sm.v_empty[sv]));
+          if (t == n_tiles - 1) umma2_commit_pair(smem_u32(&sm.o_full));
+        }
       }
-      umma2_commit_pair(smem_u32(&sm.v_empty[sv]));
-      umma2_commit_pair(smem_u32(&sm.pv_done));
+      __syncwarp();
     }
-    __syncwarp();
-    if (++sv == kU2Stages) { sv = 0; pv ^= 1u; }
-    if (++sk == kU2Stages) { sk = 0; pk ^= 1u; }
   }
 }
 
-// The walk over the key tiles for one softmax thread (row r, column half): scores out of tensor memory, mask, running
-// max shared with the other half, weights back into tensor memory.  False when a wait ran out (the caller still
-// joins its barriers).
+// The walk over the key tiles for one softmax thread (row r).  The eight warps are two groups that take the even and the odd tiles,
+// a thread a whole row of 64 scores: out of tensor memory, masked, weights back into tensor memory.  What a tile costs from its
+// scores to its weights (~2000 cycles: barriers, the trips to tensor memory, 64 exponentials per row) is longer than its products
+// (1640), so two tiles have to be on their way.  (With each tile shared by all eight warps, half a row per thread, a lone pair took
+// 2050 cycles per tile.)  What stays in turn is the row's reference (the running maximum, moved only when a tile exceeds it
+// by 2^kU2RescaleGap): a group settles its tile's reference behind the other's, before its exponentials.  False when a
+// wait ran out (the caller still joins its barriers).
 __device__ __forceinline__ bool u2_softmax_tiles(Umma2Smem& sm, const Umma2Params& p, uint32_t my_tmem, int tok0, int ntok,
-                                                 int kv_len, int tile0, int n_tiles, int half, int r, int token, float& m_row,
+                                                 int kv_len, int tile0, int n_tiles, int group, int r, int token, float& m_row,
                                                  float& l_row) {
   const int my_pos = token < ntok ? p.positions[tok0 + token] : -1;
   const int last_key = my_pos < kv_len - 1 ? my_pos : kv_len - 1;
   const float scale_log2 = p.scale * kU2Log2e;
-  for (int t = 0; t < n_tiles; ++t) {
-    const int b = t & 1;
-    if (!um_wait(&sm.s_full, t & 1, &sm.abort_flag, p.status)) return false;
+  const int quarter = r >> 5;
+  for (int t = group; t < n_tiles; t += 2) {
+    const uint32_t mine = (t >> 1) & 1, before = ((t - 1) >> 1) & 1;  // parities of this tile's and the tile before's barriers
+    if (!um_wait(&sm.s_full[group], mine, &sm.abort_flag, p.status)) return false;
     if (t == 0) NVJ_U2_PHASE(3);
     tc_fence_after_sync();
-    float s[32];
-    tmem_ld32(my_tmem + kU2ColS + half * 32, s);
+    float s[kU2Keys];
+    tmem_ld64(my_tmem + kU2ColS, s);
     tc_fence_before_sync();
     u2_arrive_warp(smem_u32(&sm.s_read));
-    const int lim = last_key - (tile0 + t) * kU2Keys - half * 32;
-    float hmax = -INFINITY;
-    if (lim >= 31) {
+    const int lim = last_key - (tile0 + t) * kU2Keys;
+    float tmax = -INFINITY;
+    if (lim >= kU2Keys - 1) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) hmax = fmaxf(hmax, fmaxf(s[i], s[i + 1]));
+      for (int i = 0; i < kU2Keys; i += 2) tmax = fmaxf(tmax, fmaxf(s[i], s[i + 1]));
     } else {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) { s[i] = i <= lim ? s[i] : -INFINITY; hmax = fmaxf(hmax, s[i]); }
+      for (int i = 0; i < kU2Keys; ++i) { s[i] = i <= lim ? s[i] : -INFINITY; tmax = fmaxf(tmax, s[i]); }
     }
-    sm.xchg[b][half][r] = hmax;
-    __syncwarp();
-    if ((r & 31) == 0) mbar_arrive(smem_u32(&sm.x_full[r >> 5]));
-    if (!um_wait(&sm.x_full[r >> 5], t & 1, &sm.abort_flag, p.status)) return false;
-    const float tmax = fmaxf(hmax, sm.xchg[b][half ^ 1][r]) * scale_log2;  // scale > 0
-    if (t == 0) {
-      m_row = tmax;
-    } else if (__any_sync(0xffffffffu, tmax > m_row + kU2RescaleGap)) {
-      if (!um_wait(&sm.pv_done, (t - 1) & 1, &sm.abort_flag, p.status)) return false;
-      tc_fence_after_sync();
-      const float m_new = fmaxf(m_row, tmax);
-      const float f = m_new == -INFINITY ? 1.f : ex2_approx(m_row - m_new);
-      m_row = m_new;
-      l_row *= f;
+    tmax *= scale_log2;  // scale > 0
+    float m_new = tmax;
+    if (t > 0) {
+      if (!um_wait(&sm.m_full[quarter][group ^ 1], before, &sm.abort_flag, p.status)) return false;
+      m_new = sm.m_row[group ^ 1][r];
+      if (__any_sync(0xffffffffu, tmax > m_new + kU2RescaleGap)) {
+        if (!um_wait(&sm.pv_done[group ^ 1][1], before, &sm.abort_flag, p.status)) return false;
+        tc_fence_after_sync();
+        const float m_old = m_new;
+        m_new = fmaxf(m_old, tmax);
+        const float f = m_new == -INFINITY ? 1.f : ex2_approx(m_old - m_new);
 #pragma unroll 1
-      for (int cc = 0; cc < kD / 64; ++cc) {
-        float o[32];
-        tmem_ld32(my_tmem + kU2ColO + half * (kD / 2) + cc * 32, o);
+        for (int cc = 0; cc < kD / 32; ++cc) {
+          float o[32];
+          tmem_ld32(my_tmem + kU2ColO + cc * 32, o);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] *= f;
-        tmem_st32(my_tmem + kU2ColO + half * (kD / 2) + cc * 32, o);
+          for (int i = 0; i < 32; ++i) o[i] *= f;
+          tmem_st32(my_tmem + kU2ColO + cc * 32, o);
+        }
       }
     }
+    if (t + 1 < n_tiles) {  // the other group's next tile
+      sm.m_row[group][r] = m_new;
+      __syncwarp();
+      if ((r & 31) == 0) mbar_arrive(smem_u32(&sm.m_full[quarter][group]));
+    }
+    if (m_new != m_row) {  // (this group's first tile included: no weights so far)
+      l_row *= m_new == -INFINITY ? 1.f : ex2_approx(m_row - m_new);
+      m_row = m_new;
+    }
     const float neg_m = m_row == -INFINITY ? 0.f : -m_row;
-    uint32_t hi[16], lo[16];
+    uint32_t hi[2][16], lo[2][16];
     const float2 c2 = make_float2(scale_log2, scale_log2), m2 = make_float2(neg_m, neg_m);
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {  // two keys at a time, packed fp32 arithmetic
+    for (int e = 0; e < kU2Keys / 2; ++e) {  // two keys at a time, packed fp32 arithmetic
       float2 w = fma2(make_float2(s[2 * e], s[2 * e + 1]), c2, m2);
       w.x = ex2_approx(w.x);
       w.y = ex2_approx(w.y);
@@ -306,17 +327,18 @@ __device__ __forceinline__ bool u2_softmax_tiles(Umma2Smem& sm, const Umma2Param
       const __nv_bfloat162 h = __floats2bfloat162_rn(w.x, w.y);
       const float2 rest = fma2(make_float2(__low2float(h), __high2float(h)), make_float2(-1.f, -1.f), w);  // exact
       const __nv_bfloat162 g = __floats2bfloat162_rn(rest.x, rest.y);
-      hi[e] = *reinterpret_cast<const uint32_t*>(&h);
-      lo[e] = *reinterpret_cast<const uint32_t*>(&g);
+      hi[e >> 4][e & 15] = *reinterpret_cast<const uint32_t*>(&h);
+      lo[e >> 4][e & 15] = *reinterpret_cast<const uint32_t*>(&g);
     }
-    // P V of the tile before has read its weights; every phase of pv_done is observed in turn (parity waits tell only two phases
-    // apart)
-    if (t >= 1 && !um_wait(&sm.pv_done, (t - 1) & 1, &sm.abort_flag, p.status)) return false;
-    tmem_st16(my_tmem + kU2ColP + half * 16, hi);
-    if (p.split_p) tmem_st16(my_tmem + kU2ColP + 32 + half * 16, lo);
-    tmem_st_wait();
-    tc_fence_before_sync();
-    u2_arrive_warp(smem_u32(&sm.p_full));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // as soon as P V of the tile before has read this half of its weights
+      if (t >= 1 && !um_wait(&sm.pv_done[group ^ 1][h], before, &sm.abort_flag, p.status)) return false;
+      tmem_st16(my_tmem + kU2ColP + h * 16, hi[h]);
+      if (p.split_p) tmem_st16(my_tmem + kU2ColP + 32 + h * 16, lo[h]);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      u2_arrive_warp(smem_u32(&sm.p_full[h]));
+    }
   }
   return true;
 }
@@ -404,16 +426,16 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
   // ---- epilogue.  From here on the softmax threads meet at CTA-wide named barriers, so a thread whose wait ran out
   // does not leave: it skips the work and everybody returns together once the barrier has made the flag visible.
   NVJ_U2_PHASE(4);
-  if (alive) {
-    sm.xchg[n_tiles & 1][half][r] = l_row;
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&sm.x_full[quarter]));
-    alive = um_wait(&sm.x_full[quarter], n_tiles & 1, &sm.abort_flag, p.status);
+  sm.sums[half][r] = make_float2(m_row, l_row);
+  named_bar_sync(2 + quarter, 64);  // the quarter's two warps
+  {  // the last tile's group holds the row's reference (they grow); the other's sum comes to it
+    const float2 other = sm.sums[half ^ 1][r];
+    const float m = fmaxf(m_row, other.x);
+    const float mine = m == -INFINITY ? 0.f : ex2_approx(m_row - m) * l_row, others = m == -INFINITY ? 0.f : ex2_approx(other.x - m) * other.y;
+    m_row = m;
+    l_row = half == 0 ? mine + others : others + mine;  // (the same in both)
   }
-  if (alive) {
-    l_row += sm.xchg[n_tiles & 1][half ^ 1][r];
-    alive = um_wait(&sm.pv_done, (n_tiles - 1) & 1, &sm.abort_flag, p.status);
-  }
+  if (alive) alive = um_wait(&sm.o_full, 0, &sm.abort_flag, p.status);
   tc_fence_after_sync();
   const float inv = splits > 1 ? 1.f : (l_row > 0.f ? 1.f / l_row : 0.f);  // a split leaves its rows un-normalised
   if (splits > 1 && half == 0) sm.own_ml[r] = make_float2(m_row, l_row);
@@ -508,22 +530,24 @@ __device__ __forceinline__ void u2_fold_splits(const Umma2Smem& sm, const Umma2P
 }
 
 // Which (table row, 32-token tile) the CTA with cluster index `cluster` of `clusters` and rank `rank` serves: the
-// heaviest pairs (the last tokens of a row see the most keys) get the lowest cluster indices.  One warp runs this, 32 rows
+// heaviest pairs (the last tokens of a row see the most keys) get the lowest cluster indices.  Every warp runs this for itself, 32 rows
 // at a time (one thread walking the rows paid a trip to the L2 for each: 7 of 24 us on a batch of 32 decode rows and two
-// chunks).  row < 0: no tile (`idle` then numbers the clusters beyond the last pair 0, 1, ...).  `total` (the batch's
-// number of pairs) is complete only when `need_total`.
+// chunks); a row's length and whether any is long enough to be split come with the same trip.  row < 0: no tile (`idle` then numbers
+// the clusters beyond the last pair 0, 1, ...).  `total` (the batch's number of pairs) and `any_long` are complete only when `need_total`.
 struct U2Tile {
-  int row, tok0, ntok, pair_last_tok, idle, total;
+  int row, tok0, ntok, pair_last_tok, kv_len, idle, total;
+  bool any_long;
 };
 __device__ __forceinline__ U2Tile u2_find_tile(const Umma2Params& p, int cluster, int clusters, int rank, bool need_total, int lane) {
-  U2Tile t{-1, 0, 0, 0, -1, 0};
+  U2Tile t{-1, 0, 0, 0, 0, -1, 0, false};
   int idx = clusters - 1 - cluster;
   for (int base = 0; base < p.rows && (need_total || t.row < 0); base += 32) {
     const int r = base + lane;
-    int lo = 0, hi = 0, pairs = 0;
+    int lo = 0, hi = 0, pairs = 0, len = 0;
     if (r < p.rows) {
       lo = p.query_start_loc[r];
       const int end = p.query_start_loc[r + 1];
+      len = p.kv_lens[r];
       hi = end < p.token_bucket ? end : p.token_bucket;
       pairs = hi > lo ? (hi - lo + 2 * kU2Tokens - 1) / (2 * kU2Tokens) : 0;
       if (p.skip_single && end - lo == 1) pairs = 0;
@@ -536,6 +560,7 @@ __device__ __forceinline__ U2Tile u2_find_tile(const Umma2Params& p, int cluster
     }
     const int group = __shfl_sync(0xffffffffu, incl, 31);
     t.total += group;
+    if (need_total) t.any_long |= __any_sync(0xffffffffu, len > (kU2SplitFrom - 1) * kU2Keys) != 0;
     if (t.row >= 0) continue;
     const unsigned hit = __ballot_sync(0xffffffffu, idx >= incl - pairs && idx < incl);
     if (hit == 0) {
@@ -545,6 +570,7 @@ __device__ __forceinline__ U2Tile u2_find_tile(const Umma2Params& p, int cluster
     const int at = __ffs(hit) - 1;
     const int row_lo = __shfl_sync(0xffffffffu, lo, at), row_hi = __shfl_sync(0xffffffffu, hi, at);
     const int pair = idx - __shfl_sync(0xffffffffu, incl - pairs, at);
+    t.kv_len = __shfl_sync(0xffffffffu, len, at);
     t.row = base + at;
     t.tok0 = row_lo + (2 * pair + rank) * kU2Tokens;
     t.ntok = row_hi - t.tok0 < kU2Tokens ? row_hi - t.tok0 : kU2Tokens;
@@ -556,17 +582,13 @@ __device__ __forceinline__ U2Tile u2_find_tile(const Umma2Params& p, int cluster
   return t;
 }
 // Key tiles of the pair (warp-collective; the same in every warp of both CTAs): the token of the pair that sees the most
-// keys bounds the key range (positions need not grow along the tiles).  `kv_len` comes back clipped to the table.
-__device__ __forceinline__ int u2_key_tiles(const Umma2Params& p, int row, int tok0, int rank, int pair_last_tok, int lane,
-                                            int& kv_len, bool flag) {
-  kv_len = p.kv_lens[row];
-  if (kv_len > p.table_width * kBlk) {
-    if (flag) atomicOr(p.status, NVJ_DEV_BAD_LENGTH);
-    kv_len = p.table_width * kBlk;
-  }
-  const int pair_tok0 = tok0 - rank * kU2Tokens, pair_n = pair_last_tok - pair_tok0 + 1;
-  int seen = lane < pair_n ? p.positions[pair_tok0 + lane] : -1;
-  if (lane + 32 < pair_n) seen = max(seen, p.positions[pair_tok0 + lane + 32]);
+// keys bounds the key range (positions need not grow along the tiles).  `seen`: the larger position of this lane's two tokens.
+__device__ __forceinline__ int u2_last_positions(const Umma2Params& p, const U2Tile& t, int rank, int lane) {
+  const int tok0 = t.tok0 - rank * kU2Tokens, n = t.pair_last_tok - tok0 + 1;
+  const int a = lane < n ? ld_in_turn(p.positions + tok0 + lane) : -1, b = lane + 32 < n ? ld_in_turn(p.positions + tok0 + lane + 32) : -1;
+  return a > b ? a : b;
+}
+__device__ __forceinline__ int u2_key_tiles(int seen, int kv_len) {
   const int max_pos = __reduce_max_sync(0xffffffffu, seen);
   const int key_end = kv_len < max_pos + 1 ? kv_len : max_pos + 1;
   return key_end > 0 ? (key_end + kU2Keys - 1) / kU2Keys : 0;
@@ -593,6 +615,10 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   NVJ_U2_NOTE(7, 0ull);
   // The pair's barriers are set up before anything is read: this runs while the kernel in front (the append of the same
   // tokens, usually) is still at work.
+  if (threadIdx.x == 32) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&k_map)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&v_map)) : "memory");
+  }
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&sm.q_full), 2 * kU2SoftmaxThreads / 32);
     for (int i = 0; i < kU2Stages; ++i) {
@@ -601,11 +627,16 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
       mbar_init(smem_u32(&sm.k_empty[i]), 1);
       mbar_init(smem_u32(&sm.v_empty[i]), 1);
     }
-    mbar_init(smem_u32(&sm.s_full), 1);
-    mbar_init(smem_u32(&sm.s_read), 2 * kU2SoftmaxThreads / 32);
-    mbar_init(smem_u32(&sm.p_full), 2 * kU2SoftmaxThreads / 32);
-    mbar_init(smem_u32(&sm.pv_done), 1);
-    for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&sm.x_full[i]), 2);
+    mbar_init(smem_u32(&sm.s_read), kU2SoftmaxThreads / 32);  // one group of each CTA
+    mbar_init(smem_u32(&sm.o_full), 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&sm.s_full[i]), 1);
+      mbar_init(smem_u32(&sm.p_full[i]), kU2SoftmaxThreads / 32);
+      mbar_init(smem_u32(&sm.pv_done[i][0]), 1);
+      mbar_init(smem_u32(&sm.pv_done[i][1]), 1);
+      for (int q = 0; q < 4; ++q) mbar_init(smem_u32(&sm.m_full[q][i]), 1);
+    }
+    sm.abort_flag = 0;
     mbar_fence_init();
   }
   cl_sync();  // the peer's barriers exist before anything is sent to them (this barrier covers the CTA's own threads)
@@ -623,27 +654,14 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     cl_sync();
     if (warp == 1) tmem2_dealloc(sm.tmem_base, kU2TmemCols);
   };
-  if (blockIdx.z > 0) {  // the extra splits leave at once when no row's key range is long enough to be split
-    int any = 0;
-    for (int rr = threadIdx.x; rr < p.rows; rr += kU2Threads) any |= p.kv_lens[rr] > (kU2SplitFrom - 1) * kU2Keys ? 1 : 0;
-    if (!__syncthreads_or(any)) return leave();
-  }
 
-  // ---- which (table row, pair of 32-token tiles) this cluster serves; both CTAs compute the same
-  if (warp == 0) {
-    const U2Tile t = u2_find_tile(p, blockIdx.x >> 1, gridDim.x >> 1, rank, gridDim.z > 1, lane);
-    if (lane == 0) {
-      sm.row = t.row; sm.tok0 = t.tok0; sm.ntok = t.ntok; sm.pair_last_tok = t.pair_last_tok; sm.abort_flag = 0;
-      sm.total_pairs = t.total; sm.idle_index = t.idle;
-    }
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const int row = sm.row, tok0 = sm.tok0, ntok = sm.ntok;
+  // ---- which (table row, pair of 32-token tiles) this cluster serves; every warp of its CTAs computes the same
+  const U2Tile tile = u2_find_tile(p, blockIdx.x >> 1, gridDim.x >> 1, rank, gridDim.z > 1, lane);
+  const int row = tile.row, tok0 = tile.tok0, ntok = tile.ntok;
+  if (blockIdx.z > 0 && !tile.any_long) return leave();  // no row's key range is long enough to be split
   if (p.counted && blockIdx.x == 0 && row >= 0 && threadIdx.x == 0) atomicOr(p.status, NVJ_DEV_BAD_LENGTH);
   if (row < 0) {
-    if (p.zero_fill && sm.idle_index == 0 && blockIdx.z == 0) {
+    if (p.zero_fill && tile.idle == 0 && blockIdx.z == 0) {
       // the first idle cluster (there is always one) zeroes the padding tokens, a quarter per CTA of the cluster pair x KV head
       int real = p.query_start_loc[p.rows];
       real = real < p.token_bucket ? real : p.token_bucket;
@@ -656,15 +674,23 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     return leave();
   }
 
-  // the query rows, and the block ids of the producer's first eight tiles where those do not depend on the number of splits, are
-  // asked for together with what bounds the key range
+  // What bounds the key range, the row's first 128 block ids (the producer's first eight tiles are among them, mostly, whichever split this
+  // is) and the query rows are asked for together, and in this order: behind the 64 KiB of queries the few positions came 0.5 us later.
+  const int seen = u2_last_positions(p, tile, rank, lane);
+  int early_ids[4] = {-1, -1, -1, -1};
+  if (warp == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i * 32 + lane < p.table_width && (i == 0 || gridDim.z > 1)) early_ids[i] = ld_in_turn(p.block_tables + (long long)row * p.table_width + i * 32 + lane);
+  }
   uint4 qv[4][4];
   if (warp >= 2 && p.q_dtype == NVJ_BF16) u2_request_q(p, tok0, ntok, kvh, warp, lane, qv);
-  int first_ids = -1;
-  if (warp == 0 && gridDim.z == 1 && lane < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + lane];
-
-  int kv_len;
-  const int n_tiles = u2_key_tiles(p, row, tok0, rank, sm.pair_last_tok, lane, kv_len, threadIdx.x == 0 && rank == 0);
+  int kv_len = tile.kv_len;
+  if (kv_len > p.table_width * kBlk) {
+    if (threadIdx.x == 0 && rank == 0) atomicOr(p.status, NVJ_DEV_BAD_LENGTH);
+    kv_len = p.table_width * kBlk;
+  }
+  const int n_tiles = u2_key_tiles(seen, kv_len);
   if (n_tiles == 0) {  // same decision in both CTAs; a row without keys produces zeros
     if (p.zero_fill && blockIdx.z == 0) {
       for (int i = threadIdx.x; i < ntok * kG * (kD / 4); i += kU2Threads) {
@@ -679,7 +705,7 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   // leave pair slots for; the splits beyond that have nothing to do (all CTAs of the cluster decide alike).
   int splits = 1, tile0 = 0, my_tiles = n_tiles;
   if (gridDim.z > 1) {
-    splits = u2_split_count(p, n_tiles, sm.total_pairs, (int)gridDim.z);
+    splits = u2_split_count(p, n_tiles, tile.total, (int)gridDim.z);
     if ((int)blockIdx.z >= splits) {
       if (splits > 1) cl_sync();  // the others' barrier in front of their fold
       return leave();
@@ -688,12 +714,26 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     my_tiles = ((int)blockIdx.z + 1) * n_tiles / splits - tile0;
   }
 
-  if (warp == 0 && gridDim.z > 1) {
+  int first_ids = early_ids[0];
+  if (warp == 0 && tile0 > 0) {
     const int bi = tile0 * 4 + lane;
-    if (bi < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + bi];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int id = __shfl_sync(0xffffffffu, early_ids[i], bi & 31);
+      if (bi >> 5 == i) first_ids = id;
+    }
+    if (bi >= 128 && bi < p.table_width) first_ids = p.block_tables[(long long)row * p.table_width + bi];
   }
-
-  const uint32_t tmem = sm.tmem_base;
+  // The tensor memory's address goes from warp 1 to the softmax warps, which have their queries on the way; the producer, which
+  // needs neither, is not held up (behind a barrier of the whole CTA its first copies went out 0.6 us later).
+  if (warp == 1) {
+    tc_fence_before_sync();
+    asm volatile("bar.arrive %0, %1;" ::"r"(6), "r"(kU2SoftmaxThreads + 32) : "memory");
+  } else if (warp >= 2) {
+    named_bar_sync(6, kU2SoftmaxThreads + 32);
+    tc_fence_after_sync();
+  }
+  const uint32_t tmem = sm.tmem_base;  // (not used by warp 0)
   NVJ_U2_PHASE(1);
   NVJ_U2_NOTE(7, (unsigned long long)my_tiles);
 
@@ -712,7 +752,9 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     const unsigned long long t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
-  cl_sync();  // CTA 0's MMAs read this CTA's shared and tensor memory until its last commit; the other splits its rows
+  // CTA 0's MMAs read this CTA's shared and tensor memory until its last commit; the other splits its rows (their loads have returned
+  // what they stored).  Nobody reads another's output, so nobody waits for its stores to arrive.
+  cl_sync_relaxed();
   NVJ_U2_PHASE(6);
   if (warp == 1) tmem2_dealloc(tmem, kU2TmemCols);
 }

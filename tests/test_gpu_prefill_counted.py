@@ -91,3 +91,31 @@ def test_key_ranges_stay_whole_where_the_caller_says_so(monkeypatch, route):
     assert not torch.equal(whole, split) and float((whole - split).abs().max()) <= 2e-3
     monkeypatch.setenv("NVJ_PREFILL_KEY_SPLITS", "0")
     assert torch.equal(run(2).view(torch.int32), whole.view(torch.int32))
+
+
+# 1 - 10 key tiles (one and two of them per softmax group, odd and even numbers), key ranges whole and split, splits that begin behind the
+# row's first 128 blocks; keys that grow by more than the rescale gap from every tile to the next, shrink, or neither
+@pytest.mark.parametrize("growth", [0.0, 3.0, -3.0])
+@pytest.mark.parametrize("qlens,cached", [((64,), (0,)), ((40, 64, 2), (64, 128, 190)), ((64, 33), (250, 300)), ((64,), (576,)), ((17,), (2900,)),
+                                          ((64,) * 24, (37,) * 12 + (290,) * 12)])
+def test_tiles_taken_in_turn_follow_the_rows_maximum(qlens, cached, growth, monkeypatch):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    q, (k, v), tables, lens, pos, rid, qsl = _batch(qlens, cached, 0, sum(qlens))
+    for r, n in enumerate(lens.tolist()):
+        blocks = tables[r, :-(-n // BS)].long()
+        tile = torch.arange(len(blocks), device="cuda") // 4
+        size = 1 + abs(growth) * (tile if growth > 0 else tile.max() - tile).clamp(max=10)
+        k[0, blocks] = (k[0, blocks].float() * size[:, None, None, None]).to(torch.bfloat16)
+    ref = torch.zeros(q.shape[1], 8, 256, dtype=torch.float64, device="cuda")
+    for r, n in enumerate(lens.tolist()):
+        a, b = qsl[r].item(), qsl[r + 1].item()
+        keys, values = (c[0, tables[r].long()].double().reshape(-1, 2, 256)[:n].repeat_interleave(4, 1) for c in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q[0, a:b].double(), keys) * SCALE
+        s.masked_fill_(torch.arange(n, device="cuda") > pos[0, a:b, None], float("-inf"))
+        ref[a:b] = torch.einsum("hqk,khd->qhd", s.softmax(-1), values)
+    args = (q, k[0], v[0], tables, lens, pos, qsl, BS, SCALE, 4)
+    for splits in ("1", "0"):
+        monkeypatch.setenv("NVJ_PREFILL_KEY_SPLITS", splits)
+        out = K.packed_paged_prefill_attention(*args, num_decode_rows=0, query_tile_pairs=sum(-(-n // 64) for n in qlens))
+        # scores of up to ~130 natural units carry 2^-21 of rounding of their 256 products' sum: 1e-4 of a weight, values below 6
+        assert float((out[0].reshape(-1, 8, 256).double() - ref).abs().max()) <= 2e-3
