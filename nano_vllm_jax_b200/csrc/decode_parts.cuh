@@ -134,7 +134,11 @@ struct Partition {
   long long total;
   int n;
 
-  __device__ __forceinline__ long long start(int c) const { return (long long)c * total / n; }
+  // (a division of 64-bit numbers takes five times as long as one of 32 bits)
+  __device__ __forceinline__ long long start(int c) const {
+    const unsigned long long x = (unsigned long long)c * total;
+    return x >> 32 ? (long long)(x / n) : (long long)((unsigned)x / (unsigned)n);
+  }
   // The CTA whose range holds global block g (the last CTA whose start is <= g).
   __device__ __forceinline__ int cta_of(long long g) const { return (int)(((g + 1) * n - 1) / total); }
 };
@@ -147,6 +151,74 @@ __device__ __forceinline__ Partition make_partition(long long total, int grid) {
   const long long cap = (total + kMinBlocksPerCta - 1) / kMinBlocksPerCta;
   pt.n = cap < grid ? (int)cap : grid;
   return pt;
+}
+
+// While the rest of the CTA waits for the kernel in front, whose CTAs do not all end together (an attention launch's last folds take
+// 6 - 8 us, an append 2, in which memory is idle): the first `blocks` (at most 32) of the CTA's range on their way into the L2, K or V or both, by
+// a warp that has nothing else to do.  What it reads may be about to change, so it is a hint and nothing else: relaxed loads (they
+// leave no line in the L1 that a load behind the wait could find), lengths and ids checked, prefetches.  It ends as soon as the wait has
+// (`begun`), so that behind a kernel that has long ended it costs nothing (8 rows of 8192 - 32768 keys behind a torch kernel 63.9 :
+// 63.6 us).  Batches of up to kAheadRows rows.  The mma.sync form for 2 - 4 tokens, which the power limit slows, has no use for it (128 rows of 2
+// tokens 115.5 without, 117.5 with).  (The range found by every warp like this instead of by a scan over the CTA, behind the
+// wait as well: 0.2 us later.)
+constexpr int kAheadRows = 256;
+// Whether a call's CTAs do so (DecodeParams::early_ctas): a cap by positions, a page list per row or a packed batch is not looked through.
+inline int ahead_ctas(const DecodeParams& p, int ctas) {
+  return p.kv_indptr || p.packed_rows || p.cap_positions || p.batch > kAheadRows ? 0 : ctas;
+}
+__device__ __forceinline__ void prefetch_ahead(const DecodeParams& p, int range, int ranges, int blocks, bool k, bool v,
+                                               volatile int* begun, int lane) {
+  auto blocks_of = [&](int b) {
+    int len = ld_relaxed_gpu(p.seq_lens + b);
+    len = len > 0 && p.pre_append ? len + 1 : len;
+    len = p.max_len > 0 && p.max_len < len ? p.max_len : len;
+    const int nb = len > 0 ? (len - 1) / kBlk + 1 : 0;
+    return nb < p.table_width ? nb : p.table_width;
+  };
+  int n[kAheadRows / 32], total = 0;
+#pragma unroll
+  for (int i = 0; i < kAheadRows / 32; ++i) n[i] = i * 32 + lane < p.batch ? blocks_of(i * 32 + lane) : 0;
+#pragma unroll
+  for (int i = 0; i < kAheadRows / 32; ++i) {
+    n[i] = blocks_in_sequence(p, n[i]);
+    total += n[i];
+  }
+  total = (int)__reduce_add_sync(kFullMask, (unsigned)total);
+  if (total <= 0 || *begun) return;
+  const Partition pt = make_partition(total, ranges);
+  if (range >= pt.n) return;
+  const int g1 = (int)pt.start(range + 1);
+  int g = (int)pt.start(range), row = p.batch, j = 0, carry = 0;
+#pragma unroll
+  for (int i = 0; i < kAheadRows / 32; ++i) {
+    if (i * 32 >= p.batch) break;
+    int incl = n[i];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(kFullMask, incl, o);
+      if (lane >= o) incl += x;
+    }
+    const int at = carry + incl - n[i];
+    const unsigned hit = __ballot_sync(kFullMask, n[i] > 0 && at <= g && g < at + n[i]);
+    if (hit) {
+      row = i * 32 + __ffs(hit) - 1;
+      j = g - __shfl_sync(kFullMask, at, __ffs(hit) - 1);
+    }
+    carry += __shfl_sync(kFullMask, incl, 31);
+  }
+  for (int left = blocks; left > 0 && g < g1 && row < p.batch && !*begun; ++row, j = 0) {
+    const int nb = blocks_of(row), room = g1 - g < left ? g1 - g : left;
+    const int take = nb - j < room ? nb - j : room;
+    if (lane < take) {
+      const int id = ld_relaxed_gpu(p.block_tables + (long long)row * p.table_width + j + lane);
+      if (id >= 0 && id < p.num_blocks) {
+        if (k) l2_prefetch(p.k_cache + (long long)id * kTileBytes, kTileBytes);
+        if (v) l2_prefetch(p.v_cache + (long long)id * kTileBytes, kTileBytes);
+      }
+    }
+    left -= take > 0 ? take : 0;
+    g += blocks_in_sequence(p, nb) - j;
+  }
 }
 
 // What the tcgen05 wide kernels tell the launch that folds their partials: per range, the row that its beginning cuts first (its blocks
@@ -267,6 +339,15 @@ __device__ __forceinline__ void fold_parts(const DecodeParams& p, float* red, in
   }
 }
 
+// Counts one in.  What the CTA has stored before the barrier in front of this is released, and what others have counted in is acquired
+// for the threads behind the next barrier: one fence by one thread, where a __threadfence() of all threads on either side took
+// longer (8 rows of 8192 - 32768 keys 56.5 -> 56.2 us, one of 20000 18.2 -> 17.4).
+__device__ __forceinline__ int count_in(int32_t* counter) {
+  int before;
+  asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+  return before;
+}
+
 // A row that several CTAs share, once this CTA (its kDecodeThreads threads, all of which call it) has stored its partial: counts
 // the partial in; the CTA that delivers the row's last one folds them all, token by token, in two levels when there are many.
 // `qbase`: the row's first query token in the output.  `red` is the fold's scratch, `last_flag` a word of shared memory.
@@ -283,12 +364,10 @@ __device__ __forceinline__ void finish_shared_row(const DecodeParams& p, float* 
   const int first = tree ? max(c_lo, cg * kMergeGroup) : c_lo;
   const int last = tree ? min(c_hi, cg * kMergeGroup + kMergeGroup - 1) : c_hi;
   int32_t* counter = tree ? p.group_counters + 2 * cg + (cg == g_lo ? 1 : 0) : p.counters + s.b;
-  __threadfence();
   named_bar_sync(1, kDecodeThreads);
-  if (tid == 0) last_flag = (atomicAdd(counter, 1) == last - first) ? 1 : 0;
+  if (tid == 0) last_flag = (count_in(counter) == last - first) ? 1 : 0;
   named_bar_sync(1, kDecodeThreads);
   if (!last_flag) return;
-  __threadfence();
   if (!tree) {
     for (int tok = 0; tok < p.width; ++tok) {
       fold_parts<true, kBatch>(p, red, tid, 0, c_lo, c_lo, c_hi - c_lo + 1, (qbase + tok) * kHq, slot_rows, tok * kHq);
@@ -303,12 +382,9 @@ __device__ __forceinline__ void finish_shared_row(const DecodeParams& p, float* 
     named_bar_sync(1, kDecodeThreads);
   }
   if (tid == 0) *counter = 0;
-  __threadfence();
-  named_bar_sync(1, kDecodeThreads);
-  if (tid == 0) last_flag = (atomicAdd(p.counters + s.b, 1) == g_hi - g_lo) ? 1 : 0;
+  if (tid == 0) last_flag = (count_in(p.counters + s.b) == g_hi - g_lo) ? 1 : 0;
   named_bar_sync(1, kDecodeThreads);
   if (!last_flag) return;
-  __threadfence();
   for (int tok = 0; tok < p.width; ++tok) {
     fold_parts<true, kBatch>(p, red, tid, 2LL * grid, g_lo, g_lo, g_hi - g_lo + 1, (qbase + tok) * kHq, slot_rows, tok * kHq);
     named_bar_sync(1, kDecodeThreads);

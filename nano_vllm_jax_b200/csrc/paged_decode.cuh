@@ -58,8 +58,8 @@ struct DecodeParams {
   // in front like any other.  The launch ends only after the kernel in front has, so that the stream's order holds behind
   // both, and leaves the word zero.
   int32_t* beside;
-  // cluster kernel: the launch's first so many CTAs, those that find a place together, prefetch ahead of pdl_wait()
-  // (cm_prefetch_block); set by its launcher
+  // the launch's first so many CTAs, those that find a place together, prefetch ahead of pdl_wait() (cm_prefetch_block,
+  // prefetch_ahead); set by the launchers
   int early_ctas;
   // token pick in the same launch (nullable; pre-append form on the cluster kernel only, decode_cluster_picks): the index of the
   // row's first largest output value goes to pick_tokens[b], and the row's resident metadata is advanced as advance_row does

@@ -48,6 +48,11 @@ static_assert(kDecodeThreads * kStConsumerRegs + 128 * kStProducerRegs <= kStThr
 constexpr int kStPitch = kD + 4;  // floats between the heads of a warp's sums: conflict-free stores
 constexpr int kStRowEndCost = 9;  // blocks that a row end costs a CTA (decode_parts.cuh): 32 rows of 512 - 4096 keys 34.1 us with 1, 33.3 with 6, 32.5 with 9
 
+// Blocks of a CTA's range that are prefetched ahead of the wait (prefetch_ahead).  Passes back to back without it : with it: 8 rows of 8192 -
+// 32768 keys 61.4 : 56.5 us, one row of 20000 19.4 : 18.2, 24 of 4096 - 16384 82.0 : 78.4, 32 of 2000 - 8000 59.2 : 54.4, 128 of 8192 - 32768
+// 770 : 764.  With six blocks the first 57.2, with 18 57.2, with 26 58.1.
+constexpr int kStAheadBlocks = 12;
+
 struct StreamSmem {
   alignas(1024) char tiles[kStWalkers][kStSlots][kTileBytes];
   union {
@@ -58,7 +63,7 @@ struct StreamSmem {
   alignas(8) unsigned long long full_bar[kStWalkers][kStSlots], empty_bar[kStWalkers][kStSlots];
   int in_pool[kStWalkers][kStSlots];  // whether the slot's block lies in the pool (read with K)
   int scan[16];
-  int start_b, start_j, is_last, abort_flag;
+  int start_b, start_j, is_last, abort_flag, begun;
 };
 
 // A position in one walker's ring.
@@ -355,10 +360,13 @@ decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
         mbar_init(smem_u32(&sm.empty_bar[w][i]), kHkv);
       }
     mbar_fence_init();
-    sm.start_b = p.batch; sm.start_j = 0; sm.abort_flag = 0; sm.is_last = 0;
+    sm.start_b = p.batch; sm.start_j = 0; sm.abort_flag = 0; sm.is_last = 0; sm.begun = 0;
   }
+  __syncthreads();
+  if (warp == kDecodeThreads / 32 + 1 && p.early_ctas > 0) prefetch_ahead(p, blockIdx.x, grid, kStAheadBlocks, true, true, &sm.begun, lane);
   pdl_wait();
   pdl_release();
+  if (threadIdx.x == 0) *static_cast<volatile int*>(&sm.begun) = 1;
   if (!p.kv_indptr && counts) {
     const long long lines = ((long long)p.batch * p.table_width * (long long)sizeof(int32_t) + 127) / 128;
     const long long line = (long long)blockIdx.x * kDecodeThreads + threadIdx.x;
@@ -447,6 +455,7 @@ int launch_decode_stream(const DecodeParams& p, cudaStream_t stream) {
                cudaFuncSetAttribute(decode_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess;
       }))
     return NVJ_ERR_LAUNCH;
+  q.early_ctas = ahead_ctas(q, n);
   auto* kernel = q.max_len > 0 || q.cap_positions ? decode_stream_kernel<true> : decode_stream_kernel<false>;
   launch_after(kernel, n, kStThreads, kSmemBytes, stream, k_map, v_map, q);
   return cudaGetLastError() == cudaSuccess ? NVJ_OK : NVJ_ERR_LAUNCH;

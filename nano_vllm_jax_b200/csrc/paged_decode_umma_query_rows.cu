@@ -31,6 +31,7 @@ namespace query_rows {
 
 constexpr int kUdStages = 3;      // tiles (K and V of one KV head for up to 64 keys: 64 KiB) in flight
 constexpr int kUdTileBlocks = 4;  // blocks per tile: 64 keys
+constexpr int kUdAheadBlocks = 28;  // prefetched ahead of the wait, as in paged_decode_umma.cu
 constexpr int kUdTmemCols = 512;
 constexpr int kUdColQ = 0;        // query rows as the A operand: 256 bf16 per row = 128 columns
 constexpr int kUdColS = 128;      // scores of a tile
@@ -46,7 +47,7 @@ struct UdSmem {
       q_full, q_free, s_full, s_read, p_full, pv_done, o_ready[2], o_free;
   float inv[64];  // per query row: what the segment's output is scaled by
   int scan[16];
-  int start_b, start_j, abort_flag;
+  int start_b, start_j, abort_flag, begun;
   uint32_t tmem_base;
 };
 
@@ -374,7 +375,7 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&k_map)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&v_map)) : "memory");
-    sm.start_b = p.batch; sm.start_j = 0; sm.abort_flag = 0;
+    sm.start_b = p.batch; sm.start_j = 0; sm.abort_flag = 0; sm.begun = 0;
     for (int i = 0; i < kUdStages; ++i) {
       mbar_init(smem_u32(&sm.k_full[i]), 1);
       mbar_init(smem_u32(&sm.k_empty[i]), 1);
@@ -393,7 +394,10 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
     mbar_init(smem_u32(&sm.o_free), 64 * quarters);
     mbar_fence_init();
   }
+  __syncthreads();
+  if (warp == 7 && p.early_ctas > 0) prefetch_ahead(p, range, ranges, kUdAheadBlocks, kvh == 0, kvh == 1, &sm.begun, lane);
   pdl_wait();
+  if (threadIdx.x == 0) *static_cast<volatile int*>(&sm.begun) = 1;
   // this CTA's share of the block tables into the L2, while the lengths are on their way
   {
     const long long lines = ((long long)p.batch * p.table_width * (long long)sizeof(int32_t) + 127) / 128;

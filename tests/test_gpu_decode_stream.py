@@ -63,3 +63,36 @@ def test_stream_decode_flags_a_bad_block_and_leaves_its_keys_out(monkeypatch, at
         K.check_device_status()
     ref = K.paged_decode_attention(q, k[0], v[0], without, torch.tensor([192, 90], dtype=torch.int32, device="cuda"), SCALE, variant=1)
     assert float((got - ref).abs().max()) <= TIGHT
+
+
+# what a launch looks at ahead of its wait may still change: lengths and tables that a kernel in front replaces (values far outside
+# the pool for a moment), batches of 1, 33 and 257 rows (one more than are looked through), and verification rows of 5 and 9 tokens
+@pytest.mark.parametrize("rows,width", [(1, 1), (33, 1), (257, 1), (24, 5), (80, 5), (80, 9)])
+def test_launches_that_follow_one_another_read_what_the_kernel_in_front_left(rows, width):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    blocks = 96 if rows == 1 else 24
+    k, v = (torch.randn((1, 4096, BS, 2, 256), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    sets = [(torch.randint(width, blocks * BS + 1, (rows,), generator=g, device="cuda", dtype=torch.int32),
+             torch.randint(0, 4096, (rows, blocks), generator=g, device="cuda", dtype=torch.int32)) for _ in range(3)]
+    q = torch.randn((rows, width, 8, 256), generator=g, device="cuda").to(torch.bfloat16)
+
+    def attend(lens, tables):
+        if width == 1:
+            return K.paged_decode_attention(q[:, 0].contiguous(), k[0], v[0], tables, lens, SCALE, variant=3)
+        return K.paged_decode_attention_wide(q, k[0], v[0], tables, lens, None, SCALE, form=2)
+
+    alone = []
+    for s in sets:
+        alone.append(attend(*s))
+        torch.cuda.synchronize()
+    lens, tables = (t.clone() for t in sets[0])
+    outs = []
+    for i in range(9):
+        outs.append(attend(lens, tables))
+        lens.fill_(2_000_000_000)
+        tables.fill_(-5 if i % 2 else 2_000_000_000)
+        lens.copy_(sets[(i + 1) % 3][0])
+        tables.copy_(sets[(i + 1) % 3][1])
+    for i, out in enumerate(outs):
+        assert torch.equal(out, alone[i % 3])
