@@ -191,7 +191,9 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
     for (int i = 0; i < 4; ++i) { q2[h][i].x *= c; q2[h][i].y *= c; }
   }
 
-  // ---- fused append: where the new row goes; its key (if attended) is read from the operand
+  // ---- fused append: where the new row goes; its key (if attended) is read from the operand.  The warp that the row's unit falls to
+  // stores it: it has the block's id among its own.  (With the warp of unit 0, which had to fetch it, every warp waited for one trip more:
+  // f32, 8 rows of 64 - 512 keys 8.05 us : 7.67.)
   int new_key = -1;
   const char* new_k = nullptr;
   const char* new_v = nullptr;
@@ -199,25 +201,22 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
     const int pos = p.pre_append ? p.seq_lens[b] : p.positions[b];
     new_k = static_cast<const char*>(p.new_k) + (long long)b * kTokB + kvh * kRowB;
     new_v = static_cast<const char*>(p.new_v) + (long long)b * kTokB + kvh * kRowB;
-    if (pos >= 0) {
-      const int jt = pos / kBlk;
-      const long long tgt = jt < p.table_width ? (long long)p.block_tables[tbase + jt] : -1;
+    const int jt = pos / kBlk, unit = pos / kClUnit, turn = (unit - first) / stride;
+    if (pos < 0 ? first == 0 : unit % stride == first) {
+      const int held = __shfl_sync(kFullMask, ids, turn & 31);
+      const long long tgt = pos < 0 || jt >= p.table_width ? -1 : !p.kv_indptr && turn < 32 ? held : p.block_tables[tbase + jt];
       if (tgt >= 0 && tgt < p.num_blocks) {
         if (pos < len) new_key = pos;
-        if (first == 0) {
-          const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB;
+        const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB;
 #pragma unroll
-          for (int i = 0; i < (int)sizeof(T) / 2; ++i) {
-            const int o = (i * 32 + lane) * 16;
-            *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst + o) = *reinterpret_cast<const uint4*>(new_k + o);
-            *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst + o) = *reinterpret_cast<const uint4*>(new_v + o);
-          }
+        for (int i = 0; i < (int)sizeof(T) / 2; ++i) {
+          const int o = (i * 32 + lane) * 16;
+          *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst + o) = *reinterpret_cast<const uint4*>(new_k + o);
+          *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst + o) = *reinterpret_cast<const uint4*>(new_v + o);
         }
-      } else if (first == 0 && lane == 0) {
+      } else if (lane == 0) {
         atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
       }
-    } else if (first == 0 && lane == 0) {
-      atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
     }
   }
 
@@ -364,7 +363,7 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   cl_sync();
   cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, (int)rank, 0, kClThreads,
                       [&](int piece, float4 y) { reinterpret_cast<float4*>(dst)[piece] = y; });
-  cl_sync();  // nobody leaves while its shared memory is being read
+  cl_sync_relaxed();  // nobody leaves while its shared memory is being read
 }
 
 // ---- 16-bit caches: the products on tensor-core tiles -------------------------------------------------------------
@@ -386,7 +385,7 @@ struct CmSmem {
   union {
     char ring[kCmWarps][2][kBlk][kD * 2];  // [warp][K | V][key][16-byte piece c of the row at c ^ (key & 7)]
     struct {
-      float acc[kCmWarps][2 * kG][kCmPitch];  // [warp][column][dim]; the CTA's merged sums end up in acc[0][0 .. 3]
+      float acc[kCmWarps * kG][kCmPitch];  // [warp, head][dim]; the CTA's merged sums end up in the first rows, one per head
       float2 ml[kCmWarps][kG];
       float2 ML[kHq];
     } m;
@@ -452,7 +451,8 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     }
   }
 
-  // ---- fused append: where the new row goes; its key (if attended) is read from the operand
+  // ---- fused append: where the new row goes; its key (if attended) is read from the operand.  As above the warp stores it that its
+  // block falls to (150 rows of 512 - 1024 keys 48.4 us : 47.0, 64 of 512 - 4096 54.0 : 53.4, with the terms added before the merge).
   int new_key = -1;
   const char* new_k = nullptr;
   const char* new_v = nullptr;
@@ -460,20 +460,19 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     const int pos = p.pre_append ? p.seq_lens[b] : p.positions[b];
     new_k = static_cast<const char*>(p.new_k) + (long long)b * kTokB + kvh * kRowB + lane * 16;
     new_v = static_cast<const char*>(p.new_v) + (long long)b * kTokB + kvh * kRowB + lane * 16;
-    if (pos >= 0) {
-      const int jt = pos / kBlk;
-      const long long tgt = jt < p.table_width ? (long long)p.block_tables[tbase + jt] : -1;
+    const int jt = pos / kBlk, turn = (jt - first) / stride;
+    if (pos >= 0 && jt % stride == first) {
+      const int held = __shfl_sync(kFullMask, ids, turn & 31);
+      const long long tgt = jt >= p.table_width ? -1 : !p.kv_indptr && turn < 32 ? held : p.block_tables[tbase + jt];
       if (tgt >= 0 && tgt < p.num_blocks) {
         if (pos < len) new_key = pos;
-        if (first == 0) {
-          const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB + lane * 16;
-          *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst) = *reinterpret_cast<const uint4*>(new_k);
-          *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst) = *reinterpret_cast<const uint4*>(new_v);
-        }
-      } else if (first == 0 && lane == 0) {
+        const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB + lane * 16;
+        *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst) = *reinterpret_cast<const uint4*>(new_k);
+        *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst) = *reinterpret_cast<const uint4*>(new_v);
+      } else if (lane == 0) {
         atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
       }
-    } else if (!std::is_same<T, __nv_bfloat16>::value && first == 0 && lane == 0) {
+    } else if (!std::is_same<T, __nv_bfloat16>::value && pos < 0 && first == 0 && lane == 0) {
       atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
     }
   }
@@ -589,12 +588,12 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     if (lane < 2) sm.m.ml[warp][2 * t + c] = make_float2(m[c], l[c]);
   }
 #pragma unroll
-  for (int n = 0; n < 16; ++n) {
-    sm.m.acc[warp][2 * t][n * 16 + g] = o[n][0];
-    sm.m.acc[warp][2 * t + 1][n * 16 + g] = o[n][1];
-    sm.m.acc[warp][2 * t][n * 16 + g + 8] = o[n][2];
-    sm.m.acc[warp][2 * t + 1][n * 16 + g + 8] = o[n][3];
-  }
+  for (int k = 0; k < 8; ++k)  // both terms of a column are added: of two tiles a lane keeps one and gives the other away
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float keep = t < 2 ? o[2 * k][e] : o[2 * k + 1][e], give = t < 2 ? o[2 * k + 1][e] : o[2 * k][e];
+      sm.m.acc[warp * kG + 2 * (t & 1) + (e & 1)][(2 * k + (t >> 1)) * 16 + g + 8 * (e >> 1)] = keep + __shfl_xor_sync(kFullMask, give, 2);
+    }
   __syncthreads();
   constexpr int kHeads = kBoth ? kHq : kG;
   constexpr int kPieces = kHeads * kD / 4, kPer = kPieces / kCmThreads;  // float4 pieces of the output, and per thread
@@ -621,11 +620,10 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     for (int w = 0; w < kWalkers; ++w) {
       const float2 e = sm.m.ml[w0 + w * kStep][h];
       const float f = ex2_approx(e.x - M);
-      const float4 x = *reinterpret_cast<const float4*>(&sm.m.acc[w0 + w * kStep][h][d4]);
-      const float4 y = *reinterpret_cast<const float4*>(&sm.m.acc[w0 + w * kStep][h + kG][d4]);
+      const float4 x = *reinterpret_cast<const float4*>(&sm.m.acc[(w0 + w * kStep) * kG + h][d4]);
       L = fmaf(e.y, f, L);
-      sum[k].x = fmaf(x.x + y.x, f, sum[k].x); sum[k].y = fmaf(x.y + y.y, f, sum[k].y);
-      sum[k].z = fmaf(x.z + y.z, f, sum[k].z); sum[k].w = fmaf(x.w + y.w, f, sum[k].w);
+      sum[k].x = fmaf(x.x, f, sum[k].x); sum[k].y = fmaf(x.y, f, sum[k].y);
+      sum[k].z = fmaf(x.z, f, sum[k].z); sum[k].w = fmaf(x.w, f, sum[k].w);
     }
     if (ctas == 1) {
       const float inv = L > 0.f ? 1.f / L : 0.f;
@@ -635,14 +633,14 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     }
   }
   if (ctas > 1) {
-    __syncthreads();  // acc[0] is overwritten
+    __syncthreads();  // the first rows are overwritten
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
       const int piece = k * kCmThreads + threadIdx.x;
-      *reinterpret_cast<float4*>(&sm.m.acc[0][piece >> 6][(piece & 63) * 4]) = sum[k];
+      *reinterpret_cast<float4*>(&sm.m.acc[piece >> 6][(piece & 63) * 4]) = sum[k];
     }
     cl_sync();
-    cl_fold_cluster<kHeads>(&sm.m.acc[0][0][0], kCmPitch, sm.m.ML, ctas, rank, kPick && !kBoth ? kvh * ctas : 0, kCmThreads, store);
+    cl_fold_cluster<kHeads>(&sm.m.acc[0][0], kCmPitch, sm.m.ML, ctas, rank, kPick && !kBoth ? kvh * ctas : 0, kCmThreads, store);
   }
   const int members = kPick && !kBoth ? kHkv * ctas : ctas;  // CTAs of the cluster
   if constexpr (kPick) {
@@ -656,7 +654,11 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
       if (members > 1) cl_st2(cl_map(&sm.pick[kBoth ? rank : kvh * ctas + rank], 0), best.v, best.i);
     }
   }
-  if (members > 1) cl_sync();  // nobody leaves while its shared memory is being read; every candidate has arrived
+  // nobody leaves while its shared memory is being read; every candidate has arrived
+  if (members > 1) {
+    if constexpr (kPick) cl_sync();
+    else cl_sync_relaxed();
+  }
   if constexpr (kPick) {
     if (threadIdx.x == 0 && rank == 0 && (kBoth || kvh == 0)) {
       for (int c = 1; c < members; ++c) best.take(sm.pick[c].x, __float_as_int(sm.pick[c].y));

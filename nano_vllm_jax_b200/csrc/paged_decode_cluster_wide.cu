@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kCwThreads, 3) decode_cluster_wide_kernel(Deco
     const float inv = L > 0.f ? 1.f / L : 0.f;
     dst[piece] = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
   }
-  if (ctas > 1) cl_sync();  // nobody leaves while its shared memory is being read
+  if (ctas > 1) cl_sync_relaxed();  // nobody leaves while its shared memory is being read
 }
 
 template <int kTiles>

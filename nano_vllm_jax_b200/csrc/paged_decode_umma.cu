@@ -622,7 +622,7 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   if constexpr (kCluster) {
     cl_sync();
     ud_fold_cluster<kN>(sm, p, kvh, blockIdx.z, blockIdx.x, gridDim.x);
-    cl_sync();  // nobody leaves while its shared memory is being read
+    cl_sync_relaxed();  // nobody leaves while its shared memory is being read
   }
 }
 

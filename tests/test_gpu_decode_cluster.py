@@ -156,3 +156,25 @@ def test_lengths_that_the_kernel_in_front_changes(rows, width, monkeypatch):
         got = K.paged_decode_attention(q, k[0], v[0], tables, now, SCALE, variant=4)
         assert torch.equal(now, lens)
         assert float((got - ref).abs().max()) <= 2e-3
+
+
+# the warp that stores the new row is the one whose block it falls into: among its first 32 blocks or behind them, in a block that the
+# row does not attend, and in the last one of the table
+@pytest.mark.parametrize("cache", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("lens,at", [([33605, 90, 20], [33604, 89, 19]), ([100, 1, 200], [170, 63, 991]), ([16, 32, 48], [16, 31, 300])])
+def test_cluster_decode_appends_wherever_the_position_lies(cache, lens, at):
+    from nano_vllm_jax_b200.kernels import paged_kv as K
+    width = max(max(lens), max(at) + 1) // BS + 1
+    g = torch.Generator(device="cuda").manual_seed(sum(at))
+    k, v = (torch.randn((1, 3 * width + 4, BS, 2, 256), generator=g, device="cuda").to(cache) for _ in range(2))
+    tables = torch.randperm(3 * width + 4, generator=g, device="cuda").to(torch.int32)[:3 * width].view(3, width).contiguous()
+    t_lens, pos = torch.tensor(lens, dtype=torch.int32, device="cuda"), torch.tensor(at, dtype=torch.int32, device="cuda").view(3, 1)
+    q, nk, nv = (torch.randn((3, 1, h, 256), generator=g, device="cuda").to(cache) for h in (8, 2, 2))
+    k2, v2 = k.clone(), v.clone()
+    for b, p in enumerate(at):
+        k2[0, int(tables[b, p // BS]), p % BS], v2[0, int(tables[b, p // BS]), p % BS] = nk[b, 0], nv[b, 0]
+    ref = K.paged_decode_attention(q[:, 0].contiguous(), k2[0], v2[0], tables, t_lens, SCALE, variant=1)
+    out, k, v = K.paged_decode_attention_with_kv_append(q, nk, nv, k, v, tables, t_lens, pos, 0, BS, SCALE, 4, variant=4)
+    assert float((out.view(3, 8, 256) - ref).abs().max()) <= TIGHT[cache]
+    for a, b in ((k, k2), (v, v2)):
+        np.testing.assert_array_equal(bits(to_numpy(a)), bits(to_numpy(b)))
