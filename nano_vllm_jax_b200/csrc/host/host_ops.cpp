@@ -707,6 +707,18 @@ int same_token(PyObject* x, PyObject* y) {
   return int_of(x, &u) && int_of(y, &v) ? u == v : PyObject_RichCompareBool(x, y, Py_EQ);
 }
 
+// Whether a block holds exactly the tokens [at, at + bs) of the list under this digest: 1, 0, or -1 with a Python error set.
+int holds(PyObject* block, PyObject* digest, PyObject* tokens, long long at, long long bs) {
+  PyObject *hash = block_slots.get(block, kHash), *held = block_slots.get(block, kTokenIds);
+  int same = hash && held ? PyObject_RichCompareBool(hash, digest, Py_EQ) : -1;
+  if (same == 1) same = PyList_Check(held) && PyList_GET_SIZE(held) == bs ? 1 : 0;
+  for (long long k = 0; same == 1 && k < bs; ++k)
+    same = same_token(PyList_GET_ITEM(held, (Py_ssize_t)k), PyList_GET_ITEM(tokens, (Py_ssize_t)(at + k)));
+  Py_XDECREF(hash);
+  Py_XDECREF(held);
+  return same;
+}
+
 // cached_run(token_ids, digests | None, block_size, full blocks, published {digest: block id}, blocks, cacheable digests |
 // None, used ids) -> (ids of the published blocks of the longest reusable prefix, its digest | None, how many of them are in
 // use): a block counts when it holds exactly these tokens.  Digests are taken as the walk needs them when none are given;
@@ -740,21 +752,12 @@ PyObject* cached_run(PyObject* const* a, Py_ssize_t n) {
     PyObject* id = PyDict_GetItemWithError(a[4], digest);  // borrowed
     PyObject* block = id ? block_at(a[5], id) : nullptr;
     ok = block || (!id && !PyErr_Occurred());
-    int same = 0;
-    if (block) {
-      PyObject *hash = block_slots.get(block, kHash), *held = block_slots.get(block, kTokenIds);
-      same = hash && held ? PyObject_RichCompareBool(hash, digest, Py_EQ) : -1;
-      if (same == 1) same = PyList_Check(held) && PyList_GET_SIZE(held) == bs ? 1 : 0;
-      for (long long k = 0; same == 1 && k < bs; ++k)
-        same = same_token(PyList_GET_ITEM(held, (Py_ssize_t)k), PyList_GET_ITEM(a[0], (Py_ssize_t)(i * bs + k)));
-      Py_XDECREF(hash);
-      Py_XDECREF(held);
-    }
+    const int same = block ? holds(block, digest, a[0], i * bs, bs) : 0;
     if (same == 1) {
       const int used = PySet_Contains(a[7], id), usable = a[6] == Py_None ? 1 : PySequence_Contains(a[6], digest);
-      if (used < 0 || usable < 0 || PyList_Append(hits, id) < 0) same = -1;
+      ok = ok && used >= 0 && usable >= 0 && PyList_Append(hits, id) == 0;
       live += used > 0;
-      if (same == 1 && usable) {
+      if (ok && usable) {
         best = (Py_ssize_t)i + 1;
         best_live = live;
         Py_XDECREF(best_digest);
@@ -800,6 +803,36 @@ PyObject* add_owner(PyObject* const* a, Py_ssize_t n) {
   return idle;
 }
 
+// Block `id` becomes a sequence's: owned once, with its digest and the tokens [at, at + bs) when it is a full block (else `digest` is
+// null); what it published before is withdrawn.  False: Python error set.
+bool fresh_block(PyObject* blocks, PyObject* id, PyObject* published, PyObject* no_hash, PyObject* one, PyObject* digest, PyObject* tokens,
+                 long long at, long long bs) {
+  PyObject* block = block_at(blocks, id);
+  if (!block) return false;
+  PyObject *owners = block_slots.get(block, kRefCount), *old = block_slots.get(block, kHash);
+  bool ok = owners && old;
+  if (ok && PyObject_IsTrue(owners) != 0) {
+    PyErr_SetString(PyExc_AssertionError, "a free block has an owner");
+    ok = false;
+  }
+  const int had = ok ? PyObject_RichCompareBool(old, no_hash, Py_NE) : 0;
+  if (had == 1) {  // its old content is about to be overwritten
+    PyObject* holder = PyDict_GetItemWithError(published, old);
+    const int mine = holder ? PyObject_RichCompareBool(holder, id, Py_EQ) : 0;
+    if (mine == 1) ok = PyDict_DelItem(published, old) == 0;
+    else ok = mine == 0 && !PyErr_Occurred();
+  } else if (had < 0) {
+    ok = false;
+  }
+  Py_XDECREF(owners);
+  Py_XDECREF(old);
+  PyObject* held = ok ? (digest ? PyList_GetSlice(tokens, (Py_ssize_t)at, (Py_ssize_t)(at + bs)) : PyList_New(0)) : nullptr;
+  ok = ok && held && block_slots.set(block, kRefCount, one) && block_slots.set(block, kHash, digest ? digest : no_hash) &&
+       block_slots.set(block, kTokenIds, held);
+  Py_XDECREF(held);
+  return ok;
+}
+
 // take_fresh(blocks, ids, first, digests, token_ids, block_size, published, no_hash): block ids[k] becomes block first + k of
 // a sequence: owned once, with its digest and tokens when it is a full block; what it published before is withdrawn.
 PyObject* take_fresh(PyObject* const* a, Py_ssize_t n) {
@@ -813,36 +846,99 @@ PyObject* take_fresh(PyObject* const* a, Py_ssize_t n) {
   PyObject* one = PyLong_FromLong(1);
   bool ok = one != nullptr;
   for (Py_ssize_t k = 0; ok && k < PyList_GET_SIZE(a[1]); ++k) {
-    PyObject* id = PyList_GET_ITEM(a[1], k);
-    PyObject* block = block_at(a[0], id);
-    if (!(ok = block != nullptr)) break;
-    PyObject *owners = block_slots.get(block, kRefCount), *old = block_slots.get(block, kHash);
-    ok = owners && old;
-    if (ok && PyObject_IsTrue(owners) != 0) {
-      PyErr_SetString(PyExc_AssertionError, "a free block has an owner");
-      ok = false;
-    }
-    const int had = ok ? PyObject_RichCompareBool(old, a[7], Py_NE) : 0;
-    if (had == 1) {  // its old content is about to be overwritten
-      PyObject* holder = PyDict_GetItemWithError(a[6], old);
-      const int mine = holder ? PyObject_RichCompareBool(holder, id, Py_EQ) : 0;
-      if (mine == 1) ok = PyDict_DelItem(a[6], old) == 0;
-      else ok = mine == 0 && !PyErr_Occurred();
-    } else if (had < 0) {
-      ok = false;
-    }
-    Py_XDECREF(owners);
-    Py_XDECREF(old);
     const long long index = first + k;
-    const bool full = index < PyList_GET_SIZE(a[3]);
-    PyObject* tokens = ok ? (full ? PyList_GetSlice(a[4], (Py_ssize_t)(index * bs), (Py_ssize_t)((index + 1) * bs)) : PyList_New(0)) : nullptr;
-    ok = ok && tokens && block_slots.set(block, kRefCount, one) &&
-         block_slots.set(block, kHash, full ? PyList_GET_ITEM(a[3], (Py_ssize_t)index) : a[7]) && block_slots.set(block, kTokenIds, tokens);
-    Py_XDECREF(tokens);
+    PyObject* digest = index < PyList_GET_SIZE(a[3]) ? PyList_GET_ITEM(a[3], (Py_ssize_t)index) : nullptr;
+    ok = fresh_block(a[0], PyList_GET_ITEM(a[1], k), a[6], a[7], one, digest, a[4], index * bs, bs);
   }
   Py_XDECREF(one);
   if (!ok) return nullptr;
   Py_RETURN_NONE;
+}
+
+PyObject* name_num_cached;
+
+// allocate(seq, token_ids, block_size, full blocks, blocks in all, published, blocks, cacheable digests | None, used ids, whether published
+// blocks are shared, the sequence's table, take(n), take_cached(id), no_hash) -> (digest of the reused prefix | None,): a sequence's
+// blocks in one pass over its tokens, the published ones of its longest reusable prefix (cached_run, add_owner), then fresh ones (take_fresh).
+// None, and nothing changed, when the tokens are not machine-size integers.
+PyObject* allocate(PyObject* const* a, Py_ssize_t n) {
+  if (!args_are(n, 14)) return nullptr;
+  PyObject *tokens = a[1], *published = a[5], *blocks = a[6], *used = a[8], *table = a[10];
+  const long long bs = PyLong_AsLongLong(a[2]), full = PyLong_AsLongLong(a[3]), want = PyLong_AsLongLong(a[4]);
+  const int share = PyObject_IsTrue(a[9]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!PyList_CheckExact(tokens) || !PyDict_Check(published) || !PyList_Check(blocks) || !PySet_Check(used) || !PyList_Check(table) || bs < 1 ||
+      full < 0 || full > PyList_GET_SIZE(tokens) / bs)
+    NVJ_NONE();
+  HashChain chain(tokens, bs);
+  std::vector<uint64_t> digests((size_t)full);
+  PyObject *hits = PyList_New(0), *best_digest = nullptr;
+  Py_ssize_t best = 0;
+  bool ok = hits != nullptr, whole = true, run = share != 0;
+  for (long long i = 0; ok && i < full; ++i) {
+    if (!(whole = chain.next(i, &digests[(size_t)i]))) break;
+    if (!run) continue;
+    PyObject* digest = PyLong_FromUnsignedLongLong(digests[(size_t)i]);
+    PyObject* id = digest ? PyDict_GetItemWithError(published, digest) : nullptr;  // borrowed
+    PyObject* block = id ? block_at(blocks, id) : nullptr;
+    ok = digest && (block || (!id && !PyErr_Occurred()));
+    const int same = block ? holds(block, digest, tokens, i * bs, bs) : 0;
+    if (same == 1) {
+      const int usable = a[7] == Py_None ? 1 : PySequence_Contains(a[7], digest);
+      ok = ok && usable >= 0 && PyList_Append(hits, id) == 0;
+      if (ok && usable) {
+        best = (Py_ssize_t)i + 1;
+        Py_XDECREF(best_digest);
+        Py_INCREF(digest);
+        best_digest = digest;
+      }
+    }
+    Py_XDECREF(digest);
+    ok = ok && same >= 0;
+    run = same == 1;
+  }
+  ok = ok && PyList_SetSlice(hits, best, PyList_GET_SIZE(hits), nullptr) == 0;
+  if (!ok || !whole) {
+    Py_XDECREF(hits);
+    Py_XDECREF(best_digest);
+    if (!ok) return nullptr;
+    NVJ_NONE();
+  }
+  // the shared ones: owned once more, those that nobody holds taken back from the free list
+  PyObject* owner_args[3] = {blocks, hits, used};
+  PyObject* idle = add_owner(owner_args, 3);
+  ok = idle != nullptr;
+  for (Py_ssize_t k = 0; ok && k < PyList_GET_SIZE(idle); ++k) {
+    PyObject* r = PyObject_CallOneArg(a[12], PyList_GET_ITEM(idle, k));
+    ok = r != nullptr;
+    Py_XDECREF(r);
+  }
+  Py_XDECREF(idle);
+  ok = ok && PyList_SetSlice(table, PyList_GET_SIZE(table), PyList_GET_SIZE(table), hits) == 0;
+  PyObject* cached = ok ? PyLong_FromLongLong((long long)best * bs) : nullptr;
+  ok = cached && PyObject_SetAttr(a[0], name_num_cached, cached) == 0;
+  Py_XDECREF(cached);
+  Py_DECREF(hits);
+  // the rest
+  PyObject* rest = ok ? PyLong_FromLongLong(want - best) : nullptr;
+  PyObject* fresh = rest ? PyObject_CallOneArg(a[11], rest) : nullptr;
+  Py_XDECREF(rest);
+  PyObject* one = PyLong_FromLong(1);
+  ok = fresh && one && PyList_Check(fresh);
+  for (Py_ssize_t k = 0; ok && k < PyList_GET_SIZE(fresh); ++k) {
+    const long long index = (long long)best + k;
+    PyObject* digest = index < full ? PyLong_FromUnsignedLongLong(digests[(size_t)index]) : nullptr;
+    ok = (digest || index >= full) && fresh_block(blocks, PyList_GET_ITEM(fresh, k), published, a[13], one, digest, tokens, index * bs, bs);
+    Py_XDECREF(digest);
+  }
+  for (Py_ssize_t k = 0; ok && k < PyList_GET_SIZE(fresh); ++k) ok = PySet_Add(used, PyList_GET_ITEM(fresh, k)) == 0;
+  ok = ok && PyList_SetSlice(table, PyList_GET_SIZE(table), PyList_GET_SIZE(table), fresh) == 0;
+  Py_XDECREF(one);
+  Py_XDECREF(fresh);
+  PyObject* out = ok ? PyTuple_Pack(1, best_digest ? best_digest : Py_None) : nullptr;
+  Py_XDECREF(best_digest);
+  if (!out && !PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "allocate: take() has to return a list");
+  return out;
 }
 
 // drop_owner(blocks, table) -> ids that have no owner left, last block of the table first
@@ -1061,6 +1157,7 @@ PyMethodDef methods[] = {
     NVJ_FAST(cached_run, "published blocks of a sequence's longest reusable prefix"),
     NVJ_FAST(add_owner, "a sequence shares blocks that are in use"),
     NVJ_FAST(take_fresh, "free blocks become a sequence's"),
+    NVJ_FAST(allocate, "a sequence's blocks, shared and fresh, or None"),
     NVJ_FAST(drop_owner, "a sequence gives its blocks up"),
     NVJ_FAST(hash_chain, "chained digests of a token list's blocks, or None"),
     NVJ_FAST(stage_in, "a step's operands to the device, or None"),
@@ -1081,5 +1178,6 @@ PyMODINIT_FUNC PyInit__nvj_host(void) {
   const char* names[kBlockFields] = {"ref_count", "hash", "token_ids"};
   for (int k = 0; k < kBlockFields; ++k)
     if (!(block_field_names[k] = PyUnicode_InternFromString(names[k]))) return nullptr;
+  if (!(name_num_cached = PyUnicode_InternFromString("num_cached_tokens"))) return nullptr;
   return PyModule_Create(&module);
 }

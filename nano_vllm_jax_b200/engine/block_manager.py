@@ -247,6 +247,13 @@ class BlockManager:
         seq.cached_prefix_hash = None
         seq.cached_prefix_hybrid_seeded = False
         seq.prefix_cache_enabled = bool(use_prefix_cache)
+        tokens = seq.token_ids
+        done = _host.allocate(seq, tokens, self.block_size, min(seq.num_tokens, len(tokens)) // self.block_size, self._num_blocks(seq),
+                              self.hash_to_block_id, self.blocks, cacheable_hashes, self.used_block_ids, use_prefix_cache,
+                              seq.block_table, self.free_block_ids.take, self._take_cached, NO_HASH)
+        if done is not None:
+            seq.cached_prefix_hash = done[0] if seq.num_cached_tokens > 0 else None
+            return
         digests = self._digests(seq)
         hits, cached_hash, _ = self._cached_run(seq, cacheable_hashes, digests) if use_prefix_cache else ([], None, 0)
         blocks, used, free, bs, tokens, table = (self.blocks, self.used_block_ids, self.free_block_ids, self.block_size,

@@ -70,6 +70,10 @@ def take_fresh(blocks, ids, first, digests, token_ids, block_size, published, no
             block.update(digests[index], token_ids[index * block_size:(index + 1) * block_size])
 
 
+def allocate(*_):
+    return None  # the block manager takes the steps above one by one
+
+
 def drop_owner(blocks, table):
     gone = []
     for block_id in reversed(table):

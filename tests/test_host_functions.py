@@ -86,3 +86,27 @@ def test_the_python_form_refuses_alike(parts, rows, error):
             f.pack_batch(parts, rows, 2, -1)
         messages.append(str(e.value))
     assert messages[0] == messages[1]
+
+
+# no room for the rest behind shared blocks, tokens that are no machine-size integers (equal ones share all the same), a tuple of tokens
+@pytest.mark.parametrize("tokens", [list(range(9)) + [7] * 40, [1, 2, 3, 4, 5.0, 6], [0, 1, 2, 3, 2 ** 70, 5, 6, 7], tuple(range(8)), [True, 1, 2, 3, 4]])
+def test_an_allocation_in_one_call_leaves_what_the_steps_leave(tokens, monkeypatch):
+    def life(functions):
+        monkeypatch.setattr(block_manager, "_host", functions)
+        monkeypatch.setattr(block_manager, "_hash_chain", functions.hash_chain)
+        m = block_manager.BlockManager(8, 4)
+        first, gone, s = Sequence(range(8), seq_id=0), Sequence([1] * 12, seq_id=1), Sequence([0], seq_id=2)
+        for q in (first, gone):
+            m.allocate(q)
+            m.record_computed_prefix(q, q.num_tokens, publish=True)
+        m.deallocate(gone)
+        s.token_ids, s.num_tokens = tokens, len(tokens)
+        try:
+            m.allocate(s)
+            error = None
+        except (StopIteration, OverflowError, TypeError) as e:
+            error = type(e)
+        return (error, s.block_table, s.num_cached_tokens, s.cached_prefix_hash, list(m.free_block_ids), sorted(m.used_block_ids), dict(m.hash_to_block_id),
+                [(b.ref_count, b.hash, list(b.token_ids)) for b in m.blocks])
+
+    assert life(_lib.host_module()) == life(host_functions)
