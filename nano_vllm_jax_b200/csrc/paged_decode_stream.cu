@@ -17,7 +17,8 @@
 // The split over CTAs, the partials and their fold are the CUDA-core kernel's (decode_parts.cuh).
 // Measured (us per launch, back to back; before: the untransposed form): 128 rows of 8192 - 32768 keys 906 -> 775 once the board
 // has warmed up (the form before ran at its power limit), 200 of 3000 - 9000 368 -> 368, 128 of 512 - 4096 101 -> 96, 256 of 128 - 1024
-// 65 -> 55, 8 of 8192 - 32768 63.4 -> 61.5, one of 32768 26.1 -> 25.2.
+// 65 -> 55, 8 of 8192 - 32768 63.4 -> 61.5, one of 32768 26.1 -> 25.2; with the prefetch
+// ahead of the wait and one fence per partial the 128 rows 782, the 8 rows 56 - 58.
 // Semantics: nanovllm_jax/kv_cache.py:852-998 for width-1 queries; the fused append follows
 // nanovllm_jax/kernels/full_attention_triton.py:373-485.
 

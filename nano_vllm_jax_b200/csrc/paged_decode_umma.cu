@@ -8,7 +8,7 @@
 //                  when the output is read.
 // A tile of 128 keys takes 1024 tensor cycles (what reading K and V from shared memory takes) where the query rows as the tile's rows
 // took 3000, most of them for lanes without a row; 64 rows of 5 tokens over 1024 - 4096 keys then ran at the board's power limit, 80 us,
-// and now take 66 (append, this and the fold; 52 at the copy rate).  kN = 32 for up to 8 tokens: three accumulators take the tiles
+// and now take 64 (append, this and the fold; 52 at the copy rate).  kN = 32 for up to 8 tokens: three accumulators take the tiles
 // in turn, so that a sum is a third as long (error against 64 bits 4.4e-6 -> 2.5e-6 there).  More than 8 tokens: 64 columns,
 // on clusters only; on ranges the query rows stay the tile's rows (paged_decode_umma_query_rows.cu), 64 columns and two slots are no faster.
 //
