@@ -102,13 +102,14 @@ __device__ __forceinline__ void cl_end_beside(const DecodeParams& p) {
   }
 }
 // The CTAs' sums [head][pitch] and (max, sum) pairs, at the same places in every CTA of the cluster, into the output: rank
-// r takes its 1 / ctas of the float4 pieces of [heads][256 dims].
+// r takes its 1 / ctas of the float4 pieces of [heads][256 dims].  Returns what cl_sync_read() asks for.
 // `store` gets a piece's index and its four values; `base`: the cluster's rank of the first of these CTAs.
 template <int kHeads, class Store>
-__device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, const float2* ML, int ctas, int rank, int base, int threads,
+__device__ __forceinline__ bool cl_fold_cluster(const float* acc, int pitch, const float2* ML, int ctas, int rank, int base, int threads,
                                                 Store store) {
   constexpr int kPieces = kHeads * kD / 4;
   const int per = (kPieces + ctas - 1) / ctas;
+  bool odd = false;
   for (int i = threadIdx.x; i < per; i += threads) {
     const int piece = rank * per + i, h = piece >> 6, d = (piece & 63) * 4;
     if (piece >= kPieces) break;
@@ -139,8 +140,11 @@ __device__ __forceinline__ void cl_fold_cluster(const float* acc, int pitch, con
       y.x = fmaf(x[c].x, f, y.x); y.y = fmaf(x[c].y, f, y.y); y.z = fmaf(x[c].z, f, y.z); y.w = fmaf(x[c].w, f, y.w);
     }
     const float inv = L > 0.f ? 1.f / L : 0.f;
-    store(piece, make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv));
+    y = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+    odd |= cl_not_finite(y);
+    store(piece, y);
   }
+  return odd;
 }
 
 template <typename T>
@@ -366,9 +370,9 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   *reinterpret_cast<float4*>(&sm.acc[0][h][d4]) = o;
   if (d4 == 0) sm.ML[h] = make_float2(M, L);
   cl_sync();
-  cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, (int)rank, 0, kClThreads,
-                      [&](int piece, float4 y) { reinterpret_cast<float4*>(dst)[piece] = y; });
-  cl_sync_relaxed();  // nobody leaves while its shared memory is being read
+  const bool odd = cl_fold_cluster<kG>(&sm.acc[0][0][0], kD, sm.ML, ctas, (int)rank, 0, kClThreads,
+                                       [&](int piece, float4 y) { reinterpret_cast<float4*>(dst)[piece] = y; });
+  cl_sync_read(odd);  // nobody leaves while its shared memory is being read
 }
 
 // ---- 16-bit caches: the products on tensor-core tiles -------------------------------------------------------------
@@ -637,6 +641,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
       sm.m.ML[head] = make_float2(M, L);
     }
   }
+  bool odd = false;
   if (ctas > 1) {
     __syncthreads();  // the first rows are overwritten
 #pragma unroll
@@ -645,7 +650,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
       *reinterpret_cast<float4*>(&sm.m.acc[piece >> 6][(piece & 63) * 4]) = sum[k];
     }
     cl_sync();
-    cl_fold_cluster<kHeads>(&sm.m.acc[0][0], kCmPitch, sm.m.ML, ctas, rank, kPick && !kBoth ? kvh * ctas : 0, kCmThreads, store);
+    odd = cl_fold_cluster<kHeads>(&sm.m.acc[0][0], kCmPitch, sm.m.ML, ctas, rank, kPick && !kBoth ? kvh * ctas : 0, kCmThreads, store);
   }
   const int members = kPick && !kBoth ? kHkv * ctas : ctas;  // CTAs of the cluster
   if constexpr (kPick) {
@@ -662,7 +667,7 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
   // nobody leaves while its shared memory is being read; every candidate has arrived
   if (members > 1) {
     if constexpr (kPick) cl_sync();
-    else cl_sync_relaxed();
+    else cl_sync_read(odd);
   }
   if constexpr (kPick) {
     if (threadIdx.x == 0 && rank == 0 && (kBoth || kvh == 0)) {

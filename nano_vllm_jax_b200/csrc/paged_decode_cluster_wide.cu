@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(kCwThreads, 3) decode_cluster_wide_kernel(Deco
   const int pieces = p.width * kHq * (kD / 4), per = (pieces + ctas - 1) / ctas;
   const int end = (rank + 1) * per < pieces ? (rank + 1) * per : pieces;
   float4* dst = reinterpret_cast<float4*>(p.out + (long long)b * p.width * kHq * kD);
+  bool odd = false;
   for (int piece = rank * per + threadIdx.x; piece < end; piece += kCwThreads) {
     const int row = piece >> 6, tok = row / kHq, head = row - tok * kHq;
     const int col = (head / kG) * kCols + tok * 4 + (head % kG), d = (piece & 63) * 4;
@@ -258,9 +259,11 @@ __global__ void __launch_bounds__(kCwThreads, 3) decode_cluster_wide_kernel(Deco
       }
     }
     const float inv = L > 0.f ? 1.f / L : 0.f;
-    dst[piece] = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+    y = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+    odd |= cl_not_finite(y);
+    dst[piece] = y;
   }
-  if (ctas > 1) cl_sync_relaxed();  // nobody leaves while its shared memory is being read
+  if (ctas > 1) cl_sync_read(odd);  // nobody leaves while its shared memory is being read
 }
 
 template <int kTiles>

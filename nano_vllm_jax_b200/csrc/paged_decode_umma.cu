@@ -461,10 +461,12 @@ __device__ __forceinline__ void ud_query_warps(UdSmem<kN>& sm, const DecodeParam
 }
 
 // The sums of a cluster's CTAs [query row][dim] and their (max, sum) into the output: rank r takes its share of the float4 pieces.
+// Returns what cl_sync_read() asks for.
 template <int kN>
-__device__ __forceinline__ void ud_fold_cluster(UdSmem<kN>& sm, const DecodeParams& p, int kvh, int b, int rank, int ctas) {
+__device__ __forceinline__ bool ud_fold_cluster(UdSmem<kN>& sm, const DecodeParams& p, int kvh, int b, int rank, int ctas) {
   const int pieces = 4 * p.width * (kD / 4), per = (pieces + ctas - 1) / ctas;
   float* out = p.out + ((long long)b * p.width * kHq + kvh * kG) * kD;
+  bool odd = false;
   for (int i = threadIdx.x; i < per; i += kDecodeThreads) {
     const int piece = rank * per + i, c = piece >> 6, d = (piece & 63) * 4;
     if (piece >= pieces) break;
@@ -487,8 +489,11 @@ __device__ __forceinline__ void ud_fold_cluster(UdSmem<kN>& sm, const DecodePara
         y.x = fmaf(x[r].x, f, y.x); y.y = fmaf(x[r].y, f, y.y); y.z = fmaf(x[r].z, f, y.z); y.w = fmaf(x[r].w, f, y.w);
       }
     const float inv = L > 0.f ? 1.f / L : 0.f;
-    *reinterpret_cast<float4*>(out + ((c >> 2) * kHq + (c & 3)) * kD + d) = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+    y = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+    odd |= cl_not_finite(y);
+    *reinterpret_cast<float4*>(out + ((c >> 2) * kHq + (c & 3)) * kD + d) = y;
   }
+  return odd;
 }
 
 template <int kN, bool kCluster>
@@ -621,8 +626,8 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
   if (warp == 4) tmem_dealloc(tmem, kUdTmemCols);
   if constexpr (kCluster) {
     cl_sync();
-    ud_fold_cluster<kN>(sm, p, kvh, blockIdx.z, blockIdx.x, gridDim.x);
-    cl_sync_relaxed();  // nobody leaves while its shared memory is being read
+    const bool odd = ud_fold_cluster<kN>(sm, p, kvh, blockIdx.z, blockIdx.x, gridDim.x);
+    cl_sync_read(odd);  // nobody leaves while its shared memory is being read
   }
 }
 

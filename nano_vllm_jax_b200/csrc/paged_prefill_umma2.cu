@@ -480,7 +480,8 @@ __device__ __forceinline__ void u2_softmax_warps(Umma2Smem& sm, const Umma2Param
 // requested before anything is used.  The (max, sum) pairs of a warp's rows come in one load: what counts between the CTAs is the number of
 // requests, and with a load of its own for every row the fold took 3.8 us instead of 3.1 (512 tokens behind 1024: 20.2 -> 19.2 us, behind 256
 // 17.7 -> 16.5, 64 behind 400 16.1 -> 15.3).  Three rows at a time, or half rows: no faster.
-__device__ __forceinline__ void u2_fold_splits(const Umma2Smem& sm, const Umma2Params& p, int tok0, int ntok, int kvh, int rank, int splits,
+// Returns what cl_sync_read() asks for.
+__device__ __forceinline__ bool u2_fold_splits(const Umma2Smem& sm, const Umma2Params& p, int tok0, int ntok, int kvh, int rank, int splits,
                                                int warp, int lane) {
   const float* stage = reinterpret_cast<const float*>(&sm.k[0][0][0]);
   constexpr int kWarps = kU2Threads / 32;
@@ -501,6 +502,7 @@ __device__ __forceinline__ void u2_fold_splits(const Umma2Smem& sm, const Umma2P
     for (int o = 1; o < kU2MaxSplits; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
     w = total > 0.f ? w / total : 0.f;
   }
+  bool odd = !(w <= 1.f);
   for (int r0 = first; r0 < last; r0 += 2) {
     float4 x[2][kU2MaxSplits][2];
     bool real[2];
@@ -531,10 +533,12 @@ __device__ __forceinline__ void u2_fold_splits(const Umma2Smem& sm, const Umma2P
           acc[h].z = fmaf(x[k][s][h].z, ws, acc[h].z); acc[h].w = fmaf(x[k][s][h].w, ws, acc[h].w);
         }
       }
+      odd |= cl_not_finite(acc[0]) || cl_not_finite(acc[1]);
       dst[lane] = acc[0];
       dst[32 + lane] = acc[1];
     }
   }
+  return odd;
 }
 
 // Which (table row, 32-token tile) the CTA with cluster index `cluster` of `clusters` and rank `rank` serves: the
@@ -751,18 +755,19 @@ prefill_umma2_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
 
   tc_fence_before_sync();
   __syncthreads();
+  bool odd = false;
   if (splits > 1) {
     cl_sync();  // every split's rows are staged
-    u2_fold_splits(sm, p, tok0, ntok, kvh, rank, splits, warp, lane);
+    odd = u2_fold_splits(sm, p, tok0, ntok, kvh, rank, splits, warp, lane);
     NVJ_U2_PHASE(5);
   }
   if (sm.abort_flag) {  // give copies and MMAs in flight time to land before memory is released
     const unsigned long long t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
-  // CTA 0's MMAs read this CTA's shared and tensor memory until its last commit; the other splits its rows (their loads have returned
-  // what they stored).  Nobody reads another's output, so nobody waits for its stores to arrive.
-  cl_sync_relaxed();
+  // CTA 0's MMAs read this CTA's shared and tensor memory until its last commit, which its softmax warps have waited for; the other splits
+  // its rows.
+  cl_sync_read(odd);
   NVJ_U2_PHASE(6);
   if (warp == 1) tmem2_dealloc(tmem, kU2TmemCols);
 }
