@@ -10,7 +10,8 @@
 //     and V are the second trip to memory;
 //   * the warps merge through shared memory, the C CTAs through distributed shared memory: two cluster barriers instead
 //     of fences and counters; rank r writes its 1 / C of the output;
-//   * fused append: the cluster's first warp stores the new row, and whoever attends its key reads it from the operand.
+//   * fused append: the cluster's first warp (f32: the one that the row's unit falls to) stores the new row, and whoever attends its key
+//     reads it from the operand.
 // Nothing waits on memory that somebody else must fill, so there is no wait to bound.
 // Measured (us per launch, K/V cold, lengths spread over [n / 4, n]; the streaming kernel : this one): 4 rows of n = 512 tokens
 // 10.6 : 5.5, 8 of 4096 19.1 : 13.2, 48 of 1024 19.1 : 16.5, 256 of 2048 108 : 106, 256 of 4096 204 : 200 (a first build, whose every
@@ -201,8 +202,8 @@ __global__ void __launch_bounds__(kClThreads, 2) decode_cluster_kernel(DecodePar
   }
 
   // ---- fused append: where the new row goes; its key (if attended) is read from the operand.  The warp that the row's unit falls to
-  // stores it: it has the block's id among its own.  (With the warp of unit 0, which had to fetch it, every warp waited for one trip more:
-  // f32, 8 rows of 64 - 512 keys 8.05 us : 7.67.)
+  // stores it: it has the block's id among its own.  (With the warp of unit 0, which has to fetch it, every warp waits for one trip more:
+  // f32, 8 rows of 64 - 512 keys 7.7 us : 7.6, 32 of 1000 - 2000 41.6 : 41.3.)
   int new_key = -1;
   const char* new_k = nullptr;
   const char* new_v = nullptr;
@@ -460,8 +461,10 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     }
   }
 
-  // ---- fused append: where the new row goes; its key (if attended) is read from the operand.  As above the warp stores it that its
-  // block falls to (150 rows of 512 - 1024 keys 48.4 us : 47.0, 64 of 512 - 4096 54.0 : 53.4, with the terms added before the merge).
+  // ---- fused append: where the new row goes; its key (if attended) is read from the operand.  The row's first warp stores it, not the
+  // one that its block falls to, which has the id but also the longest walk: eight steps of a graph, stored by that one : by the first,
+  // 39 rows of 200 - 800 keys 129.9 us : 115.7, 40 of 700 - 2800 276.5 : 267.1, 256 of 200 - 800 468.5 : 459.9; one launch, 16 rows of 500 -
+  // 2000 10.7 : 10.2, 150 of 512 - 1024 45.3 : 45.1.
   int new_key = -1;
   const char* new_k = nullptr;
   const char* new_v = nullptr;
@@ -469,19 +472,20 @@ __global__ void __launch_bounds__(kCmThreads, 3) decode_cluster_mma_kernel(Decod
     const int pos = p.pre_append ? p.seq_lens[b] : p.positions[b];
     new_k = static_cast<const char*>(p.new_k) + (long long)b * kTokB + kvh * kRowB + lane * 16;
     new_v = static_cast<const char*>(p.new_v) + (long long)b * kTokB + kvh * kRowB + lane * 16;
-    const int jt = pos / kBlk, turn = (jt - first) / stride;
-    if (pos >= 0 && jt % stride == first) {
-      const int held = __shfl_sync(kFullMask, ids, turn & 31);
-      const long long tgt = jt >= p.table_width ? -1 : !p.kv_indptr && turn < 32 ? held : p.block_tables[tbase + jt];
+    if (pos >= 0) {
+      const int jt = pos / kBlk;
+      const long long tgt = jt < p.table_width ? (long long)p.block_tables[tbase + jt] : -1;
       if (tgt >= 0 && tgt < p.num_blocks) {
         if (pos < len) new_key = pos;
-        const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB + lane * 16;
-        *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst) = *reinterpret_cast<const uint4*>(new_k);
-        *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst) = *reinterpret_cast<const uint4*>(new_v);
-      } else if (lane == 0) {
+        if (first == 0) {
+          const long long dst = (tgt * kBlk + pos % kBlk) * kTokB + kvh * kRowB + lane * 16;
+          *reinterpret_cast<uint4*>(const_cast<char*>(p.k_cache) + dst) = *reinterpret_cast<const uint4*>(new_k);
+          *reinterpret_cast<uint4*>(const_cast<char*>(p.v_cache) + dst) = *reinterpret_cast<const uint4*>(new_v);
+        }
+      } else if (first == 0 && lane == 0) {
         atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
       }
-    } else if (!std::is_same<T, __nv_bfloat16>::value && pos < 0 && first == 0 && lane == 0) {
+    } else if (!std::is_same<T, __nv_bfloat16>::value && first == 0 && lane == 0) {
       atomicOr(p.status, NVJ_DEV_BAD_BLOCK_ID);
     }
   }
