@@ -219,13 +219,14 @@ __device__ __forceinline__ void ud_softmax_warp(UdSmem& sm, const DecodeParams& 
   const bool real = tok < p.width;
   const float scale_log2 = p.scale * kLog2e;
   Seg s;
+  UdRing at;
   uint32_t done = 0;  // tiles so far
   while (next_seg(p, b, j, g, g1, s)) {
     const int my_pos = real ? (p.positions ? p.positions[(long long)s.b * p.width + tok] : 0x7fffffff) : -1;
     const int last_key = my_pos < s.len - 1 ? my_pos : s.len - 1;  // last key this row may see
     float m_row = -INFINITY, l_row = 0.f;                           // m_row in units of log2(e) * scale
     const int nblk = s.j1 - s.j0, nt = (nblk + kUdTileBlocks - 1) / kUdTileBlocks;
-    for (int t = 0; t < nt; ++t, ++done) {
+    for (int t = 0; t < nt; ++t, ++done, at.step()) {
       if (!um_wait(&sm.s_full, done & 1u, &sm.abort_flag, p.status)) return;
       tc_fence_after_sync();
       float sc[64];
@@ -293,6 +294,17 @@ __device__ __forceinline__ void ud_softmax_warp(UdSmem& sm, const DecodeParams& 
         }
       }
       tmem_st_wait();
+      if (t == nt - 1 && s.j1 == s.nb && (s.len & (kBlk - 1))) {
+        // V rows of the last block behind the last key weigh nothing, but may hold anything: 0 x infinity is not 0.  The 64 threads of
+        // the two warps are the block's 4 chunks x 16 keys.
+        if (!um_wait(&sm.v_full[at.at], at.phase, &sm.abort_flag, p.status)) return;
+        if ((row & (kBlk - 1)) >= (s.len & (kBlk - 1))) {
+          char* rest = &sm.v[at.at][cnt - 1][row * 128];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(rest + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async_smem();
+      }
       tc_fence_before_sync();
       mbar_arrive(smem_u32(&sm.p_full));
     }
