@@ -239,6 +239,10 @@ __device__ __forceinline__ UmmaCut umma_cut(const DecodeParams& p, const Partiti
   if (j == 0 || j >= nb || first != range - 1) return kNoCut;
   return UmmaCut{b, first, pt.cta_of(row_g0 + nb - 1), 0};
 }
+// Registers per thread of the tile kernel for 9 - 16 tokens and of the launch behind it that folds the partials: a CTA of either (256
+// threads) on an SM at once, so that the fold waits in place.
+constexpr int kUmmaQueryRowsRegs = 168, kUmmaMergeRegs = 88;
+static_assert(256 * (kUmmaQueryRowsRegs + kUmmaMergeRegs) <= 65536, "the fold does not fit beside the tile kernel");
 // Where a CTA parks its partial result for a row it shares with other CTAs: a
 // CTA holds at most one segment that continues a row begun elsewhere (slot 2c)
 // and at most one that begins a row finished elsewhere (slot 2c + 1).

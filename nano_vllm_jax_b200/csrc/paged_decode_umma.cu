@@ -634,8 +634,11 @@ decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_const
 // One CTA per (boundary between two ranges, query token): the first boundary that cuts a row folds the row from the ranges' partials.
 // Runs behind the tile kernel in stream order, so it needs neither counters nor fences, and is told by it what was cut where.  (One
 // CTA per row and token, each of which found that out for itself, took 10 - 15 us behind 256 rows and 6 behind 64; one per row that
-// folded its tokens in turn 8.2 for 64 rows of 8 tokens: every fold is three round trips to the L2.)
-__global__ void __launch_bounds__(kDecodeThreads)
+// folded its tokens in turn 8.2 for 64 rows of 8 tokens: every fold is three round trips to the L2.)  Beside the kernel for 9 - 16
+// tokens its CTAs wait in place (with 92 registers, where they do not fit, 5 rows of 9 tokens over 8000 - 12000 keys 35.2 us, so 34.1, 64 of 9
+// over 256 - 1024 34.1 and 33.8), which seven parts in flight leave room for; beside the one for fewer tokens, which takes the registers
+// and the shared memory of a whole SM, they cannot.
+__global__ void __maxnreg__(kUmmaMergeRegs)
 decode_umma_merge_kernel(DecodeParams p, int ranges) {
   __shared__ float red[384];
   const int tok = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -648,7 +651,7 @@ decode_umma_merge_kernel(DecodeParams p, int ranges) {
   const long long qbase = (long long)b * p.width;
   int first = c_lo, n = c_hi - c_lo + 1;
   if (n <= 32) {
-    fold_parts<true>(p, red, tid, 0, first, c_lo, n, (qbase + tok) * kHq, slot_rows, tok * kHq);
+    fold_parts<true, 7>(p, red, tid, 0, first, c_lo, n, (qbase + tok) * kHq, slot_rows, tok * kHq);
     return;
   }
   // more than 32 parts (a few very long rows): a plain running fold, thread = (head, 8 dims), four parts in flight

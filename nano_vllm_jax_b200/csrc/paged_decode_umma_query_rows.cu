@@ -376,8 +376,8 @@ __device__ __forceinline__ void ud_helper_warp(UdSmem& sm, const DecodeParams& p
   }
 }
 
-// 168 registers: a CTA of the merge launch (256 x 88) then fits beside this one and waits in place.
-__global__ void __maxnreg__(168)
+// A CTA of the launch that folds the partials fits beside this one and waits in place.
+__global__ void __maxnreg__(kUmmaQueryRowsRegs)
 decode_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, DecodeParams p) {
   extern __shared__ unsigned char ud_smem_raw[];
   UdSmem& sm = *reinterpret_cast<UdSmem*>((reinterpret_cast<uintptr_t>(ud_smem_raw) + 1023) & ~(uintptr_t)1023);
