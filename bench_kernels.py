@@ -136,7 +136,7 @@ def decode_cases(dev, iters, small=False):
                wbytes, {"workload": "c2, width %d" % width})
         if width > 8:  # the mma.sync form ends at 8
             continue
-        other, name = (1, "mma.sync tiles, two row tiles per warp pair") if width > 4 else (2, "tcgen05, query rows in a 128-row tile")
+        other, name = (1, "mma.sync tiles, two row tiles per warp pair") if width > 4 else (2, "tcgen05, keys and dims as the tile's rows")
         report("wide decode, %d query tokens per row (%s)" % (width, name),
                big.run(lambda: K.paged_decode_attention_wide(qw, k[0], v[0], tables, t_lens, wpos, SCALE, form=other)),
                wbytes, {"workload": "c2, width %d" % width})

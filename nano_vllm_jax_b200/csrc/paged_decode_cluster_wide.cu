@@ -278,21 +278,30 @@ static bool cw_takes(const DecodeParams& p) {
 // Two CTAs at least where the mma.sync form is the alternative: it sums every other block of a row apart, one CTA all of them in a
 // row, which is further from 64-bit attention (600 rows under 8 blocks, 2 tokens, plain / peaked / offset values: 1.84e-6 / 7.5e-7 / 4.1e-7 of
 // the result's size with one CTA, 1.71e-6 / 6.5e-7 / 3.5e-7 with two, 1.70e-6 / 6.4e-7 / 3.5e-7 mma.sync; tcgen05, the alternative below
-// that line, 2.03e-6 / 1.1e-6 / 4.5e-7).  They cost 33 -> 38 us there (mma.sync 48).
+// that line, 2.1e-6 / 1.1e-6 / 3.5e-7 over 1000 rows under 12).  They cost 33 -> 38 us there (mma.sync 48).
 static int cw_cluster(const DecodeParams& p, int sms) {
   const int c = cluster_size(p.batch, p.table_width, sms, 1, kCmPerSm, 8, kClMaxCluster);
   return c == 1 && p.table_width > 1 && wide_takes_mma_sync(p) ? 2 : c;
 }
 
-// Where the clusters beat the form that serves the rows otherwise: tcgen05 up to 4096 blocks of table (2 tokens) and 12288 (3 and 4),
-// mma.sync beyond (wide_takes_mma_sync).  First, few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs that
-// are resident at once.  Clusters : tcgen05, us, by table width, rows and CTAs per row: 3 tokens, 7 blocks per CTA, 32 x 64 (10 CTAs)
-// 20.7 : 21.1, 64 x 40 (6) 21.0 : 24.0, 128 x 16 (3, 6 blocks) 18.4 : 25.9; 8 blocks per CTA, 16 x 128 (16) 22.1 : 20.7, 4 x 128 15.9 : 15.9;
-// more CTAs than places, 140 x 40 40.7 : 36.2.  4 tokens: 64 x 40 22.9 : 24.9, 16 x 32 15.1 : 14.8, 16 x 128 23.7 : 21.4.  2 tokens: 16 x 128
-// 18.3 : 21.2, 64 x 40 18.5 : 24.0, 2 x 157 (10 blocks) 14.6 : 15.3, 8 x 256 (16 blocks) 23.4 : 22.7; mma.sync: 50 x 96 30.6 : 30.1.
+// Where the clusters serve the rows instead of tcgen05 (up to 4096 blocks of table with 2 tokens, 12288 with 3 and 4) or mma.sync
+// (beyond, wide_takes_mma_sync).  First, few blocks per CTA (a block takes 0.7 us at 2 tokens, 0.9 at 3 and 4) and CTAs that are resident
+// at once.  There tcgen05, which has clusters of its own, is as fast or faster by now, but further from 64-bit attention, so the lines
+// stay where the clusters were ahead.  Clusters : tcgen05, rows of 1/4 - 1 and of 1/32 - 1/8 of the table (us, each launch behind a small kernel)
+// and error relative to the result's size with plain, peaked and offset values:
+//   2 tokens  16 x 128  19.1 : 16.5 and  9.7 :  9.4   1.8e-6 : 2.3e-6, 0.81e-6 : 1.7e-6, 2.0e-7 : 1.7e-7
+//             64 x 40   18.8 : 19.3 and  9.5 : 10.1   1.8e-6 : 2.3e-6, 0.75e-6 : 2.0e-6, 2.3e-7 : 2.6e-7
+//              2 x 157  12.9 :  9.8 and  7.5 :  8.8   1.9e-6 : 2.0e-6, 0.81e-6 : 0.73e-6, 2.3e-7 : 1.4e-7
+//   3 tokens  32 x 64   21.3 : 18.0 and 12.0 : 10.3   1.8e-6 : 2.3e-6, 0.76e-6 : 1.8e-6, 2.0e-7 : 2.0e-7
+//            128 x 16   19.9 : 25.1 and 10.6 : 17.7   1.7e-6 : 2.1e-6, 0.75e-6 : 1.3e-6, 2.8e-7 : 3.2e-7
+//              4 x 128  17.9 : 11.5 and  9.1 :  9.1   1.8e-6 : 2.1e-6, 0.78e-6 : 0.80e-6, 2.1e-7 : 1.4e-7
+//   4 tokens  64 x 40   23.8 : 21.5 and 13.3 : 11.8   1.8e-6 : 2.3e-6, 0.74e-6 : 1.9e-6, 2.3e-7 : 2.6e-7
+//             16 x 32   16.6 : 10.7 and 13.8 :  9.5   1.6e-6 : 1.9e-6, 0.64e-6 : 0.76e-6, 1.9e-7 : 2.1e-7
+// Beyond the line: 3 tokens, 16 x 128 (8 blocks per CTA, more CTAs than SMs) 22.9 : 17.6, 140 x 40 41.0 : 35.0; 2 tokens, 8 x 256 25.3 : 19.4; mma.sync,
+// 50 x 96 30.6 : 30.1.
 // Second, many short rows, of which every one costs the other forms a change of rows.  Rows of 1/4 - 1 and of 1/32 - 1/8 of the
-// table; against tcgen05: 100 x 16 14.7 : 23.1 and 8.7 : 15.9 (2 tokens), 256 x 16 36.3 : 39.1 and 18.1 : 24.5 (3), 39.4 : 41.6 and
-// 20.6 : 26.8 (4), 1000 x 12 70.3 : 110.7 and 33.3 : 78.4 (3).  Against mma.sync, 2 tokens: up to 24 blocks, which two CTAs share, 400 x
+// table; against tcgen05: 100 x 16 14.2 : 22.1 and 8.6 : 16.4 (2 tokens), 256 x 16 35.3 : 34.7 and 19.4 : 25.6 (3), 38.4 : 35.2 and
+// 23.0 : 25.9 (4), 1000 x 12 72.4 : 92.8 and 34.6 : 68.5 (3), and closer to 64 bits.  Against mma.sync, 2 tokens: up to 24 blocks, which two CTAs share, 400 x
 // 12 32.5 : 41.3 and 16.0 : 24.1, 2000 x 24 186.8 : 222.7 and 82.3 : 94.0, 4000 x 2 148 : 165 and 144 : 156, 16000 x 12 917 : 1151 and 572 : 674;
 // from 25 on four CTAs, which only pay while they are few: 200 x 25 32.5 : 35.7 and 15.8 : 19.5, 400 x 25 56.9 : 56.8 and 29.5 : 29.3, 600 x
 // 25 80.8 : 77.5 and 44.2 : 37.6, 2000 x 25 243 : 228 and 143 : 93.  3 and 4 tokens against mma.sync: ahead by 3 - 8% where the rows fill
@@ -305,7 +314,7 @@ bool decode_cluster_wide_pays(const DecodeParams& p) {
   const int c = cw_cluster(p, sms), per_cta = (p.table_width + c - 1) / c;
   const long long ctas = (long long)c * p.batch;
   if (p.batch >= 100 && (p.width == 2 ? p.table_width <= (p.batch <= 400 ? 25 : 24) : p.table_width <= 16 && !wide_takes_mma_sync(p))) return true;
-  if (p.width > 2 && per_cta == 8) return ctas <= sms;  // 0 - 2 us slower than tcgen05 there, at half its error against 64 bits
+  if (p.width > 2 && per_cta == 8) return ctas <= sms;  // slower than tcgen05 there (4 x 128 above), at up to half its error
   return per_cta <= (p.width == 2 ? 12 : 7) && 100 * ctas <= (long long)kCmPerSm * sms;
 }
 

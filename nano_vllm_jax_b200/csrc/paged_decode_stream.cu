@@ -17,8 +17,8 @@
 // The split over CTAs, the partials and their fold are the CUDA-core kernel's (decode_parts.cuh).
 // Measured (us per launch, back to back; before: the untransposed form): 128 rows of 8192 - 32768 keys 906 -> 775 once the board
 // has warmed up (the form before ran at its power limit), 200 of 3000 - 9000 368 -> 368, 128 of 512 - 4096 101 -> 96, 256 of 128 - 1024
-// 65 -> 55, 8 of 8192 - 32768 63.4 -> 61.5, one of 32768 26.1 -> 25.2; with the prefetch
-// ahead of the wait and one fence per partial the 128 rows 782, the 8 rows 56 - 58.
+// 65 -> 55, 8 of 8192 - 32768 63.4 -> 61.5, one of 32768 26.1 -> 25.2; what the
+// prefetch ahead of the wait gives stands at kStAheadBlocks.
 // Semantics: nanovllm_jax/kv_cache.py:852-998 for width-1 queries; the fused append follows
 // nanovllm_jax/kernels/full_attention_triton.py:373-485.
 
@@ -49,9 +49,10 @@ static_assert(kDecodeThreads * kStConsumerRegs + 128 * kStProducerRegs <= kStThr
 constexpr int kStPitch = kD + 4;  // floats between the heads of a warp's sums: conflict-free stores
 constexpr int kStRowEndCost = 9;  // blocks that a row end costs a CTA (decode_parts.cuh): 32 rows of 512 - 4096 keys 34.1 us with 1, 33.3 with 6, 32.5 with 9
 
-// Blocks of a CTA's range that are prefetched ahead of the wait (prefetch_ahead).  Passes back to back without it : with it: 8 rows of 8192 -
-// 32768 keys 61.4 : 56.5 us, one row of 20000 19.4 : 18.2, 24 of 4096 - 16384 82.0 : 78.4, 32 of 2000 - 8000 59.2 : 54.4, 128 of 8192 - 32768
-// 770 : 764.  With six blocks the first 57.2, with 18 57.2, with 26 58.1.
+// Blocks of a CTA's range that are prefetched ahead of the wait (prefetch_ahead).  Passes back to back, each behind another of this kernel,
+// without it : with it: 8 rows of 8192 - 32768 keys 60.1 : 55.9 us, 24 of 4096 - 16384 83.7 : 79.1, 32 of 2000 - 8000 58.4 : 53.0, one row of 20000
+// and 128 of 8192 - 32768 the same (16.9 : 16.8, 783 : 785); behind a kernel that ends all at once there is nothing to gain (63.9 : 63.6).
+// With six blocks the first case is 0.7 us later, with 18 as well, with 26 1.6.
 constexpr int kStAheadBlocks = 12;
 
 struct StreamSmem {

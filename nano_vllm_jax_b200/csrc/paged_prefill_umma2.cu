@@ -323,7 +323,9 @@ __device__ __forceinline__ bool u2_softmax_tiles(Umma2Smem& sm, const Umma2Param
       float2 w = fma2(make_float2(s[2 * e], s[2 * e + 1]), c2, m2);
       w.x = ex2_approx(w.x);
       w.y = ex2_approx(w.y);
-      l_row += w.x + w.y;  // one running sum; two summed at the end measured a 20% larger error on peaked scores
+      // One running sum per thread: even and odd keys apart, added at the end, measured a 20% larger error on peaked scores.  (The two
+      // groups' sums, over the even and the odd tiles, are added at the end without one: 1.257e-6 before as after.)
+      l_row += w.x + w.y;
       const __nv_bfloat162 h = __floats2bfloat162_rn(w.x, w.y);
       const float2 rest = fma2(make_float2(__low2float(h), __high2float(h)), make_float2(-1.f, -1.f), w);  // exact
       const __nv_bfloat162 g = __floats2bfloat162_rn(rest.x, rest.y);

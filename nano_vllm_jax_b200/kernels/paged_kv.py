@@ -661,7 +661,7 @@ def packed_paged_prefill_attention(query, k_cache_layer, v_cache_layer, block_ta
     # kernels that write different rows of `out` and neither fills the machine, so they can run side by side on two
     # streams, the decode pass leaving the tile kernel's SMs free.  That paid when the launches come from a CUDA graph
     # (one 6-layer step: 328 -> 229 us; where the decode rows' clusters start beside the tiles in one stream, as they now do, that takes
-    # 170 and the fork 225: NVJ_MIXED_SIDE_BY_SIDE=0 avoids it); launched eagerly the extra stream bookkeeping costs the host more than the
+    # 136 - 146 and the fork 195 - 208: NVJ_MIXED_SIDE_BY_SIDE=0 avoids it); launched eagerly the extra stream bookkeeping costs the host more than the
     # overlap saves, so the fork is taken only while the current stream is being captured (NVJ_MIXED_SIDE_BY_SIDE=1
     # forces it, =0 forbids it).
     mixed = model_shape and variant in (0, 4, 5) and num_decode_rows is not None and 0 < num_decode_rows < rows
