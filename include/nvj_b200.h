@@ -303,9 +303,8 @@ size_t nvj_paged_decode_wide_workspace_bytes(int max_batch);
  * nvj_paged_decode_wide_form: the same call with the kernel chosen by the caller.  form 0 = automatic (what
  * nvj_paged_decode_wide does: width 1 on the streaming decode kernel; rows of 2-4 tokens, where they are few or short, in
  * thread-block clusters, else on tcgen05 while the batch is small and on mma.sync tiles beyond; widths 5-16 on tcgen05 (5-8 under a
- * scale <= 0 on mma.sync tiles), the 4 x width
- * query rows of a KV head in a 128-row tile with scores and output in tensor memory, a row cut over several CTA pairs
- * folded by a second small launch), 1 = mma.sync tiles (widths 5-8: two row tiles per warp pair, ~1.9x the time of one
+ * scale <= 0 on mma.sync tiles), scores and output in tensor memory: rows that find a place all at once on a cluster per KV head, others
+ * cut over CTA pairs and folded by a second small launch), 1 = mma.sync tiles (widths 5-8: two row tiles per warp pair, ~1.9x the time of one
  * token per row; NVJ_ERR_UNSUPPORTED beyond 8), 2 = tcgen05 at any width 1-16 (NVJ_ERR_UNSUPPORTED without a tensor-map
  * encoder or for scale <= 0), 3 = thread-block clusters (NVJ_ERR_UNSUPPORTED but for 2-4 tokens).
  */
